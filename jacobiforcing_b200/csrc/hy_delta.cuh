@@ -1,11 +1,13 @@
-// hy_delta.cuh — gated delta rule with one decay per head, and what its neighbour in the layer needs: cosine / sine tables of
+// hy_delta.cuh — gated delta rule (one decay per head, or one per head and key channel), and what its neighbour in the layer needs: cosine / sine tables of
 // a step and the preparation of queries, rotated keys and unrotated keys-as-values (libjf_hybrid.so).
 //
 // Per head, S [dim, vdim], unit vectors k, q (q also times dim^(-1/2)), decay g and step size beta:
 //   S <- g S ;  u = beta (v - S^T k) ;  S <- S + k u^T ;  o = S^T q        (the read-out sees the current token's write)
 // Both dot products are taken over the state as the token finds it, side by side:
 //   p = S^T k, r = S^T q ;  u = beta (v - g p) ;  o = g r + (k.q) u ;  S <- g S + k u^T
-// so a token costs one pass over the state, one exchange between lanes and one update.  Value columns are independent of each
+// so a token costs one pass over the state, one exchange between lanes and one update.  With a decay per key channel the pass
+// first multiplies the state by it and g drops out of the two formulas: one more product per element, one less in the
+// update.  Value columns are independent of each
 // other, so a head is cut into blocks of 128 / PARTS columns that run side by side on different SMs, and PARTS lanes share a
 // column, each holding DR / PARTS of its key rows in registers.  With one warp per scheduler the recurrence runs at about a
 // third of the issue rate whatever the layout, so its time is its instruction count: everything that does not depend on the
@@ -104,12 +106,16 @@ __global__ void __launch_bounds__(1024) linear_rows_kernel(const AT* __restrict_
 // (see conv_kernel: w [C, taps], state [slot][taps - 1][C]), values into v [T, ldv] in the activation type, queries and keys made
 // unit vectors per head, and per head (decay, step size, k.q) into sc [T][H].  ba [T, ldba] fp32: step-size pre-activations at
 // column h, decay pre-activations at column H + h.  One block per token.
-template <typename AT, typename WT>
+// CHAN: one decay per head and key channel.  Their pre-activations stand in dec [T, ldd] (H heads of dim) and are replaced by the
+// decays; step-size pre-activations in the activation type, beta [T, ldb], column h; sc holds (unused, step size, k.q).
+template <typename AT, typename WT, bool CHAN = false>
 __global__ void __launch_bounds__(1024) delta_rows_kernel(Batch b, const AT* __restrict__ u, int ldu, int col0, int H, int G, int dim, int vdim,
                                                          int taps, const WT* __restrict__ w, const float* __restrict__ state,
                                                          const float* __restrict__ ba, int ldba, const float* __restrict__ A_log,
                                                          const float* __restrict__ dt_bias, AT* __restrict__ v, int ldv,
-                                                         float* __restrict__ qk, float4* __restrict__ sc) {
+                                                         float* __restrict__ qk, float4* __restrict__ sc,
+                                                         const AT* __restrict__ beta = nullptr, int ldb = 0, float* __restrict__ dec = nullptr,
+                                                         int ldd = 0) {
   extern __shared__ __align__(16) unsigned char hy_smem[];
   float* row = reinterpret_cast<float*>(hy_smem);              // [2 G dim] convolved queries, then keys
   const int t = blockIdx.x, e = b.tok_ent[t];
@@ -129,6 +135,11 @@ __global__ void __launch_bounds__(1024) delta_rows_kernel(Batch b, const AT* __r
     if (c < 2 * nk) row[c] = acc;
     else v[(size_t)t * ldv + c - 2 * nk] = from_f<AT>(acc);
   }
+  if (CHAN)
+    for (int i = threadIdx.x; i < H * dim; i += blockDim.x) {
+      float* d = dec + (size_t)t * ldd + i;
+      *d = expf(-expf(A_log[i / dim]) * softplus_f(*d + dt_bias[i]));
+    }
   __syncthreads();
   const int lane = threadIdx.x & 31, R = H / G;
   const float qscale = 1.0f / sqrtf((float)dim);
@@ -143,6 +154,10 @@ __global__ void __launch_bounds__(1024) delta_rows_kernel(Batch b, const AT* __r
     for (int k = lane; k < dim; k += 32) { out[k] = qr[k] * qi; out[dim + k] = kr[k] * ki; }
     for (int r = lane; r < R; r += 32) {
       const int h = g * R + r;
+      if (CHAN) {
+        sc[(size_t)t * H + h] = make_float4(1.0f, sigmoid_f(to_f(beta[(size_t)t * ldb + h])), kq * qi * ki, 0.0f);
+        continue;
+      }
       const float decay = expf(-expf(A_log[h]) * softplus_f(ba[(size_t)t * ldba + H + h] + dt_bias[h]));
       sc[(size_t)t * H + h] = make_float4(decay, sigmoid_f(ba[(size_t)t * ldba + h]), kq * qi * ki, 0.0f);
     }
@@ -184,21 +199,26 @@ __device__ __forceinline__ void copy_values(AT* dst, int dld, const AT* src, siz
   }
 }
 
-// ---- gated delta rule, one decay per head ---------------------------------------------------------------------------------------------
+// ---- gated delta rule ---------------------------------------------------------------------------------------------------------------
 // qk [T][G][q dim | k dim] and sc [T][H] from delta_rows_kernel, v [T, ldv] (H heads of vdim).  o [T, ldo] fp32 (H heads of vdim),
 // before the output norm.  state [slot][H][dim][vdim] fp32.  grid (H * blocks_per_head, entries), 128 threads.
 // Lane layout: column = warp * (32 / PARTS) + lane % (32 / PARTS), part = lane / (32 / PARTS); part r holds the key rows
 // 4 (r + PARTS i) .. + 3, so the PARTS row quadruples a warp reads from shared memory at once lie next to each other.  vec: key
 // rows are multiples of 16 bytes; vvec: a block's value rows are.
-template <typename AT, int DR, int PARTS>
+// CHAN: decays per head and key channel, dec [T, ldd] (H heads of dim), staged behind q and k.  A head in one block, a column
+// per thread (128 rows of it in registers), took 5650 us for 2048 tokens of 16 heads of 128 x 128 (16 of 148 SMs busy, one warp
+// per scheduler); cut into 16 blocks of 8 columns it is 469 us.
+template <typename AT, int DR, int PARTS, bool CHAN = false>
 __global__ void __launch_bounds__(128) delta_head_kernel(Batch b, const float* __restrict__ qk, const AT* __restrict__ v, int ldv,
                                                          const float4* __restrict__ scal, int H, int G, int dim, int vdim,
                                                          int blocks_per_head, int vec, int vvec, float* __restrict__ state,
-                                                         float* __restrict__ o, int ldo) {
+                                                         float* __restrict__ o, int ldo, const float* __restrict__ dec = nullptr,
+                                                         int ldd = 0) {
   constexpr int TB = lin_tb(DR), RP = DR / PARTS, CW = 32 / PARTS, CPB = lin_cpb(PARTS), VW = CPB < 8 ? 8 : CPB;
+  constexpr int RW = CHAN ? 3 * DR : 2 * DR;                   // floats of a staged row: q | k (| decays)
   extern __shared__ __align__(16) unsigned char hy_smem[];
-  float* sqk = reinterpret_cast<float*>(hy_smem);              // [2][TB][2 DR]
-  float4* ssc = reinterpret_cast<float4*>(sqk + 2 * TB * 2 * DR);      // [2][TB]
+  float* sqk = reinterpret_cast<float*>(hy_smem);              // [2][TB][RW]
+  float4* ssc = reinterpret_cast<float4*>(sqk + 2 * TB * RW);  // [2][TB]
   AT* sv = reinterpret_cast<AT*>(ssc + 2 * TB);                // [2][TB][VW]
   const int h = blockIdx.x / blocks_per_head, c0 = (blockIdx.x % blocks_per_head) * CPB, e = blockIdx.y;
   const int g = h / (H / G);
@@ -215,15 +235,16 @@ __global__ void __launch_bounds__(128) delta_head_kernel(Batch b, const float* _
     S[i] = (live && r < dim && pos0 > 0) ? st[(size_t)r * vdim + col] : 0.0f;
   }
   if (dim < DR)                                                // rows beyond the head's key size stay zero
-    for (int i = tid; i < 2 * TB * 2 * DR; i += 128) if (i % DR >= dim) sqk[i] = 0.0f;
+    for (int i = tid; i < 2 * TB * RW; i += 128) if (i % DR >= dim) sqk[i] = 0.0f;
   auto fetch = [&](int j0, int buf) {
     const int nb = min(TB, cnt - j0);
     const size_t t0 = (size_t)(start + j0);
-    float* d = sqk + (size_t)buf * TB * 2 * DR;
+    float* d = sqk + (size_t)buf * TB * RW;
     const float* src = qk + (t0 * G + g) * 2 * dim;
     const size_t ld = (size_t)G * 2 * dim;
-    copy_rows(d, 2 * DR, src, ld, nb, dim, vec);
-    copy_rows(d + DR, 2 * DR, src + dim, ld, nb, dim, vec);
+    copy_rows(d, RW, src, ld, nb, dim, vec);
+    copy_rows(d + DR, RW, src + dim, ld, nb, dim, vec);
+    if (CHAN) copy_rows(d + 2 * DR, RW, dec + t0 * ldd + h * dim, ldd, nb, dim, vec);
     if (tid < nb) jf::cp_async_16(ssc + buf * TB + tid, scal + (t0 + tid) * H + h, 16u);
     copy_values(sv + (size_t)buf * TB * VW, VW, v + t0 * ldv + h * vdim + c0, ldv, nb, ncol, vvec);
     jf::cp_async_commit();
@@ -235,19 +256,23 @@ __global__ void __launch_bounds__(128) delta_head_kernel(Batch b, const float* _
     jf::cp_async_wait_all();
     __syncthreads();                                           // this batch has landed; the batch before it is finished
     if (j0 + TB < cnt) fetch(j0 + TB, buf ^ 1);
-    const float* qb = sqk + (size_t)buf * TB * 2 * DR + 4 * part;
+    const float* qb = sqk + (size_t)buf * TB * RW + 4 * part;
     const AT* vb = sv + (size_t)buf * TB * VW + min(cl, ncol - 1);
     float* po = o + (size_t)(start + j0) * ldo + h * vdim + col;
     float keep = 0.0f;                                         // lane `part` keeps the read-out of token tt = part (mod PARTS)
-    float k[RP], q[RP], vv;
+    float k[RP], q[RP], a[CHAN ? RP : 1], vv;
     float4 s;
     auto rows = [&](int tt) {
 #pragma unroll
       for (int i = 0; i < RP / 4; ++i) {
-        const float4 qq = *reinterpret_cast<const float4*>(qb + tt * 2 * DR + 4 * PARTS * i);
-        const float4 kk = *reinterpret_cast<const float4*>(qb + tt * 2 * DR + DR + 4 * PARTS * i);
+        const float4 qq = *reinterpret_cast<const float4*>(qb + tt * RW + 4 * PARTS * i);
+        const float4 kk = *reinterpret_cast<const float4*>(qb + tt * RW + DR + 4 * PARTS * i);
         q[4 * i] = qq.x; q[4 * i + 1] = qq.y; q[4 * i + 2] = qq.z; q[4 * i + 3] = qq.w;
         k[4 * i] = kk.x; k[4 * i + 1] = kk.y; k[4 * i + 2] = kk.z; k[4 * i + 3] = kk.w;
+        if constexpr (CHAN) {
+          const float4 aa = *reinterpret_cast<const float4*>(qb + tt * RW + 2 * DR + 4 * PARTS * i);
+          a[4 * i] = aa.x; a[4 * i + 1] = aa.y; a[4 * i + 2] = aa.z; a[4 * i + 3] = aa.w;
+        }
       }
       s = ssc[buf * TB + tt];
       vv = to_f(vb[tt * VW]);
@@ -256,6 +281,10 @@ __global__ void __launch_bounds__(128) delta_head_kernel(Batch b, const float* _
 #pragma unroll 2
     for (int tt = 0; tt < nb; ++tt) {
       float p0 = 0.0f, p1 = 0.0f, r0 = 0.0f, r1 = 0.0f, kc[RP];
+      if constexpr (CHAN) {
+#pragma unroll
+        for (int i = 0; i < RP; ++i) S[i] *= a[i];
+      }
 #pragma unroll
       for (int i = 0; i < RP; i += 2) {
         p0 = fmaf(S[i], k[i], p0); p1 = fmaf(S[i + 1], k[i + 1], p1);
@@ -269,11 +298,11 @@ __global__ void __launch_bounds__(128) delta_head_kernel(Batch b, const float* _
       rows(min(tt + 1, nb - 1));                               // the next token's rows fly under the exchange
 #pragma unroll
       for (int x = CW; x < 32; x <<= 1) { p += __shfl_xor_sync(0xffffffffu, p, x); r += __shfl_xor_sync(0xffffffffu, r, x); }
-      const float u = sn.y * fmaf(-sn.x, p, vn);
+      const float u = CHAN ? sn.y * (vn - p) : sn.y * fmaf(-sn.x, p, vn);
 #pragma unroll
-      for (int i = 0; i < RP; ++i) S[i] = fmaf(sn.x, S[i], kc[i] * u);
+      for (int i = 0; i < RP; ++i) S[i] = CHAN ? fmaf(kc[i], u, S[i]) : fmaf(sn.x, S[i], kc[i] * u);
       const int slot = tt & (PARTS - 1);
-      if (slot == part) keep = fmaf(sn.z, u, sn.x * r);
+      if (slot == part) keep = CHAN ? fmaf(sn.z, u, r) : fmaf(sn.z, u, sn.x * r);
       if ((slot == PARTS - 1 || tt == nb - 1) && live && part <= slot) po[(size_t)(tt - slot + part) * ldo] = keep;
     }
   }

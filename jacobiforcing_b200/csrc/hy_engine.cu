@@ -483,6 +483,11 @@ void rotation_table(const hy_layer_cfg& c, std::vector<double>& f, float* mag) {
 
 struct Maxima { int in = 1, out = 1, cv = 1, f1 = 1, f2 = 1, lin = 0, lin_sc = 0; };
 
+// Whether a delta rule with a decay per key channel runs with its value columns spread over blocks (delta_head_kernel): key sizes
+// that the register layouts cover and key rows of one token that fit the row kernel's shared memory.  Other sizes keep a head's
+// state in the shared memory of one block (delta_kernel).
+bool channel_delta_columns(const hy_layer_cfg& c) { return c.d_dim <= 1024 && (size_t)2 * c.d_kv_heads * c.d_dim * 4 <= 200 * 1024; }
+
 bool tanh_norm_load(Builder& B, const std::string& name, int W, TanhNorm* n) {
   const HostTensor* w = B.get(name, W, -1);
   const HostTensor* b = B.get(name + ".b", W, -1);
@@ -650,7 +655,7 @@ int finalize_sandwich_layer(hy_engine* h, Builder& B, size_t i, Maxima& mx) {
     if (auto t = B.get(d + "lower", nq, -1)) L.g_lower = B.up_f32(t->v);
     if (auto t = B.get(d + "norm", c.g_vdim, -1)) L.g_norm = B.up_f32(t->v);
     k_out = nv;
-    mx.in = std::max(mx.in, n_in);
+    mx.in = std::max(mx.in, n_in); mx.lin = std::max(mx.lin, 2 * nq); mx.f2 = std::max(mx.f2, nv);
     if (dev_alloc(h, (void**)&L.rec_state, (size_t)rt.num_slots * H * c.g_dim * c.g_vdim * 4, &h->bytes_state)) return HY_ERR_CUDA;
   }
   const HostTensor* wo = B.get(d + "o", W, k_out);
@@ -1282,7 +1287,8 @@ extern "C" int hy_finalize(hy_handle h) {
       L.o_mix = 0; L.o_scan = nv; L.o_ff = nv;
       max_cv = std::max(max_cv, 2 * nq + nv);
       max_f1 = std::max(max_f1, c.d_heads * c.d_dim);
-      max_f2 = std::max(max_f2, nv);
+      max_f2 = std::max(max_f2, channel_delta_columns(c) ? ((nv + 3) & ~3) + nv : nv);
+      if (channel_delta_columns(c)) { mx.lin = std::max(mx.lin, 2 * nq); mx.lin_sc = std::max(mx.lin_sc, c.d_heads); }
       if (dev_alloc(h, (void**)&L.conv_state, (size_t)rt.num_slots * (c.d_conv - 1) * (2 * nq + nv) * 4, &h->bytes_state)) return HY_ERR_CUDA;
       if (dev_alloc(h, (void**)&L.rec_state, (size_t)rt.num_slots * c.d_heads * c.d_dim * c.d_vdim * 4, &h->bytes_state)) return HY_ERR_CUDA;
     }
@@ -1583,6 +1589,28 @@ const UnitList* biased_units(hy_engine* h, int E, int T, const BiasedCfg& c, int
   return w.commit(3, H, G, c.window, c.chunk, 0, ns);
 }
 
+// Register layout of a matrix-state recurrence by key size: fn(padded key size, lanes per column), both compile-time.
+constexpr int HY_LIN_MAX_DIM = 1024;
+template <typename AT, typename Fn>
+void launch_linear(int dk, Fn fn) {
+  if (dk <= 16) fn(std::integral_constant<int, 16>{}, std::integral_constant<int, 4>{});
+  else if (dk <= 32) fn(std::integral_constant<int, 32>{}, std::integral_constant<int, 8>{});
+  else if (dk <= 64) fn(std::integral_constant<int, 64>{}, std::integral_constant<int, 16>{});
+  else if (dk <= 128) fn(std::integral_constant<int, 128>{}, std::integral_constant<int, 16>{});
+  else if (dk <= 256) fn(std::integral_constant<int, 256>{}, std::integral_constant<int, 32>{});
+  else if (dk <= 512) fn(std::integral_constant<int, 512>{}, std::integral_constant<int, 32>{});
+  else fn(std::integral_constant<int, 1024>{}, std::integral_constant<int, 32>{});
+}
+
+// Blocks per head of a recurrence and which of its rows may travel by 16-byte copies.
+struct LinearLaunch { int bph, vec, vvec; };
+template <typename AT>
+LinearLaunch linear_launch(int parts, int dk, int dv, const AT* v, int ldv) {
+  const int cpb = lin_cpb(parts), ch = 16 / (int)sizeof(AT);
+  return LinearLaunch{(dv + cpb - 1) / cpb, dk % 4 == 0 ? 1 : 0,
+                      dv % ch == 0 && cpb % ch == 0 && ldv % ch == 0 && (reinterpret_cast<uintptr_t>(v) & 15) == 0 ? 1 : 0};
+}
+
 // Attention over a shared latent: down-projections in h->f1 ([query latent | key / value latent | raw rotated key part]; with
 // full-rank queries those are in h->pin already), result (heads concatenated) in h->cat.
 template <typename AT>
@@ -1747,23 +1775,25 @@ int sandwich_layer(hy_engine* h, const Batch& b, size_t li) {
       gemm<AT, WT, AT>(h, hb, W, (const WT*)L.w_in, W, T, L.n_in, W, to_buf(pin, h->ld_pin), L.w_in_t);
     }
     ProfScope ps(h, HY_PROF_DELTA);
-    static bool glr_attr = false;
-    if (!glr_attr) {
-      cudaFuncSetAttribute(glr_reg_kernel<AT, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
-      cudaFuncSetAttribute(glr_reg_kernel<AT, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
-      cudaFuncSetAttribute(glr_reg_kernel<AT, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
-      cudaFuncSetAttribute(glr_kernel<AT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-      glr_attr = true;
+    if (dk <= HY_LIN_MAX_DIM) {
+      forget_rows_kernel<AT><<<T, T <= 8 ? 1024 : 256, 0, s>>>(pin, h->ld_pin, L.c_q, L.c_k, L.g_fb, L.g_lower, H, dk, h->lin);
+      launch_linear<AT>(dk, [&](auto dr, auto parts) {
+        constexpr int DR = decltype(dr)::value, PARTS = decltype(parts)::value;
+        const LinearLaunch g = linear_launch<AT>(PARTS, dk, dv, pin + L.c_v, h->ld_pin);
+        const size_t smem = lin_smem<AT>(DR, PARTS, 0);
+        cudaFuncSetAttribute(gla_kernel<AT, DR, PARTS, GLA_FORGET>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        gla_kernel<AT, DR, PARTS, GLA_FORGET><<<dim3(H * g.bph, E), 128, smem, s>>>(b, h->lin, pin + L.c_v, h->ld_pin, nullptr, 0, nullptr, H, dk,
+                                                                                    dv, g.bph, g.vec, g.vvec, L.rec_state, h->f2, h->ld_f2);
+      });
+      gla_out_kernel<AT, AT, GATE_NONE><<<(T * H + 3) / 4, 128, 0, s>>>(T, H, dv, h->f2, h->ld_f2, nullptr, 0, L.g_norm, eps, 1.0f, cat, h->ld_cat);
+      h->launches += 3;
+    } else {
+      static bool glr_attr = false;
+      if (!glr_attr) { cudaFuncSetAttribute(glr_kernel<AT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024); glr_attr = true; }
+      glr_kernel<AT><<<dim3(H, E), 256, ((size_t)dk * dv + 2 * dk + dv + 40) * 4, s>>>(
+          b, pin, h->ld_pin, L.c_q, L.c_k, L.c_v, L.g_fb, L.g_lower, L.g_norm, H, dk, dv, eps, L.rec_state, cat, h->ld_cat);
+      h->launches++;
     }
-#define HY_GLR_ARGS b, pin, h->ld_pin, L.c_q, L.c_k, L.c_v, L.g_fb, L.g_lower, L.g_norm, H, dk, dv, eps, L.rec_state, cat, h->ld_cat
-    const int nthr = std::max(((dv + 31) / 32) * 32, 32);
-    auto gsm = [](int dr, int nt) { return (size_t)HY_GLR_TB * (2 * dr + 2 * nt) * 4; };
-    if (dk <= 32 && nthr <= 512) glr_reg_kernel<AT, 32><<<dim3(H, E), nthr, gsm(32, nthr), s>>>(HY_GLR_ARGS);
-    else if (dk <= 64 && nthr <= 512) glr_reg_kernel<AT, 64><<<dim3(H, E), nthr, gsm(64, nthr), s>>>(HY_GLR_ARGS);
-    else if (dk <= 128 && nthr <= 256) glr_reg_kernel<AT, 128><<<dim3(H, E), nthr, gsm(128, nthr), s>>>(HY_GLR_ARGS);
-    else glr_kernel<AT><<<dim3(H, E), 256, ((size_t)dk * dv + 2 * dk + dv + 40) * 4, s>>>(HY_GLR_ARGS);
-#undef HY_GLR_ARGS
-    h->launches++;
   }
   {
     ProfScope ps(h, HY_PROF_GEMM_OUT);
@@ -2318,27 +2348,6 @@ int prenorm_layer(hy_engine* h, const Batch& b, size_t li) {
   return HY_OK;
 }
 
-// Register layout of a matrix-state recurrence by key size: fn(padded key size, lanes per column), both compile-time.
-template <typename AT, typename Fn>
-void launch_linear(int dk, Fn fn) {
-  if (dk <= 16) fn(std::integral_constant<int, 16>{}, std::integral_constant<int, 4>{});
-  else if (dk <= 32) fn(std::integral_constant<int, 32>{}, std::integral_constant<int, 8>{});
-  else if (dk <= 64) fn(std::integral_constant<int, 64>{}, std::integral_constant<int, 16>{});
-  else if (dk <= 128) fn(std::integral_constant<int, 128>{}, std::integral_constant<int, 16>{});
-  else if (dk <= 256) fn(std::integral_constant<int, 256>{}, std::integral_constant<int, 32>{});
-  else if (dk <= 512) fn(std::integral_constant<int, 512>{}, std::integral_constant<int, 32>{});
-  else fn(std::integral_constant<int, 1024>{}, std::integral_constant<int, 32>{});
-}
-
-// Blocks per head of a recurrence and which of its rows may travel by 16-byte copies.
-struct LinearLaunch { int bph, vec, vvec; };
-template <typename AT>
-LinearLaunch linear_launch(int parts, int dk, int dv, const AT* v, int ldv) {
-  const int cpb = lin_cpb(parts), ch = 16 / (int)sizeof(AT);
-  return LinearLaunch{(dv + cpb - 1) / cpb, dk % 4 == 0 ? 1 : 0,
-                      dv % ch == 0 && cpb % ch == 0 && ldv % ch == 0 && (reinterpret_cast<uintptr_t>(v) & 15) == 0 ? 1 : 0};
-}
-
 // Gated linear attention: projections in h->pin (q, k, v, gate), the decay's first step in h->f1; result in h->cat.
 template <typename AT>
 void gla_mixer(hy_engine* h, const Batch& b, const LayerW& L, const hy_layer_cfg& c) {
@@ -2358,8 +2367,8 @@ void gla_mixer(hy_engine* h, const Batch& b, const LayerW& L, const hy_layer_cfg
     constexpr int DR = decltype(dr)::value, PARTS = decltype(parts)::value;
     const LinearLaunch g = linear_launch<AT>(PARTS, dk, dv, pin + L.c_v, h->ld_pin);
     const size_t smem = lin_smem<AT>(DR, PARTS, DR);
-    cudaFuncSetAttribute(gla_kernel<AT, DR, PARTS, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    gla_kernel<AT, DR, PARTS, false><<<dim3(H * g.bph, E), 128, smem, s>>>(b, h->lin, pin + L.c_v, h->ld_pin, h->f2, h->ld_f2, nullptr, H, dk,
+    cudaFuncSetAttribute(gla_kernel<AT, DR, PARTS, GLA_CHANNEL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    gla_kernel<AT, DR, PARTS, GLA_CHANNEL><<<dim3(H * g.bph, E), 128, smem, s>>>(b, h->lin, pin + L.c_v, h->ld_pin, h->f2, h->ld_f2, nullptr, H, dk,
                                                                            dv, g.bph, g.vec, g.vvec, L.rec_state, h->f2 + c_o, h->ld_f2);
   });
   gla_out_kernel<AT><<<(T * H + 3) / 4, 128, 0, s>>>(T, H, dv, h->f2 + c_o, h->ld_f2, pin + L.c_g, h->ld_pin, L.g_norm, h->m.norm_eps,
@@ -2381,8 +2390,8 @@ void retention_mixer(hy_engine* h, const Batch& b, const LayerW& L, const hy_lay
     constexpr int DR = decltype(dr)::value, PARTS = decltype(parts)::value;
     const LinearLaunch g = linear_launch<AT>(PARTS, dk, dv, pin + L.c_v, h->ld_pin);
     const size_t smem = lin_smem<AT>(DR, PARTS, 0);
-    cudaFuncSetAttribute(gla_kernel<AT, DR, PARTS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    gla_kernel<AT, DR, PARTS, true><<<dim3(H * g.bph, E), 128, smem, s>>>(b, h->lin, pin + L.c_v, h->ld_pin, nullptr, 0, L.decay, H, dk, dv,
+    cudaFuncSetAttribute(gla_kernel<AT, DR, PARTS, GLA_HEAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    gla_kernel<AT, DR, PARTS, GLA_HEAD><<<dim3(H * g.bph, E), 128, smem, s>>>(b, h->lin, pin + L.c_v, h->ld_pin, nullptr, 0, L.decay, H, dk, dv,
                                                                           g.bph, g.vec, g.vvec, L.rec_state, h->f2, h->ld_f2);
   });
   gla_out_kernel<AT><<<(T * H + 3) / 4, 128, 0, s>>>(T, H, dv, h->f2, h->ld_f2, pin + L.c_g, h->ld_pin, nullptr, h->m.norm_eps, 1.0f, cat,
@@ -2683,48 +2692,52 @@ int run_step(hy_engine* h, const Batch& b, int n_want, const int* want_d, float*
     } else {
       const int nq = c.d_kv_heads * c.d_dim, nv = c.d_heads * c.d_vdim, C = 2 * nq + nv;
       {
-      ProfScope ps(h, HY_PROF_CONV);
-      conv_kernel<AT, WT><<<dim3((C + 127) / 128, T), 128, 0, s>>>(b, pin, h->ld_pin, L.c_q, C, c.d_conv, (const WT*)L.conv_qkv,
-                                                                   (const WT*)nullptr, 1, L.conv_state, cv, h->ld_cv);
-      conv_tail_kernel<AT><<<dim3((C + 127) / 128, E), 128, 0, s>>>(b, pin, h->ld_pin, L.c_q, C, c.d_conv, L.conv_state);
+        ProfScope ps(h, HY_PROF_SMALL_GEMM);
+        gemm<AT, WT, float>(h, pin + L.c_a1, h->ld_pin, (const WT*)L.w_a2, c.d_low_a, T, c.d_heads * c.d_dim, c.d_low_a,
+                            to_buf(h->f1, h->ld_f1), L.w_a2_t);
+        gemm<AT, WT, float>(h, pin + L.c_g1, h->ld_pin, (const WT*)L.w_g2, c.d_low_g, T, nv, c.d_low_g, to_buf(h->f2, h->ld_f2),
+                            L.w_g2_t);
       }
-      h->launches += 2;
-      {
-      ProfScope ps(h, HY_PROF_SMALL_GEMM);
-      gemm<AT, WT, float>(h, pin + L.c_a1, h->ld_pin, (const WT*)L.w_a2, c.d_low_a, T, c.d_heads * c.d_dim, c.d_low_a,
-                          to_buf(h->f1, h->ld_f1), L.w_a2_t);
-      gemm<AT, WT, float>(h, pin + L.c_g1, h->ld_pin, (const WT*)L.w_g2, c.d_low_g, T, nv, c.d_low_g, to_buf(h->f2, h->ld_f2),
-                          L.w_g2_t);
-      }
-      ProfScope ps(h, HY_PROF_DELTA);
-      const int threads = ((std::max(c.d_dim, c.d_vdim) + 31) / 32) * 32;
-#define HY_DELTA_ARGS b, cv, h->ld_cv, 0, nq, 2 * nq, pin, h->ld_pin, L.c_b, h->f1, h->ld_f1, h->f2, h->ld_f2, \
-      (const float*)L.A_log, (const float*)L.dt_bias, (const float*)L.norm_w, c.d_heads, c.d_kv_heads, c.d_dim, c.d_vdim, eps, \
-      L.rec_state, cat + L.o_mix, h->ld_cat
-      static bool delta_attr = false;
-      if (!delta_attr) {
-        cudaFuncSetAttribute(delta_reg_kernel<AT, float, 32, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
-        cudaFuncSetAttribute(delta_reg_kernel<AT, float, 64, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
-        cudaFuncSetAttribute(delta_reg_kernel<AT, float, 128, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
-        delta_attr = true;
-      }
-      // one thread per value column, whole warps
-      const int nthr = std::max(((c.d_vdim + 31) / 32) * 32, 32);
-      auto dsm = [](int dr, int nt) { return (size_t)HY_DELTA_TB * (3 * dr + 3 * nt + 1) * 4; };
-      if (c.d_dim <= 32 && nthr <= 512)
-        delta_reg_kernel<AT, float, 32, 1><<<dim3(c.d_heads, E), nthr, dsm(32, nthr), s>>>(HY_DELTA_ARGS);
-      else if (c.d_dim <= 64 && nthr <= 256)
-        delta_reg_kernel<AT, float, 64, 1><<<dim3(c.d_heads, E), nthr, dsm(64, nthr), s>>>(HY_DELTA_ARGS);
-      else if (c.d_dim <= 128 && nthr <= 256)
-        delta_reg_kernel<AT, float, 128, 1><<<dim3(c.d_heads, E), nthr, dsm(128, nthr), s>>>(HY_DELTA_ARGS);
-      else {
-        const size_t smem = ((size_t)c.d_dim * c.d_vdim + 3 * c.d_dim + 40) * 4;
+      const int H = c.d_heads, G = c.d_kv_heads, dk = c.d_dim, dv = c.d_vdim;
+      if (channel_delta_columns(c)) {
+        {
+          ProfScope ps(h, HY_PROF_CONV);
+          static bool attr = false;                          // per AT: this function is a template
+          if (!attr) { cudaFuncSetAttribute(delta_rows_kernel<AT, WT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024); attr = true; }
+          delta_rows_kernel<AT, WT, true><<<T, T <= 8 ? 1024 : 256, (size_t)2 * nq * 4, s>>>(
+              b, pin, h->ld_pin, L.c_q, H, G, dk, dv, c.d_conv, (const WT*)L.conv_qkv, L.conv_state, nullptr, 0, (const float*)L.A_log,
+              (const float*)L.dt_bias, cv, h->ld_cv, h->lin, h->lin_sc, pin + L.c_b, h->ld_pin, h->f1, h->ld_f1);
+          conv_tail_kernel<AT><<<dim3((C + 127) / 128, E), 128, 0, s>>>(b, pin, h->ld_pin, L.c_q, C, c.d_conv, L.conv_state);
+        }
+        ProfScope ps(h, HY_PROF_DELTA);
+        float* o = h->f2 + ((nv + 3) & ~3);                  // behind the output gates
+        launch_linear<AT>(dk, [&](auto dr, auto parts) {
+          constexpr int DR = decltype(dr)::value, PARTS = decltype(parts)::value;
+          const LinearLaunch g = linear_launch<AT>(PARTS, dk, dv, cv, h->ld_cv);
+          const size_t smem = lin_smem<AT>(DR, PARTS, DR + 4);
+          cudaFuncSetAttribute(delta_head_kernel<AT, DR, PARTS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+          delta_head_kernel<AT, DR, PARTS, true><<<dim3(H * g.bph, E), 128, smem, s>>>(b, h->lin, cv, h->ld_cv, h->lin_sc, H, G, dk, dv, g.bph,
+                                                                                       g.vec, g.vvec, L.rec_state, o, h->ld_f2, h->f1, h->ld_f1);
+        });
+        gla_out_kernel<AT, float, GATE_SIGMOID><<<(T * H + 3) / 4, 128, 0, s>>>(T, H, dv, o, h->ld_f2, h->f2, h->ld_f2, (const float*)L.norm_w, eps,
+                                                                                1.0f, cat + L.o_mix, h->ld_cat);
+        h->launches += 4;
+      } else {
+        {
+          ProfScope ps(h, HY_PROF_CONV);
+          conv_kernel<AT, WT><<<dim3((C + 127) / 128, T), 128, 0, s>>>(b, pin, h->ld_pin, L.c_q, C, c.d_conv, (const WT*)L.conv_qkv,
+                                                                       (const WT*)nullptr, 1, L.conv_state, cv, h->ld_cv);
+          conv_tail_kernel<AT><<<dim3((C + 127) / 128, E), 128, 0, s>>>(b, pin, h->ld_pin, L.c_q, C, c.d_conv, L.conv_state);
+        }
+        ProfScope ps(h, HY_PROF_DELTA);
         static bool dk_attr = false;
         if (!dk_attr) { cudaFuncSetAttribute(delta_kernel<AT, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024); dk_attr = true; }
-        delta_kernel<AT, float><<<dim3(c.d_heads, E), threads, smem, s>>>(HY_DELTA_ARGS);
+        const int threads = ((std::max(dk, dv) + 31) / 32) * 32;
+        delta_kernel<AT, float><<<dim3(H, E), threads, ((size_t)dk * dv + 3 * dk + 40) * 4, s>>>(
+            b, cv, h->ld_cv, 0, nq, 2 * nq, pin, h->ld_pin, L.c_b, h->f1, h->ld_f1, h->f2, h->ld_f2, (const float*)L.A_log,
+            (const float*)L.dt_bias, (const float*)L.norm_w, H, G, dk, dv, eps, L.rec_state, cat + L.o_mix, h->ld_cat);
+        h->launches += 3;
       }
-#undef HY_DELTA_ARGS
-      h->launches++;
     }
     (void)ff;
     // merged output projections, added to the residual stream

@@ -1,6 +1,7 @@
 // hy_gla.cuh — gated linear attention with one decay per key channel, retention (one fixed decay per head, rotated queries and
 // keys), and the row kernels between the sublayers of blocks with plain RMS weights (libjf_hybrid.so).
 //
+// and the gated linear recurrence whose forget gate also sets what is written.
 // Per head, S [dim, vdim]:  S <- diag(a) S + k v^T ;  o = S^T q dim^(-1/2)   (the read-out sees the current token's write)
 //   out = o / rms(o) * norm_w * silu(g)        (norm over the head's vdim, one weight shared by the heads)
 // The decay a = sigmoid(z)^(1 / tau) leaves the decay projection's epilogue as fp32 (gemm_store).  Retention is the same
@@ -19,15 +20,19 @@
 namespace hy {
 
 // qk [T][H][q dim | k dim] fp32 from linear_rows_kernel, v [T, ldv] (H heads of vdim).  Decays: decay [T, ldd] fp32 (H heads of dim),
-// or with HEAD one number per head, head_decay [H].  o [T, ldo] fp32 (H heads of vdim).  state [slot][H][dim][vdim] fp32.
+// or with GLA_HEAD one number per head, head_decay [H].  With GLA_FORGET the rows hold [q | f] (forget_rows_kernel) and the
+// update is S <- f S + (1 - f) v^T, written as v + f (S - v).  o [T, ldo] fp32 (H heads of vdim).  state [slot][H][dim][vdim] fp32.
 // grid (H * blocks_per_head, entries), 128 threads.  Lane layout, vec and vvec as in delta_head_kernel.
-template <typename AT, int DR, int PARTS, bool HEAD>
+// GLA_FORGET, 2048 tokens of 8 heads of 128 x 128: one block per head with a column per thread took 1927 us, this layout 202 us.
+enum GlaMode : int { GLA_CHANNEL = 0, GLA_HEAD = 1, GLA_FORGET = 2 };
+template <typename AT, int DR, int PARTS, int MODE>
 __global__ void __launch_bounds__(128) gla_kernel(Batch b, const float* __restrict__ qk, const AT* __restrict__ v, int ldv,
                                                   const float* __restrict__ decay, int ldd, const float* __restrict__ head_decay, int H,
                                                   int dim, int vdim, int blocks_per_head, int vec, int vvec, float* __restrict__ state,
                                                   float* __restrict__ o, int ldo) {
   constexpr int TB = lin_tb(DR), RP = DR / PARTS, CW = 32 / PARTS, CPB = lin_cpb(PARTS), VW = CPB < 8 ? 8 : CPB;
-  constexpr int RW = HEAD ? 2 * DR : 3 * DR;                   // floats of a staged row: q | k (| decays)
+  constexpr bool HEAD = MODE == GLA_HEAD;
+  constexpr int RW = MODE == GLA_CHANNEL ? 3 * DR : 2 * DR;    // floats of a staged row: q | k (| decays)
   extern __shared__ __align__(16) unsigned char hy_smem[];
   float* sqk = reinterpret_cast<float*>(hy_smem);              // [2][TB][RW]
   AT* sv = reinterpret_cast<AT*>(sqk + 2 * TB * RW);           // [2][TB][VW]
@@ -55,7 +60,7 @@ __global__ void __launch_bounds__(128) gla_kernel(Batch b, const float* __restri
     const size_t ld = (size_t)H * 2 * dim;
     copy_rows(d, RW, src, ld, nb, dim, vec);
     copy_rows(d + DR, RW, src + dim, ld, nb, dim, vec);
-    if (!HEAD) copy_rows(d + 2 * DR, RW, decay + t0 * ldd + h * dim, ldd, nb, dim, vec);
+    if (MODE == GLA_CHANNEL) copy_rows(d + 2 * DR, RW, decay + t0 * ldd + h * dim, ldd, nb, dim, vec);
     copy_values(sv + (size_t)buf * TB * VW, VW, v + t0 * ldv + h * vdim + c0, ldv, nb, ncol, vvec);
     jf::cp_async_commit();
   };
@@ -78,8 +83,15 @@ __global__ void __launch_bounds__(128) gla_kernel(Batch b, const float* __restri
       for (int i = 0; i < RP / 4; ++i) {
         const float4 q = *reinterpret_cast<const float4*>(rb + tt * RW + 4 * PARTS * i);
         const float4 k = *reinterpret_cast<const float4*>(rb + tt * RW + DR + 4 * PARTS * i);
-        const float4 a = HEAD ? make_float4(hd, hd, hd, hd) : *reinterpret_cast<const float4*>(rb + tt * RW + 2 * DR + 4 * PARTS * i);
         float* R = &S[4 * i];
+        if constexpr (MODE == GLA_FORGET) {
+          R[0] = fmaf(k.x, R[0] - vv, vv); p0 = fmaf(R[0], q.x, p0);
+          R[1] = fmaf(k.y, R[1] - vv, vv); p1 = fmaf(R[1], q.y, p1);
+          R[2] = fmaf(k.z, R[2] - vv, vv); p0 = fmaf(R[2], q.z, p0);
+          R[3] = fmaf(k.w, R[3] - vv, vv); p1 = fmaf(R[3], q.w, p1);
+          continue;
+        }
+        const float4 a = HEAD ? make_float4(hd, hd, hd, hd) : *reinterpret_cast<const float4*>(rb + tt * RW + (MODE == GLA_CHANNEL ? 2 * DR : 0) + 4 * PARTS * i);
         R[0] = fmaf(a.x, R[0], k.x * vv); p0 = fmaf(R[0], q.x, p0);
         R[1] = fmaf(a.y, R[1], k.y * vv); p1 = fmaf(R[1], q.y, p1);
         R[2] = fmaf(a.z, R[2], k.z * vv); p0 = fmaf(R[2], q.z, p0);
@@ -132,10 +144,27 @@ __global__ void __launch_bounds__(128) gla_kernel(Batch b, const float* __restri
   }
 }
 
-// Norm per head, weight (NULL: none), output gate: out[t, h, :] = o / rms(o) * w * silu(g) * out_scale.  One warp per (token, head).
+// Operand rows of the recurrence with a forget gate: [T][H][silu(q) | f], f = lower + (1 - lower) sigmoid(f_raw + f_bias).
 template <typename AT>
+__global__ void __launch_bounds__(1024) forget_rows_kernel(const AT* __restrict__ in, int ld, int col_q, int col_f,
+                                                           const float* __restrict__ f_bias, const float* __restrict__ lower, int H, int dim,
+                                                           float* __restrict__ qf) {
+  const AT* row = in + (size_t)blockIdx.x * ld;
+  float* out = qf + (size_t)blockIdx.x * H * 2 * dim;
+  for (int i = threadIdx.x; i < H * dim; i += blockDim.x) {
+    const size_t at = (size_t)(i / dim) * 2 * dim + i % dim;
+    const float lo = lower[i];
+    out[at] = silu_f(to_f(row[col_q + i]));
+    out[at + dim] = fmaf(1.0f - lo, sigmoid_f(to_f(row[col_f + i]) + f_bias[i]), lo);
+  }
+}
+
+// Norm per head, weight (NULL: none), output gate: out[t, h, :] = o / rms(o) * w * gate * out_scale, gate = silu(g), sigmoid(g) or one.
+// One warp per (token, head).
+enum OutGate : int { GATE_SILU = 0, GATE_SIGMOID = 1, GATE_NONE = 2 };
+template <typename AT, typename GT = AT, int GATE = GATE_SILU>
 __global__ void __launch_bounds__(128) gla_out_kernel(int T, int H, int vdim, const float* __restrict__ o, int ldi,
-                                                      const AT* __restrict__ g, int ldg, const float* __restrict__ w, float eps,
+                                                      const GT* __restrict__ g, int ldg, const float* __restrict__ w, float eps,
                                                       float out_scale, AT* __restrict__ out, int ldo) {
   const int unit = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (unit >= T * H) return;
@@ -144,8 +173,12 @@ __global__ void __launch_bounds__(128) gla_out_kernel(int T, int H, int vdim, co
   float ss = 0.0f;
   for (int k = lane; k < vdim; k += 32) ss = fmaf(orow[k], orow[k], ss);
   const float inv = out_scale / sqrtf(warp_sum(ss) / (float)vdim + eps);
-  for (int k = lane; k < vdim; k += 32)
-    out[t * ldo + c0 + k] = from_f<AT>(orow[k] * inv * (w ? w[k] : 1.0f) * silu_f(to_f(g[t * ldg + c0 + k])));
+  for (int k = lane; k < vdim; k += 32) {
+    float v = orow[k] * inv * (w ? w[k] : 1.0f);
+    if constexpr (GATE == GATE_SILU) v *= silu_f(to_f(g[t * ldg + c0 + k]));
+    else if constexpr (GATE == GATE_SIGMOID) v *= sigmoid_f(to_f(g[t * ldg + c0 + k]));
+    out[t * ldo + c0 + k] = from_f<AT>(v);
+  }
 }
 
 // ---- one token's row between two sublayers ----------------------------------------------------------------------------------

@@ -655,122 +655,6 @@ __device__ __forceinline__ float2 block_sum2(float a, float b, float* red) {
   return make_float2(red[32], red[65]);
 }
 
-// The same recurrence with thread j keeping column j of S in registers (key size <= DR): no shared-memory traffic for
-// the state, four partial sums per dot product so the per-token chain is short.  Same results up to summation order.
-// Inputs of HY_DELTA_TB tokens are staged by the whole block; unit vectors and decays of those tokens are made by one
-// warp per token (shuffles only), the per-token recurrence then runs without any block barrier, and the output norms of
-// the batch are again made by one warp per token: four barriers per batch of tokens instead of seven per token.
-constexpr int HY_DELTA_TB = 16;
-
-// PARTS neighbouring lanes share a column of S, each keeping DR / PARTS of its rows in registers (PARTS > 1 ends each dot
-// product in log2(PARTS) shuffles).  Measured at key size 128, 128 value columns: PARTS = 1 (one warp per scheduler, 128
-// rows in registers) 2.1 us per token, PARTS = 4 (four warps per scheduler) 3.6 us: the chain through shuffles and the
-// read-out store costs more than the shorter loops save, so the dispatcher uses PARTS = 1.
-template <typename AT, typename WT, int DR, int PARTS>
-__global__ void __launch_bounds__(DR / PARTS > 32 ? 256 : 512)
-delta_reg_kernel(Batch b, const AT* __restrict__ qkv, int ldq, int col_q, int col_k, int col_v,
-                 const AT* __restrict__ beta_in, int ldb, int col_beta, const float* __restrict__ a_in, int lda,
-                 const float* __restrict__ gate_in, int ldg, const WT* __restrict__ A_log, const WT* __restrict__ dt_bias,
-                 const WT* __restrict__ norm_w, int H, int G, int dim, int vdim, float eps, float* __restrict__ state,
-                 AT* __restrict__ out, int ldo) {
-  constexpr int RP = DR / PARTS;
-  extern __shared__ __align__(16) unsigned char hy_smem[];
-  const int nt = blockDim.x, nwarps = nt >> 5, nc = nt / PARTS;
-  float* sq = reinterpret_cast<float*>(hy_smem);               // [TB][DR] unit queries (times dim^-1/2)
-  float* skk = sq + HY_DELTA_TB * DR;                           // [TB][DR] unit keys
-  float* sa = skk + HY_DELTA_TB * DR;                           // [TB][DR] decays
-  float* sv = sa + HY_DELTA_TB * DR;                            // [TB][nc] values
-  float* sg = sv + HY_DELTA_TB * nc;                            // [TB][nc] output gates (pre-sigmoid)
-  float* so = sg + HY_DELTA_TB * nc;                            // [TB][nc] raw read-outs
-  float* sbeta = so + HY_DELTA_TB * nc;                         // [TB]
-  const int h = blockIdx.x, e = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int jc = tid / PARTS, r0 = (tid % PARTS) * RP;
-  const int g = h / (H / G);
-  const int start = b.ent_start[e], cnt = b.ent_start[e + 1] - start, pos0 = b.ent_pos0[e];
-  float* st = state + ((size_t)b.ent_slot[e] * H + h) * dim * vdim;
-  const bool col = jc < vdim;
-  float S[RP];
-#pragma unroll
-  for (int i = 0; i < RP; ++i) S[i] = (col && r0 + i < dim && pos0 > 0) ? st[(size_t)(r0 + i) * vdim + jc] : 0.0f;
-  const float rate = expf(to_f(A_log[h]));
-  const float qscale = rsqrtf((float)dim);
-  for (int j0 = 0; j0 < cnt; j0 += HY_DELTA_TB) {
-    const int nb = min(HY_DELTA_TB, cnt - j0);
-    __syncthreads();                                           // the previous batch is finished with the staging area
-    for (int i = tid; i < nb * DR; i += nt) {
-      const int tt = i / DR, k = i % DR;
-      const size_t t = (size_t)(start + j0 + tt);
-      const bool ok = k < dim;
-      sq[i] = ok ? to_f(qkv[t * ldq + col_q + g * dim + k]) : 0.0f;
-      skk[i] = ok ? to_f(qkv[t * ldq + col_k + g * dim + k]) : 0.0f;
-      sa[i] = ok ? expf(-rate * softplus_f(a_in[t * lda + h * dim + k] + to_f(dt_bias[h * dim + k]))) : 1.0f;
-    }
-    for (int i = tid; i < nb * nc; i += nt) {
-      const int tt = i / nc, k = i % nc;
-      const size_t t = (size_t)(start + j0 + tt);
-      sv[i] = k < vdim ? to_f(qkv[t * ldq + col_v + h * vdim + k]) : 0.0f;
-      sg[i] = k < vdim ? gate_in[t * ldg + h * vdim + k] : 0.0f;
-    }
-    if (tid < nb) sbeta[tid] = sigmoid_f(to_f(beta_in[(size_t)(start + j0 + tid) * ldb + col_beta + h]));
-    __syncthreads();
-    for (int tt = warp; tt < nb; tt += nwarps) {               // unit vectors: one warp per token
-      float q2 = 0.0f, k2 = 0.0f;
-      for (int k = lane; k < DR; k += 32) { q2 = fmaf(sq[tt * DR + k], sq[tt * DR + k], q2); k2 = fmaf(skk[tt * DR + k], skk[tt * DR + k], k2); }
-      q2 = warp_sum(q2); k2 = warp_sum(k2);
-      const float qi = qscale / sqrtf(q2 + 1e-6f), ki = 1.0f / sqrtf(k2 + 1e-6f);
-      for (int k = lane; k < DR; k += 32) { sq[tt * DR + k] *= qi; skk[tt * DR + k] *= ki; }
-    }
-    __syncthreads();
-    for (int tt = 0; tt < nb; ++tt) {
-      const float* gs = sa + tt * DR + r0;
-      const float* ks = skk + tt * DR + r0;
-      const float* qs = sq + tt * DR + r0;
-      float p0 = 0.0f, p1 = 0.0f, p2 = 0.0f, p3 = 0.0f;
-#pragma unroll
-      for (int i = 0; i < RP; i += 4) {
-        const float4 g4 = *reinterpret_cast<const float4*>(&gs[i]);
-        const float4 k4 = *reinterpret_cast<const float4*>(&ks[i]);
-        S[i] *= g4.x; S[i + 1] *= g4.y; S[i + 2] *= g4.z; S[i + 3] *= g4.w;
-        p0 = fmaf(S[i], k4.x, p0); p1 = fmaf(S[i + 1], k4.y, p1);
-        p2 = fmaf(S[i + 2], k4.z, p2); p3 = fmaf(S[i + 3], k4.w, p3);
-      }
-      float sk = (p0 + p1) + (p2 + p3);
-#pragma unroll
-      for (int o = 1; o < PARTS; o <<= 1) sk += __shfl_xor_sync(0xffffffffu, sk, o);
-      const float u = sbeta[tt] * (sv[tt * nc + jc] - sk);
-      p0 = p1 = p2 = p3 = 0.0f;
-#pragma unroll
-      for (int i = 0; i < RP; i += 4) {
-        const float4 k4 = *reinterpret_cast<const float4*>(&ks[i]);
-        const float4 q4 = *reinterpret_cast<const float4*>(&qs[i]);
-        S[i] = fmaf(k4.x, u, S[i]); S[i + 1] = fmaf(k4.y, u, S[i + 1]);
-        S[i + 2] = fmaf(k4.z, u, S[i + 2]); S[i + 3] = fmaf(k4.w, u, S[i + 3]);
-        p0 = fmaf(S[i], q4.x, p0); p1 = fmaf(S[i + 1], q4.y, p1);
-        p2 = fmaf(S[i + 2], q4.z, p2); p3 = fmaf(S[i + 3], q4.w, p3);
-      }
-      float ov = (p0 + p1) + (p2 + p3);
-#pragma unroll
-      for (int o = 1; o < PARTS; o <<= 1) ov += __shfl_xor_sync(0xffffffffu, ov, o);
-      if (tid % PARTS == 0) so[tt * nc + jc] = ov;
-    }
-    __syncthreads();
-    for (int tt = warp; tt < nb; tt += nwarps) {               // output norm and gate: one warp per token
-      float o2 = 0.0f;
-      for (int k = lane; k < vdim; k += 32) o2 = fmaf(so[tt * nc + k], so[tt * nc + k], o2);
-      o2 = warp_sum(o2);
-      const float inv = 1.0f / sqrtf(o2 / (float)vdim + eps);
-      for (int k = lane; k < vdim; k += 32)
-        out[(size_t)(start + j0 + tt) * ldo + h * vdim + k] =
-            from_f<AT>(so[tt * nc + k] * inv * to_f(norm_w[k]) * sigmoid_f(sg[tt * nc + k]));
-    }
-  }
-  if (col) {
-#pragma unroll
-    for (int i = 0; i < RP; ++i)
-      if (r0 + i < dim) st[(size_t)(r0 + i) * vdim + jc] = S[i];
-  }
-}
-
 // ---- sampling: argmax, or Gumbel-max at a temperature with a counter-based generator ---------------------------------------------
 __device__ __forceinline__ uint32_t mix32(uint64_t key, uint32_t ctr) {
   uint64_t z = key + 0x9E3779B97F4A7C15ull * (uint64_t)(ctr + 1);

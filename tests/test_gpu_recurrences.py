@@ -1,0 +1,49 @@
+"""Recurrences whose value columns are spread over blocks, at the edges of their layouts: key sizes at and beside the padded sizes,
+value columns that fill a block's eight, miss one or need another block, portions that end at, before and behind a staged
+batch, and the size behind which another kernel takes over; fp32 build against the plain fp64 restatements, within the
+bound of the other fp32 tests (3e-4)."""
+import pytest
+
+from oracle import famepel_plain, kinetar_plain
+from tests import famepel_helpers as fam
+from tests import hybrid_helpers as kin
+
+pytestmark = pytest.mark.gpu
+
+CUTS = [31, 1, 33, 2, 32, 8, 64]                               # staged batches hold 32 tokens (16 or fewer at large key sizes)
+
+
+def _kinetar(layer, cuts=CUTS, width=48):
+    cfg = kin.model_config([layer], width=width)
+    toks = kin.rand_tokens(sum(cuts), cfg["vocab"], 3)
+    w = kinetar_plain.random_weights(cfg, 0, 8)
+    hz = kin.Harness(cfg, w, dtype="float32", low=8)
+    try:
+        got = hz.feed("a", toks, cuts)
+    finally:
+        hz.close()
+    return kin.rel_err(got, kin.oracle_logits(cfg, w, toks))
+
+
+@pytest.mark.parametrize("dim,vdim,heads,kv", [(16, 8, 4, 2), (17, 7, 2, 1), (32, 9, 2, 2), (33, 1, 3, 1), (64, 16, 1, 1), (128, 24, 2, 1),
+                                               (130, 12, 2, 1), (257, 8, 1, 1), (600, 10, 1, 1)])
+def test_channel_delta_columns(dim, vdim, heads, kv):
+    assert _kinetar(kin.delta(heads=heads, kv_heads=kv, dim=dim, vdim=vdim, ff=0)) < kin.TOL["float32"]
+
+
+def test_channel_delta_beside_the_row_kernels_limit():
+    """Key rows of one token that no longer fit the row kernel's shared memory: a head's state in one block."""
+    assert _kinetar(kin.delta(heads=52, kv_heads=26, dim=1000, vdim=4, ff=0), cuts=[5, 1, 3], width=16) < kin.TOL["float32"]
+
+
+@pytest.mark.parametrize("dim,vdim", [(16, 8), (15, 7), (33, 9), (64, 1), (128, 40), (136, 8), (520, 3), (1030, 5)])
+def test_forget_gate_columns(dim, vdim):
+    cfg = fam.model_config([fam.glr(heads=2, dim=dim, vdim=vdim, mlp=None)])
+    toks = kin.rand_tokens(sum(CUTS), cfg["vocab"], 4)
+    w = famepel_plain.random_weights(cfg, 0)
+    hz = fam.Harness(cfg, w, "float32")
+    try:
+        got = hz.feed("a", toks, CUTS)
+    finally:
+        hz.close()
+    assert kin.rel_err(got, fam.oracle_logits(cfg, w, toks)) < fam.TOL["float32"]
