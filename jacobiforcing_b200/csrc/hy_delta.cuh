@@ -102,65 +102,40 @@ __global__ void __launch_bounds__(1024) linear_rows_kernel(const AT* __restrict_
   }
 }
 
-// The delta rule's: causal convolution over time with silu of the columns [q (G heads of dim) | k | v (H heads of vdim)] at col0
-// (see conv_kernel: w [C, taps], state [slot][taps - 1][C]), values into v [T, ldv] in the activation type, queries and keys made
-// unit vectors per head, and per head (decay, step size, k.q) into sc [T][H].  ba [T, ldba] fp32: step-size pre-activations at
-// column h, decay pre-activations at column H + h.  One block per token.
+// The delta rule's: conv_kernel has left the convolved queries and keys in qk [T][G][q dim | k dim]; they are made unit vectors per
+// head (queries times dim^(-1/2)) in place, and (decay, step size, k.q) go into sc [T][H].  ba [T, ldba] fp32: step-size
+// pre-activations at column h, decay pre-activations at column H + h.  One warp per (token, key head).
 // CHAN: one decay per head and key channel.  Their pre-activations stand in dec [T, ldd] (H heads of dim) and are replaced by the
 // decays; step-size pre-activations in the activation type, beta [T, ldb], column h; sc holds (unused, step size, k.q).
-template <typename AT, typename WT, bool CHAN = false>
-__global__ void __launch_bounds__(1024) delta_rows_kernel(Batch b, const AT* __restrict__ u, int ldu, int col0, int H, int G, int dim, int vdim,
-                                                         int taps, const WT* __restrict__ w, const float* __restrict__ state,
-                                                         const float* __restrict__ ba, int ldba, const float* __restrict__ A_log,
-                                                         const float* __restrict__ dt_bias, AT* __restrict__ v, int ldv,
-                                                         float* __restrict__ qk, float4* __restrict__ sc,
-                                                         const AT* __restrict__ beta = nullptr, int ldb = 0, float* __restrict__ dec = nullptr,
-                                                         int ldd = 0) {
-  extern __shared__ __align__(16) unsigned char hy_smem[];
-  float* row = reinterpret_cast<float*>(hy_smem);              // [2 G dim] convolved queries, then keys
-  const int t = blockIdx.x, e = b.tok_ent[t];
-  const int start = b.ent_start[e], pos0 = b.ent_pos0[e], j = t - start;
-  const int nk = G * dim, C = 2 * nk + H * vdim;
-  const float* st = state + (size_t)b.ent_slot[e] * (taps - 1) * C;
-  for (int c = threadIdx.x; c < C; c += blockDim.x) {
-    float acc = 0.0f;
-    for (int i = 0; i < taps; ++i) {
-      const int src = j - (taps - 1) + i;
-      float x = 0.0f;
-      if (src >= 0) x = to_f(u[(size_t)(start + src) * ldu + col0 + c]);
-      else if (pos0 + src >= 0) x = st[(size_t)(taps - 1 + src) * C + c];
-      acc = fmaf(to_f(w[(size_t)c * taps + i]), x, acc);
-    }
-    acc = silu_f(acc);
-    if (c < 2 * nk) row[c] = acc;
-    else v[(size_t)t * ldv + c - 2 * nk] = from_f<AT>(acc);
+template <typename AT, bool CHAN>
+__global__ void __launch_bounds__(128) delta_unit_kernel(int T, int H, int G, int dim, const float* __restrict__ ba, int ldba,
+                                                         const float* __restrict__ A_log, const float* __restrict__ dt_bias,
+                                                         const AT* __restrict__ beta, int ldb, float* __restrict__ dec, int ldd,
+                                                         float* __restrict__ qk, float4* __restrict__ sc) {
+  const int unit = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31, R = H / G;
+  if (unit >= T * G) return;
+  const size_t t = unit / G;
+  const int g = unit % G;
+  float* row = qk + (size_t)unit * 2 * dim;
+  float q2 = 0.0f, k2 = 0.0f, kq = 0.0f;
+  for (int k = lane; k < dim; k += 32) {
+    const float q = row[k], kk = row[dim + k];
+    q2 = fmaf(q, q, q2); k2 = fmaf(kk, kk, k2); kq = fmaf(q, kk, kq);
   }
   if (CHAN)
-    for (int i = threadIdx.x; i < H * dim; i += blockDim.x) {
-      float* d = dec + (size_t)t * ldd + i;
-      *d = expf(-expf(A_log[i / dim]) * softplus_f(*d + dt_bias[i]));
+    for (int i = lane; i < R * dim; i += 32) {
+      const int h = g * R + i / dim;
+      float* d = dec + t * ldd + g * R * dim + i;
+      *d = expf(-expf(A_log[h]) * softplus_f(*d + dt_bias[g * R * dim + i]));
     }
-  __syncthreads();
-  const int lane = threadIdx.x & 31, R = H / G;
-  const float qscale = 1.0f / sqrtf((float)dim);
-  for (int g = threadIdx.x >> 5; g < G; g += blockDim.x >> 5) {
-    const float* qr = row + g * dim;
-    const float* kr = row + nk + g * dim;
-    float q2 = 0.0f, k2 = 0.0f, kq = 0.0f;
-    for (int k = lane; k < dim; k += 32) { q2 = fmaf(qr[k], qr[k], q2); k2 = fmaf(kr[k], kr[k], k2); kq = fmaf(qr[k], kr[k], kq); }
-    q2 = warp_sum(q2); k2 = warp_sum(k2); kq = warp_sum(kq);
-    const float qi = qscale / sqrtf(q2 + 1e-6f), ki = 1.0f / sqrtf(k2 + 1e-6f);
-    float* out = qk + ((size_t)t * G + g) * 2 * dim;
-    for (int k = lane; k < dim; k += 32) { out[k] = qr[k] * qi; out[dim + k] = kr[k] * ki; }
-    for (int r = lane; r < R; r += 32) {
-      const int h = g * R + r;
-      if (CHAN) {
-        sc[(size_t)t * H + h] = make_float4(1.0f, sigmoid_f(to_f(beta[(size_t)t * ldb + h])), kq * qi * ki, 0.0f);
-        continue;
-      }
-      const float decay = expf(-expf(A_log[h]) * softplus_f(ba[(size_t)t * ldba + H + h] + dt_bias[h]));
-      sc[(size_t)t * H + h] = make_float4(decay, sigmoid_f(ba[(size_t)t * ldba + h]), kq * qi * ki, 0.0f);
-    }
+  q2 = warp_sum(q2); k2 = warp_sum(k2); kq = warp_sum(kq);
+  const float qi = 1.0f / sqrtf((float)dim) / sqrtf(q2 + 1e-6f), ki = 1.0f / sqrtf(k2 + 1e-6f);
+  for (int k = lane; k < dim; k += 32) { row[k] *= qi; row[dim + k] *= ki; }
+  for (int r = lane; r < R; r += 32) {
+    const int h = g * R + r;
+    const float step = sigmoid_f(CHAN ? to_f(beta[t * ldb + h]) : ba[t * ldba + h]);
+    const float decay = CHAN ? 1.0f : expf(-expf(A_log[h]) * softplus_f(ba[t * ldba + H + h] + dt_bias[h]));
+    sc[t * H + h] = make_float4(decay, step, kq * qi * ki, 0.0f);
   }
 }
 
@@ -200,7 +175,7 @@ __device__ __forceinline__ void copy_values(AT* dst, int dld, const AT* src, siz
 }
 
 // ---- gated delta rule ---------------------------------------------------------------------------------------------------------------
-// qk [T][G][q dim | k dim] and sc [T][H] from delta_rows_kernel, v [T, ldv] (H heads of vdim).  o [T, ldo] fp32 (H heads of vdim),
+// qk [T][G][q dim | k dim] and sc [T][H] from delta_unit_kernel, v [T, ldv] (H heads of vdim).  o [T, ldo] fp32 (H heads of vdim),
 // before the output norm.  state [slot][H][dim][vdim] fp32.  grid (H * blocks_per_head, entries), 128 threads.
 // Lane layout: column = warp * (32 / PARTS) + lane % (32 / PARTS), part = lane / (32 / PARTS); part r holds the key rows
 // 4 (r + PARTS i) .. + 3, so the PARTS row quadruples a warp reads from shared memory at once lie next to each other.  vec: key

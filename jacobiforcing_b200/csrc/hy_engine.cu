@@ -483,11 +483,6 @@ void rotation_table(const hy_layer_cfg& c, std::vector<double>& f, float* mag) {
 
 struct Maxima { int in = 1, out = 1, cv = 1, f1 = 1, f2 = 1, lin = 0, lin_sc = 0; };
 
-// Whether a delta rule with a decay per key channel runs with its value columns spread over blocks (delta_head_kernel): key sizes
-// that the register layouts cover and key rows of one token that fit the row kernel's shared memory.  Other sizes keep a head's
-// state in the shared memory of one block (delta_kernel).
-bool channel_delta_columns(const hy_layer_cfg& c) { return c.d_dim <= 1024 && (size_t)2 * c.d_kv_heads * c.d_dim * 4 <= 200 * 1024; }
-
 bool tanh_norm_load(Builder& B, const std::string& name, int W, TanhNorm* n) {
   const HostTensor* w = B.get(name, W, -1);
   const HostTensor* b = B.get(name + ".b", W, -1);
@@ -620,7 +615,7 @@ int finalize_sandwich_layer(hy_engine* h, Builder& B, size_t i, Maxima& mx) {
     if (auto t = B.get(d + "D", H, -1)) L.m_D = B.up_f32(t->v);
     if (auto t = B.get(d + "norm", inner, -1)) L.m_norm = B.up_f32(t->v);
     k_out = inner;
-    mx.in = std::max(mx.in, n_in); mx.cv = std::max(mx.cv, C); mx.f2 = std::max(mx.f2, inner);
+    mx.in = std::max(mx.in, n_in); mx.cv = std::max(mx.cv, inner); mx.f2 = std::max(mx.f2, inner); mx.lin = std::max(mx.lin, 2 * GN);
     if (dev_alloc(h, (void**)&L.conv_state, (size_t)rt.num_slots * (c.m_conv - 1) * C * 4, &h->bytes_state)) return HY_ERR_CUDA;
     if (dev_alloc(h, (void**)&L.rec_state, (size_t)rt.num_slots * inner * c.m_state * 4, &h->bytes_state)) return HY_ERR_CUDA;
   } else if (c.mixer == HY_MIX_LATENT) {
@@ -1287,8 +1282,8 @@ extern "C" int hy_finalize(hy_handle h) {
       L.o_mix = 0; L.o_scan = nv; L.o_ff = nv;
       max_cv = std::max(max_cv, 2 * nq + nv);
       max_f1 = std::max(max_f1, c.d_heads * c.d_dim);
-      max_f2 = std::max(max_f2, channel_delta_columns(c) ? ((nv + 3) & ~3) + nv : nv);
-      if (channel_delta_columns(c)) { mx.lin = std::max(mx.lin, 2 * nq); mx.lin_sc = std::max(mx.lin_sc, c.d_heads); }
+      max_f2 = std::max(max_f2, ((nv + 3) & ~3) + nv);
+      mx.lin = std::max(mx.lin, 2 * nq); mx.lin_sc = std::max(mx.lin_sc, c.d_heads);
       if (dev_alloc(h, (void**)&L.conv_state, (size_t)rt.num_slots * (c.d_conv - 1) * (2 * nq + nv) * 4, &h->bytes_state)) return HY_ERR_CUDA;
       if (dev_alloc(h, (void**)&L.rec_state, (size_t)rt.num_slots * c.d_heads * c.d_dim * c.d_vdim * 4, &h->bytes_state)) return HY_ERR_CUDA;
     }
@@ -1589,6 +1584,28 @@ const UnitList* biased_units(hy_engine* h, int E, int T, const BiasedCfg& c, int
   return w.commit(3, H, G, c.window, c.chunk, 0, ns);
 }
 
+// Short convolution with its carried tail (see conv_kernel): four columns per thread where every boundary allows it.
+template <typename AT>
+void launch_conv(hy_engine* h, const Batch& b, const AT* u, int ldu, int col0, int C, int taps, const void* w, const void* bias, int silu,
+                 float* state, const ConvOut<AT>& o) {
+  typedef AT WT;
+  int chunks = 0;
+  for (int e = 0; e < b.E; ++e) chunks += (h->step_start[e + 1] - h->step_start[e] + HY_CONV_TT - 1) / HY_CONV_TT;
+  const int any = ldu | col0 | C | o.ldo | o.out_lo | o.out_hi | (o.rows ? o.r_lo | o.n : 0) | (o.cache ? o.k_lo | o.dim : 0);
+  const bool vec = any % 4 == 0 && ((reinterpret_cast<uintptr_t>(u) | reinterpret_cast<uintptr_t>(o.out) | reinterpret_cast<uintptr_t>(o.rows) |
+                                     reinterpret_cast<uintptr_t>(o.cache)) & 15) == 0;
+  auto go = [&](auto v, auto tp) {
+    constexpr int V = decltype(v)::value, TP = decltype(tp)::value;
+    const int per = 128 * V;
+    conv_kernel<AT, WT, V, TP><<<dim3((C + per - 1) / per, chunks), 128, 0, h->stream>>>(b, u, ldu, col0, C, taps, (const WT*)w, (const WT*)bias, silu,
+                                                                                        state, o);
+  };
+  if (vec && taps == 4) go(std::integral_constant<int, 4>{}, std::integral_constant<int, 4>{});
+  else if (taps == 4) go(std::integral_constant<int, 1>{}, std::integral_constant<int, 4>{});
+  else go(std::integral_constant<int, 1>{}, std::integral_constant<int, 0>{});
+  h->launches++;
+}
+
 // Register layout of a matrix-state recurrence by key size: fn(padded key size, lanes per column), both compile-time.
 constexpr int HY_LIN_MAX_DIM = 1024;
 template <typename AT, typename Fn>
@@ -1738,26 +1755,22 @@ int sandwich_layer(hy_engine* h, const Batch& b, size_t li) {
     }
     {
       ProfScope ps(h, HY_PROF_CONV);
-      conv_kernel<AT, WT><<<dim3((C + 127) / 128, T), 128, 0, s>>>(b, pin, h->ld_pin, inner, C, c.m_conv, (const WT*)L.m_conv_w,
-                                                                   (const WT*)L.m_conv_b, 1, L.conv_state, cv, h->ld_cv);
-      conv_tail_kernel<AT><<<dim3((C + 127) / 128, E), 128, 0, s>>>(b, pin, h->ld_pin, inner, C, c.m_conv, L.conv_state);
-      h->launches += 2;
+      ConvOut<AT> co{};                                        // x in the activation type, rows [C | B] per group in fp32
+      co.out = cv; co.ldo = h->ld_cv; co.out_hi = inner;
+      co.rows = h->lin; co.r_lo = inner; co.G = G; co.n = N; co.flip = 1;
+      launch_conv<AT>(h, b, pin, h->ld_pin, inner, C, c.m_conv, L.m_conv_w, L.m_conv_b, 1, L.conv_state, co);
     }
     {
       ProfScope ps(h, HY_PROF_SCAN);
-      // 4 states per thread up to 16 states, 16 per thread beyond; lanes = the power of two that covers the state size
-      const int nper = N <= 16 ? 4 : 16;
-      int lanes = 1;
-      while (lanes * nper < N) lanes <<= 1;
-      const int per_block = 128 / lanes, bph = (P + per_block - 1) / per_block;
-      dim3 grid(H * bph, E);
-#define HY_SSD_ARGS b, cv, h->ld_cv, inner, inner + GN, pin + 2 * inner + 2 * GN, h->ld_pin, L.m_dt_bias, L.m_A_log, L.m_D, H, P, N, \
-      G, bph, L.rec_state, h->f2, h->ld_f2
-#define HY_SSD_CASE(NP, LL) if (nper == NP && lanes == LL) ssd_scan_kernel<AT, NP, LL><<<grid, 128, 0, s>>>(HY_SSD_ARGS)
-      HY_SSD_CASE(4, 1); else HY_SSD_CASE(4, 2); else HY_SSD_CASE(4, 4);
-      else HY_SSD_CASE(16, 2); else HY_SSD_CASE(16, 4); else HY_SSD_CASE(16, 8); else HY_SSD_CASE(16, 16); else HY_SSD_CASE(16, 32);
-#undef HY_SSD_CASE
-#undef HY_SSD_ARGS
+      const GlaToken tk{G, pin + 2 * inner + 2 * GN, h->ld_pin, L.m_dt_bias, L.m_A_log, L.m_D};
+      launch_linear<AT>(N, [&](auto dr, auto parts) {
+        constexpr int DR = decltype(dr)::value, PARTS = decltype(parts)::value;
+        const LinearLaunch g = linear_launch<AT>(PARTS, N, P, cv, h->ld_cv);
+        const size_t smem = lin_smem<AT>(DR, PARTS, 0);
+        cudaFuncSetAttribute(gla_kernel<AT, DR, PARTS, GLA_TOKEN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        gla_kernel<AT, DR, PARTS, GLA_TOKEN><<<dim3(H * g.bph, E), 128, smem, s>>>(b, h->lin, cv, h->ld_cv, nullptr, 0, nullptr, H, N, P, g.bph,
+                                                                                   g.vec, g.vvec, L.rec_state, h->f2, h->ld_f2, tk);
+      });
       gated_group_norm_kernel<AT><<<dim3(T, c.m_norm_groups), 128, 0, s>>>(h->f2, h->ld_f2, pin, h->ld_pin, L.m_norm, inner,
                                                                           c.m_norm_groups, eps, cat, h->ld_cat);
       h->launches += 2;
@@ -2403,7 +2416,6 @@ void retention_mixer(hy_engine* h, const Batch& b, const LayerW& L, const hy_lay
 // (q, k | convolved q, k, v | gate), fp32 columns in h->f1 (head gates | step sizes | decays); both results in h->cat.
 template <typename AT>
 void attn_delta_mixer(hy_engine* h, const Batch& b, const LayerW& L, const hy_layer_cfg& c) {
-  typedef AT WT;
   const int T = b.T, E = b.E;
   cudaStream_t s = h->stream;
   AT* pin = (AT*)h->pin; AT* cat = (AT*)h->cat; AT* cv = (AT*)h->cv;
@@ -2413,13 +2425,13 @@ void attn_delta_mixer(hy_engine* h, const Batch& b, const LayerW& L, const hy_la
     ProfScope ps(h, HY_PROF_CONV);
     key_value_prep_kernel<AT><<<T, 128, 0, s>>>(b, pin, h->ld_pin, L.c_q, L.c_k, c.b_heads, c.b_kv_heads, c.b_dim, rot.out, rot.ld,
                                                 RotPair{rot.pairs, c.r_half}, (AT*)L.cache, (AT*)L.cache_v);
-    static bool attr = false;                                // per AT: this function is a template
-    if (!attr) { cudaFuncSetAttribute(delta_rows_kernel<AT, WT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024); attr = true; }
-    delta_rows_kernel<AT, WT><<<T, T <= 8 ? 1024 : 256, (size_t)2 * nk * 4, s>>>(b, pin, h->ld_pin, L.c_x, H, G, dk, dv, c.d_conv, (const WT*)L.conv_qkv,
-                                                                 L.conv_state, h->f1 + c.b_heads, h->ld_f1, (const float*)L.A_log,
-                                                                 (const float*)L.dt_bias, cv, h->ld_cv, h->lin, h->lin_sc);
-    conv_tail_kernel<AT><<<dim3((C + 127) / 128, E), 128, 0, s>>>(b, pin, h->ld_pin, L.c_x, C, c.d_conv, L.conv_state);
-    h->launches += 3;
+    ConvOut<AT> co{};                                          // values in the activation type, queries and keys as fp32 rows
+    co.out = cv; co.ldo = h->ld_cv; co.out_lo = 2 * nk; co.out_hi = C;
+    co.rows = h->lin; co.G = G; co.n = dk;
+    launch_conv<AT>(h, b, pin, h->ld_pin, L.c_x, C, c.d_conv, L.conv_qkv, nullptr, 1, L.conv_state, co);
+    delta_unit_kernel<AT, false><<<(T * G + 3) / 4, 128, 0, s>>>(T, H, G, dk, h->f1 + c.b_heads, h->ld_f1, (const float*)L.A_log,
+                                                                 (const float*)L.dt_bias, nullptr, 0, nullptr, 0, h->lin, h->lin_sc);
+    h->launches += 2;
   }
   const BiasedCfg bc{c.b_heads, c.b_kv_heads, c.b_dim, c.b_vdim, 0, 0, c.b_scale, 0.0f, nullptr, nullptr, nullptr, 0, HY_BIAS_NONE,
                      h->f1, h->ld_f1, c.left_scale};
@@ -2629,10 +2641,10 @@ int run_step(hy_engine* h, const Batch& b, int n_want, const int* want_d, float*
       // attention side: conv over q | k, keys into their pages, attention over the pages
       {
       ProfScope ps(h, HY_PROF_CONV);
-      conv_kernel<AT, WT><<<dim3((nq + nk + 127) / 128, T), 128, 0, s>>>(b, pin, h->ld_pin, L.c_q, nq + nk, c.a_conv,
-          (const WT*)L.conv_qk, (const WT*)nullptr, 0, L.conv_state, cv, h->ld_cv);
-      conv_tail_kernel<AT><<<dim3((nq + nk + 127) / 128, E), 128, 0, s>>>(b, pin, h->ld_pin, L.c_q, nq + nk, c.a_conv, L.conv_state);
-      cache_append_kernel<AT><<<T, 128, 0, s>>>(b, cv, h->ld_cv, nq, c.a_kv_heads, c.a_dim, (AT*)L.cache);
+      ConvOut<AT> co{};                                        // queries, and keys straight into their pages
+      co.out = cv; co.ldo = h->ld_cv; co.out_hi = nq;
+      co.cache = (AT*)L.cache; co.k_lo = nq; co.kv_heads = c.a_kv_heads; co.dim = c.a_dim;
+      launch_conv<AT>(h, b, pin, h->ld_pin, L.c_q, nq + nk, c.a_conv, L.conv_qk, nullptr, 0, L.conv_state, co);
       }
       {
       ProfScope ps(h, HY_PROF_ATTN);
@@ -2658,15 +2670,14 @@ int run_step(hy_engine* h, const Batch& b, int n_want, const int* want_d, float*
           b, cv, h->ld_cv, (const AT*)L.cache, (const WT*)L.sink, pin + L.c_g, h->ld_pin, c.a_heads, c.a_kv_heads, c.a_dim, c.a_dim,
           c.a_scale, c.a_qt_coef, c.a_qt_every, 0, c.left_scale, cat + L.o_mix, h->ld_cat);
       }
-      h->launches += 4;
+      h->launches++;
       // scan side
       {
       ProfScope ps(h, HY_PROF_CONV);
-      conv_kernel<AT, WT><<<dim3((I + 127) / 128, T), 128, 0, s>>>(b, pin, h->ld_pin, L.c_x, I, c.s_conv, (const WT*)L.conv_x,
-                                                                   (const WT*)L.conv_xb, 1, L.conv_state2, cv, h->ld_cv);
-      conv_tail_kernel<AT><<<dim3((I + 127) / 128, E), 128, 0, s>>>(b, pin, h->ld_pin, L.c_x, I, c.s_conv, L.conv_state2);
+      ConvOut<AT> co{};
+      co.out = cv; co.ldo = h->ld_cv; co.out_hi = I;
+      launch_conv<AT>(h, b, pin, h->ld_pin, L.c_x, I, c.s_conv, L.conv_x, L.conv_xb, 1, L.conv_state2, co);
       }
-      h->launches += 2;
       {
       ProfScope ps(h, HY_PROF_SMALL_GEMM);
       gemm<AT, WT, float>(h, cv, h->ld_cv, (const WT*)L.w_x, I, T, R + 2 * N, I, to_buf(h->f1, h->ld_f1), L.w_x_t);
@@ -2674,19 +2685,28 @@ int run_step(hy_engine* h, const Batch& b, int n_want, const int* want_d, float*
       }
       {
         ProfScope ps(h, HY_PROF_SCAN);
-        const int nper = N <= 32 ? 1 : N <= 64 ? 2 : N <= 128 ? 4 : 8;
-        int lanes = 1;
-        while (lanes * nper < N) lanes <<= 1;
-        const int per_block = 128 / lanes;
-        dim3 grid((I + per_block - 1) / per_block, E);
-        const size_t smem = (size_t)HY_SCAN_TB * (2 * N + 3 * per_block) * 4;
-#define HY_SCAN_ARGS b, cv, h->ld_cv, pin + L.c_z, h->ld_pin, h->f2, h->ld_f2, (const WT*)L.dt_b, h->f1, h->ld_f1, R, R + N, L.A_neg, \
-        (const WT*)L.D, I, N, lanes, c.right_scale, L.rec_state, cat + L.o_scan, h->ld_cat
-        if (nper == 1) scan_kernel<AT, WT, 1><<<grid, 128, smem, s>>>(HY_SCAN_ARGS);
-        else if (nper == 2) scan_kernel<AT, WT, 2><<<grid, 128, smem, s>>>(HY_SCAN_ARGS);
-        else if (nper == 4) scan_kernel<AT, WT, 4><<<grid, 128, smem, s>>>(HY_SCAN_ARGS);
-        else scan_kernel<AT, WT, 8><<<grid, 128, smem, s>>>(HY_SCAN_ARGS);
-#undef HY_SCAN_ARGS
+        // four states per lane up to 128 states, eight beyond (up to 256)
+        const int ch = 16 / (int)sizeof(AT);
+        auto go = [&](auto np, auto ln) {
+          constexpr int NPER = decltype(np)::value, LN = decltype(ln)::value, PB = 128 / LN;
+          const size_t smem = scan_smem(NPER * LN, PB, sizeof(AT));
+          static bool attr = false;                            // per kernel: go is a template
+          if (!attr) { cudaFuncSetAttribute(scan_kernel<AT, WT, NPER, LN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); attr = true; }
+          // 16-byte copies: whole blocks of channels, rows and columns on 16-byte boundaries
+          const int v32 = (R | N | h->ld_f1 | h->ld_f2 | I) % 4 == 0 && PB % 4 == 0;
+          const int vat = (h->ld_cv | h->ld_pin | L.c_z | I) % ch == 0 && PB % ch == 0;
+          scan_kernel<AT, WT, NPER, LN><<<dim3((I + PB - 1) / PB, E), 128, smem, s>>>(
+              b, cv, h->ld_cv, pin + L.c_z, h->ld_pin, h->f2, h->ld_f2, (const WT*)L.dt_b, h->f1, h->ld_f1, R, R + N, L.A_neg, (const WT*)L.D, I, N,
+              v32 | vat << 1, c.right_scale, L.rec_state, cat + L.o_scan, h->ld_cat);
+        };
+        typedef std::integral_constant<int, 4> four;
+        if (N <= 4) go(four{}, std::integral_constant<int, 1>{});
+        else if (N <= 8) go(four{}, std::integral_constant<int, 2>{});
+        else if (N <= 16) go(four{}, std::integral_constant<int, 4>{});
+        else if (N <= 32) go(four{}, std::integral_constant<int, 8>{});
+        else if (N <= 64) go(four{}, std::integral_constant<int, 16>{});
+        else if (N <= 128) go(four{}, std::integral_constant<int, 32>{});
+        else go(std::integral_constant<int, 8>{}, std::integral_constant<int, 32>{});
         h->launches++;
       }
     } else {
@@ -2699,45 +2719,28 @@ int run_step(hy_engine* h, const Batch& b, int n_want, const int* want_d, float*
                             L.w_g2_t);
       }
       const int H = c.d_heads, G = c.d_kv_heads, dk = c.d_dim, dv = c.d_vdim;
-      if (channel_delta_columns(c)) {
-        {
-          ProfScope ps(h, HY_PROF_CONV);
-          static bool attr = false;                          // per AT: this function is a template
-          if (!attr) { cudaFuncSetAttribute(delta_rows_kernel<AT, WT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024); attr = true; }
-          delta_rows_kernel<AT, WT, true><<<T, T <= 8 ? 1024 : 256, (size_t)2 * nq * 4, s>>>(
-              b, pin, h->ld_pin, L.c_q, H, G, dk, dv, c.d_conv, (const WT*)L.conv_qkv, L.conv_state, nullptr, 0, (const float*)L.A_log,
-              (const float*)L.dt_bias, cv, h->ld_cv, h->lin, h->lin_sc, pin + L.c_b, h->ld_pin, h->f1, h->ld_f1);
-          conv_tail_kernel<AT><<<dim3((C + 127) / 128, E), 128, 0, s>>>(b, pin, h->ld_pin, L.c_q, C, c.d_conv, L.conv_state);
-        }
-        ProfScope ps(h, HY_PROF_DELTA);
-        float* o = h->f2 + ((nv + 3) & ~3);                  // behind the output gates
-        launch_linear<AT>(dk, [&](auto dr, auto parts) {
-          constexpr int DR = decltype(dr)::value, PARTS = decltype(parts)::value;
-          const LinearLaunch g = linear_launch<AT>(PARTS, dk, dv, cv, h->ld_cv);
-          const size_t smem = lin_smem<AT>(DR, PARTS, DR + 4);
-          cudaFuncSetAttribute(delta_head_kernel<AT, DR, PARTS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-          delta_head_kernel<AT, DR, PARTS, true><<<dim3(H * g.bph, E), 128, smem, s>>>(b, h->lin, cv, h->ld_cv, h->lin_sc, H, G, dk, dv, g.bph,
-                                                                                       g.vec, g.vvec, L.rec_state, o, h->ld_f2, h->f1, h->ld_f1);
-        });
-        gla_out_kernel<AT, float, GATE_SIGMOID><<<(T * H + 3) / 4, 128, 0, s>>>(T, H, dv, o, h->ld_f2, h->f2, h->ld_f2, (const float*)L.norm_w, eps,
-                                                                                1.0f, cat + L.o_mix, h->ld_cat);
-        h->launches += 4;
-      } else {
-        {
-          ProfScope ps(h, HY_PROF_CONV);
-          conv_kernel<AT, WT><<<dim3((C + 127) / 128, T), 128, 0, s>>>(b, pin, h->ld_pin, L.c_q, C, c.d_conv, (const WT*)L.conv_qkv,
-                                                                       (const WT*)nullptr, 1, L.conv_state, cv, h->ld_cv);
-          conv_tail_kernel<AT><<<dim3((C + 127) / 128, E), 128, 0, s>>>(b, pin, h->ld_pin, L.c_q, C, c.d_conv, L.conv_state);
-        }
-        ProfScope ps(h, HY_PROF_DELTA);
-        static bool dk_attr = false;
-        if (!dk_attr) { cudaFuncSetAttribute(delta_kernel<AT, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024); dk_attr = true; }
-        const int threads = ((std::max(dk, dv) + 31) / 32) * 32;
-        delta_kernel<AT, float><<<dim3(H, E), threads, ((size_t)dk * dv + 3 * dk + 40) * 4, s>>>(
-            b, cv, h->ld_cv, 0, nq, 2 * nq, pin, h->ld_pin, L.c_b, h->f1, h->ld_f1, h->f2, h->ld_f2, (const float*)L.A_log,
-            (const float*)L.dt_bias, (const float*)L.norm_w, H, G, dk, dv, eps, L.rec_state, cat + L.o_mix, h->ld_cat);
-        h->launches += 3;
+      {
+        ProfScope ps(h, HY_PROF_CONV);
+        ConvOut<AT> co{};                                      // values in the activation type, queries and keys as fp32 rows
+        co.out = cv; co.ldo = h->ld_cv; co.out_lo = 2 * nq; co.out_hi = C;
+        co.rows = h->lin; co.G = G; co.n = dk;
+        launch_conv<AT>(h, b, pin, h->ld_pin, L.c_q, C, c.d_conv, L.conv_qkv, nullptr, 1, L.conv_state, co);
+        delta_unit_kernel<AT, true><<<(T * G + 3) / 4, 128, 0, s>>>(T, H, G, dk, nullptr, 0, (const float*)L.A_log, (const float*)L.dt_bias,
+                                                                    pin + L.c_b, h->ld_pin, h->f1, h->ld_f1, h->lin, h->lin_sc);
       }
+      ProfScope ps(h, HY_PROF_DELTA);
+      float* o = h->f2 + ((nv + 3) & ~3);                      // behind the output gates
+      launch_linear<AT>(dk, [&](auto dr, auto parts) {
+        constexpr int DR = decltype(dr)::value, PARTS = decltype(parts)::value;
+        const LinearLaunch g = linear_launch<AT>(PARTS, dk, dv, cv, h->ld_cv);
+        const size_t smem = lin_smem<AT>(DR, PARTS, DR + 4);
+        cudaFuncSetAttribute(delta_head_kernel<AT, DR, PARTS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        delta_head_kernel<AT, DR, PARTS, true><<<dim3(H * g.bph, E), 128, smem, s>>>(b, h->lin, cv, h->ld_cv, h->lin_sc, H, G, dk, dv, g.bph, g.vec,
+                                                                                     g.vvec, L.rec_state, o, h->ld_f2, h->f1, h->ld_f1);
+      });
+      gla_out_kernel<AT, float, GATE_SIGMOID><<<(T * H + 3) / 4, 128, 0, s>>>(T, H, dv, o, h->ld_f2, h->f2, h->ld_f2, (const float*)L.norm_w, eps,
+                                                                              1.0f, cat + L.o_mix, h->ld_cat);
+      h->launches += 3;
     }
     (void)ff;
     // merged output projections, added to the residual stream
@@ -2825,7 +2828,7 @@ extern "C" int hy_step(hy_handle h, int32_t n_entries, const int32_t* tokens, co
       HY_CUDA(cudaMemcpyAsync(h->temp_d, temperature, (size_t)n_want * 4, cudaMemcpyHostToDevice, h->stream));
       td = h->temp_d;
     }
-    sample_kernel<<<n_want, 256, 0, h->stream>>>(h->logits, h->m.vocab, td, seed, h->sampled);
+    sample_kernel<<<n_want, 1024, 0, h->stream>>>(h->logits, h->m.vocab, td, seed, h->sampled);
     h->launches++;
     HY_CUDA(cudaMemcpyAsync(sampled_out, h->sampled, (size_t)n_want * 4, cudaMemcpyDeviceToHost, h->stream));
   }

@@ -23,19 +23,26 @@ namespace hy {
 // or with GLA_HEAD one number per head, head_decay [H].  With GLA_FORGET the rows hold [q | f] (forget_rows_kernel) and the
 // update is S <- f S + (1 - f) v^T, written as v + f (S - v).  o [T, ldo] fp32 (H heads of vdim).  state [slot][H][dim][vdim] fp32.
 // grid (H * blocks_per_head, entries), 128 threads.  Lane layout, vec and vvec as in delta_head_kernel.
+// With GLA_TOKEN (state-space recurrence with one decay per head) the rows [q | k] = [C | B] are shared by the H / G heads of a
+// group, a head's step size dt = softplus(dt_raw + bias) and decay exp(-exp(A_log) dt) are made per token from dt_raw [T, lddt]
+// (column h), the value is dt x and the read-out gets D_h x added.
+// GLA_TOKEN, 2048 tokens of 32 heads of 64 channels x 128 states: eight lanes with sixteen consecutive states each (staged rows read
+// with four-way bank conflicts, one exchange per token) took 766 us, this layout 284 us.
 // GLA_FORGET, 2048 tokens of 8 heads of 128 x 128: one block per head with a column per thread took 1927 us, this layout 202 us.
-enum GlaMode : int { GLA_CHANNEL = 0, GLA_HEAD = 1, GLA_FORGET = 2 };
+enum GlaMode : int { GLA_CHANNEL = 0, GLA_HEAD = 1, GLA_FORGET = 2, GLA_TOKEN = 3 };
+struct GlaToken { int G; const void* dt_raw; int lddt; const float* dt_bias; const float* A_log; const float* D; };
 template <typename AT, int DR, int PARTS, int MODE>
 __global__ void __launch_bounds__(128) gla_kernel(Batch b, const float* __restrict__ qk, const AT* __restrict__ v, int ldv,
                                                   const float* __restrict__ decay, int ldd, const float* __restrict__ head_decay, int H,
                                                   int dim, int vdim, int blocks_per_head, int vec, int vvec, float* __restrict__ state,
-                                                  float* __restrict__ o, int ldo) {
+                                                  float* __restrict__ o, int ldo, GlaToken tk = GlaToken{}) {
   constexpr int TB = lin_tb(DR), RP = DR / PARTS, CW = 32 / PARTS, CPB = lin_cpb(PARTS), VW = CPB < 8 ? 8 : CPB;
   constexpr bool HEAD = MODE == GLA_HEAD;
   constexpr int RW = MODE == GLA_CHANNEL ? 3 * DR : 2 * DR;    // floats of a staged row: q | k (| decays)
   extern __shared__ __align__(16) unsigned char hy_smem[];
   float* sqk = reinterpret_cast<float*>(hy_smem);              // [2][TB][RW]
   AT* sv = reinterpret_cast<AT*>(sqk + 2 * TB * RW);           // [2][TB][VW]
+  __shared__ float2 sdt[MODE == GLA_TOKEN ? 2 * TB : 1];       // [2][TB] decay, step size
   const int h = blockIdx.x / blocks_per_head, c0 = (blockIdx.x % blocks_per_head) * CPB, e = blockIdx.y;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int cl = warp * CW + lane % CW, part = lane / CW, col = c0 + cl;
@@ -50,14 +57,19 @@ __global__ void __launch_bounds__(128) gla_kernel(Batch b, const float* __restri
     S[i] = (live && r < dim && pos0 > 0) ? st[(size_t)r * vdim + col] : 0.0f;
   }
   const float hd = HEAD ? head_decay[h] : 0.0f;
+  const int rows_per_token = MODE == GLA_TOKEN ? tk.G : H, row_of = MODE == GLA_TOKEN ? h / (H / tk.G) : h;
+  const float rate = MODE == GLA_TOKEN ? expf(tk.A_log[h]) : 0.0f, dt_bias = MODE == GLA_TOKEN ? tk.dt_bias[h] : 0.0f;
+  const float skip = MODE == GLA_TOKEN ? tk.D[h] : 0.0f;
+  float raw = 0.0f;                                            // raw step size of token tid of the batch in flight
   if (dim < DR)                                                // rows beyond the head's key size stay zero
     for (int i = tid; i < 2 * TB * RW; i += 128) if (i % DR >= dim) sqk[i] = 0.0f;
   auto fetch = [&](int j0, int buf) {
     const int nb = min(TB, cnt - j0);
     const size_t t0 = (size_t)(start + j0);
     float* d = sqk + (size_t)buf * TB * RW;
-    const float* src = qk + (t0 * H + h) * 2 * dim;
-    const size_t ld = (size_t)H * 2 * dim;
+    const float* src = qk + (t0 * rows_per_token + row_of) * 2 * dim;
+    const size_t ld = (size_t)rows_per_token * 2 * dim;
+    if (MODE == GLA_TOKEN && tid < nb) raw = to_f(((const AT*)tk.dt_raw)[(t0 + tid) * tk.lddt + h]);
     copy_rows(d, RW, src, ld, nb, dim, vec);
     copy_rows(d + DR, RW, src + dim, ld, nb, dim, vec);
     if (MODE == GLA_CHANNEL) copy_rows(d + 2 * DR, RW, decay + t0 * ldd + h * dim, ldd, nb, dim, vec);
@@ -69,15 +81,24 @@ __global__ void __launch_bounds__(128) gla_kernel(Batch b, const float* __restri
   int buf = 0;
   for (int j0 = 0; j0 < cnt; j0 += TB, buf ^= 1) {
     const int nb = min(TB, cnt - j0);
+    if (MODE == GLA_TOKEN && tid < nb) {
+      const float dt = softplus_f(raw + dt_bias);
+      sdt[buf * TB + tid] = make_float2(expf(-rate * dt), dt);
+    }
     jf::cp_async_wait_all();
     __syncthreads();                                           // this batch has landed; the batch before it is finished
     if (j0 + TB < cnt) fetch(j0 + TB, buf ^ 1);
     const float* rb = sqk + (size_t)buf * TB * RW + 4 * part;
     const AT* vb = sv + (size_t)buf * TB * VW + min(cl, ncol - 1);
     float* po = o + (size_t)(start + j0) * ldo + h * vdim + col;
+    auto leave = [&](int tt, float p) {
+      if constexpr (MODE == GLA_TOKEN) p = fmaf(skip, to_f(vb[tt * VW]), p);
+      po[(size_t)tt * ldo] = p;
+    };
     // one token's update of this lane's key rows; returns its part of the read-out
     auto update = [&](int tt) {
-      const float vv = to_f(vb[tt * VW]);
+      float vv = to_f(vb[tt * VW]), td = hd;
+      if constexpr (MODE == GLA_TOKEN) { const float2 sd = sdt[buf * TB + tt]; td = sd.x; vv *= sd.y; }
       float p0 = 0.0f, p1 = 0.0f;
 #pragma unroll
       for (int i = 0; i < RP / 4; ++i) {
@@ -91,7 +112,7 @@ __global__ void __launch_bounds__(128) gla_kernel(Batch b, const float* __restri
           R[3] = fmaf(k.w, R[3] - vv, vv); p1 = fmaf(R[3], q.w, p1);
           continue;
         }
-        const float4 a = HEAD ? make_float4(hd, hd, hd, hd) : *reinterpret_cast<const float4*>(rb + tt * RW + (MODE == GLA_CHANNEL ? 2 * DR : 0) + 4 * PARTS * i);
+        const float4 a = HEAD || MODE == GLA_TOKEN ? make_float4(td, td, td, td) : *reinterpret_cast<const float4*>(rb + tt * RW + (MODE == GLA_CHANNEL ? 2 * DR : 0) + 4 * PARTS * i);
         R[0] = fmaf(a.x, R[0], k.x * vv); p0 = fmaf(R[0], q.x, p0);
         R[1] = fmaf(a.y, R[1], k.y * vv); p1 = fmaf(R[1], q.y, p1);
         R[2] = fmaf(a.z, R[2], k.z * vv); p0 = fmaf(R[2], q.z, p0);
@@ -125,14 +146,14 @@ __global__ void __launch_bounds__(128) gla_kernel(Batch b, const float* __restri
       constexpr int LEFT = TG > PARTS ? TG / PARTS : 1, SAME = PARTS > TG ? PARTS / TG : 1;     // tokens per lane, lanes per token
       if (live && (part & (SAME - 1)) == 0) {
 #pragma unroll
-        for (int u = 0; u < LEFT; ++u) po[(size_t)(tt + base + u) * ldo] = p[u];
+        for (int u = 0; u < LEFT; ++u) leave(tt + base + u, p[u]);
       }
     }
     for (; tt < nb; ++tt) {
       float p = update(tt);
 #pragma unroll
       for (int s = CW; s < 32; s <<= 1) p += __shfl_xor_sync(0xffffffffu, p, s);
-      if (live && part == 0) po[(size_t)tt * ldo] = p;
+      if (live && part == 0) leave(tt, p);
     }
   }
   if (live) {

@@ -11,6 +11,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "jf_ptx.cuh"
+
 namespace hy {
 
 typedef __nv_bfloat16 bf16;
@@ -21,6 +23,9 @@ template <> __device__ __forceinline__ float to_f<bf16>(bf16 v) { return __bfloa
 template <typename T> __device__ __forceinline__ T from_f(float v);
 template <> __device__ __forceinline__ float from_f<float>(float v) { return v; }
 template <> __device__ __forceinline__ bf16 from_f<bf16>(float v) { return __float2bfloat16_rn(v); }
+
+template <typename T, int N>
+struct alignas(sizeof(T) * N < 16 ? sizeof(T) * N : 16) VecN { T v[N]; };
 
 __device__ __forceinline__ float sigmoid_f(float z) { return 1.0f / (1.0f + expf(-z)); }
 __device__ __forceinline__ float silu_f(float z) { return z * sigmoid_f(z); }
@@ -267,8 +272,6 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(const TA* __restrict__ A
 // Few-row kernel (decode steps): the weight matrix is streamed once, 16 bytes per lane per load, four loads in flight per
 // lane; one warp owns one output column for up to ROWS rows; the rows' operand sits in shared memory in its own type and
 // is read back 16 bytes at a time (conflict-free).  K order: lane-strided partial sums, then an xor tree.
-template <typename T, int N>
-struct alignas(sizeof(T) * N < 16 ? sizeof(T) * N : 16) VecN { T v[N]; };
 
 template <typename TA, typename TW, typename TO, int ROWS>
 __global__ void __launch_bounds__(256) gemm_rows_kernel(const TA* __restrict__ A, int lda, const TW* __restrict__ W, int ldw,
@@ -358,32 +361,105 @@ __global__ void __launch_bounds__(256) gemm_rows_kernel(const TA* __restrict__ A
 // ---- short causal convolution over time with a carried tail ------------------------------------------------------------------
 // u [T, ldu] (columns col0 .. col0 + C), w [C, taps] (last tap = current token), state [slot][taps - 1][C] fp32 holds the
 // last taps - 1 inputs of the request in time order.  Inputs before the request's start are zero.
-template <typename AT, typename WT>
-__global__ void conv_kernel(Batch b, const AT* __restrict__ u, int ldu, int col0, int C, int taps, const WT* __restrict__ w,
-                            const WT* __restrict__ bias, int act_silu, const float* __restrict__ state, AT* __restrict__ out,
-                            int ldo) {
-  const int t = blockIdx.y;
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= C) return;
-  const int e = b.tok_ent[t];
-  const int start = b.ent_start[e], pos0 = b.ent_pos0[e];
-  const int j = t - start;                                   // index inside the entry
-  const float* st = state + (size_t)b.ent_slot[e] * (taps - 1) * C;
-  float acc = bias ? to_f(bias[c]) : 0.0f;
-  for (int i = 0; i < taps; ++i) {
-    const int src = j - (taps - 1) + i;
-    float v;
-    if (src >= 0) v = to_f(u[(size_t)(start + src) * ldu + col0 + c]);
-    else if (pos0 + src >= 0) v = st[(size_t)(taps - 1 + src) * C + c];
-    else v = 0.0f;
-    acc = fmaf(to_f(w[(size_t)c * taps + i]), v, acc);
+// Where a column goes: [out_lo, out_hi) to out (from its column 0 on, activation type); [r_lo, r_lo + 2 G n) to fp32 rows
+// [T][G][2 n], the operands of a matrix-state recurrence: the span's first half to the first n of a head's row, the second half
+// to the last n (flip: the other way round); the columns from k_lo on (when cache is given: kv heads of dim) to their pages.
+template <typename AT>
+struct ConvOut {
+  AT* out; int ldo, out_lo, out_hi;
+  float* rows; int r_lo, G, n, flip;
+  AT* cache; int k_lo, kv_heads, dim;
+};
+constexpr int HY_MAX_TAPS = 16;
+constexpr int HY_CONV_TT = 16;                                 // tokens per thread: taps - 1 at most, so that only an entry's
+                                                               // first chunk meets the carried tail
+// V columns per thread (V = 4: every boundary above, C, col0 and the leading dimensions are multiples of 4), HY_CONV_TT tokens of
+// one entry: weights and the last taps - 1 inputs stay in registers (TAPS = 0: any number of taps, inputs read again per tap).
+// The thread of an entry's first chunk is the only one that reads the carried tail, so it also leaves the new one.
+// One token and one column per thread with the tail, the cache rows and the unit vectors as kernels of their own took 63 us for
+// 2048 tokens x 4096 columns (0.5 TB/s) and 4.5 us per launch in decode steps; this form 23 us and one launch.
+template <typename AT, typename WT, int V, int TAPS>
+__global__ void __launch_bounds__(128) conv_kernel(Batch b, const AT* __restrict__ u, int ldu, int col0, int C, int taps_, const WT* __restrict__ w,
+                                                   const WT* __restrict__ bias, int act_silu, float* __restrict__ state, ConvOut<AT> o) {
+  const int taps = TAPS ? TAPS : taps_;
+  int e = 0, chunk = blockIdx.y, start, cnt;
+  for (;; ++e) {                                               // entry and chunk of this block
+    start = b.ent_start[e]; cnt = b.ent_start[e + 1] - start;
+    const int n = (cnt + HY_CONV_TT - 1) / HY_CONV_TT;
+    if (chunk < n) break;
+    chunk -= n;
   }
-  if (act_silu) acc = silu_f(acc);
-  out[(size_t)t * ldo + c] = from_f<AT>(acc);
+  const int c = (blockIdx.x * blockDim.x + threadIdx.x) * V;
+  if (c >= C) return;
+  const int j0 = chunk * HY_CONV_TT, j1 = min(cnt, j0 + HY_CONV_TT), pos0 = b.ent_pos0[e];
+  float* st = state + (size_t)b.ent_slot[e] * (taps - 1) * C + c;
+  const AT* uc = u + (size_t)start * ldu + col0 + c;
+  auto input = [&](int j, int k) {                             // column c + k of the entry's token j (j < 0: before the entry)
+    if (j >= 0) return to_f(uc[(size_t)j * ldu + k]);
+    return pos0 + j >= 0 ? st[(size_t)(taps - 1 + j) * C + k] : 0.0f;
+  };
+  constexpr int NW = TAPS > 1 ? TAPS - 1 : 1;
+  float win[NW][V], wv[V][TAPS ? TAPS : 1], bv[V];
+#pragma unroll
+  for (int k = 0; k < V; ++k) {
+    bv[k] = bias ? to_f(bias[c + k]) : 0.0f;
+#pragma unroll
+    for (int i = 0; i < TAPS; ++i) wv[k][i] = to_f(w[(size_t)(c + k) * TAPS + i]);
+#pragma unroll
+    for (int i = 0; i < TAPS - 1; ++i) win[i][k] = input(j0 - (TAPS - 1) + i, k);
+  }
+#pragma unroll 4
+  for (int j = j0; j < j1; ++j) {
+    const int t = start + j;
+    float y[V];
+    if constexpr (TAPS > 0) {
+      const VecN<AT, V> x = *reinterpret_cast<const VecN<AT, V>*>(uc + (size_t)j * ldu);
+#pragma unroll
+      for (int k = 0; k < V; ++k) {
+        float acc = bv[k];
+#pragma unroll
+        for (int i = 0; i < TAPS - 1; ++i) acc = fmaf(wv[k][i], win[i][k], acc);
+        const float xk = to_f(x.v[k]);
+        y[k] = fmaf(wv[k][TAPS - 1], xk, acc);
+#pragma unroll
+        for (int i = 0; i + 1 < TAPS - 1; ++i) win[i][k] = win[i + 1][k];
+        if (TAPS > 1) win[NW - 1][k] = xk;
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < V; ++k) {
+        y[k] = bv[k];
+        for (int i = 0; i < taps; ++i) y[k] = fmaf(to_f(w[(size_t)(c + k) * taps + i]), input(j - (taps - 1) + i, k), y[k]);
+      }
+    }
+    if (act_silu) {
+#pragma unroll
+      for (int k = 0; k < V; ++k) y[k] = silu_f(y[k]);
+    }
+    if (o.rows && c >= o.r_lo && c < o.r_lo + 2 * o.G * o.n) {
+      const int r = c - o.r_lo, half = r >= o.G * o.n, g = (r - half * o.G * o.n) / o.n, k0 = r - half * o.G * o.n - g * o.n;
+      float* p = o.rows + ((size_t)t * o.G + g) * 2 * o.n + (half ^ o.flip) * o.n + k0;
+      *reinterpret_cast<VecN<float, V>*>(p) = *reinterpret_cast<VecN<float, V>*>(y);
+      continue;
+    }
+    VecN<AT, V> q;
+#pragma unroll
+    for (int k = 0; k < V; ++k) q.v[k] = from_f<AT>(y[k]);
+    if (o.cache && c >= o.k_lo) {
+      const int g = (c - o.k_lo) / o.dim, d = (c - o.k_lo) % o.dim, pos = pos0 + j;
+      const int page = b.pages[(size_t)e * b.max_pages + pos / b.page_size];
+      *reinterpret_cast<VecN<AT, V>*>(o.cache + (((size_t)page * o.kv_heads + g) * b.page_size + pos % b.page_size) * o.dim + d) = q;
+    } else if (c >= o.out_lo && c < o.out_hi) {
+      *reinterpret_cast<VecN<AT, V>*>(o.out + (size_t)t * o.ldo + c - o.out_lo) = q;
+    }
+  }
+  if (chunk == 0)
+    for (int s = 0; s < taps - 1; ++s)                         // ascending: row s is read (as row cnt + s) only before it is written
+#pragma unroll
+      for (int k = 0; k < V; ++k) st[(size_t)s * C + k] = input(cnt - (taps - 1) + s, k);
 }
 
-// New tail = the last taps - 1 of (old tail ++ this entry's inputs).  Runs after conv_kernel of the same step.
-constexpr int HY_MAX_TAPS = 16;
+// New tail = the last taps - 1 of (old tail ++ this entry's inputs).  Runs after the convolution of the same step.
 template <typename AT>
 __global__ void conv_tail_kernel(Batch b, const AT* __restrict__ u, int ldu, int col0, int C, int taps, float* __restrict__ state) {
   const int e = blockIdx.y;
@@ -400,18 +476,6 @@ __global__ void conv_tail_kernel(Batch b, const AT* __restrict__ u, int ldu, int
     nv[s] = v;
   }
   for (int s = 0; s < taps - 1; ++s) st[(size_t)s * C + c] = nv[s];
-}
-
-// ---- key cache: [page][kv head][slot in page][dim] ---------------------------------------------------------------------------
-template <typename AT>
-__global__ void cache_append_kernel(Batch b, const AT* __restrict__ k, int ldk, int col0, int G, int dim, AT* __restrict__ cache) {
-  const int t = blockIdx.x;
-  const int e = b.tok_ent[t], pos = b.tok_pos[t];
-  const int page = b.pages[(size_t)e * b.max_pages + pos / b.page_size], in_page = pos % b.page_size;
-  for (int i = threadIdx.x; i < G * dim; i += blockDim.x) {
-    const int g = i / dim, d = i % dim;
-    cache[(((size_t)page * G + g) * b.page_size + in_page) * dim + d] = k[(size_t)t * ldk + col0 + i];
-  }
 }
 
 // first position that the query at p sees through a sliding window (0: no window)
@@ -491,152 +555,164 @@ __global__ void __launch_bounds__(128) attn_sink_kernel(Batch b, const AT* __res
 
 // ---- selective scan -------------------------------------------------------------------------------------------------------------
 // S[c, n] <- exp(dt_c A[c, n]) S[c, n] + dt_c x_c B_n ; y_c = sum_n S[c, n] C_n + D_c x_c ; out = y silu(z) out_scale.
-// L lanes (a power of two) share a channel, each holding NPER states.  dt_raw is the step-size projection before bias
-// and softplus.  low [T, ldl] holds [dt-rank part | B | C].  state [slot][inner][nstate] fp32.
-// Inputs of HY_SCAN_TB tokens are staged in shared memory by the whole block (one exposed load latency per batch of
-// tokens instead of one per token); the recurrence itself then runs out of shared memory and registers.
-constexpr int HY_SCAN_TB = 16;
-template <typename AT, typename WT, int NPER>
+// dt_raw is the step-size projection before bias and softplus.  low [T, ldl] holds [dt-rank part | B | C].
+// state [slot][inner][nstate] fp32.
+// L lanes share a channel, each holding NPER CONSECUTIVE states (NPER * L >= nstate; the staged B and C are zero beyond nstate).
+// Inputs of TB tokens are copied asynchronously while the batch before them runs; the read-outs of eight tokens are reduced
+// in one exchange in which every step halves the tokens a lane keeps, so eight tokens run without a shuffle between them.
+// The arithmetic bounds it: about 13 instructions per state and token (the exponential takes 8 of them), so the fewer lanes
+// share a channel the less is spent on the exchange and on indices: four states per lane.
+// 2048 tokens, 4096 channels of 16 states: one state per lane, a five-step exchange per token and loads waited for took 949 us
+// (0.46 us per token), this form 369 us.
+__host__ __device__ constexpr int scan_tb(int np) { return np <= 64 ? 32 : np <= 128 ? 16 : 8; }
+__host__ __device__ constexpr size_t scan_smem(int np, int pb, size_t esz) {
+  return 2 * (size_t)scan_tb(np) * (2 * (size_t)np * 4 + (size_t)pb * (4 + 2 * esz));
+}
+// vec: rows of B, C and dt (fp32) and of x, z may travel by 16-byte copies (bits 0 and 1; see launch_scan)
+template <typename AT, typename WT, int NPER, int L>
 __global__ void __launch_bounds__(128) scan_kernel(Batch b, const AT* __restrict__ x, int ldx, const AT* __restrict__ z, int ldz,
                                                    const float* __restrict__ dt_raw, int lddt, const WT* __restrict__ dt_bias,
                                                    const float* __restrict__ low, int ldl, int col_b, int col_c,
                                                    const float* __restrict__ A, const WT* __restrict__ D, int inner, int nstate,
-                                                   int L, float out_scale, float* __restrict__ state, AT* __restrict__ out, int ldo) {
+                                                   int vec, float out_scale, float* __restrict__ state, AT* __restrict__ out, int ldo) {
+  constexpr int NP = NPER * L, PB = 128 / L, TB = scan_tb(NP), TG = 8, CH = 16 / (int)sizeof(AT);
   extern __shared__ __align__(16) unsigned char hy_smem[];
-  const int e = blockIdx.y;
-  const int per_block = blockDim.x / L;
-  float* sB = reinterpret_cast<float*>(hy_smem);              // [TB][nstate]
-  float* sC = sB + HY_SCAN_TB * nstate;                       // [TB][nstate]
-  float* sdt = sC + HY_SCAN_TB * nstate;                      // [TB][per_block]
-  float* sx = sdt + HY_SCAN_TB * per_block;
-  float* sz = sx + HY_SCAN_TB * per_block;
-  const int c0 = blockIdx.x * per_block;
-  const int cl = threadIdx.x / L;
-  const int c = c0 + cl;
-  const int sub = threadIdx.x % L;
+  float* sB = reinterpret_cast<float*>(hy_smem);               // [2][TB][NP]
+  float* sC = sB + 2 * TB * NP;                                // [2][TB][NP]
+  float* sdt = sC + 2 * TB * NP;                               // [2][TB][PB], step sizes once their batch has landed
+  AT* sx = reinterpret_cast<AT*>(sdt + 2 * TB * PB);           // [2][TB][PB]
+  AT* sz = sx + 2 * TB * PB;                                   // [2][TB][PB]
+  const int e = blockIdx.y, tid = threadIdx.x, c0 = blockIdx.x * PB;
+  const int cl = tid / L, sub = tid % L, n0 = sub * NPER, c = c0 + cl;
   const bool live = c < inner;
-  const int cc = live ? c : inner - 1;
+  const int cc = live ? c : inner - 1, npb = min(PB, inner - c0);
   const int start = b.ent_start[e], cnt = b.ent_start[e + 1] - start, pos0 = b.ent_pos0[e];
   float* st = state + ((size_t)b.ent_slot[e] * inner + cc) * nstate;
   float S[NPER], a[NPER];
 #pragma unroll
   for (int i = 0; i < NPER; ++i) {
-    const int n = sub + i * L;
+    const int n = n0 + i;
     S[i] = (n < nstate && pos0 > 0) ? st[n] : 0.0f;
     a[i] = n < nstate ? A[(size_t)cc * nstate + n] : 0.0f;
   }
   const float dd = to_f(D[cc]);
-  for (int j0 = 0; j0 < cnt; j0 += HY_SCAN_TB) {
-    const int nb = min(HY_SCAN_TB, cnt - j0);
-    __syncthreads();
-    for (int i = threadIdx.x; i < nb * nstate; i += blockDim.x) {
-      const int tt = i / nstate, n = i % nstate;
-      const size_t row = (size_t)(start + j0 + tt) * ldl;
-      sB[tt * nstate + n] = low[row + col_b + n];
-      sC[tt * nstate + n] = low[row + col_c + n];
+  if (nstate < NP)                                             // states beyond the last stay zero
+    for (int i = tid; i < 2 * TB * NP; i += 128) if (i % NP >= nstate) { sB[i] = 0.0f; sC[i] = 0.0f; }
+  auto fetch = [&](int j0, int buf) {
+    const int nb = min(TB, cnt - j0);
+    const size_t t0 = (size_t)(start + j0);
+    float* db = sB + buf * TB * NP;
+    float* dc = sC + buf * TB * NP;
+    float* dt = sdt + buf * TB * PB;
+    if (vec & 1) {
+      const int nc = nstate / 4, nd = npb / 4;
+      for (int i = tid; i < nb * nc; i += 128) {
+        const int r = i / nc, k = i % nc * 4;
+        const float* src = low + (t0 + r) * ldl + k;
+        jf::cp_async_16(db + r * NP + k, src + col_b, 16u);
+        jf::cp_async_16(dc + r * NP + k, src + col_c, 16u);
+      }
+      for (int i = tid; i < nb * nd; i += 128) jf::cp_async_16(dt + i / nd * PB + i % nd * 4, dt_raw + (t0 + i / nd) * lddt + c0 + i % nd * 4, 16u);
+    } else {
+      for (int i = tid; i < nb * nstate; i += 128) {
+        const int r = i / nstate, k = i % nstate;
+        db[r * NP + k] = low[(t0 + r) * ldl + col_b + k];
+        dc[r * NP + k] = low[(t0 + r) * ldl + col_c + k];
+      }
+      for (int i = tid; i < nb * npb; i += 128) dt[i / npb * PB + i % npb] = dt_raw[(t0 + i / npb) * lddt + c0 + i % npb];
     }
-    for (int i = threadIdx.x; i < nb * per_block; i += blockDim.x) {
-      const int tt = i / per_block, k = i % per_block;
-      const int ch = min(c0 + k, inner - 1);
-      const size_t t = (size_t)(start + j0 + tt);
-      sdt[i] = softplus_f(dt_raw[t * lddt + ch] + to_f(dt_bias[ch]));
-      sx[i] = to_f(x[t * ldx + ch]);
-      sz[i] = to_f(z[t * ldz + ch]);
+    AT* dx = sx + buf * TB * PB;
+    AT* dz = sz + buf * TB * PB;
+    if (vec & 2) {
+      const int nx = npb / CH;
+      for (int i = tid; i < nb * nx; i += 128) {
+        const int r = i / nx, k = i % nx * CH;
+        jf::cp_async_16(dx + r * PB + k, x + (t0 + r) * ldx + c0 + k, 16u);
+        jf::cp_async_16(dz + r * PB + k, z + (t0 + r) * ldz + c0 + k, 16u);
+      }
+    } else {
+      for (int i = tid; i < nb * npb; i += 128) {
+        dx[i / npb * PB + i % npb] = x[(t0 + i / npb) * ldx + c0 + i % npb];
+        dz[i / npb * PB + i % npb] = z[(t0 + i / npb) * ldz + c0 + i % npb];
+      }
     }
+    jf::cp_async_commit();
+  };
+  fetch(0, 0);
+  int buf = 0;
+  for (int j0 = 0; j0 < cnt; j0 += TB, buf ^= 1) {
+    const int nb = min(TB, cnt - j0);
+    jf::cp_async_wait_all();
+    __syncthreads();                                           // this batch has landed; the batch before it is finished
+    if (j0 + TB < cnt) fetch(j0 + TB, buf ^ 1);
+    float* bdt = sdt + buf * TB * PB;
+    for (int i = tid; i < nb * PB; i += 128)
+      if (i % PB < npb) bdt[i] = softplus_f(bdt[i] + to_f(dt_bias[c0 + i % PB]));
     __syncthreads();
-    for (int tt = 0; tt < nb; ++tt) {
-      const float dt = sdt[tt * per_block + cl], xv = sx[tt * per_block + cl];
-      const float dx = dt * xv;
-      float y = 0.0f;
+    const float* rb = sB + buf * TB * NP + n0;
+    const float* rc = sC + buf * TB * NP + n0;
+    const int ck = min(cl, npb - 1);
+    const AT* rx = sx + buf * TB * PB + ck;
+    const AT* rz = sz + buf * TB * PB + ck;
+    AT* po = out + (size_t)(start + j0) * ldo + cc;
+    auto update = [&](int tt) {                                // one token; returns this lane's part of the read-out
+      const float dt = bdt[tt * PB + ck], dx = dt * to_f(rx[tt * PB]);
+      float y0 = 0.0f, y1 = 0.0f;
 #pragma unroll
-      for (int i = 0; i < NPER; ++i) {
-        const int n = sub + i * L;
-        if (n < nstate) {
-          S[i] = fmaf(expf(dt * a[i]), S[i], dx * sB[tt * nstate + n]);
-          y = fmaf(S[i], sC[tt * nstate + n], y);
+      for (int i = 0; i < NPER; i += 4) {
+        const float4 bb = *reinterpret_cast<const float4*>(rb + tt * NP + i);
+        const float4 cv = *reinterpret_cast<const float4*>(rc + tt * NP + i);
+        S[i] = fmaf(expf(dt * a[i]), S[i], dx * bb.x); y0 = fmaf(S[i], cv.x, y0);
+        S[i + 1] = fmaf(expf(dt * a[i + 1]), S[i + 1], dx * bb.y); y1 = fmaf(S[i + 1], cv.y, y1);
+        S[i + 2] = fmaf(expf(dt * a[i + 2]), S[i + 2], dx * bb.z); y0 = fmaf(S[i + 2], cv.z, y0);
+        S[i + 3] = fmaf(expf(dt * a[i + 3]), S[i + 3], dx * bb.w); y1 = fmaf(S[i + 3], cv.w, y1);
+      }
+      return y0 + y1;
+    };
+    auto leave = [&](int tt, float y) {
+      y = fmaf(dd, to_f(rx[tt * PB]), y);
+      po[(size_t)tt * ldo] = from_f<AT>(y * silu_f(to_f(rz[tt * PB])) * out_scale);
+    };
+    int tt = 0;
+    for (; tt + TG <= nb; tt += TG) {
+      float p[TG];
+#pragma unroll
+      for (int u = 0; u < TG; ++u) p[u] = update(tt + u);
+      int n = TG, base = 0;
+#pragma unroll
+      for (int s = L >> 1; s >= 1; s >>= 1) {
+        const bool hi = (sub & s) != 0;
+        if (n > 1) {
+          n >>= 1;
+#pragma unroll
+          for (int u = 0; u < TG / 2; ++u) {
+            if (u >= n) break;
+            const float other = __shfl_xor_sync(0xffffffffu, hi ? p[u] : p[u + n], s);
+            p[u] = (hi ? p[u + n] : p[u]) + other;
+          }
+          base += hi ? n : 0;
+        } else {
+          p[0] += __shfl_xor_sync(0xffffffffu, p[0], s);
         }
       }
-      for (int o = L >> 1; o > 0; o >>= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
-      if (live && sub == 0) {
-        y = fmaf(dd, xv, y);
-        out[(size_t)(start + j0 + tt) * ldo + c] = from_f<AT>(y * silu_f(sz[tt * per_block + cl]) * out_scale);
+      constexpr int LEFT = TG > L ? TG / L : 1, SAME = L > TG ? L / TG : 1;        // tokens per lane, lanes per token
+      if (live && (sub & (SAME - 1)) == 0) {
+#pragma unroll
+        for (int u = 0; u < LEFT; ++u) leave(tt + base + u, p[u]);
       }
+    }
+    for (; tt < nb; ++tt) {
+      float y = update(tt);
+#pragma unroll
+      for (int s = L >> 1; s >= 1; s >>= 1) y += __shfl_xor_sync(0xffffffffu, y, s);
+      if (live && sub == 0) leave(tt, y);
     }
   }
   if (live) {
 #pragma unroll
-    for (int i = 0; i < NPER; ++i) {
-      const int n = sub + i * L;
-      if (n < nstate) st[n] = S[i];
-    }
+    for (int i = 0; i < NPER; ++i)
+      if (n0 + i < nstate) st[n0 + i] = S[i];
   }
-}
-
-// ---- gated delta rule with one decay per head and key channel ---------------------------------------------------------------------
-// Per head, S [dim, vdim] in shared memory, one block per (head, entry), thread j owns column j of S:
-//   S <- g * S (rows) ; u = beta (v - S^T k) ; S <- S + k u^T ; o = S^T q   (the read-out sees the current token's write)
-// q, k are made unit vectors per head (q also times dim^-1/2); g = exp(-exp(A_log_h) softplus(a + dt_bias));
-// out = o / rms(o) * norm_w * sigmoid(gate).  state [slot][H][dim][vdim] fp32.
-template <typename AT, typename WT>
-__global__ void delta_kernel(Batch b, const AT* __restrict__ qkv, int ldq, int col_q, int col_k, int col_v,
-                             const AT* __restrict__ beta_in, int ldb, int col_beta, const float* __restrict__ a_in, int lda,
-                             const float* __restrict__ gate_in, int ldg, const WT* __restrict__ A_log,
-                             const WT* __restrict__ dt_bias, const WT* __restrict__ norm_w, int H, int G, int dim, int vdim,
-                             float eps, float* __restrict__ state, AT* __restrict__ out, int ldo) {
-  extern __shared__ __align__(16) unsigned char hy_smem[];
-  float* S = reinterpret_cast<float*>(hy_smem);                // [dim][vdim]
-  float* ks = S + (size_t)dim * vdim;
-  float* qs = ks + dim;
-  float* gs = qs + dim;
-  float* red = gs + dim;                                       // 33
-  const int h = blockIdx.x, e = blockIdx.y, tid = threadIdx.x;
-  const int g = h / (H / G);
-  const int start = b.ent_start[e], cnt = b.ent_start[e + 1] - start, pos0 = b.ent_pos0[e];
-  float* st = state + ((size_t)b.ent_slot[e] * H + h) * dim * vdim;
-  for (int i = tid; i < dim * vdim; i += blockDim.x) S[i] = pos0 > 0 ? st[i] : 0.0f;
-  const float rate = expf(to_f(A_log[h]));
-  const float qscale = rsqrtf((float)dim);
-  __syncthreads();
-  for (int j = 0; j < cnt; ++j) {
-    const int t = start + j;
-    float qv = 0.0f, kv = 0.0f;
-    if (tid < dim) {
-      qv = to_f(qkv[(size_t)t * ldq + col_q + g * dim + tid]);
-      kv = to_f(qkv[(size_t)t * ldq + col_k + g * dim + tid]);
-      gs[tid] = expf(-rate * softplus_f(a_in[(size_t)t * lda + h * dim + tid] + to_f(dt_bias[h * dim + tid])));
-    }
-    const float q2 = block_sum(qv * qv, red);
-    const float k2 = block_sum(kv * kv, red);
-    if (tid < dim) {
-      qs[tid] = qv / sqrtf(q2 + 1e-6f) * qscale;
-      ks[tid] = kv / sqrtf(k2 + 1e-6f);
-    }
-    __syncthreads();
-    float o = 0.0f;
-    if (tid < vdim) {
-      float sk = 0.0f;
-      for (int i = 0; i < dim; ++i) {
-        const float s = S[i * vdim + tid] * gs[i];
-        S[i * vdim + tid] = s;
-        sk = fmaf(s, ks[i], sk);
-      }
-      const float bt = sigmoid_f(to_f(beta_in[(size_t)t * ldb + col_beta + h]));
-      const float u = bt * (to_f(qkv[(size_t)t * ldq + col_v + h * vdim + tid]) - sk);
-      for (int i = 0; i < dim; ++i) {
-        const float s = fmaf(ks[i], u, S[i * vdim + tid]);
-        S[i * vdim + tid] = s;
-        o = fmaf(s, qs[i], o);
-      }
-    }
-    const float o2 = block_sum(tid < vdim ? o * o : 0.0f, red);
-    if (tid < vdim) {
-      const float r = o / sqrtf(o2 / (float)vdim + eps);
-      const float gt = sigmoid_f(gate_in[(size_t)t * ldg + h * vdim + tid]);
-      out[(size_t)t * ldo + h * vdim + tid] = from_f<AT>(r * to_f(norm_w[tid]) * gt);
-    }
-  }
-  __syncthreads();
-  for (int i = tid; i < dim * vdim; i += blockDim.x) st[i] = S[i];
 }
 
 // Sum of two values over the block in one pass (same order rules as block_sum).  red: >= 66 floats.
@@ -662,21 +738,32 @@ __device__ __forceinline__ uint32_t mix32(uint64_t key, uint32_t ctr) {
   z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
   return (uint32_t)((z ^ (z >> 31)) >> 32);
 }
-__global__ void sample_kernel(const float* __restrict__ logits, int vocab, const float* __restrict__ temperature, uint64_t seed,
-                              int* __restrict__ out) {
+// One block per row.  256 threads with one 4-byte load in flight each took 62 us for 32000 logits; 1024 threads with four
+// independent loads 10 us.
+__global__ void __launch_bounds__(1024) sample_kernel(const float* __restrict__ logits, int vocab, const float* __restrict__ temperature,
+                                                      uint64_t seed, int* __restrict__ out) {
   __shared__ float bv[32];
   __shared__ int bi[32];
   const int r = blockIdx.x;
   const float temp = temperature ? temperature[r] : 0.0f;
+  const float* row = logits + (size_t)r * vocab;
   float best = -INFINITY;
   int besti = 0x7fffffff;
-  for (int v = threadIdx.x; v < vocab; v += blockDim.x) {
-    float s = logits[(size_t)r * vocab + v];
-    if (temp > 0.0f) {
-      const float uu = ((float)mix32(seed + (uint64_t)r * 0x100000001B3ull, (uint32_t)v) + 0.5f) * (1.0f / 4294967296.0f);
-      s = s / temp - logf(-logf(uu));
+  for (int v0 = threadIdx.x; v0 < vocab; v0 += 4 * blockDim.x) {
+    float x[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) x[k] = v0 + k * (int)blockDim.x < vocab ? row[v0 + k * blockDim.x] : 0.0f;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int v = v0 + k * blockDim.x;
+      if (v >= vocab) break;
+      float s = x[k];
+      if (temp > 0.0f) {
+        const float uu = ((float)mix32(seed + (uint64_t)r * 0x100000001B3ull, (uint32_t)v) + 0.5f) * (1.0f / 4294967296.0f);
+        s = s / temp - logf(-logf(uu));
+      }
+      if (s > best || (s == best && v < besti)) { best = s; besti = v; }
     }
-    if (s > best || (s == best && v < besti)) { best = s; besti = v; }
   }
   for (int o = 16; o > 0; o >>= 1) {
     const float ov = __shfl_xor_sync(0xffffffffu, best, o);

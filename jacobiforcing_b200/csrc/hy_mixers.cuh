@@ -41,140 +41,7 @@ __device__ __forceinline__ float rotated(const Rotation& r, const float* cs, int
 // ---- state-space recurrence, one decay per head ----------------------------------------------------------------------------
 // Per head h (group g = h / (heads / groups)), channel p, state n:
 //   dt = softplus(dt_raw_h + dt_bias_h) ; S[p, n] <- exp(-exp(A_log_h) dt) S[p, n] + dt x_p B_n ; y_p = sum_n S[p, n] C_n + D_h x_p
-// L lanes share a channel, each holding NPER CONSECUTIVE states in registers (state sizes up to NPER * L; B and C are
-// staged zero-padded to that size, so the inner loop has no bounds checks and reads them four at a time).  xbc [T, ldx]:
-// x at column 0 (heads * vdim), B at col_b, C at col_c (groups * nstate each), after convolution and activation.
-// state [slot][heads * vdim][nstate] fp32.  y leaves in fp32 (it enters a norm).  Inputs of HY_SSD_TB tokens (fewer for 256 states and more) are staged per
-// block as fp32; a block's 128 / L channels lie in one head.  Per token a thread spends about 3.5 instructions per state
-// plus a short shuffle tree: measured, the per-token overhead (indices, conversions, bounds, a 5-step tree for 4 states)
-// was four fifths of an earlier one-state-per-lane layout's instructions.
-constexpr int HY_SSD_TB = 32;
-template <typename AT, int NPER, int L>
-__global__ void __launch_bounds__(128) ssd_scan_kernel(Batch b, const AT* __restrict__ xbc, int ldx, int col_b, int col_c,
-                                                       const AT* __restrict__ dt_raw, int lddt, const float* __restrict__ dt_bias,
-                                                       const float* __restrict__ A_log, const float* __restrict__ D, int heads,
-                                                       int vdim, int nstate, int groups, int blocks_per_head,
-                                                       float* __restrict__ state, float* __restrict__ y, int ldy) {
-  constexpr int NP = NPER * L, PB = 128 / L, TB = NP >= 512 ? HY_SSD_TB / 4 : NP >= 256 ? HY_SSD_TB / 2 : HY_SSD_TB;
-  __shared__ __align__(16) float sB[TB * NP];
-  __shared__ __align__(16) float sC[TB * NP];
-  __shared__ float sx[TB * PB];
-  __shared__ float sdt[TB], sdec[TB];
-  const int e = blockIdx.y;
-  const int h = blockIdx.x / blocks_per_head;
-  const int p0 = (blockIdx.x % blocks_per_head) * PB;
-  const int g = h / (heads / groups);
-  const int cl = threadIdx.x / L, sub = threadIdx.x % L, n0 = sub * NPER;
-  const int p = p0 + cl;
-  const bool live = p < vdim;
-  const int pc = live ? p : vdim - 1;
-  const int start = b.ent_start[e], cnt = b.ent_start[e + 1] - start, pos0 = b.ent_pos0[e];
-  float* st = state + (((size_t)b.ent_slot[e] * heads + h) * vdim + pc) * nstate;
-  float S[NPER];
-#pragma unroll
-  for (int i = 0; i < NPER; ++i) S[i] = (n0 + i < nstate && pos0 > 0) ? st[n0 + i] : 0.0f;
-  const float rate = expf(A_log[h]), dd = D[h], bias = dt_bias[h];
-  const AT* xb = xbc + col_b + g * nstate;
-  const AT* xc = xbc + col_c + g * nstate;
-  const AT* xx = xbc + h * vdim;
-  float* yp = y + h * vdim + p;
-  // long entries: the raw inputs of the NEXT batch of tokens are fetched into registers before the current batch runs
-  constexpr int UB = TB * NP / 128, UX = (TB * PB + 127) / 128;
-  const bool ahead = cnt > TB;
-  AT rb[UB], rc[UB], rx[UX], rdt = from_f<AT>(0.0f);
-  auto fetch = [&](int j0, int nb) {
-#pragma unroll
-    for (int u = 0; u < UB; ++u) {
-      const int i = threadIdx.x + u * 128, tt = i / NP, n = i % NP;
-      const bool ok = tt < nb && n < nstate;
-      const size_t row = (size_t)(start + j0 + tt) * ldx;
-      rb[u] = ok ? xb[row + n] : from_f<AT>(0.0f);
-      rc[u] = ok ? xc[row + n] : from_f<AT>(0.0f);
-    }
-#pragma unroll
-    for (int u = 0; u < UX; ++u) {
-      const int i = threadIdx.x + u * 128, tt = i / PB, k = i % PB;
-      rx[u] = tt < nb ? xx[(size_t)(start + j0 + tt) * ldx + min(p0 + k, vdim - 1)] : from_f<AT>(0.0f);
-    }
-    if (threadIdx.x < nb) rdt = dt_raw[(size_t)(start + j0 + threadIdx.x) * lddt + h];
-  };
-  if (ahead) fetch(0, min(TB, cnt));
-  for (int j0 = 0; j0 < cnt; j0 += TB) {
-    const int nb = min(TB, cnt - j0);
-    __syncthreads();
-    if (ahead) {
-#pragma unroll
-      for (int u = 0; u < UB; ++u) {
-        const int i = threadIdx.x + u * 128;
-        sB[i] = to_f(rb[u]);
-        sC[i] = to_f(rc[u]);
-      }
-#pragma unroll
-      for (int u = 0; u < UX; ++u) {
-        const int i = threadIdx.x + u * 128;
-        if (i < TB * PB) sx[i] = to_f(rx[u]);
-      }
-      if (threadIdx.x < nb) {
-        const float dt = softplus_f(to_f(rdt) + bias);
-        sdt[threadIdx.x] = dt;
-        sdec[threadIdx.x] = expf(-rate * dt);
-      }
-    } else {
-#pragma unroll 4
-    for (int i = threadIdx.x; i < nb * NP; i += 128) {
-      const int tt = i / NP, n = i % NP;
-      const size_t row = (size_t)(start + j0 + tt) * ldx;
-      const bool ok = n < nstate;
-      sB[i] = ok ? to_f(xb[row + n]) : 0.0f;
-      sC[i] = ok ? to_f(xc[row + n]) : 0.0f;
-    }
-    for (int i = threadIdx.x; i < nb * PB; i += 128) {
-      const int tt = i / PB, k = i % PB;
-      sx[i] = to_f(xx[(size_t)(start + j0 + tt) * ldx + min(p0 + k, vdim - 1)]);
-    }
-    if (threadIdx.x < nb) {
-      const float dt = softplus_f(to_f(dt_raw[(size_t)(start + j0 + threadIdx.x) * lddt + h]) + bias);
-      sdt[threadIdx.x] = dt;
-      sdec[threadIdx.x] = expf(-rate * dt);
-    }
-    }
-    __syncthreads();
-    if (ahead && j0 + TB < cnt) fetch(j0 + TB, min(TB, cnt - j0 - TB));
-    float* yr = yp + (size_t)(start + j0) * ldy;
-    for (int tt = 0; tt < nb; ++tt, yr += ldy) {
-      const float dec = sdec[tt], xv = sx[tt * PB + cl];
-      const float dx = sdt[tt] * xv;
-      float a0 = 0.0f, a1 = 0.0f, a2 = 0.0f, a3 = 0.0f;
-      if constexpr (NPER % 4 == 0) {
-        const float4* b4 = reinterpret_cast<const float4*>(sB + tt * NP + n0);
-        const float4* c4 = reinterpret_cast<const float4*>(sC + tt * NP + n0);
-#pragma unroll
-        for (int i = 0; i < NPER / 4; ++i) {
-          const float4 bv = b4[i], cv = c4[i];
-          S[4 * i] = fmaf(dec, S[4 * i], dx * bv.x);         a0 = fmaf(S[4 * i], cv.x, a0);
-          S[4 * i + 1] = fmaf(dec, S[4 * i + 1], dx * bv.y); a1 = fmaf(S[4 * i + 1], cv.y, a1);
-          S[4 * i + 2] = fmaf(dec, S[4 * i + 2], dx * bv.z); a2 = fmaf(S[4 * i + 2], cv.z, a2);
-          S[4 * i + 3] = fmaf(dec, S[4 * i + 3], dx * bv.w); a3 = fmaf(S[4 * i + 3], cv.w, a3);
-        }
-      } else {
-#pragma unroll
-        for (int i = 0; i < NPER; ++i) {
-          S[i] = fmaf(dec, S[i], dx * sB[tt * NP + n0 + i]);
-          a0 = fmaf(S[i], sC[tt * NP + n0 + i], a0);
-        }
-      }
-      float acc = (a0 + a1) + (a2 + a3);
-#pragma unroll
-      for (int o = L >> 1; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-      if (live && sub == 0) *yr = fmaf(dd, xv, acc);
-    }
-  }
-  if (live) {
-#pragma unroll
-    for (int i = 0; i < NPER; ++i)
-      if (n0 + i < nstate) st[n0 + i] = S[i];
-  }
-}
+// It runs as gla_kernel<GLA_TOKEN> (hy_gla.cuh); its state is [slot][heads][nstate][vdim] fp32.  y leaves in fp32 (it enters a norm).
 
 // Gate, then norm: v = y silu(z); each of `parts` equal slices of a row is divided by its own root mean square; times w.
 template <typename AT>

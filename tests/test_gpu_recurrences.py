@@ -1,6 +1,7 @@
 """Recurrences whose value columns are spread over blocks, at the edges of their layouts: key sizes at and beside the padded sizes,
 value columns that fill a block's eight, miss one or need another block, portions that end at, before and behind a staged
-batch, and the size behind which another kernel takes over; fp32 build against the plain fp64 restatements, within the
+batch, and the size behind which another kernel takes over; the selective scan's lane layouts and the short convolution's
+chunks; fp32 build against the plain fp64 restatements, within the
 bound of the other fp32 tests (3e-4)."""
 import pytest
 
@@ -31,9 +32,40 @@ def test_channel_delta_columns(dim, vdim, heads, kv):
     assert _kinetar(kin.delta(heads=heads, kv_heads=kv, dim=dim, vdim=vdim, ff=0)) < kin.TOL["float32"]
 
 
-def test_channel_delta_beside_the_row_kernels_limit():
-    """Key rows of one token that no longer fit the row kernel's shared memory: a head's state in one block."""
+def test_channel_delta_many_wide_key_heads():
     assert _kinetar(kin.delta(heads=52, kv_heads=26, dim=1000, vdim=4, ff=0), cuts=[5, 1, 3], width=16) < kin.TOL["float32"]
+
+
+@pytest.mark.parametrize("state,inner,rank", [(1, 40, 1), (4, 132, 4), (5, 128, 4), (8, 64, 3), (9, 66, 4), (16, 32, 4), (16, 35, 2), (17, 48, 1), (33, 20, 4),
+                                              (65, 16, 2), (128, 12, 4), (129, 8, 4), (256, 5, 4)])
+def test_selective_scan_layouts(state, inner, rank):
+    """State sizes at and beside what one, two, ... thirty-two lanes hold; channels that fill a block, miss some or leave one over;
+    sizes that allow 16-byte copies beside sizes that do not."""
+    layer = kin.attn_scan(left_scale=0.0, inner=inner, state=state, dt_rank=rank)
+    layer["mlp"] = None
+    assert _kinetar(layer) < kin.TOL["float32"]
+
+
+@pytest.mark.parametrize("conv,width", [(4, 48), (4, 44), (2, 48), (16, 48)])
+@pytest.mark.parametrize("cuts", [[1, 2, 1, 15, 16, 17, 3], [33, 1, 48]])
+def test_convolution_chunks(conv, width, cuts):
+    """Portions shorter than the taps, ending at, before and behind a chunk of 16 tokens; four columns per thread or one."""
+    layer = kin.attn_scan(dim=16, conv=conv, sconv=conv, inner=40 if width == 48 else 42)
+    assert _kinetar(layer, cuts=cuts, width=width) < kin.TOL["float32"]
+
+
+@pytest.mark.parametrize("state,vdim,heads,groups", [(1, 3, 2, 1), (10, 8, 4, 2), (16, 9, 2, 2), (33, 12, 4, 1), (64, 8, 2, 1), (128, 20, 2, 1), (130, 4, 1, 1),
+                                                     (512, 4, 1, 1)])
+def test_state_space_columns(state, vdim, heads, groups):
+    cfg = fam.model_config([fam.ssd(heads=heads, vdim=vdim, state=state, groups=groups, norm_groups=1, conv=4, mlp=None)])
+    toks = kin.rand_tokens(sum(CUTS), cfg["vocab"], 5)
+    w = famepel_plain.random_weights(cfg, 0)
+    hz = fam.Harness(cfg, w, "float32")
+    try:
+        got = hz.feed("a", toks, CUTS)
+    finally:
+        hz.close()
+    assert kin.rel_err(got, fam.oracle_logits(cfg, w, toks)) < fam.TOL["float32"]
 
 
 @pytest.mark.parametrize("dim,vdim", [(16, 8), (15, 7), (33, 9), (64, 1), (128, 40), (136, 8), (520, 3), (1030, 5)])
