@@ -124,9 +124,10 @@ struct hy_engine {
   // repeated span of layers: the projection its passes begin with, its operand [step tokens, 2 width] (stream | embedding output)
   void* loop_w = nullptr; void* loop_w_t = nullptr; void* loop_cat = nullptr;
   // routed feed-forward: choices and weights per (token, choice) pair, the sorted order, the tile list
-  int* x_ids = nullptr; float* x_wts = nullptr; int* x_counts = nullptr; int* x_offs = nullptr; int* x_fill = nullptr;
-  int* x_tile_e = nullptr; int* x_tile_r0 = nullptr; int* x_meta = nullptr; int* x_row_tok = nullptr; int* x_pair_row = nullptr;
-  int x_max_tiles = 0;
+  int* x_ids = nullptr; float* x_wts = nullptr; int* x_counts = nullptr; int* x_offs = nullptr;
+  int* x_tile_e = nullptr; int* x_tile_r0 = nullptr; int* x_meta = nullptr; int* x_pair_row = nullptr;
+  void* x_rows = nullptr;                        // activation rows in the expert-sorted order
+  int x_max_tiles = 0, x_max_experts = 0, x_set = 0;
   int* err_d = nullptr; int* err_h = nullptr;
   // per-category device times (hy_profile_enable): event pairs recorded around groups of launches
   bool prof_on = false;
@@ -1382,15 +1383,15 @@ extern "C" int hy_finalize(hy_handle h) {
       h->x_max_tiles = (int)(P / HY_XT) + maxE + 1;          // enough for tiles of HY_XT rows and of 128 rows
       if (dev_alloc(h, (void**)&h->x_ids, P * 4, &h->bytes_ws)) return HY_ERR_CUDA;
       if (dev_alloc(h, (void**)&h->x_wts, P * 4, &h->bytes_ws)) return HY_ERR_CUDA;
-      if (dev_alloc(h, (void**)&h->x_row_tok, P * 4, &h->bytes_ws)) return HY_ERR_CUDA;
+      if (dev_alloc(h, &h->x_rows, P * W * es, &h->bytes_ws)) return HY_ERR_CUDA;
       if (dev_alloc(h, (void**)&h->x_pair_row, P * 4, &h->bytes_ws)) return HY_ERR_CUDA;
-      if (dev_alloc(h, (void**)&h->x_counts, (size_t)maxE * 4, &h->bytes_ws)) return HY_ERR_CUDA;
+      h->x_max_experts = maxE;                               // [2 sets][counts | fill][experts]
+      if (dev_alloc(h, (void**)&h->x_counts, (size_t)maxE * 16, &h->bytes_ws)) return HY_ERR_CUDA;
       if (dev_alloc(h, (void**)&h->x_offs, ((size_t)maxE + 1) * 4, &h->bytes_ws)) return HY_ERR_CUDA;
-      if (dev_alloc(h, (void**)&h->x_fill, (size_t)maxE * 4, &h->bytes_ws)) return HY_ERR_CUDA;
       if (dev_alloc(h, (void**)&h->x_tile_e, (size_t)h->x_max_tiles * 4, &h->bytes_ws)) return HY_ERR_CUDA;
       if (dev_alloc(h, (void**)&h->x_tile_r0, (size_t)h->x_max_tiles * 4, &h->bytes_ws)) return HY_ERR_CUDA;
       if (dev_alloc(h, (void**)&h->x_meta, 16, &h->bytes_ws)) return HY_ERR_CUDA;
-      HY_CUDA(cudaMemset(h->x_counts, 0, (size_t)maxE * 4));
+      HY_CUDA(cudaMemset(h->x_counts, 0, (size_t)maxE * 16));
       HY_CUDA(cudaMemset(h->x_meta, 0, 16));
     }
   }
@@ -1419,6 +1420,33 @@ inline bool gemm_takes_tiles(const void* A, int lda, int T, int K) {
   return !rows_fit && K % 8 == 0 && lda % 8 == 0 && (reinterpret_cast<uintptr_t>(A) & 15) == 0;
 }
 
+// The product on pairs of SMs: X [x_rows, K] (leading dimension lda), weight tiles of `groups` matrices [N, K], w_stride elements apart.
+// Tiles of 128 token rows when they fit one wave of the pairs (the wave is over sooner: N 1024, T 2048, K 6144: 45 us against 48 with
+// 256 rows), of 256 otherwise (N 2048, T 2048, K 2048: 27 us against 35).  Grouped: tile_rows as the tile list was made.
+template <typename TO>
+int pair_product(hy_engine* h, const bf16* X, int lda, int x_rows, const void* tiled, int groups, size_t w_stride, int T, int N, int K,
+                 const GemmOut& o, int tile_rows, TpGroup grp) {
+  static bool attr = false;                                  // per TO: this function is a template
+  if (!attr) {
+    cudaFuncSetAttribute(gemm_pair_kernel<TO, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tp_smem_bytes(128));
+    cudaFuncSetAttribute(gemm_pair_kernel<TO, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tp_smem_bytes(256));
+    attr = true;
+  }
+  const int nx = (N + 255) / 256, KT = (K + 63) / 64, NT = (N + 127) / 128;
+  const int bt = tile_rows ? tile_rows : (long long)nx * ((T + 127) / 128) <= TP_CLUSTERS ? 128 : 256;
+  const uint64_t w_rows = groups > 1 ? (uint64_t)groups * (w_stride / 64) : (uint64_t)NT * KT * 128;
+  CUtensorMap xm, wm;
+  if (!tp_map(&xm, X, (uint64_t)x_rows, (uint64_t)K, (uint64_t)lda, bt / 2, true) || !tp_map(&wm, tiled, w_rows, 64, 64, 128, false))
+    return fail(h, HY_ERR_CUDA, "a tensor map of the matrix product could not be made");
+  grp.w_rows = (int)(w_stride / 64);
+  const long long most = (long long)nx * (grp.meta ? x_rows / bt + groups : (T + bt - 1) / bt);      // tiles (grouped: at most)
+  const int grid = 2 * (int)std::min<long long>(most, TP_CLUSTERS);
+  if (bt == 128) gemm_pair_kernel<TO, 128><<<grid, TP_THREADS, tp_smem_bytes(128), h->stream>>>(xm, wm, T, N, K, o, h->err_d, grp);
+  else gemm_pair_kernel<TO, 256><<<grid, TP_THREADS, tp_smem_bytes(256), h->stream>>>(xm, wm, T, N, K, o, h->err_d, grp);
+  h->launches++;
+  return HY_OK;
+}
+
 template <typename TA, typename TW, typename TO>
 int gemm(hy_engine* h, const TA* A, int lda, const TW* Wt, int ldw, int T, int N, int K, GemmOut o,
          const void* tiled = nullptr) {
@@ -1426,21 +1454,7 @@ int gemm(hy_engine* h, const TA* A, int lda, const TW* Wt, int ldw, int T, int N
   if (o.alpha == 0.0f) o.alpha = 1.0f;
   if constexpr (std::is_same<TA, bf16>::value && std::is_same<TW, bf16>::value) {
     if (tiled && gemm_takes_tiles(A, lda, T, K)) {
-      static bool attr_set = false;
-      if (!attr_set) {
-        cudaFuncSetAttribute(gemm_tc_kernel<TO, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc_smem_bytes(128));
-        cudaFuncSetAttribute(gemm_tc_kernel<TO, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc_smem_bytes(256));
-        attr_set = true;
-      }
-      // 256-row tiles halve the weight traffic per row; 128-row tiles when the wider ones would leave SMs without a CTA
-      if (T > 128 && (long long)((N + 127) / 128) * ((T + 255) / 256) >= 148)
-        gemm_tc_kernel<TO, 256><<<dim3((N + 127) / 128, (T + 255) / 256), 192, tc_smem_bytes(256), h->stream>>>(
-            A, lda, (const bf16*)tiled, T, N, K, o, h->err_d, TcGroup{});
-      else
-        gemm_tc_kernel<TO, 128><<<dim3((N + 127) / 128, (T + 127) / 128), 192, tc_smem_bytes(128), h->stream>>>(
-            A, lda, (const bf16*)tiled, T, N, K, o, h->err_d, TcGroup{});
-      h->launches++;
-      return HY_OK;
+      return pair_product<TO>(h, (const bf16*)A, lda, T, tiled, 1, 0, T, N, K, o, 0, TpGroup{});
     }
   }
   constexpr int VECW = 16 / (int)sizeof(TW);
@@ -1723,6 +1737,23 @@ void latent_mixer(hy_engine* h, const Batch& b, const LayerW& L, const hy_layer_
   }
 }
 
+// Routing tables of a layer: the counters that its route kernel fills (the two sets alternate, see route_place_kernel), rows per
+// tile of the grouped products, the expert-sorted order with the activation rows copied into it.
+int* next_counts(hy_engine* h) { h->x_set ^= 1; return h->x_counts + (size_t)h->x_set * 2 * h->x_max_experts; }
+// 256 rows per tile once experts have about that many (2048 tokens x 4 choices over 32 experts); 128 below
+int expert_tile_rows(int P, int NE) { return P >= 192 * NE ? 256 : 128; }
+template <typename AT>
+void place_rows(hy_engine* h, int T, const AT* hb, const LayerW& L, const hy_layer_cfg& c, AT* rows) {
+  const int P = T * c.x_top, W = h->m.width, E = h->x_max_experts;
+  const bool tc = std::is_same<AT, bf16>::value && L.w_gu_t != nullptr;
+  int* now = h->x_counts + (size_t)h->x_set * 2 * E;
+  int* old = h->x_counts + (size_t)(h->x_set ^ 1) * 2 * E;
+  route_place_kernel<AT><<<P + 1, 128, 0, h->stream>>>(P, c.x_top, c.x_experts, E, tc ? expert_tile_rows(P, c.x_experts) : HY_XT, h->x_ids, now, now + E,
+                                                       old, old + E, hb, W, W % (16 / (int)sizeof(AT)) == 0, h->x_offs, h->x_tile_e, h->x_tile_r0,
+                                                       h->x_meta, h->x_pair_row, rows);
+  h->launches++;
+}
+
 // One layer of a norm - sublayer - norm model:  x += ls1 * n1b(mixer(n1(x)));  x += ls2 * n2b(experts(n2(x))).
 // The output norms are element-wise, so they run in the epilogue of the mixer's output projection and in the experts'
 // combine kernel, on the fp32 accumulators, together with the layer scale and the residual sum.
@@ -1816,6 +1847,7 @@ int sandwich_layer(hy_engine* h, const Batch& b, size_t li) {
   }
   if (!routed) return HY_OK;
   const int NE = c.x_experts, top = c.x_top, ff = c.ff, P = T * top, ldh = (ff + 7) & ~7;
+  AT* x_rows = (AT*)h->x_rows;
   const bool tc_experts = std::is_same<AT, bf16>::value && L.w_gu_t != nullptr;
   // a handful of pairs: one block row per pair; beyond that the sorted order, where pairs that share an expert share its
   // stream (measured at 8 tokens x 4 experts of 32: the tensor-core product over the sorted order is 2.5 - 5 times faster)
@@ -1825,13 +1857,10 @@ int sandwich_layer(hy_engine* h, const Batch& b, size_t li) {
     ProfScope ps(h, HY_PROF_ROUTE);
     gemm<AT, WT, float>(h, hb, W, (const WT*)L.w_router, W, T, NE, W, to_buf(h->f1, h->ld_f1), L.w_router_t);
     const RouteCfg rc{NE, top, c.x_groups, c.x_keep, c.x_scale};
-    route_kernel<<<T, 32, (size_t)(NE + c.x_groups) * 4, s>>>(h->f1, h->ld_f1, rc, h->x_ids, h->x_wts, few ? nullptr : h->x_counts);
+    route_kernel<<<T, 32, (size_t)(NE + c.x_groups) * 4, s>>>(h->f1, h->ld_f1, rc, h->x_ids, h->x_wts, few ? nullptr : next_counts(h));
     h->launches++;
     if (!few) {
-      route_offsets_kernel<<<1, 32, 0, s>>>(h->x_counts, NE, tc_experts ? 128 : HY_XT, h->x_offs, h->x_fill, h->x_tile_e,
-                                            h->x_tile_r0, h->x_meta);
-      route_scatter_kernel<<<(P + 255) / 256, 256, 0, s>>>(P, top, NE, h->x_ids, h->x_offs, h->x_fill, h->x_row_tok, h->x_pair_row);
-      h->launches += 2;
+      place_rows<AT>(h, T, hb, L, c, x_rows);
     }
   }
   {
@@ -1850,28 +1879,18 @@ int sandwich_layer(hy_engine* h, const Batch& b, size_t li) {
           pin, ldh, h->x_ids, top, 0, NE, (const WT*)L.w_down, (size_t)W * ff, W, ff, ys, W, -1, 0.0f);
     } else if (tc_experts) {
       if constexpr (std::is_same<AT, bf16>::value) {
-        static bool attr_set = false;
-        if (!attr_set) {
-          cudaFuncSetAttribute(gemm_tc_kernel<bf16, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc_smem_bytes(128));
-          cudaFuncSetAttribute(gemm_tc_kernel<float, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc_smem_bytes(128));
-          attr_set = true;
-        }
-        const int tiles = std::min(h->x_max_tiles, P / 128 + NE + 1);
-        const TcGroup g1{h->x_meta, h->x_offs, h->x_tile_e, h->x_tile_r0, h->x_row_tok, L.gu_t_stride};
-        const TcGroup g2{h->x_meta, h->x_offs, h->x_tile_e, h->x_tile_r0, nullptr, L.down_t_stride};
+        const TpGroup grp{h->x_meta, h->x_offs, h->x_tile_e, h->x_tile_r0, 0};
         GemmOut o1{pin, ldh, ff, nullptr, 0, 2, nullptr, 0, 1.0f};
-        gemm_tc_kernel<bf16, 128><<<dim3((L.gu_rows + 127) / 128, tiles), 192, tc_smem_bytes(128), s>>>(
-            hb, W, (const bf16*)L.w_gu_t, P, L.gu_rows, W, o1, h->err_d, g1);
+        pair_product<bf16>(h, x_rows, W, P, L.w_gu_t, NE, L.gu_t_stride, P, L.gu_rows, W, o1, expert_tile_rows(P, NE), grp);
         GemmOut o2 = to_buf(ys, W);
-        gemm_tc_kernel<float, 128><<<dim3((W + 127) / 128, tiles), 192, tc_smem_bytes(128), s>>>(
-            pin, ldh, (const bf16*)L.w_down_t, P, W, ff, o2, h->err_d, g2);
+        pair_product<float>(h, pin, ldh, P, L.w_down_t, NE, L.down_t_stride, P, W, ff, o2, expert_tile_rows(P, NE), grp);
       }
     } else {
       const int tiles = std::min(h->x_max_tiles, P / HY_XT + NE + 1);
       expert_gemm_simt_kernel<AT, WT, AT, true><<<dim3((ff + 63) / 64, tiles), 256, 0, s>>>(
-          hb, W, h->x_row_tok, (const WT*)L.w_gu, (size_t)2 * ff * W, ff, W, h->x_offs, h->x_tile_e, h->x_tile_r0, h->x_meta, pin, ldh, 0, 0.0f);
+          x_rows, W, (const WT*)L.w_gu, (size_t)2 * ff * W, ff, W, h->x_offs, h->x_tile_e, h->x_tile_r0, h->x_meta, pin, ldh, 0, 0.0f);
       expert_gemm_simt_kernel<AT, WT, float, false><<<dim3((W + 63) / 64, tiles), 256, 0, s>>>(
-          pin, ldh, nullptr, (const WT*)L.w_down, (size_t)W * ff, W, ff, h->x_offs, h->x_tile_e, h->x_tile_r0, h->x_meta, ys, W, -1, 0.0f);
+          pin, ldh, (const WT*)L.w_down, (size_t)W * ff, W, ff, h->x_offs, h->x_tile_e, h->x_tile_r0, h->x_meta, ys, W, -1, 0.0f);
     }
     expert_combine_kernel<AT><<<T, 256, 0, s>>>(ys, W, few ? nullptr : h->x_pair_row, h->x_wts, top, W, L.n2b, L.ls2, h->x, after_ff, hb);
     h->launches += 3;
@@ -2033,6 +2052,7 @@ int postnorm_layer(hy_engine* h, const Batch& b, size_t li) {
   }
   // routed plain experts: down(act(up x)), beside a shared expert of the same form
   const int NE = c.x_experts, top = c.x_top, ff = c.ff, P = T * top, ldh = (ff + 7) & ~7;
+  AT* x_rows = (AT*)h->x_rows;
   const bool tc_experts = std::is_same<AT, bf16>::value && L.w_gu_t != nullptr;
   static const int rows_max_env = getenv("HY_EXPERT_ROWS_MAX") ? atoi(getenv("HY_EXPERT_ROWS_MAX")) : -1;   // developer switch
   const bool few = P <= (rows_max_env >= 0 ? rows_max_env : tc_experts ? 8 : 16);
@@ -2040,17 +2060,14 @@ int postnorm_layer(hy_engine* h, const Batch& b, size_t li) {
     ProfScope ps(h, HY_PROF_ROUTE);
     gemm<AT, WT, float>(h, hb, W, (const WT*)L.w_router, W, T, NE, W, to_buf(h->f1, h->ld_f1), L.w_router_t);
     if (c.x_route == HY_ROUTE_TOP_SOFTMAX) {
-      route_top_kernel<<<T, 32, (size_t)NE * 4, s>>>(h->f1, h->ld_f1, L.x_rb, NE, top, h->x_ids, h->x_wts, few ? nullptr : h->x_counts);
+      route_top_kernel<<<T, 32, (size_t)NE * 4, s>>>(h->f1, h->ld_f1, L.x_rb, NE, top, h->x_ids, h->x_wts, few ? nullptr : next_counts(h));
     } else {
       const RouteCfg rc{NE, top, c.x_groups, c.x_keep, c.x_scale};
-      route_kernel<<<T, 32, (size_t)(NE + c.x_groups) * 4, s>>>(h->f1, h->ld_f1, rc, h->x_ids, h->x_wts, few ? nullptr : h->x_counts);
+      route_kernel<<<T, 32, (size_t)(NE + c.x_groups) * 4, s>>>(h->f1, h->ld_f1, rc, h->x_ids, h->x_wts, few ? nullptr : next_counts(h));
     }
     h->launches++;
     if (!few) {
-      route_offsets_kernel<<<1, 32, 0, s>>>(h->x_counts, NE, tc_experts ? 128 : HY_XT, h->x_offs, h->x_fill, h->x_tile_e,
-                                            h->x_tile_r0, h->x_meta);
-      route_scatter_kernel<<<(P + 255) / 256, 256, 0, s>>>(P, top, NE, h->x_ids, h->x_offs, h->x_fill, h->x_row_tok, h->x_pair_row);
-      h->launches += 2;
+      place_rows<AT>(h, T, hb, L, c, x_rows);
     }
   }
   float* ys = h->f2;                                          // [pairs (+ tokens: the shared expert's rows), width] fp32
@@ -2070,29 +2087,19 @@ int postnorm_layer(hy_engine* h, const Batch& b, size_t li) {
           pin, ldh, h->x_ids, top, 0, NE, (const WT*)L.w_down, (size_t)W * ff, W, ff, ys, W, -1, 0.0f);
     } else if (tc_experts) {
       if constexpr (std::is_same<AT, bf16>::value) {
-        static bool attr_set = false;
-        if (!attr_set) {
-          cudaFuncSetAttribute(gemm_tc_kernel<bf16, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc_smem_bytes(128));
-          cudaFuncSetAttribute(gemm_tc_kernel<float, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc_smem_bytes(128));
-          attr_set = true;
-        }
-        const int tiles = std::min(h->x_max_tiles, P / 128 + NE + 1);
-        const TcGroup g1{h->x_meta, h->x_offs, h->x_tile_e, h->x_tile_r0, h->x_row_tok, L.gu_t_stride};
-        const TcGroup g2{h->x_meta, h->x_offs, h->x_tile_e, h->x_tile_r0, nullptr, L.down_t_stride};
+        const TpGroup grp{h->x_meta, h->x_offs, h->x_tile_e, h->x_tile_r0, 0};
         GemmOut o1 = to_buf(pin, ldh);
         o1.act2 = 3; o1.act_kind = c.x_act;
-        gemm_tc_kernel<bf16, 128><<<dim3((ff + 127) / 128, tiles), 192, tc_smem_bytes(128), s>>>(
-            hb, W, (const bf16*)L.w_gu_t, P, ff, W, o1, h->err_d, g1);
+        pair_product<bf16>(h, x_rows, W, P, L.w_gu_t, NE, L.gu_t_stride, P, ff, W, o1, expert_tile_rows(P, NE), grp);
         GemmOut o2 = to_buf(ys, W);
-        gemm_tc_kernel<float, 128><<<dim3((W + 127) / 128, tiles), 192, tc_smem_bytes(128), s>>>(
-            pin, ldh, (const bf16*)L.w_down_t, P, W, ff, o2, h->err_d, g2);
+        pair_product<float>(h, pin, ldh, P, L.w_down_t, NE, L.down_t_stride, P, W, ff, o2, expert_tile_rows(P, NE), grp);
       }
     } else {
       const int tiles = std::min(h->x_max_tiles, P / HY_XT + NE + 1);
       expert_gemm_simt_kernel<AT, WT, AT, false><<<dim3((ff + 63) / 64, tiles), 256, 0, s>>>(
-          hb, W, h->x_row_tok, (const WT*)L.w_gu, (size_t)ff * W, ff, W, h->x_offs, h->x_tile_e, h->x_tile_r0, h->x_meta, pin, ldh, c.x_act, c.ff_limit);
+          x_rows, W, (const WT*)L.w_gu, (size_t)ff * W, ff, W, h->x_offs, h->x_tile_e, h->x_tile_r0, h->x_meta, pin, ldh, c.x_act, c.ff_limit);
       expert_gemm_simt_kernel<AT, WT, float, false><<<dim3((W + 63) / 64, tiles), 256, 0, s>>>(
-          pin, ldh, nullptr, (const WT*)L.w_down, (size_t)W * ff, W, ff, h->x_offs, h->x_tile_e, h->x_tile_r0, h->x_meta, ys, W, -1, 0.0f);
+          pin, ldh, (const WT*)L.w_down, (size_t)W * ff, W, ff, h->x_offs, h->x_tile_e, h->x_tile_r0, h->x_meta, ys, W, -1, 0.0f);
     }
     h->launches += 2;
     if (c.x_shared_ff > 0) {
@@ -2119,6 +2126,7 @@ bool routed_gated_experts(hy_engine* h, int T, const AT* hb, const LayerW& L, co
   cudaStream_t s = h->stream;
   AT* pin = (AT*)h->pin;
   const int NE = c.x_experts, top = c.x_top, ff = c.ff, P = T * top, ldh = (ff + 7) & ~7;
+  AT* x_rows = (AT*)h->x_rows;
   const bool tc_experts = std::is_same<AT, bf16>::value && L.w_gu_t != nullptr;
   const bool few = P <= (tc_experts ? 8 : 16);
   {
@@ -2127,17 +2135,14 @@ bool routed_gated_experts(hy_engine* h, int T, const AT* hb, const LayerW& L, co
       const int outputs = NE + c.x_identity;
       if (L.w_router) gemm<AT, WT, float>(h, hb, W, (const WT*)L.w_router, W, T, outputs, W, to_buf(h->f1, h->ld_f1), L.w_router_t);
       route_corrected_kernel<<<T, 32, (size_t)(2 * outputs + c.x_groups) * 4, s>>>(h->f1 + L.c_router, h->ld_f1, L.x_corr, NE, outputs, top,
-                                                                                   c.x_groups, c.x_keep, h->x_ids, h->x_wts, few ? nullptr : h->x_counts);
+                                                                                   c.x_groups, c.x_keep, h->x_ids, h->x_wts, few ? nullptr : next_counts(h));
     } else {
       gemm<AT, WT, float>(h, hb, W, (const WT*)L.w_router, W, T, NE, W, to_buf(h->f1, h->ld_f1), L.w_router_t);
-      route_top_kernel<<<T, 32, (size_t)NE * 4, s>>>(h->f1, h->ld_f1, nullptr, NE, top, h->x_ids, h->x_wts, few ? nullptr : h->x_counts);
+      route_top_kernel<<<T, 32, (size_t)NE * 4, s>>>(h->f1, h->ld_f1, nullptr, NE, top, h->x_ids, h->x_wts, few ? nullptr : next_counts(h));
     }
     h->launches++;
     if (!few) {
-      route_offsets_kernel<<<1, 32, 0, s>>>(h->x_counts, NE, tc_experts ? 128 : HY_XT, h->x_offs, h->x_fill, h->x_tile_e,
-                                            h->x_tile_r0, h->x_meta);
-      route_scatter_kernel<<<(P + 255) / 256, 256, 0, s>>>(P, top, NE, h->x_ids, h->x_offs, h->x_fill, h->x_row_tok, h->x_pair_row);
-      h->launches += 2;
+      place_rows<AT>(h, T, hb, L, c, x_rows);
     }
   }
   ProfScope ps(h, HY_PROF_EXPERTS);
@@ -2155,29 +2160,19 @@ bool routed_gated_experts(hy_engine* h, int T, const AT* hb, const LayerW& L, co
         pin, ldh, h->x_ids, top, 0, NE, (const WT*)L.w_down, (size_t)W * ff, W, ff, ys, W, -1, 0.0f);
   } else if (tc_experts) {
     if constexpr (std::is_same<AT, bf16>::value) {
-      static bool attr_set = false;
-      if (!attr_set) {
-        cudaFuncSetAttribute(gemm_tc_kernel<bf16, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc_smem_bytes(128));
-        cudaFuncSetAttribute(gemm_tc_kernel<float, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc_smem_bytes(128));
-        attr_set = true;
-      }
-      const int tiles = std::min(h->x_max_tiles, P / 128 + NE + 1);
-      const TcGroup g1{h->x_meta, h->x_offs, h->x_tile_e, h->x_tile_r0, h->x_row_tok, L.gu_t_stride};
-      const TcGroup g2{h->x_meta, h->x_offs, h->x_tile_e, h->x_tile_r0, nullptr, L.down_t_stride};
+      const TpGroup grp{h->x_meta, h->x_offs, h->x_tile_e, h->x_tile_r0, 0};
       GemmOut o1{pin, ldh, ff, nullptr, 0, 2, nullptr, 0, 1.0f};
       o1.act_kind = c.x_act; o1.act_limit = c.ff_limit;
-      gemm_tc_kernel<bf16, 128><<<dim3((L.gu_rows + 127) / 128, tiles), 192, tc_smem_bytes(128), s>>>(
-          hb, W, (const bf16*)L.w_gu_t, P, L.gu_rows, W, o1, h->err_d, g1);
+      pair_product<bf16>(h, x_rows, W, P, L.w_gu_t, NE, L.gu_t_stride, P, L.gu_rows, W, o1, expert_tile_rows(P, NE), grp);
       GemmOut o2 = to_buf(ys, W);
-      gemm_tc_kernel<float, 128><<<dim3((W + 127) / 128, tiles), 192, tc_smem_bytes(128), s>>>(
-          pin, ldh, (const bf16*)L.w_down_t, P, W, ff, o2, h->err_d, g2);
+      pair_product<float>(h, pin, ldh, P, L.w_down_t, NE, L.down_t_stride, P, W, ff, o2, expert_tile_rows(P, NE), grp);
     }
   } else {
     const int tiles = std::min(h->x_max_tiles, P / HY_XT + NE + 1);
     expert_gemm_simt_kernel<AT, WT, AT, true><<<dim3((ff + 63) / 64, tiles), 256, 0, s>>>(
-        hb, W, h->x_row_tok, (const WT*)L.w_gu, (size_t)2 * ff * W, ff, W, h->x_offs, h->x_tile_e, h->x_tile_r0, h->x_meta, pin, ldh, c.x_act, c.ff_limit);
+        x_rows, W, (const WT*)L.w_gu, (size_t)2 * ff * W, ff, W, h->x_offs, h->x_tile_e, h->x_tile_r0, h->x_meta, pin, ldh, c.x_act, c.ff_limit);
     expert_gemm_simt_kernel<AT, WT, float, false><<<dim3((W + 63) / 64, tiles), 256, 0, s>>>(
-        pin, ldh, nullptr, (const WT*)L.w_down, (size_t)W * ff, W, ff, h->x_offs, h->x_tile_e, h->x_tile_r0, h->x_meta, ys, W, -1, 0.0f);
+        pin, ldh, (const WT*)L.w_down, (size_t)W * ff, W, ff, h->x_offs, h->x_tile_e, h->x_tile_r0, h->x_meta, ys, W, -1, 0.0f);
   }
   h->launches += 2;
   return few;

@@ -153,45 +153,70 @@ __global__ void gated_act_kernel(const AT* __restrict__ in, int ldi, int n, int 
   if (f < n) out[(size_t)t * ldo + f] = from_f<AT>(gated_pair_f(act, to_f(in[(size_t)t * ldi + f]), to_f(in[(size_t)t * ldi + n + f]), limit));
 }
 
-// Tiles of tile_rows rows of one expert (HY_XT for the SIMT product, 128 for the tensor-core product).  meta: [0] number
-// of tiles; offs [experts + 1]; fill [experts] zeroed here.
+// The expert-sorted order.  One block per (token, choice) pair and one more: a pair's block finds the pair's row (behind the
+// rows of the experts before its own, in order of arrival among its own) and copies the token's activation row there; the last block
+// leaves the offsets, the tiles of tile_rows rows of one expert each (meta[0]: their number), and clears the counters of the
+// routed layer before this one (most_experts of them; counts and fill of two layers alternate, so nobody clears what another
+// block still reads).  A choice that is no expert (an identity choice) gets no row: pair_row -1.  vec: rows are copied 16 bytes
+// at a time.  Offsets by one thread, the order, and rows fetched through it inside the products took 7 + 4 us and held the products
+// back; this takes PLACE_US us for 2048 tokens x 4 choices of 1024 channels.
 constexpr int HY_XT = 64;
-__global__ void route_offsets_kernel(int* __restrict__ counts, int experts, int tile_rows, int* __restrict__ offs,
-                                     int* __restrict__ fill, int* __restrict__ tile_expert, int* __restrict__ tile_row0,
-                                     int* __restrict__ meta) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  int at = 0, nt = 0;
-  for (int e = 0; e < experts; ++e) {
-    const int n = counts[e];
-    offs[e] = at;
-    for (int r = 0; r < n; r += tile_rows) { tile_expert[nt] = e; tile_row0[nt] = at + r; ++nt; }
-    at += n;
-    fill[e] = 0;
-    counts[e] = 0;                                             // ready for the next routed layer
+template <typename AT>
+__global__ void __launch_bounds__(128) route_place_kernel(int pairs, int top, int experts, int most_experts, int tile_rows,
+                                                          const int* __restrict__ ids, const int* __restrict__ counts, int* __restrict__ fill,
+                                                          int* __restrict__ old_counts, int* __restrict__ old_fill, const AT* __restrict__ h,
+                                                          int width, int vec, int* __restrict__ offs, int* __restrict__ tile_expert,
+                                                          int* __restrict__ tile_row0, int* __restrict__ meta, int* __restrict__ pair_row,
+                                                          AT* __restrict__ rows) {
+  const int i = blockIdx.x, lane = threadIdx.x & 31;
+  if (i == pairs) {
+    for (int e = threadIdx.x; e < most_experts; e += blockDim.x) { old_counts[e] = 0; old_fill[e] = 0; }
+    if (threadIdx.x >= 32) return;
+    int at = 0, nt = 0;
+    for (int e0 = 0; e0 < experts; e0 += 32) {                 // running sums of rows and of tiles, 32 experts at a time
+      const int e = e0 + lane, n = e < experts ? counts[e] : 0, m = (n + tile_rows - 1) / tile_rows;
+      int sn = n, sm = m;
+#pragma unroll
+      for (int s = 1; s < 32; s <<= 1) {
+        const int a = __shfl_up_sync(0xffffffffu, sn, s), c = __shfl_up_sync(0xffffffffu, sm, s);
+        if (lane >= s) { sn += a; sm += c; }
+      }
+      if (e < experts) {
+        offs[e] = at + sn - n;
+        for (int r = 0; r < m; ++r) { tile_expert[nt + sm - m + r] = e; tile_row0[nt + sm - m + r] = at + sn - n + r * tile_rows; }
+      }
+      at += __shfl_sync(0xffffffffu, sn, 31);
+      nt += __shfl_sync(0xffffffffu, sm, 31);
+    }
+    if (lane == 0) { offs[experts] = at; meta[0] = nt; }
+    return;
   }
-  offs[experts] = at;
-  meta[0] = nt;
-}
-
-// pair i = (token i / top, choice i % top) -> row of the sorted order; row_tok[row] = token, pair_row[i] = row.
-// A choice that is no expert (an identity choice) gets no row.
-__global__ void route_scatter_kernel(int pairs, int top, int experts, const int* __restrict__ ids, const int* __restrict__ offs,
-                                     int* __restrict__ fill, int* __restrict__ row_tok, int* __restrict__ pair_row) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= pairs) return;
   const int e = ids[i];
-  if (e >= experts) { pair_row[i] = -1; return; }
-  const int row = offs[e] + atomicAdd(&fill[e], 1);
-  row_tok[row] = i / top;
-  pair_row[i] = row;
+  if (e >= experts) { if (threadIdx.x == 0) pair_row[i] = -1; return; }
+  __shared__ int srow;
+  if (threadIdx.x < 32) {
+    int before = 0;
+    for (int k = lane; k < e; k += 32) before += counts[k];
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) before += __shfl_xor_sync(0xffffffffu, before, s);
+    if (lane == 0) { srow = before + atomicAdd(&fill[e], 1); pair_row[i] = srow; }
+  }
+  __syncthreads();
+  const AT* src = h + (size_t)(i / top) * width;
+  AT* dst = rows + (size_t)srow * width;
+  if (vec) {
+    constexpr int CH = 16 / (int)sizeof(AT);
+    for (int k = threadIdx.x; k < width / CH; k += blockDim.x) reinterpret_cast<uint4*>(dst)[k] = reinterpret_cast<const uint4*>(src)[k];
+  } else {
+    for (int k = threadIdx.x; k < width; k += blockDim.x) dst[k] = src[k];
+  }
 }
 
-// Grouped product over the sorted rows: C[row, n] = sum_k A[src(row), k] W_e[n, k], e the expert of the row's tile.
+// Grouped product over the sorted rows: C[row, n] = sum_k A[row, k] W_e[n, k], e the expert of the row's tile.
 // GLU: W_e is [2 N, K] (gate rows, then up rows) and the result is the gated pair (see gated_pair_f); without GLU the result passes through
-// the activation when act >= 0 (act: 0 silu, 1 tanh-gelu, 2 erf-gelu; see act_f).  src(row) = row_map[row] when a map
-// is given (activation rows of the tokens), else row.  Tiled SIMT, fp32 FMAs in k order: both builds can use it.
+// the activation when act >= 0 (act: 0 silu, 1 tanh-gelu, 2 erf-gelu; see act_f).  Tiled SIMT, fp32 FMAs in k order: both builds can use it.
 template <typename TA, typename TW, typename TO, bool GLU>
-__global__ void __launch_bounds__(256) expert_gemm_simt_kernel(const TA* __restrict__ A, int lda, const int* __restrict__ row_map,
+__global__ void __launch_bounds__(256) expert_gemm_simt_kernel(const TA* __restrict__ A, int lda,
                                                                const TW* __restrict__ W, size_t w_stride, int N, int K,
                                                                const int* __restrict__ offs, const int* __restrict__ tile_expert,
                                                                const int* __restrict__ tile_row0, const int* __restrict__ meta,
@@ -208,7 +233,7 @@ __global__ void __launch_bounds__(256) expert_gemm_simt_kernel(const TA* __restr
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
     __syncthreads();
     const int tid = (int)threadIdx.x;
-    if (tid < BM) src[tid] = tid < rows ? (row_map ? row_map[r0 + tid] : r0 + tid) : -1;
+    if (tid < BM) src[tid] = tid < rows ? r0 + tid : -1;
     __syncthreads();
     float acc[4][4] = {}, acc2[GLU ? 4 : 1][4] = {};
     for (int k0 = 0; k0 < K; k0 += BK) {

@@ -1,232 +1,288 @@
-// hy_gemm.cuh — tcgen05 matrix product of the layered hybrid decoders' prefill path (bf16 operands, fp32 accumulation in
-// tensor memory):  C[t, n] = sum_k X[t, k] W[n, k].
+// hy_gemm.cuh — tcgen05 matrix product of the layered hybrid decoders' prompt steps on pairs of SMs (bf16 operands, fp32
+// accumulation in tensor memory):  C[t, n] = sum_k X[t, k] W[n, k].
 //
-// Swap-AB like the Jacobi engine's GEMMs: the WEIGHT tile is the MMA's A operand (M = 128 output features, so the
-// accumulator's lanes are features and a warp's epilogue stores are contiguous along n), the token rows are the B operand
-// (N = BT tokens, 128 or 256).  Weights are stored in HBM already in the K-major SWIZZLE_128B tile layout (one contiguous
-// 16 KiB tile per 128 features x 64 k: one bulk copy per pipeline stage, no tensor map); the activation tile travels
-// row-major by asynchronous 16-byte copies of four producer warps, each copy to its swizzled place in shared memory.  The
-// copies of all stages but one are in flight at any time; a thread hands a stage over once its own copies have landed.
+// A cluster of two CTAs works on one tile of 256 features x BT tokens: each holds the weight rows of its 128 features and half of the
+// token rows in shared memory, and one thread of the first issues tcgen05.mma.cta_group::2, which reads both halves from both
+// SMs and leaves 128 features in each SM's tensor memory.  An SM so takes in 32 KiB per 64 k for 128 x 256 products instead of
+// 48 KiB; what an SM takes in was what bounded a kernel of 128 x 256 tiles on one SM with its activation rows copied by threads.
+// Both operands travel by TMA: weight tiles lie in HBM in the K-major SWIZZLE_128B layout already (an unswizzled map of 128-byte
+// rows), activation rows are row-major and swizzled on the way in (rows and columns beyond the operand read as zeros).  The kernel
+// is persistent: one cluster per pair of SMs walks the tiles, and the epilogue of a tile runs under the products of the next
+// (two accumulators).
+// Measured cold, TFLOP/s, that kernel -> this one:  N 24576, T 2048, K 2048: 825 -> 1325;  N 2048, T 2048, K 10240: 736 -> 1198;
+// N 37888, T 1000, K 3584: 975 -> 1441 (0.87 of the measured cuBLAS burst);  few tiles (N 1024, T 512, K 6144): 68 -> 43 us.
 //
-// Warps 0-3: activation producers, then the epilogue (TMEM -> registers -> global, through GemmOut).
-// Warp 4:    weight producer (one lane, cp.async.bulk + mbarrier expect_tx).
-// Warp 5:    owns tensor memory; one lane issues tcgen05.mma and commits.
-// Every wait is bounded: on a timeout the kernel raises the error flag, stops waiting and still frees its tensor memory.
+// Warp 0:     producer (one lane in each CTA, seven or nine stages; all bytes of a stage count on the first CTA's mbarrier).
+// Warp 1:     owns tensor memory; in the first CTA one lane issues the products and commits to both CTAs' mbarriers.
+// Warps 2-9:  epilogue (two per quarter of the lanes, one half of the columns each).
+// Every wait is bounded: on a timeout the kernel raises the error flag, stops waiting, lets its copies land and frees its
+// tensor memory.
 #pragma once
+#include <cuda.h>
+
+#include <vector>
+
 #include "hy_kernels.cuh"
 #include "jf_ptx.cuh"
 
 namespace hy {
 
-// Two stages: three blocks of 128 rows (two of 256) share an SM, and their prologues and epilogues run under the other blocks'
-// products; more stages in fewer blocks were slower at every size measured.
-constexpr int TC_STAGES = 2;
-constexpr int TC_WTILE = 128 * 64 * 2;                 // 16 KiB
-constexpr uint32_t TC_SPIN_LIMIT = 1u << 22;           // try_wait probes (each blocks for a bounded time itself)
+constexpr int TC_WTILE = 128 * 64 * 2;                  // 16 KiB
+constexpr uint32_t TC_SPIN_LIMIT = 1u << 22;            // try_wait probes (each blocks for a bounded time itself)
+// as many stages as fit: what few tiles with a long k wait for is the latency of their loads
+__host__ __device__ constexpr int tp_stages(int bt) { return bt == 256 ? 7 : 9; }
+constexpr int TP_MAX_STAGES = 9;
+constexpr int TP_THREADS = 320;
+constexpr int TP_CLUSTERS = 74;                         // pairs of SMs
 
-struct TcSmem {
-  uint64_t full[TC_STAGES], empty[TC_STAGES], acc_full;
+struct TpSmem {
+  uint64_t full[TP_MAX_STAGES], empty[TP_MAX_STAGES], acc_full[2], acc_empty[2];
   uint32_t tmem_base;
   uint32_t failed;
 };
 
-__device__ __forceinline__ bool tc_wait(uint64_t* bar, uint32_t parity, TcSmem* sm, int* err) {
+__device__ __forceinline__ uint32_t tp_rank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
+__device__ __forceinline__ void tp_cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// the address of a shared-memory object of this CTA in the first CTA of the pair
+__device__ __forceinline__ uint32_t tp_in_first(const void* p) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(a) : "r"(jf::smem_u32(p)));
+  return a;
+}
+__device__ __forceinline__ void tp_arrive_cluster(uint32_t bar) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ bool tp_wait(uint64_t* bar, uint32_t parity, TpSmem* sm, int* err) {
   if (sm->failed) return false;
-  for (uint32_t i = 0; i < TC_SPIN_LIMIT; ++i)
-    if (jf::mbar_try_wait(bar, parity)) return true;
+  for (uint32_t i = 0; i < TC_SPIN_LIMIT; ++i) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(jf::smem_u32(bar)), "r"(parity)
+        : "memory");
+    if (ok) return true;
+  }
   sm->failed = 1;
   atomicExch(err, 1);
   return false;
 }
+__device__ __forceinline__ void tp_load(void* dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+  asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+               ::"r"(jf::smem_u32(dst)), "l"(map), "r"(x), "r"(y), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void tp_mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// arrive on the mbarrier at this offset in both CTAs when the products issued so far have completed
+__device__ __forceinline__ void tp_commit(uint64_t* bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+               ::"r"(jf::smem_u32(bar)), "h"((uint16_t)3) : "memory");
+}
 
-// Grouped mode (routed experts): blockIdx.y names a tile of a list; a tile is up to BT consecutive rows [row0, ...) of the
-// expert-sorted order that belong to one expert; its weight tiles start at Wt + expert * w_stride; activation rows are
-// fetched through row_map (NULL: the sorted order itself).  Blocks beyond the list's length leave at once.
-struct TcGroup {
-  const int* meta; const int* offs; const int* tile_expert; const int* tile_row0; const int* row_map; size_t w_stride;
-};
-
+// Epilogue of one warp: the accumulators at taddr (its 32 lanes, `cols` columns, a multiple of 32: two loads in flight) leave
+// through GemmOut.  n: this lane's feature, t0: the token of the first column.
 // GemmOut.act2 == 2 (gated pair): the weight rows alternate 16 gate features and the 16 up features that go with them, so
 // lanes l and l + 16 of an epilogue warp hold one pair; act(gate) * up (act = GemmOut.act_kind) leaves through out1 at
 // feature n / 2.  act2 == 5: the same for the columns of one range, see GemmOut.
+template <typename TO>
+__device__ __forceinline__ void tc_store_columns(const GemmOut& o, uint32_t taddr, int n, int t0, int cols, int T, int N, int lane) {
+  const bool pairs = o.act2 == 2 || (o.act2 == 5 && n - lane >= o.pair_lo && n - lane < o.pair_hi);
+  const int pf = (o.act2 == 5 ? (n - lane - o.pair_lo) >> 1 : (n - lane) >> 1) + lane;      // this lane's feature of a pair
+  const int pn = o.act2 == 5 ? o.pair_n : o.split, pld = o.act2 == 5 ? o.ld_pair : o.ld1;
+  TO* pout = (TO*)(o.act2 == 5 ? o.pair_out : o.out1);
+  // what a column does with its elements is decided once: plain columns only scale and store (the general store's chain of
+  // tests per element cost more than the whole main loop at k = 1024)
+  const bool plain = !pairs && !o.resid && !o.bias && (o.act2 == 0 || o.act2 == 5);
+  const bool adds = o.resid && !o.post_w && !o.next_w && !o.bias;
+  const bool second = n >= o.split, wide = second ? (o.out2_f32 || sizeof(TO) == 4) : sizeof(TO) == 4;
+  const int pitch = second ? o.ld2 : o.ld1;
+  char* dst = second ? (char*)o.out2 + (size_t)(n - o.split) * (wide ? 4 : 2) : (char*)o.out1 + (size_t)n * sizeof(TO);
+  auto store16 = [&](const uint32_t (&v)[16], int c0) {
+    const int rows = min(16, T - t0 - c0);
+    if (adds) {
+      if (n < N) {
+        float* p = o.resid + (size_t)(t0 + c0) * o.ldr + n;
+        float x[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) x[j] = j < rows ? p[(size_t)j * o.ldr] : 0.0f;
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+          if (j < rows) p[(size_t)j * o.ldr] = fmaf(__uint_as_float(v[j]), o.alpha, x[j]);
+      }
+      return;
+    }
+    if (plain) {
+      if (n >= N) {
+      } else if (wide) {
+        float* p = (float*)dst + (size_t)(t0 + c0) * pitch;
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+          if (j < rows) p[(size_t)j * pitch] = __uint_as_float(v[j]) * o.alpha;
+      } else {
+        bf16* p = (bf16*)dst + (size_t)(t0 + c0) * pitch;
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+          if (j < rows) p[(size_t)j * pitch] = __float2bfloat16_rn(__uint_as_float(v[j]) * o.alpha);
+      }
+      return;
+    }
+    if (pairs && o.act_kind == 0) {                      // silu pairs: both halves of the warp work on 8 of the 16 tokens each
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        // lanes < 16 hold gates, the others ups: exchange so that a lane < 16 gets token j's pair and lane + 16 token j + 8's
+        const float give = __uint_as_float(lane < 16 ? v[j + 8] : v[j]);
+        const float got = __shfl_xor_sync(0xffffffffu, give, 16);
+        const float g = lane < 16 ? __uint_as_float(v[j]) : got, up = lane < 16 ? got : __uint_as_float(v[j + 8]);
+        const int row = lane < 16 ? j : j + 8, feat = pf - (lane & 16);
+        if (feat < pn && row < rows) pout[(size_t)(t0 + c0 + row) * pld + feat] = from_f<TO>(silu_f(g) * up);
+      }
+      return;
+    }
+    if (pairs) {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        const float mine = __uint_as_float(v[j]);
+        const float other = __shfl_xor_sync(0xffffffffu, mine, 16);
+        if (lane < 16 && pf < pn && t0 + c0 + j < T)
+          pout[(size_t)(t0 + c0 + j) * pld + pf] = from_f<TO>(gated_pair_f(o.act_kind, mine, other, o.act_limit));
+      }
+      return;
+    }
+    if (n < N) {
+#pragma unroll
+      for (int j = 0; j < 16; ++j)
+        if (t0 + c0 + j < T) gemm_store<TO>(o, t0 + c0 + j, n, __uint_as_float(v[j]));
+    }
+  };
+  for (int c0 = 0; c0 < cols; c0 += 32) {
+    if (t0 + c0 >= T) break;
+    __syncwarp();                                          // the loads from tensor memory are warp-wide
+    uint32_t a[16], b[16];
+    jf::tmem_ld16(taddr + c0, a);
+    jf::tmem_ld16(taddr + c0 + 16, b);
+    jf::tmem_ld_wait();
+    store16(a, c0);
+    if (t0 + c0 + 16 < T) store16(b, c0 + 16);
+  }
+}
+
+// Grouped mode (routed experts): the tiles of a device-made list, each up to BT consecutive rows of the expert-sorted activation
+// rows that belong to one expert; the weight tiles of expert e start e * w_rows map rows further on.  Rows of the next expert
+// that a tile reads along are left out by the epilogue.
+struct TpGroup { const int* meta; const int* offs; const int* tile_expert; const int* tile_row0; int w_rows; };
+
 template <typename TO, int BT>
-__global__ void __launch_bounds__(192) gemm_tc_kernel(const bf16* __restrict__ X, int lda, const bf16* __restrict__ Wt, int T,
-                                                      int N, int K, GemmOut o, int* err, TcGroup grp) {
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TP_THREADS, 1)
+gemm_pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap, int T, int N, int K, GemmOut o, int* err,
+                 TpGroup grp) {
   extern __shared__ __align__(16) unsigned char hy_smem[];
   unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(hy_smem) + 1023) & ~(uintptr_t)1023);
-  constexpr int XTILE = BT * 128;                        // BT rows of 64 bf16
-  constexpr int SLOT = TC_WTILE + XTILE;
-  TcSmem* sm = reinterpret_cast<TcSmem*>(base + TC_STAGES * SLOT);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n0 = blockIdx.x * 128;
-  int t0 = blockIdx.y * BT;
-  if (grp.meta) {
-    if ((int)blockIdx.y >= grp.meta[0]) return;           // the whole block, before any barrier or tensor memory exists
-    const int e = grp.tile_expert[blockIdx.y];
-    t0 = grp.tile_row0[blockIdx.y];
-    T = grp.offs[e + 1];
-    Wt += (size_t)e * grp.w_stride;
-  }
-  const int KT = (K + 63) / 64;
+  constexpr int TP_STAGES = tp_stages(BT), XTILE = BT / 2 * 128, SLOT = TC_WTILE + XTILE;
+  TpSmem* sm = reinterpret_cast<TpSmem*>(base + TP_STAGES * SLOT);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rank = (int)tp_rank();
+  const int KT = (K + 63) / 64, nx = (N + 255) / 256, ny = grp.meta ? grp.meta[0] : (T + BT - 1) / BT;
+  const int tiles = nx * ny, first = blockIdx.x >> 1, step = gridDim.x >> 1;
   if (threadIdx.x == 0) {
-    for (int i = 0; i < TC_STAGES; ++i) { jf::mbar_init(&sm->full[i], 129); jf::mbar_init(&sm->empty[i], 1); }
-    jf::mbar_init(&sm->acc_full, 1);
+    for (int i = 0; i < TP_STAGES; ++i) { jf::mbar_init(&sm->full[i], 1); jf::mbar_init(&sm->empty[i], 1); }
+    for (int i = 0; i < 2; ++i) { jf::mbar_init(&sm->acc_full[i], 1); jf::mbar_init(&sm->acc_empty[i], 16); }
     sm->failed = 0;
     jf::fence_mbar_init();
   }
-  if (warp == 5) jf::tmem_alloc(&sm->tmem_base, BT);
-  jf::tc_fence_before();
-  __syncthreads();
-  jf::tc_fence_after();
-
-  if (warp < 4) {
-    // ---- activation producers ------------------------------------------------------------------------------------
-    int srow[BT / 16];                                    // source row of each of this thread's loads (-1: beyond the rows)
-#pragma unroll
-    for (int u = 0; u < BT / 16; ++u) {
-      const int t = t0 + ((threadIdx.x + u * 128) >> 3);
-      srow[u] = t < T ? (grp.row_map ? grp.row_map[t] : t) : -1;
-    }
-    constexpr int AHEAD = TC_STAGES - 1;                  // stages in flight behind the one that is handed over
-    for (int kt = 0; kt < KT + AHEAD; ++kt) {
-      if (kt < KT) {
-        const int s = kt % TC_STAGES;
-        unsigned char* xt = base + s * SLOT + TC_WTILE;
-        if (!tc_wait(&sm->empty[s], ((kt / TC_STAGES) & 1) ^ 1, sm, err)) break;   // the slot is free: MMAs that read it retired
-#pragma unroll
-        for (int u = 0; u < BT / 16; ++u) {
-          const int i = threadIdx.x + u * 128;
-          const int r = i >> 3, c = i & 7, k = kt * 64 + c * 8;
-          const bool ok = srow[u] >= 0 && k < K;          // rows and columns beyond the operand are zeros
-          jf::cp_async_16(xt + r * 128 + ((c ^ (r & 7)) << 4), ok ? X + (size_t)srow[u] * lda + k : X, ok ? 16u : 0u);
-        }
-      }
-      jf::cp_async_commit();                              // one group per turn, empty ones behind the last stage
-      if (kt >= AHEAD) {
-        jf::cp_async_wait<AHEAD>();                       // this thread's copies of stage kt - AHEAD have landed
-        jf::fence_proxy_async_smem();
-        jf::mbar_arrive(&sm->full[(kt - AHEAD) % TC_STAGES]);
-      }
-    }
-    jf::cp_async_wait_all();
-    // ---- epilogue ----------------------------------------------------------------------------------------------------
-    if (tc_wait(&sm->acc_full, 0, sm, err)) {
-      jf::tc_fence_after();
-      const uint32_t taddr = sm->tmem_base + ((uint32_t)(warp * 32) << 16);
-      const int n = n0 + warp * 32 + lane;
-      const bool pairs = o.act2 == 2 || (o.act2 == 5 && n - lane >= o.pair_lo && n - lane < o.pair_hi);
-      const int pf = (o.act2 == 5 ? (n - lane - o.pair_lo) >> 1 : (n - lane) >> 1) + lane;      // this lane's feature of a pair
-      const int pn = o.act2 == 5 ? o.pair_n : o.split, pld = o.act2 == 5 ? o.ld_pair : o.ld1;
-      TO* pout = (TO*)(o.act2 == 5 ? o.pair_out : o.out1);
-      // what a column does with its elements is decided once: plain columns only scale and store (the general store's chain of
-      // tests per element cost more than the whole main loop at k = 1024)
-      const bool plain = !pairs && !o.resid && !o.bias && (o.act2 == 0 || o.act2 == 5);
-      const bool adds = o.resid && !o.post_w && !o.next_w && !o.bias;
-      const bool second = n >= o.split, wide = second ? (o.out2_f32 || sizeof(TO) == 4) : sizeof(TO) == 4;
-      const int pitch = second ? o.ld2 : o.ld1;
-      char* dst = second ? (char*)o.out2 + (size_t)(n - o.split) * (wide ? 4 : 2) : (char*)o.out1 + (size_t)n * sizeof(TO);
-      for (int c0 = 0; c0 < BT; c0 += 16) {
-        if (t0 + c0 >= T) break;
-        __syncwarp();                                        // the loads from tensor memory are warp-wide
-        uint32_t v[16];
-        jf::tmem_ld16(taddr + c0, v);
-        jf::tmem_ld_wait();
-        const int rows = min(16, T - t0 - c0);
-        if (adds) {
-          if (n < N) {
-            float* p = o.resid + (size_t)(t0 + c0) * o.ldr + n;
-            float x[16];
-#pragma unroll
-            for (int j = 0; j < 16; ++j) x[j] = j < rows ? p[(size_t)j * o.ldr] : 0.0f;
-#pragma unroll
-            for (int j = 0; j < 16; ++j)
-              if (j < rows) p[(size_t)j * o.ldr] = fmaf(__uint_as_float(v[j]), o.alpha, x[j]);
-          }
-          continue;
-        }
-        if (plain) {
-          if (n >= N) {
-          } else if (wide) {
-            float* p = (float*)dst + (size_t)(t0 + c0) * pitch;
-#pragma unroll
-            for (int j = 0; j < 16; ++j)
-              if (j < rows) p[(size_t)j * pitch] = __uint_as_float(v[j]) * o.alpha;
-          } else {
-            bf16* p = (bf16*)dst + (size_t)(t0 + c0) * pitch;
-#pragma unroll
-            for (int j = 0; j < 16; ++j)
-              if (j < rows) p[(size_t)j * pitch] = __float2bfloat16_rn(__uint_as_float(v[j]) * o.alpha);
-          }
-          continue;
-        }
-        if (pairs && o.act_kind == 0) {                      // silu pairs: both halves of the warp work on 8 of the 16 tokens each
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            // lanes < 16 hold gates, the others ups: exchange so that a lane < 16 gets token j's pair and lane + 16 token j + 8's
-            const float give = __uint_as_float(lane < 16 ? v[j + 8] : v[j]);
-            const float got = __shfl_xor_sync(0xffffffffu, give, 16);
-            const float g = lane < 16 ? __uint_as_float(v[j]) : got, up = lane < 16 ? got : __uint_as_float(v[j + 8]);
-            const int row = lane < 16 ? j : j + 8, feat = pf - (lane & 16);
-            if (feat < pn && row < rows) pout[(size_t)(t0 + c0 + row) * pld + feat] = from_f<TO>(silu_f(g) * up);
-          }
-          continue;
-        }
-        if (pairs) {
-#pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            const float mine = __uint_as_float(v[j]);
-            const float other = __shfl_xor_sync(0xffffffffu, mine, 16);
-            if (lane < 16 && pf < pn && t0 + c0 + j < T)
-              pout[(size_t)(t0 + c0 + j) * pld + pf] = from_f<TO>(gated_pair_f(o.act_kind, mine, other, o.act_limit));
-          }
-          continue;
-        }
-        if (n < N) {
-#pragma unroll
-          for (int j = 0; j < 16; ++j)
-            if (t0 + c0 + j < T) gemm_store<TO>(o, t0 + c0 + j, n, __uint_as_float(v[j]));
-        }
-      }
-    }
-  } else if (warp == 4) {
-    // ---- weight producer -----------------------------------------------------------------------------------------------
-    if (lane == 0) {
-      const unsigned char* wsrc = reinterpret_cast<const unsigned char*>(Wt) + (size_t)blockIdx.x * KT * TC_WTILE;
-      for (int kt = 0; kt < KT; ++kt) {
-        const int s = kt % TC_STAGES;
-        if (!tc_wait(&sm->empty[s], ((kt / TC_STAGES) & 1) ^ 1, sm, err)) break;
-        jf::mbar_expect_tx(&sm->full[s], TC_WTILE);
-        jf::bulk_g2s(base + s * SLOT, wsrc + (size_t)kt * TC_WTILE, TC_WTILE, &sm->full[s]);
-      }
-    }
-  } else {
-    // ---- MMA issuer -----------------------------------------------------------------------------------------------------
-    if (lane == 0) {
-      const uint32_t idesc = jf::umma_idesc_bf16(128, BT);
-      const uint32_t d0 = sm->tmem_base;
-      bool ok = true;
-      for (int kt = 0; kt < KT && ok; ++kt) {
-        const int s = kt % TC_STAGES;
-        ok = tc_wait(&sm->full[s], (kt / TC_STAGES) & 1, sm, err);
-        if (!ok) break;
-        jf::tc_fence_after();
-        const uint32_t sa = jf::smem_u32(base + s * SLOT);
-        const uint32_t sb = sa + TC_WTILE;
-#pragma unroll
-        for (int kk = 0; kk < 4; ++kk)
-          jf::umma_bf16(d0, jf::umma_desc_sw128(sa + kk * 32), jf::umma_desc_sw128(sb + kk * 32), idesc, (kt > 0 || kk > 0) ? 1u : 0u);
-        jf::umma_commit(&sm->empty[s]);
-      }
-      if (ok) jf::umma_commit(&sm->acc_full);
-    }
-    __syncwarp();
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(jf::smem_u32(&sm->tmem_base)), "r"((uint32_t)(2 * BT)) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
   jf::tc_fence_before();
   __syncthreads();
-  if (warp == 5) jf::tmem_dealloc(sm->tmem_base, BT);
+  tp_cluster_sync();
+  jf::tc_fence_after();
+  // token tile and feature tile of a tile number: neighbours share the weight rows (grouped: the expert's activation rows)
+  auto place = [&](int tile, int& x, int& y) {
+    if (grp.meta) { x = tile % nx; y = tile / nx; }
+    else { x = tile / ny; y = tile % ny; }
+  };
+
+  if (warp == 0) {
+    if (lane == 0) {
+      int it = 0;
+      bool ok = true;
+      for (int tile = first; tile < tiles && ok; tile += step) {
+        int x, y;
+        place(tile, x, y);
+        const int t0 = (grp.meta ? grp.tile_row0[y] : y * BT) + rank * (BT / 2);
+        const int w0 = (grp.meta ? grp.tile_expert[y] * grp.w_rows : 0) + (2 * x + rank) * KT * 128;
+        for (int kt = 0; kt < KT; ++kt, ++it) {
+          const int s = it % TP_STAGES;
+          ok = tp_wait(&sm->empty[s], ((it / TP_STAGES) & 1) ^ 1, sm, err);      // the products that read the slot retired
+          if (!ok) break;
+          if (rank == 0) jf::mbar_expect_tx(&sm->full[s], 2 * SLOT);
+          const uint32_t bar = tp_in_first(&sm->full[s]);
+          tp_load(base + s * SLOT, &wmap, 0, w0 + kt * 128, bar);
+          tp_load(base + s * SLOT + TC_WTILE, &xmap, kt * 64, t0, bar);
+        }
+      }
+      if (!ok) for (int i = 0; i < 1000; ++i) __nanosleep(1000);    // copies in flight land before the block leaves
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    if (lane == 0 && rank == 0) {
+      const uint32_t idesc = jf::umma_idesc_bf16(256, BT);
+      int it = 0, i = 0;
+      bool ok = true;
+      for (int tile = first; tile < tiles && ok; tile += step, ++i) {
+        const uint32_t d = sm->tmem_base + (i & 1) * BT;
+        ok = tp_wait(&sm->acc_empty[i & 1], ((i >> 1) & 1) ^ 1, sm, err);        // both CTAs have read it
+        jf::tc_fence_after();
+        for (int kt = 0; kt < KT && ok; ++kt, ++it) {
+          const int s = it % TP_STAGES;
+          ok = tp_wait(&sm->full[s], (it / TP_STAGES) & 1, sm, err);
+          if (!ok) break;
+          jf::tc_fence_after();
+          const uint32_t sa = jf::smem_u32(base + s * SLOT), sb = sa + TC_WTILE;
+#pragma unroll
+          for (int kk = 0; kk < 4; ++kk)
+            tp_mma(d, jf::umma_desc_sw128(sa + kk * 32), jf::umma_desc_sw128(sb + kk * 32), idesc, (kt > 0 || kk > 0) ? 1u : 0u);
+          tp_commit(&sm->empty[s]);
+        }
+        if (ok) tp_commit(&sm->acc_full[i & 1]);
+      }
+    }
+    __syncwarp();
+  } else {
+    const int q = warp & 3, half = (warp - 2) >> 2;                 // quarter of the lanes that this warp may read, half of the columns
+    int i = 0;
+    for (int tile = first; tile < tiles; tile += step, ++i) {
+      int x, y;
+      place(tile, x, y);
+      if (!tp_wait(&sm->acc_full[i & 1], (i >> 1) & 1, sm, err)) break;
+      jf::tc_fence_after();
+      const int t0 = (grp.meta ? grp.tile_row0[y] : y * BT) + half * (BT / 2);
+      const int rows = grp.meta ? grp.offs[grp.tile_expert[y] + 1] : T;
+      tc_store_columns<TO>(o, sm->tmem_base + (i & 1) * BT + half * (BT / 2) + ((uint32_t)(q * 32) << 16), x * 256 + rank * 128 + q * 32 + lane, t0,
+                           BT / 2, rows, N, lane);
+      jf::tc_fence_before();
+      __syncwarp();
+      if (lane == 0) tp_arrive_cluster(tp_in_first(&sm->acc_empty[i & 1]));
+    }
+  }
+  jf::tc_fence_before();
+  __syncthreads();
+  tp_cluster_sync();                                                // nothing of the pair still reads or signals this CTA
+  if (warp == 1)
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(sm->tmem_base), "r"((uint32_t)(2 * BT)) : "memory");
 }
 
-constexpr size_t tc_smem_bytes(int bt) { return (size_t)TC_STAGES * (TC_WTILE + bt * 128) + sizeof(TcSmem) + 1024; }
+constexpr size_t tp_smem_bytes(int bt) { return (size_t)tp_stages(bt) * (TC_WTILE + bt / 2 * 128) + sizeof(TpSmem) + 1024; }
 
 // Host-side packer: row-major [N, K] floats -> bf16 tiles [ceil(N/128)][ceil(K/64)] of 128 x 64 in the swizzled layout.
 inline void pack_tiles(const float* w, int N, int K, std::vector<uint16_t>& out) {
@@ -241,6 +297,29 @@ inline void pack_tiles(const float* w, int N, int K, std::vector<uint16_t>& out)
       memcpy(&bits, &b, 2);
       out[tile * 8192 + off / 2] = bits;
     }
+}
+
+// ---- host: tensor maps ------------------------------------------------------------------------------------------------------------
+typedef CUresult (*TpEncode)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
+                             const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+inline TpEncode tp_encode() {
+  static const TpEncode f = [] {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult r;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &r) != cudaSuccess || r != cudaDriverEntryPointSuccess) p = nullptr;
+    return (TpEncode)p;
+  }();
+  return f;
+}
+// rows x cols bf16 elements, `ld` elements from row to row, in boxes of box_rows x 64
+inline bool tp_map(CUtensorMap* m, const void* p, uint64_t rows, uint64_t cols, uint64_t ld, int box_rows, bool swizzle) {
+  const TpEncode f = tp_encode();
+  if (!f) return false;
+  const cuuint64_t dims[2] = {cols, rows}, strides[1] = {ld * 2};
+  const cuuint32_t box[2] = {64, (cuuint32_t)box_rows}, one[2] = {1, 1};
+  return f(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(p), dims, strides, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
+           swizzle ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 }  // namespace hy
