@@ -94,86 +94,107 @@ __device__ __forceinline__ void tp_commit(uint64_t* bar) {
 // GemmOut.act2 == 2 (gated pair): the weight rows alternate 16 gate features and the 16 up features that go with them, so
 // lanes l and l + 16 of an epilogue warp hold one pair; act(gate) * up (act = GemmOut.act_kind) leaves through out1 at
 // feature n / 2.  act2 == 5: the same for the columns of one range, see GemmOut.
+// What a column does with its elements, and its parameters, are decided and read once per tile: gemm_store's chain of tests and loads
+// per element took longer than the products of the next tile (N 20992, T 2048, K 2048 with the squared ReLU: 409 us against 118).
 template <typename TO>
 __device__ __forceinline__ void tc_store_columns(const GemmOut& o, uint32_t taddr, int n, int t0, int cols, int T, int N, int lane) {
   const bool pairs = o.act2 == 2 || (o.act2 == 5 && n - lane >= o.pair_lo && n - lane < o.pair_hi);
-  const int pf = (o.act2 == 5 ? (n - lane - o.pair_lo) >> 1 : (n - lane) >> 1) + lane;      // this lane's feature of a pair
-  const int pn = o.act2 == 5 ? o.pair_n : o.split, pld = o.act2 == 5 ? o.ld_pair : o.ld1;
-  TO* pout = (TO*)(o.act2 == 5 ? o.pair_out : o.out1);
-  // what a column does with its elements is decided once: plain columns only scale and store (the general store's chain of
-  // tests per element cost more than the whole main loop at k = 1024)
-  const bool plain = !pairs && !o.resid && !o.bias && (o.act2 == 0 || o.act2 == 5);
-  const bool adds = o.resid && !o.post_w && !o.next_w && !o.bias;
-  const bool second = n >= o.split, wide = second ? (o.out2_f32 || sizeof(TO) == 4) : sizeof(TO) == 4;
-  const int pitch = second ? o.ld2 : o.ld1;
-  char* dst = second ? (char*)o.out2 + (size_t)(n - o.split) * (wide ? 4 : 2) : (char*)o.out1 + (size_t)n * sizeof(TO);
-  auto store16 = [&](const uint32_t (&v)[16], int c0) {
-    const int rows = min(16, T - t0 - c0);
-    if (adds) {
-      if (n < N) {
-        float* p = o.resid + (size_t)(t0 + c0) * o.ldr + n;
-        float x[16];
-#pragma unroll
-        for (int j = 0; j < 16; ++j) x[j] = j < rows ? p[(size_t)j * o.ldr] : 0.0f;
-#pragma unroll
-        for (int j = 0; j < 16; ++j)
-          if (j < rows) p[(size_t)j * o.ldr] = fmaf(__uint_as_float(v[j]), o.alpha, x[j]);
-      }
-      return;
-    }
-    if (plain) {
-      if (n >= N) {
-      } else if (wide) {
-        float* p = (float*)dst + (size_t)(t0 + c0) * pitch;
-#pragma unroll
-        for (int j = 0; j < 16; ++j)
-          if (j < rows) p[(size_t)j * pitch] = __uint_as_float(v[j]) * o.alpha;
-      } else {
-        bf16* p = (bf16*)dst + (size_t)(t0 + c0) * pitch;
-#pragma unroll
-        for (int j = 0; j < 16; ++j)
-          if (j < rows) p[(size_t)j * pitch] = __float2bfloat16_rn(__uint_as_float(v[j]) * o.alpha);
-      }
-      return;
-    }
-    if (pairs && o.act_kind == 0) {                      // silu pairs: both halves of the warp work on 8 of the 16 tokens each
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        // lanes < 16 hold gates, the others ups: exchange so that a lane < 16 gets token j's pair and lane + 16 token j + 8's
-        const float give = __uint_as_float(lane < 16 ? v[j + 8] : v[j]);
-        const float got = __shfl_xor_sync(0xffffffffu, give, 16);
-        const float g = lane < 16 ? __uint_as_float(v[j]) : got, up = lane < 16 ? got : __uint_as_float(v[j + 8]);
-        const int row = lane < 16 ? j : j + 8, feat = pf - (lane & 16);
-        if (feat < pn && row < rows) pout[(size_t)(t0 + c0 + row) * pld + feat] = from_f<TO>(silu_f(g) * up);
-      }
-      return;
-    }
-    if (pairs) {
-#pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        const float mine = __uint_as_float(v[j]);
-        const float other = __shfl_xor_sync(0xffffffffu, mine, 16);
-        if (lane < 16 && pf < pn && t0 + c0 + j < T)
-          pout[(size_t)(t0 + c0 + j) * pld + pf] = from_f<TO>(gated_pair_f(o.act_kind, mine, other, o.act_limit));
-      }
-      return;
-    }
-    if (n < N) {
-#pragma unroll
-      for (int j = 0; j < 16; ++j)
-        if (t0 + c0 + j < T) gemm_store<TO>(o, t0 + c0 + j, n, __uint_as_float(v[j]));
+  const bool second = n >= o.split, wide = second ? (o.out2_f32 || sizeof(TO) == 4) : sizeof(TO) == 4, in = n < N;
+  const float bias = o.bias && in ? o.bias[n] : 0.0f;
+  // one pass over the columns with what to do with sixteen of them (rows: how many exist) given as a function
+  auto each = [&](auto store16) {
+    for (int c0 = 0; c0 < cols; c0 += 32) {
+      if (t0 + c0 >= T) break;
+      __syncwarp();                                        // the loads from tensor memory are warp-wide
+      uint32_t a[16], b[16];
+      jf::tmem_ld16(taddr + c0, a);
+      jf::tmem_ld16(taddr + c0 + 16, b);
+      jf::tmem_ld_wait();
+      store16(a, t0 + c0, min(16, T - t0 - c0));
+      if (t0 + c0 + 16 < T) store16(b, t0 + c0 + 16, min(16, T - t0 - c0 - 16));
     }
   };
-  for (int c0 = 0; c0 < cols; c0 += 32) {
-    if (t0 + c0 >= T) break;
-    __syncwarp();                                          // the loads from tensor memory are warp-wide
-    uint32_t a[16], b[16];
-    jf::tmem_ld16(taddr + c0, a);
-    jf::tmem_ld16(taddr + c0 + 16, b);
-    jf::tmem_ld_wait();
-    store16(a, c0);
-    if (t0 + c0 + 16 < T) store16(b, c0 + 16);
+  if (pairs) {
+    const int pf = (o.act2 == 5 ? (n - lane - o.pair_lo) >> 1 : (n - lane) >> 1) + (lane & 15);      // this lane's feature of a pair
+    const int pn = o.act2 == 5 ? o.pair_n : o.split, pld = o.act2 == 5 ? o.ld_pair : o.ld1;
+    TO* pout = (TO*)(o.act2 == 5 ? o.pair_out : o.out1) + pf;
+    const bool low = lane < 16, live = pf < pn;
+    auto go = [&](auto pair) {
+      each([&](const uint32_t (&v)[16], int t, int rows) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          // lanes < 16 hold gates, the others ups: exchange so that a lane < 16 gets token j's pair and lane + 16 token j + 8's
+          const float give = __uint_as_float(low ? v[j + 8] : v[j]);
+          const float got = __shfl_xor_sync(0xffffffffu, give, 16);
+          const float g = low ? __uint_as_float(v[j]) : got, up = low ? got : __uint_as_float(v[j + 8]);
+          const int row = low ? j : j + 8;
+          if (live && row < rows) pout[(size_t)(t + row) * pld] = from_f<TO>(pair(g, up));
+        }
+      });
+    };
+    if (o.act_kind == 0) go([](float g, float u) { return silu_f(g) * u; });
+    else if (o.act_kind == 1) go([](float g, float u) { return gelu_tanh_f(g) * u; });
+    else go([&](float g, float u) { return gated_pair_f(o.act_kind, g, u, o.act_limit); });
+    return;
   }
+  if (o.resid) {
+    float* col = o.resid + n;
+    const size_t ld = (size_t)o.ldr;
+    const bool post = o.post_w != nullptr, next = o.next_w != nullptr;
+    const float pw = post && in ? o.post_w[n] : 0.0f, pb = post && in ? o.post_b[n] : 0.0f, pl = post && in ? o.post_ls[n] : 0.0f;
+    const float nw = next && in ? o.next_w[n] : 0.0f, nb = next && in ? o.next_b[n] : 0.0f;
+    auto go = [&](auto sublayer, auto leave) {
+      each([&](const uint32_t (&v)[16], int t, int rows) {
+        if (!in) return;
+        float* p = col + t * ld;
+        float x[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) x[j] = j < rows ? p[j * ld] : 0.0f;
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          if (j >= rows) continue;
+          const float y = x[j] + sublayer(__uint_as_float(v[j]) * o.alpha + bias);
+          p[j * ld] = y;
+          leave((t + j) * ld + n, y);
+        }
+      });
+    };
+    auto plain = [](float c) { return c; };
+    auto normed = [&](float c) { return pl * fmaf(tanhf(o.post_alpha * c), pw, pb); };
+    auto nothing = [](size_t, float) {};
+    auto half = [&](size_t at, float y) { ((bf16*)o.next_out)[at] = __float2bfloat16_rn(fmaf(tanhf(o.next_alpha * y), nw, nb)); };
+    auto full = [&](size_t at, float y) { ((float*)o.next_out)[at] = fmaf(tanhf(o.next_alpha * y), nw, nb); };
+    if (!post && !next) go(plain, nothing);
+    else if (post && !next) go(normed, nothing);
+    else if (post && !o.next_f32) go(normed, half);
+    else if (post) go(normed, full);
+    else if (!o.next_f32) go(plain, half);
+    else go(plain, full);
+    return;
+  }
+  const int pitch = second ? o.ld2 : o.ld1;
+  char* dst = second ? (char*)o.out2 + (size_t)(n - o.split) * (wide ? 4 : 2) : (char*)o.out1 + (size_t)n * sizeof(TO);
+  auto go = [&](auto value) {
+    each([&](const uint32_t (&v)[16], int t, int rows) {
+      if (!in) return;
+      if (wide) {
+        float* p = (float*)dst + (size_t)t * pitch;
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+          if (j < rows) p[(size_t)j * pitch] = value(__uint_as_float(v[j]) * o.alpha + bias);
+      } else {
+        bf16* p = (bf16*)dst + (size_t)t * pitch;
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+          if (j < rows) p[(size_t)j * pitch] = __float2bfloat16_rn(value(__uint_as_float(v[j]) * o.alpha + bias));
+      }
+    });
+  };
+  const bool square = o.act2 == 1 && second;
+  if (o.act2 == 1) go([&](float c) { const float r = fmaxf(c, 0.0f); return square ? r * r : c; });
+  else if (o.act2 == 3) go([&](float c) { return act_f(o.act_kind, c); });
+  else if (o.act2 == 4) go([&](float c) { return expf(o.act_limit * log_sigmoid_f(c)); });
+  else go([](float c) { return c; });
 }
 
 // Grouped mode (routed experts): the tiles of a device-made list, each up to BT consecutive rows of the expert-sorted activation
