@@ -28,6 +28,7 @@ __global__ void __launch_bounds__(128) attn_mma_kernel(Batch b, const AttnUnit* 
                                                        int ldq, const bf16* __restrict__ cache, int H, int G, float scale,
                                                        float qt_coef, int qt_every, int window, int split_keys, int n_splits, int vdim,
                                                        float* __restrict__ part_o, float* __restrict__ part_ml) {
+  pdl_begin();
   constexpr int LD = DIM + 8;                           // padded row (elements): ldmatrix rows fall into distinct banks
   __shared__ __align__(16) bf16 qs[64 * LD];
   __shared__ __align__(16) bf16 ks[64 * LD];
@@ -202,6 +203,7 @@ __global__ void __launch_bounds__(256, 1) attn_wide_kernel(Batch b, const AttnUn
                                                            int ldq, const bf16* __restrict__ cache, int H, int dk, int vdim,
                                                            float scale, int window, int split_keys, int n_splits, int pstride,
                                                            float* __restrict__ part_o, float* __restrict__ part_ml) {
+  pdl_begin();
   extern __shared__ __align__(16) unsigned char hy_smem[];
   const int dkp = (dk + 15) & ~15, LD = dkp + 8;          // padded row (elements): ldmatrix rows fall into distinct banks
   constexpr int LDP = 64 + 8;
@@ -438,6 +440,7 @@ template <typename WT, typename OT>
 __global__ void attn_combine_kernel(Batch b, const float* __restrict__ part_o, const float* __restrict__ part_ml,
                                     const WT* __restrict__ sink, const bf16* __restrict__ gate, int ldg, int H, int G, int dim,
                                     int vdim, int window, int split_keys, int n_splits, float out_scale, OT* __restrict__ out, int ldo) {
+  pdl_begin();
   const int t = blockIdx.x / H, h = blockIdx.x % H;
   int from = 0, live = b.tok_pos[t] / split_keys + 1;      // splits that hold a key this row may see
   if (window > 0) {

@@ -42,6 +42,7 @@ template <typename WT>
 __global__ void embed_pair_kernel(Batch b, const WT* __restrict__ table, float scale, const WT* __restrict__ pair, int buckets,
                                   int mul_prev, int mul_cur, const int* __restrict__ prev_tok, int width, float* __restrict__ x,
                                   float* __restrict__ kept) {
+  pdl_begin();
   const int t = blockIdx.x;
   const int tok = b.tok[t], e = b.tok_ent[t];
   long long row = -1;
@@ -65,6 +66,7 @@ __global__ void embed_pair_kernel(Batch b, const WT* __restrict__ table, float s
 
 // after embed_pair_kernel of the same step: the request's last token of this step
 __global__ void prev_token_kernel(Batch b, int* __restrict__ prev_tok) {
+  pdl_begin();
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e < b.E) prev_tok[b.ent_slot[e]] = b.tok[b.ent_start[e + 1] - 1];
 }
@@ -83,6 +85,7 @@ struct StreamOp {
 
 template <typename WT>
 __global__ void __launch_bounds__(256) stream_row_kernel(Batch b, StreamOp o, int width, float* __restrict__ x) {
+  pdl_begin();
   extern __shared__ __align__(16) unsigned char hy_smem[];
   float* xs = reinterpret_cast<float*>(hy_smem);             // [width] the row
   float* ys = xs + width;                                    // [width] the token input's row
@@ -199,6 +202,7 @@ __global__ void __launch_bounds__(256) stream_row_kernel(Batch b, StreamOp o, in
 template <typename AT, int CH>
 __global__ void canon_kernel(Batch b, const float* __restrict__ hn, int width, int taps, const float* __restrict__ w,
                              const float* __restrict__ state, AT* __restrict__ out) {
+  pdl_begin();
   struct alignas(4 * CH) Row { float v[CH]; };                        // CH consecutive channels per thread (width % CH == 0)
   const int t = blockIdx.y;
   const int c = (blockIdx.x * blockDim.x + threadIdx.x) * CH;
@@ -231,6 +235,7 @@ __global__ void __launch_bounds__(128) biased_prep_kernel(Batch b, AT* __restric
                                                           int G, int dim, int vdim, const float* __restrict__ qn,
                                                           const float* __restrict__ kn, float eps, int mix, float lambda,
                                                           AT* __restrict__ vfirst, int ldvf, AT* __restrict__ kc, AT* __restrict__ vc) {
+  pdl_begin();
   __shared__ float red[66];
   const int t = blockIdx.x;
   const int e = b.tok_ent[t], pos = b.tok_pos[t];
@@ -267,6 +272,7 @@ template <typename AT, typename OT>
 __global__ void __launch_bounds__(128) biased_attn_kernel(Batch b, const AT* __restrict__ q, int ldq, BiasedCfg c,
                                                           const AT* __restrict__ kc, const AT* __restrict__ vc,
                                                           OT* __restrict__ out, int ldo) {
+  pdl_begin();
   extern __shared__ __align__(16) unsigned char hy_smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float* qs = reinterpret_cast<float*>(hy_smem) + warp * c.dim;
@@ -342,6 +348,7 @@ __global__ void __launch_bounds__(128) biased_mma_kernel(Batch b, const AttnUnit
                                                          int ldq, BiasedCfg c, const bf16* __restrict__ kc,
                                                          const bf16* __restrict__ vc, bf16* __restrict__ out, int ldo,
                                                          int n_splits, float* __restrict__ part_o, float* __restrict__ part_ml) {
+  pdl_begin();
   constexpr int LD = DP + 8;                            // padded row (elements): ldmatrix rows fall into distinct banks
   extern __shared__ __align__(16) unsigned char hy_smem[];
   bf16* kbuf = reinterpret_cast<bf16*>(hy_smem);        // [2][64 * LD] key tiles: one in use, one in flight
@@ -582,6 +589,7 @@ __global__ void __launch_bounds__(128) biased_mma_kernel(Batch b, const AttnUnit
 template <typename OT>
 __global__ void biased_combine_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml, BiasedCfg c,
                                       int pstride, int n_splits, OT* __restrict__ out, int ldo) {
+  pdl_begin();
   const int H = c.H, vdim = c.vdim;
   const int t = blockIdx.x / H, h = blockIdx.x % H;
   const size_t slot0 = ((size_t)t * H + h) * n_splits;

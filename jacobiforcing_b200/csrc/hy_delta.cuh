@@ -25,6 +25,7 @@ namespace hy {
 struct RotTable { const double* freq; int pairs; float mag; float* out; int ld; };
 
 __global__ void rot_tables_kernel(Batch b, const RotTable* __restrict__ tables) {
+  pdl_begin();
   const RotTable r = tables[blockIdx.y];
   const int t = blockIdx.x;
   const double pos = (double)b.tok_pos[t];
@@ -55,6 +56,7 @@ template <typename AT>
 __global__ void __launch_bounds__(128) key_value_prep_kernel(Batch b, AT* __restrict__ in, int ld, int col_q, int col_k, int H, int G, int dim,
                                                              const float* __restrict__ cs, int ldc, RotPair r, AT* __restrict__ kc,
                                                              AT* __restrict__ vc) {
+  pdl_begin();
   const int t = blockIdx.x;
   const int e = b.tok_ent[t], pos = b.tok_pos[t];
   const int page = b.pages[(size_t)e * b.max_pages + pos / b.page_size], in_page = pos % b.page_size;
@@ -82,6 +84,7 @@ __global__ void __launch_bounds__(128) key_value_prep_kernel(Batch b, AT* __rest
 template <typename AT>
 __global__ void __launch_bounds__(1024) linear_rows_kernel(const AT* __restrict__ in, int ld, int col_q, int col_k, int H, int dim,
                                                           const float* __restrict__ cs, int ldc, RotPair rp, float* __restrict__ qk) {
+  pdl_begin();
   const int t = blockIdx.x;
   const AT* row = in + (size_t)t * ld;
   const float* c = rp.pairs > 0 ? cs + (size_t)t * ldc : nullptr;
@@ -112,6 +115,7 @@ __global__ void __launch_bounds__(128) delta_unit_kernel(int T, int H, int G, in
                                                          const float* __restrict__ A_log, const float* __restrict__ dt_bias,
                                                          const AT* __restrict__ beta, int ldb, float* __restrict__ dec, int ldd,
                                                          float* __restrict__ qk, float4* __restrict__ sc) {
+  pdl_begin();
   const int unit = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31, R = H / G;
   if (unit >= T * G) return;
   const size_t t = unit / G;
@@ -187,8 +191,8 @@ template <typename AT, int DR, int PARTS, bool CHAN = false>
 __global__ void __launch_bounds__(128) delta_head_kernel(Batch b, const float* __restrict__ qk, const AT* __restrict__ v, int ldv,
                                                          const float4* __restrict__ scal, int H, int G, int dim, int vdim,
                                                          int blocks_per_head, int vec, int vvec, float* __restrict__ state,
-                                                         float* __restrict__ o, int ldo, const float* __restrict__ dec = nullptr,
-                                                         int ldd = 0) {
+                                                         float* __restrict__ o, int ldo, const float* __restrict__ dec, int ldd) {
+  pdl_begin();
   constexpr int TB = lin_tb(DR), RP = DR / PARTS, CW = 32 / PARTS, CPB = lin_cpb(PARTS), VW = CPB < 8 ? 8 : CPB;
   constexpr int RW = CHAN ? 3 * DR : 2 * DR;                   // floats of a staged row: q | k (| decays)
   extern __shared__ __align__(16) unsigned char hy_smem[];

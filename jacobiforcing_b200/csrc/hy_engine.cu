@@ -10,6 +10,7 @@
 
 #include <algorithm>
 #include <type_traits>
+#include <utility>
 #include <map>
 #include <set>
 #include <string>
@@ -157,6 +158,7 @@ struct hy_engine {
   // tensor-core attention: work units of the step (per head layout), partial results per (row, key split)
   AttnUnit* units_d = nullptr; AttnUnit* units_h = nullptr; size_t units_cap = 0, units_used = 0;
   std::vector<UnitList> unit_lists;
+  int step_tokens = 0;
   // cosines and sines of the step's positions, one table per distinct rotation: the layer configuration that names it, the table,
   // its column count; rot_tables_d is what the kernel reads
   struct RotEntry { hy_layer_cfg c; RotTable t; };
@@ -174,6 +176,23 @@ struct hy_engine {
       return HY_ERR_CUDA;                                                                               \
     }                                                                                                   \
   } while (0)
+
+// Launch of a kernel of a step.  In steps of few tokens it may start once every block of the kernel before it has started (see
+// pdl_wait), so that its own start, its barriers and its first weights overlap the end of that kernel: a Kinetar decode step is 42
+// kernels of 2 to 9 us each (request of 512 + 24 tokens: 10.66 -> 9.47 ms).  Prompt steps keep plain launches: the blocks of a
+// kernel that starts under another one's tail pile up on the SMs that are free already, and a recurrence with one block per
+// SM then runs two or three on some of them (two Kinetar layers, 2048 tokens: 2.02 ms plain, 2.35 ms overlapped).
+constexpr int HY_OVERLAP_TOKENS = 64;
+template <typename... P, typename... A>
+inline void go_kernel(const hy_engine* h, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c = {};
+  c.gridDim = grid; c.blockDim = block; c.dynamicSmemBytes = smem; c.stream = stream; c.attrs = &at;
+  c.numAttrs = h->step_tokens <= HY_OVERLAP_TOKENS ? 1 : 0;
+  cudaLaunchKernelEx(&c, kernel, std::forward<A>(args)...);
+}
 
 struct ProfScope {
   hy_engine* h; int cat; cudaEvent_t a{}, b{};
@@ -1441,8 +1460,8 @@ int pair_product(hy_engine* h, const bf16* X, int lda, int x_rows, const void* t
   grp.w_rows = (int)(w_stride / 64);
   const long long most = (long long)nx * (grp.meta ? x_rows / bt + groups : (T + bt - 1) / bt);      // tiles (grouped: at most)
   const int grid = 2 * (int)std::min<long long>(most, TP_CLUSTERS);
-  if (bt == 128) gemm_pair_kernel<TO, 128><<<grid, TP_THREADS, tp_smem_bytes(128), h->stream>>>(xm, wm, T, N, K, o, h->err_d, grp);
-  else gemm_pair_kernel<TO, 256><<<grid, TP_THREADS, tp_smem_bytes(256), h->stream>>>(xm, wm, T, N, K, o, h->err_d, grp);
+  if (bt == 128) go_kernel(h, gemm_pair_kernel<TO, 128>, grid, TP_THREADS, tp_smem_bytes(128), h->stream, xm, wm, T, N, K, o, h->err_d, grp);
+  else go_kernel(h, gemm_pair_kernel<TO, 256>, grid, TP_THREADS, tp_smem_bytes(256), h->stream, xm, wm, T, N, K, o, h->err_d, grp);
   h->launches++;
   return HY_OK;
 }
@@ -1476,14 +1495,14 @@ int gemm(hy_engine* h, const TA* A, int lda, const TW* Wt, int ldw, int T, int N
     }
     auto launch = [&](auto kern, int rows) {
       const size_t smem = (size_t)rows * row_bytes;
-      kern<<<dim3(blocks, (T + rows - 1) / rows), 256, smem, h->stream>>>(A, lda, Wt, ldw, T, N, K, ksplit, o);
+      go_kernel(h, kern, dim3(blocks, (T + rows - 1) / rows), 256, smem, h->stream, A, lda, Wt, ldw, T, N, K, ksplit, o);
     };
     if (T == 1 || fit < 2) launch(gemm_rows_kernel<TA, TW, TO, 1>, 1);
     else if (T == 2 || fit < 4) launch(gemm_rows_kernel<TA, TW, TO, 2>, 2);
     else if (T <= 4 || fit < 8) launch(gemm_rows_kernel<TA, TW, TO, 4>, 4);
     else launch(gemm_rows_kernel<TA, TW, TO, 8>, 8);
   } else {
-    gemm_simt_kernel<TA, TW, TO><<<dim3((N + 63) / 64, (T + 63) / 64), 256, 0, h->stream>>>(A, lda, Wt, ldw, T, N, K, o);
+    go_kernel(h, gemm_simt_kernel<TA, TW, TO>, dim3((N + 63) / 64, (T + 63) / 64), 256, 0, h->stream, A, lda, Wt, ldw, T, N, K, o);
   }
   h->launches++;
   return HY_OK;
@@ -1611,7 +1630,7 @@ void launch_conv(hy_engine* h, const Batch& b, const AT* u, int ldu, int col0, i
   auto go = [&](auto v, auto tp) {
     constexpr int V = decltype(v)::value, TP = decltype(tp)::value;
     const int per = 128 * V;
-    conv_kernel<AT, WT, V, TP><<<dim3((C + per - 1) / per, chunks), 128, 0, h->stream>>>(b, u, ldu, col0, C, taps, (const WT*)w, (const WT*)bias, silu,
+    go_kernel(h, conv_kernel<AT, WT, V, TP>, dim3((C + per - 1) / per, chunks), 128, 0, h->stream, b, u, ldu, col0, C, taps, (const WT*)w, (const WT*)bias, silu,
                                                                                         state, o);
   };
   if (vec && taps == 4) go(std::integral_constant<int, 4>{}, std::integral_constant<int, 4>{});
@@ -1642,6 +1661,29 @@ LinearLaunch linear_launch(int parts, int dk, int dv, const AT* v, int ldv) {
                       dv % ch == 0 && cpb % ch == 0 && ldv % ch == 0 && (reinterpret_cast<uintptr_t>(v) & 15) == 0 ? 1 : 0};
 }
 
+// All unit lists that the layers of a step will ask for, before its first kernel: a copy between two kernels would keep the second from
+// starting under the first.
+template <typename AT>
+void prepare_units(hy_engine* h, int E, int T) {
+  if (!std::is_same<AT, bf16>::value || !h->part_o) return;
+  for (const hy_layer_cfg& c : h->lc) {
+    if (c.mixer == HY_MIX_ATTN_SCAN) {
+      if (c.a_dim == 32 || c.a_dim == 64 || c.a_dim == 128) attn_units(h, E, T, c.a_heads, c.a_kv_heads);
+    } else if (c.mixer == HY_MIX_LATENT) {
+      const int Dk = c.l_kv_rank + c.l_rot_dim;
+      const bool narrow = (Dk == 32 || Dk == 64 || Dk == 128) && attn_units(h, E, T, c.l_heads, 1, false, c.l_window);
+      if (!narrow && Dk % 8 == 0 && c.l_kv_rank <= 512) attn_units(h, E, T, c.l_heads, 1, true, c.l_window);
+    } else if (c.mixer == HY_MIX_WINDOW) {
+      if (c.w_dim % 8 == 0 && c.w_vdim % 8 == 0 && c.w_dim <= 128 && c.w_vdim <= 128) window_units(h, E, c.w_heads, c.w_kv_heads);
+    } else if (c.mixer == HY_MIX_BIASED || c.mixer == HY_MIX_ATTN_DELTA) {
+      BiasedCfg bc{};
+      bc.H = c.b_heads; bc.G = c.b_kv_heads; bc.window = c.mixer == HY_MIX_BIASED ? c.b_window : 0;
+      bc.keep = c.mixer == HY_MIX_BIASED ? c.b_keep_first : 0; bc.chunk = c.mixer == HY_MIX_BIASED ? c.b_chunk : 0;
+      if (c.b_dim % 8 == 0 && c.b_vdim % 8 == 0 && c.b_dim <= 128 && c.b_vdim <= 128) biased_units(h, E, T, bc, c.b_dim <= 64 && c.b_vdim <= 64 ? 64 : 128);
+    }
+  }
+}
+
 // Attention over a shared latent: down-projections in h->f1 ([query latent | key / value latent | raw rotated key part]; with
 // full-rank queries those are in h->pin already), result (heads concatenated) in h->cat.
 template <typename AT>
@@ -1655,7 +1697,7 @@ void latent_mixer(hy_engine* h, const Batch& b, const LayerW& L, const hy_layer_
   const int own = c.l_kv_from < 0 ? 1 : 0;
   {
     ProfScope ps(h, HY_PROF_CONV);
-    latent_prep_kernel<AT><<<T, 128, (size_t)(2 * L.rot.pairs + 2) * 4, s>>>(b, h->f1, h->ld_f1, c.l_q_rank, R, rot, own, L.l_qn,
+    go_kernel(h, latent_prep_kernel<AT>, T, 128, (size_t)(2 * L.rot.pairs + 2) * 4, s, b, h->f1, h->ld_f1, c.l_q_rank, R, rot, own, L.l_qn,
                                                                              L.l_kn, eps, L.rot, cv, h->ld_cv, (AT*)L.cache);
     h->launches++;
   }
@@ -1664,13 +1706,12 @@ void latent_mixer(hy_engine* h, const Batch& b, const LayerW& L, const hy_layer_
     if (c.l_q_rank > 0)
       gemm<AT, WT, AT>(h, cv, h->ld_cv, (const WT*)L.w_uq, c.l_q_rank, T, H * (dn + rot), c.l_q_rank, to_buf(pin, h->ld_pin), L.w_uq_t);
     const int fold = T > 8 ? 1 : 0;
-    latent_query_kernel<AT, WT><<<dim3((T + HY_LAT_TB - 1) / HY_LAT_TB, H, fold ? (R + 127) / 128 : 1), 128,
-                                  (size_t)(HY_LAT_TB * dn + 2 * L.rot.pairs + 2) * 4, s>>>(b, pin, h->ld_pin, (const WT*)L.w_uk, H, dn,
+    go_kernel(h, latent_query_kernel<AT, WT>, dim3((T + HY_LAT_TB - 1) / HY_LAT_TB, H, fold ? (R + 127) / 128 : 1), 128, (size_t)(HY_LAT_TB * dn + 2 * L.rot.pairs + 2) * 4, s, b, pin, h->ld_pin, (const WT*)L.w_uk, H, dn,
                                                                                            rot, R, fold, L.rot, cv, h->ld_cv);
     h->launches++;
     if (!fold) {
-      head_rows_kernel<AT, WT, AT><<<(H * R + 7) / 8, 256, 0, s>>>(T, pin, h->ld_pin, dn + rot, (const WT*)L.w_ukT, H, R, dn, cv,
-                                                                   h->ld_cv, Dk);
+      go_kernel(h, head_rows_kernel<AT, WT, AT>, (H * R + 7) / 8, 256, 0, s, T, pin, h->ld_pin, dn + rot, (const WT*)L.w_ukT, H, R, dn, cv,
+                                                                   h->ld_cv, Dk, (const AT*)nullptr, 0);
       h->launches++;
     }
   }
@@ -1684,11 +1725,11 @@ void latent_mixer(hy_engine* h, const Batch& b, const LayerW& L, const hy_layer_
         tc = true;
 #define HY_ATTN_ARGS b, u->d, cv, h->ld_cv, (const bf16*)L.cache, H, 1, c.l_scale, 0.0f, 1, c.l_window, u->split, u->ns, R, \
         h->part_o, h->part_ml
-        if (Dk == 32) attn_mma_kernel<32><<<u->n, 128, 0, s>>>(HY_ATTN_ARGS);
-        else if (Dk == 64) attn_mma_kernel<64><<<u->n, 128, 0, s>>>(HY_ATTN_ARGS);
-        else attn_mma_kernel<128><<<u->n, 128, 0, s>>>(HY_ATTN_ARGS);
+        if (Dk == 32) go_kernel(h, attn_mma_kernel<32>, u->n, 128, 0, s, HY_ATTN_ARGS);
+        else if (Dk == 64) go_kernel(h, attn_mma_kernel<64>, u->n, 128, 0, s, HY_ATTN_ARGS);
+        else go_kernel(h, attn_mma_kernel<128>, u->n, 128, 0, s, HY_ATTN_ARGS);
 #undef HY_ATTN_ARGS
-        attn_combine_kernel<WT, float><<<T * H, 64, 0, s>>>(b, h->part_o, h->part_ml, (const WT*)L.sink, nullptr, 0, H, 1, Dk, R,
+        go_kernel(h, attn_combine_kernel<WT, float>, T * H, 64, 0, s, b, h->part_o, h->part_ml, (const WT*)L.sink, nullptr, 0, H, 1, Dk, R,
                                                             c.l_window, u->split, u->ns, 1.0f, h->f2, h->ld_f2);
         h->launches += 2;
       }
@@ -1708,17 +1749,17 @@ void latent_mixer(hy_engine* h, const Batch& b, const LayerW& L, const hy_layer_
         }
 #define HY_WIDE_ARGS b, u->d, cv, h->ld_cv, (const bf16*)L.cache, H, Dk, R, c.l_scale, c.l_window, u->split, u->ns, pstride, \
         h->part_o, h->part_ml
-        if (nt == 2) attn_wide_kernel<2><<<u->n, 256, smem, s>>>(HY_WIDE_ARGS);
-        else if (nt == 4) attn_wide_kernel<4><<<u->n, 256, smem, s>>>(HY_WIDE_ARGS);
-        else attn_wide_kernel<8><<<u->n, 256, smem, s>>>(HY_WIDE_ARGS);
+        if (nt == 2) go_kernel(h, attn_wide_kernel<2>, u->n, 256, smem, s, HY_WIDE_ARGS);
+        else if (nt == 4) go_kernel(h, attn_wide_kernel<4>, u->n, 256, smem, s, HY_WIDE_ARGS);
+        else go_kernel(h, attn_wide_kernel<8>, u->n, 256, smem, s, HY_WIDE_ARGS);
 #undef HY_WIDE_ARGS
-        attn_combine_kernel<WT, float><<<T * H, 128, 0, s>>>(b, h->part_o, h->part_ml, (const WT*)L.sink, nullptr, 0, H, 1, pstride, R,
+        go_kernel(h, attn_combine_kernel<WT, float>, T * H, 128, 0, s, b, h->part_o, h->part_ml, (const WT*)L.sink, nullptr, 0, H, 1, pstride, R,
                                                             c.l_window, u->split, u->ns, 1.0f, h->f2, h->ld_f2);
         h->launches += 2;
       }
     }
     if (!tc) {
-      attn_sink_kernel<AT, WT, float><<<(T * H + 3) / 4, 128, 4 * Dk * sizeof(float), s>>>(
+      go_kernel(h, attn_sink_kernel<AT, WT, float>, (T * H + 3) / 4, 128, 4 * Dk * sizeof(float), s, 
           b, cv, h->ld_cv, (const AT*)L.cache, (const WT*)L.sink, (const AT*)nullptr, 0, H, 1, Dk, R, c.l_scale, 0.0f, 1, c.l_window, 1.0f,
           h->f2, h->ld_f2);
       h->launches++;
@@ -1728,10 +1769,10 @@ void latent_mixer(hy_engine* h, const Batch& b, const LayerW& L, const hy_layer_
     ProfScope ps(h, HY_PROF_SMALL_GEMM);
     const AT* gate = c.l_gate ? pin + L.c_g : nullptr;
     if (T <= 8)
-      head_rows_kernel<float, WT, AT><<<(H * dv + 7) / 8, 256, 0, s>>>(T, h->f2, h->ld_f2, R, (const WT*)L.w_uv, H, dv, R, cat,
+      go_kernel(h, head_rows_kernel<float, WT, AT>, (H * dv + 7) / 8, 256, 0, s, T, h->f2, h->ld_f2, R, (const WT*)L.w_uv, H, dv, R, cat,
                                                                        h->ld_cat, dv, gate, h->ld_pin);
     else
-    latent_value_kernel<AT, WT><<<dim3((T + HY_LAT_TB - 1) / HY_LAT_TB, H, (dv + 127) / 128), 128, (size_t)HY_LAT_TB * R * 4, s>>>(
+    go_kernel(h, latent_value_kernel<AT, WT>, dim3((T + HY_LAT_TB - 1) / HY_LAT_TB, H, (dv + 127) / 128), 128, (size_t)HY_LAT_TB * R * 4, s, 
         T, h->f2, h->ld_f2, (const WT*)L.w_uvT, H, R, dv, gate, h->ld_pin, cat, h->ld_cat);
     h->launches++;
   }
@@ -1748,7 +1789,7 @@ void place_rows(hy_engine* h, int T, const AT* hb, const LayerW& L, const hy_lay
   const bool tc = std::is_same<AT, bf16>::value && L.w_gu_t != nullptr;
   int* now = h->x_counts + (size_t)h->x_set * 2 * E;
   int* old = h->x_counts + (size_t)(h->x_set ^ 1) * 2 * E;
-  route_place_kernel<AT><<<P + 1, 128, 0, h->stream>>>(P, c.x_top, c.x_experts, E, tc ? expert_tile_rows(P, c.x_experts) : HY_XT, h->x_ids, now, now + E,
+  go_kernel(h, route_place_kernel<AT>, P + 1, 128, 0, h->stream, P, c.x_top, c.x_experts, E, tc ? expert_tile_rows(P, c.x_experts) : HY_XT, h->x_ids, now, now + E,
                                                        old, old + E, hb, W, W % (16 / (int)sizeof(AT)) == 0, h->x_offs, h->x_tile_e, h->x_tile_r0,
                                                        h->x_meta, h->x_pair_row, rows);
   h->launches++;
@@ -1775,7 +1816,7 @@ int sandwich_layer(hy_engine* h, const Batch& b, size_t li) {
   const TanhNorm after_ff = last ? none : h->lw[li + 1].n1;
   if (li == 0) {
     ProfScope ps(h, HY_PROF_NORM);
-    tanh_norm_kernel<AT><<<T, 256, 0, s>>>(h->x, nullptr, L.n1, W, hb);
+    go_kernel(h, tanh_norm_kernel<AT>, T, 256, 0, s, h->x, nullptr, L.n1, W, hb);
     h->launches++;
   }
   if (c.mixer == HY_MIX_SSD) {
@@ -1799,10 +1840,10 @@ int sandwich_layer(hy_engine* h, const Batch& b, size_t li) {
         const LinearLaunch g = linear_launch<AT>(PARTS, N, P, cv, h->ld_cv);
         const size_t smem = lin_smem<AT>(DR, PARTS, 0);
         cudaFuncSetAttribute(gla_kernel<AT, DR, PARTS, GLA_TOKEN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        gla_kernel<AT, DR, PARTS, GLA_TOKEN><<<dim3(H * g.bph, E), 128, smem, s>>>(b, h->lin, cv, h->ld_cv, nullptr, 0, nullptr, H, N, P, g.bph,
+        go_kernel(h, gla_kernel<AT, DR, PARTS, GLA_TOKEN>, dim3(H * g.bph, E), 128, smem, s, b, h->lin, cv, h->ld_cv, nullptr, 0, nullptr, H, N, P, g.bph,
                                                                                    g.vec, g.vvec, L.rec_state, h->f2, h->ld_f2, tk);
       });
-      gated_group_norm_kernel<AT><<<dim3(T, c.m_norm_groups), 128, 0, s>>>(h->f2, h->ld_f2, pin, h->ld_pin, L.m_norm, inner,
+      go_kernel(h, gated_group_norm_kernel<AT>, dim3(T, c.m_norm_groups), 128, 0, s, h->f2, h->ld_f2, pin, h->ld_pin, L.m_norm, inner,
                                                                           c.m_norm_groups, eps, cat, h->ld_cat);
       h->launches += 2;
     }
@@ -1820,21 +1861,21 @@ int sandwich_layer(hy_engine* h, const Batch& b, size_t li) {
     }
     ProfScope ps(h, HY_PROF_DELTA);
     if (dk <= HY_LIN_MAX_DIM) {
-      forget_rows_kernel<AT><<<T, T <= 8 ? 1024 : 256, 0, s>>>(pin, h->ld_pin, L.c_q, L.c_k, L.g_fb, L.g_lower, H, dk, h->lin);
+      go_kernel(h, forget_rows_kernel<AT>, T, T <= 8 ? 1024 : 256, 0, s, pin, h->ld_pin, L.c_q, L.c_k, L.g_fb, L.g_lower, H, dk, h->lin);
       launch_linear<AT>(dk, [&](auto dr, auto parts) {
         constexpr int DR = decltype(dr)::value, PARTS = decltype(parts)::value;
         const LinearLaunch g = linear_launch<AT>(PARTS, dk, dv, pin + L.c_v, h->ld_pin);
         const size_t smem = lin_smem<AT>(DR, PARTS, 0);
         cudaFuncSetAttribute(gla_kernel<AT, DR, PARTS, GLA_FORGET>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        gla_kernel<AT, DR, PARTS, GLA_FORGET><<<dim3(H * g.bph, E), 128, smem, s>>>(b, h->lin, pin + L.c_v, h->ld_pin, nullptr, 0, nullptr, H, dk,
-                                                                                    dv, g.bph, g.vec, g.vvec, L.rec_state, h->f2, h->ld_f2);
+        go_kernel(h, gla_kernel<AT, DR, PARTS, GLA_FORGET>, dim3(H * g.bph, E), 128, smem, s, b, h->lin, pin + L.c_v, h->ld_pin, nullptr, 0, nullptr, H, dk,
+                                                                                    dv, g.bph, g.vec, g.vvec, L.rec_state, h->f2, h->ld_f2, GlaToken{});
       });
-      gla_out_kernel<AT, AT, GATE_NONE><<<(T * H + 3) / 4, 128, 0, s>>>(T, H, dv, h->f2, h->ld_f2, nullptr, 0, L.g_norm, eps, 1.0f, cat, h->ld_cat);
+      go_kernel(h, gla_out_kernel<AT, AT, GATE_NONE>, (T * H + 3) / 4, 128, 0, s, T, H, dv, h->f2, h->ld_f2, nullptr, 0, L.g_norm, eps, 1.0f, cat, h->ld_cat);
       h->launches += 3;
     } else {
       static bool glr_attr = false;
       if (!glr_attr) { cudaFuncSetAttribute(glr_kernel<AT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024); glr_attr = true; }
-      glr_kernel<AT><<<dim3(H, E), 256, ((size_t)dk * dv + 2 * dk + dv + 40) * 4, s>>>(
+      go_kernel(h, glr_kernel<AT>, dim3(H, E), 256, ((size_t)dk * dv + 2 * dk + dv + 40) * 4, s, 
           b, pin, h->ld_pin, L.c_q, L.c_k, L.c_v, L.g_fb, L.g_lower, L.g_norm, H, dk, dv, eps, L.rec_state, cat, h->ld_cat);
       h->launches++;
     }
@@ -1857,7 +1898,7 @@ int sandwich_layer(hy_engine* h, const Batch& b, size_t li) {
     ProfScope ps(h, HY_PROF_ROUTE);
     gemm<AT, WT, float>(h, hb, W, (const WT*)L.w_router, W, T, NE, W, to_buf(h->f1, h->ld_f1), L.w_router_t);
     const RouteCfg rc{NE, top, c.x_groups, c.x_keep, c.x_scale};
-    route_kernel<<<T, 32, (size_t)(NE + c.x_groups) * 4, s>>>(h->f1, h->ld_f1, rc, h->x_ids, h->x_wts, few ? nullptr : next_counts(h));
+    go_kernel(h, route_kernel, T, 32, (size_t)(NE + c.x_groups) * 4, s, h->f1, h->ld_f1, rc, h->x_ids, h->x_wts, few ? nullptr : next_counts(h));
     h->launches++;
     if (!few) {
       place_rows<AT>(h, T, hb, L, c, x_rows);
@@ -1873,9 +1914,9 @@ int sandwich_layer(hy_engine* h, const Batch& b, size_t li) {
         cudaFuncSetAttribute(expert_rows_kernel<AT, WT, float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
         rows_attr = true;
       }
-      expert_rows_kernel<AT, WT, AT, true><<<dim3(std::min((ff + 7) / 8, 256), P), 256, (size_t)W * sizeof(AT), s>>>(
+      go_kernel(h, expert_rows_kernel<AT, WT, AT, true>, dim3(std::min((ff + 7) / 8, 256), P), 256, (size_t)W * sizeof(AT), s, 
           hb, W, h->x_ids, top, 1, NE, (const WT*)L.w_gu, (size_t)2 * ff * W, ff, W, pin, ldh, 0, 0.0f);
-      expert_rows_kernel<AT, WT, float, false><<<dim3(std::min((W + 7) / 8, 256), P), 256, (size_t)ff * sizeof(AT), s>>>(
+      go_kernel(h, expert_rows_kernel<AT, WT, float, false>, dim3(std::min((W + 7) / 8, 256), P), 256, (size_t)ff * sizeof(AT), s, 
           pin, ldh, h->x_ids, top, 0, NE, (const WT*)L.w_down, (size_t)W * ff, W, ff, ys, W, -1, 0.0f);
     } else if (tc_experts) {
       if constexpr (std::is_same<AT, bf16>::value) {
@@ -1887,12 +1928,12 @@ int sandwich_layer(hy_engine* h, const Batch& b, size_t li) {
       }
     } else {
       const int tiles = std::min(h->x_max_tiles, P / HY_XT + NE + 1);
-      expert_gemm_simt_kernel<AT, WT, AT, true><<<dim3((ff + 63) / 64, tiles), 256, 0, s>>>(
+      go_kernel(h, expert_gemm_simt_kernel<AT, WT, AT, true>, dim3((ff + 63) / 64, tiles), 256, 0, s, 
           x_rows, W, (const WT*)L.w_gu, (size_t)2 * ff * W, ff, W, h->x_offs, h->x_tile_e, h->x_tile_r0, h->x_meta, pin, ldh, 0, 0.0f);
-      expert_gemm_simt_kernel<AT, WT, float, false><<<dim3((W + 63) / 64, tiles), 256, 0, s>>>(
+      go_kernel(h, expert_gemm_simt_kernel<AT, WT, float, false>, dim3((W + 63) / 64, tiles), 256, 0, s, 
           pin, ldh, (const WT*)L.w_down, (size_t)W * ff, W, ff, h->x_offs, h->x_tile_e, h->x_tile_r0, h->x_meta, ys, W, -1, 0.0f);
     }
-    expert_combine_kernel<AT><<<T, 256, 0, s>>>(ys, W, few ? nullptr : h->x_pair_row, h->x_wts, top, W, L.n2b, L.ls2, h->x, after_ff, hb);
+    go_kernel(h, expert_combine_kernel<AT>, T, 256, 0, s, ys, W, few ? nullptr : h->x_pair_row, h->x_wts, top, W, L.n2b, L.ls2, h->x, after_ff, hb);
     h->launches += 3;
   }
   return HY_OK;
@@ -1906,7 +1947,7 @@ void post_norm_add(hy_engine* h, int T, const float* y, int ldy, const float* ro
   const int W = h->m.width;
   static bool attr = false;                                  // per AT: this function is a template
   if (!attr) { cudaFuncSetAttribute(post_norm_add_kernel<AT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024); attr = true; }
-  post_norm_add_kernel<AT><<<T, 256, (size_t)W * 4, h->stream>>>(y, ldy, rows, W, pair_row, wts, top, shared_rows, w, ls, h->m.norm_eps,
+  go_kernel(h, post_norm_add_kernel<AT>, T, 256, (size_t)W * 4, h->stream, y, ldy, rows, W, pair_row, wts, top, shared_rows, w, ls, h->m.norm_eps,
                                                                W, add, h->x, (AT*)h->hbuf);
   h->launches++;
 }
@@ -1932,7 +1973,7 @@ int postnorm_layer(hy_engine* h, const Batch& b, size_t li) {
     }
     {
       ProfScope ps(h, HY_PROF_CONV);
-      window_prep_kernel<AT><<<T, 128, (size_t)(2 * L.rot.pairs + 2 * L.rot_v.pairs + 2) * 4, s>>>(
+      go_kernel(h, window_prep_kernel<AT>, T, 128, (size_t)(2 * L.rot.pairs + 2 * L.rot_v.pairs + 2) * 4, s, 
           b, pin, h->ld_pin, L.c_q, L.c_k, L.c_v, wc, L.w_qn, L.w_kn, eps, L.rot, L.rot_v, cv, h->ld_cv, (AT*)L.cache, (AT*)L.cache_v,
           h->f1, h->ld_f1);
       int most = 0;                                           // blocks one entry completes in this step
@@ -1942,7 +1983,7 @@ int postnorm_layer(hy_engine* h, const Batch& b, size_t li) {
       }
       h->launches++;
       if (most > 0) {
-        window_pool_kernel<AT><<<dim3(most, E), 128, 0, s>>>(b, wc, (const AT*)L.cache, (const AT*)L.cache_v, (AT*)L.pool_k, (AT*)L.pool_v);
+        go_kernel(h, window_pool_kernel<AT>, dim3(most, E), 128, 0, s, b, wc, (const AT*)L.cache, (const AT*)L.cache_v, (AT*)L.pool_k, (AT*)L.pool_v);
         h->launches++;
       }
     }
@@ -1964,13 +2005,13 @@ int postnorm_layer(hy_engine* h, const Batch& b, size_t li) {
             cudaFuncSetAttribute(window_mma_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)window_mma_smem(128));
             win_attr = true;
           }
-          if (c.w_dim <= 64 && c.w_vdim <= 64) window_mma_kernel<64><<<u->n, 128, window_mma_smem(64), s>>>(HY_WIN_ARGS);
-          else window_mma_kernel<128><<<u->n, 128, window_mma_smem(128), s>>>(HY_WIN_ARGS);
+          if (c.w_dim <= 64 && c.w_vdim <= 64) go_kernel(h, window_mma_kernel<64>, u->n, 128, window_mma_smem(64), s, HY_WIN_ARGS);
+          else go_kernel(h, window_mma_kernel<128>, u->n, 128, window_mma_smem(128), s, HY_WIN_ARGS);
 #undef HY_WIN_ARGS
         }
       }
       if (!tc)
-        window_attn_kernel<AT, AT><<<(T * c.w_heads + 3) / 4, 128, 4 * c.w_dim * sizeof(float), s>>>(
+        go_kernel(h, window_attn_kernel<AT, AT>, (T * c.w_heads + 3) / 4, 128, 4 * c.w_dim * sizeof(float), s, 
             b, cv, h->ld_cv, wc, (const AT*)L.cache, (const AT*)L.cache_v, (const AT*)L.pool_k, (const AT*)L.pool_v, h->f1, h->ld_f1,
             cat, h->ld_cat);
       h->launches++;
@@ -2004,10 +2045,10 @@ int postnorm_layer(hy_engine* h, const Batch& b, size_t li) {
       const size_t tb = (size_t)mlstm_tb(dr);
       return (tb * (2 * dr + 3 * nt) + 9 * tb + 4) * 4 + 2 * tb * (2 * dr + 2 * nt) * sizeof(AT);
     };
-    if (dk <= 32 && nthr <= 256 && msm(32, nthr) <= 220 * 1024) mlstm_reg_kernel<AT, 32><<<dim3(H, E), nthr, msm(32, nthr), s>>>(HY_MLSTM_ARGS);
-    else if (dk <= 64 && nthr <= 256 && msm(64, nthr) <= 220 * 1024) mlstm_reg_kernel<AT, 64><<<dim3(H, E), nthr, msm(64, nthr), s>>>(HY_MLSTM_ARGS);
-    else if (dk <= 128 && nthr <= 256 && msm(128, nthr) <= 220 * 1024) mlstm_reg_kernel<AT, 128><<<dim3(H, E), nthr, msm(128, nthr), s>>>(HY_MLSTM_ARGS);
-    else mlstm_kernel<AT><<<dim3(H, E), 256, ((size_t)dk * (dv + 1) + 2 * dk + dv + 1 + 40) * 4, s>>>(HY_MLSTM_GEN_ARGS);
+    if (dk <= 32 && nthr <= 256 && msm(32, nthr) <= 220 * 1024) go_kernel(h, mlstm_reg_kernel<AT, 32>, dim3(H, E), nthr, msm(32, nthr), s, HY_MLSTM_ARGS);
+    else if (dk <= 64 && nthr <= 256 && msm(64, nthr) <= 220 * 1024) go_kernel(h, mlstm_reg_kernel<AT, 64>, dim3(H, E), nthr, msm(64, nthr), s, HY_MLSTM_ARGS);
+    else if (dk <= 128 && nthr <= 256 && msm(128, nthr) <= 220 * 1024) go_kernel(h, mlstm_reg_kernel<AT, 128>, dim3(H, E), nthr, msm(128, nthr), s, HY_MLSTM_ARGS);
+    else go_kernel(h, mlstm_kernel<AT>, dim3(H, E), 256, ((size_t)dk * (dv + 1) + 2 * dk + dv + 1 + 40) * 4, s, HY_MLSTM_GEN_ARGS);
 #undef HY_MLSTM_ARGS
 #undef HY_MLSTM_GEN_ARGS
     h->launches++;
@@ -2038,7 +2079,7 @@ int postnorm_layer(hy_engine* h, const Batch& b, size_t li) {
       }
       if (!fused) {
         gemm<AT, WT, AT>(h, hb, W, (const WT*)L.w_ff_in, W, T, 2 * ff, W, to_buf(pin, h->ld_pin));
-        gated_act_kernel<AT><<<dim3((ff + 255) / 256, T), 256, 0, s>>>(pin, h->ld_pin, ff, c.ff_act, c.ff_limit, cat, h->ld_cat);
+        go_kernel(h, gated_act_kernel<AT>, dim3((ff + 255) / 256, T), 256, 0, s, pin, h->ld_pin, ff, c.ff_act, c.ff_limit, cat, h->ld_cat);
         h->launches++;
       }
     }
@@ -2060,10 +2101,10 @@ int postnorm_layer(hy_engine* h, const Batch& b, size_t li) {
     ProfScope ps(h, HY_PROF_ROUTE);
     gemm<AT, WT, float>(h, hb, W, (const WT*)L.w_router, W, T, NE, W, to_buf(h->f1, h->ld_f1), L.w_router_t);
     if (c.x_route == HY_ROUTE_TOP_SOFTMAX) {
-      route_top_kernel<<<T, 32, (size_t)NE * 4, s>>>(h->f1, h->ld_f1, L.x_rb, NE, top, h->x_ids, h->x_wts, few ? nullptr : next_counts(h));
+      go_kernel(h, route_top_kernel, T, 32, (size_t)NE * 4, s, h->f1, h->ld_f1, L.x_rb, NE, top, h->x_ids, h->x_wts, few ? nullptr : next_counts(h));
     } else {
       const RouteCfg rc{NE, top, c.x_groups, c.x_keep, c.x_scale};
-      route_kernel<<<T, 32, (size_t)(NE + c.x_groups) * 4, s>>>(h->f1, h->ld_f1, rc, h->x_ids, h->x_wts, few ? nullptr : next_counts(h));
+      go_kernel(h, route_kernel, T, 32, (size_t)(NE + c.x_groups) * 4, s, h->f1, h->ld_f1, rc, h->x_ids, h->x_wts, few ? nullptr : next_counts(h));
     }
     h->launches++;
     if (!few) {
@@ -2081,9 +2122,9 @@ int postnorm_layer(hy_engine* h, const Batch& b, size_t li) {
         cudaFuncSetAttribute(expert_rows_kernel<AT, WT, float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
         rows_attr = true;
       }
-      expert_rows_kernel<AT, WT, AT, false><<<dim3(std::min((ff + 7) / 8, 256), P), 256, (size_t)W * sizeof(AT), s>>>(
+      go_kernel(h, expert_rows_kernel<AT, WT, AT, false>, dim3(std::min((ff + 7) / 8, 256), P), 256, (size_t)W * sizeof(AT), s, 
           hb, W, h->x_ids, top, 1, NE, (const WT*)L.w_gu, (size_t)ff * W, ff, W, pin, ldh, c.x_act, c.ff_limit);
-      expert_rows_kernel<AT, WT, float, false><<<dim3(std::min((W + 7) / 8, 256), P), 256, (size_t)ff * sizeof(AT), s>>>(
+      go_kernel(h, expert_rows_kernel<AT, WT, float, false>, dim3(std::min((W + 7) / 8, 256), P), 256, (size_t)ff * sizeof(AT), s, 
           pin, ldh, h->x_ids, top, 0, NE, (const WT*)L.w_down, (size_t)W * ff, W, ff, ys, W, -1, 0.0f);
     } else if (tc_experts) {
       if constexpr (std::is_same<AT, bf16>::value) {
@@ -2096,9 +2137,9 @@ int postnorm_layer(hy_engine* h, const Batch& b, size_t li) {
       }
     } else {
       const int tiles = std::min(h->x_max_tiles, P / HY_XT + NE + 1);
-      expert_gemm_simt_kernel<AT, WT, AT, false><<<dim3((ff + 63) / 64, tiles), 256, 0, s>>>(
+      go_kernel(h, expert_gemm_simt_kernel<AT, WT, AT, false>, dim3((ff + 63) / 64, tiles), 256, 0, s, 
           x_rows, W, (const WT*)L.w_gu, (size_t)ff * W, ff, W, h->x_offs, h->x_tile_e, h->x_tile_r0, h->x_meta, pin, ldh, c.x_act, c.ff_limit);
-      expert_gemm_simt_kernel<AT, WT, float, false><<<dim3((W + 63) / 64, tiles), 256, 0, s>>>(
+      go_kernel(h, expert_gemm_simt_kernel<AT, WT, float, false>, dim3((W + 63) / 64, tiles), 256, 0, s, 
           pin, ldh, (const WT*)L.w_down, (size_t)W * ff, W, ff, h->x_offs, h->x_tile_e, h->x_tile_r0, h->x_meta, ys, W, -1, 0.0f);
     }
     h->launches += 2;
@@ -2134,11 +2175,11 @@ bool routed_gated_experts(hy_engine* h, int T, const AT* hb, const LayerW& L, co
     if (c.x_route == HY_ROUTE_CORRECTED_SOFTMAX) {
       const int outputs = NE + c.x_identity;
       if (L.w_router) gemm<AT, WT, float>(h, hb, W, (const WT*)L.w_router, W, T, outputs, W, to_buf(h->f1, h->ld_f1), L.w_router_t);
-      route_corrected_kernel<<<T, 32, (size_t)(2 * outputs + c.x_groups) * 4, s>>>(h->f1 + L.c_router, h->ld_f1, L.x_corr, NE, outputs, top,
+      go_kernel(h, route_corrected_kernel, T, 32, (size_t)(2 * outputs + c.x_groups) * 4, s, h->f1 + L.c_router, h->ld_f1, L.x_corr, NE, outputs, top,
                                                                                    c.x_groups, c.x_keep, h->x_ids, h->x_wts, few ? nullptr : next_counts(h));
     } else {
       gemm<AT, WT, float>(h, hb, W, (const WT*)L.w_router, W, T, NE, W, to_buf(h->f1, h->ld_f1), L.w_router_t);
-      route_top_kernel<<<T, 32, (size_t)NE * 4, s>>>(h->f1, h->ld_f1, nullptr, NE, top, h->x_ids, h->x_wts, few ? nullptr : next_counts(h));
+      go_kernel(h, route_top_kernel, T, 32, (size_t)NE * 4, s, h->f1, h->ld_f1, nullptr, NE, top, h->x_ids, h->x_wts, few ? nullptr : next_counts(h));
     }
     h->launches++;
     if (!few) {
@@ -2154,9 +2195,9 @@ bool routed_gated_experts(hy_engine* h, int T, const AT* hb, const LayerW& L, co
       cudaFuncSetAttribute(expert_rows_kernel<AT, WT, float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
       rows_attr = true;
     }
-    expert_rows_kernel<AT, WT, AT, true><<<dim3(std::min((ff + 7) / 8, 256), P), 256, (size_t)W * sizeof(AT), s>>>(
+    go_kernel(h, expert_rows_kernel<AT, WT, AT, true>, dim3(std::min((ff + 7) / 8, 256), P), 256, (size_t)W * sizeof(AT), s, 
         hb, W, h->x_ids, top, 1, NE, (const WT*)L.w_gu, (size_t)2 * ff * W, ff, W, pin, ldh, c.x_act, c.ff_limit);
-    expert_rows_kernel<AT, WT, float, false><<<dim3(std::min((W + 7) / 8, 256), P), 256, (size_t)ff * sizeof(AT), s>>>(
+    go_kernel(h, expert_rows_kernel<AT, WT, float, false>, dim3(std::min((W + 7) / 8, 256), P), 256, (size_t)ff * sizeof(AT), s, 
         pin, ldh, h->x_ids, top, 0, NE, (const WT*)L.w_down, (size_t)W * ff, W, ff, ys, W, -1, 0.0f);
   } else if (tc_experts) {
     if constexpr (std::is_same<AT, bf16>::value) {
@@ -2169,9 +2210,9 @@ bool routed_gated_experts(hy_engine* h, int T, const AT* hb, const LayerW& L, co
     }
   } else {
     const int tiles = std::min(h->x_max_tiles, P / HY_XT + NE + 1);
-    expert_gemm_simt_kernel<AT, WT, AT, true><<<dim3((ff + 63) / 64, tiles), 256, 0, s>>>(
+    go_kernel(h, expert_gemm_simt_kernel<AT, WT, AT, true>, dim3((ff + 63) / 64, tiles), 256, 0, s, 
         x_rows, W, (const WT*)L.w_gu, (size_t)2 * ff * W, ff, W, h->x_offs, h->x_tile_e, h->x_tile_r0, h->x_meta, pin, ldh, c.x_act, c.ff_limit);
-    expert_gemm_simt_kernel<AT, WT, float, false><<<dim3((W + 63) / 64, tiles), 256, 0, s>>>(
+    go_kernel(h, expert_gemm_simt_kernel<AT, WT, float, false>, dim3((W + 63) / 64, tiles), 256, 0, s, 
         pin, ldh, (const WT*)L.w_down, (size_t)W * ff, W, ff, h->x_offs, h->x_tile_e, h->x_tile_r0, h->x_meta, ys, W, -1, 0.0f);
   }
   h->launches += 2;
@@ -2183,7 +2224,7 @@ void stream_row(hy_engine* h, const Batch& b, const StreamOp& o) {
   const int W = h->m.width;
   static bool attr = false;                                  // per WT: this function is a template
   if (!attr) { cudaFuncSetAttribute(stream_row_kernel<WT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024); attr = true; }
-  stream_row_kernel<WT><<<b.T, 256, ((size_t)2 * W + (size_t)std::max(o.side_dim, 0)) * 4, h->stream>>>(b, o, W, h->x);
+  go_kernel(h, stream_row_kernel<WT>, b.T, 256, ((size_t)2 * W + (size_t)std::max(o.side_dim, 0)) * 4, h->stream, b, o, W, h->x);
   h->launches++;
 }
 
@@ -2191,11 +2232,11 @@ void stream_row(hy_engine* h, const Batch& b, const StreamOp& o) {
 template <typename AT>
 void canon_input(hy_engine* h, const Batch& b, const float* w, float* tails) {
   const int W = h->m.width, taps = h->m.canon_taps;
-  if (W % 4 == 0) canon_kernel<AT, 4><<<dim3((W / 4 + 127) / 128, b.T), 128, 0, h->stream>>>(b, h->hn, W, taps, w, tails, (AT*)h->hbuf);
-  else canon_kernel<AT, 1><<<dim3((W + 127) / 128, b.T), 128, 0, h->stream>>>(b, h->hn, W, taps, w, tails, (AT*)h->hbuf);
+  if (W % 4 == 0) go_kernel(h, canon_kernel<AT, 4>, dim3((W / 4 + 127) / 128, b.T), 128, 0, h->stream, b, h->hn, W, taps, w, tails, (AT*)h->hbuf);
+  else go_kernel(h, canon_kernel<AT, 1>, dim3((W + 127) / 128, b.T), 128, 0, h->stream, b, h->hn, W, taps, w, tails, (AT*)h->hbuf);
   h->launches++;
   if (taps > 1) {
-    conv_tail_kernel<float><<<dim3((W + 127) / 128, b.E), 128, 0, h->stream>>>(b, h->hn, W, 0, W, taps, tails);
+    go_kernel(h, conv_tail_kernel<float>, dim3((W + 127) / 128, b.E), 128, 0, h->stream, b, h->hn, W, 0, W, taps, tails);
     h->launches++;
   }
 }
@@ -2215,7 +2256,7 @@ void biased_mixer(hy_engine* h, const Batch& b, const LayerW& L, const hy_layer_
                      c.b_chunk, c.b_bias, nullptr, 0, 1.0f};
   {
     ProfScope ps(h, HY_PROF_CONV);
-    biased_prep_kernel<AT><<<T, 128, 0, s>>>(b, pin, h->ld_pin, L.c_q, c.b_heads * c.b_dim, L.c_k, L.c_v, c.b_kv_heads, c.b_dim, c.b_vdim,
+    go_kernel(h, biased_prep_kernel<AT>, T, 128, 0, s, b, pin, h->ld_pin, L.c_q, c.b_heads * c.b_dim, L.c_k, L.c_v, c.b_kv_heads, c.b_dim, c.b_vdim,
                                              L.b_qn, L.b_kn, h->m.norm_eps, L.b_mix, L.b_lambda,
                                              (AT*)h->vfirst, h->ld_vf, (AT*)L.cache, (AT*)L.cache_v);
     h->launches++;
@@ -2250,21 +2291,21 @@ void biased_attend(hy_engine* h, const Batch& b, const LayerW& L, const hy_layer
 #define HY_BIASED_ARGS b, u->d, pin + L.c_q, h->ld_pin, bc, (const bf16*)L.cache, (const bf16*)L.cache_v, cat, h->ld_cat, u->ns, h->part_o, h->part_ml
         const bool pl = bc.bias == HY_BIAS_NONE && bc.cap <= 0.0f && !bc.window && !bc.keep && !bc.chunk;
         if (dp == 64) {
-          if (pl) biased_mma_kernel<64, true><<<u->n, 128, window_mma_smem(64), s>>>(HY_BIASED_ARGS);
-          else biased_mma_kernel<64, false><<<u->n, 128, window_mma_smem(64), s>>>(HY_BIASED_ARGS);
+          if (pl) go_kernel(h, biased_mma_kernel<64, true>, u->n, 128, window_mma_smem(64), s, HY_BIASED_ARGS);
+          else go_kernel(h, biased_mma_kernel<64, false>, u->n, 128, window_mma_smem(64), s, HY_BIASED_ARGS);
         } else {
-          if (pl) biased_mma_kernel<128, true><<<u->n, 128, window_mma_smem(128), s>>>(HY_BIASED_ARGS);
-          else biased_mma_kernel<128, false><<<u->n, 128, window_mma_smem(128), s>>>(HY_BIASED_ARGS);
+          if (pl) go_kernel(h, biased_mma_kernel<128, true>, u->n, 128, window_mma_smem(128), s, HY_BIASED_ARGS);
+          else go_kernel(h, biased_mma_kernel<128, false>, u->n, 128, window_mma_smem(128), s, HY_BIASED_ARGS);
         }
 #undef HY_BIASED_ARGS
         if (u->ns > 1) {
-          biased_combine_kernel<bf16><<<T * c.b_heads, 64, 0, s>>>(h->part_o, h->part_ml, bc, dp, u->ns, cat, h->ld_cat);
+          go_kernel(h, biased_combine_kernel<bf16>, T * c.b_heads, 64, 0, s, h->part_o, h->part_ml, bc, dp, u->ns, cat, h->ld_cat);
           h->launches++;
         }
       }
     }
     if (!tc)
-      biased_attn_kernel<AT, AT><<<(T * c.b_heads + 3) / 4, 128, 4 * c.b_dim * sizeof(float), s>>>(
+      go_kernel(h, biased_attn_kernel<AT, AT>, (T * c.b_heads + 3) / 4, 128, 4 * c.b_dim * sizeof(float), s, 
           b, pin + L.c_q, h->ld_pin, bc, (const AT*)L.cache, (const AT*)L.cache_v, cat, h->ld_cat);
     h->launches++;
   }
@@ -2338,7 +2379,7 @@ int prenorm_layer(hy_engine* h, const Batch& b, size_t li) {
       }
       if (!fused) {
         gemm<AT, WT, AT>(h, hb, W, (const WT*)L.w_ff_in, W, T, 2 * ff, W, to_buf(pin, h->ld_pin));
-        gated_act_kernel<AT><<<dim3((ff + 255) / 256, T), 256, 0, s>>>(pin, h->ld_pin, ff, c.ff_act, c.ff_limit, cat, h->ld_cat);
+        go_kernel(h, gated_act_kernel<AT>, dim3((ff + 255) / 256, T), 256, 0, s, pin, h->ld_pin, ff, c.ff_act, c.ff_limit, cat, h->ld_cat);
         h->launches++;
       }
     }
@@ -2370,16 +2411,16 @@ void gla_mixer(hy_engine* h, const Batch& b, const LayerW& L, const hy_layer_cfg
     gemm<float, WT, float>(h, h->f1, h->ld_f1, (const WT*)L.w_a2, c.g_low, T, nq, c.g_low, o);
   }
   ProfScope ps(h, HY_PROF_DELTA);
-  linear_rows_kernel<AT><<<T, T <= 8 ? 1024 : 128, 0, s>>>(pin, h->ld_pin, L.c_q, L.c_k, H, dk, nullptr, 0, RotPair{0, 1}, h->lin);
+  go_kernel(h, linear_rows_kernel<AT>, T, T <= 8 ? 1024 : 128, 0, s, pin, h->ld_pin, L.c_q, L.c_k, H, dk, nullptr, 0, RotPair{0, 1}, h->lin);
   launch_linear<AT>(dk, [&](auto dr, auto parts) {
     constexpr int DR = decltype(dr)::value, PARTS = decltype(parts)::value;
     const LinearLaunch g = linear_launch<AT>(PARTS, dk, dv, pin + L.c_v, h->ld_pin);
     const size_t smem = lin_smem<AT>(DR, PARTS, DR);
     cudaFuncSetAttribute(gla_kernel<AT, DR, PARTS, GLA_CHANNEL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    gla_kernel<AT, DR, PARTS, GLA_CHANNEL><<<dim3(H * g.bph, E), 128, smem, s>>>(b, h->lin, pin + L.c_v, h->ld_pin, h->f2, h->ld_f2, nullptr, H, dk,
-                                                                           dv, g.bph, g.vec, g.vvec, L.rec_state, h->f2 + c_o, h->ld_f2);
+    go_kernel(h, gla_kernel<AT, DR, PARTS, GLA_CHANNEL>, dim3(H * g.bph, E), 128, smem, s, b, h->lin, pin + L.c_v, h->ld_pin, h->f2, h->ld_f2, nullptr, H, dk,
+                                                                           dv, g.bph, g.vec, g.vvec, L.rec_state, h->f2 + c_o, h->ld_f2, GlaToken{});
   });
-  gla_out_kernel<AT><<<(T * H + 3) / 4, 128, 0, s>>>(T, H, dv, h->f2 + c_o, h->ld_f2, pin + L.c_g, h->ld_pin, L.g_norm, h->m.norm_eps,
+  go_kernel(h, gla_out_kernel<AT>, (T * H + 3) / 4, 128, 0, s, T, H, dv, h->f2 + c_o, h->ld_f2, pin + L.c_g, h->ld_pin, L.g_norm, h->m.norm_eps,
                                                      1.0f, cat, h->ld_cat);
   h->launches += 3;
 }
@@ -2393,16 +2434,16 @@ void retention_mixer(hy_engine* h, const Batch& b, const LayerW& L, const hy_lay
   const RotTable& rot = h->rot_tables[(size_t)L.rot_table].t;
   const RotPair rp{rot.pairs, c.r_half};
   ProfScope ps(h, HY_PROF_DELTA);
-  linear_rows_kernel<AT><<<T, T <= 8 ? 1024 : 128, 0, s>>>(pin, h->ld_pin, L.c_q, L.c_k, H, dk, rot.out, rot.ld, rp, h->lin);
+  go_kernel(h, linear_rows_kernel<AT>, T, T <= 8 ? 1024 : 128, 0, s, pin, h->ld_pin, L.c_q, L.c_k, H, dk, rot.out, rot.ld, rp, h->lin);
   launch_linear<AT>(dk, [&](auto dr, auto parts) {
     constexpr int DR = decltype(dr)::value, PARTS = decltype(parts)::value;
     const LinearLaunch g = linear_launch<AT>(PARTS, dk, dv, pin + L.c_v, h->ld_pin);
     const size_t smem = lin_smem<AT>(DR, PARTS, 0);
     cudaFuncSetAttribute(gla_kernel<AT, DR, PARTS, GLA_HEAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    gla_kernel<AT, DR, PARTS, GLA_HEAD><<<dim3(H * g.bph, E), 128, smem, s>>>(b, h->lin, pin + L.c_v, h->ld_pin, nullptr, 0, L.decay, H, dk, dv,
-                                                                          g.bph, g.vec, g.vvec, L.rec_state, h->f2, h->ld_f2);
+    go_kernel(h, gla_kernel<AT, DR, PARTS, GLA_HEAD>, dim3(H * g.bph, E), 128, smem, s, b, h->lin, pin + L.c_v, h->ld_pin, nullptr, 0, L.decay, H, dk, dv,
+                                                                          g.bph, g.vec, g.vvec, L.rec_state, h->f2, h->ld_f2, GlaToken{});
   });
-  gla_out_kernel<AT><<<(T * H + 3) / 4, 128, 0, s>>>(T, H, dv, h->f2, h->ld_f2, pin + L.c_g, h->ld_pin, nullptr, h->m.norm_eps, 1.0f, cat,
+  go_kernel(h, gla_out_kernel<AT>, (T * H + 3) / 4, 128, 0, s, T, H, dv, h->f2, h->ld_f2, pin + L.c_g, h->ld_pin, nullptr, h->m.norm_eps, 1.0f, cat,
                                                      h->ld_cat);
   h->launches += 3;
 }
@@ -2418,13 +2459,13 @@ void attn_delta_mixer(hy_engine* h, const Batch& b, const LayerW& L, const hy_la
   const int H = c.d_heads, G = c.d_kv_heads, dk = c.d_dim, dv = c.d_vdim, nk = G * dk, C = 2 * nk + H * dv;
   {
     ProfScope ps(h, HY_PROF_CONV);
-    key_value_prep_kernel<AT><<<T, 128, 0, s>>>(b, pin, h->ld_pin, L.c_q, L.c_k, c.b_heads, c.b_kv_heads, c.b_dim, rot.out, rot.ld,
+    go_kernel(h, key_value_prep_kernel<AT>, T, 128, 0, s, b, pin, h->ld_pin, L.c_q, L.c_k, c.b_heads, c.b_kv_heads, c.b_dim, rot.out, rot.ld,
                                                 RotPair{rot.pairs, c.r_half}, (AT*)L.cache, (AT*)L.cache_v);
     ConvOut<AT> co{};                                          // values in the activation type, queries and keys as fp32 rows
     co.out = cv; co.ldo = h->ld_cv; co.out_lo = 2 * nk; co.out_hi = C;
     co.rows = h->lin; co.G = G; co.n = dk;
     launch_conv<AT>(h, b, pin, h->ld_pin, L.c_x, C, c.d_conv, L.conv_qkv, nullptr, 1, L.conv_state, co);
-    delta_unit_kernel<AT, false><<<(T * G + 3) / 4, 128, 0, s>>>(T, H, G, dk, h->f1 + c.b_heads, h->ld_f1, (const float*)L.A_log,
+    go_kernel(h, delta_unit_kernel<AT, false>, (T * G + 3) / 4, 128, 0, s, T, H, G, dk, h->f1 + c.b_heads, h->ld_f1, (const float*)L.A_log,
                                                                  (const float*)L.dt_bias, nullptr, 0, nullptr, 0, h->lin, h->lin_sc);
     h->launches += 2;
   }
@@ -2437,10 +2478,10 @@ void attn_delta_mixer(hy_engine* h, const Batch& b, const LayerW& L, const hy_la
     const LinearLaunch g = linear_launch<AT>(PARTS, dk, dv, cv, h->ld_cv);
     const size_t smem = lin_smem<AT>(DR, PARTS, 4);
     cudaFuncSetAttribute(delta_head_kernel<AT, DR, PARTS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    delta_head_kernel<AT, DR, PARTS><<<dim3(H * g.bph, E), 128, smem, s>>>(b, h->lin, cv, h->ld_cv, h->lin_sc, H, G, dk, dv, g.bph, g.vec, g.vvec,
-                                                                           L.rec_state, h->f2, h->ld_f2);
+    go_kernel(h, delta_head_kernel<AT, DR, PARTS>, dim3(H * g.bph, E), 128, smem, s, b, h->lin, cv, h->ld_cv, h->lin_sc, H, G, dk, dv, g.bph, g.vec, g.vvec,
+                                                                           L.rec_state, h->f2, h->ld_f2, nullptr, 0);
   });
-  gla_out_kernel<AT><<<(T * H + 3) / 4, 128, 0, s>>>(T, H, dv, h->f2, h->ld_f2, pin + L.c_g, h->ld_pin, L.g_norm, h->m.norm_eps,
+  go_kernel(h, gla_out_kernel<AT>, (T * H + 3) / 4, 128, 0, s, T, H, dv, h->f2, h->ld_f2, pin + L.c_g, h->ld_pin, L.g_norm, h->m.norm_eps,
                                                      c.right_scale, cat + L.o_scan, h->ld_cat);
   h->launches += 2;
 }
@@ -2459,8 +2500,8 @@ void launch_row_close(hy_engine* h, int T, RowClose rc) {
   rc.eps = h->m.norm_eps;
   if (!rc.rows && !rc.y && !rc.cast_out && !rc.norm_w) return;
   ProfScope ps(h, HY_PROF_NORM);
-  if (W % 4 == 0) row_close_kernel<AT, WT, 4><<<T, 256, (size_t)W * 4, h->stream>>>(rc, W, h->x, (AT*)h->hbuf);
-  else row_close_kernel<AT, WT, 1><<<T, 256, (size_t)W * 4, h->stream>>>(rc, W, h->x, (AT*)h->hbuf);
+  if (W % 4 == 0) go_kernel(h, row_close_kernel<AT, WT, 4>, T, 256, (size_t)W * 4, h->stream, rc, W, h->x, (AT*)h->hbuf);
+  else go_kernel(h, row_close_kernel<AT, WT, 1>, T, 256, (size_t)W * 4, h->stream, rc, W, h->x, (AT*)h->hbuf);
   h->launches++;
 }
 
@@ -2548,7 +2589,7 @@ int parallel_layer(hy_engine* h, const Batch& b, size_t li) {
       o.split = L.n_mix + 2 * ff;
       gemm<AT, WT, AT>(h, hb, W, (const WT*)L.w_in, W, T, L.n_in, W, o);
       if (ff) {
-        gated_act_kernel<AT><<<dim3((ff + 255) / 256, T), 256, 0, s>>>(pin + L.n_mix, h->ld_pin, ff, c.ff_act, c.ff_limit, cat + L.o_ff, h->ld_cat);
+        go_kernel(h, gated_act_kernel<AT>, dim3((ff + 255) / 256, T), 256, 0, s, pin + L.n_mix, h->ld_pin, ff, c.ff_act, c.ff_limit, cat + L.o_ff, h->ld_cat);
         h->launches++;
       }
     }
@@ -2578,27 +2619,28 @@ int run_step(hy_engine* h, const Batch& b, int n_want, const int* want_d, float*
   const float eps = h->m.norm_eps;
   cudaStream_t s = h->stream;
   AT* hb = (AT*)h->hbuf; AT* pin = (AT*)h->pin; AT* cat = (AT*)h->cat; AT* cv = (AT*)h->cv;
+  prepare_units<AT>(h, E, T);
   {
     ProfScope ps(h, HY_PROF_NORM);
     if (h->m.block_kind == HY_BLOCK_PRENORM) {
-      embed_pair_kernel<WT><<<T, 128, 0, s>>>(b, (const WT*)h->embed, h->m.emb_scale, (const WT*)h->pair_table, h->m.pair_buckets,
+      go_kernel(h, embed_pair_kernel<WT>, T, 128, 0, s, b, (const WT*)h->embed, h->m.emb_scale, (const WT*)h->pair_table, h->m.pair_buckets,
                                               h->m.pair_mul_prev, h->m.pair_mul_cur, h->prev_tok, W, h->x, h->kept);
-      prev_token_kernel<<<(E + 127) / 128, 128, 0, s>>>(b, h->prev_tok);
+      go_kernel(h, prev_token_kernel, (E + 127) / 128, 128, 0, s, b, h->prev_tok);
       StreamOp o{};                                            // the first layer's first norm
       o.eps = eps; o.next_w = h->lw[0].pn1; o.next_out = h->hn;
       stream_row<WT>(h, b, o);
       h->launches++;
     } else {
-      embed_kernel<WT><<<T, 128, 0, s>>>(b, (const WT*)h->embed, h->inv_freq, h->m.emb_scale, W, h->x);
+      go_kernel(h, embed_kernel<WT>, T, 128, 0, s, b, (const WT*)h->embed, h->inv_freq, h->m.emb_scale, W, h->x);
     }
     h->launches++;
     if (!h->rot_tables.empty()) {
-      rot_tables_kernel<<<dim3(T, (unsigned)h->rot_tables.size()), 32, 0, s>>>(b, h->rot_tables_d);
+      go_kernel(h, rot_tables_kernel, dim3(T, (unsigned)h->rot_tables.size()), 32, 0, s, b, h->rot_tables_d);
       h->launches++;
     }
     // output-normed blocks read the stream itself: it leaves here in the activation type too, normed when the model says so
     if (h->m.loop_times > 0) {
-      loop_origin_kernel<AT><<<T, 128, 0, s>>>(h->x, W, (AT*)h->loop_cat);
+      go_kernel(h, loop_origin_kernel<AT>, T, 128, 0, s, h->x, W, (AT*)h->loop_cat);
       h->launches++;
     }
     if (h->m.block_kind == HY_BLOCK_POSTNORM) post_norm_add<AT>(h, T, h->x, W, nullptr, nullptr, nullptr, 0, nullptr, h->embed_norm, nullptr, 0);
@@ -2621,7 +2663,7 @@ int run_step(hy_engine* h, const Batch& b, int n_want, const int* want_d, float*
     const int ff = c.ff_kind == HY_FF_NONE ? 0 : c.ff;
     {
       ProfScope ps(h, HY_PROF_NORM);
-      rmsnorm_kernel<WT, AT><<<T, 256, 0, s>>>(h->x, nullptr, (const WT*)L.norm1, eps, W, 1.0f, hb);
+      go_kernel(h, rmsnorm_kernel<WT, AT>, T, 256, 0, s, h->x, nullptr, (const WT*)L.norm1, eps, W, 1.0f, hb);
       h->launches++;
     }
     // every projection that reads the normed input, in one product; the feed-forward's hidden part leaves activated,
@@ -2651,17 +2693,17 @@ int run_step(hy_engine* h, const Batch& b, int n_want, const int* want_d, float*
           tc = true;
 #define HY_ATTN_ARGS b, u->d, cv, h->ld_cv, (const bf16*)L.cache, c.a_heads, c.a_kv_heads, c.a_scale, c.a_qt_coef, \
           c.a_qt_every, 0, u->split, u->ns, c.a_dim, h->part_o, h->part_ml
-          if (c.a_dim == 32) attn_mma_kernel<32><<<u->n, 128, 0, s>>>(HY_ATTN_ARGS);
-          else if (c.a_dim == 64) attn_mma_kernel<64><<<u->n, 128, 0, s>>>(HY_ATTN_ARGS);
-          else attn_mma_kernel<128><<<u->n, 128, 0, s>>>(HY_ATTN_ARGS);
+          if (c.a_dim == 32) go_kernel(h, attn_mma_kernel<32>, u->n, 128, 0, s, HY_ATTN_ARGS);
+          else if (c.a_dim == 64) go_kernel(h, attn_mma_kernel<64>, u->n, 128, 0, s, HY_ATTN_ARGS);
+          else go_kernel(h, attn_mma_kernel<128>, u->n, 128, 0, s, HY_ATTN_ARGS);
 #undef HY_ATTN_ARGS
-          attn_combine_kernel<WT, bf16><<<T * c.a_heads, 64, 0, s>>>(b, h->part_o, h->part_ml, (const WT*)L.sink, pin + L.c_g, h->ld_pin,
+          go_kernel(h, attn_combine_kernel<WT, bf16>, T * c.a_heads, 64, 0, s, b, h->part_o, h->part_ml, (const WT*)L.sink, pin + L.c_g, h->ld_pin,
               c.a_heads, c.a_kv_heads, c.a_dim, c.a_dim, 0, u->split, u->ns, c.left_scale, cat + L.o_mix, h->ld_cat);
           h->launches++;
         }
       }
       if (!tc)
-      attn_sink_kernel<AT, WT, AT><<<(T * c.a_heads + 3) / 4, 128, 4 * c.a_dim * sizeof(float), s>>>(
+      go_kernel(h, attn_sink_kernel<AT, WT, AT>, (T * c.a_heads + 3) / 4, 128, 4 * c.a_dim * sizeof(float), s, 
           b, cv, h->ld_cv, (const AT*)L.cache, (const WT*)L.sink, pin + L.c_g, h->ld_pin, c.a_heads, c.a_kv_heads, c.a_dim, c.a_dim,
           c.a_scale, c.a_qt_coef, c.a_qt_every, 0, c.left_scale, cat + L.o_mix, h->ld_cat);
       }
@@ -2690,7 +2732,7 @@ int run_step(hy_engine* h, const Batch& b, int n_want, const int* want_d, float*
           // 16-byte copies: whole blocks of channels, rows and columns on 16-byte boundaries
           const int v32 = (R | N | h->ld_f1 | h->ld_f2 | I) % 4 == 0 && PB % 4 == 0;
           const int vat = (h->ld_cv | h->ld_pin | L.c_z | I) % ch == 0 && PB % ch == 0;
-          scan_kernel<AT, WT, NPER, LN><<<dim3((I + PB - 1) / PB, E), 128, smem, s>>>(
+          go_kernel(h, scan_kernel<AT, WT, NPER, LN>, dim3((I + PB - 1) / PB, E), 128, smem, s, 
               b, cv, h->ld_cv, pin + L.c_z, h->ld_pin, h->f2, h->ld_f2, (const WT*)L.dt_b, h->f1, h->ld_f1, R, R + N, L.A_neg, (const WT*)L.D, I, N,
               v32 | vat << 1, c.right_scale, L.rec_state, cat + L.o_scan, h->ld_cat);
         };
@@ -2720,7 +2762,7 @@ int run_step(hy_engine* h, const Batch& b, int n_want, const int* want_d, float*
         co.out = cv; co.ldo = h->ld_cv; co.out_lo = 2 * nq; co.out_hi = C;
         co.rows = h->lin; co.G = G; co.n = dk;
         launch_conv<AT>(h, b, pin, h->ld_pin, L.c_q, C, c.d_conv, L.conv_qkv, nullptr, 1, L.conv_state, co);
-        delta_unit_kernel<AT, true><<<(T * G + 3) / 4, 128, 0, s>>>(T, H, G, dk, nullptr, 0, (const float*)L.A_log, (const float*)L.dt_bias,
+        go_kernel(h, delta_unit_kernel<AT, true>, (T * G + 3) / 4, 128, 0, s, T, H, G, dk, nullptr, 0, (const float*)L.A_log, (const float*)L.dt_bias,
                                                                     pin + L.c_b, h->ld_pin, h->f1, h->ld_f1, h->lin, h->lin_sc);
       }
       ProfScope ps(h, HY_PROF_DELTA);
@@ -2730,10 +2772,10 @@ int run_step(hy_engine* h, const Batch& b, int n_want, const int* want_d, float*
         const LinearLaunch g = linear_launch<AT>(PARTS, dk, dv, cv, h->ld_cv);
         const size_t smem = lin_smem<AT>(DR, PARTS, DR + 4);
         cudaFuncSetAttribute(delta_head_kernel<AT, DR, PARTS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        delta_head_kernel<AT, DR, PARTS, true><<<dim3(H * g.bph, E), 128, smem, s>>>(b, h->lin, cv, h->ld_cv, h->lin_sc, H, G, dk, dv, g.bph, g.vec,
+        go_kernel(h, delta_head_kernel<AT, DR, PARTS, true>, dim3(H * g.bph, E), 128, smem, s, b, h->lin, cv, h->ld_cv, h->lin_sc, H, G, dk, dv, g.bph, g.vec,
                                                                                      g.vvec, L.rec_state, o, h->ld_f2, h->f1, h->ld_f1);
       });
-      gla_out_kernel<AT, float, GATE_SIGMOID><<<(T * H + 3) / 4, 128, 0, s>>>(T, H, dv, o, h->ld_f2, h->f2, h->ld_f2, (const float*)L.norm_w, eps,
+      go_kernel(h, gla_out_kernel<AT, float, GATE_SIGMOID>, (T * H + 3) / 4, 128, 0, s, T, H, dv, o, h->ld_f2, h->f2, h->ld_f2, (const float*)L.norm_w, eps,
                                                                               1.0f, cat + L.o_mix, h->ld_cat);
       h->launches += 3;
     }
@@ -2750,8 +2792,8 @@ int run_step(hy_engine* h, const Batch& b, int n_want, const int* want_d, float*
   }
   if (n_want > 0) {
     ProfScope ps(h, HY_PROF_HEAD);
-    if (h->m.norm_kind == HY_NORM_TANH) tanh_norm_kernel<AT><<<n_want, 256, 0, s>>>(h->x, want_d, h->final_tanh, W, (AT*)h->hw);
-    else rmsnorm_kernel<WT, AT><<<n_want, 256, 0, s>>>(h->x, want_d, (const WT*)h->final_norm, eps, W,
+    if (h->m.norm_kind == HY_NORM_TANH) go_kernel(h, tanh_norm_kernel<AT>, n_want, 256, 0, s, h->x, want_d, h->final_tanh, W, (AT*)h->hw);
+    else go_kernel(h, rmsnorm_kernel<WT, AT>, n_want, 256, 0, s, h->x, want_d, (const WT*)h->final_norm, eps, W,
                                                        h->m.norm_kind == HY_NORM_RMS ? 0.0f : 1.0f, (AT*)h->hw);
     h->launches++;
     GemmOut o = to_buf(h->logits, h->m.vocab);
@@ -2813,7 +2855,7 @@ extern "C" int hy_step(hy_handle h, int32_t n_entries, const int32_t* tokens, co
   b.ent_slot = b.ent_pos0 + E; b.pages = b.ent_slot + E;
   b.T = T; b.E = E; b.max_pages = rt.max_pages_per_seq; b.page_size = rt.page_size;
   const int* want_d = b.pages + (size_t)E * rt.max_pages_per_seq;
-  h->step_start = ent_start; h->step_pos0 = ent_pos0; h->units_used = 0; h->unit_lists.clear();
+  h->step_start = ent_start; h->step_pos0 = ent_pos0; h->step_tokens = T; h->units_used = 0; h->unit_lists.clear();
   HY_CUDA(cudaEventRecord(h->ev0, h->stream));
   if (h->m.dtype == HY_DTYPE_F32) run_step<float>(h, b, n_want, want_d, layers_out);
   else run_step<__nv_bfloat16>(h, b, n_want, want_d, layers_out);
@@ -2823,7 +2865,7 @@ extern "C" int hy_step(hy_handle h, int32_t n_entries, const int32_t* tokens, co
       HY_CUDA(cudaMemcpyAsync(h->temp_d, temperature, (size_t)n_want * 4, cudaMemcpyHostToDevice, h->stream));
       td = h->temp_d;
     }
-    sample_kernel<<<n_want, 1024, 0, h->stream>>>(h->logits, h->m.vocab, td, seed, h->sampled);
+    go_kernel(h, sample_kernel, n_want, 1024, 0, h->stream, h->logits, h->m.vocab, td, seed, h->sampled);
     h->launches++;
     HY_CUDA(cudaMemcpyAsync(sampled_out, h->sampled, (size_t)n_want * 4, cudaMemcpyDeviceToHost, h->stream));
   }

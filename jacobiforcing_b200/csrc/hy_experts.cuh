@@ -21,6 +21,7 @@ struct RouteCfg { int experts, top, groups, keep; float scale; };
 // A group is worth the sum of its two best scores (its single score when groups hold one expert).
 __global__ void __launch_bounds__(32) route_kernel(const float* __restrict__ logits, int ldl, RouteCfg c, int* __restrict__ ids,
                                                    float* __restrict__ wts, int* __restrict__ counts) {
+  pdl_begin();
   extern __shared__ __align__(16) unsigned char hy_smem[];
   float* s = reinterpret_cast<float*>(hy_smem);                // [experts] scores, negated once chosen
   float* gs = s + c.experts;                                   // [groups]; -1 once kept
@@ -66,6 +67,7 @@ __global__ void __launch_bounds__(32) route_kernel(const float* __restrict__ log
 __global__ void __launch_bounds__(32) route_top_kernel(const float* __restrict__ logits, int ldl, const float* __restrict__ bias,
                                                        int experts, int top, int* __restrict__ ids, float* __restrict__ wts,
                                                        int* __restrict__ counts) {
+  pdl_begin();
   extern __shared__ __align__(16) unsigned char hy_smem[];
   float* s = reinterpret_cast<float*>(hy_smem);                // [experts] logits, -inf once chosen
   const int t = blockIdx.x, lane = threadIdx.x;
@@ -95,6 +97,7 @@ __global__ void __launch_bounds__(32) route_top_kernel(const float* __restrict__
 __global__ void __launch_bounds__(32) route_corrected_kernel(const float* __restrict__ logits, int ldl, const float* __restrict__ correction,
                                                              int experts, int outputs, int top, int groups, int keep, int* __restrict__ ids,
                                                              float* __restrict__ wts, int* __restrict__ counts) {
+  pdl_begin();
   extern __shared__ __align__(16) unsigned char hy_smem[];
   float* s = reinterpret_cast<float*>(hy_smem);                // [outputs] scores
   float* ch = s + outputs;                                     // [outputs] choice scores, -inf once chosen
@@ -148,6 +151,7 @@ __global__ void __launch_bounds__(32) route_corrected_kernel(const float* __rest
 // out[t, f] = act(in[t, f]) * in[t, n + f] (or the clamped pair, see gated_pair_f): the gated pair of a dense feed-forward whose gate and up rows are stacked.
 template <typename AT>
 __global__ void gated_act_kernel(const AT* __restrict__ in, int ldi, int n, int act, float limit, AT* __restrict__ out, int ldo) {
+  pdl_begin();
   const int t = blockIdx.y;
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
   if (f < n) out[(size_t)t * ldo + f] = from_f<AT>(gated_pair_f(act, to_f(in[(size_t)t * ldi + f]), to_f(in[(size_t)t * ldi + n + f]), limit));
@@ -168,6 +172,7 @@ __global__ void __launch_bounds__(128) route_place_kernel(int pairs, int top, in
                                                           int width, int vec, int* __restrict__ offs, int* __restrict__ tile_expert,
                                                           int* __restrict__ tile_row0, int* __restrict__ meta, int* __restrict__ pair_row,
                                                           AT* __restrict__ rows) {
+  pdl_begin();
   const int i = blockIdx.x, lane = threadIdx.x & 31;
   if (i == pairs) {
     for (int e = threadIdx.x; e < most_experts; e += blockDim.x) { old_counts[e] = 0; old_fill[e] = 0; }
@@ -221,6 +226,7 @@ __global__ void __launch_bounds__(256) expert_gemm_simt_kernel(const TA* __restr
                                                                const int* __restrict__ offs, const int* __restrict__ tile_expert,
                                                                const int* __restrict__ tile_row0, const int* __restrict__ meta,
                                                                TO* __restrict__ out, int ldo, int act, float limit) {
+  pdl_begin();
   constexpr int BM = HY_XT, BN = 64, BK = 16;
   __shared__ float As[BK][BM + 4];
   __shared__ float Ws[GLU ? 2 : 1][BK][BN + 4];
@@ -287,6 +293,7 @@ template <typename TA, typename TW, typename TO, bool GLU>
 __global__ void __launch_bounds__(256) expert_rows_kernel(const TA* __restrict__ A, int lda, const int* __restrict__ ids, int top,
                                                           int a_per_token, int experts, const TW* __restrict__ W, size_t w_stride,
                                                           int N, int K, TO* __restrict__ out, int ldo, int act, float limit) {
+  pdl_begin();
   extern __shared__ __align__(16) unsigned char hy_smem[];
   TA* As = reinterpret_cast<TA*>(hy_smem);
   constexpr int VEC = 16 / sizeof(TW);
@@ -336,6 +343,7 @@ __global__ void expert_combine_kernel(const float* __restrict__ rows, int ldr, c
                                       const float* __restrict__ wts, int top, int width, TanhNorm post,
                                       const float* __restrict__ ls, float* __restrict__ x, TanhNorm next,
                                       AT* __restrict__ next_out) {
+  pdl_begin();
   const int t = blockIdx.x;
   for (int c = threadIdx.x; c < width; c += blockDim.x) {
     float y = 0.0f;

@@ -211,8 +211,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
   constexpr int TP_STAGES = tp_stages(BT), XTILE = BT / 2 * 128, SLOT = TC_WTILE + XTILE;
   TpSmem* sm = reinterpret_cast<TpSmem*>(base + TP_STAGES * SLOT);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rank = (int)tp_rank();
-  const int KT = (K + 63) / 64, nx = (N + 255) / 256, ny = grp.meta ? grp.meta[0] : (T + BT - 1) / BT;
-  const int tiles = nx * ny, first = blockIdx.x >> 1, step = gridDim.x >> 1;
+  const int KT = (K + 63) / 64, nx = (N + 255) / 256, first = blockIdx.x >> 1, step = gridDim.x >> 1;
+  pdl_trigger();
   if (threadIdx.x == 0) {
     for (int i = 0; i < TP_STAGES; ++i) { jf::mbar_init(&sm->full[i], 1); jf::mbar_init(&sm->empty[i], 1); }
     for (int i = 0; i < 2; ++i) { jf::mbar_init(&sm->acc_full[i], 1); jf::mbar_init(&sm->acc_empty[i], 16); }
@@ -227,6 +227,18 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
   __syncthreads();
   tp_cluster_sync();
   jf::tc_fence_after();
+  // the weight tiles of the first stages travel while the kernel before this one ends (which tile is the first is known when the
+  // tiles are not a list that it makes)
+  int ahead = 0;
+  if (warp == 0 && lane == 0 && !grp.meta) {
+    const int x = first / ((T + BT - 1) / BT);
+    for (; ahead < min(TP_STAGES, KT); ++ahead) {
+      if (rank == 0) jf::mbar_expect_tx(&sm->full[ahead], 2 * SLOT);
+      tp_load(base + ahead * SLOT, &wmap, 0, ((2 * x + rank) * KT + ahead) * 128, tp_in_first(&sm->full[ahead]));
+    }
+  }
+  pdl_wait();
+  const int ny = grp.meta ? grp.meta[0] : (T + BT - 1) / BT, tiles = nx * ny;
   // token tile and feature tile of a tile number: neighbours share the weight rows (grouped: the expert's activation rows)
   auto place = [&](int tile, int& x, int& y) {
     if (grp.meta) { x = tile % nx; y = tile / nx; }
@@ -246,9 +258,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
           const int s = it % TP_STAGES;
           ok = tp_wait(&sm->empty[s], ((it / TP_STAGES) & 1) ^ 1, sm, err);      // the products that read the slot retired
           if (!ok) break;
-          if (rank == 0) jf::mbar_expect_tx(&sm->full[s], 2 * SLOT);
           const uint32_t bar = tp_in_first(&sm->full[s]);
-          tp_load(base + s * SLOT, &wmap, 0, w0 + kt * 128, bar);
+          if (it >= ahead) {
+            if (rank == 0) jf::mbar_expect_tx(&sm->full[s], 2 * SLOT);
+            tp_load(base + s * SLOT, &wmap, 0, w0 + kt * 128, bar);
+          }
           tp_load(base + s * SLOT + TC_WTILE, &xmap, kt * 64, t0, bar);
         }
       }

@@ -35,7 +35,8 @@ template <typename AT, int DR, int PARTS, int MODE>
 __global__ void __launch_bounds__(128) gla_kernel(Batch b, const float* __restrict__ qk, const AT* __restrict__ v, int ldv,
                                                   const float* __restrict__ decay, int ldd, const float* __restrict__ head_decay, int H,
                                                   int dim, int vdim, int blocks_per_head, int vec, int vvec, float* __restrict__ state,
-                                                  float* __restrict__ o, int ldo, GlaToken tk = GlaToken{}) {
+                                                  float* __restrict__ o, int ldo, GlaToken tk) {
+  pdl_begin();
   constexpr int TB = lin_tb(DR), RP = DR / PARTS, CW = 32 / PARTS, CPB = lin_cpb(PARTS), VW = CPB < 8 ? 8 : CPB;
   constexpr bool HEAD = MODE == GLA_HEAD;
   constexpr int RW = MODE == GLA_CHANNEL ? 3 * DR : 2 * DR;    // floats of a staged row: q | k (| decays)
@@ -170,6 +171,7 @@ template <typename AT>
 __global__ void __launch_bounds__(1024) forget_rows_kernel(const AT* __restrict__ in, int ld, int col_q, int col_f,
                                                            const float* __restrict__ f_bias, const float* __restrict__ lower, int H, int dim,
                                                            float* __restrict__ qf) {
+  pdl_begin();
   const AT* row = in + (size_t)blockIdx.x * ld;
   float* out = qf + (size_t)blockIdx.x * H * 2 * dim;
   for (int i = threadIdx.x; i < H * dim; i += blockDim.x) {
@@ -187,6 +189,7 @@ template <typename AT, typename GT = AT, int GATE = GATE_SILU>
 __global__ void __launch_bounds__(128) gla_out_kernel(int T, int H, int vdim, const float* __restrict__ o, int ldi,
                                                       const GT* __restrict__ g, int ldg, const float* __restrict__ w, float eps,
                                                       float out_scale, AT* __restrict__ out, int ldo) {
+  pdl_begin();
   const int unit = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (unit >= T * H) return;
   const size_t t = unit / H, c0 = (size_t)(unit % H) * vdim;
@@ -219,6 +222,7 @@ struct RowClose {
 constexpr int HY_CLOSE_TOP = 64;                               // choices whose rows and weights are staged in shared memory
 template <typename AT, typename WT, int V>
 __global__ void __launch_bounds__(256) row_close_kernel(RowClose c, int width, float* __restrict__ x, AT* h) {
+  pdl_begin();
   typedef VecN<float, V> F;
   extern __shared__ __align__(16) unsigned char hy_smem[];
   float* xs = reinterpret_cast<float*>(hy_smem);               // [width]
@@ -307,6 +311,7 @@ __global__ void __launch_bounds__(256) row_close_kernel(RowClose c, int width, f
 // The embedding output x0 into the second half of the loop projection's operand [T, 2 width].
 template <typename AT>
 __global__ void loop_origin_kernel(const float* __restrict__ x, int width, AT* __restrict__ out) {
+  pdl_begin();
   const int t = blockIdx.x;
   for (int c = threadIdx.x; c < width; c += blockDim.x) out[(size_t)t * 2 * width + width + c] = from_f<AT>(x[(size_t)t * width + c]);
 }

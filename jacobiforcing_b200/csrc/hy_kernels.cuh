@@ -17,6 +17,13 @@ namespace hy {
 
 typedef __nv_bfloat16 bf16;
 
+// Programmatic dependent launch: every kernel of a step may start while the one before it still runs (see go_kernel) and must not
+// touch anything that an earlier kernel reads or writes before pdl_wait.  What comes before it (weights, which nothing
+// writes; barriers, tensor memory) overlaps the end of the kernel before.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_begin() { pdl_trigger(); pdl_wait(); }
+
 template <typename T> __device__ __forceinline__ float to_f(T v);
 template <> __device__ __forceinline__ float to_f<float>(float v) { return v; }
 template <> __device__ __forceinline__ float to_f<bf16>(bf16 v) { return __bfloat162float(v); }
@@ -91,6 +98,7 @@ struct Batch {
 template <typename WT>
 __global__ void embed_kernel(Batch b, const WT* __restrict__ table, const double* __restrict__ inv_freq, float scale,
                              int width, float* __restrict__ x) {
+  pdl_begin();
   const int t = blockIdx.x;
   const int tok = b.tok[t];
   const double p = (double)b.tok_pos[t];
@@ -110,6 +118,7 @@ struct TanhNorm { const float* w; const float* b; float alpha; };
 template <typename OT>
 __global__ void tanh_norm_kernel(const float* __restrict__ x, const int* __restrict__ rows, TanhNorm n, int width,
                                  OT* __restrict__ out) {
+  pdl_begin();
   const int r = blockIdx.x;
   const float* xr = x + (size_t)(rows ? rows[r] : r) * width;
   for (int c = threadIdx.x; c < width; c += blockDim.x)
@@ -121,6 +130,7 @@ __global__ void tanh_norm_kernel(const float* __restrict__ x, const int* __restr
 template <typename WT, typename OT>
 __global__ void rmsnorm_kernel(const float* __restrict__ x, const int* __restrict__ rows, const WT* __restrict__ w,
                                float eps, int width, float w_offset, OT* __restrict__ out) {
+  pdl_begin();
   __shared__ float red[33];
   const int r = blockIdx.x;
   const float* xr = x + (size_t)(rows ? rows[r] : r) * width;
@@ -191,6 +201,7 @@ __global__ void post_norm_add_kernel(const float* ybuf, int ldy, const float* __
                                      const float* __restrict__ shared_rows, const float* __restrict__ w,
                                      const float* __restrict__ ls, float eps, int width, int add, float* x,
                                      AT* __restrict__ next_out) {
+  pdl_begin();
   extern __shared__ __align__(16) unsigned char hy_smem[];
   float* ys = reinterpret_cast<float*>(hy_smem);               // [width]
   __shared__ float red[33];
@@ -225,6 +236,7 @@ __global__ void post_norm_add_kernel(const float* ybuf, int ldy, const float* __
 template <typename TA, typename TW, typename TO>
 __global__ void __launch_bounds__(256) gemm_simt_kernel(const TA* __restrict__ A, int lda, const TW* __restrict__ W, int ldw,
                                                         int T, int N, int K, GemmOut o) {
+  pdl_begin();
   constexpr int BM = 64, BN = 64, BK = 16;
   __shared__ float As[BK][BM + 4];
   __shared__ float Ws[BK][BN + 4];
@@ -282,6 +294,28 @@ __global__ void __launch_bounds__(256) gemm_rows_kernel(const TA* __restrict__ A
   constexpr int VEC = 16 / sizeof(TW);
   const int Kp = (K + VEC - 1) / VEC * VEC;
   const int t0 = blockIdx.y * ROWS;
+  pdl_trigger();
+  // ksplit warps share a column (long k, few columns: more loads in flight); their sums are added in part order
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int cpb = 8 / ksplit, part = warp % ksplit, cib = warp / ksplit;
+  const int Kc = ((K + ksplit - 1) / ksplit + 32 * VEC - 1) / (32 * VEC) * (32 * VEC);
+  const int lo = part * Kc, hi = min(K, lo + Kc), kv = min(hi, K / VEC * VEC);
+  // the first AHEAD vectors of a column travel while the columns before it are summed up; those of the warp's first column while the
+  // kernel before this one ends (weights do not depend on it)
+  constexpr int AHEAD = 4;
+  VecN<TW, VEC> w0[AHEAD];
+  auto fetch = [&](int n) {
+    const TW* wr = W + (size_t)n * ldw;
+    if (n < N && (reinterpret_cast<uintptr_t>(wr) & 15) == 0) {
+#pragma unroll
+      for (int i = 0; i < AHEAD; ++i) {
+        const int k = lo + (lane + 32 * i) * VEC;
+        if (k < kv) w0[i] = *reinterpret_cast<const VecN<TW, VEC>*>(wr + k);
+      }
+    }
+  };
+  fetch(blockIdx.x * cpb + cib);
+  pdl_wait();
   constexpr int VA = 16 / sizeof(TA);
   if (K % VA == 0 && lda % VA == 0 && (reinterpret_cast<uintptr_t>(A) & 15) == 0 && Kp == K) {
     const int kv = K / VA;                                     // 16 bytes per thread per load
@@ -298,11 +332,6 @@ __global__ void __launch_bounds__(256) gemm_rows_kernel(const TA* __restrict__ A
     }
   }
   __syncthreads();
-  // ksplit warps share a column (long k, few columns: more loads in flight); their sums are added in part order
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int cpb = 8 / ksplit, part = warp % ksplit, cib = warp / ksplit;
-  const int Kc = ((K + ksplit - 1) / ksplit + 32 * VEC - 1) / (32 * VEC) * (32 * VEC);
-  const int lo = part * Kc, hi = min(K, lo + Kc);
   for (int base = blockIdx.x * cpb; base < N; base += gridDim.x * cpb) {
     const int n = base + cib;
     float acc[ROWS];
@@ -313,17 +342,22 @@ __global__ void __launch_bounds__(256) gemm_rows_kernel(const TA* __restrict__ A
       const bool vec_ok = ((reinterpret_cast<uintptr_t>(wr) & 15) == 0);
       int kdone = lo;
       if (vec_ok) {
-        const int kv = min(hi, K / VEC * VEC);
-#pragma unroll 4
-        for (int k = lo + lane * VEC; k < kv; k += 32 * VEC) {
-          const VecN<TW, VEC> wv = *reinterpret_cast<const VecN<TW, VEC>*>(wr + k);
+        auto add = [&](const VecN<TW, VEC>& wv, int k) {
 #pragma unroll
           for (int r = 0; r < ROWS; ++r) {
             const VecN<TA, VEC> av = *reinterpret_cast<const VecN<TA, VEC>*>(As + r * Kp + k);
 #pragma unroll
             for (int j = 0; j < VEC; ++j) acc[r] = fmaf(to_f(av.v[j]), to_f(wv.v[j]), acc[r]);
           }
+        };
+#pragma unroll
+        for (int i = 0; i < AHEAD; ++i) {
+          const int k = lo + (lane + 32 * i) * VEC;
+          if (k < kv) add(w0[i], k);
         }
+        fetch(n + gridDim.x * cpb);
+#pragma unroll 4
+        for (int k = lo + (lane + 32 * AHEAD) * VEC; k < kv; k += 32 * VEC) add(*reinterpret_cast<const VecN<TW, VEC>*>(wr + k), k);
         kdone = max(lo, kv);
       }
       for (int k = kdone + lane; k < hi; k += 32) {
@@ -381,6 +415,7 @@ constexpr int HY_CONV_TT = 16;                                 // tokens per thr
 template <typename AT, typename WT, int V, int TAPS>
 __global__ void __launch_bounds__(128) conv_kernel(Batch b, const AT* __restrict__ u, int ldu, int col0, int C, int taps_, const WT* __restrict__ w,
                                                    const WT* __restrict__ bias, int act_silu, float* __restrict__ state, ConvOut<AT> o) {
+  pdl_begin();
   const int taps = TAPS ? TAPS : taps_;
   int e = 0, chunk = blockIdx.y, start, cnt;
   for (;; ++e) {                                               // entry and chunk of this block
@@ -462,6 +497,7 @@ __global__ void __launch_bounds__(128) conv_kernel(Batch b, const AT* __restrict
 // New tail = the last taps - 1 of (old tail ++ this entry's inputs).  Runs after the convolution of the same step.
 template <typename AT>
 __global__ void conv_tail_kernel(Batch b, const AT* __restrict__ u, int ldu, int col0, int C, int taps, float* __restrict__ state) {
+  pdl_begin();
   const int e = blockIdx.y;
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= C) return;
@@ -495,6 +531,7 @@ __global__ void __launch_bounds__(128) attn_sink_kernel(Batch b, const AT* __res
                                                         const WT* __restrict__ sink, const AT* __restrict__ gate, int ldg,
                                                         int H, int G, int dim, int vdim, float scale, float qt_coef,
                                                         int qt_every, int window, float out_scale, OT* __restrict__ out, int ldo) {
+  pdl_begin();
   extern __shared__ __align__(16) unsigned char hy_smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float* qs = reinterpret_cast<float*>(hy_smem) + warp * dim;
@@ -575,6 +612,7 @@ __global__ void __launch_bounds__(128) scan_kernel(Batch b, const AT* __restrict
                                                    const float* __restrict__ low, int ldl, int col_b, int col_c,
                                                    const float* __restrict__ A, const WT* __restrict__ D, int inner, int nstate,
                                                    int vec, float out_scale, float* __restrict__ state, AT* __restrict__ out, int ldo) {
+  pdl_begin();
   constexpr int NP = NPER * L, PB = 128 / L, TB = scan_tb(NP), TG = 8, CH = 16 / (int)sizeof(AT);
   extern __shared__ __align__(16) unsigned char hy_smem[];
   float* sB = reinterpret_cast<float*>(hy_smem);               // [2][TB][NP]
@@ -742,6 +780,7 @@ __device__ __forceinline__ uint32_t mix32(uint64_t key, uint32_t ctr) {
 // independent loads 10 us.
 __global__ void __launch_bounds__(1024) sample_kernel(const float* __restrict__ logits, int vocab, const float* __restrict__ temperature,
                                                       uint64_t seed, int* __restrict__ out) {
+  pdl_begin();
   __shared__ float bv[32];
   __shared__ int bi[32];
   const int r = blockIdx.x;

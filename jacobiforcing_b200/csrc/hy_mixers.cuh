@@ -48,6 +48,7 @@ template <typename AT>
 __global__ void gated_group_norm_kernel(const float* __restrict__ y, int ldy, const AT* __restrict__ z, int ldz,
                                         const float* __restrict__ w, int inner, int parts, float eps, AT* __restrict__ out,
                                         int ldo) {
+  pdl_begin();
   __shared__ float red[33];
   const int t = blockIdx.x, part = blockIdx.y, n = inner / parts, c0 = part * n;
   float ss = 0.0f;
@@ -74,6 +75,7 @@ template <typename AT>
 __global__ void latent_prep_kernel(Batch b, const float* __restrict__ d, int ldd, int q_rank, int rank, int rot, int own_kv,
                                    const float* __restrict__ qn_w, const float* __restrict__ kn_w, float eps, Rotation r,
                                    AT* __restrict__ cq, int ldq, AT* __restrict__ cache) {
+  pdl_begin();
   extern __shared__ __align__(16) unsigned char hy_smem[];
   float* cs = reinterpret_cast<float*>(hy_smem);              // [2 * pairs]
   __shared__ float red[33];
@@ -111,6 +113,7 @@ template <typename AT, typename WT>
 __global__ void __launch_bounds__(128) latent_query_kernel(Batch b, const AT* __restrict__ q, int ldq, const WT* __restrict__ w_uk,
                                                            int H, int dim, int rot, int rank, int fold, Rotation r,
                                                            AT* __restrict__ out, int ldo) {
+  pdl_begin();
   extern __shared__ __align__(16) unsigned char hy_smem[];
   float* qs = reinterpret_cast<float*>(hy_smem);              // [TB][dim]
   float* cs = qs + HY_LAT_TB * dim;                           // [2 * pairs] of one token at a time
@@ -151,6 +154,7 @@ template <typename AT, typename WT>
 __global__ void __launch_bounds__(128) latent_value_kernel(int T, const float* __restrict__ o, int ldi, const WT* __restrict__ w_uvT,
                                                            int H, int rank, int vdim, const AT* __restrict__ gate, int ldg,
                                                            AT* __restrict__ out, int ldo) {
+  pdl_begin();
   extern __shared__ __align__(16) unsigned char hy_smem[];
   float* os = reinterpret_cast<float*>(hy_smem);              // [TB][rank]
   const int t0 = blockIdx.x * HY_LAT_TB, h = blockIdx.y, nb = min(HY_LAT_TB, T - t0);
@@ -183,7 +187,8 @@ __global__ void __launch_bounds__(128) latent_value_kernel(int T, const float* _
 template <typename TI, typename TW, typename TO>
 __global__ void __launch_bounds__(256) head_rows_kernel(int T, const TI* __restrict__ in, int ldi, int in_hs, const TW* __restrict__ w,
                                                         int H, int N, int K, TO* __restrict__ out, int ldo, int out_hs,
-                                                        const TO* __restrict__ gate = nullptr, int ldg = 0) {
+                                                        const TO* __restrict__ gate, int ldg) {
+  pdl_begin();
   constexpr int VEC = 16 / sizeof(TW);
   const int lane = threadIdx.x & 31;
   const int id = blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -235,6 +240,7 @@ __global__ void __launch_bounds__(256)
 glr_kernel(Batch b, const AT* __restrict__ in, int ld, int col_q, int col_f, int col_v, const float* __restrict__ f_bias,
            const float* __restrict__ lower, const float* __restrict__ norm_w, int H, int dim, int vdim, float eps,
            float* __restrict__ state, AT* __restrict__ out, int ldo) {
+  pdl_begin();
   extern __shared__ __align__(16) unsigned char hy_smem[];
   float* S = reinterpret_cast<float*>(hy_smem);                // [dim][vdim]
   float* qs = S + (size_t)dim * vdim;                          // [dim]
@@ -295,6 +301,7 @@ mlstm_reg_kernel(Batch b, const AT* __restrict__ in, int ld, int col_q, int col_
                  const float* __restrict__ gates, int ldg, int col_i, int col_f, const float* __restrict__ i_bias,
                  const float* __restrict__ f_bias, const float* __restrict__ norm_w, int H, int dim, int vdim, float cap,
                  float eps, int async_ok, float* __restrict__ state, AT* __restrict__ out, int ldo) {
+  pdl_begin();
   extern __shared__ __align__(16) unsigned char hy_smem[];
   constexpr int TB = mlstm_tb(DR), CH = 16 / (int)sizeof(AT);  // elements per 16-byte copy
   const int nt = blockDim.x, nwarps = nt >> 5;
@@ -441,6 +448,7 @@ mlstm_kernel(Batch b, const AT* __restrict__ in, int ld, int col_q, int col_k, i
              const float* __restrict__ gates, int ldg, int col_i, int col_f, const float* __restrict__ i_bias,
              const float* __restrict__ f_bias, const float* __restrict__ norm_w, int H, int dim, int vdim, float cap, float eps,
              float* __restrict__ state, AT* __restrict__ out, int ldo) {
+  pdl_begin();
   extern __shared__ __align__(16) unsigned char hy_smem[];
   const int vs = vdim + 1;
   float* S = reinterpret_cast<float*>(hy_smem);                // [dim][vs]

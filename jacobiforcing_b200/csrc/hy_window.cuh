@@ -40,6 +40,7 @@ __global__ void __launch_bounds__(128) window_prep_kernel(Batch b, const AT* __r
                                                           WindowCfg c, const float* __restrict__ qn, const float* __restrict__ kn,
                                                           float eps, Rotation rot, Rotation rot_v, AT* __restrict__ q_out, int ldq,
                                                           AT* __restrict__ kc, AT* __restrict__ vc, float* __restrict__ vrot, int ldv) {
+  pdl_begin();
   extern __shared__ __align__(16) unsigned char hy_smem[];
   float* cs = reinterpret_cast<float*>(hy_smem);               // [2 * rot.pairs]
   float* csv = cs + 2 * rot.pairs;                             // [2 * rot_v.pairs]
@@ -91,6 +92,7 @@ __global__ void __launch_bounds__(128) window_prep_kernel(Batch b, const AT* __r
 template <typename AT>
 __global__ void __launch_bounds__(128) window_pool_kernel(Batch b, WindowCfg c, const AT* __restrict__ kc, const AT* __restrict__ vc,
                                                           AT* __restrict__ kp, AT* __restrict__ vp) {
+  pdl_begin();
   const int e = blockIdx.y;
   const int pos0 = b.ent_pos0[e], end = pos0 + b.ent_start[e + 1] - b.ent_start[e];
   const int blk = pos0 / c.pool + blockIdx.x;
@@ -119,6 +121,7 @@ __global__ void __launch_bounds__(128) window_attn_kernel(Batch b, const AT* __r
                                                           const AT* __restrict__ kc, const AT* __restrict__ vc,
                                                           const AT* __restrict__ kp, const AT* __restrict__ vp,
                                                           const float* __restrict__ vrot, int ldv, OT* __restrict__ out, int ldo) {
+  pdl_begin();
   extern __shared__ __align__(16) unsigned char hy_smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float* qs = reinterpret_cast<float*>(hy_smem) + warp * c.dim;
@@ -210,6 +213,7 @@ __global__ void __launch_bounds__(128) window_mma_kernel(Batch b, const AttnUnit
                                                          const bf16* __restrict__ vc, const bf16* __restrict__ kp,
                                                          const bf16* __restrict__ vp, const float* __restrict__ vrot, int ldv,
                                                          bf16* __restrict__ out, int ldo) {
+  pdl_begin();
   constexpr int LD = DP + 8;                            // padded row (elements): ldmatrix rows fall into distinct banks
   extern __shared__ __align__(16) unsigned char hy_smem[];
   bf16* kbuf = reinterpret_cast<bf16*>(hy_smem);        // [2][64 * LD] key tiles: one in use, one in flight
