@@ -26,6 +26,7 @@
 #include "hy_biased.cuh"
 #include "hy_delta.cuh"
 #include "hy_gla.cuh"
+#include "jf_flash.cuh"
 
 namespace hy {
 
@@ -62,6 +63,7 @@ struct LayerW {
   // attention over a shared latent
   float* l_qn = nullptr; float* l_kn = nullptr;
   void* w_uq = nullptr; void* w_uq_t = nullptr; void* w_uk = nullptr; void* w_uvT = nullptr;
+  void* w_kv_t = nullptr;                                 // both up-projections as one product of the cache rows (prompt steps)
   void* w_ukT = nullptr; void* w_uv = nullptr;            // [H][rank][dim] and [H][vdim][rank]: the few-row kernel's layouts
   Rotation rot{};
   // gated linear recurrence
@@ -159,6 +161,12 @@ struct hy_engine {
   AttnUnit* units_d = nullptr; AttnUnit* units_h = nullptr; size_t units_cap = 0, units_used = 0;
   std::vector<UnitList> unit_lists;
   int step_tokens = 0;
+  // prompt steps of latent attention: keys of a step's requests one after the other (cache rows, then per-head keys and values),
+  // row units and the requests' first rows for the kernels
+  void* kv_rows = nullptr; void* kv_heads = nullptr; int kv_cap = 0;
+  unsigned char* fl_h = nullptr; unsigned char* fl_d = nullptr; size_t fl_cap = 0, fl_used = 0;
+  struct FlashList { int H; const jf::FlashUnit* units; const int* key_off; int n, keys; };
+  std::vector<FlashList> fl_lists;
   // cosines and sines of the step's positions, one table per distinct rotation: the layer configuration that names it, the table,
   // its column count; rot_tables_d is what the kernel reads
   struct RotEntry { hy_layer_cfg c; RotTable t; };
@@ -372,6 +380,7 @@ extern "C" void hy_destroy(hy_handle h) {
   for (void* p : h->allocs) cudaFree(p);
   if (h->meta_h) cudaFreeHost(h->meta_h);
   if (h->units_h) cudaFreeHost(h->units_h);
+  if (h->fl_h) cudaFreeHost(h->fl_h);
   if (h->err_h) cudaFreeHost(h->err_h);
   cudaEventDestroy(h->ev0);
   cudaEventDestroy(h->ev1);
@@ -577,6 +586,12 @@ int load_gated_experts(hy_engine* h, Builder& B, LayerW& L, const hy_layer_cfg& 
   return B.rc;
 }
 
+// Whether prompt steps of a latent-attention layer may run over per-head keys and values (head sizes that jf::flash_kernel is built for).
+bool latent_prompt_sizes(const hy_engine* h, const hy_layer_cfg& c) {
+  const int hk = c.l_dim + c.l_rot_dim;
+  return h->m.dtype == HY_DTYPE_BF16 && (hk == 64 || hk == 128 || hk == 192) && (c.l_vdim == 64 || c.l_vdim == 128) && (c.l_kv_rank + c.l_rot_dim) % 8 == 0;
+}
+
 // What follows the down-projections of a latent-attention layer: the key and value up-projections in the layouts of their
 // kernels, the sinks, the rotation's frequencies.
 int load_latent_up(hy_engine* h, Builder& B, LayerW& L, const hy_layer_cfg& c, const std::string& d) {
@@ -596,6 +611,21 @@ int load_latent_up(hy_engine* h, Builder& B, LayerW& L, const hy_layer_cfg& c, c
       for (int j = 0; j < c.l_vdim; ++j)
         for (int r = 0; r < R; ++r) tr[((size_t)hh * R + r) * c.l_vdim + j] = t->v[((size_t)hh * c.l_vdim + j) * R + r];
     L.w_uvT = B.up(tr);
+  }
+  if (latent_prompt_sizes(h, c)) {
+    // rows [key head h: dim rows of the key up-projection, then rot rows that pass the rotated part on | values of all heads], columns
+    // [latent | rotated part]
+    const HostTensor* uk = B.get(d + "uk", H * c.l_dim, R);
+    const HostTensor* uv = B.get(d + "uv", H * c.l_vdim, R);
+    if (B.rc != HY_OK) return B.rc;
+    const int rot = c.l_rot_dim, K = R + rot, hk = c.l_dim + rot, N = H * (hk + c.l_vdim);
+    std::vector<float> w((size_t)N * K, 0.0f);
+    for (int hh = 0; hh < H; ++hh) {
+      for (int k = 0; k < c.l_dim; ++k) memcpy(&w[((size_t)hh * hk + k) * K], &uk->v[((size_t)hh * c.l_dim + k) * R], (size_t)R * 4);
+      for (int k = 0; k < rot; ++k) w[((size_t)hh * hk + c.l_dim + k) * K + R + k] = 1.0f;
+    }
+    for (int j = 0; j < H * c.l_vdim; ++j) memcpy(&w[((size_t)H * hk + j) * K], &uv->v[(size_t)j * R], (size_t)R * 4);
+    L.w_kv_t = B.up_tiled(w, N, K);
   }
   if (!c.l_no_sink) { if (auto t = B.get(d + "sink", H, -1)) L.sink = B.up(t->v); }
   {
@@ -1394,6 +1424,25 @@ extern "C" int hy_finalize(hy_handle h) {
     }
   }
   {
+    int lists = 0;
+    size_t row = 0, heads = 0, maxH = 0;
+    for (auto& c : h->lc)
+      if (c.mixer == HY_MIX_LATENT && latent_prompt_sizes(h, c)) {
+        ++lists;
+        row = std::max(row, (size_t)(c.l_kv_rank + c.l_rot_dim));
+        heads = std::max(heads, (size_t)c.l_heads * (c.l_dim + c.l_rot_dim + c.l_vdim));
+        maxH = std::max(maxH, (size_t)c.l_heads);
+      }
+    if (lists) {
+      h->kv_cap = 4 * rt.max_step_tokens;
+      h->fl_cap = (size_t)lists * ((T / 128 + rt.max_step_entries) * maxH * sizeof(jf::FlashUnit) + ((size_t)rt.max_step_entries + 1) * 4 + 64);
+      if (dev_alloc(h, &h->kv_rows, (size_t)h->kv_cap * row * 2, &h->bytes_ws)) return HY_ERR_CUDA;
+      if (dev_alloc(h, &h->kv_heads, (size_t)h->kv_cap * heads * 2, &h->bytes_ws)) return HY_ERR_CUDA;
+      if (dev_alloc(h, (void**)&h->fl_d, h->fl_cap, &h->bytes_ws)) return HY_ERR_CUDA;
+      HY_CUDA(cudaMallocHost((void**)&h->fl_h, h->fl_cap));
+    }
+  }
+  {
     int maxE = 0, maxTop = 0;
     for (auto& c : h->lc)
       if (c.ff_kind == HY_FF_ROUTED) { maxE = std::max(maxE, c.x_experts); maxTop = std::max(maxTop, c.x_top); }
@@ -1440,28 +1489,28 @@ inline bool gemm_takes_tiles(const void* A, int lda, int T, int K) {
 }
 
 // The product on pairs of SMs: X [x_rows, K] (leading dimension lda), weight tiles of `groups` matrices [N, K], w_stride elements apart.
-// Tiles of 128 token rows when they fit one wave of the pairs (the wave is over sooner: N 1024, T 2048, K 6144: 45 us against 48 with
-// 256 rows), of 256 otherwise (N 2048, T 2048, K 2048: 27 us against 35).  Grouped: tile_rows as the tile list was made.
+// Grouped: tile_rows as the tile list was made.
 template <typename TO>
 int pair_product(hy_engine* h, const bf16* X, int lda, int x_rows, const void* tiled, int groups, size_t w_stride, int T, int N, int K,
-                 const GemmOut& o, int tile_rows, TpGroup grp) {
+                 const GemmOut& o, int tile_rows, jf::TpGroup grp) {
+  typedef HyEpilogue<TO> Epi;
   static bool attr = false;                                  // per TO: this function is a template
   if (!attr) {
-    cudaFuncSetAttribute(gemm_pair_kernel<TO, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tp_smem_bytes(128));
-    cudaFuncSetAttribute(gemm_pair_kernel<TO, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tp_smem_bytes(256));
+    cudaFuncSetAttribute(jf::pair_kernel<Epi, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)jf::tp_smem_bytes(128));
+    cudaFuncSetAttribute(jf::pair_kernel<Epi, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)jf::tp_smem_bytes(256));
     attr = true;
   }
   const int nx = (N + 255) / 256, KT = (K + 63) / 64, NT = (N + 127) / 128;
-  const int bt = tile_rows ? tile_rows : (long long)nx * ((T + 127) / 128) <= TP_CLUSTERS ? 128 : 256;
+  const int bt = tile_rows ? tile_rows : jf::tp_tile_rows(N, T);
   const uint64_t w_rows = groups > 1 ? (uint64_t)groups * (w_stride / 64) : (uint64_t)NT * KT * 128;
   CUtensorMap xm, wm;
-  if (!tp_map(&xm, X, (uint64_t)x_rows, (uint64_t)K, (uint64_t)lda, bt / 2, true) || !tp_map(&wm, tiled, w_rows, 64, 64, 128, false))
+  if (!jf::tp_map(&xm, X, (uint64_t)x_rows, (uint64_t)K, (uint64_t)lda, bt / 2, true) || !jf::tp_map(&wm, tiled, w_rows, 64, 64, 128, false))
     return fail(h, HY_ERR_CUDA, "a tensor map of the matrix product could not be made");
   grp.w_rows = (int)(w_stride / 64);
   const long long most = (long long)nx * (grp.meta ? x_rows / bt + groups : (T + bt - 1) / bt);      // tiles (grouped: at most)
-  const int grid = 2 * (int)std::min<long long>(most, TP_CLUSTERS);
-  if (bt == 128) go_kernel(h, gemm_pair_kernel<TO, 128>, grid, TP_THREADS, tp_smem_bytes(128), h->stream, xm, wm, T, N, K, o, h->err_d, grp);
-  else go_kernel(h, gemm_pair_kernel<TO, 256>, grid, TP_THREADS, tp_smem_bytes(256), h->stream, xm, wm, T, N, K, o, h->err_d, grp);
+  const int grid = 2 * (int)std::min<long long>(most, jf::TP_CLUSTERS);
+  auto kern = bt == 128 ? jf::pair_kernel<Epi, 128> : jf::pair_kernel<Epi, 256>;
+  go_kernel(h, kern, grid, jf::TP_THREADS, jf::tp_smem_bytes(bt), h->stream, xm, wm, T, N, K, Epi{o}, h->err_d, grp, jf::PairLayout{0, 0, 0});
   h->launches++;
   return HY_OK;
 }
@@ -1473,7 +1522,7 @@ int gemm(hy_engine* h, const TA* A, int lda, const TW* Wt, int ldw, int T, int N
   if (o.alpha == 0.0f) o.alpha = 1.0f;
   if constexpr (std::is_same<TA, bf16>::value && std::is_same<TW, bf16>::value) {
     if (tiled && gemm_takes_tiles(A, lda, T, K)) {
-      return pair_product<TO>(h, (const bf16*)A, lda, T, tiled, 1, 0, T, N, K, o, 0, TpGroup{});
+      return pair_product<TO>(h, (const bf16*)A, lda, T, tiled, 1, 0, T, N, K, o, 0, jf::TpGroup{});
     }
   }
   constexpr int VECW = 16 / (int)sizeof(TW);
@@ -1684,6 +1733,73 @@ void prepare_units(hy_engine* h, int E, int T) {
   }
 }
 
+// Row units of a prompt step's latent attention with H heads (one head's 128 tokens each, late tokens first) and where each request's
+// keys begin in the gathered rows; NULL: the step's contexts do not fit the gathered rows.
+const hy_engine::FlashList* flash_units(hy_engine* h, int E, int H) {
+  for (const auto& l : h->fl_lists) if (l.H == H) return &l;
+  long long keys = 0;
+  for (int e = 0; e < E; ++e) keys += h->step_pos0[e] + h->step_start[e + 1] - h->step_start[e];
+  if (keys > h->kv_cap) return nullptr;
+  unsigned char* at = h->fl_h + h->fl_used;
+  int* off = reinterpret_cast<int*>(at);
+  jf::FlashUnit* u = reinterpret_cast<jf::FlashUnit*>(at + (((size_t)E + 1) * 4 + 15) / 16 * 16);
+  int n = 0;
+  off[0] = 0;
+  for (int e = 0; e < E; ++e) off[e + 1] = off[e] + h->step_pos0[e] + h->step_start[e + 1] - h->step_start[e];
+  for (int e = 0; e < E; ++e) {
+    const int len = h->step_start[e + 1] - h->step_start[e];
+    for (int p = (len - 1) / 128 * 128; p >= 0; p -= 128)
+      for (int hd = 0; hd < H; ++hd) u[n++] = jf::FlashUnit{h->step_start[e], len, p, len, hd, hd, h->step_pos0[e], off[e], 0, 0, 0};
+  }
+  const size_t bytes = (unsigned char*)(u + n) - at;
+  unsigned char* d = h->fl_d + h->fl_used;
+  cudaMemcpyAsync(d, at, bytes, cudaMemcpyHostToDevice, h->stream);
+  h->fl_lists.push_back({H, reinterpret_cast<const jf::FlashUnit*>(d + ((unsigned char*)u - at)), reinterpret_cast<const int*>(d), n, (int)keys});
+  h->fl_used += (bytes + 63) / 64 * 64;
+  return &h->fl_lists.back();
+}
+
+// Latent attention of a prompt step over per-head keys and values: one product of all cache rows that the step's requests hold gives
+// them (each head's key: its part of the up-projection, then the rotated part as it is), and attention runs over heads of dim + rot
+// and vdim instead of rank + rot and rank.  1531 tokens behind 2048, 16 heads of 128 + 64 over a rank of 512: the folded form does
+// 3.4 times the score and value products (1150 us on mma.sync) and folds queries and values itself (223 + 237 us); this form
+// 220 us in all (160 of them attention).  Worth it from about 64 tokens per request (the product is made for the whole context every step); steps
+// whose contexts exceed the gathered rows keep the folded form.  Queries in h->pin (rotated here), results in h->cat.
+bool latent_prompt(hy_engine* h, const Batch& b, const LayerW& L, const hy_layer_cfg& c) {
+  if (!L.w_kv_t || b.T < 64 * b.E) return false;
+  const int H = c.l_heads, hk = c.l_dim + c.l_rot_dim, dv = c.l_vdim, K = c.l_kv_rank + c.l_rot_dim, N = H * (hk + dv);
+  const hy_engine::FlashList* l = flash_units(h, b.E, H);
+  if (!l) return false;
+  cudaStream_t s = h->stream;
+  bf16* pin = (bf16*)h->pin; bf16* kv = (bf16*)h->kv_heads;
+  {
+    ProfScope ps(h, HY_PROF_SMALL_GEMM);
+    go_kernel(h, latent_rotate_kernel<bf16>, b.T, 128, (size_t)(2 * L.rot.pairs + 2) * 4, s, b, pin, h->ld_pin, H, c.l_dim, c.l_rot_dim, L.rot);
+    go_kernel(h, latent_gather_kernel, l->keys, 128, 0, s, b, l->key_off, (const bf16*)L.cache, K, (bf16*)h->kv_rows);
+    h->launches += 2;
+    pair_product<bf16>(h, (const bf16*)h->kv_rows, K, l->keys, L.w_kv_t, 1, 0, l->keys, N, K, to_buf(kv, N), 0, jf::TpGroup{});
+  }
+  ProfScope ps(h, HY_PROF_ATTN);
+  CUtensorMap km, vm;
+  if (!jf::tp_map(&km, kv, (uint64_t)l->keys, (uint64_t)H * hk, (uint64_t)N, 128, true) ||
+      !jf::tp_map(&vm, kv + (size_t)H * hk, (uint64_t)l->keys, (uint64_t)H * dv, (uint64_t)N, 128, true)) return false;
+  const jf::FlashArgs fa{l->units, pin, (size_t)h->ld_pin, hk, nullptr, 1, c.l_scale, c.l_window, (const bf16*)L.sink,
+                         c.l_gate ? pin + L.c_g : nullptr, (size_t)h->ld_pin, (bf16*)h->cat, (size_t)h->ld_cat, 0, h->err_d};
+  auto go = [&](auto dk, auto dvv) {
+    constexpr int DK = decltype(dk)::value, DV = decltype(dvv)::value;
+    constexpr size_t smem = jf::fl_smem_bytes(DK, DV);
+    static bool attr = false;                                // per kernel: go is a template
+    if (!attr) { cudaFuncSetAttribute(jf::flash_kernel<DK, DV, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); attr = true; }
+    go_kernel(h, jf::flash_kernel<DK, DV, true>, l->n, jf::FL_THREADS, smem, s, km, vm, km, vm, fa);
+  };
+  typedef std::integral_constant<int, 64> c64; typedef std::integral_constant<int, 128> c128; typedef std::integral_constant<int, 192> c192;
+  if (hk == 64) { if (dv == 64) go(c64{}, c64{}); else go(c64{}, c128{}); }
+  else if (hk == 128) { if (dv == 64) go(c128{}, c64{}); else go(c128{}, c128{}); }
+  else { if (dv == 64) go(c192{}, c64{}); else go(c192{}, c128{}); }
+  h->launches++;
+  return true;
+}
+
 // Attention over a shared latent: down-projections in h->f1 ([query latent | key / value latent | raw rotated key part]; with
 // full-rank queries those are in h->pin already), result (heads concatenated) in h->cat.
 template <typename AT>
@@ -1705,6 +1821,10 @@ void latent_mixer(hy_engine* h, const Batch& b, const LayerW& L, const hy_layer_
     ProfScope ps(h, HY_PROF_SMALL_GEMM);
     if (c.l_q_rank > 0)
       gemm<AT, WT, AT>(h, cv, h->ld_cv, (const WT*)L.w_uq, c.l_q_rank, T, H * (dn + rot), c.l_q_rank, to_buf(pin, h->ld_pin), L.w_uq_t);
+  }
+  if constexpr (std::is_same<AT, bf16>::value) { if (latent_prompt(h, b, L, c)) return; }
+  {
+    ProfScope ps(h, HY_PROF_SMALL_GEMM);
     const int fold = T > 8 ? 1 : 0;
     go_kernel(h, latent_query_kernel<AT, WT>, dim3((T + HY_LAT_TB - 1) / HY_LAT_TB, H, fold ? (R + 127) / 128 : 1), 128, (size_t)(HY_LAT_TB * dn + 2 * L.rot.pairs + 2) * 4, s, b, pin, h->ld_pin, (const WT*)L.w_uk, H, dn,
                                                                                            rot, R, fold, L.rot, cv, h->ld_cv);
@@ -1920,7 +2040,7 @@ int sandwich_layer(hy_engine* h, const Batch& b, size_t li) {
           pin, ldh, h->x_ids, top, 0, NE, (const WT*)L.w_down, (size_t)W * ff, W, ff, ys, W, -1, 0.0f);
     } else if (tc_experts) {
       if constexpr (std::is_same<AT, bf16>::value) {
-        const TpGroup grp{h->x_meta, h->x_offs, h->x_tile_e, h->x_tile_r0, 0};
+        const jf::TpGroup grp{h->x_meta, h->x_offs, h->x_tile_e, h->x_tile_r0, 0};
         GemmOut o1{pin, ldh, ff, nullptr, 0, 2, nullptr, 0, 1.0f};
         pair_product<bf16>(h, x_rows, W, P, L.w_gu_t, NE, L.gu_t_stride, P, L.gu_rows, W, o1, expert_tile_rows(P, NE), grp);
         GemmOut o2 = to_buf(ys, W);
@@ -2128,7 +2248,7 @@ int postnorm_layer(hy_engine* h, const Batch& b, size_t li) {
           pin, ldh, h->x_ids, top, 0, NE, (const WT*)L.w_down, (size_t)W * ff, W, ff, ys, W, -1, 0.0f);
     } else if (tc_experts) {
       if constexpr (std::is_same<AT, bf16>::value) {
-        const TpGroup grp{h->x_meta, h->x_offs, h->x_tile_e, h->x_tile_r0, 0};
+        const jf::TpGroup grp{h->x_meta, h->x_offs, h->x_tile_e, h->x_tile_r0, 0};
         GemmOut o1 = to_buf(pin, ldh);
         o1.act2 = 3; o1.act_kind = c.x_act;
         pair_product<bf16>(h, x_rows, W, P, L.w_gu_t, NE, L.gu_t_stride, P, ff, W, o1, expert_tile_rows(P, NE), grp);
@@ -2201,7 +2321,7 @@ bool routed_gated_experts(hy_engine* h, int T, const AT* hb, const LayerW& L, co
         pin, ldh, h->x_ids, top, 0, NE, (const WT*)L.w_down, (size_t)W * ff, W, ff, ys, W, -1, 0.0f);
   } else if (tc_experts) {
     if constexpr (std::is_same<AT, bf16>::value) {
-      const TpGroup grp{h->x_meta, h->x_offs, h->x_tile_e, h->x_tile_r0, 0};
+      const jf::TpGroup grp{h->x_meta, h->x_offs, h->x_tile_e, h->x_tile_r0, 0};
       GemmOut o1{pin, ldh, ff, nullptr, 0, 2, nullptr, 0, 1.0f};
       o1.act_kind = c.x_act; o1.act_limit = c.ff_limit;
       pair_product<bf16>(h, x_rows, W, P, L.w_gu_t, NE, L.gu_t_stride, P, L.gu_rows, W, o1, expert_tile_rows(P, NE), grp);
@@ -2856,6 +2976,7 @@ extern "C" int hy_step(hy_handle h, int32_t n_entries, const int32_t* tokens, co
   b.T = T; b.E = E; b.max_pages = rt.max_pages_per_seq; b.page_size = rt.page_size;
   const int* want_d = b.pages + (size_t)E * rt.max_pages_per_seq;
   h->step_start = ent_start; h->step_pos0 = ent_pos0; h->step_tokens = T; h->units_used = 0; h->unit_lists.clear();
+  h->fl_used = 0; h->fl_lists.clear();
   HY_CUDA(cudaEventRecord(h->ev0, h->stream));
   if (h->m.dtype == HY_DTYPE_F32) run_step<float>(h, b, n_want, want_d, layers_out);
   else run_step<__nv_bfloat16>(h, b, n_want, want_d, layers_out);

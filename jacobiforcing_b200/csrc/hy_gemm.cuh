@@ -1,93 +1,12 @@
-// hy_gemm.cuh — tcgen05 matrix product of the layered hybrid decoders' prompt steps on pairs of SMs (bf16 operands, fp32
-// accumulation in tensor memory):  C[t, n] = sum_k X[t, k] W[n, k].
-//
-// A cluster of two CTAs works on one tile of 256 features x BT tokens: each holds the weight rows of its 128 features and half of the
-// token rows in shared memory, and one thread of the first issues tcgen05.mma.cta_group::2, which reads both halves from both
-// SMs and leaves 128 features in each SM's tensor memory.  An SM so takes in 32 KiB per 64 k for 128 x 256 products instead of
-// 48 KiB; what an SM takes in was what bounded a kernel of 128 x 256 tiles on one SM with its activation rows copied by threads.
-// Both operands travel by TMA: weight tiles lie in HBM in the K-major SWIZZLE_128B layout already (an unswizzled map of 128-byte
-// rows), activation rows are row-major and swizzled on the way in (rows and columns beyond the operand read as zeros).  The kernel
-// is persistent: one cluster per pair of SMs walks the tiles, and the epilogue of a tile runs under the products of the next
-// (two accumulators).
-// Measured cold, TFLOP/s, that kernel -> this one:  N 24576, T 2048, K 2048: 825 -> 1325;  N 2048, T 2048, K 10240: 736 -> 1198;
-// N 37888, T 1000, K 3584: 975 -> 1441 (0.87 of the measured cuBLAS burst);  few tiles (N 1024, T 512, K 6144): 68 -> 43 us.
-//
-// Warp 0:     producer (one lane in each CTA, seven or nine stages; all bytes of a stage count on the first CTA's mbarrier).
-// Warp 1:     owns tensor memory; in the first CTA one lane issues the products and commits to both CTAs' mbarriers.
-// Warps 2-9:  epilogue (two per quarter of the lanes, one half of the columns each).
-// Every wait is bounded: on a timeout the kernel raises the error flag, stops waiting, lets its copies land and frees its
-// tensor memory.
+// hy_gemm.cuh — the hybrid decoders' use of the product on pairs of SMs (jf_pair.cuh): what leaves with the accumulators, and the
+// packing of weights into its tiles.
 #pragma once
-#include <cuda.h>
-
 #include <vector>
 
 #include "hy_kernels.cuh"
-#include "jf_ptx.cuh"
+#include "jf_pair.cuh"
 
 namespace hy {
-
-constexpr int TC_WTILE = 128 * 64 * 2;                  // 16 KiB
-constexpr uint32_t TC_SPIN_LIMIT = 1u << 22;            // try_wait probes (each blocks for a bounded time itself)
-// as many stages as fit: what few tiles with a long k wait for is the latency of their loads
-__host__ __device__ constexpr int tp_stages(int bt) { return bt == 256 ? 7 : 9; }
-constexpr int TP_MAX_STAGES = 9;
-constexpr int TP_THREADS = 320;
-constexpr int TP_CLUSTERS = 74;                         // pairs of SMs
-
-struct TpSmem {
-  uint64_t full[TP_MAX_STAGES], empty[TP_MAX_STAGES], acc_full[2], acc_empty[2];
-  uint32_t tmem_base;
-  uint32_t failed;
-};
-
-__device__ __forceinline__ uint32_t tp_rank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
-__device__ __forceinline__ void tp_cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// the address of a shared-memory object of this CTA in the first CTA of the pair
-__device__ __forceinline__ uint32_t tp_in_first(const void* p) {
-  uint32_t a;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(a) : "r"(jf::smem_u32(p)));
-  return a;
-}
-__device__ __forceinline__ void tp_arrive_cluster(uint32_t bar) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ bool tp_wait(uint64_t* bar, uint32_t parity, TpSmem* sm, int* err) {
-  if (sm->failed) return false;
-  for (uint32_t i = 0; i < TC_SPIN_LIMIT; ++i) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(jf::smem_u32(bar)), "r"(parity)
-        : "memory");
-    if (ok) return true;
-  }
-  sm->failed = 1;
-  atomicExch(err, 1);
-  return false;
-}
-__device__ __forceinline__ void tp_load(void* dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
-  asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-               ::"r"(jf::smem_u32(dst)), "l"(map), "r"(x), "r"(y), "r"(bar) : "memory");
-}
-__device__ __forceinline__ void tp_mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// arrive on the mbarrier at this offset in both CTAs when the products issued so far have completed
-__device__ __forceinline__ void tp_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-               ::"r"(jf::smem_u32(bar)), "h"((uint16_t)3) : "memory");
-}
 
 // Epilogue of one warp: the accumulators at taddr (its 32 lanes, `cols` columns, a multiple of 32: two loads in flight) leave
 // through GemmOut.  n: this lane's feature, t0: the token of the first column.
@@ -102,18 +21,7 @@ __device__ __forceinline__ void tc_store_columns(const GemmOut& o, uint32_t tadd
   const bool second = n >= o.split, wide = second ? (o.out2_f32 || sizeof(TO) == 4) : sizeof(TO) == 4, in = n < N;
   const float bias = o.bias && in ? o.bias[n] : 0.0f;
   // one pass over the columns with what to do with sixteen of them (rows: how many exist) given as a function
-  auto each = [&](auto store16) {
-    for (int c0 = 0; c0 < cols; c0 += 32) {
-      if (t0 + c0 >= T) break;
-      __syncwarp();                                        // the loads from tensor memory are warp-wide
-      uint32_t a[16], b[16];
-      jf::tmem_ld16(taddr + c0, a);
-      jf::tmem_ld16(taddr + c0 + 16, b);
-      jf::tmem_ld_wait();
-      store16(a, t0 + c0, min(16, T - t0 - c0));
-      if (t0 + c0 + 16 < T) store16(b, t0 + c0 + 16, min(16, T - t0 - c0 - 16));
-    }
-  };
+  auto each = [&](auto store16) { jf::tp_columns(taddr, t0, cols, T, store16); };
   if (pairs) {
     const int pf = (o.act2 == 5 ? (n - lane - o.pair_lo) >> 1 : (n - lane) >> 1) + (lane & 15);      // this lane's feature of a pair
     const int pn = o.act2 == 5 ? o.pair_n : o.split, pld = o.act2 == 5 ? o.ld_pair : o.ld1;
@@ -197,127 +105,13 @@ __device__ __forceinline__ void tc_store_columns(const GemmOut& o, uint32_t tadd
   else go([](float c) { return c; });
 }
 
-// Grouped mode (routed experts): the tiles of a device-made list, each up to BT consecutive rows of the expert-sorted activation
-// rows that belong to one expert; the weight tiles of expert e start e * w_rows map rows further on.  Rows of the next expert
-// that a tile reads along are left out by the epilogue.
-struct TpGroup { const int* meta; const int* offs; const int* tile_expert; const int* tile_row0; int w_rows; };
-
-template <typename TO, int BT>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TP_THREADS, 1)
-gemm_pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap, int T, int N, int K, GemmOut o, int* err,
-                 TpGroup grp) {
-  extern __shared__ __align__(16) unsigned char hy_smem[];
-  unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(hy_smem) + 1023) & ~(uintptr_t)1023);
-  constexpr int TP_STAGES = tp_stages(BT), XTILE = BT / 2 * 128, SLOT = TC_WTILE + XTILE;
-  TpSmem* sm = reinterpret_cast<TpSmem*>(base + TP_STAGES * SLOT);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rank = (int)tp_rank();
-  const int KT = (K + 63) / 64, nx = (N + 255) / 256, first = blockIdx.x >> 1, step = gridDim.x >> 1;
-  pdl_trigger();
-  if (threadIdx.x == 0) {
-    for (int i = 0; i < TP_STAGES; ++i) { jf::mbar_init(&sm->full[i], 1); jf::mbar_init(&sm->empty[i], 1); }
-    for (int i = 0; i < 2; ++i) { jf::mbar_init(&sm->acc_full[i], 1); jf::mbar_init(&sm->acc_empty[i], 16); }
-    sm->failed = 0;
-    jf::fence_mbar_init();
+template <typename TO>
+struct HyEpilogue {
+  GemmOut o;
+  __device__ __forceinline__ void operator()(uint32_t taddr, int n, int t0, int cols, int T, int N, int lane) const {
+    tc_store_columns<TO>(o, taddr, n, t0, cols, T, N, lane);
   }
-  if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(jf::smem_u32(&sm->tmem_base)), "r"((uint32_t)(2 * BT)) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-  }
-  jf::tc_fence_before();
-  __syncthreads();
-  tp_cluster_sync();
-  jf::tc_fence_after();
-  // the weight tiles of the first stages travel while the kernel before this one ends (which tile is the first is known when the
-  // tiles are not a list that it makes)
-  int ahead = 0;
-  if (warp == 0 && lane == 0 && !grp.meta) {
-    const int x = first / ((T + BT - 1) / BT);
-    for (; ahead < min(TP_STAGES, KT); ++ahead) {
-      if (rank == 0) jf::mbar_expect_tx(&sm->full[ahead], 2 * SLOT);
-      tp_load(base + ahead * SLOT, &wmap, 0, ((2 * x + rank) * KT + ahead) * 128, tp_in_first(&sm->full[ahead]));
-    }
-  }
-  pdl_wait();
-  const int ny = grp.meta ? grp.meta[0] : (T + BT - 1) / BT, tiles = nx * ny;
-  // token tile and feature tile of a tile number: neighbours share the weight rows (grouped: the expert's activation rows)
-  auto place = [&](int tile, int& x, int& y) {
-    if (grp.meta) { x = tile % nx; y = tile / nx; }
-    else { x = tile / ny; y = tile % ny; }
-  };
-
-  if (warp == 0) {
-    if (lane == 0) {
-      int it = 0;
-      bool ok = true;
-      for (int tile = first; tile < tiles && ok; tile += step) {
-        int x, y;
-        place(tile, x, y);
-        const int t0 = (grp.meta ? grp.tile_row0[y] : y * BT) + rank * (BT / 2);
-        const int w0 = (grp.meta ? grp.tile_expert[y] * grp.w_rows : 0) + (2 * x + rank) * KT * 128;
-        for (int kt = 0; kt < KT; ++kt, ++it) {
-          const int s = it % TP_STAGES;
-          ok = tp_wait(&sm->empty[s], ((it / TP_STAGES) & 1) ^ 1, sm, err);      // the products that read the slot retired
-          if (!ok) break;
-          const uint32_t bar = tp_in_first(&sm->full[s]);
-          if (it >= ahead) {
-            if (rank == 0) jf::mbar_expect_tx(&sm->full[s], 2 * SLOT);
-            tp_load(base + s * SLOT, &wmap, 0, w0 + kt * 128, bar);
-          }
-          tp_load(base + s * SLOT + TC_WTILE, &xmap, kt * 64, t0, bar);
-        }
-      }
-      if (!ok) for (int i = 0; i < 1000; ++i) __nanosleep(1000);    // copies in flight land before the block leaves
-    }
-    __syncwarp();
-  } else if (warp == 1) {
-    if (lane == 0 && rank == 0) {
-      const uint32_t idesc = jf::umma_idesc_bf16(256, BT);
-      int it = 0, i = 0;
-      bool ok = true;
-      for (int tile = first; tile < tiles && ok; tile += step, ++i) {
-        const uint32_t d = sm->tmem_base + (i & 1) * BT;
-        ok = tp_wait(&sm->acc_empty[i & 1], ((i >> 1) & 1) ^ 1, sm, err);        // both CTAs have read it
-        jf::tc_fence_after();
-        for (int kt = 0; kt < KT && ok; ++kt, ++it) {
-          const int s = it % TP_STAGES;
-          ok = tp_wait(&sm->full[s], (it / TP_STAGES) & 1, sm, err);
-          if (!ok) break;
-          jf::tc_fence_after();
-          const uint32_t sa = jf::smem_u32(base + s * SLOT), sb = sa + TC_WTILE;
-#pragma unroll
-          for (int kk = 0; kk < 4; ++kk)
-            tp_mma(d, jf::umma_desc_sw128(sa + kk * 32), jf::umma_desc_sw128(sb + kk * 32), idesc, (kt > 0 || kk > 0) ? 1u : 0u);
-          tp_commit(&sm->empty[s]);
-        }
-        if (ok) tp_commit(&sm->acc_full[i & 1]);
-      }
-    }
-    __syncwarp();
-  } else {
-    const int q = warp & 3, half = (warp - 2) >> 2;                 // quarter of the lanes that this warp may read, half of the columns
-    int i = 0;
-    for (int tile = first; tile < tiles; tile += step, ++i) {
-      int x, y;
-      place(tile, x, y);
-      if (!tp_wait(&sm->acc_full[i & 1], (i >> 1) & 1, sm, err)) break;
-      jf::tc_fence_after();
-      const int t0 = (grp.meta ? grp.tile_row0[y] : y * BT) + half * (BT / 2);
-      const int rows = grp.meta ? grp.offs[grp.tile_expert[y] + 1] : T;
-      tc_store_columns<TO>(o, sm->tmem_base + (i & 1) * BT + half * (BT / 2) + ((uint32_t)(q * 32) << 16), x * 256 + rank * 128 + q * 32 + lane, t0,
-                           BT / 2, rows, N, lane);
-      jf::tc_fence_before();
-      __syncwarp();
-      if (lane == 0) tp_arrive_cluster(tp_in_first(&sm->acc_empty[i & 1]));
-    }
-  }
-  jf::tc_fence_before();
-  __syncthreads();
-  tp_cluster_sync();                                                // nothing of the pair still reads or signals this CTA
-  if (warp == 1)
-    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(sm->tmem_base), "r"((uint32_t)(2 * BT)) : "memory");
-}
-
-constexpr size_t tp_smem_bytes(int bt) { return (size_t)tp_stages(bt) * (TC_WTILE + bt / 2 * 128) + sizeof(TpSmem) + 1024; }
+};
 
 // Host-side packer: row-major [N, K] floats -> bf16 tiles [ceil(N/128)][ceil(K/64)] of 128 x 64 in the swizzled layout.
 inline void pack_tiles(const float* w, int N, int K, std::vector<uint16_t>& out) {
@@ -332,29 +126,6 @@ inline void pack_tiles(const float* w, int N, int K, std::vector<uint16_t>& out)
       memcpy(&bits, &b, 2);
       out[tile * 8192 + off / 2] = bits;
     }
-}
-
-// ---- host: tensor maps ------------------------------------------------------------------------------------------------------------
-typedef CUresult (*TpEncode)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
-                             const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-inline TpEncode tp_encode() {
-  static const TpEncode f = [] {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult r;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &r) != cudaSuccess || r != cudaDriverEntryPointSuccess) p = nullptr;
-    return (TpEncode)p;
-  }();
-  return f;
-}
-// rows x cols bf16 elements, `ld` elements from row to row, in boxes of box_rows x 64
-inline bool tp_map(CUtensorMap* m, const void* p, uint64_t rows, uint64_t cols, uint64_t ld, int box_rows, bool swizzle) {
-  const TpEncode f = tp_encode();
-  if (!f) return false;
-  const cuuint64_t dims[2] = {cols, rows}, strides[1] = {ld * 2};
-  const cuuint32_t box[2] = {64, (cuuint32_t)box_rows}, one[2] = {1, 1};
-  return f(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(p), dims, strides, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
-           swizzle ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 }  // namespace hy

@@ -11,17 +11,15 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-#include "jf_ptx.cuh"
+#include "jf_pair.cuh"
 
 namespace hy {
 
 typedef __nv_bfloat16 bf16;
 
-// Programmatic dependent launch: every kernel of a step may start while the one before it still runs (see go_kernel) and must not
-// touch anything that an earlier kernel reads or writes before pdl_wait.  What comes before it (weights, which nothing
-// writes; barriers, tensor memory) overlaps the end of the kernel before.
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Every kernel of a step may start while the one before it still runs (see go_kernel; jf_pair.cuh has the two instructions).
+using jf::pdl_trigger;
+using jf::pdl_wait;
 __device__ __forceinline__ void pdl_begin() { pdl_trigger(); pdl_wait(); }
 
 template <typename T> __device__ __forceinline__ float to_f(T v);

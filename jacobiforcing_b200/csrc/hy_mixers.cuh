@@ -147,6 +147,38 @@ __global__ void __launch_bounds__(128) latent_query_kernel(Batch b, const AT* __
   }
 }
 
+// Prompt steps attend over per-head keys and values made for the step (see latent_prompt): the rotated part of the queries, in place.
+// q [T, ldq] holds heads of [dim | rot].  One block per token.
+template <typename AT>
+__global__ void __launch_bounds__(128) latent_rotate_kernel(Batch b, AT* __restrict__ q, int ldq, int H, int dim, int rot, Rotation r) {
+  pdl_begin();
+  extern __shared__ __align__(16) unsigned char hy_smem[];
+  float* cs = reinterpret_cast<float*>(hy_smem);              // [2 * pairs]
+  const int t = blockIdx.x;
+  rotation_row(r, b.tok_pos[t], cs);
+  __syncthreads();
+  for (int i = threadIdx.x; i < H * r.pairs; i += blockDim.x) {
+    const int p = i % r.pairs;
+    AT* x = q + (size_t)t * ldq + (i / r.pairs) * (dim + rot) + dim;
+    const int one = r.half ? p : 2 * p, two = r.half ? p + r.pairs : 2 * p + 1;
+    const float u = to_f(x[one]), v = to_f(x[two]), c = cs[2 * p], s = cs[2 * p + 1];
+    x[one] = from_f<AT>(fmaf(u, c, -v * s));
+    x[two] = from_f<AT>(fmaf(v, c, u * s));
+  }
+}
+
+// All cache rows of a step's requests, one after the other: out [sum of contexts, dim], entry e's from key_off[e] on.  One block per row.
+__global__ void __launch_bounds__(128) latent_gather_kernel(Batch b, const int* __restrict__ key_off, const bf16* __restrict__ cache, int dim,
+                                                            bf16* __restrict__ out) {
+  pdl_begin();
+  int e = 0;
+  while ((int)blockIdx.x >= key_off[e + 1]) ++e;
+  const int j = blockIdx.x - key_off[e];
+  const bf16* src = cache + ((size_t)b.pages[(size_t)e * b.max_pages + j / b.page_size] * b.page_size + j % b.page_size) * dim;
+  for (int k = threadIdx.x; k < dim / 8; k += blockDim.x)
+    reinterpret_cast<uint4*>(out + (size_t)blockIdx.x * dim)[k] = reinterpret_cast<const uint4*>(src)[k];
+}
+
 // The value up-projection behind the weighted sum: out[t, h, j] = sum_r w_uvT[h][r][j] o[t, h, r]  (o fp32: the weighted
 // sum of latents; w_uvT is the value up-projection transposed per head at load so that thread j reads coalesced).  gate (NULL: none):
 // the result times sigmoid(gate[t, h * vdim + j]).
