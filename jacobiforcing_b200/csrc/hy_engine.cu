@@ -161,6 +161,7 @@ struct hy_engine {
   AttnUnit* units_d = nullptr; AttnUnit* units_h = nullptr; size_t units_cap = 0, units_used = 0;
   std::vector<UnitList> unit_lists;
   int step_tokens = 0;
+  float* part_sums = nullptr; int* part_arrived = nullptr;      // partial sums of products with few tiles (jf::PairSplit)
   // prompt steps of latent attention: keys of a step's requests one after the other (cache rows, then per-head keys and values),
   // row units and the requests' first rows for the kernels
   void* kv_rows = nullptr; void* kv_heads = nullptr; int kv_cap = 0;
@@ -1395,6 +1396,9 @@ extern "C" int hy_finalize(hy_handle h) {
   if (dev_alloc(h, (void**)&h->meta_d, h->meta_words * 4, &h->bytes_ws)) return HY_ERR_CUDA;
   HY_CUDA(cudaMallocHost((void**)&h->meta_h, h->meta_words * 4));
   if (h->m.dtype == HY_DTYPE_BF16) {
+    if (dev_alloc(h, (void**)&h->part_sums, jf::TP_SUMS * 4, &h->bytes_ws)) return HY_ERR_CUDA;
+    if (dev_alloc(h, (void**)&h->part_arrived, jf::TP_ARRIVED * 4, &h->bytes_ws)) return HY_ERR_CUDA;
+    HY_CUDA(cudaMemset(h->part_arrived, 0, jf::TP_ARRIVED * 4));
     int maxH = 0, maxG = 0, maxD = 0;
     std::set<std::vector<int>> layouts;                      // attention layouts whose unit lists one step may hold
     for (auto& c : h->lc) {
@@ -1508,9 +1512,11 @@ int pair_product(hy_engine* h, const bf16* X, int lda, int x_rows, const void* t
     return fail(h, HY_ERR_CUDA, "a tensor map of the matrix product could not be made");
   grp.w_rows = (int)(w_stride / 64);
   const long long most = (long long)nx * (grp.meta ? x_rows / bt + groups : (T + bt - 1) / bt);      // tiles (grouped: at most)
-  const int grid = 2 * (int)std::min<long long>(most, jf::TP_CLUSTERS);
+  const int parts = grp.meta ? 1 : jf::tp_parts((int)std::min<long long>(most, jf::TP_CLUSTERS + 1), K);
+  const int grid = 2 * (int)std::min<long long>(most * parts, jf::TP_CLUSTERS);
   auto kern = bt == 128 ? jf::pair_kernel<Epi, 128> : jf::pair_kernel<Epi, 256>;
-  go_kernel(h, kern, grid, jf::TP_THREADS, jf::tp_smem_bytes(bt), h->stream, xm, wm, T, N, K, Epi{o}, h->err_d, grp, jf::PairLayout{0, 0, 0});
+  go_kernel(h, kern, grid, jf::TP_THREADS, jf::tp_smem_bytes(bt), h->stream, xm, wm, T, N, K, Epi{o}, h->err_d, grp, jf::PairLayout{0, 0, 0},
+            jf::PairSplit{parts, h->part_sums, h->part_arrived});
   h->launches++;
   return HY_OK;
 }
@@ -2999,6 +3005,7 @@ extern "C" int hy_step(hy_handle h, int32_t n_entries, const int32_t* tokens, co
   if (*h->err_h) {
     *h->err_h = 0;
     cudaMemset(h->err_d, 0, 4);
+    if (h->part_arrived) cudaMemset(h->part_arrived, 0, jf::TP_ARRIVED * 4);
     return fail(h, HY_ERR_CUDA, "a wait inside the tensor-core matrix product ran out (pipeline stalled)");
   }
   cudaEventElapsedTime(&h->last_ms, h->ev0, h->ev1);

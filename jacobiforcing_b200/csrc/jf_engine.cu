@@ -6,10 +6,13 @@
 #include <cstdlib>
 #include <cstring>
 #include <cmath>
+#include <algorithm>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "jf_kernel.cuh"
+#include "jf_wide.cuh"
 #include "../../include/jacobi_b200.h"
 
 using namespace jf;
@@ -52,6 +55,10 @@ struct jf_engine {
   // host mirrors
   std::vector<SeqState> h_states;
   // per-call draft sources of jf_jacobi_run (first-call tokens, MT19937 states, pad streams): grown on demand, kept
+  // forwards of many rows (jf_wide.cuh): attention row units, error flag
+  FlashUnit* wide_units_d = nullptr;
+  size_t wide_units_cap = 0;
+  int* wide_err = nullptr;
   int* run_scratch[3] = {nullptr, nullptr, nullptr};
   size_t run_scratch_words[3] = {0, 0, 0};
 };
@@ -801,6 +808,59 @@ static int launch_persistent(jf_engine* h, int run_mode, int max_forwards, float
   return JF_OK;
 }
 
+// Whether a planned forward runs as one kernel per stage (jf_wide.cuh): prompt rows, that is every row is committed at its own
+// position, kWideRows of them or more, on one GPU, without a stage profile.  Verification rows keep the persistent kernel however many they are, so
+// that planned forwards and the device-resident loop agree bit for bit.  7B shape, 28 layers, ms: 256 rows 9.28 persistent, 7.8 wide;
+// 512 rows 18.7, 9.0; 1000 rows 38.4, 12.6; below 200 rows the persistent kernel's weight stream is the faster one.
+static bool takes_wide(const jf_engine* h, int T, const std::vector<Group>& groups, const std::vector<int>& row_group, int lm_rows,
+                       const std::vector<CommitEntry>& commits, int n_commit) {
+  const DevCtx& c = h->hctx;
+  if (c.tp_size != 1 || T < kWideRows || n_commit != T || (h->md.d != 64 && h->md.d != 128) || lm_rows > kArgmaxRows || (c.prof && c.prof_forward >= 0)) return false;
+  for (int i = 0; i < n_commit; ++i) {                        // each row once, at its own position, by its own sequence
+    const CommitEntry& e = commits[i];
+    const Group& g = groups[row_group[e.src_row]];
+    if (e.src_row != i || e.seq != g.seq || e.pos != g.ctx + e.src_row - g.row0) return false;
+  }
+  for (const Group& g : groups)                               // no two groups write the same pages
+    for (const Group& o : groups)
+      if (&g != &o && g.seq == o.seq) return false;
+  return true;
+}
+
+static int run_wide(jf_engine* h, int T, const std::vector<Group>& groups, int lm_row0, int lm_rows, float* elapsed_ms) {
+  DevCtx& c = h->hctx;
+  const std::vector<FlashUnit> units = wide_units(h->md, groups, c.max_pages_per_seq);
+  if (h->wide_units_d == nullptr) {
+    h->wide_units_cap = (size_t)h->md.n_kv * ((size_t)h->md.n_rep * c.T_cap / 128 + c.G_cap + 1);
+    int rc = dev_alloc(h, &h->wide_units_d, h->wide_units_cap, &h->bytes_act);
+    if (rc == JF_OK) rc = dev_alloc(h, &h->wide_err, 4, &h->bytes_act);
+    if (rc != JF_OK) return rc;
+  }
+  if (units.size() > h->wide_units_cap) { h->err = "attention units exceed capacity"; return JF_ERR_CAPACITY; }
+  if (lm_rows > 0 && c.logits == nullptr) {
+    int rc = dev_alloc(h, &c.logits, (size_t)kArgmaxRows * h->md.vocab, &h->bytes_act);
+    if (rc != JF_OK) return rc;
+    JF_CUDA(h, cudaMemcpyAsync(h->dctx, &h->hctx, sizeof(DevCtx), cudaMemcpyHostToDevice, h->stream));
+  }
+  JF_CUDA(h, cudaMemcpyAsync(h->wide_units_d, units.data(), units.size() * sizeof(FlashUnit), cudaMemcpyHostToDevice, h->stream));
+  JF_CUDA(h, cudaEventRecord(h->ev0, h->stream));
+  const int n = wide_forward(h->stream, c, T, h->wide_units_d, (int)units.size(), lm_row0, lm_rows, h->wide_err);
+  JF_CUDA(h, cudaEventRecord(h->ev1, h->stream));
+  JF_CUDA(h, cudaStreamSynchronize(h->stream));
+  JF_CUDA(h, cudaGetLastError());
+  if (n == 0) { h->err = "a tensor map of the forward could not be made"; return JF_ERR_CUDA; }
+  h->launches += n;
+  if (elapsed_ms) cudaEventElapsedTime(elapsed_ms, h->ev0, h->ev1);
+  int e = 0;
+  JF_CUDA(h, cudaMemcpy(&e, h->wide_err, 4, cudaMemcpyDeviceToHost));
+  if (e) {
+    cudaMemset(h->wide_err, 0, 4);
+    h->err = "a wait inside a tensor-core kernel ran out (pipeline stalled)";
+    return JF_ERR_CUDA;
+  }
+  return JF_OK;
+}
+
 extern "C" int jf_forward(jf_handle h, int32_t T, const int32_t* tokens, int32_t G, const int32_t* groups,
                           int32_t n_seqs, const int32_t* block_tables, int32_t lm_row0, int32_t lm_rows,
                           int32_t n_commit, const int32_t* commits, int32_t* greedy, float* logits, void* hidden,
@@ -880,9 +940,10 @@ extern "C" int jf_forward(jf_handle h, int32_t T, const int32_t* tokens, int32_t
   if (n_commit > 0) JF_CUDA(h, cudaMemcpyAsync(c.commits, hc.data(), (size_t)n_commit * sizeof(CommitEntry), cudaMemcpyHostToDevice, h->stream));
   JF_CUDA(h, cudaMemcpyAsync(c.block_tables, block_tables, (size_t)n_seqs * c.max_pages_per_seq * 4, cudaMemcpyHostToDevice, h->stream));
   JF_CUDA(h, cudaStreamSynchronize(h->stream));     // the host vectors above go out of scope
-  int rc = launch_persistent(h, RUN_PLAN, 1, elapsed_ms);
+  const bool wide = takes_wide(h, T, hg, row_group, lm_rows, hc, n_commit);
+  int rc = wide ? run_wide(h, T, hg, lm_row0, lm_rows, elapsed_ms) : launch_persistent(h, RUN_PLAN, 1, elapsed_ms);
   if (rc != JF_OK) return rc;
-  {
+  if (!wide) {
     int dev_err = 0;
     JF_CUDA(h, cudaMemcpy(&dev_err, reinterpret_cast<const uint8_t*>(c.hdr) + offsetof(PlanHdr, error), 4, cudaMemcpyDeviceToHost));
     if (dev_err != 0) { h->err = "device-side error " + std::to_string(dev_err) + " during the forward"; return JF_ERR_CUDA; }

@@ -6,8 +6,7 @@
 // bf16 head plus a bf16 remainder and two products, so that a weight keeps about 16 bits of its mantissa).  The scores of tile
 // j + 1 are made while the softmax of tile j runs.  The accumulated output is rescaled only when a row's maximum has grown by
 // more than a factor of 2^8 (any reference point is as good as the maximum as long as nothing overflows; all sums are fp32).
-// Keys and values travel by TMA; a step's keys lie in two places, earlier tokens in pages of 256 (optional) and the step's own
-// rows, with their own maps.
+// Keys and values travel by TMA, from pages of 256 tokens or from rows made for the step.
 //
 // Warp 0: producer (one lane).  Warp 1: owns tensor memory, one lane issues the products.  Warps 2-5: softmax, one thread per row.
 // Tensor memory: scores 2 x 128 columns, output 128, weights 64 + 64 (remainder).  Every wait is bounded (see tp_wait): on a timeout
@@ -21,8 +20,8 @@ constexpr int FL_THREADS = 192;
 constexpr int FL_KEYS = 128;
 
 // Rows pair0 .. pair0 + 127 (at most heads * len) of key head `kvh`: pair p is token row0 + p % len (position pos0 + p % len) of head
-// head0 + p / len.  Own keys: position pos0 is row own_row0 of the own maps.  Earlier keys: positions 0 .. paged - 1 in pages of the
-// table at `table` (paged = 0: all keys are own ones and key_pos0 = position of row own_row0).
+// head0 + p / len.  Keys: positions 0 .. paged - 1 in pages of the table at `table`, positions key_pos0 and up as rows own_row0 and up of
+// the own maps (paged = pos0 + len = key_pos0: all in pages; paged = key_pos0 = 0: none).
 struct FlashUnit { int row0, len, pair0, pairs, head0, kvh, pos0, own_row0, key_pos0, paged, table; };
 
 struct FlashArgs {
@@ -68,9 +67,10 @@ struct FlTiles {
     const int seen = window > 0 ? max(0, u.pos0 + first_tok - window + 1) : 0;
     last = u.pos0 + last_tok;
     lo = min(seen, u.paged) / FL_KEYS * FL_KEYS;
-    n_paged = u.paged > lo ? (u.paged - lo + FL_KEYS - 1) / FL_KEYS : 0;
+    const int end = min(u.paged, last + 1);
+    n_paged = end > lo ? (end - lo + FL_KEYS - 1) / FL_KEYS : 0;
     own_lo = max(0, seen - u.key_pos0) / FL_KEYS * FL_KEYS;
-    n = n_paged + (last - u.key_pos0 - own_lo) / FL_KEYS + 1;
+    n = n_paged + (last >= u.key_pos0 ? (last - u.key_pos0 - own_lo) / FL_KEYS + 1 : 0);
   }
   int own_lo;                                            // first own key of the first own tile
 };
@@ -254,6 +254,15 @@ flash_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ C
         if constexpr (SPLIT) tmem_st16(tl + 448 + c * 16, *reinterpret_cast<uint32_t(*)[16]>(&lo[c * 16]));
       }
       tmem_st_wait();
+      if (k0 + FL_KEYS > u.pos0 + u.len) {                      // value rows behind the last key: a weight of zero does not silence what is no number
+        ok = fl_wait(&sm->v_full[s], (j >> 1) & 1, sm, a.err);
+        if (!__all_sync(0xffffffffu, ok)) break;
+        if (k0 + r >= u.pos0 + u.len) {
+#pragma unroll
+          for (int c = 0; c < VC * 8; ++c) *reinterpret_cast<uint4*>(sv + (s * VC + (c >> 3)) * CHUNK + r * 128 + (c & 7) * 16) = make_uint4(0u, 0u, 0u, 0u);
+        }
+        fence_proxy_async_smem();
+      }
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&sm->p_full);

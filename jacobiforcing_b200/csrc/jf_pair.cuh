@@ -84,6 +84,10 @@ __device__ __forceinline__ void tp_load(void* dst, const CUtensorMap* map, int x
   asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                ::"r"(smem_u32(dst)), "l"(map), "r"(x), "r"(y), "r"(bar) : "memory");
 }
+__device__ __forceinline__ void tp_load_pairs(void* dst, const CUtensorMap* map, int group, uint32_t bar) {
+  asm volatile("cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %2, %2, %3}], [%4];"
+               ::"r"(smem_u32(dst)), "l"(map), "r"(0), "r"(group), "r"(bar) : "memory");
+}
 __device__ __forceinline__ void tp_mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
@@ -121,20 +125,68 @@ struct TpGroup { const int* meta; const int* offs; const int* tile_expert; const
 // Layout of the operands beyond row-major activations and one weight matrix:
 // x_chunk_rows > 0: the activations lie as [K / 64][x_chunk_rows][64], swizzled already (the Jacobi engine's operand layout; the map
 // is the unswizzled one of its 128-byte rows); x_row0: the operand's first row (a multiple of 8).
-// up_rows > 0: gate and up matrices lie one after the other (up_rows map rows apart) in 128-row tiles, and a tile of the product takes
-// 16 gate and 16 up rows in turn (the map's boxes are 16 rows high), so that a warp of the epilogue holds whole pairs.
-struct PairLayout { int x_chunk_rows, x_row0, up_rows; };
+// pairs: gate and up matrices lie one after the other in 128-row tiles, and a tile of the product takes 16 gate and 16 up rows in
+// turn, so that a warp of the epilogue holds whole pairs.  The weight map is four-dimensional then (tp_map_pairs) and one copy
+// brings a stage; eight copies of 16 rows each held the products back (N 37888, T 1000, K 3584: 279 us against 205).
+struct PairLayout { int x_chunk_rows, x_row0, pairs; };
+
+// Few tiles (n parts > 1): every tile's k is cut into `parts` ranges that run on pairs of their own, so that a product of few features and
+// tokens still streams its weights through all SMs (N 3584, K 3584 and 18944, 24 rows: 157 us on 14 pairs, 52 us on 70).  Each
+// epilogue warp leaves its partial sums in `sums`; the last of a tile's parts to arrive (one counter per tile, CTA and warp) adds all
+// of them in the order of the ranges, whoever it is, and goes on to the epilogue.  The counters are zero before and after.
+struct PairSplit { int parts; float* sums; int* arrived; };
+
+// One epilogue warp's part: COLS columns of its 32 lanes, `live` of them in use.  Returns whether this warp came last; its tensor memory
+// holds the whole sums then.  slot: tile, CTA and warp.
+template <int COLS>
+__device__ __forceinline__ bool tp_add_parts(uint32_t taddr, const PairSplit& sp, int slot, int part, int live, int lane) {
+  float* own = sp.sums + ((size_t)slot * sp.parts + part) * COLS * 32 + lane;
+  __syncwarp();
+  for (int c = 0; c < live; c += 16) {
+    uint32_t v[16];
+    tmem_ld16(taddr + c, v);
+    tmem_ld_wait();
+#pragma unroll
+    for (int k = 0; k < 16; ++k) own[(c + k) * 32] = __uint_as_float(v[k]);
+  }
+  __threadfence();
+  __syncwarp();
+  int before = 0;
+  if (lane == 0) before = atomicAdd(&sp.arrived[slot], 1);
+  before = __shfl_sync(0xffffffffu, before, 0);
+  if (before != sp.parts - 1) return false;
+  __threadfence();
+  if (lane == 0) sp.arrived[slot] = 0;
+  const float* all = sp.sums + (size_t)slot * sp.parts * COLS * 32 + lane;
+  for (int c = 0; c < live; c += 16) {
+    float a[16];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) a[k] = __ldcg(all + (c + k) * 32);
+    for (int p = 1; p < sp.parts; ++p) {
+#pragma unroll
+      for (int k = 0; k < 16; ++k) a[k] += __ldcg(all + ((size_t)p * COLS + c + k) * 32);
+    }
+    uint32_t v[16];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) v[k] = __float_as_uint(a[k]);
+    tmem_st16(taddr + c, v);
+  }
+  tmem_st_wait();
+  return true;
+}
 
 template <class Epilogue, int BT>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TP_THREADS, 1)
 pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap, int T, int N, int K, const Epilogue epilogue, int* err,
-            TpGroup grp, PairLayout lay) {
+            TpGroup grp, PairLayout lay, PairSplit split) {
   extern __shared__ __align__(16) unsigned char tp_smem[];
   unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(tp_smem) + 1023) & ~(uintptr_t)1023);
   constexpr int TP_STAGES = tp_stages(BT), XTILE = BT / 2 * 128, SLOT = TC_WTILE + XTILE;
   TpSmem* sm = reinterpret_cast<TpSmem*>(base + TP_STAGES * SLOT);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rank = (int)tp_rank();
-  const int KT = (K + 63) / 64, nx = (N + 255) / 256, first = blockIdx.x >> 1, step = gridDim.x >> 1;
+  const int KT = (K + 63) / 64, nx = (N + 255) / 256, parts = split.parts, step = (gridDim.x >> 1) / parts;
+  // this pair's range of k and first tile (parts > 1: one tile per pair)
+  const int part = (int)(blockIdx.x >> 1) % parts, first = (int)(blockIdx.x >> 1) / parts, kt0 = part * KT / parts, kt1 = (part + 1) * KT / parts;
   pdl_trigger();
   if (threadIdx.x == 0) {
     for (int i = 0; i < TP_STAGES; ++i) { mbar_init(&sm->full[i], 1); mbar_init(&sm->empty[i], 1); }
@@ -150,14 +202,13 @@ pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CU
   __syncthreads();
   tp_cluster_sync();
   tc_fence_after();
-  // one stage's weight tile: 128 rows, or eight times 16 rows of the gate and of the up matrix in turn
+  // one stage's weight tile: 128 rows, or 64 gate and 64 up rows
   auto load_w = [&](unsigned char* dst, int x, int kt, int base_row, uint32_t bar) {
-    if (lay.up_rows == 0) {
+    if (!lay.pairs) {
       tp_load(dst, &wmap, 0, base_row + ((2 * x + rank) * KT + kt) * 128, bar);
     } else {
-      const int f0 = (2 * x + rank) * 64, row = ((f0 >> 7) * KT + kt) * 128 + (f0 & 127);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) tp_load(dst + i * 2048, &wmap, 0, row + (i >> 1) * 16 + (i & 1) * lay.up_rows, bar);
+      const int f0 = (2 * x + rank) * 64;
+      tp_load_pairs(dst, &wmap, ((f0 >> 7) * KT + kt) * 8 + (f0 & 127) / 16, bar);
     }
   };
   // the weight tiles of the first stages travel while the kernel before this one ends (which tile is the first is known when the
@@ -165,9 +216,9 @@ pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CU
   int ahead = 0;
   if (warp == 0 && lane == 0 && !grp.meta) {
     const int x = first / ((T + BT - 1) / BT);
-    for (; ahead < min(TP_STAGES, KT); ++ahead) {
+    for (; ahead < min(TP_STAGES, kt1 - kt0); ++ahead) {
       if (rank == 0) mbar_expect_tx(&sm->full[ahead], 2 * SLOT);
-      load_w(base + ahead * SLOT, x, ahead, 0, tp_in_first(&sm->full[ahead]));
+      load_w(base + ahead * SLOT, x, kt0 + ahead, 0, tp_in_first(&sm->full[ahead]));
     }
   }
   pdl_wait();
@@ -187,7 +238,7 @@ pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CU
         place(tile, x, y);
         const int t0 = (grp.meta ? grp.tile_row0[y] : y * BT) + rank * (BT / 2);
         const int w0 = grp.meta ? grp.tile_expert[y] * grp.w_rows : 0;
-        for (int kt = 0; kt < KT; ++kt, ++it) {
+        for (int kt = kt0; kt < kt1; ++kt, ++it) {
           const int s = it % TP_STAGES;
           ok = tp_wait(&sm->empty[s], ((it / TP_STAGES) & 1) ^ 1, sm, err);      // the products that read the slot retired
           if (!ok) break;
@@ -212,7 +263,7 @@ pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CU
         const uint32_t d = sm->tmem_base + (i & 1) * BT;
         ok = tp_wait(&sm->acc_empty[i & 1], ((i >> 1) & 1) ^ 1, sm, err);        // both CTAs have read it
         tc_fence_after();
-        for (int kt = 0; kt < KT && ok; ++kt, ++it) {
+        for (int kt = kt0; kt < kt1 && ok; ++kt, ++it) {
           const int s = it % TP_STAGES;
           ok = tp_wait(&sm->full[s], (it / TP_STAGES) & 1, sm, err);
           if (!ok) break;
@@ -220,7 +271,7 @@ pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CU
           const uint32_t sa = smem_u32(base + s * SLOT), sb = sa + TC_WTILE;
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk)
-            tp_mma(d, umma_desc_sw128(sa + kk * 32), umma_desc_sw128(sb + kk * 32), idesc, (kt > 0 || kk > 0) ? 1u : 0u);
+            tp_mma(d, umma_desc_sw128(sa + kk * 32), umma_desc_sw128(sb + kk * 32), idesc, (kt > kt0 || kk > 0) ? 1u : 0u);
           tp_commit(&sm->empty[s]);
         }
         if (ok) tp_commit(&sm->acc_full[i & 1]);
@@ -237,8 +288,10 @@ pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CU
       tc_fence_after();
       const int t0 = (grp.meta ? grp.tile_row0[y] : y * BT) + half * (BT / 2);
       const int rows = grp.meta ? grp.offs[grp.tile_expert[y] + 1] : T;
-      epilogue(sm->tmem_base + (i & 1) * BT + half * (BT / 2) + ((uint32_t)(q * 32) << 16), x * 256 + rank * 128 + q * 32 + lane, t0, BT / 2, rows,
-               N, lane);
+      const uint32_t taddr = sm->tmem_base + (i & 1) * BT + half * (BT / 2) + ((uint32_t)(q * 32) << 16);
+      bool mine = true;
+      if (parts > 1) mine = tp_add_parts<BT / 2>(taddr, split, tile * 16 + rank * 8 + warp - 2, part, min(BT / 2, rows - t0), lane);
+      if (mine) epilogue(taddr, x * 256 + rank * 128 + q * 32 + lane, t0, BT / 2, rows, N, lane);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) tp_arrive_cluster(tp_in_first(&sm->acc_empty[i & 1]));
@@ -276,9 +329,24 @@ inline bool tp_map(CUtensorMap* m, const void* p, uint64_t rows, uint64_t cols, 
            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// Gate and up tiles of 128 rows x 64 (both matrices [n_tiles][KT], the up matrix behind the gate matrix): boxes of four times 16 gate rows
+// and the 16 up rows that go with them.
+inline bool tp_map_pairs(CUtensorMap* m, const void* p, uint64_t n_tiles, uint64_t KT) {
+  const TpEncode f = tp_encode();
+  if (!f) return false;
+  const cuuint64_t dims[4] = {64, 16, 2, n_tiles * KT * 8}, strides[3] = {128, n_tiles * KT * 16384, 2048};
+  const cuuint32_t box[4] = {64, 16, 2, 4}, one[4] = {1, 1, 1, 1};
+  return f(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(p), dims, strides, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
+           CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
 
 // Token rows per tile: 128 when those tiles fit one wave of the pairs (the wave is over sooner: N 1024, T 2048, K 6144: 45 us against
 // 48 with 256 rows), 256 otherwise (N 2048, T 2048, K 2048: 27 us against 35).
 inline int tp_tile_rows(int N, int T) { return (long long)((N + 255) / 256) * ((T + 127) / 128) <= TP_CLUSTERS ? 128 : 256; }
+
+// Parts of k per tile: as many as pairs are idle otherwise, at least eight steps of 64 k each.
+inline int tp_parts(int tiles, int K) { return std::max(1, std::min(std::min(TP_CLUSTERS / std::max(1, tiles), (K + 63) / 64 / 8), 8)); }
+// Floats and counters that a product with parts may need (parts > 1: at most TP_CLUSTERS tiles and parts together).
+constexpr size_t TP_SUMS = (size_t)TP_CLUSTERS * 16 * 32 * 128, TP_ARRIVED = (size_t)TP_CLUSTERS * 16;
 
 }  // namespace jf

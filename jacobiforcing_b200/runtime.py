@@ -301,10 +301,15 @@ class JacobiRuntime:
         out: List[int] = []
         start = min(seq.ctx, P - 1)
         ms = 0.0
+        pages_end = (P - 1) // PAGE * PAGE     # full pages ahead of the last prompt token: chunks of their own (see below)
         while start < total:
             end = min(total, start + self.max_rows)
             if end < total and total - end < n + 1:   # keep the n+1 logit rows inside one chunk
                 end = max(start + 1, total - (n + 1))
+            # Chunks of whole pages, all of whose rows are committed, are what the library runs as one kernel per stage; the rest of
+            # the row (what a request whose pages are cached already forwards too, so that a prefix hit changes nothing) follows
+            if start % PAGE == 0 and pages_end - start >= PAGE and self.max_rows >= PAGE and self.tp_size == 1:
+                end = start + min(pages_end - start, self.max_rows // PAGE * PAGE)
             toks = row[start:end]
             T = end - start
             commits = [(i, 0, start + i) for i in range(T) if start + i < P]
