@@ -146,10 +146,34 @@ __global__ void __launch_bounds__(128) delta_unit_kernel(int T, int H, int G, in
 // ---- staging shared by the recurrences -----------------------------------------------------------------------------------------------
 // tokens per batch; two buffers of fp32 rows q | k (DR each, zero beyond dim) and of value rows in the activation type
 __host__ __device__ constexpr int lin_tb(int dr) { return dr <= 128 ? 32 : dr <= 256 ? 16 : dr <= 512 ? 8 : 4; }
-__host__ __device__ constexpr int lin_cpb(int parts) { return 128 / parts; }
+// Two fp32 lanes per instruction: the same roundings as two scalar ones at half the issue slots.
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(reinterpret_cast<unsigned long long&>(d)) : "l"(reinterpret_cast<const unsigned long long&>(a)),
+      "l"(reinterpret_cast<const unsigned long long&>(b)), "l"(reinterpret_cast<const unsigned long long&>(c)));
+  return d;
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  float2 d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(reinterpret_cast<unsigned long long&>(d)) : "l"(reinterpret_cast<const unsigned long long&>(a)),
+      "l"(reinterpret_cast<const unsigned long long&>(b)));
+  return d;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(reinterpret_cast<unsigned long long&>(d)) : "l"(reinterpret_cast<const unsigned long long&>(a)),
+      "l"(reinterpret_cast<const unsigned long long&>(b)));
+  return d;
+}
+
+// value columns per block: VC per lane.  With two and more blocks per SM the recurrences are bound by reading the staged rows from shared
+// memory (six 16-byte reads per warp and token against 24 products per column), so wide enough steps give a lane two columns, which
+// share what it read (see launch_linear).  fma.rn.f32x2 then brought 2048 tokens of the state-space recurrence from 281 to 253 us and two requests
+// of gated linear attention from 282 to 252.
+__host__ __device__ constexpr int lin_cpb(int parts, int vc) { return 128 / parts * vc; }
 template <typename AT>
-__host__ __device__ constexpr size_t lin_smem(int dr, int parts, int more_floats) {      // more_floats: per token, beside q and k
-  return 2 * (size_t)lin_tb(dr) * ((2 * (size_t)dr + more_floats) * 4 + (lin_cpb(parts) < 8 ? 8 : lin_cpb(parts)) * sizeof(AT));
+__host__ __device__ constexpr size_t lin_smem(int dr, int parts, int vc, int more_floats) {      // more_floats: per token, beside q and k
+  return 2 * (size_t)lin_tb(dr) * ((2 * (size_t)dr + more_floats) * 4 + (lin_cpb(parts, vc) < 8 ? 8 : lin_cpb(parts, vc)) * sizeof(AT));
 }
 
 // n floats of each of nb rows (row r at src + r * ld) to dst + r * dld: asynchronous 16-byte copies where everything is aligned
@@ -181,19 +205,19 @@ __device__ __forceinline__ void copy_values(AT* dst, int dld, const AT* src, siz
 // ---- gated delta rule ---------------------------------------------------------------------------------------------------------------
 // qk [T][G][q dim | k dim] and sc [T][H] from delta_unit_kernel, v [T, ldv] (H heads of vdim).  o [T, ldo] fp32 (H heads of vdim),
 // before the output norm.  state [slot][H][dim][vdim] fp32.  grid (H * blocks_per_head, entries), 128 threads.
-// Lane layout: column = warp * (32 / PARTS) + lane % (32 / PARTS), part = lane / (32 / PARTS); part r holds the key rows
+// Lane layout: columns VC (warp * (32 / PARTS) + lane % (32 / PARTS)) .. + VC - 1, part = lane / (32 / PARTS); part r holds the key rows
 // 4 (r + PARTS i) .. + 3, so the PARTS row quadruples a warp reads from shared memory at once lie next to each other.  vec: key
 // rows are multiples of 16 bytes; vvec: a block's value rows are.
 // CHAN: decays per head and key channel, dec [T, ldd] (H heads of dim), staged behind q and k.  A head in one block, a column
 // per thread (128 rows of it in registers), took 5650 us for 2048 tokens of 16 heads of 128 x 128 (16 of 148 SMs busy, one warp
 // per scheduler); cut into 16 blocks of 8 columns it is 469 us.
-template <typename AT, int DR, int PARTS, bool CHAN = false>
+template <typename AT, int DR, int PARTS, int VC, bool CHAN>
 __global__ void __launch_bounds__(128) delta_head_kernel(Batch b, const float* __restrict__ qk, const AT* __restrict__ v, int ldv,
                                                          const float4* __restrict__ scal, int H, int G, int dim, int vdim,
                                                          int blocks_per_head, int vec, int vvec, float* __restrict__ state,
                                                          float* __restrict__ o, int ldo, const float* __restrict__ dec, int ldd) {
   pdl_begin();
-  constexpr int TB = lin_tb(DR), RP = DR / PARTS, CW = 32 / PARTS, CPB = lin_cpb(PARTS), VW = CPB < 8 ? 8 : CPB;
+  constexpr int TB = lin_tb(DR), RP = DR / PARTS, CW = 32 / PARTS, CPB = lin_cpb(PARTS, VC), VW = CPB < 8 ? 8 : CPB;
   constexpr int RW = CHAN ? 3 * DR : 2 * DR;                   // floats of a staged row: q | k (| decays)
   extern __shared__ __align__(16) unsigned char hy_smem[];
   float* sqk = reinterpret_cast<float*>(hy_smem);              // [2][TB][RW]
@@ -202,16 +226,18 @@ __global__ void __launch_bounds__(128) delta_head_kernel(Batch b, const float* _
   const int h = blockIdx.x / blocks_per_head, c0 = (blockIdx.x % blocks_per_head) * CPB, e = blockIdx.y;
   const int g = h / (H / G);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int cl = warp * CW + lane % CW, part = lane / CW, col = c0 + cl;
+  const int cl = warp * CW + lane % CW, part = lane / CW, col = c0 + cl * VC;
   const int ncol = min(CPB, vdim - c0);
-  const bool live = col < vdim;
   const int start = b.ent_start[e], cnt = b.ent_start[e + 1] - start, pos0 = b.ent_pos0[e];
   float* st = state + ((size_t)b.ent_slot[e] * H + h) * dim * vdim;
-  float S[RP];
+  float2 S[VC][RP / 2];
 #pragma unroll
-  for (int i = 0; i < RP; ++i) {
+  for (int i = 0; i < RP; i += 2) {
     const int r = 4 * (part + PARTS * (i / 4)) + (i & 3);
-    S[i] = (live && r < dim && pos0 > 0) ? st[(size_t)r * vdim + col] : 0.0f;
+#pragma unroll
+    for (int c = 0; c < VC; ++c)
+      S[c][i / 2] = make_float2((col + c < vdim && r < dim && pos0 > 0) ? st[(size_t)r * vdim + col + c] : 0.0f,
+                                (col + c < vdim && r + 1 < dim && pos0 > 0) ? st[(size_t)(r + 1) * vdim + col + c] : 0.0f);
   }
   if (dim < DR)                                                // rows beyond the head's key size stay zero
     for (int i = tid; i < 2 * TB * RW; i += 128) if (i % DR >= dim) sqk[i] = 0.0f;
@@ -236,60 +262,76 @@ __global__ void __launch_bounds__(128) delta_head_kernel(Batch b, const float* _
     __syncthreads();                                           // this batch has landed; the batch before it is finished
     if (j0 + TB < cnt) fetch(j0 + TB, buf ^ 1);
     const float* qb = sqk + (size_t)buf * TB * RW + 4 * part;
-    const AT* vb = sv + (size_t)buf * TB * VW + min(cl, ncol - 1);
+    const AT* vb = sv + (size_t)buf * TB * VW + cl * VC;                     // columns beyond the head's last are never stored
     float* po = o + (size_t)(start + j0) * ldo + h * vdim + col;
-    float keep = 0.0f;                                         // lane `part` keeps the read-out of token tt = part (mod PARTS)
-    float k[RP], q[RP], a[CHAN ? RP : 1], vv;
+    float keep[VC] = {};                                       // lane `part` keeps the read-outs of token tt = part (mod PARTS)
+    float2 k[RP / 2], q[RP / 2], a[CHAN ? RP / 2 : 1];
+    float vv[VC];
     float4 s;
     auto rows = [&](int tt) {
 #pragma unroll
       for (int i = 0; i < RP / 4; ++i) {
         const float4 qq = *reinterpret_cast<const float4*>(qb + tt * RW + 4 * PARTS * i);
         const float4 kk = *reinterpret_cast<const float4*>(qb + tt * RW + DR + 4 * PARTS * i);
-        q[4 * i] = qq.x; q[4 * i + 1] = qq.y; q[4 * i + 2] = qq.z; q[4 * i + 3] = qq.w;
-        k[4 * i] = kk.x; k[4 * i + 1] = kk.y; k[4 * i + 2] = kk.z; k[4 * i + 3] = kk.w;
+        q[2 * i] = make_float2(qq.x, qq.y); q[2 * i + 1] = make_float2(qq.z, qq.w);
+        k[2 * i] = make_float2(kk.x, kk.y); k[2 * i + 1] = make_float2(kk.z, kk.w);
         if constexpr (CHAN) {
           const float4 aa = *reinterpret_cast<const float4*>(qb + tt * RW + 2 * DR + 4 * PARTS * i);
-          a[4 * i] = aa.x; a[4 * i + 1] = aa.y; a[4 * i + 2] = aa.z; a[4 * i + 3] = aa.w;
+          a[2 * i] = make_float2(aa.x, aa.y); a[2 * i + 1] = make_float2(aa.z, aa.w);
         }
       }
       s = ssc[buf * TB + tt];
-      vv = to_f(vb[tt * VW]);
+      const VecN<AT, VC> raw = *reinterpret_cast<const VecN<AT, VC>*>(vb + tt * VW);
+#pragma unroll
+      for (int c = 0; c < VC; ++c) vv[c] = to_f(raw.v[c]);
     };
     rows(0);
 #pragma unroll 2
     for (int tt = 0; tt < nb; ++tt) {
-      float p0 = 0.0f, p1 = 0.0f, r0 = 0.0f, r1 = 0.0f, kc[RP];
-      if constexpr (CHAN) {
+      float p[VC], r[VC], vn[VC];
+      float2 kc[RP / 2];
 #pragma unroll
-        for (int i = 0; i < RP; ++i) S[i] *= a[i];
-      }
+      for (int c = 0; c < VC; ++c) {
+        if constexpr (CHAN) {
 #pragma unroll
-      for (int i = 0; i < RP; i += 2) {
-        p0 = fmaf(S[i], k[i], p0); p1 = fmaf(S[i + 1], k[i + 1], p1);
-        r0 = fmaf(S[i], q[i], r0); r1 = fmaf(S[i + 1], q[i + 1], r1);
+          for (int i = 0; i < RP / 2; ++i) S[c][i] = mul2(S[c][i], a[CHAN ? i : 0]);
+        }
+        float2 ps = make_float2(0.0f, 0.0f), rs = ps;
+#pragma unroll
+        for (int i = 0; i < RP / 2; ++i) { ps = fma2(S[c][i], k[i], ps); rs = fma2(S[c][i], q[i], rs); }
+        p[c] = ps.x + ps.y; r[c] = rs.x + rs.y; vn[c] = vv[c];
       }
-      float p = p0 + p1, r = r0 + r1;
       const float4 sn = s;
-      const float vn = vv;
 #pragma unroll
-      for (int i = 0; i < RP; ++i) kc[i] = k[i];
+      for (int i = 0; i < RP / 2; ++i) kc[i] = k[i];
       rows(min(tt + 1, nb - 1));                               // the next token's rows fly under the exchange
 #pragma unroll
-      for (int x = CW; x < 32; x <<= 1) { p += __shfl_xor_sync(0xffffffffu, p, x); r += __shfl_xor_sync(0xffffffffu, r, x); }
-      const float u = CHAN ? sn.y * (vn - p) : sn.y * fmaf(-sn.x, p, vn);
+      for (int x = CW; x < 32; x <<= 1) {
 #pragma unroll
-      for (int i = 0; i < RP; ++i) S[i] = CHAN ? fmaf(kc[i], u, S[i]) : fmaf(sn.x, S[i], kc[i] * u);
+        for (int c = 0; c < VC; ++c) { p[c] += __shfl_xor_sync(0xffffffffu, p[c], x); r[c] += __shfl_xor_sync(0xffffffffu, r[c], x); }
+      }
       const int slot = tt & (PARTS - 1);
-      if (slot == part) keep = CHAN ? fmaf(sn.z, u, r) : fmaf(sn.z, u, sn.x * r);
-      if ((slot == PARTS - 1 || tt == nb - 1) && live && part <= slot) po[(size_t)(tt - slot + part) * ldo] = keep;
+#pragma unroll
+      for (int c = 0; c < VC; ++c) {
+        const float u = CHAN ? sn.y * (vn[c] - p[c]) : sn.y * fmaf(-sn.x, p[c], vn[c]);
+#pragma unroll
+        for (int i = 0; i < RP / 2; ++i)
+          S[c][i] = CHAN ? fma2(kc[i], make_float2(u, u), S[c][i]) : fma2(make_float2(sn.x, sn.x), S[c][i], mul2(kc[i], make_float2(u, u)));
+        if (slot == part) keep[c] = CHAN ? fmaf(sn.z, u, r[c]) : fmaf(sn.z, u, sn.x * r[c]);
+      }
+      if ((slot == PARTS - 1 || tt == nb - 1) && part <= slot) {
+#pragma unroll
+        for (int c = 0; c < VC; ++c) if (col + c < vdim) po[(size_t)(tt - slot + part) * ldo + c] = keep[c];
+      }
     }
   }
-  if (live) {
 #pragma unroll
-    for (int i = 0; i < RP; ++i) {
-      const int r = 4 * (part + PARTS * (i / 4)) + (i & 3);
-      if (r < dim) st[(size_t)r * vdim + col] = S[i];
+  for (int i = 0; i < RP; i += 2) {
+    const int r = 4 * (part + PARTS * (i / 4)) + (i & 3);
+#pragma unroll
+    for (int c = 0; c < VC; ++c) {
+      if (r < dim && col + c < vdim) st[(size_t)r * vdim + col + c] = S[c][i / 2].x;
+      if (r + 1 < dim && col + c < vdim) st[(size_t)(r + 1) * vdim + col + c] = S[c][i / 2].y;
     }
   }
 }

@@ -1696,22 +1696,36 @@ void launch_conv(hy_engine* h, const Batch& b, const AT* u, int ldu, int col0, i
 
 // Register layout of a matrix-state recurrence by key size: fn(padded key size, lanes per column), both compile-time.
 constexpr int HY_LIN_MAX_DIM = 1024;
+// Value columns per lane: two where that still leaves most SMs a block.  Kernel time with one -> two, 2048 tokens, heads of 128 x 128: delta
+// rule with channel decays, 16 heads 449 -> 430 us; state-space recurrence, 32 heads of 64 columns 253 -> 237; and with two requests of
+// 1024 tokens: gated linear attention, 16 heads 293 -> 252, delta rule 221 -> 186.  Four leave a warp per scheduler and lose to one (two
+// requests, gated linear attention: 437 us), as do two where half of the SMs would get no block.  bf16 builds only: a column pair of an fp32
+// build has not been measured.
 template <typename AT, typename Fn>
-void launch_linear(int dk, Fn fn) {
-  if (dk <= 16) fn(std::integral_constant<int, 16>{}, std::integral_constant<int, 4>{});
-  else if (dk <= 32) fn(std::integral_constant<int, 32>{}, std::integral_constant<int, 8>{});
-  else if (dk <= 64) fn(std::integral_constant<int, 64>{}, std::integral_constant<int, 16>{});
-  else if (dk <= 128) fn(std::integral_constant<int, 128>{}, std::integral_constant<int, 16>{});
-  else if (dk <= 256) fn(std::integral_constant<int, 256>{}, std::integral_constant<int, 32>{});
-  else if (dk <= 512) fn(std::integral_constant<int, 512>{}, std::integral_constant<int, 32>{});
-  else fn(std::integral_constant<int, 1024>{}, std::integral_constant<int, 32>{});
+void launch_linear(int dk, int heads, int dv, int E, Fn fn) {
+  typedef std::integral_constant<int, 1> c1; typedef std::integral_constant<int, 2> c2;
+  auto wide = [&](auto dr, auto parts) {
+    constexpr int CPB = lin_cpb(decltype(parts)::value, 1);
+    auto blocks = [&](int vc) { return (long long)heads * E * ((dv + CPB * vc - 1) / (CPB * vc)); };
+    if constexpr (std::is_same<AT, bf16>::value) {
+      if (blocks(2) >= 120) { fn(dr, parts, c2{}); return; }
+    }
+    fn(dr, parts, c1{});
+  };
+  if (dk <= 16) fn(std::integral_constant<int, 16>{}, std::integral_constant<int, 4>{}, c1{});
+  else if (dk <= 32) fn(std::integral_constant<int, 32>{}, std::integral_constant<int, 8>{}, c1{});
+  else if (dk <= 64) wide(std::integral_constant<int, 64>{}, std::integral_constant<int, 16>{});
+  else if (dk <= 128) wide(std::integral_constant<int, 128>{}, std::integral_constant<int, 16>{});
+  else if (dk <= 256) fn(std::integral_constant<int, 256>{}, std::integral_constant<int, 32>{}, c1{});
+  else if (dk <= 512) fn(std::integral_constant<int, 512>{}, std::integral_constant<int, 32>{}, c1{});
+  else fn(std::integral_constant<int, 1024>{}, std::integral_constant<int, 32>{}, c1{});
 }
 
 // Blocks per head of a recurrence and which of its rows may travel by 16-byte copies.
 struct LinearLaunch { int bph, vec, vvec; };
 template <typename AT>
-LinearLaunch linear_launch(int parts, int dk, int dv, const AT* v, int ldv) {
-  const int cpb = lin_cpb(parts), ch = 16 / (int)sizeof(AT);
+LinearLaunch linear_launch(int parts, int vc, int dk, int dv, const AT* v, int ldv) {
+  const int cpb = lin_cpb(parts, vc), ch = 16 / (int)sizeof(AT);
   return LinearLaunch{(dv + cpb - 1) / cpb, dk % 4 == 0 ? 1 : 0,
                       dv % ch == 0 && cpb % ch == 0 && ldv % ch == 0 && (reinterpret_cast<uintptr_t>(v) & 15) == 0 ? 1 : 0};
 }
@@ -1961,12 +1975,12 @@ int sandwich_layer(hy_engine* h, const Batch& b, size_t li) {
     {
       ProfScope ps(h, HY_PROF_SCAN);
       const GlaToken tk{G, pin + 2 * inner + 2 * GN, h->ld_pin, L.m_dt_bias, L.m_A_log, L.m_D};
-      launch_linear<AT>(N, [&](auto dr, auto parts) {
-        constexpr int DR = decltype(dr)::value, PARTS = decltype(parts)::value;
-        const LinearLaunch g = linear_launch<AT>(PARTS, N, P, cv, h->ld_cv);
-        const size_t smem = lin_smem<AT>(DR, PARTS, 0);
-        cudaFuncSetAttribute(gla_kernel<AT, DR, PARTS, GLA_TOKEN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        go_kernel(h, gla_kernel<AT, DR, PARTS, GLA_TOKEN>, dim3(H * g.bph, E), 128, smem, s, b, h->lin, cv, h->ld_cv, nullptr, 0, nullptr, H, N, P, g.bph,
+      launch_linear<AT>(N, H, P, E, [&](auto dr, auto parts, auto vcols) {
+        constexpr int DR = decltype(dr)::value, PARTS = decltype(parts)::value, VC = decltype(vcols)::value;
+        const LinearLaunch g = linear_launch<AT>(PARTS, VC, N, P, cv, h->ld_cv);
+        const size_t smem = lin_smem<AT>(DR, PARTS, VC, 0);
+        cudaFuncSetAttribute(gla_kernel<AT, DR, PARTS, VC, GLA_TOKEN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        go_kernel(h, gla_kernel<AT, DR, PARTS, VC, GLA_TOKEN>, dim3(H * g.bph, E), 128, smem, s, b, h->lin, cv, h->ld_cv, nullptr, 0, nullptr, H, N, P, g.bph,
                                                                                    g.vec, g.vvec, L.rec_state, h->f2, h->ld_f2, tk);
       });
       go_kernel(h, gated_group_norm_kernel<AT>, dim3(T, c.m_norm_groups), 128, 0, s, h->f2, h->ld_f2, pin, h->ld_pin, L.m_norm, inner,
@@ -1988,12 +2002,12 @@ int sandwich_layer(hy_engine* h, const Batch& b, size_t li) {
     ProfScope ps(h, HY_PROF_DELTA);
     if (dk <= HY_LIN_MAX_DIM) {
       go_kernel(h, forget_rows_kernel<AT>, T, T <= 8 ? 1024 : 256, 0, s, pin, h->ld_pin, L.c_q, L.c_k, L.g_fb, L.g_lower, H, dk, h->lin);
-      launch_linear<AT>(dk, [&](auto dr, auto parts) {
-        constexpr int DR = decltype(dr)::value, PARTS = decltype(parts)::value;
-        const LinearLaunch g = linear_launch<AT>(PARTS, dk, dv, pin + L.c_v, h->ld_pin);
-        const size_t smem = lin_smem<AT>(DR, PARTS, 0);
-        cudaFuncSetAttribute(gla_kernel<AT, DR, PARTS, GLA_FORGET>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        go_kernel(h, gla_kernel<AT, DR, PARTS, GLA_FORGET>, dim3(H * g.bph, E), 128, smem, s, b, h->lin, pin + L.c_v, h->ld_pin, nullptr, 0, nullptr, H, dk,
+      launch_linear<AT>(dk, H, dv, E, [&](auto dr, auto parts, auto vcols) {
+        constexpr int DR = decltype(dr)::value, PARTS = decltype(parts)::value, VC = decltype(vcols)::value;
+        const LinearLaunch g = linear_launch<AT>(PARTS, VC, dk, dv, pin + L.c_v, h->ld_pin);
+        const size_t smem = lin_smem<AT>(DR, PARTS, VC, 0);
+        cudaFuncSetAttribute(gla_kernel<AT, DR, PARTS, VC, GLA_FORGET>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        go_kernel(h, gla_kernel<AT, DR, PARTS, VC, GLA_FORGET>, dim3(H * g.bph, E), 128, smem, s, b, h->lin, pin + L.c_v, h->ld_pin, nullptr, 0, nullptr, H, dk,
                                                                                     dv, g.bph, g.vec, g.vvec, L.rec_state, h->f2, h->ld_f2, GlaToken{});
       });
       go_kernel(h, gla_out_kernel<AT, AT, GATE_NONE>, (T * H + 3) / 4, 128, 0, s, T, H, dv, h->f2, h->ld_f2, nullptr, 0, L.g_norm, eps, 1.0f, cat, h->ld_cat);
@@ -2538,12 +2552,12 @@ void gla_mixer(hy_engine* h, const Batch& b, const LayerW& L, const hy_layer_cfg
   }
   ProfScope ps(h, HY_PROF_DELTA);
   go_kernel(h, linear_rows_kernel<AT>, T, T <= 8 ? 1024 : 128, 0, s, pin, h->ld_pin, L.c_q, L.c_k, H, dk, nullptr, 0, RotPair{0, 1}, h->lin);
-  launch_linear<AT>(dk, [&](auto dr, auto parts) {
-    constexpr int DR = decltype(dr)::value, PARTS = decltype(parts)::value;
-    const LinearLaunch g = linear_launch<AT>(PARTS, dk, dv, pin + L.c_v, h->ld_pin);
-    const size_t smem = lin_smem<AT>(DR, PARTS, DR);
-    cudaFuncSetAttribute(gla_kernel<AT, DR, PARTS, GLA_CHANNEL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    go_kernel(h, gla_kernel<AT, DR, PARTS, GLA_CHANNEL>, dim3(H * g.bph, E), 128, smem, s, b, h->lin, pin + L.c_v, h->ld_pin, h->f2, h->ld_f2, nullptr, H, dk,
+  launch_linear<AT>(dk, H, dv, E, [&](auto dr, auto parts, auto vcols) {
+    constexpr int DR = decltype(dr)::value, PARTS = decltype(parts)::value, VC = decltype(vcols)::value;
+    const LinearLaunch g = linear_launch<AT>(PARTS, VC, dk, dv, pin + L.c_v, h->ld_pin);
+    const size_t smem = lin_smem<AT>(DR, PARTS, VC, DR);
+    cudaFuncSetAttribute(gla_kernel<AT, DR, PARTS, VC, GLA_CHANNEL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    go_kernel(h, gla_kernel<AT, DR, PARTS, VC, GLA_CHANNEL>, dim3(H * g.bph, E), 128, smem, s, b, h->lin, pin + L.c_v, h->ld_pin, h->f2, h->ld_f2, nullptr, H, dk,
                                                                            dv, g.bph, g.vec, g.vvec, L.rec_state, h->f2 + c_o, h->ld_f2, GlaToken{});
   });
   go_kernel(h, gla_out_kernel<AT>, (T * H + 3) / 4, 128, 0, s, T, H, dv, h->f2 + c_o, h->ld_f2, pin + L.c_g, h->ld_pin, L.g_norm, h->m.norm_eps,
@@ -2561,12 +2575,12 @@ void retention_mixer(hy_engine* h, const Batch& b, const LayerW& L, const hy_lay
   const RotPair rp{rot.pairs, c.r_half};
   ProfScope ps(h, HY_PROF_DELTA);
   go_kernel(h, linear_rows_kernel<AT>, T, T <= 8 ? 1024 : 128, 0, s, pin, h->ld_pin, L.c_q, L.c_k, H, dk, rot.out, rot.ld, rp, h->lin);
-  launch_linear<AT>(dk, [&](auto dr, auto parts) {
-    constexpr int DR = decltype(dr)::value, PARTS = decltype(parts)::value;
-    const LinearLaunch g = linear_launch<AT>(PARTS, dk, dv, pin + L.c_v, h->ld_pin);
-    const size_t smem = lin_smem<AT>(DR, PARTS, 0);
-    cudaFuncSetAttribute(gla_kernel<AT, DR, PARTS, GLA_HEAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    go_kernel(h, gla_kernel<AT, DR, PARTS, GLA_HEAD>, dim3(H * g.bph, E), 128, smem, s, b, h->lin, pin + L.c_v, h->ld_pin, nullptr, 0, L.decay, H, dk, dv,
+  launch_linear<AT>(dk, H, dv, E, [&](auto dr, auto parts, auto vcols) {
+    constexpr int DR = decltype(dr)::value, PARTS = decltype(parts)::value, VC = decltype(vcols)::value;
+    const LinearLaunch g = linear_launch<AT>(PARTS, VC, dk, dv, pin + L.c_v, h->ld_pin);
+    const size_t smem = lin_smem<AT>(DR, PARTS, VC, 0);
+    cudaFuncSetAttribute(gla_kernel<AT, DR, PARTS, VC, GLA_HEAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    go_kernel(h, gla_kernel<AT, DR, PARTS, VC, GLA_HEAD>, dim3(H * g.bph, E), 128, smem, s, b, h->lin, pin + L.c_v, h->ld_pin, nullptr, 0, L.decay, H, dk, dv,
                                                                           g.bph, g.vec, g.vvec, L.rec_state, h->f2, h->ld_f2, GlaToken{});
   });
   go_kernel(h, gla_out_kernel<AT>, (T * H + 3) / 4, 128, 0, s, T, H, dv, h->f2, h->ld_f2, pin + L.c_g, h->ld_pin, nullptr, h->m.norm_eps, 1.0f, cat,
@@ -2599,12 +2613,12 @@ void attn_delta_mixer(hy_engine* h, const Batch& b, const LayerW& L, const hy_la
                      h->f1, h->ld_f1, c.left_scale};
   biased_attend<AT>(h, b, L, c, bc);
   ProfScope ps(h, HY_PROF_DELTA);
-  launch_linear<AT>(dk, [&](auto dr, auto parts) {
-    constexpr int DR = decltype(dr)::value, PARTS = decltype(parts)::value;
-    const LinearLaunch g = linear_launch<AT>(PARTS, dk, dv, cv, h->ld_cv);
-    const size_t smem = lin_smem<AT>(DR, PARTS, 4);
-    cudaFuncSetAttribute(delta_head_kernel<AT, DR, PARTS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    go_kernel(h, delta_head_kernel<AT, DR, PARTS>, dim3(H * g.bph, E), 128, smem, s, b, h->lin, cv, h->ld_cv, h->lin_sc, H, G, dk, dv, g.bph, g.vec, g.vvec,
+  launch_linear<AT>(dk, H, dv, E, [&](auto dr, auto parts, auto vcols) {
+    constexpr int DR = decltype(dr)::value, PARTS = decltype(parts)::value, VC = decltype(vcols)::value;
+    const LinearLaunch g = linear_launch<AT>(PARTS, VC, dk, dv, cv, h->ld_cv);
+    const size_t smem = lin_smem<AT>(DR, PARTS, VC, 4);
+    cudaFuncSetAttribute(delta_head_kernel<AT, DR, PARTS, VC, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    go_kernel(h, delta_head_kernel<AT, DR, PARTS, VC, false>, dim3(H * g.bph, E), 128, smem, s, b, h->lin, cv, h->ld_cv, h->lin_sc, H, G, dk, dv, g.bph, g.vec, g.vvec,
                                                                            L.rec_state, h->f2, h->ld_f2, nullptr, 0);
   });
   go_kernel(h, gla_out_kernel<AT>, (T * H + 3) / 4, 128, 0, s, T, H, dv, h->f2, h->ld_f2, pin + L.c_g, h->ld_pin, L.g_norm, h->m.norm_eps,
@@ -2893,12 +2907,12 @@ int run_step(hy_engine* h, const Batch& b, int n_want, const int* want_d, float*
       }
       ProfScope ps(h, HY_PROF_DELTA);
       float* o = h->f2 + ((nv + 3) & ~3);                      // behind the output gates
-      launch_linear<AT>(dk, [&](auto dr, auto parts) {
-        constexpr int DR = decltype(dr)::value, PARTS = decltype(parts)::value;
-        const LinearLaunch g = linear_launch<AT>(PARTS, dk, dv, cv, h->ld_cv);
-        const size_t smem = lin_smem<AT>(DR, PARTS, DR + 4);
-        cudaFuncSetAttribute(delta_head_kernel<AT, DR, PARTS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        go_kernel(h, delta_head_kernel<AT, DR, PARTS, true>, dim3(H * g.bph, E), 128, smem, s, b, h->lin, cv, h->ld_cv, h->lin_sc, H, G, dk, dv, g.bph, g.vec,
+      launch_linear<AT>(dk, H, dv, E, [&](auto dr, auto parts, auto vcols) {
+        constexpr int DR = decltype(dr)::value, PARTS = decltype(parts)::value, VC = decltype(vcols)::value;
+        const LinearLaunch g = linear_launch<AT>(PARTS, VC, dk, dv, cv, h->ld_cv);
+        const size_t smem = lin_smem<AT>(DR, PARTS, VC, DR + 4);
+        cudaFuncSetAttribute(delta_head_kernel<AT, DR, PARTS, VC, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        go_kernel(h, delta_head_kernel<AT, DR, PARTS, VC, true>, dim3(H * g.bph, E), 128, smem, s, b, h->lin, cv, h->ld_cv, h->lin_sc, H, G, dk, dv, g.bph, g.vec,
                                                                                      g.vvec, L.rec_state, o, h->ld_f2, h->f1, h->ld_f1);
       });
       go_kernel(h, gla_out_kernel<AT, float, GATE_SIGMOID>, (T * H + 3) / 4, 128, 0, s, T, H, dv, o, h->ld_f2, h->f2, h->ld_f2, (const float*)L.norm_w, eps,

@@ -31,13 +31,13 @@ namespace hy {
 // GLA_FORGET, 2048 tokens of 8 heads of 128 x 128: one block per head with a column per thread took 1927 us, this layout 202 us.
 enum GlaMode : int { GLA_CHANNEL = 0, GLA_HEAD = 1, GLA_FORGET = 2, GLA_TOKEN = 3 };
 struct GlaToken { int G; const void* dt_raw; int lddt; const float* dt_bias; const float* A_log; const float* D; };
-template <typename AT, int DR, int PARTS, int MODE>
+template <typename AT, int DR, int PARTS, int VC, int MODE>
 __global__ void __launch_bounds__(128) gla_kernel(Batch b, const float* __restrict__ qk, const AT* __restrict__ v, int ldv,
                                                   const float* __restrict__ decay, int ldd, const float* __restrict__ head_decay, int H,
                                                   int dim, int vdim, int blocks_per_head, int vec, int vvec, float* __restrict__ state,
                                                   float* __restrict__ o, int ldo, GlaToken tk) {
   pdl_begin();
-  constexpr int TB = lin_tb(DR), RP = DR / PARTS, CW = 32 / PARTS, CPB = lin_cpb(PARTS), VW = CPB < 8 ? 8 : CPB;
+  constexpr int TB = lin_tb(DR), RP = DR / PARTS, CW = 32 / PARTS, CPB = lin_cpb(PARTS, VC), VW = CPB < 8 ? 8 : CPB;
   constexpr bool HEAD = MODE == GLA_HEAD;
   constexpr int RW = MODE == GLA_CHANNEL ? 3 * DR : 2 * DR;    // floats of a staged row: q | k (| decays)
   extern __shared__ __align__(16) unsigned char hy_smem[];
@@ -46,16 +46,18 @@ __global__ void __launch_bounds__(128) gla_kernel(Batch b, const float* __restri
   __shared__ float2 sdt[MODE == GLA_TOKEN ? 2 * TB : 1];       // [2][TB] decay, step size
   const int h = blockIdx.x / blocks_per_head, c0 = (blockIdx.x % blocks_per_head) * CPB, e = blockIdx.y;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int cl = warp * CW + lane % CW, part = lane / CW, col = c0 + cl;
+  const int cl = warp * CW + lane % CW, part = lane / CW, col = c0 + cl * VC;
   const int ncol = min(CPB, vdim - c0);
-  const bool live = col < vdim;
   const int start = b.ent_start[e], cnt = b.ent_start[e + 1] - start, pos0 = b.ent_pos0[e];
   float* st = state + ((size_t)b.ent_slot[e] * H + h) * dim * vdim;
-  float S[RP];
+  float2 S[VC][RP / 2];
 #pragma unroll
-  for (int i = 0; i < RP; ++i) {
+  for (int i = 0; i < RP; i += 2) {
     const int r = 4 * (part + PARTS * (i / 4)) + (i & 3);
-    S[i] = (live && r < dim && pos0 > 0) ? st[(size_t)r * vdim + col] : 0.0f;
+#pragma unroll
+    for (int c = 0; c < VC; ++c)
+      S[c][i / 2] = make_float2((col + c < vdim && r < dim && pos0 > 0) ? st[(size_t)r * vdim + col + c] : 0.0f,
+                                (col + c < vdim && r + 1 < dim && pos0 > 0) ? st[(size_t)(r + 1) * vdim + col + c] : 0.0f);
   }
   const float hd = HEAD ? head_decay[h] : 0.0f;
   const int rows_per_token = MODE == GLA_TOKEN ? tk.G : H, row_of = MODE == GLA_TOKEN ? h / (H / tk.G) : h;
@@ -90,43 +92,70 @@ __global__ void __launch_bounds__(128) gla_kernel(Batch b, const float* __restri
     __syncthreads();                                           // this batch has landed; the batch before it is finished
     if (j0 + TB < cnt) fetch(j0 + TB, buf ^ 1);
     const float* rb = sqk + (size_t)buf * TB * RW + 4 * part;
-    const AT* vb = sv + (size_t)buf * TB * VW + min(cl, ncol - 1);
+    const AT* vb = sv + (size_t)buf * TB * VW + cl * VC;                     // columns beyond the head's last are never stored
     float* po = o + (size_t)(start + j0) * ldo + h * vdim + col;
-    auto leave = [&](int tt, float p) {
-      if constexpr (MODE == GLA_TOKEN) p = fmaf(skip, to_f(vb[tt * VW]), p);
-      po[(size_t)tt * ldo] = p;
+    auto leave = [&](int tt, int c, float p) {
+      if constexpr (MODE == GLA_TOKEN) p = fmaf(skip, to_f(vb[tt * VW + c]), p);
+      if (col + c < vdim) po[(size_t)tt * ldo + c] = p;
     };
-    // one token's update of this lane's key rows; returns its part of the read-out
-    auto update = [&](int tt) {
-      float vv = to_f(vb[tt * VW]), td = hd;
-      if constexpr (MODE == GLA_TOKEN) { const float2 sd = sdt[buf * TB + tt]; td = sd.x; vv *= sd.y; }
-      float p0 = 0.0f, p1 = 0.0f;
+    // one token's rows in registers; where they are few, the next token's are read before this one's products, which covers their latency
+    struct Row { float4 q[RP / 4], k[RP / 4], a[MODE == GLA_CHANNEL ? RP / 4 : 1]; VecN<AT, VC> v; float2 sd; };
+    auto read = [&](Row& w, int tt) {
 #pragma unroll
       for (int i = 0; i < RP / 4; ++i) {
-        const float4 q = *reinterpret_cast<const float4*>(rb + tt * RW + 4 * PARTS * i);
-        const float4 k = *reinterpret_cast<const float4*>(rb + tt * RW + DR + 4 * PARTS * i);
-        float* R = &S[4 * i];
-        if constexpr (MODE == GLA_FORGET) {
-          R[0] = fmaf(k.x, R[0] - vv, vv); p0 = fmaf(R[0], q.x, p0);
-          R[1] = fmaf(k.y, R[1] - vv, vv); p1 = fmaf(R[1], q.y, p1);
-          R[2] = fmaf(k.z, R[2] - vv, vv); p0 = fmaf(R[2], q.z, p0);
-          R[3] = fmaf(k.w, R[3] - vv, vv); p1 = fmaf(R[3], q.w, p1);
-          continue;
-        }
-        const float4 a = HEAD || MODE == GLA_TOKEN ? make_float4(td, td, td, td) : *reinterpret_cast<const float4*>(rb + tt * RW + (MODE == GLA_CHANNEL ? 2 * DR : 0) + 4 * PARTS * i);
-        R[0] = fmaf(a.x, R[0], k.x * vv); p0 = fmaf(R[0], q.x, p0);
-        R[1] = fmaf(a.y, R[1], k.y * vv); p1 = fmaf(R[1], q.y, p1);
-        R[2] = fmaf(a.z, R[2], k.z * vv); p0 = fmaf(R[2], q.z, p0);
-        R[3] = fmaf(a.w, R[3], k.w * vv); p1 = fmaf(R[3], q.w, p1);
+        w.q[i] = *reinterpret_cast<const float4*>(rb + tt * RW + 4 * PARTS * i);
+        w.k[i] = *reinterpret_cast<const float4*>(rb + tt * RW + DR + 4 * PARTS * i);
+        if constexpr (MODE == GLA_CHANNEL) w.a[i] = *reinterpret_cast<const float4*>(rb + tt * RW + 2 * DR + 4 * PARTS * i);
       }
-      return p0 + p1;
+      w.v = *reinterpret_cast<const VecN<AT, VC>*>(vb + tt * VW);
+      if constexpr (MODE == GLA_TOKEN) w.sd = sdt[buf * TB + tt];
     };
+    // one token's update of this lane's key rows and columns; leaves its parts of the read-outs
+    auto update = [&](const Row& w, float (&out)[VC]) {
+      float2 p[VC], vv[VC];
+#pragma unroll
+      for (int c = 0; c < VC; ++c) {
+        float x = to_f(w.v.v[c]);
+        if constexpr (MODE == GLA_TOKEN) x *= w.sd.y;
+        vv[c] = make_float2(x, x);
+        p[c] = make_float2(0.0f, 0.0f);
+      }
+      const float td = MODE == GLA_TOKEN ? w.sd.x : hd;
+#pragma unroll
+      for (int i = 0; i < RP / 4; ++i) {
+        const float4 q = w.q[i], k = w.k[i], a = MODE == GLA_CHANNEL ? w.a[MODE == GLA_CHANNEL ? i : 0] : make_float4(td, td, td, td);
+#pragma unroll
+        for (int c = 0; c < VC; ++c) {
+          float2 &R0 = S[c][2 * i], &R1 = S[c][2 * i + 1];
+          if constexpr (MODE == GLA_FORGET) {
+            const float2 less = make_float2(-vv[c].x, -vv[c].y);
+            R0 = fma2(make_float2(k.x, k.y), add2(R0, less), vv[c]);
+            R1 = fma2(make_float2(k.z, k.w), add2(R1, less), vv[c]);
+          } else {
+            R0 = fma2(make_float2(a.x, a.y), R0, mul2(make_float2(k.x, k.y), vv[c]));
+            R1 = fma2(make_float2(a.z, a.w), R1, mul2(make_float2(k.z, k.w), vv[c]));
+          }
+          p[c] = fma2(R0, make_float2(q.x, q.y), p[c]);
+          p[c] = fma2(R1, make_float2(q.z, q.w), p[c]);
+        }
+      }
+#pragma unroll
+      for (int c = 0; c < VC; ++c) out[c] = p[c].x + p[c].y;
+    };
+    constexpr bool FLY = RP <= 8;
+    static_assert(!FLY || TG % 2 == 0, "a group of tokens leaves the next row where the next group begins");
+    Row w[FLY ? 2 : 1];
+    if (FLY) read(w[0], 0);
     int tt = 0;
     for (; tt + TG <= nb; tt += TG) {
       // TG tokens without a shuffle between them, then one exchange in which every step halves the tokens a lane keeps
-      float p[TG];
+      float p[TG][VC];
 #pragma unroll
-      for (int u = 0; u < TG; ++u) p[u] = update(tt + u);
+      for (int u = 0; u < TG; ++u) {
+        if constexpr (FLY) read(w[(u + 1) & 1], min(tt + u + 1, nb - 1));
+        else read(w[0], tt + u);
+        update(w[FLY ? u & 1 : 0], p[u]);
+      }
       int n = TG, base = 0;
 #pragma unroll
       for (int s = 16; s >= CW; s >>= 1) {
@@ -136,32 +165,45 @@ __global__ void __launch_bounds__(128) gla_kernel(Batch b, const float* __restri
 #pragma unroll
           for (int u = 0; u < TG / 2; ++u) {
             if (u >= n) break;
-            const float other = __shfl_xor_sync(0xffffffffu, hi ? p[u] : p[u + n], s);
-            p[u] = (hi ? p[u + n] : p[u]) + other;
+#pragma unroll
+            for (int c = 0; c < VC; ++c) {
+              const float other = __shfl_xor_sync(0xffffffffu, hi ? p[u][c] : p[u + n][c], s);
+              p[u][c] = (hi ? p[u + n][c] : p[u][c]) + other;
+            }
           }
           base += hi ? n : 0;
         } else {
-          p[0] += __shfl_xor_sync(0xffffffffu, p[0], s);
+#pragma unroll
+          for (int c = 0; c < VC; ++c) p[0][c] += __shfl_xor_sync(0xffffffffu, p[0][c], s);
         }
       }
       constexpr int LEFT = TG > PARTS ? TG / PARTS : 1, SAME = PARTS > TG ? PARTS / TG : 1;     // tokens per lane, lanes per token
-      if (live && (part & (SAME - 1)) == 0) {
+      if ((part & (SAME - 1)) == 0) {
 #pragma unroll
-        for (int u = 0; u < LEFT; ++u) leave(tt + base + u, p[u]);
+        for (int u = 0; u < LEFT; ++u)
+#pragma unroll
+          for (int c = 0; c < VC; ++c) leave(tt + base + u, c, p[u][c]);
       }
     }
     for (; tt < nb; ++tt) {
-      float p = update(tt);
+      float p[VC];
+      read(w[0], tt);
+      update(w[0], p);
 #pragma unroll
-      for (int s = CW; s < 32; s <<= 1) p += __shfl_xor_sync(0xffffffffu, p, s);
-      if (live && part == 0) leave(tt, p);
+      for (int c = 0; c < VC; ++c) {
+#pragma unroll
+        for (int s = CW; s < 32; s <<= 1) p[c] += __shfl_xor_sync(0xffffffffu, p[c], s);
+        if (part == 0) leave(tt, c, p[c]);
+      }
     }
   }
-  if (live) {
 #pragma unroll
-    for (int i = 0; i < RP; ++i) {
-      const int r = 4 * (part + PARTS * (i / 4)) + (i & 3);
-      if (r < dim) st[(size_t)r * vdim + col] = S[i];
+  for (int i = 0; i < RP; i += 2) {
+    const int r = 4 * (part + PARTS * (i / 4)) + (i & 3);
+#pragma unroll
+    for (int c = 0; c < VC; ++c) {
+      if (r < dim && col + c < vdim) st[(size_t)r * vdim + col + c] = S[c][i / 2].x;
+      if (r + 1 < dim && col + c < vdim) st[(size_t)(r + 1) * vdim + col + c] = S[c][i / 2].y;
     }
   }
 }

@@ -14,11 +14,11 @@ pytestmark = pytest.mark.gpu
 CUTS = [31, 1, 33, 2, 32, 8, 64]                               # staged batches hold 32 tokens (16 or fewer at large key sizes)
 
 
-def _kinetar(layer, cuts=CUTS, width=48):
+def _kinetar(layer, cuts=CUTS, width=48, dtype="float32"):
     cfg = kin.model_config([layer], width=width)
     toks = kin.rand_tokens(sum(cuts), cfg["vocab"], 3)
     w = kinetar_plain.random_weights(cfg, 0, 8)
-    hz = kin.Harness(cfg, w, dtype="float32", low=8)
+    hz = kin.Harness(cfg, w, dtype=dtype, low=8)
     try:
         got = hz.feed("a", toks, cuts)
     finally:
@@ -79,3 +79,19 @@ def test_forget_gate_columns(dim, vdim):
     finally:
         hz.close()
     assert kin.rel_err(got, fam.oracle_logits(cfg, w, toks)) < fam.TOL["float32"]
+
+
+@pytest.mark.parametrize("dim,vdim,heads", [(64, 120, 16), (100, 113, 16), (128, 8, 120), (33, 232, 8), (128, 15, 119)])
+def test_two_columns_per_lane(dim, vdim, heads):
+    """bf16 steps with enough heads x columns for two value columns per lane (15 columns x 119 heads stay just below): ragged last blocks and
+    odd column counts, against the fp64 restatement within the bound of the other bf16 tests."""
+    cfg = fam.model_config([fam.glr(heads=heads, dim=dim, vdim=vdim, mlp=None)])
+    toks = kin.rand_tokens(sum(CUTS), cfg["vocab"], 4)
+    w = famepel_plain.random_weights(cfg, 0)
+    hz = fam.Harness(cfg, w, "bfloat16")
+    try:
+        got = hz.feed("a", toks, CUTS)
+    finally:
+        hz.close()
+    assert kin.rel_err(got, fam.oracle_logits(cfg, w, toks)) < fam.TOL["bfloat16"]
+    assert _kinetar(kin.delta(heads=heads, kv_heads=heads, dim=dim, vdim=vdim, ff=0), dtype="bfloat16") < kin.TOL["bfloat16"]
