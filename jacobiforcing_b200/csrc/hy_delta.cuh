@@ -146,26 +146,6 @@ __global__ void __launch_bounds__(128) delta_unit_kernel(int T, int H, int G, in
 // ---- staging shared by the recurrences -----------------------------------------------------------------------------------------------
 // tokens per batch; two buffers of fp32 rows q | k (DR each, zero beyond dim) and of value rows in the activation type
 __host__ __device__ constexpr int lin_tb(int dr) { return dr <= 128 ? 32 : dr <= 256 ? 16 : dr <= 512 ? 8 : 4; }
-// Two fp32 lanes per instruction: the same roundings as two scalar ones at half the issue slots.
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-  float2 d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(reinterpret_cast<unsigned long long&>(d)) : "l"(reinterpret_cast<const unsigned long long&>(a)),
-      "l"(reinterpret_cast<const unsigned long long&>(b)), "l"(reinterpret_cast<const unsigned long long&>(c)));
-  return d;
-}
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
-  float2 d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(reinterpret_cast<unsigned long long&>(d)) : "l"(reinterpret_cast<const unsigned long long&>(a)),
-      "l"(reinterpret_cast<const unsigned long long&>(b)));
-  return d;
-}
-__device__ __forceinline__ float2 add2(float2 a, float2 b) {
-  float2 d;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(reinterpret_cast<unsigned long long&>(d)) : "l"(reinterpret_cast<const unsigned long long&>(a)),
-      "l"(reinterpret_cast<const unsigned long long&>(b)));
-  return d;
-}
-
 // value columns per block: VC per lane.  With two and more blocks per SM the recurrences are bound by reading the staged rows from shared
 // memory (six 16-byte reads per warp and token against 24 products per column), so wide enough steps give a lane two columns, which
 // share what it read (see launch_linear).  fma.rn.f32x2 then brought 2048 tokens of the state-space recurrence from 281 to 253 us and two requests

@@ -1557,7 +1557,12 @@ int gemm(hy_engine* h, const TA* A, int lda, const TW* Wt, int ldw, int T, int N
     else if (T <= 4 || fit < 8) launch(gemm_rows_kernel<TA, TW, TO, 4>, 4);
     else launch(gemm_rows_kernel<TA, TW, TO, 8>, 8);
   } else {
-    go_kernel(h, gemm_simt_kernel<TA, TW, TO>, dim3((N + 63) / 64, (T + 63) / 64), 256, 0, h->stream, A, lda, Wt, ldw, T, N, K, o);
+    // Tiles of 32 where those of 64 would leave SMs without a block: the seven products of a step of 77 tokens, width 256, 337 us in unpipelined
+    // tiles of 64, 62 in these.  With a block of 64 for every SM the larger tile reads its operands half as often.
+    if ((long long)((N + 63) / 64) * ((T + 63) / 64) >= 148)
+      go_kernel(h, gemm_simt_kernel<TA, TW, TO, 64>, dim3((N + 63) / 64, (T + 63) / 64), 256, 0, h->stream, A, lda, Wt, ldw, T, N, K, o);
+    else
+      go_kernel(h, gemm_simt_kernel<TA, TW, TO, 32>, dim3((N + 31) / 32, (T + 31) / 32), 256, 0, h->stream, A, lda, Wt, ldw, T, N, K, o);
   }
   h->launches++;
   return HY_OK;
@@ -2068,9 +2073,9 @@ int sandwich_layer(hy_engine* h, const Batch& b, size_t li) {
       }
     } else {
       const int tiles = std::min(h->x_max_tiles, P / HY_XT + NE + 1);
-      go_kernel(h, expert_gemm_simt_kernel<AT, WT, AT, true>, dim3((ff + 63) / 64, tiles), 256, 0, s, 
+      go_kernel(h, expert_gemm_simt_kernel<AT, WT, AT, true>, dim3((ff + 31) / 32, tiles), 256, 0, s, 
           x_rows, W, (const WT*)L.w_gu, (size_t)2 * ff * W, ff, W, h->x_offs, h->x_tile_e, h->x_tile_r0, h->x_meta, pin, ldh, 0, 0.0f);
-      go_kernel(h, expert_gemm_simt_kernel<AT, WT, float, false>, dim3((W + 63) / 64, tiles), 256, 0, s, 
+      go_kernel(h, expert_gemm_simt_kernel<AT, WT, float, false>, dim3((W + 31) / 32, tiles), 256, 0, s, 
           pin, ldh, (const WT*)L.w_down, (size_t)W * ff, W, ff, h->x_offs, h->x_tile_e, h->x_tile_r0, h->x_meta, ys, W, -1, 0.0f);
     }
     go_kernel(h, expert_combine_kernel<AT>, T, 256, 0, s, ys, W, few ? nullptr : h->x_pair_row, h->x_wts, top, W, L.n2b, L.ls2, h->x, after_ff, hb);
@@ -2277,9 +2282,9 @@ int postnorm_layer(hy_engine* h, const Batch& b, size_t li) {
       }
     } else {
       const int tiles = std::min(h->x_max_tiles, P / HY_XT + NE + 1);
-      go_kernel(h, expert_gemm_simt_kernel<AT, WT, AT, false>, dim3((ff + 63) / 64, tiles), 256, 0, s, 
+      go_kernel(h, expert_gemm_simt_kernel<AT, WT, AT, false>, dim3((ff + 31) / 32, tiles), 256, 0, s, 
           x_rows, W, (const WT*)L.w_gu, (size_t)ff * W, ff, W, h->x_offs, h->x_tile_e, h->x_tile_r0, h->x_meta, pin, ldh, c.x_act, c.ff_limit);
-      go_kernel(h, expert_gemm_simt_kernel<AT, WT, float, false>, dim3((W + 63) / 64, tiles), 256, 0, s, 
+      go_kernel(h, expert_gemm_simt_kernel<AT, WT, float, false>, dim3((W + 31) / 32, tiles), 256, 0, s, 
           pin, ldh, (const WT*)L.w_down, (size_t)W * ff, W, ff, h->x_offs, h->x_tile_e, h->x_tile_r0, h->x_meta, ys, W, -1, 0.0f);
     }
     h->launches += 2;
@@ -2350,9 +2355,9 @@ bool routed_gated_experts(hy_engine* h, int T, const AT* hb, const LayerW& L, co
     }
   } else {
     const int tiles = std::min(h->x_max_tiles, P / HY_XT + NE + 1);
-    go_kernel(h, expert_gemm_simt_kernel<AT, WT, AT, true>, dim3((ff + 63) / 64, tiles), 256, 0, s, 
+    go_kernel(h, expert_gemm_simt_kernel<AT, WT, AT, true>, dim3((ff + 31) / 32, tiles), 256, 0, s, 
         x_rows, W, (const WT*)L.w_gu, (size_t)2 * ff * W, ff, W, h->x_offs, h->x_tile_e, h->x_tile_r0, h->x_meta, pin, ldh, c.x_act, c.ff_limit);
-    go_kernel(h, expert_gemm_simt_kernel<AT, WT, float, false>, dim3((W + 63) / 64, tiles), 256, 0, s, 
+    go_kernel(h, expert_gemm_simt_kernel<AT, WT, float, false>, dim3((W + 31) / 32, tiles), 256, 0, s, 
         pin, ldh, (const WT*)L.w_down, (size_t)W * ff, W, ff, h->x_offs, h->x_tile_e, h->x_tile_r0, h->x_meta, ys, W, -1, 0.0f);
   }
   h->launches += 2;

@@ -95,3 +95,10 @@ def test_two_columns_per_lane(dim, vdim, heads):
         hz.close()
     assert kin.rel_err(got, fam.oracle_logits(cfg, w, toks)) < fam.TOL["bfloat16"]
     assert _kinetar(kin.delta(heads=heads, kv_heads=heads, dim=dim, vdim=vdim, ff=0), dtype="bfloat16") < kin.TOL["bfloat16"]
+
+
+@pytest.mark.parametrize("width,ff,tokens", [(48, 1630, 321), (45, 33, 70), (64, 64, 64), (31, 7, 33), (36, 100, 9)])
+def test_fp32_product_tiles(width, ff, tokens):
+    """The fp32 build's matrix products at the edges of their tiles of 32 and 64 rows and columns and of their k blocks of 32, with row
+    starts that allow four k per load and ones that do not."""
+    assert _kinetar(kin.delta(ff=ff), cuts=[tokens], width=width) < kin.TOL["float32"]
