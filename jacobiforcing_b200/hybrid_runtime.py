@@ -3,6 +3,7 @@
 entries.  numpy carries host buffers across the ABI; torch is not needed."""
 from __future__ import annotations
 
+import array
 import ctypes as C
 import glob
 import os
@@ -18,6 +19,20 @@ DTYPES = {"bfloat16": 0, "float32": 1}
 
 def _i32(x) -> np.ndarray:
     return np.ascontiguousarray(np.asarray(x, dtype=np.int32))
+
+
+def _packed(parts) -> Tuple[np.ndarray, List[int]]:
+    """Token lists end to end as int32, and where each begins (the last: their length).  array.array converts and range-checks Python integers in native code (2048 of them: 34 us, a
+    generator and numpy 161 us, a tenth of a prompt step); whatever has no integer form of its own goes through int()."""
+    out, start = array.array("i"), [0]
+    for t in parts:
+        t = t.tolist() if isinstance(t, np.ndarray) else t if isinstance(t, (list, tuple)) else list(t)
+        try:
+            out.extend(array.array("i", t))
+        except TypeError:
+            out.extend(int(x) for x in t)
+        start.append(len(out))
+    return np.array(out, dtype=np.int32), start
 
 
 def _ptr(a: Optional[np.ndarray]):
@@ -115,22 +130,19 @@ class HybridRuntime:
         """entries: (tokens, pos0, slot, pages) per request; want: indices into the packed token list.
         Returns {"logits": [n_want, vocab] float32 or None, "sampled": int32 [n_want] or None, "layers": ...}."""
         E = len(entries)
-        toks: List[int] = []
-        start = [0]
+        a_tok, start = _packed([e[0] for e in entries])
         pages = np.zeros((E, self.max_pages_per_seq), dtype=np.int32)
-        for e, (t, pos0, slot, pg) in enumerate(entries):
-            toks.extend(int(x) for x in t)
-            start.append(len(toks))
+        for e, (_, _, _, pg) in enumerate(entries):
             if len(pg) > self.max_pages_per_seq:
                 raise RuntimeError("request holds more pages than max_pages_per_seq")
             pages[e, :len(pg)] = pg
-        T = len(toks)
+        T = len(a_tok)
         n_want = len(want)
         logits = np.empty((n_want, self.vocab), dtype=np.float32) if (n_want and want_logits) else None
         sampled = np.empty((n_want,), dtype=np.int32) if (n_want and sample) else None
         temp = np.ascontiguousarray(np.asarray(temperature, dtype=np.float32)) if (temperature is not None and n_want) else None
         layers = np.empty((len(self.config.layer_runs()), T, self.width), dtype=np.float32) if want_layers else None
-        a_tok, a_start = _i32(toks), _i32(start)
+        a_start = _i32(start)
         a_pos0, a_slot = _i32([e[1] for e in entries]), _i32([e[2] for e in entries])
         a_want = _i32(list(want)) if n_want else None
         cabi.check(self.lib.hy_step(self.h, E, _ptr(a_tok), _ptr(a_start), _ptr(a_pos0), _ptr(a_slot), _ptr(pages), n_want,
