@@ -190,7 +190,7 @@ __device__ __forceinline__ void copy_values(AT* dst, int dld, const AT* src, siz
 // rows are multiples of 16 bytes; vvec: a block's value rows are.
 // CHAN: decays per head and key channel, dec [T, ldd] (H heads of dim), staged behind q and k.  A head in one block, a column
 // per thread (128 rows of it in registers), took 5650 us for 2048 tokens of 16 heads of 128 x 128 (16 of 148 SMs busy, one warp
-// per scheduler); cut into 16 blocks of 8 columns it is 469 us.
+// per scheduler); cut into 16 blocks of 8 columns it is 469 us, into 8 of 16 columns 430.
 template <typename AT, int DR, int PARTS, int VC, bool CHAN>
 __global__ void __launch_bounds__(128) delta_head_kernel(Batch b, const float* __restrict__ qk, const AT* __restrict__ v, int ldv,
                                                          const float4* __restrict__ scal, int H, int G, int dim, int vdim,

@@ -1,7 +1,7 @@
 // hy_gla.cuh — gated linear attention with one decay per key channel, retention (one fixed decay per head, rotated queries and
-// keys), and the row kernels between the sublayers of blocks with plain RMS weights (libjf_hybrid.so).
+// keys), the gated linear recurrence whose forget gate also sets what is written, the state-space recurrence with one decay per token and
+// head, and the row kernels between the sublayers of blocks with plain RMS weights (libjf_hybrid.so).
 //
-// and the gated linear recurrence whose forget gate also sets what is written.
 // Per head, S [dim, vdim]:  S <- diag(a) S + k v^T ;  o = S^T q dim^(-1/2)   (the read-out sees the current token's write)
 //   out = o / rms(o) * norm_w * silu(g)        (norm over the head's vdim, one weight shared by the heads)
 // The decay a = sigmoid(z)^(1 / tau) leaves the decay projection's epilogue as fp32 (gemm_store).  Retention is the same
@@ -9,7 +9,7 @@
 // recurrence) and no weight in the norm.
 //
 // The recurrence has no feedback from the read-out and its value columns are independent, so a head is cut into blocks of
-// CPB = 128 / PARTS columns that run side by side on different SMs, and PARTS lanes share a column, each holding DR / PARTS
+// CPB = VC 128 / PARTS columns that run side by side on different SMs, and PARTS lanes share VC columns, each holding DR / PARTS
 // of its key rows in registers; what does not depend on the state is made beforehand (linear_rows_kernel).  The norm needs
 // whole heads: it follows in a kernel of its own (gla_out_kernel).
 #pragma once
@@ -27,8 +27,9 @@ namespace hy {
 // group, a head's step size dt = softplus(dt_raw + bias) and decay exp(-exp(A_log) dt) are made per token from dt_raw [T, lddt]
 // (column h), the value is dt x and the read-out gets D_h x added.
 // GLA_TOKEN, 2048 tokens of 32 heads of 64 channels x 128 states: eight lanes with sixteen consecutive states each (staged rows read
-// with four-way bank conflicts, one exchange per token) took 766 us, this layout 284 us.
-// GLA_FORGET, 2048 tokens of 8 heads of 128 x 128: one block per head with a column per thread took 1927 us, this layout 202 us.
+// with four-way bank conflicts, one exchange per token) took 766 us, this layout 284 us, 237 with two columns per lane.
+// GLA_FORGET, 2048 tokens of 8 heads of 128 x 128: one block per head with a column per thread took 1927 us, this layout 202 us, 187 with the next
+// token's rows read ahead.
 enum GlaMode : int { GLA_CHANNEL = 0, GLA_HEAD = 1, GLA_FORGET = 2, GLA_TOKEN = 3 };
 struct GlaToken { int G; const void* dt_raw; int lddt; const float* dt_bias; const float* A_log; const float* D; };
 template <typename AT, int DR, int PARTS, int VC, int MODE>
