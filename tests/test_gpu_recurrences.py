@@ -102,3 +102,9 @@ def test_fp32_product_tiles(width, ff, tokens):
     """The fp32 build's matrix products at the edges of their tiles of 32 and 64 rows and columns and of their k blocks of 32, with row
     starts that allow four k per load and ones that do not."""
     assert _kinetar(kin.delta(ff=ff), cuts=[tokens], width=width) < kin.TOL["float32"]
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+def test_few_rows_many_columns(dtype):
+    """Products of five to eight rows with more columns than four blocks per SM hold at eight a block: warps walk several columns."""
+    assert _kinetar(kin.delta(ff=4999), cuts=[5, 8, 7, 6], dtype=dtype) < kin.TOL[dtype]
