@@ -9,8 +9,9 @@
 // Keys and values travel by TMA, from pages of 256 tokens or from rows made for the step.
 //
 // Warp 0: producer (one lane).  Warp 1: owns tensor memory, one lane issues the products.  Warps 2-5: softmax, one thread per row.
-// Tensor memory: scores 2 x 128 columns, output 128, weights 64 + 64 (remainder).  Every wait is bounded (see tp_wait): on a timeout
-// the kernel raises the error flag, stops waiting, lets its copies land and frees its tensor memory.
+// Tensor memory: scores 2 x 128 columns, output 128, weights 64 + 64 (remainder).  Every wait on an mbarrier is bounded (see tp_wait): on
+// a timeout the kernel raises the error flag, stops waiting, lets its copies land and frees its tensor memory.  The allocation of tensor
+// memory waits without a limit; jf_pair.cuh says why it ends.
 #pragma once
 #include "jf_pair.cuh"
 
@@ -87,7 +88,6 @@ flash_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ C
   unsigned char* sv = sk + 2 * KC * CHUNK;                 // [2]
   FlSmem* sm = reinterpret_cast<FlSmem*>(sv + 2 * VC * CHUNK);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  pdl_trigger();
   if (threadIdx.x == 0) {
     for (int i = 0; i < 2; ++i) {
       mbar_init(&sm->k_full[i], 1); mbar_init(&sm->k_empty[i], 1); mbar_init(&sm->v_full[i], 1); mbar_init(&sm->v_empty[i], 1);
@@ -101,6 +101,7 @@ flash_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ C
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_trigger();                                           // this block owns its columns
   pdl_wait();
   const FlashUnit u = a.units[blockIdx.x];
   const FlTiles tiles(u, a.window);

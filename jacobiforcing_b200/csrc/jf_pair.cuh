@@ -15,8 +15,9 @@
 // Warp 0:     producer (one lane in each CTA, seven or nine stages; all bytes of a stage count on the first CTA's mbarrier).
 // Warp 1:     owns tensor memory; in the first CTA one lane issues the products and commits to both CTAs' mbarriers.
 // Warps 2-9:  epilogue (two per quarter of the lanes, one half of the columns each).
-// Every wait is bounded: on a timeout the kernel raises the error flag, stops waiting, lets its copies land and frees its
-// tensor memory.
+// Every wait on an mbarrier is bounded: on a timeout the kernel raises the error flag, stops waiting, lets its copies land and frees
+// its tensor memory.  tcgen05.alloc has no such limit; it ends because who holds columns of the SM never waits for this block: the blocks
+// of a kernel that may start under this one (see pdl_trigger) start only once every block of this grid owns its columns.
 // What leaves with the accumulators is the Epilogue: a functor called by every epilogue warp with (tensor memory address of its lanes
 // and columns, this lane's feature n, token of the first column, columns, tokens T, features N, lane).
 #pragma once
@@ -33,6 +34,9 @@ namespace jf {
 // Programmatic dependent launch: a kernel may start while the one before it still runs and must not touch anything that an
 // earlier kernel reads or writes before pdl_wait.  What comes before it (weights, which nothing writes; barriers, tensor memory)
 // overlaps the end of the kernel before.
+// A kernel that allocates tensor memory triggers behind its allocation and the barrier that follows it, never before: a block of a later
+// kernel would otherwise be able to take the columns first and hold them in pdl_wait, which ends with this grid, while a block of this
+// grid waits for them in tcgen05.alloc, which has no limit.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
@@ -187,7 +191,6 @@ pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CU
   const int KT = (K + 63) / 64, nx = (N + 255) / 256, parts = split.parts, step = (gridDim.x >> 1) / parts;
   // this pair's range of k and first tile (parts > 1: one tile per pair)
   const int part = (int)(blockIdx.x >> 1) % parts, first = (int)(blockIdx.x >> 1) / parts, kt0 = part * KT / parts, kt1 = (part + 1) * KT / parts;
-  pdl_trigger();
   if (threadIdx.x == 0) {
     for (int i = 0; i < TP_STAGES; ++i) { mbar_init(&sm->full[i], 1); mbar_init(&sm->empty[i], 1); }
     for (int i = 0; i < 2; ++i) { mbar_init(&sm->acc_full[i], 1); mbar_init(&sm->acc_empty[i], 16); }
@@ -202,6 +205,7 @@ pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CU
   __syncthreads();
   tp_cluster_sync();
   tc_fence_after();
+  pdl_trigger();                                            // both CTAs own their columns (see pdl_trigger)
   // one stage's weight tile: 128 rows, or 64 gate and 64 up rows
   auto load_w = [&](unsigned char* dst, int x, int kt, int base_row, uint32_t bar) {
     if (!lay.pairs) {

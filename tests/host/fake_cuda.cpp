@@ -1,0 +1,117 @@
+// A CUDA runtime without a GPU: "device" memory is host memory, copies are copies, kernels are noted down and not run.  The engines' host
+// code is linked against it (device code as PTX that nothing loads) to test what it launches, in which order, and what it does
+// when a call fails.  Which launch, attribute or tensor map fails is set by fake_fail.
+#include <cuda.h>
+#include <cuda_runtime.h>
+
+#include <cstdlib>
+#include <cstring>
+#include <map>
+#include <set>
+#include <string>
+#include <vector>
+
+namespace {
+int g_device = 0;
+cudaError_t g_last = cudaSuccess;
+std::map<const void*, std::string> g_names;                     // host stub -> mangled kernel name
+struct Launch { const void* f; int device; size_t smem; };
+std::vector<Launch> g_launches;
+std::map<std::pair<int, const void*>, int> g_smem;              // (device, kernel) -> opted in dynamic shared memory
+long g_count[3] = {0, 0, 0}, g_fail[3] = {-1, -1, -1};          // launches, attributes, tensor maps: how many so far, which one fails
+constexpr size_t kDefaultSmem = 48 * 1024, kMostSmem = 227 * 1024;
+
+bool fails(int what) { return g_count[what]++ == g_fail[what]; }
+cudaError_t last(cudaError_t e) { if (e != cudaSuccess) g_last = e; return e; }
+cudaError_t launch(const void* f, size_t smem) {
+  if (fails(0)) return last(cudaErrorLaunchFailure);
+  const auto it = g_smem.find({g_device, f});
+  if (smem > (it == g_smem.end() ? kDefaultSmem : (size_t)it->second)) return last(cudaErrorInvalidValue);
+  g_launches.push_back({f, g_device, smem});
+  return cudaSuccess;
+}
+CUresult encode(CUtensorMap* m, CUtensorMapDataType, cuuint32_t, void* p, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
+                const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill) {
+  if (fails(2)) return CUDA_ERROR_INVALID_VALUE;
+  memset(m, 0, sizeof(*m));
+  memcpy(m, &p, sizeof(p));
+  return CUDA_SUCCESS;
+}
+}  // namespace
+
+extern "C" {
+// ---- what a test asks ---------------------------------------------------------------------------------------------------------------
+void fake_reset() { g_launches.clear(); for (int i = 0; i < 3; ++i) { g_count[i] = 0; g_fail[i] = -1; } g_last = cudaSuccess; }
+void fake_fail(int what, long at) { g_count[what] = 0; g_fail[what] = at; }
+long fake_count(int what) { return g_count[what]; }
+int fake_launches() { return (int)g_launches.size(); }
+const char* fake_launch_name(int i) { return g_names[g_launches[i].f].c_str(); }
+int fake_launch_device(int i) { return g_launches[i].device; }
+
+// ---- registration -------------------------------------------------------------------------------------------------------------------
+void** __cudaRegisterFatBinary(void*) { static void* h; return &h; }
+void __cudaRegisterFatBinaryEnd(void**) {}
+void __cudaUnregisterFatBinary(void**) {}
+void __cudaRegisterFunction(void**, const char* f, char*, const char* name, int, uint3*, uint3*, dim3*, dim3*, int*) { g_names[f] = name; }
+void __cudaRegisterVar(void**, char*, char*, const char*, int, size_t, int, int) {}
+char __cudaInitModule(void**) { return 0; }
+static dim3 g_grid, g_block; static size_t g_dyn; static cudaStream_t g_stream;
+unsigned __cudaPushCallConfiguration(dim3 g, dim3 b, size_t s, cudaStream_t st) { g_grid = g; g_block = b; g_dyn = s; g_stream = st; return 0; }
+cudaError_t __cudaPopCallConfiguration(dim3* g, dim3* b, size_t* s, void* st) { *g = g_grid; *b = g_block; *s = g_dyn; *(cudaStream_t*)st = g_stream; return cudaSuccess; }
+
+// ---- runtime ------------------------------------------------------------------------------------------------------------------------
+cudaError_t cudaGetDeviceCount(int* n) { *n = 2; return cudaSuccess; }
+cudaError_t cudaSetDevice(int d) { g_device = d; return cudaSuccess; }
+cudaError_t cudaGetDeviceProperties_v2(cudaDeviceProp* p, int) {
+  memset(p, 0, sizeof(*p));
+  p->major = 10; p->multiProcessorCount = 148;
+  return cudaSuccess;
+}
+cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr a, int) {
+  *v = a == cudaDevAttrMaxSharedMemoryPerBlockOptin ? (int)kMostSmem : a == cudaDevAttrMultiProcessorCount ? 148 : a == cudaDevAttrClockRate ? 1965000 : 1;
+  return cudaSuccess;
+}
+cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int* n, const void*, int, size_t, unsigned) { *n = 1; return cudaSuccess; }
+cudaError_t cudaMalloc(void** p, size_t n) { *p = calloc(n ? n : 1, 1); return *p ? cudaSuccess : cudaErrorMemoryAllocation; }
+cudaError_t cudaMallocHost(void** p, size_t n) { return cudaMalloc(p, n); }
+cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { return cudaMalloc(p, n); }
+cudaError_t cudaHostGetDevicePointer(void** d, void* p, unsigned) { *d = p; return cudaSuccess; }
+cudaError_t cudaFree(void* p) { free(p); return cudaSuccess; }
+cudaError_t cudaFreeHost(void* p) { free(p); return cudaSuccess; }
+cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind) { memcpy(d, s, n); return cudaSuccess; }
+cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t) { memcpy(d, s, n); return cudaSuccess; }
+cudaError_t cudaMemset(void* d, int v, size_t n) { memset(d, v, n); return cudaSuccess; }
+cudaError_t cudaMemsetAsync(void* d, int v, size_t n, cudaStream_t) { memset(d, v, n); return cudaSuccess; }
+cudaError_t cudaStreamCreate(cudaStream_t* s) { *s = nullptr; return cudaSuccess; }
+cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) { *s = nullptr; return cudaSuccess; }
+cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaDeviceSynchronize() { return cudaSuccess; }
+cudaError_t cudaEventCreate(cudaEvent_t* e) { *e = nullptr; return cudaSuccess; }
+cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
+cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t, cudaEvent_t) { *ms = 0.0f; return cudaSuccess; }
+cudaError_t cudaGetLastError() { const cudaError_t e = g_last; g_last = cudaSuccess; return e; }
+const char* cudaGetErrorString(cudaError_t e) { return e == cudaErrorInvalidValue ? "invalid argument" : e == cudaErrorLaunchFailure ? "launch refused" : "error"; }
+cudaError_t cudaFuncSetAttribute(const void* f, cudaFuncAttribute a, int v) {
+  if (fails(1)) return last(cudaErrorInvalidValue);
+  if (a == cudaFuncAttributeMaxDynamicSharedMemorySize) {
+    if (v < 0 || (size_t)v > kMostSmem) return last(cudaErrorInvalidValue);
+    g_smem[{g_device, f}] = v;
+  }
+  return cudaSuccess;
+}
+cudaError_t cudaLaunchKernel(const void* f, dim3, dim3, void**, size_t smem, cudaStream_t) { return launch(f, smem); }
+cudaError_t cudaLaunchCooperativeKernel(const void* f, dim3, dim3, void**, size_t smem, cudaStream_t) { return launch(f, smem); }
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void**) { return launch(f, c->dynamicSmemBytes); }
+cudaError_t cudaGetDriverEntryPoint(const char*, void** p, unsigned long long, cudaDriverEntryPointQueryResult* r) {
+  *p = (void*)encode;
+  *r = cudaDriverEntryPointSuccess;
+  return cudaSuccess;
+}
+cudaError_t cudaDeviceCanAccessPeer(int* v, int, int) { *v = 0; return cudaSuccess; }
+cudaError_t cudaDeviceEnablePeerAccess(int, unsigned) { return cudaErrorInvalidValue; }
+cudaError_t cudaIpcGetMemHandle(cudaIpcMemHandle_t*, void*) { return cudaErrorInvalidValue; }
+cudaError_t cudaIpcOpenMemHandle(void**, cudaIpcMemHandle_t, unsigned) { return cudaErrorInvalidValue; }
+cudaError_t cudaIpcCloseMemHandle(void*) { return cudaErrorInvalidValue; }
+}
