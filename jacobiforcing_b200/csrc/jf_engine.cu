@@ -54,11 +54,11 @@ struct jf_engine {
   bool finalized = false;
   // host mirrors
   std::vector<SeqState> h_states;
-  // per-call draft sources of jf_jacobi_run (first-call tokens, MT19937 states, pad streams): grown on demand, kept
   // forwards of many rows (jf_wide.cuh): attention row units, error flag
   FlashUnit* wide_units_d = nullptr;
   size_t wide_units_cap = 0;
   int* wide_err = nullptr;
+  // per-call draft sources of jf_jacobi_run (first-call tokens, MT19937 states, pad streams): grown on demand, kept
   int* run_scratch[3] = {nullptr, nullptr, nullptr};
   size_t run_scratch_words[3] = {0, 0, 0};
 };
@@ -410,6 +410,7 @@ extern "C" int jf_create(const jf_model_cfg* m, const jf_runtime_cfg* r, jf_hand
 #undef ALLOC
   if (cudaFuncSetAttribute(jf_persistent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, h->smem_optin) != cudaSuccess)
     return fail(JF_ERR_CUDA, "cannot opt in to the full shared memory carve-out");
+  if (tp == 1 && wide_opt_in(md.d) != cudaSuccess) return fail(JF_ERR_CUDA, "cannot opt in to the prompt kernels' shared memory");
   int occ = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, jf_persistent_kernel, kNumThreads, h->smem_optin);
   if (occ < 1) return fail(JF_ERR_CUDA, "persistent kernel does not fit on an SM");

@@ -211,13 +211,23 @@ inline void wide_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem
   cudaLaunchKernelEx(&c, kernel, std::forward<A>(args)...);
 }
 
+// Opts the kernels in to their shared memory on the current device, for heads of d.  Once per engine, like the persistent kernel: the limit belongs to
+// a device, and a process may hold engines on several.
+inline cudaError_t wide_opt_in(int d) {
+  auto opt = [](auto kernel, size_t bytes) { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes); };
+  cudaError_t e = opt(pair_kernel<WideQkv, 256>, tp_smem_bytes(256));
+  if (e == cudaSuccess) e = opt(pair_kernel<WideResidual, 256>, tp_smem_bytes(256));
+  if (e == cudaSuccess) e = opt(pair_kernel<WideSwiglu, 256>, tp_smem_bytes(256));
+  if (e == cudaSuccess) e = opt(pair_kernel<WideLogits, 256>, tp_smem_bytes(256));
+  if (e == cudaSuccess) e = d == 64 ? opt(flash_kernel<64, 64, false>, fl_smem_bytes(64, 64)) : opt(flash_kernel<128, 128, false>, fl_smem_bytes(128, 128));
+  return e;
+}
+
 // C[t, n] over packed activations [K / 64][rows_cap][64] (T rows from x_row0 on) and packed weight tiles; up_tiles > 0: a gate and an up
 // matrix of that many 128-row tiles, N = 2 * features.  Tiles of 256 rows and whole ranges of k whatever T is: a row's sums are added
 // in the same order in every forward.
 template <class Epi>
 inline bool wide_product(cudaStream_t s, const void* X, int rows_cap, int x_row0, const void* W, int up_tiles, int T, int N, int K, const Epi& epi, int* err) {
-  static bool attr = false;                                     // per epilogue: this function is a template
-  if (!attr) { cudaFuncSetAttribute(pair_kernel<Epi, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tp_smem_bytes(256)); attr = true; }
   const int KT = (K + 63) / 64, nt = (N + 127) / 128;
   CUtensorMap xm, wm;
   if (!tp_map(&xm, X, (uint64_t)KT * rows_cap, 64, 64, 128, false)) return false;
@@ -231,8 +241,6 @@ inline bool wide_product(cudaStream_t s, const void* X, int rows_cap, int x_row0
 template <int D>
 inline bool wide_attention(cudaStream_t s, const DevCtx& c, int layer, const FlashUnit* units, int n_units, int* err) {
   const ModelDims& md = c.md;
-  static bool attr = false;
-  if (!attr) { cudaFuncSetAttribute(flash_kernel<D, D, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fl_smem_bytes(D, D)); attr = true; }
   CUtensorMap paged[2];
   for (int kv = 0; kv < 2; ++kv) {
     if (!tp_map(&paged[kv], c.kv_cache + kv_cache_offset(md, c.num_pages, layer, kv, 0, 0, 0), (uint64_t)c.num_pages * md.n_kv * kPage, D, D, FL_KEYS, true)) return false;

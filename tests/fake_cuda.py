@@ -1,0 +1,56 @@
+"""The engines' host code on a CUDA runtime without a GPU (tests/host/fake_cuda.cpp): what is launched, in which order, on which device,
+and what happens when a call fails."""
+from __future__ import annotations
+
+import ctypes as C
+import os
+import shutil
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CSRC = os.path.join(ROOT, "jacobiforcing_b200", "csrc")
+FAKE = os.path.join(ROOT, "tests", "host", "fake_cuda.cpp")
+LAUNCH, ATTRIBUTE, TENSOR_MAP = 0, 1, 2
+
+
+def build(engine: str) -> str:
+    """The engine's source with device code that nothing loads, linked against the runtime that notes things down."""
+    out = os.path.join(ROOT, "build", "lib%s_fake.so" % engine)
+    srcs = [os.path.join(CSRC, f) for f in os.listdir(CSRC)] + [os.path.join(ROOT, "include", f) for f in os.listdir(os.path.join(ROOT, "include"))] + [FAKE]
+    if os.path.exists(out) and all(os.path.getmtime(s) <= os.path.getmtime(out) for s in srcs):
+        return out
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    if not os.path.exists(nvcc):
+        pytest.skip("needs nvcc")
+    os.makedirs(os.path.dirname(out), exist_ok=True)
+    tmp = "%s.%d.tmp" % (out, os.getpid())
+    subprocess.check_call([nvcc, "-gencode", "arch=compute_100a,code=compute_100a", "-Xcicc", "-O0", "-std=c++17", "-Xcompiler", "-fPIC,-O1", "-w",
+                           "-I", os.path.join(ROOT, "include"), "-I", CSRC, "-shared", "-cudart", "none", "-Xlinker", "-Bsymbolic",
+                           os.path.join(CSRC, engine + "_engine.cu"), FAKE, "-o", tmp])
+    os.replace(tmp, out)
+    return out
+
+
+class Fake:
+    def __init__(self, path):
+        self.lib = C.CDLL(path)
+        self.lib.fake_launch_name.restype = C.c_char_p
+        self.lib.fake_count.restype = C.c_long
+        self.lib.fake_fail.argtypes = [C.c_int, C.c_long]
+        self.reset()
+
+    def reset(self):
+        self.lib.fake_reset()
+
+    def fail(self, what, at):
+        """The call number `at` from here on (0: the next one) of this kind fails."""
+        self.lib.fake_fail(what, at)
+
+    def count(self, what):
+        return self.lib.fake_count(what)
+
+    def launches(self):
+        """(kernel, device) of every launch that went through since the last reset."""
+        return [(self.lib.fake_launch_name(i).decode(), self.lib.fake_launch_device(i)) for i in range(self.lib.fake_launches())]

@@ -7,14 +7,14 @@
 #include <cstdlib>
 #include <cstring>
 #include <map>
-#include <set>
 #include <string>
 #include <vector>
 
 namespace {
 int g_device = 0;
 cudaError_t g_last = cudaSuccess;
-std::map<const void*, std::string> g_names;                     // host stub -> mangled kernel name
+// host stub -> mangled kernel name; made by the first registration, which may come before this file's own objects exist
+std::map<const void*, std::string>& names() { static std::map<const void*, std::string> m; return m; }
 struct Launch { const void* f; int device; size_t smem; };
 std::vector<Launch> g_launches;
 std::map<std::pair<int, const void*>, int> g_smem;              // (device, kernel) -> opted in dynamic shared memory
@@ -45,14 +45,14 @@ void fake_reset() { g_launches.clear(); for (int i = 0; i < 3; ++i) { g_count[i]
 void fake_fail(int what, long at) { g_count[what] = 0; g_fail[what] = at; }
 long fake_count(int what) { return g_count[what]; }
 int fake_launches() { return (int)g_launches.size(); }
-const char* fake_launch_name(int i) { return g_names[g_launches[i].f].c_str(); }
+const char* fake_launch_name(int i) { return names()[g_launches[i].f].c_str(); }
 int fake_launch_device(int i) { return g_launches[i].device; }
 
 // ---- registration -------------------------------------------------------------------------------------------------------------------
 void** __cudaRegisterFatBinary(void*) { static void* h; return &h; }
 void __cudaRegisterFatBinaryEnd(void**) {}
 void __cudaUnregisterFatBinary(void**) {}
-void __cudaRegisterFunction(void**, const char* f, char*, const char* name, int, uint3*, uint3*, dim3*, dim3*, int*) { g_names[f] = name; }
+void __cudaRegisterFunction(void**, const char* f, char*, const char* name, int, uint3*, uint3*, dim3*, dim3*, int*) { names()[f] = name; }
 void __cudaRegisterVar(void**, char*, char*, const char*, int, size_t, int, int) {}
 char __cudaInitModule(void**) { return 0; }
 static dim3 g_grid, g_block; static size_t g_dyn; static cudaStream_t g_stream;

@@ -1,0 +1,58 @@
+"""Host side of the Jacobi engine's prompt forwards: kernels are set up on every device that an engine is made on."""
+import pytest
+
+from tests import fake_cuda
+
+CFG = dict(hidden_size=256, num_hidden_layers=2, num_attention_heads=4, num_key_value_heads=2, head_dim=64, intermediate_size=768, vocab_size=300,
+           tie_word_embeddings=False, rope_theta=1e6, max_position_embeddings=2048, rms_norm_eps=1e-6)
+
+
+@pytest.fixture(scope="module")
+def fake():
+    from jacobiforcing_b200 import _cabi
+    path, mp = fake_cuda.build("jf"), pytest.MonkeyPatch()
+    mp.setenv("JF_LIB_PATH", path)
+    mp.setattr(_cabi, "_lib", None)
+    yield fake_cuda.Fake(path)
+    mp.undo()
+
+
+def engine(head_dim=64, device=0):
+    import torch
+
+    from jacobiforcing_b200.runtime import JacobiRuntime
+    cfg = dict(CFG, head_dim=head_dim, hidden_size=4 * head_dim)
+    rt = JacobiRuntime(cfg, device=device, max_rows=512, max_seqs=4, num_kv_pages=8, max_pages_per_seq=4)
+    h, q, kv, inter, v = cfg["hidden_size"], 4 * head_dim, 2 * head_dim, cfg["intermediate_size"], cfg["vocab_size"]
+    shapes = {"model.embed_tokens.weight": (v, h), "lm_head.weight": (v, h), "model.norm.weight": (h,)}
+    for i in range(cfg["num_hidden_layers"]):
+        p = "model.layers.%d." % i
+        shapes.update({p + "self_attn.q_proj.weight": (q, h), p + "self_attn.k_proj.weight": (kv, h), p + "self_attn.v_proj.weight": (kv, h),
+                       p + "self_attn.q_proj.bias": (q,), p + "self_attn.k_proj.bias": (kv,), p + "self_attn.v_proj.bias": (kv,),
+                       p + "self_attn.o_proj.weight": (h, q), p + "mlp.gate_proj.weight": (inter, h), p + "mlp.up_proj.weight": (inter, h),
+                       p + "mlp.down_proj.weight": (h, inter), p + "input_layernorm.weight": (h,), p + "post_attention_layernorm.weight": (h,)})
+    rt.load_state_dict({k: torch.zeros(s, dtype=torch.bfloat16) for k, s in shapes.items()})
+    return rt
+
+
+def chunk(rt, rows=256):
+    s = rt.new_sequence()
+    rt.ensure_capacity(s, rows)
+    try:
+        return rt.forward([1] * rows, [(0, rows, 0, 0)], [s], rows - 8, 8, [(i, 0, i) for i in range(rows)])
+    finally:
+        rt.release(s)
+
+
+@pytest.mark.parametrize("head_dim", [64, 128])
+def test_prompt_chunks_on_two_devices(fake, head_dim):
+    """A kernel's shared-memory limit belongs to a device: an engine on another device of the process launches the same stages."""
+    seen = []
+    for device in (0, 1):
+        rt = engine(head_dim, device)
+        fake.reset()
+        chunk(rt)
+        assert {d for _, d in fake.launches()} == {device}
+        seen.append([n for n, _ in fake.launches()])
+        rt.close()
+    assert seen[0] == seen[1] and sum("pair_kernel" in n for n in seen[0]) == 9 and sum("flash_kernel" in n for n in seen[0]) == 2
