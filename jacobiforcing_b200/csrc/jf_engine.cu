@@ -845,12 +845,14 @@ static int run_wide(jf_engine* h, int T, const std::vector<Group>& groups, int l
   }
   JF_CUDA(h, cudaMemcpyAsync(h->wide_units_d, units.data(), units.size() * sizeof(FlashUnit), cudaMemcpyHostToDevice, h->stream));
   JF_CUDA(h, cudaEventRecord(h->ev0, h->stream));
-  const int n = wide_forward(h->stream, c, T, h->wide_units_d, (int)units.size(), lm_row0, lm_rows, h->wide_err);
+  WideStream w{h->stream};
+  wide_forward(w, c, T, h->wide_units_d, (int)units.size(), lm_row0, lm_rows, h->wide_err);
   JF_CUDA(h, cudaEventRecord(h->ev1, h->stream));
   JF_CUDA(h, cudaStreamSynchronize(h->stream));
-  JF_CUDA(h, cudaGetLastError());
-  if (n == 0) { h->err = "a tensor map of the forward could not be made"; return JF_ERR_CUDA; }
-  h->launches += n;
+  const cudaError_t last = cudaGetLastError();
+  h->launches += w.launches;
+  if (w.failed) { h->err = std::string("prompt forward: ") + w.failed; return JF_ERR_CUDA; }
+  JF_CUDA(h, last);
   if (elapsed_ms) cudaEventElapsedTime(elapsed_ms, h->ev0, h->ev1);
   int e = 0;
   JF_CUDA(h, cudaMemcpy(&e, h->wide_err, 4, cudaMemcpyDeviceToHost));

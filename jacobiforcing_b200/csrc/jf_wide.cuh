@@ -201,15 +201,25 @@ __global__ void __launch_bounds__(1024) wide_argmax_kernel(const float* __restri
 }
 
 // ---- host ----------------------------------------------------------------------------------------------------------------------------
-template <typename... P, typename... A>
-inline void wide_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
-  cudaLaunchAttribute at;
-  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t c = {};
-  c.gridDim = grid; c.blockDim = block; c.dynamicSmemBytes = smem; c.stream = stream; c.attrs = &at; c.numAttrs = 1;
-  cudaLaunchKernelEx(&c, kernel, std::forward<A>(args)...);
-}
+// The launches of a forward: behind the first that fails nothing else is launched (a stage over what another one did not make would
+// leave keys and values of stale rows in the pages).
+struct WideStream {
+  cudaStream_t s;
+  int launches = 0;
+  const char* failed = nullptr;                                 // what failed first
+  template <typename... P, typename... A>
+  void launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, A&&... args) {
+    if (failed) return;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c = {};
+    c.gridDim = grid; c.blockDim = block; c.dynamicSmemBytes = smem; c.stream = s; c.attrs = &at; c.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&c, kernel, std::forward<A>(args)...);
+    if (e == cudaSuccess) ++launches;
+    else failed = cudaGetErrorString(e);
+  }
+};
 
 // Opts the kernels in to their shared memory on the current device, for heads of d.  Once per engine, like the persistent kernel: the limit belongs to
 // a device, and a process may hold engines on several.
@@ -227,27 +237,33 @@ inline cudaError_t wide_opt_in(int d) {
 // matrix of that many 128-row tiles, N = 2 * features.  Tiles of 256 rows and whole ranges of k whatever T is: a row's sums are added
 // in the same order in every forward.
 template <class Epi>
-inline bool wide_product(cudaStream_t s, const void* X, int rows_cap, int x_row0, const void* W, int up_tiles, int T, int N, int K, const Epi& epi, int* err) {
+inline void wide_product(WideStream& w, const void* X, int rows_cap, int x_row0, const void* W, int up_tiles, int T, int N, int K, const Epi& epi, int* err) {
+  if (w.failed) return;
   const int KT = (K + 63) / 64, nt = (N + 127) / 128;
   CUtensorMap xm, wm;
-  if (!tp_map(&xm, X, (uint64_t)KT * rows_cap, 64, 64, 128, false)) return false;
-  if (!(up_tiles ? tp_map_pairs(&wm, W, up_tiles, KT) : tp_map(&wm, W, (uint64_t)nt * KT * 128, 64, 64, 128, false))) return false;
+  if (!tp_map(&xm, X, (uint64_t)KT * rows_cap, 64, 64, 128, false) ||
+      !(up_tiles ? tp_map_pairs(&wm, W, up_tiles, KT) : tp_map(&wm, W, (uint64_t)nt * KT * 128, 64, 64, 128, false))) {
+    w.failed = "a tensor map of a product could not be made";
+    return;
+  }
   const int tiles = (N + 255) / 256 * ((T + 255) / 256), grid = 2 * std::min(tiles, TP_CLUSTERS);
-  wide_launch(pair_kernel<Epi, 256>, grid, TP_THREADS, tp_smem_bytes(256), s, xm, wm, T, N, K, epi, err, TpGroup{},
-              PairLayout{rows_cap, x_row0, up_tiles > 0}, PairSplit{1, nullptr, nullptr});
-  return true;
+  w.launch(pair_kernel<Epi, 256>, grid, TP_THREADS, tp_smem_bytes(256), xm, wm, T, N, K, epi, err, TpGroup{}, PairLayout{rows_cap, x_row0, up_tiles > 0},
+           PairSplit{1, nullptr, nullptr});
 }
 
 template <int D>
-inline bool wide_attention(cudaStream_t s, const DevCtx& c, int layer, const FlashUnit* units, int n_units, int* err) {
+inline void wide_attention(WideStream& w, const DevCtx& c, int layer, const FlashUnit* units, int n_units, int* err) {
+  if (w.failed) return;
   const ModelDims& md = c.md;
   CUtensorMap paged[2];
   for (int kv = 0; kv < 2; ++kv) {
-    if (!tp_map(&paged[kv], c.kv_cache + kv_cache_offset(md, c.num_pages, layer, kv, 0, 0, 0), (uint64_t)c.num_pages * md.n_kv * kPage, D, D, FL_KEYS, true)) return false;
+    if (!tp_map(&paged[kv], c.kv_cache + kv_cache_offset(md, c.num_pages, layer, kv, 0, 0, 0), (uint64_t)c.num_pages * md.n_kv * kPage, D, D, FL_KEYS, true)) {
+      w.failed = "a tensor map of the attention could not be made";
+      return;
+    }
   }
   const FlashArgs a{units, c.qbuf, (size_t)md.q_dim, D, c.block_tables, md.n_kv, rsqrtf((float)D), 0, nullptr, nullptr, 0, c.xa, 0, c.xrows_cap, err};
-  wide_launch(flash_kernel<D, D, false>, n_units, FL_THREADS, fl_smem_bytes(D, D), s, paged[0], paged[1], paged[0], paged[1], a);
-  return true;
+  w.launch(flash_kernel<D, D, false>, n_units, FL_THREADS, fl_smem_bytes(D, D), paged[0], paged[1], paged[0], paged[1], a);
 }
 
 // Row units of a forward: 128 (head, token) pairs of one key head of one group each, most key tiles first.
@@ -265,40 +281,34 @@ inline std::vector<FlashUnit> wide_units(const ModelDims& md, const std::vector<
   return u;
 }
 
-// The whole forward on stream s; the plan's arrays (tokens, positions, groups, tables) are on the device already.  Returns the launches,
-// 0 when a tensor map could not be made.
-inline int wide_forward(cudaStream_t s, const DevCtx& c, int T, const FlashUnit* units, int n_units, int lm_row0, int lm_rows, int* err) {
+// The whole forward on w's stream; the plan's arrays (tokens, positions, groups, tables) are on the device already.
+inline void wide_forward(WideStream& w, const DevCtx& c, int T, const FlashUnit* units, int n_units, int lm_row0, int lm_rows, int* err) {
   const ModelDims& md = c.md;
   __nv_bfloat16* qkv = reinterpret_cast<__nv_bfloat16*>(c.part);       // the split-K partial sums' buffer: T_cap rows of qkv_dim floats and more
   uint8_t* xn = reinterpret_cast<uint8_t*>(c.xn);
   const int nt_i = (md.inter + 127) >> 7;
-  int n = 0;
-  auto norm = [&](bool first, const __nv_bfloat16* w) {
-    wide_launch(wide_norm_kernel, T, WIDE_NORM_THREADS, 0, s, first ? c.tok : nullptr, c.embed, md.vocab_embed, c.hidden, w, md.h, md.eps, xn, c.xrows_cap);
-    ++n;
+  auto norm = [&](bool first, const __nv_bfloat16* weight) {
+    w.launch(wide_norm_kernel, T, WIDE_NORM_THREADS, 0, first ? c.tok : nullptr, c.embed, md.vocab_embed, c.hidden, weight, md.h, md.eps, xn, c.xrows_cap);
   };
   norm(true, c.layer[0].ln1);
-  bool ok = true;
-  for (int l = 0; l < md.layers && ok; ++l) {
+  for (int l = 0; l < md.layers && !w.failed; ++l) {
     const LayerW& L = c.layer[l];
-    ok = ok && wide_product(s, c.xn, c.xrows_cap, 0, L.wqkv, 0, T, md.qkv_dim, md.h, WideQkv{qkv, md.qkv_dim, L.bqkv}, err);
-    wide_launch(wide_rope_kernel, T, 256, 0, s, qkv, md, c.row_pos, c.row_group, c.groups, c.block_tables, c.max_pages_per_seq, c.rope_cos, c.rope_sin, c.qbuf,
-                c.kv_scratch + kv_scratch_offset(md, c.T_cap, l, 0, 0, 0), c.kv_scratch + kv_scratch_offset(md, c.T_cap, l, 1, 0, 0),
-                c.kv_cache + kv_cache_offset(md, c.num_pages, l, 0, 0, 0, 0), c.kv_cache + kv_cache_offset(md, c.num_pages, l, 1, 0, 0, 0));
-    ok = ok && (md.d == 64 ? wide_attention<64>(s, c, l, units, n_units, err) : wide_attention<128>(s, c, l, units, n_units, err));
-    ok = ok && wide_product(s, c.xa, c.xrows_cap, 0, L.wo, 0, T, md.h, md.q_dim, WideResidual{c.hidden, md.h}, err);
+    wide_product(w, c.xn, c.xrows_cap, 0, L.wqkv, 0, T, md.qkv_dim, md.h, WideQkv{qkv, md.qkv_dim, L.bqkv}, err);
+    w.launch(wide_rope_kernel, T, 256, 0, qkv, md, c.row_pos, c.row_group, c.groups, c.block_tables, c.max_pages_per_seq, c.rope_cos, c.rope_sin, c.qbuf,
+             c.kv_scratch + kv_scratch_offset(md, c.T_cap, l, 0, 0, 0), c.kv_scratch + kv_scratch_offset(md, c.T_cap, l, 1, 0, 0),
+             c.kv_cache + kv_cache_offset(md, c.num_pages, l, 0, 0, 0, 0), c.kv_cache + kv_cache_offset(md, c.num_pages, l, 1, 0, 0, 0));
+    if (md.d == 64) wide_attention<64>(w, c, l, units, n_units, err);
+    else wide_attention<128>(w, c, l, units, n_units, err);
+    wide_product(w, c.xa, c.xrows_cap, 0, L.wo, 0, T, md.h, md.q_dim, WideResidual{c.hidden, md.h}, err);
     norm(false, L.ln2);
-    ok = ok && wide_product(s, c.xn, c.xrows_cap, 0, L.wgu, nt_i, T, 2 * md.inter, md.h, WideSwiglu{reinterpret_cast<uint8_t*>(c.xact), c.xrows_cap, md.inter}, err);
-    ok = ok && wide_product(s, c.xact, c.xrows_cap, 0, L.wd, 0, T, md.h, md.inter, WideResidual{c.hidden, md.h}, err);
+    wide_product(w, c.xn, c.xrows_cap, 0, L.wgu, nt_i, T, 2 * md.inter, md.h, WideSwiglu{reinterpret_cast<uint8_t*>(c.xact), c.xrows_cap, md.inter}, err);
+    wide_product(w, c.xact, c.xrows_cap, 0, L.wd, 0, T, md.h, md.inter, WideResidual{c.hidden, md.h}, err);
     norm(false, l + 1 < md.layers ? c.layer[l + 1].ln1 : c.final_norm);
-    n += 6;
   }
   if (lm_rows > 0) {
-    ok = ok && wide_product(s, c.xn, c.xrows_cap, lm_row0, c.lm_head, 0, lm_rows, md.vocab, md.h, WideLogits{c.logits, (size_t)md.vocab}, err);
-    wide_launch(wide_argmax_kernel, lm_rows, 1024, 0, s, c.logits, md.vocab, c.greedy + lm_row0);
-    n += 2;
+    wide_product(w, c.xn, c.xrows_cap, lm_row0, c.lm_head, 0, lm_rows, md.vocab, md.h, WideLogits{c.logits, (size_t)md.vocab}, err);
+    w.launch(wide_argmax_kernel, lm_rows, 1024, 0, c.logits, md.vocab, c.greedy + lm_row0);
   }
-  return ok ? n : 0;
 }
 
 }  // namespace jf

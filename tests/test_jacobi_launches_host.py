@@ -1,4 +1,5 @@
-"""Host side of the Jacobi engine's prompt forwards: kernels are set up on every device that an engine is made on."""
+"""Host side of the Jacobi engine's prompt forwards: kernels are set up on every device that an engine is made on, and a forward stops at
+the first call that fails."""
 import pytest
 
 from tests import fake_cuda
@@ -56,3 +57,32 @@ def test_prompt_chunks_on_two_devices(fake, head_dim):
         seen.append([n for n, _ in fake.launches()])
         rt.close()
     assert seen[0] == seen[1] and sum("pair_kernel" in n for n in seen[0]) == 9 and sum("flash_kernel" in n for n in seen[0]) == 2
+
+
+@pytest.mark.parametrize("what", ["launch", "tensor map"])
+def test_nothing_is_launched_behind_a_failure(fake, what):
+    """Whichever launch or tensor map of a prompt chunk fails: an error, and no stage over what another one did not make (the rotary stage
+    would leave keys and values of stale rows in the pages).  The engine then works on."""
+    kind = fake_cuda.LAUNCH if what == "launch" else fake_cuda.TENSOR_MAP
+    rt = engine()
+    fake.reset()
+    chunk(rt)
+    names, calls = [n for n, _ in fake.launches()], fake.count(kind)
+    assert len(names) == 2 * 8 + 3 and calls == (len(names) if what == "launch" else 9 * 2 + 2 * 2)
+    before = -1
+    for at in range(calls):
+        fake.reset()
+        fake.fail(kind, at)
+        with pytest.raises(RuntimeError, match="prompt forward: " + ("launch refused" if what == "launch" else "a tensor map")):
+            chunk(rt)
+        went = [n for n, _ in fake.launches()]
+        assert went == names[:len(went)] and fake.count(kind) == at + 1
+        if what == "launch":
+            assert len(went) == at
+        else:                                                # two maps for each launch that takes some
+            assert before <= len(went) < len(names) and ("pair_kernel" in names[len(went)] or "flash_kernel" in names[len(went)])
+        before = len(went)
+    fake.reset()
+    chunk(rt)
+    assert [n for n, _ in fake.launches()] == names
+    rt.close()
