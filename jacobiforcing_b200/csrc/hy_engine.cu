@@ -145,6 +145,7 @@ struct hy_engine {
   cudaStream_t stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   std::string err;
+  std::string step_err;                          // what failed first in the running step (empty: nothing); nothing is launched behind it
   int64_t launches = 0;
   float last_ms = 0.0f;
   int64_t bytes_w = 0, bytes_cache = 0, bytes_state = 0, bytes_ws = 0;
@@ -191,16 +192,19 @@ struct hy_engine {
 // kernels of 2 to 9 us each (request of 512 + 24 tokens: 10.66 -> 9.47 ms).  Prompt steps keep plain launches: the blocks of a
 // kernel that starts under another one's tail pile up on the SMs that are free already, and a recurrence with one block per
 // SM then runs two or three on some of them (two Kinetar layers, 2048 tokens: 2.02 ms plain, 2.35 ms overlapped).
+// Behind the first launch of a step that fails nothing else is launched; hy_step reports it.
 constexpr int HY_OVERLAP_TOKENS = 64;
 template <typename... P, typename... A>
-inline void go_kernel(const hy_engine* h, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
+inline void go_kernel(hy_engine* h, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
   cudaLaunchAttribute at;
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at.val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t c = {};
   c.gridDim = grid; c.blockDim = block; c.dynamicSmemBytes = smem; c.stream = stream; c.attrs = &at;
   c.numAttrs = h->step_tokens <= HY_OVERLAP_TOKENS ? 1 : 0;
-  cudaLaunchKernelEx(&c, kernel, std::forward<A>(args)...);
+  if (!h->step_err.empty()) return;
+  const cudaError_t e = cudaLaunchKernelEx(&c, kernel, std::forward<A>(args)...);
+  if (e != cudaSuccess) h->step_err = cudaGetErrorString(e);
 }
 
 struct ProfScope {
@@ -1495,7 +1499,7 @@ inline bool gemm_takes_tiles(const void* A, int lda, int T, int K) {
 // The product on pairs of SMs: X [x_rows, K] (leading dimension lda), weight tiles of `groups` matrices [N, K], w_stride elements apart.
 // Grouped: tile_rows as the tile list was made.
 template <typename TO>
-int pair_product(hy_engine* h, const bf16* X, int lda, int x_rows, const void* tiled, int groups, size_t w_stride, int T, int N, int K,
+void pair_product(hy_engine* h, const bf16* X, int lda, int x_rows, const void* tiled, int groups, size_t w_stride, int T, int N, int K,
                  const GemmOut& o, int tile_rows, jf::TpGroup grp) {
   typedef HyEpilogue<TO> Epi;
   static bool attr = false;                                  // per TO: this function is a template
@@ -1508,8 +1512,11 @@ int pair_product(hy_engine* h, const bf16* X, int lda, int x_rows, const void* t
   const int bt = tile_rows ? tile_rows : jf::tp_tile_rows(N, T);
   const uint64_t w_rows = groups > 1 ? (uint64_t)groups * (w_stride / 64) : (uint64_t)NT * KT * 128;
   CUtensorMap xm, wm;
-  if (!jf::tp_map(&xm, X, (uint64_t)x_rows, (uint64_t)K, (uint64_t)lda, bt / 2, true) || !jf::tp_map(&wm, tiled, w_rows, 64, 64, 128, false))
-    return fail(h, HY_ERR_CUDA, "a tensor map of the matrix product could not be made");
+  if (!h->step_err.empty()) return;
+  if (!jf::tp_map(&xm, X, (uint64_t)x_rows, (uint64_t)K, (uint64_t)lda, bt / 2, true) || !jf::tp_map(&wm, tiled, w_rows, 64, 64, 128, false)) {
+    h->step_err = "a tensor map of the matrix product could not be made";
+    return;
+  }
   grp.w_rows = (int)(w_stride / 64);
   const long long most = (long long)nx * (grp.meta ? x_rows / bt + groups : (T + bt - 1) / bt);      // tiles (grouped: at most)
   const int parts = grp.meta ? 1 : jf::tp_parts((int)std::min<long long>(most, jf::TP_CLUSTERS + 1), K);
@@ -1518,7 +1525,6 @@ int pair_product(hy_engine* h, const bf16* X, int lda, int x_rows, const void* t
   go_kernel(h, kern, grid, jf::TP_THREADS, jf::tp_smem_bytes(bt), h->stream, xm, wm, T, N, K, Epi{o}, h->err_d, grp, jf::PairLayout{0, 0, 0},
             jf::PairSplit{parts, h->part_sums, h->part_arrived});
   h->launches++;
-  return HY_OK;
 }
 
 template <typename TA, typename TW, typename TO>
@@ -1528,7 +1534,8 @@ int gemm(hy_engine* h, const TA* A, int lda, const TW* Wt, int ldw, int T, int N
   if (o.alpha == 0.0f) o.alpha = 1.0f;
   if constexpr (std::is_same<TA, bf16>::value && std::is_same<TW, bf16>::value) {
     if (tiled && gemm_takes_tiles(A, lda, T, K)) {
-      return pair_product<TO>(h, (const bf16*)A, lda, T, tiled, 1, 0, T, N, K, o, 0, jf::TpGroup{});
+      pair_product<TO>(h, (const bf16*)A, lda, T, tiled, 1, 0, T, N, K, o, 0, jf::TpGroup{});
+      return HY_OK;
     }
   }
   constexpr int VECW = 16 / (int)sizeof(TW);
@@ -1808,8 +1815,12 @@ bool latent_prompt(hy_engine* h, const Batch& b, const LayerW& L, const hy_layer
   }
   ProfScope ps(h, HY_PROF_ATTN);
   CUtensorMap km, vm;
+  if (!h->step_err.empty()) return true;
   if (!jf::tp_map(&km, kv, (uint64_t)l->keys, (uint64_t)H * hk, (uint64_t)N, 128, true) ||
-      !jf::tp_map(&vm, kv + (size_t)H * hk, (uint64_t)l->keys, (uint64_t)H * dv, (uint64_t)N, 128, true)) return false;
+      !jf::tp_map(&vm, kv + (size_t)H * hk, (uint64_t)l->keys, (uint64_t)H * dv, (uint64_t)N, 128, true)) {
+    h->step_err = "a tensor map of the attention could not be made";      // not the folded form: the queries are rotated already
+    return true;
+  }
   const jf::FlashArgs fa{l->units, pin, (size_t)h->ld_pin, hk, nullptr, 1, c.l_scale, c.l_window, (const bf16*)L.sink,
                          c.l_gate ? pin + L.c_g : nullptr, (size_t)h->ld_pin, (bf16*)h->cat, (size_t)h->ld_cat, 0, h->err_d};
   auto go = [&](auto dk, auto dvv) {
@@ -3003,7 +3014,7 @@ extern "C" int hy_step(hy_handle h, int32_t n_entries, const int32_t* tokens, co
   b.T = T; b.E = E; b.max_pages = rt.max_pages_per_seq; b.page_size = rt.page_size;
   const int* want_d = b.pages + (size_t)E * rt.max_pages_per_seq;
   h->step_start = ent_start; h->step_pos0 = ent_pos0; h->step_tokens = T; h->units_used = 0; h->unit_lists.clear();
-  h->fl_used = 0; h->fl_lists.clear();
+  h->fl_used = 0; h->fl_lists.clear(); h->step_err.clear();
   HY_CUDA(cudaEventRecord(h->ev0, h->stream));
   if (h->m.dtype == HY_DTYPE_F32) run_step<float>(h, b, n_want, want_d, layers_out);
   else run_step<__nv_bfloat16>(h, b, n_want, want_d, layers_out);
@@ -3022,12 +3033,17 @@ extern "C" int hy_step(hy_handle h, int32_t n_entries, const int32_t* tokens, co
     HY_CUDA(cudaMemcpyAsync(logits_out, h->logits, (size_t)n_want * h->m.vocab * 4, cudaMemcpyDeviceToHost, h->stream));
   HY_CUDA(cudaMemcpyAsync(h->err_h, h->err_d, 4, cudaMemcpyDeviceToHost, h->stream));
   HY_CUDA(cudaStreamSynchronize(h->stream));
-  HY_CUDA(cudaGetLastError());
-  if (*h->err_h) {
+  const cudaError_t last = cudaGetLastError();
+  if (h->step_err.empty()) HY_CUDA(last);
+  if (*h->err_h && h->step_err.empty()) h->step_err = "a wait inside a tensor-core kernel ran out (pipeline stalled)";
+  if (!h->step_err.empty()) {                                // counters that kernels leave at zero, as the next step expects them
     *h->err_h = 0;
     cudaMemset(h->err_d, 0, 4);
     if (h->part_arrived) cudaMemset(h->part_arrived, 0, jf::TP_ARRIVED * 4);
-    return fail(h, HY_ERR_CUDA, "a wait inside the tensor-core matrix product ran out (pipeline stalled)");
+    if (h->x_counts) cudaMemset(h->x_counts, 0, (size_t)h->x_max_experts * 16);
+    for (auto& r : h->prof_list) { h->ev_pool.push_back(r.a); h->ev_pool.push_back(r.b); }
+    h->prof_list.clear();
+    return fail(h, HY_ERR_CUDA, h->step_err);
   }
   cudaEventElapsedTime(&h->last_ms, h->ev0, h->ev1);
   for (auto& r : h->prof_list) {

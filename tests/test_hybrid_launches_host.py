@@ -1,0 +1,79 @@
+"""Host side of the hybrid decoders' steps on a CUDA runtime without a GPU: a step stops at the first call that fails, whichever it is,
+says so, and leaves the engine able to run the next."""
+import pytest
+
+from tests import fake_cuda
+from tests import famepel_helpers as fam
+from tests import hybrid_helpers as kin
+from tests import kisadra_helpers as kis
+from tests import mafalorn_helpers as maf
+from tests import sebavik_helpers as seb
+from tests import vosolorn_helpers as vos
+
+FLASH = fam.model_config([fam.latent(heads=2, dim=64, rot_dim=64, vdim=64, kv_rank=40, q_rank=24, mlp=None), fam.glr()])
+
+
+def weights(cfg):
+    import importlib
+    plain = importlib.import_module("oracle.%s_plain" % cfg["architecture"].lower())
+    return plain.random_weights(cfg, 0, 8) if cfg["architecture"] == "Kinetar" else plain.random_weights(cfg, 0)
+
+
+CONFIGS = {"kinetar": kin.SMALL, "famepel": fam.SMALL, "flash": FLASH, "mafalorn": maf.SMALL, "kisadra": kis.SMALL, "sebavik": seb.SMALL, "vosolorn": vos.SMALL}
+
+
+@pytest.fixture(scope="module")
+def fake():
+    from jacobiforcing_b200 import _hybrid_cabi
+    path, mp = fake_cuda.build("hy"), pytest.MonkeyPatch()
+    mp.setattr(_hybrid_cabi, "LIB_PATH", path)
+    mp.setattr(_hybrid_cabi, "build", lambda force=False: path)
+    mp.setattr(_hybrid_cabi, "stale", lambda: False)
+    mp.setattr(_hybrid_cabi, "_lib", None)
+    yield fake_cuda.Fake(path)
+    mp.undo()
+
+
+def engine(cfg, dtype="bfloat16", device=0):
+    from jacobiforcing_b200.hybrid_config import HybridConfig
+    from jacobiforcing_b200.hybrid_runtime import HybridRuntime
+    w = weights(cfg)
+    rt = HybridRuntime(HybridConfig.from_dict(cfg, {k: tuple(t.shape) for k, t in w.items()}), dtype=dtype, device=device, max_step_tokens=256,
+                       max_step_entries=4, page_size=16, num_pages=64, max_pages_per_seq=16, num_slots=4, max_want=16)
+    rt.load_state_dict(w)
+    return rt
+
+
+def step(rt, tokens, entries=1):
+    n = tokens // entries
+    return rt.step([([1] * n, 0, e, list(range(16 * e, 16 * e + 16))) for e in range(entries)], [tokens - 1], want_logits=True, sample=True)
+
+
+@pytest.mark.parametrize("tokens", [3, 150])
+@pytest.mark.parametrize("which", sorted(CONFIGS))
+@pytest.mark.parametrize("what", ["launch", "tensor map"])
+def test_nothing_is_launched_behind_a_failure(fake, what, which, tokens):
+    """Were the failure dropped, the step would return what its buffers happened to hold, or rotate the same queries twice."""
+    kind = fake_cuda.LAUNCH if what == "launch" else fake_cuda.TENSOR_MAP
+    rt = engine(CONFIGS[which])
+    step(rt, tokens)
+    names = []
+    for _ in range(2):                                       # routing counters alternate between two sets: two steps that are alike
+        fake.reset()
+        step(rt, tokens)
+        names.append([n for n, _ in fake.launches()])
+    calls, names = fake.count(kind), names[0]
+    assert len(names) > 3
+    if which == "flash" and tokens > 64:
+        assert any("flash_kernel" in n for n in names)
+    for at in range(calls):
+        fake.reset()
+        fake.fail(kind, at)
+        with pytest.raises(RuntimeError, match="launch refused" if what == "launch" else "a tensor map of the"):
+            step(rt, tokens)
+        went = [n for n, _ in fake.launches()]
+        assert went == names[:len(went)] and len(went) < len(names) and fake.count(kind) == at + 1
+        fake.reset()
+        step(rt, tokens)
+        assert [n for n, _ in fake.launches()] == names
+    rt.close()
