@@ -146,6 +146,7 @@ struct hy_engine {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   std::string err;
   std::string step_err;                          // what failed first in the running step (empty: nothing); nothing is launched behind it
+  std::map<const void*, size_t> smem_limit;      // dynamic shared memory that a kernel is opted in to on this engine's device
   int64_t launches = 0;
   float last_ms = 0.0f;
   int64_t bytes_w = 0, bytes_cache = 0, bytes_state = 0, bytes_ws = 0;
@@ -193,7 +194,18 @@ struct hy_engine {
 // kernel that starts under another one's tail pile up on the SMs that are free already, and a recurrence with one block per
 // SM then runs two or three on some of them (two Kinetar layers, 2048 tokens: 2.02 ms plain, 2.35 ms overlapped).
 // Behind the first launch of a step that fails nothing else is launched; hy_step reports it.
+// More shared memory than every kernel may have (48 KiB with its static part) is asked for here, once per engine, kernel and size: the limit belongs
+// to a device, and a process may hold engines on several.
 constexpr int HY_OVERLAP_TOKENS = 64;
+constexpr size_t HY_PLAIN_SMEM = 16 * 1024;
+inline cudaError_t opt_in(hy_engine* h, const void* kernel, size_t smem) {
+  if (smem <= HY_PLAIN_SMEM) return cudaSuccess;
+  size_t& limit = h->smem_limit[kernel];
+  if (limit >= smem) return cudaSuccess;
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e == cudaSuccess) limit = smem;
+  return e;
+}
 template <typename... P, typename... A>
 inline void go_kernel(hy_engine* h, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
   cudaLaunchAttribute at;
@@ -203,7 +215,8 @@ inline void go_kernel(hy_engine* h, void (*kernel)(P...), dim3 grid, dim3 block,
   c.gridDim = grid; c.blockDim = block; c.dynamicSmemBytes = smem; c.stream = stream; c.attrs = &at;
   c.numAttrs = h->step_tokens <= HY_OVERLAP_TOKENS ? 1 : 0;
   if (!h->step_err.empty()) return;
-  const cudaError_t e = cudaLaunchKernelEx(&c, kernel, std::forward<A>(args)...);
+  cudaError_t e = opt_in(h, (const void*)kernel, smem);
+  if (e == cudaSuccess) e = cudaLaunchKernelEx(&c, kernel, std::forward<A>(args)...);
   if (e != cudaSuccess) h->step_err = cudaGetErrorString(e);
 }
 
@@ -1502,12 +1515,6 @@ template <typename TO>
 void pair_product(hy_engine* h, const bf16* X, int lda, int x_rows, const void* tiled, int groups, size_t w_stride, int T, int N, int K,
                  const GemmOut& o, int tile_rows, jf::TpGroup grp) {
   typedef HyEpilogue<TO> Epi;
-  static bool attr = false;                                  // per TO: this function is a template
-  if (!attr) {
-    cudaFuncSetAttribute(jf::pair_kernel<Epi, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)jf::tp_smem_bytes(128));
-    cudaFuncSetAttribute(jf::pair_kernel<Epi, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)jf::tp_smem_bytes(256));
-    attr = true;
-  }
   const int nx = (N + 255) / 256, KT = (K + 63) / 64, NT = (N + 127) / 128;
   const int bt = tile_rows ? tile_rows : jf::tp_tile_rows(N, T);
   const uint64_t w_rows = groups > 1 ? (uint64_t)groups * (w_stride / 64) : (uint64_t)NT * KT * 128;
@@ -1549,14 +1556,6 @@ int gemm(hy_engine* h, const TA* A, int lda, const TW* Wt, int ldw, int T, int N
     // on two layers of width 1024, 16 blocks per SM at most 14.65 ms, 4 14.1, 2 14.15, 1 (too few loads in flight) 16.6.  One row: no difference.
     const int blocks = std::min((N + cpb - 1) / cpb, 148 * (T > 4 ? 4 : 16));
     const int fit = (int)((200 * 1024) / row_bytes);
-    static bool rows_attr = false;                        // per <TA, TW, TO>: this function is a template
-    if (!rows_attr) {
-      cudaFuncSetAttribute(gemm_rows_kernel<TA, TW, TO, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-      cudaFuncSetAttribute(gemm_rows_kernel<TA, TW, TO, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-      cudaFuncSetAttribute(gemm_rows_kernel<TA, TW, TO, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-      cudaFuncSetAttribute(gemm_rows_kernel<TA, TW, TO, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-      rows_attr = true;
-    }
     auto launch = [&](auto kern, int rows) {
       const size_t smem = (size_t)rows * row_bytes;
       go_kernel(h, kern, dim3(blocks, (T + rows - 1) / rows), 256, smem, h->stream, A, lda, Wt, ldw, T, N, K, ksplit, o);
@@ -1826,8 +1825,6 @@ bool latent_prompt(hy_engine* h, const Batch& b, const LayerW& L, const hy_layer
   auto go = [&](auto dk, auto dvv) {
     constexpr int DK = decltype(dk)::value, DV = decltype(dvv)::value;
     constexpr size_t smem = jf::fl_smem_bytes(DK, DV);
-    static bool attr = false;                                // per kernel: go is a template
-    if (!attr) { cudaFuncSetAttribute(jf::flash_kernel<DK, DV, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); attr = true; }
     go_kernel(h, jf::flash_kernel<DK, DV, true>, l->n, jf::FL_THREADS, smem, s, km, vm, km, vm, fa);
   };
   typedef std::integral_constant<int, 64> c64; typedef std::integral_constant<int, 128> c128; typedef std::integral_constant<int, 192> c192;
@@ -1898,13 +1895,6 @@ void latent_mixer(hy_engine* h, const Batch& b, const LayerW& L, const hy_layer_
         tc = true;
         const int nt = R <= 128 ? 2 : R <= 256 ? 4 : 8, pstride = nt * 64;
         const size_t smem = attn_wide_smem(Dk);
-        static bool wide_attr = false;
-        if (!wide_attr) {
-          cudaFuncSetAttribute(attn_wide_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)attn_wide_smem(640));
-          cudaFuncSetAttribute(attn_wide_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)attn_wide_smem(640));
-          cudaFuncSetAttribute(attn_wide_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)attn_wide_smem(640));
-          wide_attr = true;
-        }
 #define HY_WIDE_ARGS b, u->d, cv, h->ld_cv, (const bf16*)L.cache, H, Dk, R, c.l_scale, c.l_window, u->split, u->ns, pstride, \
         h->part_o, h->part_ml
         if (nt == 2) go_kernel(h, attn_wide_kernel<2>, u->n, 256, smem, s, HY_WIDE_ARGS);
@@ -1997,7 +1987,6 @@ int sandwich_layer(hy_engine* h, const Batch& b, size_t li) {
         constexpr int DR = decltype(dr)::value, PARTS = decltype(parts)::value, VC = decltype(vcols)::value;
         const LinearLaunch g = linear_launch<AT>(PARTS, VC, N, P, cv, h->ld_cv);
         const size_t smem = lin_smem<AT>(DR, PARTS, VC, 0);
-        cudaFuncSetAttribute(gla_kernel<AT, DR, PARTS, VC, GLA_TOKEN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         go_kernel(h, gla_kernel<AT, DR, PARTS, VC, GLA_TOKEN>, dim3(H * g.bph, E), 128, smem, s, b, h->lin, cv, h->ld_cv, nullptr, 0, nullptr, H, N, P, g.bph,
                                                                                    g.vec, g.vvec, L.rec_state, h->f2, h->ld_f2, tk);
       });
@@ -2024,15 +2013,12 @@ int sandwich_layer(hy_engine* h, const Batch& b, size_t li) {
         constexpr int DR = decltype(dr)::value, PARTS = decltype(parts)::value, VC = decltype(vcols)::value;
         const LinearLaunch g = linear_launch<AT>(PARTS, VC, dk, dv, pin + L.c_v, h->ld_pin);
         const size_t smem = lin_smem<AT>(DR, PARTS, VC, 0);
-        cudaFuncSetAttribute(gla_kernel<AT, DR, PARTS, VC, GLA_FORGET>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         go_kernel(h, gla_kernel<AT, DR, PARTS, VC, GLA_FORGET>, dim3(H * g.bph, E), 128, smem, s, b, h->lin, pin + L.c_v, h->ld_pin, nullptr, 0, nullptr, H, dk,
                                                                                     dv, g.bph, g.vec, g.vvec, L.rec_state, h->f2, h->ld_f2, GlaToken{});
       });
       go_kernel(h, gla_out_kernel<AT, AT, GATE_NONE>, (T * H + 3) / 4, 128, 0, s, T, H, dv, h->f2, h->ld_f2, nullptr, 0, L.g_norm, eps, 1.0f, cat, h->ld_cat);
       h->launches += 3;
     } else {
-      static bool glr_attr = false;
-      if (!glr_attr) { cudaFuncSetAttribute(glr_kernel<AT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024); glr_attr = true; }
       go_kernel(h, glr_kernel<AT>, dim3(H, E), 256, ((size_t)dk * dv + 2 * dk + dv + 40) * 4, s, 
           b, pin, h->ld_pin, L.c_q, L.c_k, L.c_v, L.g_fb, L.g_lower, L.g_norm, H, dk, dv, eps, L.rec_state, cat, h->ld_cat);
       h->launches++;
@@ -2066,12 +2052,6 @@ int sandwich_layer(hy_engine* h, const Batch& b, size_t li) {
     ProfScope ps(h, HY_PROF_EXPERTS);
     float* ys = h->f2;                                        // [pairs, width] fp32
     if (few) {
-      static bool rows_attr = false;
-      if (!rows_attr) {
-        cudaFuncSetAttribute(expert_rows_kernel<AT, WT, AT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        cudaFuncSetAttribute(expert_rows_kernel<AT, WT, float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        rows_attr = true;
-      }
       go_kernel(h, expert_rows_kernel<AT, WT, AT, true>, dim3(std::min((ff + 7) / 8, 256), P), 256, (size_t)W * sizeof(AT), s, 
           hb, W, h->x_ids, top, 1, NE, (const WT*)L.w_gu, (size_t)2 * ff * W, ff, W, pin, ldh, 0, 0.0f);
       go_kernel(h, expert_rows_kernel<AT, WT, float, false>, dim3(std::min((W + 7) / 8, 256), P), 256, (size_t)ff * sizeof(AT), s, 
@@ -2103,8 +2083,6 @@ template <typename AT>
 void post_norm_add(hy_engine* h, int T, const float* y, int ldy, const float* rows, const int* pair_row, const float* wts, int top,
                    const float* shared_rows, const float* w, const float* ls, int add) {
   const int W = h->m.width;
-  static bool attr = false;                                  // per AT: this function is a template
-  if (!attr) { cudaFuncSetAttribute(post_norm_add_kernel<AT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024); attr = true; }
   go_kernel(h, post_norm_add_kernel<AT>, T, 256, (size_t)W * 4, h->stream, y, ldy, rows, W, pair_row, wts, top, shared_rows, w, ls, h->m.norm_eps,
                                                                W, add, h->x, (AT*)h->hbuf);
   h->launches++;
@@ -2157,12 +2135,6 @@ int postnorm_layer(hy_engine* h, const Batch& b, size_t li) {
           tc = true;
 #define HY_WIN_ARGS b, u->d, cv, h->ld_cv, wc, (const bf16*)L.cache, (const bf16*)L.cache_v, (const bf16*)L.pool_k, \
           (const bf16*)L.pool_v, h->f1, h->ld_f1, cat, h->ld_cat
-          static bool win_attr = false;
-          if (!win_attr) {
-            cudaFuncSetAttribute(window_mma_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)window_mma_smem(64));
-            cudaFuncSetAttribute(window_mma_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)window_mma_smem(128));
-            win_attr = true;
-          }
           if (c.w_dim <= 64 && c.w_vdim <= 64) go_kernel(h, window_mma_kernel<64>, u->n, 128, window_mma_smem(64), s, HY_WIN_ARGS);
           else go_kernel(h, window_mma_kernel<128>, u->n, 128, window_mma_smem(128), s, HY_WIN_ARGS);
 #undef HY_WIN_ARGS
@@ -2183,14 +2155,6 @@ int postnorm_layer(hy_engine* h, const Batch& b, size_t li) {
       gemm<AT, WT, AT>(h, hb, W, (const WT*)L.w_in, W, T, L.n_in, W, o, L.w_in_t);
     }
     ProfScope ps(h, HY_PROF_DELTA);
-    static bool attr = false;
-    if (!attr) {
-      cudaFuncSetAttribute(mlstm_reg_kernel<AT, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-      cudaFuncSetAttribute(mlstm_reg_kernel<AT, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-      cudaFuncSetAttribute(mlstm_reg_kernel<AT, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-      cudaFuncSetAttribute(mlstm_kernel<AT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-      attr = true;
-    }
 #define HY_MLSTM_GEN_ARGS b, pin, h->ld_pin, L.c_q, L.c_k, L.c_v, L.c_g, h->f1, h->ld_f1, 0, H, L.t_ib, L.t_fb, L.t_norm, H, dk, dv, \
     c.t_gate_cap, eps, L.rec_state, cat, h->ld_cat
 #define HY_MLSTM_ARGS b, pin, h->ld_pin, L.c_q, L.c_k, L.c_v, L.c_g, h->f1, h->ld_f1, 0, H, L.t_ib, L.t_fb, L.t_norm, H, dk, dv, \
@@ -2274,12 +2238,6 @@ int postnorm_layer(hy_engine* h, const Batch& b, size_t li) {
   {
     ProfScope ps(h, HY_PROF_EXPERTS);
     if (few) {
-      static bool rows_attr = false;
-      if (!rows_attr) {
-        cudaFuncSetAttribute(expert_rows_kernel<AT, WT, AT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        cudaFuncSetAttribute(expert_rows_kernel<AT, WT, float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        rows_attr = true;
-      }
       go_kernel(h, expert_rows_kernel<AT, WT, AT, false>, dim3(std::min((ff + 7) / 8, 256), P), 256, (size_t)W * sizeof(AT), s, 
           hb, W, h->x_ids, top, 1, NE, (const WT*)L.w_gu, (size_t)ff * W, ff, W, pin, ldh, c.x_act, c.ff_limit);
       go_kernel(h, expert_rows_kernel<AT, WT, float, false>, dim3(std::min((W + 7) / 8, 256), P), 256, (size_t)ff * sizeof(AT), s, 
@@ -2347,12 +2305,6 @@ bool routed_gated_experts(hy_engine* h, int T, const AT* hb, const LayerW& L, co
   ProfScope ps(h, HY_PROF_EXPERTS);
   float* ys = h->f2;
   if (few) {
-    static bool rows_attr = false;
-    if (!rows_attr) {
-      cudaFuncSetAttribute(expert_rows_kernel<AT, WT, AT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-      cudaFuncSetAttribute(expert_rows_kernel<AT, WT, float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-      rows_attr = true;
-    }
     go_kernel(h, expert_rows_kernel<AT, WT, AT, true>, dim3(std::min((ff + 7) / 8, 256), P), 256, (size_t)W * sizeof(AT), s, 
         hb, W, h->x_ids, top, 1, NE, (const WT*)L.w_gu, (size_t)2 * ff * W, ff, W, pin, ldh, c.x_act, c.ff_limit);
     go_kernel(h, expert_rows_kernel<AT, WT, float, false>, dim3(std::min((W + 7) / 8, 256), P), 256, (size_t)ff * sizeof(AT), s, 
@@ -2380,8 +2332,6 @@ bool routed_gated_experts(hy_engine* h, int T, const AT* hb, const LayerW& L, co
 template <typename WT>
 void stream_row(hy_engine* h, const Batch& b, const StreamOp& o) {
   const int W = h->m.width;
-  static bool attr = false;                                  // per WT: this function is a template
-  if (!attr) { cudaFuncSetAttribute(stream_row_kernel<WT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024); attr = true; }
   go_kernel(h, stream_row_kernel<WT>, b.T, 256, ((size_t)2 * W + (size_t)std::max(o.side_dim, 0)) * 4, h->stream, b, o, W, h->x);
   h->launches++;
 }
@@ -2438,14 +2388,6 @@ void biased_attend(hy_engine* h, const Batch& b, const LayerW& L, const hy_layer
       if (!simt_only && c.b_dim % 8 == 0 && c.b_vdim % 8 == 0 && c.b_dim <= 128 && c.b_vdim <= 128 && h->ld_pin % 8 == 0 && L.c_q % 8 == 0 && h->units_d &&
           (u = biased_units(h, E, T, bc, dp))) {
         tc = true;
-        static bool attr = false;
-        if (!attr) {
-          cudaFuncSetAttribute(biased_mma_kernel<64, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)window_mma_smem(64));
-          cudaFuncSetAttribute(biased_mma_kernel<64, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)window_mma_smem(64));
-          cudaFuncSetAttribute(biased_mma_kernel<128, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)window_mma_smem(128));
-          cudaFuncSetAttribute(biased_mma_kernel<128, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)window_mma_smem(128));
-          attr = true;
-        }
 #define HY_BIASED_ARGS b, u->d, pin + L.c_q, h->ld_pin, bc, (const bf16*)L.cache, (const bf16*)L.cache_v, cat, h->ld_cat, u->ns, h->part_o, h->part_ml
         const bool pl = bc.bias == HY_BIAS_NONE && bc.cap <= 0.0f && !bc.window && !bc.keep && !bc.chunk;
         if (dp == 64) {
@@ -2574,7 +2516,6 @@ void gla_mixer(hy_engine* h, const Batch& b, const LayerW& L, const hy_layer_cfg
     constexpr int DR = decltype(dr)::value, PARTS = decltype(parts)::value, VC = decltype(vcols)::value;
     const LinearLaunch g = linear_launch<AT>(PARTS, VC, dk, dv, pin + L.c_v, h->ld_pin);
     const size_t smem = lin_smem<AT>(DR, PARTS, VC, DR);
-    cudaFuncSetAttribute(gla_kernel<AT, DR, PARTS, VC, GLA_CHANNEL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     go_kernel(h, gla_kernel<AT, DR, PARTS, VC, GLA_CHANNEL>, dim3(H * g.bph, E), 128, smem, s, b, h->lin, pin + L.c_v, h->ld_pin, h->f2, h->ld_f2, nullptr, H, dk,
                                                                            dv, g.bph, g.vec, g.vvec, L.rec_state, h->f2 + c_o, h->ld_f2, GlaToken{});
   });
@@ -2597,7 +2538,6 @@ void retention_mixer(hy_engine* h, const Batch& b, const LayerW& L, const hy_lay
     constexpr int DR = decltype(dr)::value, PARTS = decltype(parts)::value, VC = decltype(vcols)::value;
     const LinearLaunch g = linear_launch<AT>(PARTS, VC, dk, dv, pin + L.c_v, h->ld_pin);
     const size_t smem = lin_smem<AT>(DR, PARTS, VC, 0);
-    cudaFuncSetAttribute(gla_kernel<AT, DR, PARTS, VC, GLA_HEAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     go_kernel(h, gla_kernel<AT, DR, PARTS, VC, GLA_HEAD>, dim3(H * g.bph, E), 128, smem, s, b, h->lin, pin + L.c_v, h->ld_pin, nullptr, 0, L.decay, H, dk, dv,
                                                                           g.bph, g.vec, g.vvec, L.rec_state, h->f2, h->ld_f2, GlaToken{});
   });
@@ -2635,7 +2575,6 @@ void attn_delta_mixer(hy_engine* h, const Batch& b, const LayerW& L, const hy_la
     constexpr int DR = decltype(dr)::value, PARTS = decltype(parts)::value, VC = decltype(vcols)::value;
     const LinearLaunch g = linear_launch<AT>(PARTS, VC, dk, dv, cv, h->ld_cv);
     const size_t smem = lin_smem<AT>(DR, PARTS, VC, 4);
-    cudaFuncSetAttribute(delta_head_kernel<AT, DR, PARTS, VC, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     go_kernel(h, delta_head_kernel<AT, DR, PARTS, VC, false>, dim3(H * g.bph, E), 128, smem, s, b, h->lin, cv, h->ld_cv, h->lin_sc, H, G, dk, dv, g.bph, g.vec, g.vvec,
                                                                            L.rec_state, h->f2, h->ld_f2, nullptr, 0);
   });
@@ -2649,12 +2588,6 @@ template <typename AT>
 void launch_row_close(hy_engine* h, int T, RowClose rc) {
   typedef AT WT;
   const int W = h->m.width;
-  static bool attr = false;                                  // per AT: this function is a template
-  if (!attr) {
-    cudaFuncSetAttribute(row_close_kernel<AT, WT, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaFuncSetAttribute(row_close_kernel<AT, WT, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    attr = true;
-  }
   rc.eps = h->m.norm_eps;
   if (!rc.rows && !rc.y && !rc.cast_out && !rc.norm_w) return;
   ProfScope ps(h, HY_PROF_NORM);
@@ -2885,8 +2818,6 @@ int run_step(hy_engine* h, const Batch& b, int n_want, const int* want_d, float*
         auto go = [&](auto np, auto ln) {
           constexpr int NPER = decltype(np)::value, LN = decltype(ln)::value, PB = 128 / LN;
           const size_t smem = scan_smem(NPER * LN, PB, sizeof(AT));
-          static bool attr = false;                            // per kernel: go is a template
-          if (!attr) { cudaFuncSetAttribute(scan_kernel<AT, WT, NPER, LN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); attr = true; }
           // 16-byte copies: whole blocks of channels, rows and columns on 16-byte boundaries
           const int v32 = (R | N | h->ld_f1 | h->ld_f2 | I) % 4 == 0 && PB % 4 == 0;
           const int vat = (h->ld_cv | h->ld_pin | L.c_z | I) % ch == 0 && PB % ch == 0;
@@ -2929,7 +2860,6 @@ int run_step(hy_engine* h, const Batch& b, int n_want, const int* want_d, float*
         constexpr int DR = decltype(dr)::value, PARTS = decltype(parts)::value, VC = decltype(vcols)::value;
         const LinearLaunch g = linear_launch<AT>(PARTS, VC, dk, dv, cv, h->ld_cv);
         const size_t smem = lin_smem<AT>(DR, PARTS, VC, DR + 4);
-        cudaFuncSetAttribute(delta_head_kernel<AT, DR, PARTS, VC, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         go_kernel(h, delta_head_kernel<AT, DR, PARTS, VC, true>, dim3(H * g.bph, E), 128, smem, s, b, h->lin, cv, h->ld_cv, h->lin_sc, H, G, dk, dv, g.bph, g.vec,
                                                                                      g.vvec, L.rec_state, o, h->ld_f2, h->f1, h->ld_f1);
       });

@@ -1,5 +1,5 @@
 """Host side of the hybrid decoders' steps on a CUDA runtime without a GPU: a step stops at the first call that fails, whichever it is,
-says so, and leaves the engine able to run the next."""
+says so, and leaves the engine able to run the next; kernels are set up on every device that an engine is made on."""
 import pytest
 
 from tests import fake_cuda
@@ -76,4 +76,33 @@ def test_nothing_is_launched_behind_a_failure(fake, what, which, tokens):
         fake.reset()
         step(rt, tokens)
         assert [n for n, _ in fake.launches()] == names
+    rt.close()
+
+
+@pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
+@pytest.mark.parametrize("which", sorted(CONFIGS))
+def test_steps_on_two_devices(fake, which, dtype):
+    """A kernel's shared-memory limit belongs to a device: the fake refuses launches above what was asked for on theirs."""
+    seen = []
+    for device in (0, 1):
+        rt = engine(CONFIGS[which], dtype, device)
+        fake.reset()
+        for tokens in (1, 4, 150):
+            step(rt, tokens)
+        step(rt, 152, 4)
+        seen.append([n for n, _ in fake.launches()])
+        assert {d for _, d in fake.launches()} == {device}
+        rt.close()
+    assert seen[0] == seen[1]
+
+
+def test_refused_shared_memory_is_reported(fake):
+    rt = engine(FLASH)
+    fake.reset()
+    fake.fail(fake_cuda.ATTRIBUTE, 0)
+    with pytest.raises(RuntimeError, match="invalid argument"):
+        step(rt, 150)
+    went = fake.launches()
+    step(rt, 150)                                            # asked for again
+    assert len(fake.launches()) > 2 * len(went)
     rt.close()
