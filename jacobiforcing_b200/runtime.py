@@ -307,12 +307,18 @@ class JacobiRuntime:
             if end < total and total - end < n + 1:   # keep the n+1 logit rows inside one chunk
                 end = max(start + 1, total - (n + 1))
             # Chunks of whole pages, all of whose rows are committed, are what the library runs as one kernel per stage; the rest of
-            # the row (what a request whose pages are cached already forwards too, so that a prefix hit changes nothing) follows
+            # the row follows on the persistent kernel.  A prefix hit on pages that such chunks filled changes nothing, bit for bit: a row's
+            # result does not depend on the cut, and the rest is forwarded by the same kernel.  Pages that the rest of a prompt or decoding
+            # filled come from the persistent kernel; a longer prompt that hits them differs from one that does not by bf16 rounding.
             if start % PAGE == 0 and pages_end - start >= PAGE and self.max_rows >= PAGE and self.tp_size == 1:
                 end = start + min(pages_end - start, self.max_rows // PAGE * PAGE)
             toks = row[start:end]
             T = end - start
-            commits = [(i, 0, start + i) for i in range(T) if start + i < P]
+            commits, late = [(i, 0, start + i) for i in range(T) if start + i < P], []
+            # Without a draft the rest may be a whole page of committed rows.  A full hit forwards the last prompt token on the persistent
+            # kernel; the call of its own that commits the last row keeps a miss there too
+            if end == total and len(commits) == T >= PAGE and self.tp_size == 1:
+                late = [commits.pop()]
             lm0 = max(0, want_from - start)
             lm_row0, lm_rows = 0, 0
             if end > want_from:
@@ -320,6 +326,7 @@ class JacobiRuntime:
                 lm_rows = T - lm_row0
             res = self.forward(toks, [(0, T, 0, start)], [seq], lm_row0, lm_rows, commits)
             ms += res["ms"]
+            self.commit_rows([seq], late)
             self.stats["prefill_rows"] = self.stats.get("prefill_rows", 0) + T
             if end > want_from:
                 out.extend(int(t) for t in res["greedy"][lm0:T])

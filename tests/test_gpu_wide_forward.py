@@ -96,3 +96,48 @@ def test_sequences_side_by_side(pair):
     finally:
         for s in seqs:
             rt.release(s)
+
+
+def cached_copy(rt, seq, tokens):
+    """A sequence that shares the pages of `seq` for its first `tokens` tokens, as the block manager hands them out on a prefix hit."""
+    s = rt.new_sequence()
+    s.pages, s.ctx = list(seq.pages[:tokens // 256]), tokens
+    return s
+
+
+@pytest.mark.parametrize("n,cached,draft", [(256, 256, 0), (512, 512, 0), (512, 256, 0), (768, 768, 0), (512, 256, 8), (600, 512, 0), (600, 256, 8)])
+def test_prefix_hit_equals_miss(pair, n, cached, draft):
+    """Prompts that end inside a page, at its end, with a draft and without: the same tokens, and the same logits behind them bit for bit."""
+    model, rt = pair
+    toks = prompt_of(n + 8, 31, model.config.vocab_size)
+    miss = rt.new_sequence()
+    got = [rt.prefill(miss, toks[:n], toks[:draft])[:2], verify(rt, miss, toks[n:])]
+    hit = cached_copy(rt, miss, cached)
+    own = len(hit.pages)
+    try:
+        got += [rt.prefill(hit, toks[:n], toks[:draft])[:2], verify(rt, hit, toks[n:])]
+    finally:
+        hit.pages = hit.pages[own:]
+        rt.release(hit)
+        rt.release(miss)
+    assert got[0] == got[2] and np.array_equal(got[1], got[3])
+
+
+def test_hit_on_a_page_that_the_end_of_a_prompt_filled(pair):
+    """The last page of a 512-token prompt comes from the persistent kernel, the same page of a longer prompt from the stages: a hit on it
+    is a miss to bf16 rounding, no more (bound of the comparisons with HF)."""
+    model, rt = pair
+    toks = prompt_of(608, 33, model.config.vocab_size)
+    short, miss = rt.new_sequence(), rt.new_sequence()
+    rt.prefill(short, toks[:512], toks[:8])
+    rt.prefill(miss, toks[:600], toks[:8])
+    hit = cached_copy(rt, short, 512)
+    own = len(hit.pages)
+    try:
+        rt.prefill(hit, toks[:600], toks[:8])
+        a, b = verify(rt, hit, toks[600:]), verify(rt, miss, toks[600:])
+    finally:
+        hit.pages = hit.pages[own:]
+        for s in (hit, miss, short):
+            rt.release(s)
+    assert np.linalg.norm(a - b) < 2e-2 * np.linalg.norm(b)

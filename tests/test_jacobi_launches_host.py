@@ -1,5 +1,5 @@
-"""Host side of the Jacobi engine's prompt forwards: kernels are set up on every device that an engine is made on, and a forward stops at
-the first call that fails."""
+"""Host side of the Jacobi engine's prompt forwards: kernels are set up on every device that an engine is made on, a forward stops at
+the first call that fails, and which rows of a prompt run on which kernel."""
 import pytest
 
 from tests import fake_cuda
@@ -85,4 +85,36 @@ def test_nothing_is_launched_behind_a_failure(fake, what):
     fake.reset()
     chunk(rt)
     assert [n for n, _ in fake.launches()] == names
+    rt.close()
+
+
+@pytest.mark.parametrize("draft", [0, 8])
+@pytest.mark.parametrize("prompt,cached", [(1, 0), (255, 0), (256, 0), (256, 256), (257, 0), (257, 256), (300, 256), (511, 256), (512, 0), (512, 256), (512, 512), (600, 0), (600, 512),
+                                           (768, 0), (768, 512), (768, 768)])
+def test_the_last_prompt_token_runs_on_the_persistent_kernel(fake, prompt, cached, draft):
+    """Whether its pages were cached or not: the two kernels do not agree bit for bit.  Whole pages ahead of it run as stages."""
+    rt = engine()
+    s = rt.new_sequence()
+    s.ctx = cached
+    runs, commits, forward, commit_rows = [], [], rt.forward, rt.commit_rows
+
+    def spy(tokens, groups, seqs, lm_row0, lm_rows, com=(), **kw):
+        fake.reset()
+        out = forward(tokens, groups, seqs, lm_row0, lm_rows, com, **kw)
+        runs.append((groups[0][3], len(tokens), lm_rows, ["persistent" in n for n, _ in fake.launches()]))
+        commits.extend(c[2] for c in com)
+        return out
+
+    def spy_commits(seqs, com):
+        commits.extend(c[2] for c in com)
+        commit_rows(seqs, com)
+    rt.forward, rt.commit_rows = spy, spy_commits
+    rt.prefill(s, [1] * prompt, [1] * draft)
+    at, rows, lm_rows, kernels = runs[-1]
+    assert kernels == [True] and at <= prompt - 1 < at + rows == prompt + draft and lm_rows > draft
+    for at, rows, lm_rows, kernels in runs[:-1]:
+        assert at % 256 == 0 and rows % 256 == 0 and lm_rows == 0 and len(kernels) == 2 * 8 + 1 and not any(kernels)
+    assert sum(r[1] for r in runs[:-1]) == max(0, (prompt - 1) // 256 * 256 - cached)
+    assert commits == list(range(min(cached, prompt - 1), prompt))
+    rt.release(s)
     rt.close()
