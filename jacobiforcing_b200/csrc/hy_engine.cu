@@ -1782,7 +1782,7 @@ const hy_engine::FlashList* flash_units(hy_engine* h, int E, int H) {
   for (int e = 0; e < E; ++e) {
     const int len = h->step_start[e + 1] - h->step_start[e];
     for (int p = (len - 1) / 128 * 128; p >= 0; p -= 128)
-      for (int hd = 0; hd < H; ++hd) u[n++] = jf::FlashUnit{h->step_start[e], len, p, len, hd, hd, h->step_pos0[e], off[e], 0, 0, 0};
+      for (int hd = 0; hd < H; ++hd) u[n++] = jf::FlashUnit{h->step_start[e], len, p, len, hd, hd, h->step_pos0[e], off[e], -1};
   }
   const size_t bytes = (unsigned char*)(u + n) - at;
   unsigned char* d = h->fl_d + h->fl_used;
@@ -1825,7 +1825,7 @@ bool latent_prompt(hy_engine* h, const Batch& b, const LayerW& L, const hy_layer
   auto go = [&](auto dk, auto dvv) {
     constexpr int DK = decltype(dk)::value, DV = decltype(dvv)::value;
     constexpr size_t smem = jf::fl_smem_bytes(DK, DV);
-    go_kernel(h, jf::flash_kernel<DK, DV, true>, l->n, jf::FL_THREADS, smem, s, km, vm, km, vm, fa);
+    go_kernel(h, jf::flash_kernel<DK, DV, true>, l->n, jf::FL_THREADS, smem, s, km, vm, fa);
   };
   typedef std::integral_constant<int, 64> c64; typedef std::integral_constant<int, 128> c128; typedef std::integral_constant<int, 192> c192;
   if (hk == 64) { if (dv == 64) go(c64{}, c64{}); else go(c64{}, c128{}); }

@@ -21,14 +21,14 @@ constexpr int FL_THREADS = 192;
 constexpr int FL_KEYS = 128;
 
 // Rows pair0 .. pair0 + 127 (at most heads * len) of key head `kvh`: pair p is token row0 + p % len (position pos0 + p % len) of head
-// head0 + p / len.  Keys: positions 0 .. paged - 1 in pages of the table at `table`, positions key_pos0 and up as rows own_row0 and up of
-// the own maps (paged = pos0 + len = key_pos0: all in pages; paged = key_pos0 = 0: none).
-struct FlashUnit { int row0, len, pair0, pairs, head0, kvh, pos0, own_row0, key_pos0, paged, table; };
+// head0 + p / len.  The key of position j is in the pages of the table at `table`, or (table < 0) row own_row0 + j of the maps, columns of
+// key head `kvh`.
+struct FlashUnit { int row0, len, pair0, pairs, head0, kvh, pos0, own_row0, table; };
 
 struct FlashArgs {
   const FlashUnit* units;
   const __nv_bfloat16* q; size_t ldq; int q_head;        // head h's query at column h * q_head
-  const int* page_table; int kv_heads;                   // pages: row ((page * kv_heads + kvh) * 256 + slot) of the paged maps
+  const int* page_table; int kv_heads;                   // pages: row ((page * kv_heads + kvh) * 256 + slot) of the maps
   float scale; int window;                               // window > 0: only keys j with i - j < window
   const __nv_bfloat16* sink;                             // [heads] a logit without key and value (NULL: none)
   const __nv_bfloat16* gate; size_t ldg;                 // output times sigmoid(gate[row, head * DV + d]) (NULL: none)
@@ -58,28 +58,20 @@ __device__ __forceinline__ void fl_load(void* dst, const CUtensorMap* map, int x
                ::"r"(smem_u32(dst)), "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar)) : "memory");
 }
 
-// The key tiles of a unit: first the paged ones that its rows see, then the own ones.
+// The key tiles of a unit, aligned to absolute positions.
 struct FlTiles {
-  int lo, n_paged, n;                                    // first paged position (a multiple of 128), tiles
-  int last;                                              // last position that a row of the unit sees
+  int lo, n;                                             // first position of the first tile (a multiple of 128), tiles
   __device__ FlTiles(const FlashUnit& u, int window) {
     const int rows = min(128, u.pairs - u.pair0), a = u.pair0 % u.len, b = a + rows - 1;
     const int first_tok = b < u.len ? a : 0, last_tok = b < u.len ? b : u.len - 1;
-    const int seen = window > 0 ? max(0, u.pos0 + first_tok - window + 1) : 0;
-    last = u.pos0 + last_tok;
-    lo = min(seen, u.paged) / FL_KEYS * FL_KEYS;
-    const int end = min(u.paged, last + 1);
-    n_paged = end > lo ? (end - lo + FL_KEYS - 1) / FL_KEYS : 0;
-    own_lo = max(0, seen - u.key_pos0) / FL_KEYS * FL_KEYS;
-    n = n_paged + (last >= u.key_pos0 ? (last - u.key_pos0 - own_lo) / FL_KEYS + 1 : 0);
+    lo = (window > 0 ? max(0, u.pos0 + first_tok - window + 1) : 0) / FL_KEYS * FL_KEYS;
+    n = (u.pos0 + last_tok - lo) / FL_KEYS + 1;
   }
-  int own_lo;                                            // first own key of the first own tile
 };
 
 template <int DK, int DV, bool SPLIT>
 __global__ void __launch_bounds__(FL_THREADS, 1)
-flash_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap, const __grid_constant__ CUtensorMap pkmap,
-             const __grid_constant__ CUtensorMap pvmap, FlashArgs a) {
+flash_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap, FlashArgs a) {
   extern __shared__ __align__(16) unsigned char tp_smem[];
   unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(tp_smem) + 1023) & ~(uintptr_t)1023);
   constexpr int KC = DK / 64, VC = DV / 64, CHUNK = 16384;
@@ -113,26 +105,20 @@ flash_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ C
       for (int j = 0; j < tiles.n && ok; ++j) {
         const int s = j & 1;
         const uint32_t ph = ((j >> 1) & 1) ^ 1;
-        const bool paged = j < tiles.n_paged;
-        int row, xk, xv;
-        if (paged) {
-          const int p = tiles.lo + j * FL_KEYS;
-          row = (a.page_table[u.table + p / 256] * a.kv_heads + u.kvh) * 256 + p % 256;
-          xk = xv = 0;
-        } else {
-          row = u.own_row0 + tiles.own_lo + (j - tiles.n_paged) * FL_KEYS;
-          xk = u.kvh * DK; xv = u.kvh * DV;
-        }
+        const int p = tiles.lo + j * FL_KEYS;
+        const bool paged = u.table >= 0;
+        const int row = paged ? (a.page_table[u.table + p / 256] * a.kv_heads + u.kvh) * 256 + p % 256 : u.own_row0 + p;
+        const int xk = paged ? 0 : u.kvh * DK, xv = paged ? 0 : u.kvh * DV;
         ok = fl_wait(&sm->k_empty[s], ph, sm, a.err);
         if (!ok) break;
         mbar_expect_tx(&sm->k_full[s], KC * CHUNK);
 #pragma unroll
-        for (int c = 0; c < KC; ++c) fl_load(sk + (s * KC + c) * CHUNK, paged ? &pkmap : &kmap, xk + c * 64, row, &sm->k_full[s]);
+        for (int c = 0; c < KC; ++c) fl_load(sk + (s * KC + c) * CHUNK, &kmap, xk + c * 64, row, &sm->k_full[s]);
         ok = fl_wait(&sm->v_empty[s], ph, sm, a.err);
         if (!ok) break;
         mbar_expect_tx(&sm->v_full[s], VC * CHUNK);
 #pragma unroll
-        for (int c = 0; c < VC; ++c) fl_load(sv + (s * VC + c) * CHUNK, paged ? &pvmap : &vmap, xv + c * 64, row, &sm->v_full[s]);
+        for (int c = 0; c < VC; ++c) fl_load(sv + (s * VC + c) * CHUNK, &vmap, xv + c * 64, row, &sm->v_full[s]);
       }
       if (!ok) for (int i = 0; i < 1000; ++i) __nanosleep(1000);    // copies in flight land before the block leaves
     }
@@ -193,8 +179,7 @@ flash_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ C
     bool ok = true;
     for (int j = 0; j < tiles.n; ++j) {
       const int s = j & 1;
-      const bool paged = j < tiles.n_paged;
-      const int k0 = paged ? tiles.lo + j * FL_KEYS : u.key_pos0 + tiles.own_lo + (j - tiles.n_paged) * FL_KEYS;
+      const int k0 = tiles.lo + j * FL_KEYS;
       ok = fl_wait(&sm->s_full[s], (j >> 1) & 1, sm, a.err);
       if (!__all_sync(0xffffffffu, ok)) break;
       tc_fence_after();
@@ -205,7 +190,7 @@ flash_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ C
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&sm->s_free[s]);
-      const int end = min(paged ? min(u.paged, pos + 1) : pos + 1, k0 + FL_KEYS);      // keys [first, end) of this tile
+      const int end = min(pos + 1, k0 + FL_KEYS);               // keys [first, end) of this tile
       if (first > k0 || end < k0 + FL_KEYS) {
 #pragma unroll
         for (int k = 0; k < 128; ++k)
@@ -213,10 +198,10 @@ flash_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ C
       }
       float t0 = -INFINITY, t1 = -INFINITY, t2 = -INFINITY, t3 = -INFINITY;
 #pragma unroll
-      for (int k = 0; k < 128; k += 4) { 
+      for (int k = 0; k < 128; k += 4) {
         t0 = fmaxf(t0, __uint_as_float(x[k])); t1 = fmaxf(t1, __uint_as_float(x[k + 1]));
         t2 = fmaxf(t2, __uint_as_float(x[k + 2])); t3 = fmaxf(t3, __uint_as_float(x[k + 3]));
-       }
+      }
       const float top = fmaxf(fmaxf(t0, t1), fmaxf(t2, t3)) * c2;
       float grow = 1.0f;
       const bool moves = top > m + 8.0f || (m == -INFINITY && top > -INFINITY);

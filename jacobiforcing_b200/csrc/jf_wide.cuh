@@ -263,7 +263,7 @@ inline void wide_attention(WideStream& w, const DevCtx& c, int layer, const Flas
     }
   }
   const FlashArgs a{units, c.qbuf, (size_t)md.q_dim, D, c.block_tables, md.n_kv, rsqrtf((float)D), 0, nullptr, nullptr, 0, c.xa, 0, c.xrows_cap, err};
-  w.launch(flash_kernel<D, D, false>, n_units, FL_THREADS, fl_smem_bytes(D, D), paged[0], paged[1], paged[0], paged[1], a);
+  w.launch(flash_kernel<D, D, false>, n_units, FL_THREADS, fl_smem_bytes(D, D), paged[0], paged[1], a);
 }
 
 // Row units of a forward: 128 (head, token) pairs of one key head of one group each, most key tiles first.
@@ -272,7 +272,7 @@ inline std::vector<FlashUnit> wide_units(const ModelDims& md, const std::vector<
   for (const Group& g : groups)
     for (int kvh = 0; kvh < md.n_kv; ++kvh)
       for (int p = 0; p < md.n_rep * g.len; p += 128)
-        u.push_back(FlashUnit{g.row0, g.len, p, md.n_rep * g.len, kvh * md.n_rep, kvh, g.ctx, 0, g.ctx + g.len, g.ctx + g.len, g.seq * max_pages});
+        u.push_back(FlashUnit{g.row0, g.len, p, md.n_rep * g.len, kvh * md.n_rep, kvh, g.ctx, 0, g.seq * max_pages});
   auto last = [](const FlashUnit& x) {
     const int a = x.pair0 % x.len, b = a + std::min(128, x.pairs - x.pair0) - 1;
     return x.pos0 + std::min(b, x.len - 1);
