@@ -8,8 +8,8 @@
 // so a token costs one pass over the state, one exchange between lanes and one update.  With a decay per key channel the pass
 // first multiplies the state by it and g drops out of the two formulas: one more product per element, one less in the
 // update.  Value columns are independent of each
-// other, so a head is cut into blocks of 128 / PARTS columns that run side by side on different SMs, and PARTS lanes share a
-// column, each holding DR / PARTS of its key rows in registers.  With one warp per scheduler the recurrence runs at about a
+// other, so a head is cut into blocks of VC 128 / PARTS columns that run side by side on different SMs, and PARTS lanes share VC
+// columns, each holding DR / PARTS of its key rows in registers.  With one warp per scheduler the recurrence runs at about a
 // third of the issue rate whatever the layout, so its time is its instruction count: everything that does not depend on the
 // state (convolutions, unit vectors, k.q, decays, step sizes; rotations) is made beforehand, once per token and key head, by
 // kernels of their own that leave fp32 rows, and the recurrence copies those asynchronously.

@@ -1553,7 +1553,7 @@ int gemm(hy_engine* h, const TA* A, int lda, const TW* Wt, int ldw, int T, int N
     while (ksplit < 8 && (long long)N * ksplit < 148LL * 32 && K / (ksplit * 2) >= 512) ksplit *= 2;
     const int cpb = 8 / ksplit;
     // Eight rows are 16 KB of operand and more to stage before a block's first product, so a warp takes several columns: a batch of 8 requests
-    // on two layers of width 1024, 16 blocks per SM at most 14.65 ms, 4 14.1, 2 14.15, 1 (too few loads in flight) 16.6.  One row: no difference.
+    // on four layers of width 1024, 16 blocks per SM at most 14.65 ms, 4 14.1, 2 14.15, 1 (too few loads in flight) 16.6.  One row: no difference.
     const int blocks = std::min((N + cpb - 1) / cpb, 148 * (T > 4 ? 4 : 16));
     const int fit = (int)((200 * 1024) / row_bytes);
     auto launch = [&](auto kern, int rows) {

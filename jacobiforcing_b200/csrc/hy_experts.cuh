@@ -2,14 +2,14 @@
 //
 //   route     per token: sigmoid scores of the router logits, group-limited choice of `top` experts, normalised weights;
 //             per-expert pair counts by atomic add (the counts, not their order, decide the layout)
-//   offsets   exclusive prefix of the counts, the list of (expert, first row) tiles of the grouped products
-//   scatter   every (token, choice) pair gets a row in its expert's range of the sorted order
-//   products  gate/up with the gated activation in the epilogue, then down, both grouped by expert: a block looks up its
-//             tile, reads activation rows through the sorted order and the expert's weight matrix
+//   place     every (token, choice) pair gets a row in its expert's range of the sorted order, and the token's activation row is
+//             copied there; the exclusive prefix of the counts and the list of (expert, first row) tiles of the grouped products
+//   products  gate/up with the gated activation in the epilogue, then down, both grouped by expert: a tile of the list reads its
+//             rows of the sorted copy and its expert's weight matrix; a handful of pairs skip the order and take one block row each
 //   combine   per token the weighted sum of its pairs' rows in the order of its choices, then the sublayer's output norm,
 //             layer scale and the residual sum
-// A token's result does not depend on the batch: its choices, its weights and the order of its sum are its own, and a
-// row of a product does not depend on the other rows of its tile.  Router scores, weights and the combine are fp32.
+// A token's choices, its weights and the order of its sum are its own, and a row of a product does not depend on the other rows of its
+// tile; whether the few-pair kernel or the tiles make it depends on the number of pairs in the step.  Router scores, weights and the combine are fp32.
 #pragma once
 #include "hy_kernels.cuh"
 

@@ -3,9 +3,11 @@
 // Precision rule shared by every kernel here: the residual stream, norms, attention scores and weights, positions and
 // angles, recurrent states, decays, step sizes, gates of a recurrence and unit norms are fp32; projections, short
 // convolutions with their activations and the operands of the matrix products are AT (bf16 in the serving build, fp32 in
-// the all-fp32 build).  A step is a packed batch of entries (portions of prompts beside single decoded tokens); no
-// result depends on how a request was cut or on what else is in the batch: every reduction runs over absolute key
-// positions / a fixed k order.
+// the all-fp32 build).  A step is a packed batch of entries (portions of prompts beside single decoded tokens).  A request's
+// result depends on how it was cut and on what else is in the batch only by the rounding of its sums: the sizes of a step choose the kernel
+// of a product (up to eight rows, or tiles), into how many ranges of k the tiles of a small product are cut, how many key ranges
+// attention is split into and merged from, and the form of latent attention; within each of them the order of a sum is fixed (key
+// ranges at absolute positions, k in order).
 #pragma once
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>

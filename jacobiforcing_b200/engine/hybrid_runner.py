@@ -62,7 +62,7 @@ class HybridModelRunner:
         """portions: (request, n) = feed the request's next n tokens (those after `num_cached_tokens`).
         want: None = sample one token after every portion that ends the request's known tokens (generation), else for every
         portion the offsets inside it whose logits are returned (scoring).  Steps that exceed the runner's token capacity
-        are cut into sub-steps; nothing a request computes depends on the cut."""
+        are cut into sub-steps; a request's results depend on the cut only by the rounding of their sums."""
         assert portions
         if want is not None:
             logits = self._forward(portions, want, want_layers=want_layers)
