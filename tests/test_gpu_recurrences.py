@@ -5,9 +5,11 @@ chunks; fp32 build against the plain fp64 restatements, within the
 bound of the other fp32 tests (3e-4)."""
 import pytest
 
-from oracle import famepel_plain, kinetar_plain
+from oracle import famepel_plain, kinetar_plain, kisadra_plain, mafalorn_plain
 from tests import famepel_helpers as fam
 from tests import hybrid_helpers as kin
+from tests import kisadra_helpers as kis
+from tests import mafalorn_helpers as maf
 
 pytestmark = pytest.mark.gpu
 
@@ -95,6 +97,34 @@ def test_two_columns_per_lane(dim, vdim, heads):
         hz.close()
     assert kin.rel_err(got, fam.oracle_logits(cfg, w, toks)) < fam.TOL["bfloat16"]
     assert _kinetar(kin.delta(heads=heads, kv_heads=heads, dim=dim, vdim=vdim, ff=0), dtype="bfloat16") < kin.TOL["bfloat16"]
+
+
+TWO = [(64, 120, 16), (100, 113, 16), (128, 8, 120), (34, 232, 8), (128, 15, 119), (36, 17, 60), (40, 16, 119)]
+
+
+@pytest.mark.parametrize("dim,vdim,heads", TWO)
+@pytest.mark.parametrize("mode", ["state space", "gated linear", "retention", "head delta"])
+def test_two_columns_per_lane_in_the_other_modes(mode, dim, vdim, heads):
+    """Heads x blocks of 16 columns at 120 and above (two value columns per lane) and just below, with ragged last blocks and odd column counts: the modes
+    that have code of their own per column (step sizes and the skip of the state space, one decay per channel or per head, the delta rule's
+    correction), bf16 against the fp64 restatement."""
+    plain, helpers = (famepel_plain, fam) if mode == "state space" else (kisadra_plain, kis) if mode == "gated linear" else (mafalorn_plain, maf)
+    if mode == "state space":
+        cfg = fam.model_config([fam.ssd(heads=heads, vdim=vdim, state=dim, groups=1 if heads % 2 else 2, norm_groups=1, conv=4, mlp=None)])
+    elif mode == "gated linear":
+        cfg = kis.model_config([kis.gla(heads=heads, dim=dim, vdim=vdim, mlp=None)])
+    elif mode == "retention":
+        cfg = maf.model_config([maf.ret(heads=heads, dim=dim, vdim=vdim, decay=[1.0 - 2.0 ** (-2.0 - 5.0 * h / heads) for h in range(heads)], mlp=None)])
+    else:
+        cfg = maf.model_config([maf.par(d_heads=heads, d_kv_heads=heads if heads % 2 else heads // 2, d_dim=dim, d_vdim=vdim, conv=4, mlp=None)])
+    toks = kin.rand_tokens(sum(CUTS), cfg["vocab"], 4)
+    w = plain.random_weights(cfg, 0)
+    hz = helpers.Harness(cfg, w, "bfloat16")
+    try:
+        got = hz.feed("a", toks, CUTS)
+    finally:
+        hz.close()
+    assert helpers.close(got, helpers.oracle_logits(cfg, w, toks), "bfloat16")
 
 
 @pytest.mark.parametrize("width,ff,tokens", [(48, 1630, 321), (45, 33, 70), (64, 64, 64), (31, 7, 33), (36, 100, 9)])
