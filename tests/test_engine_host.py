@@ -123,7 +123,7 @@ def test_scheduler_respects_limits_and_preempts():
 
 
 def test_jacobi_requests_under_kv_memory_pressure_finish_without_crashing():
-    """ADVICE r1: 8 Jacobi requests with max_tokens=2048 on a 40-page cache.  The scheduler reserves one block's worth
+    """8 Jacobi requests with max_tokens=2048 on a 40-page cache.  The scheduler reserves one block's worth
     per admitted request and preempts the youngest when pages run out; the runner shortens a decode call whose whole
     remaining budget does not fit instead of raising 'out of KV cache blocks'."""
     from types import SimpleNamespace

@@ -48,7 +48,7 @@ def test_llm_from_checkpoint_dir_matches_hf_generate(ckpt):
 
 
 def test_missing_shard_is_an_error(ckpt, tmp_path):
-    """A checkpoint directory that lacks one safetensors shard must not load (ADVICE r1: per-layer presence check)."""
+    """A checkpoint directory that lacks one safetensors shard must not load (per-layer presence check)."""
     import shutil
     from jacobiforcing_b200 import LLM
     root, _, _ = ckpt

@@ -165,7 +165,7 @@ def test_batch8_multiblock_equals_oracle_policy_bit_exact():
 
 
 def test_finalize_rejects_partial_checkpoint():
-    """a checkpoint that lacks a layer tensor must not finalize (zero weights would decode garbage)."""
+    """A checkpoint that lacks a layer tensor must not finalize (zero weights would decode garbage)."""
     from jacobiforcing_b200.runtime import JacobiRuntime
     from oracle.hf_model import build_model, state_dict_bf16
     model = build_model("tiny", seed=0, dtype=torch.float32)

@@ -65,7 +65,7 @@ def _worker(rank, world, port, ret, shard_attn=False, skew=False):
         for rep, (mode, n) in enumerate((("single", 1), ("single", 8), ("multiblock", 8)) * (4 if skew else 1)):
             if skew and rank == rep % world:
                 import time
-                time.sleep(0.05 * (1 + rep % 3))       # host skew between the ranks' launches (ADVICE r1)
+                time.sleep(0.05 * (1 + rep % 3))       # host skew between the ranks' launches
             seqs, results, run = hf_generate(rt, [prompt], n=n, max_new_tokens=40, mode=mode, pad=0,
                                              rngs=[random.Random(2)])
             if (mode, n) in runs:

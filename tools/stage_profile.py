@@ -24,7 +24,7 @@ def main():
     ap.add_argument("--mode", default="single")
     ap.add_argument("--tp-attn", default="auto", choices=["auto", "shard", "replicate"])
     ap.add_argument("--attn-chunk", type=int, default=64)
-    ap.add_argument("--out", default=os.path.join(ROOT, "gpurun_out", "stage_profile.json"))
+    ap.add_argument("--out", default=os.path.join(ROOT, "build", "stage_profile.json"))
     a = ap.parse_args()
     import torch
     from jacobiforcing_b200.runtime import JacobiRuntime, hf_generate
