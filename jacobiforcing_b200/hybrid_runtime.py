@@ -26,7 +26,7 @@ def _packed(parts) -> Tuple[np.ndarray, List[int]]:
     generator and numpy 161 us, a tenth of a prompt step); whatever has no integer form of its own goes through int()."""
     out, start = array.array("i"), [0]
     for t in parts:
-        t = t.tolist() if isinstance(t, np.ndarray) else t if isinstance(t, (list, tuple)) else list(t)
+        t = t.tolist() if isinstance(t, np.ndarray) and t.ndim == 1 else t if isinstance(t, (list, tuple)) else list(t)
         try:
             out.extend(array.array("i", t))
         except TypeError:

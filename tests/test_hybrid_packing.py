@@ -27,3 +27,10 @@ def test_no_lists_and_empty_lists():
 def test_refusals(bad, err):
     with pytest.raises(err):
         _packed([[1], bad])
+
+
+@pytest.mark.filterwarnings("ignore::DeprecationWarning")
+def test_arrays_whose_rows_are_single_numbers():
+    for column in (np.array([[5], [6]]), np.array([[[7]]]), [np.array([4])]):
+        got, start = _packed([column, [1]])
+        assert got.tolist() == [int(x) for x in column] + [1] and start == [0, len(column), len(column) + 1]
