@@ -163,6 +163,7 @@ struct hy_engine {
   AttnUnit* units_d = nullptr; AttnUnit* units_h = nullptr; size_t units_cap = 0, units_used = 0;
   std::vector<UnitList> unit_lists;
   int step_tokens = 0;
+  bool plain = false;                            // launches of the running step do not overlap (see go_kernel)
   float* part_sums = nullptr; int* part_arrived = nullptr;      // partial sums of products with few tiles (jf::PairSplit)
   // prompt steps of latent attention: keys of a step's requests one after the other (cache rows, then per-head keys and values),
   // row units and the requests' first rows for the kernels
@@ -213,7 +214,7 @@ inline void go_kernel(hy_engine* h, void (*kernel)(P...), dim3 grid, dim3 block,
   at.val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t c = {};
   c.gridDim = grid; c.blockDim = block; c.dynamicSmemBytes = smem; c.stream = stream; c.attrs = &at;
-  c.numAttrs = h->step_tokens <= HY_OVERLAP_TOKENS ? 1 : 0;
+  c.numAttrs = h->step_tokens <= HY_OVERLAP_TOKENS && !h->plain ? 1 : 0;
   if (!h->step_err.empty()) return;
   cudaError_t e = opt_in(h, (const void*)kernel, smem);
   if (e == cudaSuccess) e = cudaLaunchKernelEx(&c, kernel, std::forward<A>(args)...);
@@ -1858,6 +1859,10 @@ void latent_mixer(hy_engine* h, const Batch& b, const LayerW& L, const hy_layer_
       gemm<AT, WT, AT>(h, cv, h->ld_cv, (const WT*)L.w_uq, c.l_q_rank, T, H * (dn + rot), c.l_q_rank, to_buf(pin, h->ld_pin), L.w_uq_t);
   }
   if constexpr (std::is_same<AT, bf16>::value) { if (latent_prompt(h, b, L, c)) return; }
+  // The folded form beyond eight tokens launches plainly: its attention has few blocks with most of an SM's shared memory each, and with the kernels
+  // around it starting early they piled up on some SMs.  16 heads over a rank of 512, us a step, overlapped -> plain: 9 tokens 244 -> 193,
+  // 33 behind 500 280 -> 214, 63 290 -> 217; one token 121 -> 129, eight the same.
+  h->plain = T > 8;
   {
     ProfScope ps(h, HY_PROF_SMALL_GEMM);
     const int fold = T > 8 ? 1 : 0;
@@ -1924,6 +1929,7 @@ void latent_mixer(hy_engine* h, const Batch& b, const LayerW& L, const hy_layer_
         T, h->f2, h->ld_f2, (const WT*)L.w_uvT, H, R, dv, gate, h->ld_pin, cat, h->ld_cat);
     h->launches++;
   }
+  h->plain = false;
 }
 
 // Routing tables of a layer: the counters that its route kernel fills (the two sets alternate, see route_place_kernel), rows per

@@ -54,3 +54,7 @@ class Fake:
     def launches(self):
         """(kernel, device) of every launch that went through since the last reset."""
         return [(self.lib.fake_launch_name(i).decode(), self.lib.fake_launch_device(i)) for i in range(self.lib.fake_launches())]
+
+    def overlaps(self):
+        """Whether each launch may start under the one before it."""
+        return [bool(self.lib.fake_launch_overlaps(i)) for i in range(self.lib.fake_launches())]

@@ -106,3 +106,17 @@ def test_refused_shared_memory_is_reported(fake):
     step(rt, 150)                                            # asked for again
     assert len(fake.launches()) > 2 * len(went)
     rt.close()
+
+
+@pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
+@pytest.mark.parametrize("tokens", [1, 8, 9, 63, 64, 65])
+def test_which_launches_overlap(fake, tokens, dtype):
+    """Steps of up to 64 tokens, but beyond eight not the folded form of latent attention."""
+    rt = engine(fam.model_config([fam.latent(mlp=None), fam.glr(mlp=None)]), dtype)
+    fake.reset()
+    step(rt, tokens)
+    folded = ("latent_query", "attn_", "head_rows", "latent_value")
+    for (name, _), overlaps in zip(fake.launches(), fake.overlaps()):
+        assert overlaps == (tokens <= 64 and not (tokens > 8 and any(f in name for f in folded))), name
+    assert sum(any(f in n for f in folded) for n, _ in fake.launches()) >= 3
+    rt.close()
