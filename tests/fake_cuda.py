@@ -26,7 +26,7 @@ def build(engine: str) -> str:
         pytest.skip("needs nvcc")
     os.makedirs(os.path.dirname(out), exist_ok=True)
     tmp = "%s.%d.tmp" % (out, os.getpid())
-    subprocess.check_call([nvcc, "-gencode", "arch=compute_100a,code=compute_100a", "-Xcicc", "-O0", "-std=c++17", "-Xcompiler", "-fPIC,-O1", "-w",
+    subprocess.check_call([nvcc, "-gencode", "arch=compute_100a,code=compute_100a", "-Xcicc", "-O0", "-std=c++17", "-Xcompiler", "-fPIC,-O1,-fno-gnu-unique", "-w",
                            "-I", os.path.join(ROOT, "include"), "-I", CSRC, "-shared", "-cudart", "none", "-Xlinker", "-Bsymbolic",
                            os.path.join(CSRC, engine + "_engine.cu"), FAKE, "-o", tmp])
     os.replace(tmp, out)
@@ -58,3 +58,7 @@ class Fake:
     def overlaps(self):
         """Whether each launch may start under the one before it."""
         return [bool(self.lib.fake_launch_overlaps(i)) for i in range(self.lib.fake_launches())]
+
+    def blocks(self, kernel):
+        """Blocks along x of every launch of the kernels whose name holds this."""
+        return [self.lib.fake_launch_blocks(i) for i in range(self.lib.fake_launches()) if kernel in self.lib.fake_launch_name(i).decode()]
