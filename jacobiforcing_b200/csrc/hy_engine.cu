@@ -605,10 +605,12 @@ int load_gated_experts(hy_engine* h, Builder& B, LayerW& L, const hy_layer_cfg& 
   return B.rc;
 }
 
-// Whether prompt steps of a latent-attention layer may run over per-head keys and values (head sizes that jf::flash_kernel is built for).
+// Whether prompt steps of a latent-attention layer may run over per-head keys and values: head sizes that jf::flash_kernel is built for, and a positive
+// scale (it looks for the largest score before it scales them, and marks what a row does not see by minus infinity there).
 bool latent_prompt_sizes(const hy_engine* h, const hy_layer_cfg& c) {
   const int hk = c.l_dim + c.l_rot_dim;
-  return h->m.dtype == HY_DTYPE_BF16 && (hk == 64 || hk == 128 || hk == 192) && (c.l_vdim == 64 || c.l_vdim == 128) && (c.l_kv_rank + c.l_rot_dim) % 8 == 0;
+  return h->m.dtype == HY_DTYPE_BF16 && c.l_scale > 0.0f && (hk == 64 || hk == 128 || hk == 192) && (c.l_vdim == 64 || c.l_vdim == 128) &&
+         (c.l_kv_rank + c.l_rot_dim) % 8 == 0;
 }
 
 // What follows the down-projections of a latent-attention layer: the key and value up-projections in the layouts of their

@@ -54,3 +54,16 @@ def test_latent_prompts_of_several_requests():
     for got, r, lo, hi in [(one[:170], "a", 0, 170), (one[170:171], "b", 0, 1), (one[171:], "c", 0, 100), (two[:140], "b", 1, 141), (two[140:270], "a", 170, 300),
                            (two[270:], "c", 100, 190)]:
         assert kin.rel_err(got, want[r][lo:hi]) < fam.TOL["bfloat16"]
+
+
+@pytest.mark.parametrize("scale", [-0.1, 0.0, -2.0])
+def test_scales_that_are_not_positive(scale):
+    cfg = maf.model_config([maf.lat(heads=2, dim=64, rot_dim=64, vdim=64, rank=24, size=None, scale=scale, mlp=None)], width=64)
+    w = mafalorn_plain.random_weights(cfg, 3)
+    toks = kin.rand_tokens(300, cfg["vocab"], 12)
+    hz = maf.Harness(cfg, w, "bfloat16", num_pages=40)
+    try:
+        got = hz.feed("a", toks, [170, 130])
+    finally:
+        hz.close()
+    assert kin.rel_err(got, maf.oracle_logits(cfg, w, toks)) < maf.TOL["bfloat16"]

@@ -120,3 +120,13 @@ def test_which_launches_overlap(fake, tokens, dtype):
         assert overlaps == (tokens <= 64 and not (tokens > 8 and any(f in name for f in folded))), name
     assert sum(any(f in n for f in folded) for n, _ in fake.launches()) >= 3
     rt.close()
+
+
+@pytest.mark.parametrize("scale,flash", [(0.4, True), (0.0, False), (-0.4, False)])
+def test_flash_takes_positive_scales_only(fake, scale, flash):
+    """It looks for the largest score before it scales them."""
+    rt = engine(maf.model_config([maf.lat(heads=2, dim=64, rot_dim=64, vdim=64, rank=24, size=None, scale=scale, mlp=None)]))
+    fake.reset()
+    step(rt, 150)
+    assert any("flash_kernel" in n for n, _ in fake.launches()) == flash
+    rt.close()
