@@ -1555,8 +1555,9 @@ int gemm(hy_engine* h, const TA* A, int lda, const TW* Wt, int ldw, int T, int N
     int ksplit = 1;
     while (ksplit < 8 && (long long)N * ksplit < 148LL * 32 && K / (ksplit * 2) >= 512) ksplit *= 2;
     const int cpb = 8 / ksplit;
-    // Eight rows are 16 KB of operand and more to stage before a block's first product, so a warp takes several columns: a batch of 8 requests
-    // on four layers of width 1024, 16 blocks per SM at most 14.65 ms, 4 14.1, 2 14.15, 1 (too few loads in flight) 16.6.  One row: no difference.
+    // Eight rows are 16 KB of operand and more to stage before a block's first product, so a warp takes several columns: at most 4 blocks per SM
+    // against 16, us behind a small kernel: N 2112, K 2048 16.9 and 19.5; N 1024, K 4096 26.1 and 31.6; N 32000, K 1024 56.7 and 55.6.  One row:
+    // no difference beyond 0.6 us but for N 32000 (20.2 and 18.5).
     const int blocks = std::min((N + cpb - 1) / cpb, 148 * (T > 4 ? 4 : 16));
     const int fit = (int)((200 * 1024) / row_bytes);
     auto launch = [&](auto kern, int rows) {

@@ -365,13 +365,15 @@ __global__ void __launch_bounds__(256) gemm_rows_kernel(const TA* __restrict__ A
   const int cpb = 8 / ksplit, part = warp % ksplit, cib = warp / ksplit;
   const int Kc = ((K + ksplit - 1) / ksplit + 32 * VEC - 1) / (32 * VEC) * (32 * VEC);
   const int lo = part * Kc, hi = min(K, lo + Kc), kv = min(hi, K / VEC * VEC);
-  // the first AHEAD vectors of a column travel while the columns before it are summed up; those of the warp's first column while the
-  // kernel before this one ends (weights do not depend on it)
-  constexpr int AHEAD = 4;
-  VecN<TW, VEC> w0[AHEAD];
+  // Up to four rows: the first AHEAD vectors of a column travel while the columns before it are summed up; those of the warp's first column
+  // while the kernel before this one ends (weights do not depend on it).  What they hold in registers is paid for in blocks per SM: behind a small
+  // kernel, N 2112, K 2048, us: one row 10.3 without overlapping launches, 8.2 with four vectors ahead (80 registers), 6.5 with two (48); eight rows
+  // 22.5, 24.9 with four (128 registers, two blocks per SM), 25.0 with two, 16.9 with none (62).
+  constexpr int AHEAD = ROWS <= 4 ? 2 : 0;
+  VecN<TW, VEC> w0[AHEAD ? AHEAD : 1];
   auto fetch = [&](int n) {
     const TW* wr = W + (size_t)n * ldw;
-    if (n < N && (reinterpret_cast<uintptr_t>(wr) & 15) == 0) {
+    if (AHEAD && n < N && (reinterpret_cast<uintptr_t>(wr) & 15) == 0) {
 #pragma unroll
       for (int i = 0; i < AHEAD; ++i) {
         const int k = lo + (lane + 32 * i) * VEC;
