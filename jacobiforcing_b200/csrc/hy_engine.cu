@@ -169,7 +169,7 @@ struct hy_engine {
   // row units and the requests' first rows for the kernels
   void* kv_rows = nullptr; void* kv_heads = nullptr; int kv_cap = 0;
   unsigned char* fl_h = nullptr; unsigned char* fl_d = nullptr; size_t fl_cap = 0, fl_used = 0;
-  struct FlashList { int H; const jf::FlashUnit* units; const int* key_off; int n, keys; };
+  struct FlashList { int H, window; const jf::FlashUnit* units; const int* keys_of; int n, keys; };
   std::vector<FlashList> fl_lists;
   // cosines and sines of the step's positions, one table per distinct rotation: the layer configuration that names it, the table,
   // its column count; rot_tables_d is what the kernel reads
@@ -1448,18 +1448,18 @@ extern "C" int hy_finalize(hy_handle h) {
     }
   }
   {
-    int lists = 0;
+    std::set<std::pair<int, int>> lists;                      // (heads, window): the unit lists one step may hold
     size_t row = 0, heads = 0, maxH = 0;
     for (auto& c : h->lc)
       if (c.mixer == HY_MIX_LATENT && latent_prompt_sizes(h, c)) {
-        ++lists;
+        lists.insert({c.l_heads, c.l_window});
         row = std::max(row, (size_t)(c.l_kv_rank + c.l_rot_dim));
         heads = std::max(heads, (size_t)c.l_heads * (c.l_dim + c.l_rot_dim + c.l_vdim));
         maxH = std::max(maxH, (size_t)c.l_heads);
       }
-    if (lists) {
+    if (!lists.empty()) {
       h->kv_cap = 4 * rt.max_step_tokens;
-      h->fl_cap = (size_t)lists * ((T / 128 + rt.max_step_entries) * maxH * sizeof(jf::FlashUnit) + ((size_t)rt.max_step_entries + 1) * 4 + 64);
+      h->fl_cap = lists.size() * ((T / 128 + rt.max_step_entries) * maxH * sizeof(jf::FlashUnit) + (2 * (size_t)rt.max_step_entries + 1) * 4 + 80);
       if (dev_alloc(h, &h->kv_rows, (size_t)h->kv_cap * row * 2, &h->bytes_ws)) return HY_ERR_CUDA;
       if (dev_alloc(h, &h->kv_heads, (size_t)h->kv_cap * heads * 2, &h->bytes_ws)) return HY_ERR_CUDA;
       if (dev_alloc(h, (void**)&h->fl_d, h->fl_cap, &h->bytes_ws)) return HY_ERR_CUDA;
@@ -1747,6 +1747,49 @@ LinearLaunch linear_launch(int parts, int vc, int dk, int dv, const AT* v, int l
                       dv % ch == 0 && cpb % ch == 0 && ldv % ch == 0 && (reinterpret_cast<uintptr_t>(v) & 15) == 0 ? 1 : 0};
 }
 
+// Whether the running step's latent attention with this window runs over per-head keys and values (latent_prompt), and then: its row units with H
+// heads (one head's 128 tokens each, late tokens first), where each request's keys begin in the gathered rows, and the position of the
+// first of them (keys_of: offsets [E + 1], then positions [E]).  NULL: the folded form.
+// Keys that no row sees (behind the window) are neither gathered nor projected: 64 to 128 tokens behind 6000 cached ones with a window of 128 took
+// 239 to 263 us with them, the folded form 220 to 244.  The projection is made for every key of the step and pays from about 64 tokens a
+// request on (64 tokens behind 0, 2048 and 8000: 158, 222 and 408 us, folded 261, 314 and 523), so keys of requests with fewer tokens are
+// made in vain, and steps with more than 32 of those per token keep the folded form: 127 prompt tokens beside a decoded one behind 4000: 313 us,
+// folded 328; behind 7000: 389 against 342.  So do steps whose keys exceed the gathered rows.
+constexpr int HY_FLASH_TOKENS = 64, HY_FLASH_VAIN = 32;
+const hy_engine::FlashList* flash_units(hy_engine* h, int E, int T, int H, int window) {
+  for (const auto& l : h->fl_lists) if (l.H == H && l.window == window) return &l;
+  if (T < HY_FLASH_TOKENS * E) return nullptr;
+  auto first_key = [&](int e) { return first_seen(h->step_pos0[e], window) / jf::FL_KEYS * jf::FL_KEYS; };
+  long long keys = 0, vain = 0;
+  for (int e = 0; e < E; ++e) {
+    const int len = h->step_start[e + 1] - h->step_start[e], n = h->step_pos0[e] + len - first_key(e);
+    keys += n;
+    if (len < HY_FLASH_TOKENS) vain += n;
+  }
+  if (keys > h->kv_cap || vain > (long long)HY_FLASH_VAIN * T) return nullptr;
+  unsigned char* at = h->fl_h + h->fl_used;
+  int* off = reinterpret_cast<int*>(at);
+  int* first = off + E + 1;
+  jf::FlashUnit* u = reinterpret_cast<jf::FlashUnit*>(at + ((2 * (size_t)E + 1) * 4 + 15) / 16 * 16);
+  int n = 0;
+  off[0] = 0;
+  for (int e = 0; e < E; ++e) {
+    first[e] = first_key(e);
+    off[e + 1] = off[e] + h->step_pos0[e] + h->step_start[e + 1] - h->step_start[e] - first[e];
+  }
+  for (int e = 0; e < E; ++e) {
+    const int len = h->step_start[e + 1] - h->step_start[e];
+    for (int p = (len - 1) / 128 * 128; p >= 0; p -= 128)
+      for (int hd = 0; hd < H; ++hd) u[n++] = jf::FlashUnit{h->step_start[e], len, p, len, hd, hd, h->step_pos0[e], off[e] - first[e], -1};
+  }
+  const size_t bytes = (unsigned char*)(u + n) - at;
+  unsigned char* d = h->fl_d + h->fl_used;
+  cudaMemcpyAsync(d, at, bytes, cudaMemcpyHostToDevice, h->stream);
+  h->fl_lists.push_back({H, window, reinterpret_cast<const jf::FlashUnit*>(d + ((unsigned char*)u - at)), reinterpret_cast<const int*>(d), n, (int)keys});
+  h->fl_used += (bytes + 63) / 64 * 64;
+  return &h->fl_lists.back();
+}
+
 // All unit lists that the layers of a step will ask for, before its first kernel: a copy between two kernels would keep the second from
 // starting under the first.
 template <typename AT>
@@ -1757,6 +1800,7 @@ void prepare_units(hy_engine* h, int E, int T) {
       if (c.a_dim == 32 || c.a_dim == 64 || c.a_dim == 128) attn_units(h, E, T, c.a_heads, c.a_kv_heads);
     } else if (c.mixer == HY_MIX_LATENT) {
       const int Dk = c.l_kv_rank + c.l_rot_dim;
+      if (latent_prompt_sizes(h, c) && flash_units(h, E, T, c.l_heads, c.l_window)) continue;
       const bool narrow = (Dk == 32 || Dk == 64 || Dk == 128) && attn_units(h, E, T, c.l_heads, 1, false, c.l_window);
       if (!narrow && Dk % 8 == 0 && c.l_kv_rank <= 512) attn_units(h, E, T, c.l_heads, 1, true, c.l_window);
     } else if (c.mixer == HY_MIX_WINDOW) {
@@ -1770,49 +1814,24 @@ void prepare_units(hy_engine* h, int E, int T) {
   }
 }
 
-// Row units of a prompt step's latent attention with H heads (one head's 128 tokens each, late tokens first) and where each request's
-// keys begin in the gathered rows; NULL: the step's contexts do not fit the gathered rows.
-const hy_engine::FlashList* flash_units(hy_engine* h, int E, int H) {
-  for (const auto& l : h->fl_lists) if (l.H == H) return &l;
-  long long keys = 0;
-  for (int e = 0; e < E; ++e) keys += h->step_pos0[e] + h->step_start[e + 1] - h->step_start[e];
-  if (keys > h->kv_cap) return nullptr;
-  unsigned char* at = h->fl_h + h->fl_used;
-  int* off = reinterpret_cast<int*>(at);
-  jf::FlashUnit* u = reinterpret_cast<jf::FlashUnit*>(at + (((size_t)E + 1) * 4 + 15) / 16 * 16);
-  int n = 0;
-  off[0] = 0;
-  for (int e = 0; e < E; ++e) off[e + 1] = off[e] + h->step_pos0[e] + h->step_start[e + 1] - h->step_start[e];
-  for (int e = 0; e < E; ++e) {
-    const int len = h->step_start[e + 1] - h->step_start[e];
-    for (int p = (len - 1) / 128 * 128; p >= 0; p -= 128)
-      for (int hd = 0; hd < H; ++hd) u[n++] = jf::FlashUnit{h->step_start[e], len, p, len, hd, hd, h->step_pos0[e], off[e], -1};
-  }
-  const size_t bytes = (unsigned char*)(u + n) - at;
-  unsigned char* d = h->fl_d + h->fl_used;
-  cudaMemcpyAsync(d, at, bytes, cudaMemcpyHostToDevice, h->stream);
-  h->fl_lists.push_back({H, reinterpret_cast<const jf::FlashUnit*>(d + ((unsigned char*)u - at)), reinterpret_cast<const int*>(d), n, (int)keys});
-  h->fl_used += (bytes + 63) / 64 * 64;
-  return &h->fl_lists.back();
-}
-
-// Latent attention of a prompt step over per-head keys and values: one product of all cache rows that the step's requests hold gives
+// Latent attention of a prompt step over per-head keys and values: one product of the cache rows that the step's requests see gives
 // them (each head's key: its part of the up-projection, then the rotated part as it is), and attention runs over heads of dim + rot
 // and vdim instead of rank + rot and rank.  1531 tokens behind 2048, 16 heads of 128 + 64 over a rank of 512: the folded form does
 // 3.4 times the score and value products (1150 us on mma.sync) and folds queries and values itself (223 + 237 us); this form
-// 220 us in all (160 of them attention).  Worth it from about 64 tokens per request (the product is made for the whole context every step); steps
-// whose contexts exceed the gathered rows keep the folded form.  Queries in h->pin (rotated here), results in h->cat.
+// 220 us in all (160 of them attention).  Queries in h->pin (rotated here), results in h->cat.  Keys and values of a head are rounded to bf16
+// (the folded form rounds the folded query instead, and holds the weighted sum of latents in fp32 up to the value up-projection: one
+// rounding fewer for the values); the weights keep a bf16 remainder in both.
 bool latent_prompt(hy_engine* h, const Batch& b, const LayerW& L, const hy_layer_cfg& c) {
-  if (!L.w_kv_t || b.T < 64 * b.E) return false;
+  if (!L.w_kv_t) return false;
   const int H = c.l_heads, hk = c.l_dim + c.l_rot_dim, dv = c.l_vdim, K = c.l_kv_rank + c.l_rot_dim, N = H * (hk + dv);
-  const hy_engine::FlashList* l = flash_units(h, b.E, H);
+  const hy_engine::FlashList* l = flash_units(h, b.E, b.T, H, c.l_window);
   if (!l) return false;
   cudaStream_t s = h->stream;
   bf16* pin = (bf16*)h->pin; bf16* kv = (bf16*)h->kv_heads;
   {
     ProfScope ps(h, HY_PROF_SMALL_GEMM);
     go_kernel(h, latent_rotate_kernel<bf16>, b.T, 128, (size_t)(2 * L.rot.pairs + 2) * 4, s, b, pin, h->ld_pin, H, c.l_dim, c.l_rot_dim, L.rot);
-    go_kernel(h, latent_gather_kernel, l->keys, 128, 0, s, b, l->key_off, (const bf16*)L.cache, K, (bf16*)h->kv_rows);
+    go_kernel(h, latent_gather_kernel, l->keys, 128, 0, s, b, l->keys_of, (const bf16*)L.cache, K, (bf16*)h->kv_rows);
     h->launches += 2;
     pair_product<bf16>(h, (const bf16*)h->kv_rows, K, l->keys, L.w_kv_t, 1, 0, l->keys, N, K, to_buf(kv, N), 0, jf::TpGroup{});
   }

@@ -167,13 +167,14 @@ __global__ void __launch_bounds__(128) latent_rotate_kernel(Batch b, AT* __restr
   }
 }
 
-// All cache rows of a step's requests, one after the other: out [sum of contexts, dim], entry e's from key_off[e] on.  One block per row.
-__global__ void __launch_bounds__(128) latent_gather_kernel(Batch b, const int* __restrict__ key_off, const bf16* __restrict__ cache, int dim,
+// The cache rows that a step's requests see, one after the other: out [keys, dim]; keys_of [E + 1] where each request's rows begin, then [E] the
+// position of its first.  One block per row.
+__global__ void __launch_bounds__(128) latent_gather_kernel(Batch b, const int* __restrict__ keys_of, const bf16* __restrict__ cache, int dim,
                                                             bf16* __restrict__ out) {
   pdl_begin();
   int e = 0;
-  while ((int)blockIdx.x >= key_off[e + 1]) ++e;
-  const int j = blockIdx.x - key_off[e];
+  while ((int)blockIdx.x >= keys_of[e + 1]) ++e;
+  const int j = blockIdx.x - keys_of[e] + keys_of[b.E + 1 + e];
   const bf16* src = cache + ((size_t)b.pages[(size_t)e * b.max_pages + j / b.page_size] * b.page_size + j % b.page_size) * dim;
   for (int k = threadIdx.x; k < dim / 8; k += blockDim.x)
     reinterpret_cast<uint4*>(out + (size_t)blockIdx.x * dim)[k] = reinterpret_cast<const uint4*>(src)[k];

@@ -15,7 +15,7 @@ int g_device = 0;
 cudaError_t g_last = cudaSuccess;
 // host stub -> mangled kernel name; made by the first registration, which may come before this file's own objects exist
 std::map<const void*, std::string>& names() { static std::map<const void*, std::string> m; return m; }
-struct Launch { const void* f; int device; int overlaps; };
+struct Launch { const void* f; int device, overlaps; unsigned blocks; };
 std::vector<Launch> g_launches;
 std::map<std::pair<int, const void*>, int> g_smem;              // (device, kernel) -> opted in dynamic shared memory
 long g_count[3] = {0, 0, 0}, g_fail[3] = {-1, -1, -1};          // launches, attributes, tensor maps: how many so far, which one fails
@@ -23,14 +23,14 @@ constexpr size_t kDefaultSmem = 48 * 1024, kMostSmem = 227 * 1024;
 
 bool fails(int what) { return g_count[what]++ == g_fail[what]; }
 cudaError_t last(cudaError_t e) { if (e != cudaSuccess) g_last = e; return e; }
-cudaError_t launch(const void* f, size_t smem, const cudaLaunchConfig_t* c = nullptr) {
+cudaError_t launch(const void* f, dim3 grid, size_t smem, const cudaLaunchConfig_t* c = nullptr) {
   if (fails(0)) return last(cudaErrorLaunchFailure);
   const auto it = g_smem.find({g_device, f});
   if (smem > (it == g_smem.end() ? kDefaultSmem : (size_t)it->second)) return last(cudaErrorInvalidValue);
   int overlaps = 0;
   for (unsigned i = 0; c && i < c->numAttrs; ++i)
     if (c->attrs[i].id == cudaLaunchAttributeProgrammaticStreamSerialization) overlaps = c->attrs[i].val.programmaticStreamSerializationAllowed;
-  g_launches.push_back({f, g_device, overlaps});
+  g_launches.push_back({f, g_device, overlaps, grid.x});
   return cudaSuccess;
 }
 CUresult encode(CUtensorMap* m, CUtensorMapDataType, cuuint32_t, void* p, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
@@ -50,6 +50,7 @@ long fake_count(int what) { return g_count[what]; }
 int fake_launches() { return (int)g_launches.size(); }
 const char* fake_launch_name(int i) { return names()[g_launches[i].f].c_str(); }
 int fake_launch_device(int i) { return g_launches[i].device; }
+int fake_launch_blocks(int i) { return (int)g_launches[i].blocks; }
 int fake_launch_overlaps(int i) { return g_launches[i].overlaps; }
 
 // ---- registration -------------------------------------------------------------------------------------------------------------------
@@ -105,9 +106,9 @@ cudaError_t cudaFuncSetAttribute(const void* f, cudaFuncAttribute a, int v) {
   }
   return cudaSuccess;
 }
-cudaError_t cudaLaunchKernel(const void* f, dim3, dim3, void**, size_t smem, cudaStream_t) { return launch(f, smem); }
-cudaError_t cudaLaunchCooperativeKernel(const void* f, dim3, dim3, void**, size_t smem, cudaStream_t) { return launch(f, smem); }
-cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void**) { return launch(f, c->dynamicSmemBytes, c); }
+cudaError_t cudaLaunchKernel(const void* f, dim3 grid, dim3, void**, size_t smem, cudaStream_t) { return launch(f, grid, smem); }
+cudaError_t cudaLaunchCooperativeKernel(const void* f, dim3 grid, dim3, void**, size_t smem, cudaStream_t) { return launch(f, grid, smem); }
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void**) { return launch(f, c->gridDim, c->dynamicSmemBytes, c); }
 cudaError_t cudaGetDriverEntryPoint(const char*, void** p, unsigned long long, cudaDriverEntryPointQueryResult* r) {
   *p = (void*)encode;
   *r = cudaDriverEntryPointSuccess;

@@ -67,3 +67,24 @@ def test_scales_that_are_not_positive(scale):
     finally:
         hz.close()
     assert kin.rel_err(got, maf.oracle_logits(cfg, w, toks)) < maf.TOL["bfloat16"]
+
+
+@pytest.mark.parametrize("size", [1, 40, 129, 256])
+def test_windows_far_behind_the_first_token(size):
+    """Only the keys that a row sees are gathered: portions that begin tiles behind their request's first token, of several requests."""
+    cfg = maf.model_config([maf.lat(heads=2, dim=64, rot_dim=64, vdim=64, rank=24, size=size, scale=0.1, mlp=None)], width=64)
+    w = mafalorn_plain.random_weights(cfg, 2)
+    toks = {r: kin.rand_tokens(n, cfg["vocab"], 40 + i) for i, (r, n) in enumerate([("a", 700), ("b", 420), ("c", 300)])}
+    want = {r: maf.oracle_logits(cfg, w, t) for r, t in toks.items()}
+    hz = maf.Harness(cfg, w, "bfloat16", num_pages=120, slots=4)
+    at = dict.fromkeys(toks, 0)
+    try:
+        for take in ({"a": 500, "b": 127}, {"b": 129, "a": 70, "c": 257}, {"c": 3, "a": 130, "b": 164}, {"c": 40}):
+            got, lo = hz.step([(r, toks[r][at[r]:at[r] + n], range(n)) for r, n in take.items()]), 0
+            for r, n in take.items():
+                assert kin.rel_err(got[lo:lo + n], want[r][at[r]:at[r] + n]) < maf.TOL["bfloat16"], (r, at[r])
+                lo += n
+                at[r] += n
+        assert at == {r: len(t) for r, t in toks.items()}
+    finally:
+        hz.close()

@@ -1,5 +1,6 @@
 """Host side of the hybrid decoders' steps on a CUDA runtime without a GPU: a step stops at the first call that fails, whichever it is,
-says so, and leaves the engine able to run the next; kernels are set up on every device that an engine is made on."""
+says so, and leaves the engine able to run the next; kernels are set up on every device that an engine is made on; the form that latent
+attention takes."""
 import pytest
 
 from tests import fake_cuda
@@ -119,6 +120,35 @@ def test_which_launches_overlap(fake, tokens, dtype):
     for (name, _), overlaps in zip(fake.launches(), fake.overlaps()):
         assert overlaps == (tokens <= 64 and not (tokens > 8 and any(f in name for f in folded))), name
     assert sum(any(f in n for f in folded) for n, _ in fake.launches()) >= 3
+
+
+def latent_engine(window):
+    from jacobiforcing_b200.hybrid_config import HybridConfig
+    from jacobiforcing_b200.hybrid_runtime import HybridRuntime
+    cfg = maf.model_config([maf.lat(heads=2, dim=64, rot_dim=64, vdim=64, rank=24, size=window, mlp=None)])
+    w = weights(cfg)
+    rt = HybridRuntime(HybridConfig.from_dict(cfg, {k: tuple(t.shape) for k, t in w.items()}), dtype="bfloat16", max_step_tokens=2048, max_step_entries=8,
+                       page_size=64, num_pages=8 * 160, max_pages_per_seq=160, num_slots=8, max_want=16)
+    rt.load_state_dict(w)
+    return rt
+
+
+@pytest.mark.parametrize("window,entries,keys", [
+    # (tokens, cached tokens) of each request -> keys that are projected (None: the folded form)
+    (None, [(64, 0)], 64), (None, [(63, 0)], None), (None, [(64, 8000)], 8064), (None, [(1024, 7168)], 8192), (None, [(1024, 7169)], None),
+    (None, [(1, 4000), (127, 0)], 4128), (None, [(1, 7000), (127, 0)], None), (None, [(127, 0), (1, 4095)], 4223), (None, [(127, 0), (1, 4096)], None),
+    (None, [(1, 1000)] * 7 + [(512, 0)], 7519), (None, [(40, 0), (600, 10), (3, 700)], 40 + 610 + 703),
+    # of a request's keys only the tiles that a row sees through the window
+    (128, [(64, 6000)], 6064 - 5760), (128, [(64, 127)], 191), (128, [(64, 254)], 318), (128, [(64, 255)], 319 - 128), (1, [(100, 300)], 400 - 256), (1024, [(64, 6000)], 6064 - 4864),
+    (128, [(1, 7000), (127, 0)], 7001 - 6784 + 127), (128, [(2000, 8000)], 10000 - 7808), (50, [(70, 500), (1, 130), (300, 0)], 570 - 384 + 131 + 300)])
+def test_form_of_latent_attention(fake, window, entries, keys):
+    rt = latent_engine(window)
+    fake.reset()
+    rt.step([([1] * n, ctx, e, list(range(160 * e, 160 * e + 160))) for e, (n, ctx) in enumerate(entries)], [0])
+    assert fake.blocks("latent_gather_kernel") == ([] if keys is None else [keys])
+    tiles = sum(-(-n // 128) for n, _ in entries)
+    assert fake.blocks("flash_kernel") == ([] if keys is None else [2 * tiles])
+    assert bool(fake.blocks("attn_mma") + fake.blocks("attn_wide")) == (keys is None)
     rt.close()
 
 
