@@ -294,7 +294,7 @@ class JacobiRuntime:
             raise ValueError("empty prompt")
         if seq.ctx < 0 or seq.ctx > P:
             raise ValueError("cached prefix longer than the prompt")
-        row = prompt + draft
+        row = _i32(prompt + draft)
         total = len(row)
         self.ensure_capacity(seq, total)
         want_from = P - 1                      # first row whose argmax is needed
@@ -314,11 +314,12 @@ class JacobiRuntime:
                 end = start + min(pages_end - start, self.max_rows // PAGE * PAGE)
             toks = row[start:end]
             T = end - start
-            commits, late = [(i, 0, start + i) for i in range(T) if start + i < P], []
+            own = np.arange(max(0, min(T, P - start)), dtype=np.int32)
+            commits, late = np.stack([own, np.zeros_like(own), own + start], axis=1), ()
             # Without a draft the rest may be a whole page of committed rows.  A full hit forwards the last prompt token on the persistent
             # kernel; the call of its own that commits the last row keeps a miss there too
             if end == total and len(commits) == T >= PAGE and self.tp_size == 1:
-                late = [commits.pop()]
+                commits, late = commits[:-1], commits[-1:]
             lm0 = max(0, want_from - start)
             lm_row0, lm_rows = 0, 0
             if end > want_from:
