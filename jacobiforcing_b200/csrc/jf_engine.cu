@@ -828,7 +828,7 @@ static bool takes_wide(const jf_engine* h, int T, const std::vector<Group>& grou
   return true;
 }
 
-static int run_wide(jf_engine* h, int T, const std::vector<Group>& groups, int lm_row0, int lm_rows, float* elapsed_ms) {
+static int run_wide(jf_engine* h, int T, const std::vector<Group>& groups, int lm_row0, int lm_rows, bool want_hidden, float* elapsed_ms) {
   DevCtx& c = h->hctx;
   const std::vector<FlashUnit> units = wide_units(h->md, groups, c.max_pages_per_seq);
   if (h->wide_units_d == nullptr) {
@@ -846,7 +846,7 @@ static int run_wide(jf_engine* h, int T, const std::vector<Group>& groups, int l
   JF_CUDA(h, cudaMemcpyAsync(h->wide_units_d, units.data(), units.size() * sizeof(FlashUnit), cudaMemcpyHostToDevice, h->stream));
   JF_CUDA(h, cudaEventRecord(h->ev0, h->stream));
   WideStream w{h->stream};
-  wide_forward(w, c, T, h->wide_units_d, (int)units.size(), lm_row0, lm_rows, h->wide_err);
+  wide_forward(w, c, T, h->wide_units_d, (int)units.size(), lm_row0, lm_rows, want_hidden, h->wide_err);
   JF_CUDA(h, cudaEventRecord(h->ev1, h->stream));
   JF_CUDA(h, cudaStreamSynchronize(h->stream));
   const cudaError_t last = cudaGetLastError();
@@ -944,7 +944,7 @@ extern "C" int jf_forward(jf_handle h, int32_t T, const int32_t* tokens, int32_t
   JF_CUDA(h, cudaMemcpyAsync(c.block_tables, block_tables, (size_t)n_seqs * c.max_pages_per_seq * 4, cudaMemcpyHostToDevice, h->stream));
   JF_CUDA(h, cudaStreamSynchronize(h->stream));     // the host vectors above go out of scope
   const bool wide = takes_wide(h, T, hg, row_group, lm_rows, hc, n_commit);
-  int rc = wide ? run_wide(h, T, hg, lm_row0, lm_rows, elapsed_ms) : launch_persistent(h, RUN_PLAN, 1, elapsed_ms);
+  int rc = wide ? run_wide(h, T, hg, lm_row0, lm_rows, hidden != nullptr, elapsed_ms) : launch_persistent(h, RUN_PLAN, 1, elapsed_ms);
   if (rc != JF_OK) return rc;
   if (!wide) {
     int dev_err = 0;

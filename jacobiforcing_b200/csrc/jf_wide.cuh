@@ -281,8 +281,9 @@ inline std::vector<FlashUnit> wide_units(const ModelDims& md, const std::vector<
   return u;
 }
 
-// The whole forward on w's stream; the plan's arrays (tokens, positions, groups, tables) are on the device already.
-inline void wide_forward(WideStream& w, const DevCtx& c, int T, const FlashUnit* units, int n_units, int lm_row0, int lm_rows, int* err) {
+// The whole forward on w's stream; the plan's arrays (tokens, positions, groups, tables) are on the device already.  Without rows that anybody
+// asks for (no logits, no hidden rows: the chunks of a prompt ahead of its end) the last layer ends with its keys and values.
+inline void wide_forward(WideStream& w, const DevCtx& c, int T, const FlashUnit* units, int n_units, int lm_row0, int lm_rows, bool want_hidden, int* err) {
   const ModelDims& md = c.md;
   __nv_bfloat16* qkv = reinterpret_cast<__nv_bfloat16*>(c.part);       // the split-K partial sums' buffer: T_cap rows of qkv_dim floats and more
   uint8_t* xn = reinterpret_cast<uint8_t*>(c.xn);
@@ -297,6 +298,7 @@ inline void wide_forward(WideStream& w, const DevCtx& c, int T, const FlashUnit*
     w.launch(wide_rope_kernel, T, 256, 0, qkv, md, c.row_pos, c.row_group, c.groups, c.block_tables, c.max_pages_per_seq, c.rope_cos, c.rope_sin, c.qbuf,
              c.kv_scratch + kv_scratch_offset(md, c.T_cap, l, 0, 0, 0), c.kv_scratch + kv_scratch_offset(md, c.T_cap, l, 1, 0, 0),
              c.kv_cache + kv_cache_offset(md, c.num_pages, l, 0, 0, 0, 0), c.kv_cache + kv_cache_offset(md, c.num_pages, l, 1, 0, 0, 0));
+    if (l + 1 == md.layers && lm_rows == 0 && !want_hidden) return;
     if (md.d == 64) wide_attention<64>(w, c, l, units, n_units, err);
     else wide_attention<128>(w, c, l, units, n_units, err);
     wide_product(w, c.xa, c.xrows_cap, 0, L.wo, 0, T, md.h, md.q_dim, WideResidual{c.hidden, md.h}, err);

@@ -141,3 +141,19 @@ def test_hit_on_a_page_that_the_end_of_a_prompt_filled(pair):
         for s in (hit, miss, short):
             rt.release(s)
     assert np.linalg.norm(a - b) < 2e-2 * np.linalg.norm(b)
+
+
+def test_chunks_whose_rows_nobody_reads(pair):
+    """Without logits the last layer ends with its keys and values: the same pages as with them, bit for bit."""
+    model, rt = pair
+    toks = prompt_of(608, 41, model.config.vocab_size)
+    got = []
+    for row0, rows in ((0, 0), (248, 8)):
+        s = rt.new_sequence()
+        rt.ensure_capacity(s, 616)
+        for at, n in ((0, 256), (256, 344)):
+            rt.forward(toks[at:at + n], [(0, n, 0, at)], [s], row0, rows, [(i, 0, at + i) for i in range(n)])
+        s.ctx = 600
+        got.append(verify(rt, s, toks[600:]))
+        rt.release(s)
+    assert np.array_equal(got[0], got[1])

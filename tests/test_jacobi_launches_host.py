@@ -113,8 +113,22 @@ def test_the_last_prompt_token_runs_on_the_persistent_kernel(fake, prompt, cache
     at, rows, lm_rows, kernels = runs[-1]
     assert kernels == [True] and at <= prompt - 1 < at + rows == prompt + draft and lm_rows > draft
     for at, rows, lm_rows, kernels in runs[:-1]:
-        assert at % 256 == 0 and rows % 256 == 0 and lm_rows == 0 and len(kernels) == 2 * 8 + 1 and not any(kernels)
+        assert at % 256 == 0 and rows % 256 == 0 and lm_rows == 0 and len(kernels) == 1 + 8 + 2 and not any(kernels)
     assert sum(r[1] for r in runs[:-1]) == max(0, (prompt - 1) // 256 * 256 - cached)
     assert commits == list(range(min(cached, prompt - 1), prompt))
+    rt.release(s)
+    rt.close()
+
+
+@pytest.mark.parametrize("logits,hidden", [(False, False), (True, False), (False, True), (True, True)])
+def test_the_last_layer_of_rows_that_nobody_reads(fake, logits, hidden):
+    """Only its keys and values are made; hidden rows or logits that are asked for need all of it."""
+    rt = engine()
+    s = rt.new_sequence()
+    rt.ensure_capacity(s, 256)
+    fake.reset()
+    rt.forward([1] * 256, [(0, 256, 0, 0)], [s], 248 if logits else 0, 8 if logits else 0, [(i, 0, i) for i in range(256)], want_hidden=hidden)
+    assert len(fake.launches()) == (1 + 2 * 8 if logits or hidden else 1 + 8 + 2) + 2 * logits
+    assert "wide_rope_kernel" in fake.launches()[10][0]
     rt.release(s)
     rt.close()
