@@ -1752,7 +1752,7 @@ LinearLaunch linear_launch(int parts, int vc, int dk, int dv, const AT* v, int l
 // first of them (keys_of: offsets [E + 1], then positions [E]).  NULL: the folded form.
 // Keys that no row sees (behind the window) are neither gathered nor projected: 64 to 128 tokens behind 6000 cached ones with a window of 128 took
 // 239 to 263 us with them, the folded form 220 to 244.  The projection is made for every key of the step and pays from about 64 tokens a
-// request on (64 tokens behind 0, 2048 and 8000: 158, 222 and 408 us, folded 261, 314 and 523), so keys of requests with fewer tokens are
+// request on (64 tokens behind 0, 2048 and 8000: 152, 217 and 395 us, folded 261, 314 and 523), so keys of requests with fewer tokens are
 // made in vain, and steps with more than 32 of those per token keep the folded form: 127 prompt tokens beside a decoded one behind 4000: 313 us,
 // folded 328; behind 7000: 389 against 342.  So do steps whose keys exceed the gathered rows.
 constexpr int HY_FLASH_TOKENS = 64, HY_FLASH_VAIN = 32;
@@ -1957,8 +1957,10 @@ void latent_mixer(hy_engine* h, const Batch& b, const LayerW& L, const hy_layer_
 // Routing tables of a layer: the counters that its route kernel fills (the two sets alternate, see route_place_kernel), rows per
 // tile of the grouped products, the expert-sorted order with the activation rows copied into it.
 int* next_counts(hy_engine* h) { h->x_set ^= 1; return h->x_counts + (size_t)h->x_set * 2 * h->x_max_experts; }
-// 256 rows per tile once experts have about that many (2048 tokens x 4 choices over 32 experts); 128 below
-int expert_tile_rows(int P, int NE) { return P >= 192 * NE ? 256 : 128; }
+// 256 rows per tile from 144 rows per expert on; below, tiles of 128 waste less on experts that do not fill one.  Both expert products of a
+// step, 32 experts, us with 128 -> 256: 128 rows per expert, width 1024 53.9 -> 61.0 and (larger experts) 72.8 -> 71.3; 160 rows 73.1 -> 61.5 and 85.5 ->
+// 77.2, width 2048 186 -> 146; 256 rows 74.7 -> 65.6, 99.6 -> 95.3, 231 -> 190.
+int expert_tile_rows(int P, int NE) { return P >= 144 * NE ? 256 : 128; }
 template <typename AT>
 void place_rows(hy_engine* h, int T, const AT* hb, const LayerW& L, const hy_layer_cfg& c, AT* rows) {
   const int P = T * c.x_top, W = h->m.width, E = h->x_max_experts;
