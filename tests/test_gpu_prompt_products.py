@@ -39,6 +39,12 @@ def test_grouped_tiles(experts, top, tokens, ff):
     assert fam.close(got, fam.oracle_logits(cfg, w, toks), "bfloat16")
 
 
+@pytest.mark.parametrize("tokens", [287, 288, 289])
+def test_grouped_tiles_at_the_line_between_their_sizes(tokens):
+    """Two experts, one per token: 144 rows per expert and more take 256-row tiles, fewer tiles of 128."""
+    test_grouped_tiles(2, 1, tokens, 40)
+
+
 @pytest.mark.parametrize("ff,tokens", [(40, 65), (10000, 260)])
 def test_gated_pairs_beside_plain_columns(ff, tokens):
     layer = {"type": "attention", "mixer": {"heads": 2, "kv_heads": 1, "dim": 16, "vdim": 16, "mask": {"size": 64}, "scale": 0.25},
