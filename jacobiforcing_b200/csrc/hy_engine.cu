@@ -146,7 +146,8 @@ struct hy_engine {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   std::string err;
   std::string step_err;                          // what failed first in the running step (empty: nothing); nothing is launched behind it
-  std::map<const void*, size_t> smem_limit;      // dynamic shared memory that a kernel is opted in to on this engine's device
+  std::set<const void*> opted_in;                // kernels that may use all shared memory of this engine's device
+  int smem_most = 0;                             // per block, static part included
   int64_t launches = 0;
   float last_ms = 0.0f;
   int64_t bytes_w = 0, bytes_cache = 0, bytes_state = 0, bytes_ws = 0;
@@ -195,16 +196,17 @@ struct hy_engine {
 // kernel that starts under another one's tail pile up on the SMs that are free already, and a recurrence with one block per
 // SM then runs two or three on some of them (two Kinetar layers, 2048 tokens: 2.02 ms plain, 2.35 ms overlapped).
 // Behind the first launch of a step that fails nothing else is launched; hy_step reports it.
-// More shared memory than every kernel may have (48 KiB with its static part) is asked for here, once per engine, kernel and size: the limit belongs
-// to a device, and a process may hold engines on several.
+// More shared memory than every kernel may have (48 KiB with its static part) is asked for here, once per engine and kernel: the limit belongs to a
+// device, and a process may hold engines on several.  Always all that the device has: engines of one device share the limit, and what a
+// smaller one asked for would be too little for a larger one.
 constexpr int HY_OVERLAP_TOKENS = 64;
 constexpr size_t HY_PLAIN_SMEM = 16 * 1024;
 inline cudaError_t opt_in(hy_engine* h, const void* kernel, size_t smem) {
-  if (smem <= HY_PLAIN_SMEM) return cudaSuccess;
-  size_t& limit = h->smem_limit[kernel];
-  if (limit >= smem) return cudaSuccess;
-  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e == cudaSuccess) limit = smem;
+  if (smem <= HY_PLAIN_SMEM || h->opted_in.count(kernel)) return cudaSuccess;
+  cudaFuncAttributes at;
+  cudaError_t e = cudaFuncGetAttributes(&at, kernel);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, h->smem_most - (int)at.sharedSizeBytes);
+  if (e == cudaSuccess) h->opted_in.insert(kernel);
   return e;
 }
 template <typename... P, typename... A>
@@ -385,6 +387,7 @@ extern "C" int hy_create(const hy_model_cfg* model, const hy_layer_cfg* layers, 
                         : (model->block_kind == HY_BLOCK_POSTNORM || model->block_kind == HY_BLOCK_PRENORM) ? HY_NORM_RMS : HY_NORM_RMS_OFFSET;
   if (model->norm_kind != want_norm && !rms_parallel && !rms_sandwich) return bad("block layout and norm kind do not go together");
   if (cudaSetDevice(rt->device) != cudaSuccess) return bad("cudaSetDevice failed");
+  if (cudaDeviceGetAttribute(&h->smem_most, cudaDevAttrMaxSharedMemoryPerBlockOptin, rt->device) != cudaSuccess) return bad("the device does not say how much shared memory it has");
   cudaStreamCreate(&h->stream);
   cudaEventCreate(&h->ev0);
   cudaEventCreate(&h->ev1);

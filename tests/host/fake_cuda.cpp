@@ -98,6 +98,7 @@ cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t, cudaEvent_t) { *ms = 0.0f; return cudaSuccess; }
 cudaError_t cudaGetLastError() { const cudaError_t e = g_last; g_last = cudaSuccess; return e; }
 const char* cudaGetErrorString(cudaError_t e) { return e == cudaErrorInvalidValue ? "invalid argument" : e == cudaErrorLaunchFailure ? "launch refused" : "error"; }
+cudaError_t cudaFuncGetAttributes(cudaFuncAttributes* a, const void*) { memset(a, 0, sizeof(*a)); return cudaSuccess; }
 cudaError_t cudaFuncSetAttribute(const void* f, cudaFuncAttribute a, int v) {
   if (fails(1)) return last(cudaErrorInvalidValue);
   if (a == cudaFuncAttributeMaxDynamicSharedMemorySize) {

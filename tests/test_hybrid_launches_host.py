@@ -97,6 +97,20 @@ def test_steps_on_two_devices(fake, which, dtype):
     assert seen[0] == seen[1]
 
 
+@pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
+@pytest.mark.parametrize("tokens", [1, 8, 150])
+def test_engines_of_unlike_sizes_take_turns(fake, tokens, dtype):
+    """The limit of a kernel is one for all engines on a device: what the smaller engine asks for must not take it from the larger one."""
+    def layers(dim, vdim, ff):
+        return kin.model_config([kin.delta(heads=2, kv_heads=1, dim=dim, vdim=vdim, ff=ff), kin.attn_scan()], width=40)
+    large, small = engine(layers(128, 128, 5000), dtype), engine(layers(120, 100, 1200), dtype)
+    fake.reset()
+    for rt in (large, small, large, small, large):
+        step(rt, tokens)
+    for rt in (large, small):
+        rt.close()
+
+
 def test_refused_shared_memory_is_reported(fake):
     rt = engine(FLASH)
     fake.reset()
