@@ -150,6 +150,10 @@ int jf_tp_import(jf_handle h, const void* handles /* tp_size x 64 bytes, rank or
  * rank order.  The ranks may sit on different devices with peer access, or share one device (num_ctas splits its SMs). */
 int jf_tp_attach_local(jf_handle h, const jf_handle* peers);
 
+/* Page-locked host memory for results (the device copies into it without a staging buffer).  0 or JF_ERR_CUDA. */
+int jf_host_alloc(int64_t bytes, void** out);
+int jf_host_free(void* p);
+
 /* Number of kernel launches issued by this handle since creation (bench.py's gpu_launches claim). */
 int64_t jf_launch_count(jf_handle h);
 

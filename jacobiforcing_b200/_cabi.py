@@ -11,7 +11,7 @@ LIB_PATH = os.path.join(_HERE, "libjacobi_b200.so")
 EXPORTS = [
     "jf_create", "jf_destroy", "jf_last_error", "jf_device_info", "jf_load_tensor", "jf_finalize_weights",
     "jf_set_rope_tables", "jf_kv_info", "jf_forward", "jf_commit_rows", "jf_jacobi_run", "jf_launch_count",
-    "jf_profile_enable", "jf_profile_read", "jf_tp_export", "jf_tp_import", "jf_tp_attach_local",
+    "jf_profile_enable", "jf_profile_read", "jf_host_alloc", "jf_host_free", "jf_tp_export", "jf_tp_import", "jf_tp_attach_local",
 ]
 
 JF_OK, JF_ERR_INVALID, JF_ERR_CUDA, JF_ERR_CAPACITY, JF_ERR_UNSUPPORTED, JF_ERR_POLICY = 0, -1, -2, -3, -4, -5
@@ -71,6 +71,9 @@ def load() -> C.CDLL:
     lib.jf_tp_import.argtypes = [vp, vp]
     if hasattr(lib, "jf_tp_attach_local"):
         lib.jf_tp_attach_local.argtypes = [vp, C.POINTER(vp)]
+    if hasattr(lib, "jf_host_alloc"):
+        lib.jf_host_alloc.argtypes = [C.c_int64, C.POINTER(vp)]
+        lib.jf_host_free.argtypes = [vp]
     lib.jf_launch_count.argtypes = [vp]
     lib.jf_launch_count.restype = C.c_int64
     for name in EXPORTS:

@@ -433,6 +433,14 @@ extern "C" int hy_memory_info(hy_handle h, int64_t* w, int64_t* c, int64_t* s, i
   return HY_OK;
 }
 
+extern "C" int hy_host_alloc(int64_t bytes, void** out) {
+  if (!out || bytes <= 0) return HY_ERR_INVALID;
+  if (cudaHostAlloc(out, (size_t)bytes, cudaHostAllocPortable) == cudaSuccess) return HY_OK;
+  cudaGetLastError();                                          // the caller goes on with pageable memory
+  return HY_ERR_CUDA;
+}
+extern "C" int hy_host_free(void* p) { return cudaFreeHost(p) == cudaSuccess ? HY_OK : HY_ERR_CUDA; }
+
 extern "C" int hy_load_tensor(hy_handle h, const char* name, const void* data, const int64_t* shape, int32_t ndim, int32_t dtype) {
   if (!h || !name || !data) return HY_ERR_INVALID;
   if (h->finalized) return fail(h, HY_ERR_INVALID, "weights are final");

@@ -608,6 +608,14 @@ static int pack_staged(jf_engine* h, __nv_bfloat16* dst, int R, int K, int dest_
   return JF_OK;
 }
 
+extern "C" int jf_host_alloc(int64_t bytes, void** out) {
+  if (!out || bytes <= 0) return JF_ERR_INVALID;
+  if (cudaHostAlloc(out, (size_t)bytes, cudaHostAllocPortable) == cudaSuccess) return JF_OK;
+  cudaGetLastError();                                          // the caller goes on with pageable memory
+  return JF_ERR_CUDA;
+}
+extern "C" int jf_host_free(void* p) { return cudaFreeHost(p) == cudaSuccess ? JF_OK : JF_ERR_CUDA; }
+
 extern "C" int jf_load_tensor(jf_handle h, const char* name, const void* data, const int64_t* shape, int32_t ndim,
                               int32_t dtype) {
   if (!h || !name || !data || !shape) return JF_ERR_INVALID;

@@ -11,7 +11,7 @@ from typing import Dict, List, Optional, Sequence, Tuple
 
 import numpy as np
 
-from . import _hybrid_cabi as cabi
+from . import _hybrid_cabi as cabi, hostmem
 from .hybrid_config import HybridConfig, iter_safetensors
 
 DTYPES = {"bfloat16": 0, "float32": 1}
@@ -67,6 +67,7 @@ class HybridRuntime:
         h = C.c_void_p()
         cabi.check(self.lib.hy_create(C.byref(m), layers, C.byref(rt), C.byref(h)), None)
         self.h = h
+        self._results = hostmem.of_library(self.lib.hy_host_alloc, self.lib.hy_host_free, 8 * self.max_want * self.vocab * 4)
         self.stats = {"steps": 0, "tokens": 0, "device_ms": 0.0}
 
     # ---- lifecycle -------------------------------------------------------------------------------------------------
@@ -74,6 +75,7 @@ class HybridRuntime:
         if getattr(self, "h", None):
             self.lib.hy_destroy(self.h)
             self.h = None
+            self._results.close()
 
     def __del__(self):
         try:
@@ -138,7 +140,7 @@ class HybridRuntime:
             pages[e, :len(pg)] = pg
         T = len(a_tok)
         n_want = len(want)
-        logits = np.empty((n_want, self.vocab), dtype=np.float32) if (n_want and want_logits) else None
+        logits = self._results.empty((n_want, self.vocab)) if (n_want and want_logits) else None
         sampled = np.empty((n_want,), dtype=np.int32) if (n_want and sample) else None
         temp = np.ascontiguousarray(np.asarray(temperature, dtype=np.float32)) if (temperature is not None and n_want) else None
         layers = np.empty((len(self.config.layer_runs()), T, self.width), dtype=np.float32) if want_layers else None

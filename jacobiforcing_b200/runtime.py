@@ -13,7 +13,7 @@ from typing import Dict, List, Optional, Sequence
 
 import numpy as np
 
-from . import _cabi
+from . import _cabi, hostmem
 from .policy import MODES, POLICY_ERRORS, STOP_REASONS, PolicyKnobs, draw_prefill_draft, mt_state_words
 from .tp import LocalTPGroup, check_divisibility, shard_tensor
 
@@ -92,6 +92,7 @@ class JacobiRuntime:
         h = C.c_void_p()
         _cabi.check(self.lib.jf_create(C.byref(self.model_cfg), C.byref(self.runtime_cfg), C.byref(h)), None)
         self.h = h
+        self._results = hostmem.of_library(self.lib.jf_host_alloc, self.lib.jf_host_free)
         self.free_pages = list(range(num_kv_pages - 1, -1, -1))
         self._next_seq = 0
         self.stats = {"forwards": 0, "device_ms": 0.0, "rows": 0}
@@ -135,6 +136,7 @@ class JacobiRuntime:
         if getattr(self, "h", None):
             self.lib.jf_destroy(self.h)
             self.h = None
+            self._results.close()
 
     def __del__(self):
         try:
@@ -260,7 +262,8 @@ class JacobiRuntime:
         commits = _i32(commits).reshape(-1, 3)
         bt = self._block_tables(seqs)
         greedy = np.zeros(T, np.int32)
-        logits = np.zeros((lm_rows, self.vocab_local), np.float32) if want_logits else None   # this rank's vocabulary slice
+        # this rank's vocabulary slice; the forward writes every row
+        logits = self._results.empty((lm_rows, self.vocab_local), np.float32) if want_logits else None
         hidden = np.zeros((T, self.hidden), np.uint16) if want_hidden else None
         ms = C.c_float()
         self._tp_sync()
