@@ -1,0 +1,599 @@
+// hy_chunk.cuh — matrix-state recurrences of prompt steps in chunks of 64 tokens (libjf_hybrid.so): the same recurrence as gla_kernel
+// (hy_gla.cuh), S <- diag(a) S + k v^T, o = S^T q, without its chain of tokens.
+//
+// Token by token a head's state is a chain as long as the prompt, and a block has no more than its 16 columns to work on: 2048 tokens of 8 heads
+// of 128 x 128 took 187 us on 64 of 148 SMs, about 170 cycles a token.  Within a chunk the recurrence is products of matrices:
+//   state behind the chunk   S' = diag(a_0 .. a_63) S + sum_j (k_j a_j+1 .. a_63) v_j^T                       (gla_chunk_state_kernel)
+//   read-outs                o_i = (q_i a_0 .. a_i)^T S + sum_(j <= i) (q_i . a_j+1 .. a_i . k_j) v_j           (gla_chunk_out_kernel)
+// so the chunks' own sums are made side by side, the states at their beginnings follow element by element (gla_chunk_scan_kernel), and the
+// read-outs again side by side.  All operands, sums and states are fp32 on the fp32 units, as they are token by token; decays are
+// products of the given decays (no logarithms, no quotients: every factor is at most one and a decay of zero is just a zero).  Per
+// channel they are applied in sub-blocks of 16: inside one, pair by pair; between two, as (q from the later one's beginning) . (whole
+// sub-blocks between) . (k to the earlier one's end).
+// Operands come from shared memory, 8 x 8 and 8 x 4 sums per thread; in turn the fma pipe (a third of the time) and the reads of shared memory (half of
+// it) bound them, with two blocks of eight warps per SM.  2048 tokens, us, token by token -> chunks (three kernels): forget gates, 8
+// heads of 128 x 128, 187 -> 72; state space, 32 heads of 64 x 128, 236 -> 140; two requests of gated linear attention, 16 heads of
+// 128 x 128, 251 -> 137; five requests of retention, 8 heads, 118 -> 66.
+#pragma once
+#include "hy_gla.cuh"
+
+namespace hy {
+
+constexpr int CH_T = 64, CH_SUB = 16, CH_SUBS = CH_T / CH_SUB;
+constexpr int CH_MAX_DIM = 128;
+
+// The chunk'th chunk of a step's entries (entry by entry).
+struct ChunkPlace {
+  int e, index, t0, n;                                         // entry, its chunk, first row of the step, tokens
+  __device__ ChunkPlace(const Batch& b, int chunk) {
+    index = chunk;
+    for (e = 0; e < b.E - 1; ++e) {
+      const int nc = (b.ent_start[e + 1] - b.ent_start[e] + CH_T - 1) / CH_T;
+      if (index < nc) break;
+      index -= nc;
+    }
+    t0 = b.ent_start[e] + index * CH_T;
+    n = min(CH_T, b.ent_start[e + 1] - t0);
+  }
+};
+
+// Operands as gla_kernel's; states [chunk][H][DK / 2][DV][2]: a chunk's own sum, then the state at its beginning, two rows side by side so that
+// the read-outs' products take pairs of rows without moving registers; ends [chunk][H][DK]: the product of a chunk's decays.
+template <typename AT>
+struct ChunkArgs {
+  Batch b;
+  const float* qk; const AT* v; int ldv;
+  const float* decay; int ldd; const float* head_decay;
+  int H, dim, vdim, vec, vvec, ovec;                           // 16-byte accesses: key rows and decays; value rows and the state; read-outs
+  float* states; float* ends; float* state;
+  float* o; int ldo;
+  GlaToken tk;
+};
+
+// rows of n floats, `cols` of DK in use, to sw [64][DK] (chunks of 16 bytes xor the row's low bits with SWZ); the rest becomes `fill`
+template <int DK, bool SWZ>
+__device__ __forceinline__ int ch_at(int r, int c) { return r * DK + (SWZ ? (((c >> 2) ^ (r & 7)) << 2) + (c & 3) : c); }
+template <int DK, bool SWZ>
+__device__ __forceinline__ void ch_rows(float* dst, const float* src, size_t ld, int n, int cols, bool vec, float fill) {
+  if (vec) {
+    for (int i = threadIdx.x; i < CH_T * (DK / 4); i += 256) {
+      const int r = i / (DK / 4), c = i % (DK / 4) * 4;
+      float* d = dst + ch_at<DK, SWZ>(r, c);
+      if (r < n && c < cols) jf::cp_async_16(d, src + (size_t)r * ld + c, 16u);
+      else *reinterpret_cast<float4*>(d) = make_float4(fill, fill, fill, fill);
+    }
+  } else {
+    for (int i = threadIdx.x; i < CH_T * DK; i += 256) {
+      const int r = i / DK, c = i % DK;
+      dst[ch_at<DK, SWZ>(r, c)] = r < n && c < cols ? src[(size_t)r * ld + c] : fill;
+    }
+  }
+}
+// A token's decay and the factor of its value, one number per head (GLA_HEAD, GLA_TOKEN).
+template <typename AT, int MODE>
+__device__ __forceinline__ void ch_scalars(const ChunkArgs<AT>& a, const ChunkPlace& p, int h, float* sa, float* sx) {
+  if (threadIdx.x < CH_T) {
+    const int t = threadIdx.x;
+    float d = 1.0f, x = 1.0f;
+    if (t < p.n) {
+      if constexpr (MODE == GLA_HEAD) d = a.head_decay[h];
+      else {
+        x = softplus_f(to_f(((const AT*)a.tk.dt_raw)[(size_t)(p.t0 + t) * a.tk.lddt + h]) + a.tk.dt_bias[h]);
+        d = expf(-expf(a.tk.A_log[h]) * x);
+      }
+    }
+    sa[t] = d; sx[t] = x;
+  }
+}
+
+template <int DK, int DV, int MODE>
+__host__ __device__ constexpr size_t ch_state_smem() {
+  return ((size_t)CH_T * DK + (MODE == GLA_CHANNEL ? (size_t)CH_T * DK : 0) + (size_t)CH_T * DV + CH_SUBS * DK + 3 * CH_T) * 4;
+}
+
+// A chunk's own sum and its decays' product.  grid (chunks, H), 256 threads, each DK / 16 x DV / 16 sums.
+template <typename AT, int DK, int DV, int MODE>
+__global__ void __launch_bounds__(256, 2) gla_chunk_state_kernel(ChunkArgs<AT> a) {
+  pdl_begin();
+  constexpr bool SCALAR = MODE == GLA_HEAD || MODE == GLA_TOKEN;
+  constexpr int TD = DK / 16, TV = DV / 16;
+  extern __shared__ __align__(16) unsigned char hy_smem[];
+  float* sk = reinterpret_cast<float*>(hy_smem);               // [64][DK] keys (GLA_FORGET: decays first)
+  float* sd = sk + CH_T * DK;                                  // [64][DK] decays (GLA_CHANNEL)
+  float* sv = sd + (MODE == GLA_CHANNEL ? CH_T * DK : 0);      // [64][DV]
+  float* se = sv + CH_T * DV;                                  // [4][DK] product of a sub-block's decays
+  float* sa = se + CH_SUBS * DK;                               // [64] decay, [64] factor of the value
+  const ChunkPlace p(a.b, blockIdx.x);
+  const int h = blockIdx.y, tid = threadIdx.x;
+  const int per = MODE == GLA_TOKEN ? a.tk.G : a.H, row = MODE == GLA_TOKEN ? h / (a.H / a.tk.G) : h;
+  ch_rows<DK, false>(sk, a.qk + ((size_t)p.t0 * per + row) * 2 * a.dim + a.dim, (size_t)per * 2 * a.dim, p.n, a.dim, a.vec, MODE == GLA_FORGET ? 1.0f : 0.0f);
+  if constexpr (MODE == GLA_CHANNEL) ch_rows<DK, false>(sd, a.decay + (size_t)p.t0 * a.ldd + h * a.dim, a.ldd, p.n, a.dim, a.vec, 1.0f);
+  if constexpr (SCALAR) ch_scalars<AT, MODE>(a, p, h, sa, sa + CH_T);
+  if (a.vvec) {
+    for (int i = tid; i < CH_T * DV / 4; i += 256) {
+      const int r = i / (DV / 4), c = i % (DV / 4) * 4;
+      float4 x = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      if (r < p.n && c < a.vdim) {
+        const VecN<AT, 4> v = *reinterpret_cast<const VecN<AT, 4>*>(a.v + (size_t)(p.t0 + r) * a.ldv + h * a.vdim + c);
+        x = make_float4(to_f(v.v[0]), to_f(v.v[1]), to_f(v.v[2]), to_f(v.v[3]));
+      }
+      *reinterpret_cast<float4*>(sv + 4 * i) = x;
+    }
+  } else {
+    for (int i = tid; i < CH_T * DV; i += 256) {
+      const int r = i / DV, c = i % DV;
+      sv[i] = r < p.n && c < a.vdim ? to_f(a.v[(size_t)(p.t0 + r) * a.ldv + h * a.vdim + c]) : 0.0f;
+    }
+  }
+  jf::cp_async_wait_all();
+  __syncthreads();
+  // keys times the decays behind them in their sub-block, the sub-blocks' products
+  for (int i = tid; i < CH_SUBS * DK; i += 256) {
+    const int s = i / DK, d = i % DK;
+    float w = 1.0f;
+#pragma unroll
+    for (int j = CH_SUB - 1; j >= 0; --j) {
+      const int t = s * CH_SUB + j;
+      float& k = sk[t * DK + d];
+      if constexpr (MODE == GLA_FORGET) { const float f = k; k = (1.0f - f) * w; w *= f; }
+      else if constexpr (MODE == GLA_CHANNEL) { k *= w; w *= sd[t * DK + d]; }
+      else { k *= w * sa[CH_T + t]; w *= sa[t]; }
+    }
+    se[i] = w;
+  }
+  __syncthreads();
+  const int tx = tid & 15, ty = tid >> 4;
+  float2 acc[TD][TV / 2] = {};
+  auto dcol = [&](int i) { return (i >> 2) * 64 + ty * 4 + (i & 3); };
+#pragma unroll 1
+  for (int s = 0; s < CH_SUBS; ++s) {
+    if (s * CH_SUB >= p.n) {                                   // nothing behind the last token; its decays are ones
+      break;
+    }
+    if (s > 0) {
+#pragma unroll
+      for (int i = 0; i < TD; ++i) {
+        const float e = se[s * DK + dcol(i)];
+#pragma unroll
+        for (int c = 0; c < TV / 2; ++c) acc[i][c] = mul2(acc[i][c], make_float2(e, e));
+      }
+    }
+#pragma unroll 4
+    for (int j = s * CH_SUB; j < (s + 1) * CH_SUB; ++j) {
+      float4 k[TD / 4], v[TV / 4];
+#pragma unroll
+      for (int i = 0; i < TD / 4; ++i) k[i] = *reinterpret_cast<const float4*>(sk + j * DK + i * 64 + ty * 4);
+#pragma unroll
+      for (int i = 0; i < TV / 4; ++i) v[i] = *reinterpret_cast<const float4*>(sv + j * DV + i * 64 + tx * 4);
+#pragma unroll
+      for (int i = 0; i < TD; ++i) {
+        const float kk = reinterpret_cast<const float*>(k)[i];
+#pragma unroll
+        for (int c = 0; c < TV / 4; ++c) {
+          acc[i][2 * c] = fma2(make_float2(kk, kk), make_float2(v[c].x, v[c].y), acc[i][2 * c]);
+          acc[i][2 * c + 1] = fma2(make_float2(kk, kk), make_float2(v[c].z, v[c].w), acc[i][2 * c + 1]);
+        }
+      }
+    }
+  }
+  const size_t at = (size_t)blockIdx.x * a.H + h;
+  float* out = a.states + at * DK * DV;
+#pragma unroll
+  for (int i = 0; i < TD; i += 2)
+#pragma unroll
+    for (int c = 0; c < TV / 2; ++c)
+      *reinterpret_cast<float4*>(out + (size_t)dcol(i) * DV + 2 * ((c >> 1) * 64 + tx * 4 + (c & 1) * 2)) =
+          make_float4(acc[i][c].x, acc[i + 1][c].x, acc[i][c].y, acc[i + 1][c].y);
+  if (tid < DK) {
+    float e = 1.0f;
+#pragma unroll
+    for (int s = 0; s < CH_SUBS; ++s) e *= se[s * DK + tid];
+    a.ends[at * DK + tid] = e;
+  }
+}
+
+// The states at the chunks' beginnings in the place of the chunks' own sums, the last one to the slot.  grid (DK DV / 1024, H, entries), 256
+// threads of two rows x two columns each; four chunks' sums are on their way at a time.
+template <typename AT, int DK, int DV>
+__global__ void __launch_bounds__(256) gla_chunk_scan_kernel(ChunkArgs<AT> a) {
+  pdl_begin();
+  const int e = blockIdx.z, h = blockIdx.y, i = (blockIdx.x * 256 + threadIdx.x) * 4, d = i / (2 * DV) * 2, c = i % (2 * DV) / 2;
+  int c0 = 0;
+  for (int f = 0; f < e; ++f) c0 += (a.b.ent_start[f + 1] - a.b.ent_start[f] + CH_T - 1) / CH_T;
+  const int n = (a.b.ent_start[e + 1] - a.b.ent_start[e] + CH_T - 1) / CH_T;
+  if (d >= a.dim || c >= a.vdim) return;                       // the padding's sums are zeros and stay
+  float* st = a.state + (((size_t)a.b.ent_slot[e] * a.H + h) * a.dim + d) * a.vdim + c;
+  const bool c1 = c + 1 < a.vdim, d1 = d + 1 < a.dim;
+  float s[4] = {};                                             // (d, c), (d + 1, c), (d, c + 1), (d + 1, c + 1)
+  if (a.b.ent_pos0[e] > 0) {
+    s[0] = st[0];
+    if (d1) s[1] = st[a.vdim];
+    if (c1) s[2] = st[1];
+    if (d1 && c1) s[3] = st[a.vdim + 1];
+  }
+  const size_t step = (size_t)a.H * DK * DV;
+  float* p = a.states + ((size_t)c0 * a.H + h) * DK * DV + i;
+  const float* w = a.ends + ((size_t)c0 * a.H + h) * DK + d;
+  for (int j = 0; j < n; j += 4) {
+    float4 x[4];
+    float2 f[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (j + k < n) {
+        x[k] = *reinterpret_cast<const float4*>(p + (j + k) * step);
+        f[k] = *reinterpret_cast<const float2*>(w + (size_t)(j + k) * a.H * DK);
+      }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (j + k >= n) break;
+      *reinterpret_cast<float4*>(p + (j + k) * step) = make_float4(s[0], s[1], s[2], s[3]);
+      s[0] = fmaf(f[k].x, s[0], x[k].x); s[1] = fmaf(f[k].y, s[1], x[k].y); s[2] = fmaf(f[k].x, s[2], x[k].z); s[3] = fmaf(f[k].y, s[3], x[k].w);
+    }
+  }
+  st[0] = s[0];
+  if (d1) st[a.vdim] = s[1];
+  if (c1) st[1] = s[2];
+  if (d1 && c1) st[a.vdim + 1] = s[3];
+}
+
+// Shared memory of the read-outs: queries, keys (then two slices of the state), decays (then values and weights), per sub-block products and scalars.
+template <typename AT, int DK, int DV>
+__host__ __device__ constexpr size_t ch_third_bytes() {
+  const size_t vw = (size_t)CH_T * DV * sizeof(AT) + CH_T * CH_T * 4, d = (size_t)CH_T * DK * 4;
+  return vw > d ? vw : d;
+}
+template <int DK, int DV>
+__host__ __device__ constexpr size_t ch_second_bytes() {
+  const size_t s = 2 * 32 * (size_t)DV * 4, k = (size_t)CH_T * DK * 4;
+  return s > k ? s : k;
+}
+template <typename AT, int DK, int DV>
+__host__ __device__ constexpr size_t ch_out_smem() {
+  return (size_t)CH_T * DK * 4 + ch_second_bytes<DK, DV>() + ch_third_bytes<AT, DK, DV>() + (CH_SUBS * DK + 4 * CH_T) * 4;
+}
+
+// Weights of pairs inside one sub-block, decays per channel: half a warp takes key j of the sub-block, a lane 4 or 8 of its channels, and the
+// running product k_j a_j+1 .. a_i meets the queries i = j .. 15; the sixteen sums are then exchanged so that lane i keeps that of query i.
+template <int DK, bool FORGET>
+__device__ __forceinline__ float ch_pairs(const float* sq, const float* sk, const float* sd, int s, int j, int jw, int l) {
+  constexpr int NC = DK / 64;
+  float p[CH_SUB];
+  float2 w[2 * NC];
+#pragma unroll
+  for (int c = 0; c < 2 * NC; ++c) w[c] = make_float2(0.0f, 0.0f);
+#pragma unroll
+  for (int i = 0; i < CH_SUB; ++i) {
+    p[i] = 0.0f;
+    if (i < CH_SUB / 2 && jw >= CH_SUB / 2) continue;          // the same for the whole warp
+    const int r = s * CH_SUB + i;
+    float2 sum = make_float2(0.0f, 0.0f);
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      const int at = ch_at<DK, true>(r, c * 64 + l * 4);
+      const float4 d = *reinterpret_cast<const float4*>(sd + at), q = *reinterpret_cast<const float4*>(sq + at);
+      if (i == j) {
+        const float4 k = FORGET ? make_float4(1.0f - d.x, 1.0f - d.y, 1.0f - d.z, 1.0f - d.w) : *reinterpret_cast<const float4*>(sk + at);
+        w[2 * c] = make_float2(k.x, k.y); w[2 * c + 1] = make_float2(k.z, k.w);
+      } else {
+        w[2 * c] = mul2(w[2 * c], make_float2(d.x, d.y)); w[2 * c + 1] = mul2(w[2 * c + 1], make_float2(d.z, d.w));
+      }
+      sum = fma2(w[2 * c], make_float2(q.x, q.y), sum);
+      sum = fma2(w[2 * c + 1], make_float2(q.z, q.w), sum);
+    }
+    p[i] = sum.x + sum.y;
+  }
+  int n = CH_SUB;
+#pragma unroll
+  for (int x = 8; x >= 1; x >>= 1) {
+    n >>= 1;
+    const bool hi = (l & x) != 0;
+#pragma unroll
+    for (int u = 0; u < CH_SUB / 2; ++u) {
+      if (u >= n) break;
+      const float other = __shfl_xor_sync(0xffffffffu, hi ? p[u] : p[u + n], x);
+      p[u] = (hi ? p[u + n] : p[u]) + other;
+    }
+  }
+  return p[0];                                                 // of query l
+}
+
+// Weights of the queries of sub-block I and the keys of the sub-blocks before it: x [i][d] . y [j][d], both carried to I's beginning.  A thread
+// takes 4 queries x I keys over a quarter of the channels; the quarters meet by shuffles.
+template <int DK>
+__device__ __forceinline__ void ch_block_row(const float* x, const float* y, float* w, int I) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, dg = lane >> 3, jt = (warp & 1) * 8 + (lane & 7), i0 = I * CH_SUB + (warp >> 1) * 4;
+  float2 acc[4][3] = {};
+#pragma unroll 2
+  for (int c = 0; c < DK / 16; ++c) {
+    const int d = (c * 4 + dg) * 4;
+    float4 q[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) q[i] = *reinterpret_cast<const float4*>(x + ch_at<DK, true>(i0 + i, d));
+#pragma unroll
+    for (int jj = 0; jj < 3; ++jj) {
+      if (jj >= I) break;
+      const float4 k = *reinterpret_cast<const float4*>(y + ch_at<DK, true>(jj * CH_SUB + jt, d));
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        acc[i][jj] = fma2(make_float2(q[i].x, q[i].y), make_float2(k.x, k.y), acc[i][jj]);
+        acc[i][jj] = fma2(make_float2(q[i].z, q[i].w), make_float2(k.z, k.w), acc[i][jj]);
+      }
+    }
+  }
+#pragma unroll
+  for (int jj = 0; jj < 3; ++jj) {
+    if (jj >= I) break;
+    float mine = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      float s = acc[i][jj].x + acc[i][jj].y;
+      s += __shfl_xor_sync(0xffffffffu, s, 8);
+      s += __shfl_xor_sync(0xffffffffu, s, 16);
+      if (i == dg) mine = s;
+    }
+    w[(i0 + dg) * CH_T + jj * CH_SUB + jt] = mine;
+  }
+}
+
+// The read-outs of a chunk.  grid (chunks, H), 256 threads; the products with the state and with the values run with 8 rows per warp and DV / 32
+// columns per lane.
+template <typename AT, int DK, int DV, int MODE>
+__global__ void __launch_bounds__(256, 2) gla_chunk_out_kernel(ChunkArgs<AT> a) {
+  pdl_begin();
+  constexpr bool SCALAR = MODE == GLA_HEAD || MODE == GLA_TOKEN;
+  constexpr int TV = DV / 32;
+  extern __shared__ __align__(16) unsigned char hy_smem[];
+  float* sq = reinterpret_cast<float*>(hy_smem);               // [64][DK] queries
+  float* sk = sq + CH_T * DK;                                  // [64][DK] keys, then [2][32][DV] rows of the state
+  float* sd = reinterpret_cast<float*>(hy_smem + (size_t)CH_T * DK * 4 + ch_second_bytes<DK, DV>());     // [64][DK] decays, then:
+  AT* sv = reinterpret_cast<AT*>(sd);                          // [64][DV] values
+  float* sw = reinterpret_cast<float*>(sv + CH_T * DV);        // [64][64] weights
+  float* se = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(sd) + ch_third_bytes<AT, DK, DV>());   // [4][DK]
+  float* sa = se + CH_SUBS * DK;                               // [64] decay, [64] factor of the value, [64] from the sub-block's beginning, [64] to its end
+  const ChunkPlace p(a.b, blockIdx.x);
+  const int h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int per = MODE == GLA_TOKEN ? a.tk.G : a.H, row = MODE == GLA_TOKEN ? h / (a.H / a.tk.G) : h;
+  const float* rows = a.qk + ((size_t)p.t0 * per + row) * 2 * a.dim;
+  const size_t ld = (size_t)per * 2 * a.dim;
+  ch_rows<DK, true>(sq, rows, ld, p.n, a.dim, a.vec, 0.0f);
+  if constexpr (MODE == GLA_FORGET) ch_rows<DK, true>(sd, rows + a.dim, ld, p.n, a.dim, a.vec, 1.0f);
+  else ch_rows<DK, true>(sk, rows + a.dim, ld, p.n, a.dim, a.vec, 0.0f);
+  if constexpr (MODE == GLA_CHANNEL) ch_rows<DK, true>(sd, a.decay + (size_t)p.t0 * a.ldd + h * a.dim, a.ldd, p.n, a.dim, a.vec, 1.0f);
+  if constexpr (SCALAR) ch_scalars<AT, MODE>(a, p, h, sa, sa + CH_T);
+  auto values = [&]() {
+    constexpr int CH = 16 / (int)sizeof(AT);
+    const AT* src = a.v + (size_t)p.t0 * a.ldv + h * a.vdim;
+    if (a.vvec) {
+      for (int i = tid; i < CH_T * (DV / CH); i += 256) {
+        const int r = i / (DV / CH), c = i % (DV / CH) * CH;
+        AT* d = sv + r * DV + c;
+        if (r < p.n && c < a.vdim) jf::cp_async_16(d, src + (size_t)r * a.ldv + c, 16u);
+        else *reinterpret_cast<uint4*>(d) = make_uint4(0u, 0u, 0u, 0u);
+      }
+    } else {
+      for (int i = tid; i < CH_T * DV; i += 256) {
+        const int r = i / DV, c = i % DV;
+        sv[i] = r < p.n && c < a.vdim ? src[(size_t)r * a.ldv + c] : from_f<AT>(0.0f);
+      }
+    }
+    jf::cp_async_commit();
+  };
+  const bool first = p.index == 0 && a.b.ent_pos0[p.e] == 0;   // behind nothing: the state is zero
+  const float* S = a.states + ((size_t)blockIdx.x * a.H + h) * DK * DV;
+  auto slice = [&](int i) {                                    // rows 32 i .. of the state
+    float* d = sk + (i & 1) * 32 * DV;
+    for (int k = tid; k < 32 * DV / 4; k += 256) jf::cp_async_16(d + 4 * k, S + (size_t)i * 32 * DV + 4 * k, 16u);
+    jf::cp_async_commit();
+  };
+  if constexpr (SCALAR) values();
+  jf::cp_async_commit();
+  jf::cp_async_wait_all();
+  __syncthreads();
+  if constexpr (!SCALAR) {
+    float own[CH_SUBS];                                        // weight (query l, key j) of each sub-block
+    const int l = tid & 15, hw = tid >> 4;
+#pragma unroll
+    for (int s = 0; s < CH_SUBS; ++s) {
+      const int j = s & 1 ? 15 - hw : hw, jw = s & 1 ? 14 - 2 * warp : 2 * warp;
+      own[s] = s * CH_SUB < p.n ? ch_pairs<DK, MODE == GLA_FORGET>(sq, sk, sd, s, j, jw, l) : 0.0f;
+    }
+    __syncthreads();
+    for (int i = tid; i < CH_SUBS * DK; i += 256) {            // queries from their sub-block's beginning, keys to its end
+      const int s = i / DK, d = i % DK;
+      float w = 1.0f, dec[CH_SUB];
+#pragma unroll
+      for (int t = 0; t < CH_SUB; ++t) {
+        const int at = ch_at<DK, true>(s * CH_SUB + t, d);
+        dec[t] = sd[at];
+        w *= dec[t];
+        sq[at] *= w;
+      }
+      se[i] = w;
+      w = 1.0f;
+#pragma unroll
+      for (int t = CH_SUB - 1; t >= 0; --t) {
+        const int at = ch_at<DK, true>(s * CH_SUB + t, d);
+        sk[at] = (MODE == GLA_FORGET ? 1.0f - dec[t] : sk[at]) * w;
+        w *= dec[t];
+      }
+    }
+    __syncthreads();                                           // the decays are done with: values and weights take their place
+    values();
+#pragma unroll
+    for (int s = 0; s < CH_SUBS; ++s) sw[(s * CH_SUB + l) * CH_T + s * CH_SUB + (s & 1 ? 15 - hw : hw)] = own[s];
+#pragma unroll 1
+    for (int I = 1; I < CH_SUBS && I * CH_SUB < p.n; ++I) {
+      if (I > 1) {                                             // keys of the earlier sub-blocks: on over sub-block I - 1
+        for (int i = tid; i < (I - 1) * CH_SUB * DK; i += 256) {
+          const int r = i / DK, d = i % DK;
+          sk[ch_at<DK, true>(r, d)] *= se[(I - 1) * DK + d];
+        }
+        __syncthreads();
+      }
+      ch_block_row<DK>(sq, sk, sw, I);
+      __syncthreads();
+    }
+    if (!first) {                                              // queries from the chunk's beginning
+      constexpr int PER = 256 / DK;
+      const int d = tid % DK;
+      float w = 1.0f;
+#pragma unroll
+      for (int I = 1; I < CH_SUBS; ++I) {
+        w *= se[(I - 1) * DK + d];
+#pragma unroll
+        for (int r = 0; r < CH_SUB / PER; ++r) sq[ch_at<DK, true>(I * CH_SUB + r * PER + tid / DK, d)] *= w;
+      }
+    }
+    __syncthreads();
+  } else {
+    float* sl = sa + 2 * CH_T;                                 // from the sub-block's beginning on; to its end
+    float* sr = sa + 3 * CH_T;
+    if (tid < 2 * CH_SUBS) {
+      const int s = tid >> 1;
+      float w = 1.0f;
+      if ((tid & 1) == 0) {
+        for (int t = 0; t < CH_SUB; ++t) { w *= sa[s * CH_SUB + t]; sl[s * CH_SUB + t] = w; }
+        se[s] = w;
+      } else {
+        for (int t = CH_SUB - 1; t >= 0; --t) { sr[s * CH_SUB + t] = w; w *= sa[s * CH_SUB + t]; }
+      }
+    }
+    // q . k of 4 queries x 4 keys per thread (keys tx, tx + 16, ..); what lies above the diagonal's blocks is left out
+    const int tx = tid & 15, ty = tid >> 4, I = ty >> 2;
+    float2 acc[4][4] = {};
+#pragma unroll 2
+    for (int d = 0; d < DK; d += 4) {
+      float4 q[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) q[i] = *reinterpret_cast<const float4*>(sq + ch_at<DK, true>(ty * 4 + i, d));
+#pragma unroll
+      for (int jj = 0; jj < 4; ++jj) {
+        if (jj > I) break;
+        const float4 k = *reinterpret_cast<const float4*>(sk + ch_at<DK, true>(jj * 16 + tx, d));
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          acc[i][jj] = fma2(make_float2(q[i].x, q[i].y), make_float2(k.x, k.y), acc[i][jj]);
+          acc[i][jj] = fma2(make_float2(q[i].z, q[i].w), make_float2(k.z, k.w), acc[i][jj]);
+        }
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int r = ty * 4 + i;
+#pragma unroll
+      for (int jj = 0; jj < 4; ++jj) {
+        if (jj > I) break;
+        const int j = jj * 16 + tx;
+        float w = j <= r ? sa[CH_T + j] : 0.0f;                // the value's factor
+        if (jj == I) { for (int m = j + 1; m <= r; ++m) w *= sa[m]; }
+        else {
+          w *= sl[r] * sr[j];
+          for (int s = jj + 1; s < I; ++s) w *= se[s];
+        }
+        sw[r * CH_T + j] = (acc[i][jj].x + acc[i][jj].y) * w;
+      }
+    }
+    __syncthreads();                                           // the keys are done with
+  }
+  const int r0 = warp * 8, c0 = lane * TV;
+  float2 acc[8][TV] = {};                                      // sums over even and over odd rows of the second operand
+  if (!first) {
+    slice(0);
+#pragma unroll 1
+    for (int i = 0; i < DK / 32; ++i) {
+      if (i + 1 < DK / 32) { slice(i + 1); jf::cp_async_wait_1(); }
+      else jf::cp_async_wait_all();
+      __syncthreads();
+      const float* s = sk + (i & 1) * 32 * DV + 2 * c0;
+      const float* q = sq + r0 * DK + i * 32;
+#pragma unroll
+      for (int d = 0; d < 32; d += 4) {
+        VecN<float, 4> x[TV];                                  // two row pairs of TV columns
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+#pragma unroll
+          for (int c = 0; c < TV / 2; ++c) x[k * (TV / 2) + c] = *reinterpret_cast<const VecN<float, 4>*>(s + (d + 2 * k) * DV + 4 * c);
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+          const float4 qq = *reinterpret_cast<const float4*>(q + r * DK + (((d >> 2) ^ r) << 2));
+#pragma unroll
+          for (int c = 0; c < TV; ++c) {
+            const VecN<float, 4>&u = x[c / 2], &v = x[TV / 2 + c / 2];
+            acc[r][c] = fma2(make_float2(qq.x, qq.y), make_float2(u.v[2 * (c & 1)], u.v[2 * (c & 1) + 1]), acc[r][c]);
+            acc[r][c] = fma2(make_float2(qq.z, qq.w), make_float2(v.v[2 * (c & 1)], v.v[2 * (c & 1) + 1]), acc[r][c]);
+          }
+        }
+      }
+      __syncthreads();                                         // the slice may be written over
+    }
+    if constexpr (SCALAR) {                                    // the decays from the chunk's beginning on
+      float e = 1.0f;
+      for (int s = 0; s < r0 / CH_SUB; ++s) e *= se[s];
+#pragma unroll
+      for (int r = 0; r < 8; ++r) {
+        const float w = e * sa[2 * CH_T + r0 + r];
+#pragma unroll
+        for (int c = 0; c < TV; ++c) acc[r][c] = mul2(acc[r][c], make_float2(w, w));
+      }
+    }
+  } else {
+    jf::cp_async_wait_all();
+    __syncthreads();
+  }
+  auto value = [&](int j, float (&x)[TV]) {
+    const VecN<AT, TV> v = *reinterpret_cast<const VecN<AT, TV>*>(sv + j * DV + c0);
+#pragma unroll
+    for (int c = 0; c < TV; ++c) x[c] = to_f(v.v[c]);
+  };
+  const int jend = min(r0 + 8, (p.n + 3) & ~3);
+#pragma unroll 1
+  for (int j = 0; j < jend; j += 4) {
+    float x[4][TV];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) value(j + k, x[k]);
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      const float4 w = *reinterpret_cast<const float4*>(sw + (r0 + r) * CH_T + j);
+#pragma unroll
+      for (int c = 0; c < TV; ++c) {
+        acc[r][c] = fma2(make_float2(w.x, w.y), make_float2(x[0][c], x[1][c]), acc[r][c]);
+        acc[r][c] = fma2(make_float2(w.z, w.w), make_float2(x[2][c], x[3][c]), acc[r][c]);
+      }
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < 8; ++r) {
+    const int t = r0 + r;
+    if (t >= p.n) break;
+    VecN<float, TV> y;
+#pragma unroll
+    for (int c = 0; c < TV; ++c) y.v[c] = acc[r][c].x + acc[r][c].y;
+    if constexpr (MODE == GLA_TOKEN) {
+      float x[TV];
+      value(t, x);
+      const float skip = a.tk.D[h];
+#pragma unroll
+      for (int c = 0; c < TV; ++c) y.v[c] = fmaf(skip, x[c], y.v[c]);
+    }
+    float* out = a.o + (size_t)(p.t0 + t) * a.ldo + h * a.vdim + c0;
+    if (a.ovec) {
+      if (c0 < a.vdim) *reinterpret_cast<VecN<float, TV>*>(out) = y;
+      continue;
+    }
+#pragma unroll
+    for (int c = 0; c < TV; ++c)
+      if (c0 + c < a.vdim) out[c] = y.v[c];
+  }
+}
+
+// ---- host: which recurrences run in chunks, in which steps (see step_chunks) ------------------------------------------------------------
+// From 512 tokens of the longest request on: three launches and a block's own time cost 40 us, the chain of tokens 0.1 us each.  Token by token and in
+// chunks, us: 8 heads with forget gates 512 tokens 66 and 62, 384 tokens 53 and 61; state space 512 tokens 78 and 61; gated linear, 16 heads, 512
+// tokens 97 and 75, 320 tokens 70 and 71.  Key and value sizes up to 32 have too little work per chunk for it.
+constexpr int HY_CHUNK_TOKENS = 512, HY_CHUNK_ENTRIES = 64;
+inline bool chunk_sizes(int dk, int dv) { return dk > 32 && dk <= CH_MAX_DIM && dv > 32 && dv <= CH_MAX_DIM; }
+// chunks that a step of max_step_tokens may be cut into
+inline int chunk_cap(int max_tokens) { return (5 * max_tokens + 4 * CH_T) / (4 * CH_T); }
+
+}  // namespace hy

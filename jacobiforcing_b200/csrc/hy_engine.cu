@@ -26,6 +26,7 @@
 #include "hy_biased.cuh"
 #include "hy_delta.cuh"
 #include "hy_gla.cuh"
+#include "hy_chunk.cuh"
 #include "jf_flash.cuh"
 
 namespace hy {
@@ -176,6 +177,7 @@ struct hy_engine {
   // its column count; rot_tables_d is what the kernel reads
   struct RotEntry { hy_layer_cfg c; RotTable t; };
   std::vector<RotEntry> rot_tables; RotTable* rot_tables_d = nullptr;
+  float* ch_states = nullptr; float* ch_ends = nullptr; int ch_cap = 0;    // chunked recurrences (hy_chunk.cuh): chunks that the sums have room for
   float* part_o = nullptr; float* part_ml = nullptr; size_t part_rows = 0, part_dim = 0;
   const int32_t* step_start = nullptr; const int32_t* step_pos0 = nullptr;     // host views of the running step
   size_t esz() const { return m.dtype == HY_DTYPE_F32 ? 4 : 2; }
@@ -1498,6 +1500,23 @@ extern "C" int hy_finalize(hy_handle h) {
       HY_CUDA(cudaMemset(h->x_meta, 0, 16));
     }
   }
+  {
+    size_t states = 0, ends = 0;                              // floats per chunk of the largest layer
+    auto layer = [&](int H, int dk, int dv) {
+      if (!chunk_sizes(dk, dv)) return;
+      const size_t k = dk <= 64 ? 64 : 128, v = dv <= 64 ? 64 : 128;
+      states = std::max(states, (size_t)H * k * v); ends = std::max(ends, (size_t)H * k);
+    };
+    for (auto& c : h->lc) {
+      if (c.mixer == HY_MIX_SSD) layer(c.m_heads, c.m_state, c.m_vdim);
+      if (c.mixer == HY_MIX_GLR || c.mixer == HY_MIX_GLA || c.mixer == HY_MIX_RETENTION) layer(c.g_heads, c.g_dim, c.g_vdim);
+    }
+    if (states > 0 && rt.max_step_tokens >= HY_CHUNK_TOKENS) {
+      h->ch_cap = chunk_cap(rt.max_step_tokens);
+      if (dev_alloc(h, (void**)&h->ch_states, (size_t)h->ch_cap * states * 4, &h->bytes_ws)) return HY_ERR_CUDA;
+      if (dev_alloc(h, (void**)&h->ch_ends, (size_t)h->ch_cap * ends * 4, &h->bytes_ws)) return HY_ERR_CUDA;
+    }
+  }
   if (!h->rot_tables.empty()) {
     std::vector<RotTable> t;
     for (auto& r : h->rot_tables) t.push_back(r.t);
@@ -1756,6 +1775,45 @@ LinearLaunch linear_launch(int parts, int vc, int dk, int dv, const AT* v, int l
   const int cpb = lin_cpb(parts, vc), ch = 16 / (int)sizeof(AT);
   return LinearLaunch{(dv + cpb - 1) / cpb, dk % 4 == 0 ? 1 : 0,
                       dv % ch == 0 && cpb % ch == 0 && ldv % ch == 0 && (reinterpret_cast<uintptr_t>(v) & 15) == 0 ? 1 : 0};
+}
+
+// Chunks of the running step if its matrix-state recurrences of this size run in chunks of 64 tokens (hy_chunk.cuh), else 0.
+int step_chunks(const hy_engine* h, const Batch& b, int dk, int dv) {
+  if (!chunk_sizes(dk, dv) || b.E > HY_CHUNK_ENTRIES) return 0;
+  int most = 0, n = 0;
+  for (int e = 0; e < b.E; ++e) {
+    const int cnt = h->step_start[e + 1] - h->step_start[e];
+    most = std::max(most, cnt);
+    n += (cnt + CH_T - 1) / CH_T;
+  }
+  return most >= HY_CHUNK_TOKENS && n <= h->ch_cap && 4LL * n * CH_T <= 5LL * b.T + 4 * CH_T ? n : 0;
+}
+
+// The recurrence of gla_kernel over a step in chunks, if the step is one for them.
+template <typename AT, int MODE>
+bool gla_chunked(hy_engine* h, const Batch& b, int H, int dk, int dv, const AT* v, int ldv, const float* decay, int ldd, const float* head_decay, float* state,
+                 float* o, int ldo, const GlaToken& tk) {
+  const int chunks = step_chunks(h, b, dk, dv);
+  if (chunks == 0) return false;
+  const int ch = 16 / (int)sizeof(AT);
+  ChunkArgs<AT> a{b, h->lin, v, ldv, decay, ldd, head_decay, H, dk, dv};
+  a.vec = dk % 4 == 0 && ldd % 4 == 0 && (reinterpret_cast<uintptr_t>(decay) & 15) == 0;
+  a.vvec = dv % ch == 0 && ldv % ch == 0 && (reinterpret_cast<uintptr_t>(v) & 15) == 0;
+  a.ovec = dv % 4 == 0 && ldo % 4 == 0 && (reinterpret_cast<uintptr_t>(o) & 15) == 0;
+  a.states = h->ch_states; a.ends = h->ch_ends; a.state = state; a.o = o; a.ldo = ldo; a.tk = tk;
+  auto go = [&](auto k, auto c) {
+    constexpr int DK = decltype(k)::value, DV = decltype(c)::value;
+    go_kernel(h, gla_chunk_state_kernel<AT, DK, DV, MODE>, dim3(chunks, H), 256, ch_state_smem<DK, DV, MODE>(), h->stream, a);
+    go_kernel(h, gla_chunk_scan_kernel<AT, DK, DV>, dim3(DK * DV / 1024, H, b.E), 256, 0, h->stream, a);
+    go_kernel(h, gla_chunk_out_kernel<AT, DK, DV, MODE>, dim3(chunks, H), 256, ch_out_smem<AT, DK, DV>(), h->stream, a);
+  };
+  typedef std::integral_constant<int, 64> c64; typedef std::integral_constant<int, 128> c128;
+  if (dk <= 64 && dv <= 64) go(c64{}, c64{});
+  else if (dk <= 64) go(c64{}, c128{});
+  else if (dv <= 64) go(c128{}, c64{});
+  else go(c128{}, c128{});
+  h->launches += 2;                                            // the caller counts one for the recurrence
+  return true;
 }
 
 // Whether the running step's latent attention with this window runs over per-head keys and values (latent_prompt), and then: its row units with H
@@ -2024,6 +2082,7 @@ int sandwich_layer(hy_engine* h, const Batch& b, size_t li) {
     {
       ProfScope ps(h, HY_PROF_SCAN);
       const GlaToken tk{G, pin + 2 * inner + 2 * GN, h->ld_pin, L.m_dt_bias, L.m_A_log, L.m_D};
+      if (!gla_chunked<AT, GLA_TOKEN>(h, b, H, N, P, cv, h->ld_cv, nullptr, 0, nullptr, L.rec_state, h->f2, h->ld_f2, tk))
       launch_linear<AT>(N, H, P, E, [&](auto dr, auto parts, auto vcols) {
         constexpr int DR = decltype(dr)::value, PARTS = decltype(parts)::value, VC = decltype(vcols)::value;
         const LinearLaunch g = linear_launch<AT>(PARTS, VC, N, P, cv, h->ld_cv);
@@ -2050,6 +2109,7 @@ int sandwich_layer(hy_engine* h, const Batch& b, size_t li) {
     ProfScope ps(h, HY_PROF_DELTA);
     if (dk <= HY_LIN_MAX_DIM) {
       go_kernel(h, forget_rows_kernel<AT>, T, T <= 8 ? 1024 : 256, 0, s, pin, h->ld_pin, L.c_q, L.c_k, L.g_fb, L.g_lower, H, dk, h->lin);
+      if (!gla_chunked<AT, GLA_FORGET>(h, b, H, dk, dv, pin + L.c_v, h->ld_pin, nullptr, 0, nullptr, L.rec_state, h->f2, h->ld_f2, GlaToken{}))
       launch_linear<AT>(dk, H, dv, E, [&](auto dr, auto parts, auto vcols) {
         constexpr int DR = decltype(dr)::value, PARTS = decltype(parts)::value, VC = decltype(vcols)::value;
         const LinearLaunch g = linear_launch<AT>(PARTS, VC, dk, dv, pin + L.c_v, h->ld_pin);
@@ -2553,6 +2613,7 @@ void gla_mixer(hy_engine* h, const Batch& b, const LayerW& L, const hy_layer_cfg
   }
   ProfScope ps(h, HY_PROF_DELTA);
   go_kernel(h, linear_rows_kernel<AT>, T, T <= 8 ? 1024 : 128, 0, s, pin, h->ld_pin, L.c_q, L.c_k, H, dk, nullptr, 0, RotPair{0, 1}, h->lin);
+  if (!gla_chunked<AT, GLA_CHANNEL>(h, b, H, dk, dv, pin + L.c_v, h->ld_pin, h->f2, h->ld_f2, nullptr, L.rec_state, h->f2 + c_o, h->ld_f2, GlaToken{}))
   launch_linear<AT>(dk, H, dv, E, [&](auto dr, auto parts, auto vcols) {
     constexpr int DR = decltype(dr)::value, PARTS = decltype(parts)::value, VC = decltype(vcols)::value;
     const LinearLaunch g = linear_launch<AT>(PARTS, VC, dk, dv, pin + L.c_v, h->ld_pin);
@@ -2575,6 +2636,7 @@ void retention_mixer(hy_engine* h, const Batch& b, const LayerW& L, const hy_lay
   const RotPair rp{rot.pairs, c.r_half};
   ProfScope ps(h, HY_PROF_DELTA);
   go_kernel(h, linear_rows_kernel<AT>, T, T <= 8 ? 1024 : 128, 0, s, pin, h->ld_pin, L.c_q, L.c_k, H, dk, rot.out, rot.ld, rp, h->lin);
+  if (!gla_chunked<AT, GLA_HEAD>(h, b, H, dk, dv, pin + L.c_v, h->ld_pin, nullptr, 0, L.decay, L.rec_state, h->f2, h->ld_f2, GlaToken{}))
   launch_linear<AT>(dk, H, dv, E, [&](auto dr, auto parts, auto vcols) {
     constexpr int DR = decltype(dr)::value, PARTS = decltype(parts)::value, VC = decltype(vcols)::value;
     const LinearLaunch g = linear_launch<AT>(PARTS, VC, dk, dv, pin + L.c_v, h->ld_pin);

@@ -1,0 +1,83 @@
+"""Matrix-state recurrences of prompt steps in chunks of 64 tokens, against the plain fp64 restatements: portions that end at, before and
+behind a chunk, portions too short for chunks between them (the state passes from one form to the other), key and value sizes at and beside
+the padded ones (with and without 16-byte rows), several requests of a step, decays of nearly zero and of one."""
+import numpy as np
+import pytest
+
+from oracle import famepel_plain, kisadra_plain, mafalorn_plain
+from tests import famepel_helpers as fam
+from tests import hybrid_helpers as kin
+from tests import kisadra_helpers as kis
+from tests import mafalorn_helpers as maf
+
+pytestmark = pytest.mark.gpu
+
+CUTS = [512, 3, 575, 1, 61]                                    # chunks from 512 tokens on
+
+
+def _model(mode, dim, vdim, heads=2):
+    if mode == "state space":
+        return famepel_plain, fam, fam.model_config([fam.ssd(heads=heads, vdim=vdim, state=dim, groups=1, norm_groups=1, conv=4, mlp=None)])
+    if mode == "forget":
+        return famepel_plain, fam, fam.model_config([fam.glr(heads=heads, dim=dim, vdim=vdim, mlp=None)])
+    if mode == "gated linear":
+        return kisadra_plain, kis, kis.model_config([kis.gla(heads=heads, dim=dim, vdim=vdim, mlp=None)])
+    return mafalorn_plain, maf, maf.model_config([maf.ret(heads=heads, dim=dim, vdim=vdim, decay=[1.0 - 2.0 ** (-2.0 - 3.0 * h) for h in range(heads)], mlp=None)])
+
+
+MODES = ["state space", "forget", "gated linear", "retention"]
+
+
+@pytest.mark.parametrize("dim,vdim,dtype", [(33, 35, "float32"), (64, 64, "float32"), (66, 40, "bfloat16"), (128, 64, "bfloat16"), (100, 128, "float32"), (128, 127, "bfloat16")])
+@pytest.mark.parametrize("mode", MODES)
+def test_chunked_portions(mode, dim, vdim, dtype):
+    if mode == "retention" and dim % 2:
+        dim += 1
+    plain, helpers, cfg = _model(mode, dim, vdim)
+    toks = kin.rand_tokens(sum(CUTS), cfg["vocab"], 5)
+    w = plain.random_weights(cfg, 0)
+    hz = helpers.Harness(cfg, w, dtype, num_pages=80, max_step_tokens=640)
+    try:
+        got = hz.feed("a", toks, CUTS)
+    finally:
+        hz.close()
+    assert helpers.close(got, helpers.oracle_logits(cfg, w, toks), dtype)
+
+
+@pytest.mark.parametrize("mode", MODES)
+def test_chunked_requests_of_a_step(mode):
+    """Requests of 575, 1 and 576 tokens in one step, then again behind themselves."""
+    plain, helpers, cfg = _model(mode, 64, 36)
+    w = plain.random_weights(cfg, 1)
+    lens = {"a": 575, "b": 1, "c": 576}
+    toks = {k: kin.rand_tokens(2 * n if n < 100 else n + 530, cfg["vocab"], i) for i, (k, n) in enumerate(lens.items())}
+    hz = helpers.Harness(cfg, w, "float32", num_pages=160, max_step_tokens=1280)
+    try:
+        first = hz.step([(k, toks[k][:n], range(n)) for k, n in lens.items()])
+        second = hz.step([(k, toks[k][n:], range(len(toks[k]) - n)) for k, n in lens.items()])
+    finally:
+        hz.close()
+    a = b = 0
+    for k, n in lens.items():
+        m = len(toks[k]) - n
+        got = np.concatenate([first[a:a + n], second[b:b + m]], 0)
+        a, b = a + n, b + m
+        assert helpers.close(got, helpers.oracle_logits(cfg, w, toks[k]), "float32"), k
+
+
+def test_chunked_forget_gates_of_zero_and_one():
+    """Forget gates at their ends: a channel that keeps everything beside one that keeps nothing."""
+    plain, helpers, cfg = _model("forget", 64, 64)
+    w = plain.random_weights(cfg, 2)
+    w["l0.mix.lower"] = w["l0.mix.lower"] * 0
+    bias = w["l0.mix.f.b"]
+    for i in range(bias.numel()):
+        if i % 4 < 2:
+            bias.view(-1)[i] = 60.0 if i % 4 else -120.0
+    toks = kin.rand_tokens(530, cfg["vocab"], 6)
+    hz = helpers.Harness(cfg, w, "float32", num_pages=80, max_step_tokens=640)
+    try:
+        got = hz.feed("a", toks, [530])
+    finally:
+        hz.close()
+    assert helpers.close(got, helpers.oracle_logits(cfg, w, toks), "float32")
