@@ -177,6 +177,7 @@ struct hy_engine {
   // its column count; rot_tables_d is what the kernel reads
   struct RotEntry { hy_layer_cfg c; RotTable t; };
   std::vector<RotEntry> rot_tables; RotTable* rot_tables_d = nullptr;
+  float* scan_own = nullptr;                     // own states and sums of step sizes of a selective scan's segments (see scan_segments)
   float* ch_states = nullptr; float* ch_ends = nullptr; int ch_cap = 0;    // chunked recurrences (hy_chunk.cuh): chunks that the sums have room for
   float* part_o = nullptr; float* part_ml = nullptr; size_t part_rows = 0, part_dim = 0;
   const int32_t* step_start = nullptr; const int32_t* step_pos0 = nullptr;     // host views of the running step
@@ -1511,6 +1512,13 @@ extern "C" int hy_finalize(hy_handle h) {
       if (c.mixer == HY_MIX_SSD) layer(c.m_heads, c.m_state, c.m_vdim);
       if (c.mixer == HY_MIX_GLR || c.mixer == HY_MIX_GLA || c.mixer == HY_MIX_RETENTION) layer(c.g_heads, c.g_dim, c.g_vdim);
     }
+    size_t scan = 0;
+    for (auto& c : h->lc)
+      if (c.mixer == HY_MIX_ATTN_SCAN) {
+        const int lanes = c.s_state <= 4 ? 1 : c.s_state <= 8 ? 2 : c.s_state <= 16 ? 4 : c.s_state <= 32 ? 8 : c.s_state <= 64 ? 16 : 32, per = 128 / lanes;
+        scan = std::max(scan, (size_t)scan_segment_rows((c.s_inner + per - 1) / per) * c.s_inner * (c.s_state + 1));
+      }
+    if (scan > 0 && rt.max_step_tokens >= 3 * SCAN_SEG_TOKENS && dev_alloc(h, (void**)&h->scan_own, scan * 4, &h->bytes_ws)) return HY_ERR_CUDA;
     if (states > 0 && rt.max_step_tokens >= HY_CHUNK_TOKENS) {
       h->ch_cap = chunk_cap(rt.max_step_tokens);
       if (dev_alloc(h, (void**)&h->ch_states, (size_t)h->ch_cap * states * 4, &h->bytes_ws)) return HY_ERR_CUDA;
@@ -2924,9 +2932,21 @@ int run_step(hy_engine* h, const Batch& b, int n_want, const int* want_d, float*
           // 16-byte copies: whole blocks of channels, rows and columns on 16-byte boundaries
           const int v32 = (R | N | h->ld_f1 | h->ld_f2 | I) % 4 == 0 && PB % 4 == 0;
           const int vat = (h->ld_cv | h->ld_pin | L.c_z | I) % ch == 0 && PB % ch == 0;
-          go_kernel(h, scan_kernel<AT, WT, NPER, LN>, dim3((I + PB - 1) / PB, E), 128, smem, s, 
-              b, cv, h->ld_cv, pin + L.c_z, h->ld_pin, h->f2, h->ld_f2, (const WT*)L.dt_b, h->f1, h->ld_f1, R, R + N, L.A_neg, (const WT*)L.D, I, N,
-              v32 | vat << 1, c.right_scale, L.rec_state, cat + L.o_scan, h->ld_cat);
+          auto pass = [&](auto which, int rows, ScanSegments seg) {
+            go_kernel(h, scan_kernel<AT, WT, NPER, LN, decltype(which)::value>, dim3((I + PB - 1) / PB, rows), 128, smem, s,
+                b, cv, h->ld_cv, pin + L.c_z, h->ld_pin, h->f2, h->ld_f2, (const WT*)L.dt_b, h->f1, h->ld_f1, R, R + N, L.A_neg, (const WT*)L.D, I, N,
+                v32 | vat << 1, c.right_scale, L.rec_state, cat + L.o_scan, h->ld_cat, seg);
+            h->launches++;
+          };
+          int most = 0;
+          for (int e = 0; e < E; ++e) most = std::max(most, h->step_start[e + 1] - h->step_start[e]);
+          const ScanSegments seg = scan_segments(h->scan_own, (I + PB - 1) / PB, E, most, I, N);
+          if (seg.count > 1) {
+            pass(std::integral_constant<int, SCAN_OWN>{}, E * seg.count, seg);
+            pass(std::integral_constant<int, SCAN_READ>{}, E * seg.count, seg);
+          } else {
+            pass(std::integral_constant<int, SCAN_WHOLE>{}, E, seg);
+          }
         };
         typedef std::integral_constant<int, 4> four;
         if (N <= 4) go(four{}, std::integral_constant<int, 1>{});
@@ -2936,7 +2956,6 @@ int run_step(hy_engine* h, const Batch& b, int n_want, const int* want_d, float*
         else if (N <= 64) go(four{}, std::integral_constant<int, 16>{});
         else if (N <= 128) go(four{}, std::integral_constant<int, 32>{});
         else go(std::integral_constant<int, 8>{}, std::integral_constant<int, 32>{});
-        h->launches++;
       }
     } else {
       const int nq = c.d_kv_heads * c.d_dim, nv = c.d_heads * c.d_vdim, C = 2 * nq + nv;

@@ -657,6 +657,32 @@ __global__ void __launch_bounds__(128) attn_sink_kernel(Batch b, const AT* __res
   }
 }
 
+// ---- decays exp(dt a) of two states at a time ---------------------------------------------------------------------------------------
+// dt a log2(e) as a rounded product and its remainder: 2^(y + e) = 2^y + 2^y e ln 2 for the |e| <= 2^-24 |y| that is left.  expf spends eight
+// instructions per state on its argument and its result's exponent, this five and a half; its error
+// against 64 bits is 2.0e-7 at most and 6.5e-8 root mean square from |dt a| = 1 to 80, where expf of the rounded product comes to 3.9e-6 and 9.0e-7, and
+// below one the same as expf's (1.9e-7 and 4.4e-8 against 1.6e-7 and 4.0e-8).
+struct RatePair {
+  float2 hi, neg, lo;                                          // a log2(e), its negative, what rounding took off it
+  RatePair() = default;
+  __device__ __forceinline__ RatePair(float a0, float a1) {
+    const float l2 = 1.4426950408889634f, l2_rest = 1.9259629911266175e-8f, most = -1e18f;      // products with dt <= 1e18 stay finite
+    a0 = a0 < most ? most : a0; a1 = a1 < most ? most : a1;
+    hi = make_float2(a0 * l2, a1 * l2);
+    neg = make_float2(-hi.x, -hi.y);
+    lo = make_float2(fmaf(a0, l2_rest, fmaf(a0, l2, neg.x)), fmaf(a1, l2_rest, fmaf(a1, l2, neg.y)));
+  }
+};
+__device__ __forceinline__ float ex2_f(float y) { float r; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(y)); return r; }
+__device__ __forceinline__ float2 exp_rates(float dt, const RatePair& a) {
+  const float2 d = make_float2(dt, dt), y = mul2(d, a.hi);
+  float2 e = fma2(d, a.hi, mul2(d, a.neg));
+  e = mul2(fma2(d, a.lo, e), make_float2(0.6931471805599453f, 0.6931471805599453f));
+  const float2 x = make_float2(ex2_f(y.x), ex2_f(y.y));
+  return fma2(x, e, x);
+}
+__device__ __forceinline__ float finite_step(float dt) { return dt > 1e18f ? 1e18f : dt; }
+
 // ---- selective scan -------------------------------------------------------------------------------------------------------------
 // S[c, n] <- exp(dt_c A[c, n]) S[c, n] + dt_c x_c B_n ; y_c = sum_n S[c, n] C_n + D_c x_c ; out = y silu(z) out_scale.
 // dt_raw is the step-size projection before bias and softplus.  low [T, ldl] holds [dt-rank part | B | C].
@@ -664,21 +690,31 @@ __global__ void __launch_bounds__(128) attn_sink_kernel(Batch b, const AT* __res
 // L lanes share a channel, each holding NPER CONSECUTIVE states (NPER * L >= nstate; the staged B and C are zero beyond nstate).
 // Inputs of TB tokens are copied asynchronously while the batch before them runs; the read-outs of eight tokens are reduced
 // in one exchange in which every step halves the tokens a lane keeps, so eight tokens run without a shuffle between them.
-// The arithmetic bounds it: about 13 instructions per state and token (the exponential takes 8 of them), so the fewer lanes
+// The arithmetic bounds it: about 6 instructions and one exponential per state and token (exp_rates), so the fewer lanes
 // share a channel the less is spent on the exchange and on indices: four states per lane.
 // 2048 tokens, 4096 channels of 16 states: one state per lane, a five-step exchange per token and loads waited for took 949 us
 // (0.46 us per token), this form 369 us.
+// That is a chain of tokens with less than a warp per scheduler, so long portions of few requests are cut into segments that run side by side: a first
+// pass (SCAN_OWN) leaves each segment's own state (the first one's behind the request's, the others' from zero; in the last one's place
+// the request's, which the second pass writes over) and the sum of its step sizes, of which exp(A sum) is the decay over the segment; the
+// second (SCAN_READ) begins with what the segments before it add up to and makes the read-outs.  Most of the arithmetic is
+// done twice, so with the blocks of four requests and more a scan stays whole.  2048 tokens, 4096 channels of 16 states, us, whole -> segments: one
+// request 371 -> 221 (195 with exp_rates), two 286 -> 250 (224); 288 tokens of one request 60 -> 49 (44), of two 49 -> 46 (43).
+enum ScanPass : int { SCAN_WHOLE = 0, SCAN_OWN = 1, SCAN_READ = 2 };
+// tokens per segment, segments per entry (grid y: entry by entry); own states [entry, segment][inner][nstate], sums of step sizes
+// [entry, segment][inner]
+struct ScanSegments { int tokens, count; float* own; float* dt; };
 __host__ __device__ constexpr int scan_tb(int np) { return np <= 64 ? 32 : np <= 128 ? 16 : 8; }
 __host__ __device__ constexpr size_t scan_smem(int np, int pb, size_t esz) {
   return 2 * (size_t)scan_tb(np) * (2 * (size_t)np * 4 + (size_t)pb * (4 + 2 * esz));
 }
 // vec: rows of B, C and dt (fp32) and of x, z may travel by 16-byte copies (bits 0 and 1; see launch_scan)
-template <typename AT, typename WT, int NPER, int L>
+template <typename AT, typename WT, int NPER, int L, int PASS>
 __global__ void __launch_bounds__(128) scan_kernel(Batch b, const AT* __restrict__ x, int ldx, const AT* __restrict__ z, int ldz,
                                                    const float* __restrict__ dt_raw, int lddt, const WT* __restrict__ dt_bias,
                                                    const float* __restrict__ low, int ldl, int col_b, int col_c,
                                                    const float* __restrict__ A, const WT* __restrict__ D, int inner, int nstate,
-                                                   int vec, float out_scale, float* __restrict__ state, AT* __restrict__ out, int ldo) {
+                                                   int vec, float out_scale, float* __restrict__ state, AT* __restrict__ out, int ldo, ScanSegments seg) {
   pdl_begin();
   constexpr int NP = NPER * L, PB = 128 / L, TB = scan_tb(NP), TG = 8, CH = 16 / (int)sizeof(AT);
   extern __shared__ __align__(16) unsigned char hy_smem[];
@@ -687,19 +723,52 @@ __global__ void __launch_bounds__(128) scan_kernel(Batch b, const AT* __restrict
   float* sdt = sC + 2 * TB * NP;                               // [2][TB][PB], step sizes once their batch has landed
   AT* sx = reinterpret_cast<AT*>(sdt + 2 * TB * PB);           // [2][TB][PB]
   AT* sz = sx + 2 * TB * PB;                                   // [2][TB][PB]
-  const int e = blockIdx.y, tid = threadIdx.x, c0 = blockIdx.x * PB;
+  const int e = PASS == SCAN_WHOLE ? blockIdx.y : blockIdx.y / seg.count, tid = threadIdx.x, c0 = blockIdx.x * PB;
   const int cl = tid / L, sub = tid % L, n0 = sub * NPER, c = c0 + cl;
   const bool live = c < inner;
   const int cc = live ? c : inner - 1, npb = min(PB, inner - c0);
-  const int start = b.ent_start[e], cnt = b.ent_start[e + 1] - start, pos0 = b.ent_pos0[e];
+  const int at = PASS == SCAN_WHOLE ? 0 : (int)blockIdx.y % seg.count, all = b.ent_start[e + 1] - b.ent_start[e], pos0 = b.ent_pos0[e];
+  const int start = b.ent_start[e] + (PASS == SCAN_WHOLE ? 0 : at * seg.tokens);
+  const int cnt = PASS == SCAN_WHOLE ? all : min(seg.tokens, all - at * seg.tokens);
+  const bool ends = PASS == SCAN_WHOLE || (at + 1) * seg.tokens >= all;          // the entry's last segment
+  if (cnt <= 0) return;
   float* st = state + ((size_t)b.ent_slot[e] * inner + cc) * nstate;
-  float S[NPER], a[NPER];
+  float2 S[NPER / 2];
+  RatePair a[NPER / 2];
+  auto from_rows = [&](const float* row, bool there) {         // this lane's states of a row of nstate
 #pragma unroll
-  for (int i = 0; i < NPER; ++i) {
-    const int n = n0 + i;
-    S[i] = (n < nstate && pos0 > 0) ? st[n] : 0.0f;
-    a[i] = n < nstate ? A[(size_t)cc * nstate + n] : 0.0f;
+    for (int i = 0; i < NPER; i += 2)
+      S[i / 2] = make_float2(there && n0 + i < nstate ? row[n0 + i] : 0.0f, there && n0 + i + 1 < nstate ? row[n0 + i + 1] : 0.0f);
+  };
+  auto to_rows = [&](float* row) {
+#pragma unroll
+    for (int i = 0; i < NPER; i += 2) {
+      if (n0 + i < nstate) row[n0 + i] = S[i / 2].x;
+      if (n0 + i + 1 < nstate) row[n0 + i + 1] = S[i / 2].y;
+    }
+  };
+  from_rows(st, PASS != SCAN_READ && (at == 0 || ends) && pos0 > 0);
+#pragma unroll
+  for (int i = 0; i < NPER; i += 2) {
+    const float* row = A + (size_t)cc * nstate;
+    a[i / 2] = RatePair(n0 + i < nstate ? row[n0 + i] : 0.0f, n0 + i + 1 < nstate ? row[n0 + i + 1] : 0.0f);
   }
+  if (PASS == SCAN_OWN && ends) {                              // what the request came with, for the first segment of the second pass
+    if (live) to_rows(seg.own + ((size_t)blockIdx.y * inner + c) * nstate);
+    return;
+  }
+  if constexpr (PASS == SCAN_READ) {
+    if (at == 0) from_rows(seg.own + ((size_t)(e * seg.count + (all - 1) / seg.tokens) * inner + cc) * nstate, true);
+    for (int k = 0; k < at; ++k) {
+      const size_t row = (size_t)(e * seg.count + k) * inner + cc;
+      const float dt = finite_step(seg.dt[row]);
+      const float* own = seg.own + row * nstate;
+#pragma unroll
+      for (int i = 0; i < NPER; i += 2)
+        S[i / 2] = fma2(exp_rates(dt, a[i / 2]), S[i / 2], make_float2(n0 + i < nstate ? own[n0 + i] : 0.0f, n0 + i + 1 < nstate ? own[n0 + i + 1] : 0.0f));
+    }
+  }
+  float dt_sum = 0.0f;
   const float dd = to_f(D[cc]);
   if (nstate < NP)                                             // states beyond the last stay zero
     for (int i = tid; i < 2 * TB * NP; i += 128) if (i % NP >= nstate) { sB[i] = 0.0f; sC[i] = 0.0f; }
@@ -715,7 +784,7 @@ __global__ void __launch_bounds__(128) scan_kernel(Batch b, const AT* __restrict
         const int r = i / nc, k = i % nc * 4;
         const float* src = low + (t0 + r) * ldl + k;
         jf::cp_async_16(db + r * NP + k, src + col_b, 16u);
-        jf::cp_async_16(dc + r * NP + k, src + col_c, 16u);
+        if (PASS != SCAN_OWN) jf::cp_async_16(dc + r * NP + k, src + col_c, 16u);
       }
       for (int i = tid; i < nb * nd; i += 128) jf::cp_async_16(dt + i / nd * PB + i % nd * 4, dt_raw + (t0 + i / nd) * lddt + c0 + i % nd * 4, 16u);
     } else {
@@ -733,7 +802,7 @@ __global__ void __launch_bounds__(128) scan_kernel(Batch b, const AT* __restrict
       for (int i = tid; i < nb * nx; i += 128) {
         const int r = i / nx, k = i % nx * CH;
         jf::cp_async_16(dx + r * PB + k, x + (t0 + r) * ldx + c0 + k, 16u);
-        jf::cp_async_16(dz + r * PB + k, z + (t0 + r) * ldz + c0 + k, 16u);
+        if (PASS != SCAN_OWN) jf::cp_async_16(dz + r * PB + k, z + (t0 + r) * ldz + c0 + k, 16u);
       }
     } else {
       for (int i = tid; i < nb * npb; i += 128) {
@@ -761,63 +830,83 @@ __global__ void __launch_bounds__(128) scan_kernel(Batch b, const AT* __restrict
     const AT* rz = sz + buf * TB * PB + ck;
     AT* po = out + (size_t)(start + j0) * ldo + cc;
     auto update = [&](int tt) {                                // one token; returns this lane's part of the read-out
-      const float dt = bdt[tt * PB + ck], dx = dt * to_f(rx[tt * PB]);
-      float y0 = 0.0f, y1 = 0.0f;
+      const float raw = bdt[tt * PB + ck], dx = raw * to_f(rx[tt * PB]), dt = finite_step(raw);
+      if constexpr (PASS == SCAN_OWN) dt_sum += raw;
+      float2 y = make_float2(0.0f, 0.0f);
 #pragma unroll
       for (int i = 0; i < NPER; i += 4) {
         const float4 bb = *reinterpret_cast<const float4*>(rb + tt * NP + i);
         const float4 cv = *reinterpret_cast<const float4*>(rc + tt * NP + i);
-        S[i] = fmaf(expf(dt * a[i]), S[i], dx * bb.x); y0 = fmaf(S[i], cv.x, y0);
-        S[i + 1] = fmaf(expf(dt * a[i + 1]), S[i + 1], dx * bb.y); y1 = fmaf(S[i + 1], cv.y, y1);
-        S[i + 2] = fmaf(expf(dt * a[i + 2]), S[i + 2], dx * bb.z); y0 = fmaf(S[i + 2], cv.z, y0);
-        S[i + 3] = fmaf(expf(dt * a[i + 3]), S[i + 3], dx * bb.w); y1 = fmaf(S[i + 3], cv.w, y1);
+        float2 &s0 = S[i / 2], &s1 = S[i / 2 + 1];
+        s0 = fma2(exp_rates(dt, a[i / 2]), s0, mul2(make_float2(dx, dx), make_float2(bb.x, bb.y)));
+        s1 = fma2(exp_rates(dt, a[i / 2 + 1]), s1, mul2(make_float2(dx, dx), make_float2(bb.z, bb.w)));
+        y = fma2(s0, make_float2(cv.x, cv.y), y);
+        y = fma2(s1, make_float2(cv.z, cv.w), y);
       }
-      return y0 + y1;
+      return y.x + y.y;
     };
     auto leave = [&](int tt, float y) {
       y = fmaf(dd, to_f(rx[tt * PB]), y);
       po[(size_t)tt * ldo] = from_f<AT>(y * silu_f(to_f(rz[tt * PB])) * out_scale);
     };
     int tt = 0;
-    for (; tt + TG <= nb; tt += TG) {
-      float p[TG];
+    if constexpr (PASS == SCAN_OWN) {
+#pragma unroll 4
+      for (; tt < nb; ++tt) update(tt);
+    } else {
+      for (; tt + TG <= nb; tt += TG) {
+        float p[TG];
 #pragma unroll
-      for (int u = 0; u < TG; ++u) p[u] = update(tt + u);
-      int n = TG, base = 0;
+        for (int u = 0; u < TG; ++u) p[u] = update(tt + u);
+        int n = TG, base = 0;
 #pragma unroll
-      for (int s = L >> 1; s >= 1; s >>= 1) {
-        const bool hi = (sub & s) != 0;
-        if (n > 1) {
-          n >>= 1;
+        for (int s = L >> 1; s >= 1; s >>= 1) {
+          const bool hi = (sub & s) != 0;
+          if (n > 1) {
+            n >>= 1;
 #pragma unroll
-          for (int u = 0; u < TG / 2; ++u) {
-            if (u >= n) break;
-            const float other = __shfl_xor_sync(0xffffffffu, hi ? p[u] : p[u + n], s);
-            p[u] = (hi ? p[u + n] : p[u]) + other;
+            for (int u = 0; u < TG / 2; ++u) {
+              if (u >= n) break;
+              const float other = __shfl_xor_sync(0xffffffffu, hi ? p[u] : p[u + n], s);
+              p[u] = (hi ? p[u + n] : p[u]) + other;
+            }
+            base += hi ? n : 0;
+          } else {
+            p[0] += __shfl_xor_sync(0xffffffffu, p[0], s);
           }
-          base += hi ? n : 0;
-        } else {
-          p[0] += __shfl_xor_sync(0xffffffffu, p[0], s);
+        }
+        constexpr int LEFT = TG > L ? TG / L : 1, SAME = L > TG ? L / TG : 1;        // tokens per lane, lanes per token
+        if (live && (sub & (SAME - 1)) == 0) {
+#pragma unroll
+          for (int u = 0; u < LEFT; ++u) leave(tt + base + u, p[u]);
         }
       }
-      constexpr int LEFT = TG > L ? TG / L : 1, SAME = L > TG ? L / TG : 1;        // tokens per lane, lanes per token
-      if (live && (sub & (SAME - 1)) == 0) {
+      for (; tt < nb; ++tt) {
+        float y = update(tt);
 #pragma unroll
-        for (int u = 0; u < LEFT; ++u) leave(tt + base + u, p[u]);
+        for (int s = L >> 1; s >= 1; s >>= 1) y += __shfl_xor_sync(0xffffffffu, y, s);
+        if (live && sub == 0) leave(tt, y);
       }
     }
-    for (; tt < nb; ++tt) {
-      float y = update(tt);
-#pragma unroll
-      for (int s = L >> 1; s >= 1; s >>= 1) y += __shfl_xor_sync(0xffffffffu, y, s);
-      if (live && sub == 0) leave(tt, y);
-    }
   }
-  if (live) {
-#pragma unroll
-    for (int i = 0; i < NPER; ++i)
-      if (n0 + i < nstate) st[n0 + i] = S[i];
+  if constexpr (PASS == SCAN_OWN) {
+    if (!live) return;
+    const size_t row = (size_t)blockIdx.y * inner + c;
+    if (sub == 0) seg.dt[row] = dt_sum;
+    to_rows(seg.own + row * nstate);
+    return;
   }
+  if (live && ends) to_rows(st);
+}
+
+// Segments of a scan: as many as give every SM SCAN_BLOCKS blocks, at least three of at least SCAN_SEG_TOKENS tokens.
+constexpr int SCAN_BLOCKS = 6, SCAN_SEG_TOKENS = 96;
+inline int scan_segment_rows(int blocks) { return 148 * SCAN_BLOCKS / (blocks < 1 ? 1 : blocks); }      // entries x segments at most
+inline ScanSegments scan_segments(float* own, int blocks, int entries, int longest, int inner, int nstate) {
+  const int fit = scan_segment_rows(blocks) / entries, n = fit < longest / SCAN_SEG_TOKENS ? fit : longest / SCAN_SEG_TOKENS;
+  if (n < 3) return ScanSegments{0, 1, nullptr, nullptr};
+  const int tokens = ((longest + n - 1) / n + 31) / 32 * 32, count = (longest + tokens - 1) / tokens;
+  return ScanSegments{tokens, count, own, own + (size_t)entries * count * inner * nstate};
 }
 
 // Sum of two values over the block in one pass (same order rules as block_sum).  red: >= 66 floats.

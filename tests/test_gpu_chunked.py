@@ -4,7 +4,7 @@ the padded ones (with and without 16-byte rows), several requests of a step, dec
 import numpy as np
 import pytest
 
-from oracle import famepel_plain, kisadra_plain, mafalorn_plain
+from oracle import famepel_plain, kinetar_plain, kisadra_plain, mafalorn_plain
 from tests import famepel_helpers as fam
 from tests import hybrid_helpers as kin
 from tests import kisadra_helpers as kis
@@ -81,3 +81,26 @@ def test_chunked_forget_gates_of_zero_and_one():
     finally:
         hz.close()
     assert helpers.close(got, helpers.oracle_logits(cfg, w, toks), "float32")
+
+
+@pytest.mark.parametrize("state,inner,rank", [(1, 300, 1), (5, 128, 4), (16, 64, 4), (17, 33, 2), (130, 8, 4)])
+def test_selective_scan_in_segments(state, inner, rank):
+    """Portions long enough for segments (three of 96 tokens and more), whole and with a rest, behind and before shorter ones; two requests of unlike
+    lengths in a step, of which the shorter has fewer segments."""
+    layer = kin.attn_scan(left_scale=0.0, inner=inner, state=state, dt_rank=rank)
+    layer["mlp"] = None
+    cfg = kin.model_config([layer])
+    w = kinetar_plain.random_weights(cfg, 0, 8)
+    cuts = [288, 5, 401, 40, 100]
+    toks = {k: kin.rand_tokens(n, cfg["vocab"], i) for i, (k, n) in enumerate({"a": sum(cuts), "b": 500, "c": 130}.items())}
+    hz = kin.Harness(cfg, w, num_pages=160, max_step_tokens=1280)
+    try:
+        got = {"a": hz.feed("a", toks["a"], cuts)}
+        first = hz.step([("b", toks["b"][:70], range(70)), ("c", toks["c"][:20], range(20))])
+        second = hz.step([("b", toks["b"][70:], range(430)), ("c", toks["c"][20:], range(110))])
+    finally:
+        hz.close()
+    got["b"] = np.concatenate([first[:70], second[:430]], 0)
+    got["c"] = np.concatenate([first[70:], second[430:]], 0)
+    for k in toks:
+        assert kin.rel_err(got[k], kin.oracle_logits(cfg, w, toks[k])) < kin.TOL["float32"], k
