@@ -27,6 +27,7 @@
 #include "hy_delta.cuh"
 #include "hy_gla.cuh"
 #include "hy_chunk.cuh"
+#include "hy_few.cuh"
 #include "jf_flash.cuh"
 
 namespace hy {
@@ -1586,6 +1587,15 @@ int gemm(hy_engine* h, const TA* A, int lda, const TW* Wt, int ldw, int T, int N
       return HY_OK;
     }
   }
+  if constexpr (std::is_same<TA, bf16>::value && std::is_same<TW, bf16>::value) {
+    if (few_pays(T, N, K) && few_takes(A, lda, Wt, ldw, T, K)) {
+      const int tiles = (N + 15) / 16, ksplit = few_ksplit(tiles, K), per = 8 / ksplit;
+      if (few_wide(tiles, K)) go_kernel(h, gemm_few_kernel<TO, 16>, tiles, 512, few_smem(K), h->stream, A, lda, Wt, ldw, T, N, K, 16, o);
+      else go_kernel(h, gemm_few_kernel<TO, 8>, std::min((tiles + per - 1) / per, 148 * 2), 256, few_smem(K), h->stream, A, lda, Wt, ldw, T, N, K, ksplit, o);
+      h->launches++;
+      return HY_OK;
+    }
+  }
   constexpr int VECW = 16 / (int)sizeof(TW);
   const size_t row_bytes = (size_t)((K + VECW - 1) / VECW * VECW) * sizeof(TA);
   const int want_rows = T == 1 ? 1 : T == 2 ? 2 : T <= 4 ? 4 : 8;
@@ -1594,8 +1604,7 @@ int gemm(hy_engine* h, const TA* A, int lda, const TW* Wt, int ldw, int T, int N
     while (ksplit < 8 && (long long)N * ksplit < 148LL * 32 && K / (ksplit * 2) >= 512) ksplit *= 2;
     const int cpb = 8 / ksplit;
     // Eight rows are 16 KB of operand and more to stage before a block's first product, so a warp takes several columns: at most 4 blocks per SM
-    // against 16, us behind a small kernel: N 2112, K 2048 16.9 and 19.5; N 1024, K 4096 26.1 and 31.6; N 32000, K 1024 56.7 and 55.6.  One row:
-    // no difference beyond 0.6 us but for N 32000 (20.2 and 18.5).
+    // against 16, us behind a small kernel: N 2112, K 2048 16.9 and 19.5; N 1024, K 4096 26.1 and 31.6.  One row: no difference beyond 0.6 us.
     const int blocks = std::min((N + cpb - 1) / cpb, 148 * (T > 4 ? 4 : 16));
     const int fit = (int)((200 * 1024) / row_bytes);
     auto launch = [&](auto kern, int rows) {
@@ -2050,6 +2059,35 @@ void place_rows(hy_engine* h, int T, const AT* hb, const LayerW& L, const hy_lay
   h->launches++;
 }
 
+// Whether the experts of a step run by expert over its pairs as they stand (up to eight tokens of a bf16 build), without the sorted order.
+template <typename AT>
+bool experts_few(const hy_engine* h, int T, const AT* hb, int lda, const LayerW& L, int W, int ff, int ldh) {
+  if (!std::is_same<AT, bf16>::value) return false;
+  return few_takes(hb, lda, L.w_gu, W, T, W) && few_takes(h->pin, ldh, L.w_down, ff, T, ff);
+}
+// Both products of a step's chosen experts with their rows in pair order: hb [T, width] -> h->pin [pairs, ff] -> ys [pairs, width].
+template <typename AT, bool GLU>
+void pair_order_experts(hy_engine* h, bool by_expert, const AT* hb, const LayerW& L, int P, int top, int NE, int ff, float* ys, int act, float limit) {
+  const int W = h->m.width, ldh = (ff + 7) & ~7;
+  AT* pin = (AT*)h->pin;
+  if constexpr (std::is_same<AT, bf16>::value) {
+    if (by_expert) {
+      auto go = [&](auto kernel, int tile, const bf16* A, int lda, int per_token, const void* Wt, size_t stride, int N, int K, auto* out, int ldo, int a, float l) {
+        const int tiles = (N + tile - 1) / tile, ksplit = few_ksplit((long long)tiles * std::min(NE, P), K), per = 8 / ksplit;
+        go_kernel(h, kernel, dim3((tiles + per - 1) / per, NE), 256, few_smem(K), h->stream, A, lda, h->x_ids, P, top, per_token, (const bf16*)Wt, stride, N, K,
+                  ksplit, out, ldo, a, l);
+      };
+      go(expert_few_kernel<bf16, GLU>, GLU ? 8 : 16, hb, W, 1, L.w_gu, (size_t)(GLU ? 2 : 1) * ff * W, ff, W, pin, ldh, act, limit);
+      go(expert_few_kernel<float, false>, 16, pin, ldh, 0, L.w_down, (size_t)W * ff, W, ff, ys, W, -1, 0.0f);
+      return;
+    }
+  }
+  go_kernel(h, expert_rows_kernel<AT, AT, AT, GLU>, dim3(std::min((ff + 7) / 8, 256), P), 256, (size_t)W * sizeof(AT), h->stream,
+      hb, W, h->x_ids, top, 1, NE, (const AT*)L.w_gu, (size_t)(GLU ? 2 : 1) * ff * W, ff, W, pin, ldh, act, limit);
+  go_kernel(h, expert_rows_kernel<AT, AT, float, false>, dim3(std::min((W + 7) / 8, 256), P), 256, (size_t)ff * sizeof(AT), h->stream,
+      pin, ldh, h->x_ids, top, 0, NE, (const AT*)L.w_down, (size_t)W * ff, W, ff, ys, W, -1, 0.0f);
+}
+
 // One layer of a norm - sublayer - norm model:  x += ls1 * n1b(mixer(n1(x)));  x += ls2 * n2b(experts(n2(x))).
 // The output norms are element-wise, so they run in the epilogue of the mixer's output projection and in the experts'
 // combine kernel, on the fp32 accumulators, together with the layer scale and the residual sum.
@@ -2146,7 +2184,7 @@ int sandwich_layer(hy_engine* h, const Batch& b, size_t li) {
   // a handful of pairs: one block row per pair; beyond that the sorted order, where pairs that share an expert share its
   // stream (measured at 8 tokens x 4 experts of 32: the tensor-core product over the sorted order is 2.5 - 5 times faster)
   static const int rows_max_env = getenv("HY_EXPERT_ROWS_MAX") ? atoi(getenv("HY_EXPERT_ROWS_MAX")) : -1;   // developer switch
-  const bool few = P <= (rows_max_env >= 0 ? rows_max_env : tc_experts ? 8 : 16);
+  const bool by_expert = rows_max_env < 0 && experts_few<AT>(h, T, hb, W, L, W, ff, ldh), few = by_expert || P <= (rows_max_env >= 0 ? rows_max_env : tc_experts ? 8 : 16);
   {
     ProfScope ps(h, HY_PROF_ROUTE);
     gemm<AT, WT, float>(h, hb, W, (const WT*)L.w_router, W, T, NE, W, to_buf(h->f1, h->ld_f1), L.w_router_t);
@@ -2161,10 +2199,7 @@ int sandwich_layer(hy_engine* h, const Batch& b, size_t li) {
     ProfScope ps(h, HY_PROF_EXPERTS);
     float* ys = h->f2;                                        // [pairs, width] fp32
     if (few) {
-      go_kernel(h, expert_rows_kernel<AT, WT, AT, true>, dim3(std::min((ff + 7) / 8, 256), P), 256, (size_t)W * sizeof(AT), s, 
-          hb, W, h->x_ids, top, 1, NE, (const WT*)L.w_gu, (size_t)2 * ff * W, ff, W, pin, ldh, 0, 0.0f);
-      go_kernel(h, expert_rows_kernel<AT, WT, float, false>, dim3(std::min((W + 7) / 8, 256), P), 256, (size_t)ff * sizeof(AT), s, 
-          pin, ldh, h->x_ids, top, 0, NE, (const WT*)L.w_down, (size_t)W * ff, W, ff, ys, W, -1, 0.0f);
+      pair_order_experts<AT, true>(h, by_expert, hb, L, P, top, NE, ff, ys, 0, 0.0f);
     } else if (tc_experts) {
       if constexpr (std::is_same<AT, bf16>::value) {
         const jf::TpGroup grp{h->x_meta, h->x_offs, h->x_tile_e, h->x_tile_r0, 0};
@@ -2327,7 +2362,7 @@ int postnorm_layer(hy_engine* h, const Batch& b, size_t li) {
   AT* x_rows = (AT*)h->x_rows;
   const bool tc_experts = std::is_same<AT, bf16>::value && L.w_gu_t != nullptr;
   static const int rows_max_env = getenv("HY_EXPERT_ROWS_MAX") ? atoi(getenv("HY_EXPERT_ROWS_MAX")) : -1;   // developer switch
-  const bool few = P <= (rows_max_env >= 0 ? rows_max_env : tc_experts ? 8 : 16);
+  const bool by_expert = rows_max_env < 0 && experts_few<AT>(h, T, hb, W, L, W, ff, ldh), few = by_expert || P <= (rows_max_env >= 0 ? rows_max_env : tc_experts ? 8 : 16);
   {
     ProfScope ps(h, HY_PROF_ROUTE);
     gemm<AT, WT, float>(h, hb, W, (const WT*)L.w_router, W, T, NE, W, to_buf(h->f1, h->ld_f1), L.w_router_t);
@@ -2347,10 +2382,7 @@ int postnorm_layer(hy_engine* h, const Batch& b, size_t li) {
   {
     ProfScope ps(h, HY_PROF_EXPERTS);
     if (few) {
-      go_kernel(h, expert_rows_kernel<AT, WT, AT, false>, dim3(std::min((ff + 7) / 8, 256), P), 256, (size_t)W * sizeof(AT), s, 
-          hb, W, h->x_ids, top, 1, NE, (const WT*)L.w_gu, (size_t)ff * W, ff, W, pin, ldh, c.x_act, c.ff_limit);
-      go_kernel(h, expert_rows_kernel<AT, WT, float, false>, dim3(std::min((W + 7) / 8, 256), P), 256, (size_t)ff * sizeof(AT), s, 
-          pin, ldh, h->x_ids, top, 0, NE, (const WT*)L.w_down, (size_t)W * ff, W, ff, ys, W, -1, 0.0f);
+      pair_order_experts<AT, false>(h, by_expert, hb, L, P, top, NE, ff, ys, c.x_act, c.ff_limit);
     } else if (tc_experts) {
       if constexpr (std::is_same<AT, bf16>::value) {
         const jf::TpGroup grp{h->x_meta, h->x_offs, h->x_tile_e, h->x_tile_r0, 0};
@@ -2394,7 +2426,7 @@ bool routed_gated_experts(hy_engine* h, int T, const AT* hb, const LayerW& L, co
   const int NE = c.x_experts, top = c.x_top, ff = c.ff, P = T * top, ldh = (ff + 7) & ~7;
   AT* x_rows = (AT*)h->x_rows;
   const bool tc_experts = std::is_same<AT, bf16>::value && L.w_gu_t != nullptr;
-  const bool few = P <= (tc_experts ? 8 : 16);
+  const bool by_expert = experts_few<AT>(h, T, hb, W, L, W, ff, ldh), few = by_expert || P <= (tc_experts ? 8 : 16);
   {
     ProfScope ps(h, HY_PROF_ROUTE);
     if (c.x_route == HY_ROUTE_CORRECTED_SOFTMAX) {
@@ -2414,10 +2446,7 @@ bool routed_gated_experts(hy_engine* h, int T, const AT* hb, const LayerW& L, co
   ProfScope ps(h, HY_PROF_EXPERTS);
   float* ys = h->f2;
   if (few) {
-    go_kernel(h, expert_rows_kernel<AT, WT, AT, true>, dim3(std::min((ff + 7) / 8, 256), P), 256, (size_t)W * sizeof(AT), s, 
-        hb, W, h->x_ids, top, 1, NE, (const WT*)L.w_gu, (size_t)2 * ff * W, ff, W, pin, ldh, c.x_act, c.ff_limit);
-    go_kernel(h, expert_rows_kernel<AT, WT, float, false>, dim3(std::min((W + 7) / 8, 256), P), 256, (size_t)ff * sizeof(AT), s, 
-        pin, ldh, h->x_ids, top, 0, NE, (const WT*)L.w_down, (size_t)W * ff, W, ff, ys, W, -1, 0.0f);
+    pair_order_experts<AT, true>(h, by_expert, hb, L, P, top, NE, ff, ys, c.x_act, c.ff_limit);
   } else if (tc_experts) {
     if constexpr (std::is_same<AT, bf16>::value) {
       const jf::TpGroup grp{h->x_meta, h->x_offs, h->x_tile_e, h->x_tile_r0, 0};
