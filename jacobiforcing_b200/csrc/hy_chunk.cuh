@@ -254,19 +254,21 @@ __host__ __device__ constexpr size_t ch_out_smem() {
 
 // Weights of pairs inside one sub-block, decays per channel: half a warp takes key j of the sub-block, a lane 4 or 8 of its channels, and the
 // running product k_j a_j+1 .. a_i meets the queries i = j .. 15; the sixteen sums are then exchanged so that lane i keeps that of query i.
-template <int DK, bool FORGET>
-__device__ __forceinline__ float ch_pairs(const float* sq, const float* sk, const float* sd, int s, int j, int jw, int l) {
+// TWO: and with the keys in the queries' place (w2).
+template <int DK, bool FORGET, bool TWO = false>
+__device__ __forceinline__ float ch_pairs(const float* sq, const float* sk, const float* sd, int s, int j, int jw, int l, float* w2 = nullptr) {
   constexpr int NC = DK / 64;
-  float p[CH_SUB];
+  float p[CH_SUB], p2[TWO ? CH_SUB : 1];
   float2 w[2 * NC];
 #pragma unroll
   for (int c = 0; c < 2 * NC; ++c) w[c] = make_float2(0.0f, 0.0f);
 #pragma unroll
   for (int i = 0; i < CH_SUB; ++i) {
     p[i] = 0.0f;
+    if constexpr (TWO) p2[i] = 0.0f;
     if (i < CH_SUB / 2 && jw >= CH_SUB / 2) continue;          // the same for the whole warp
     const int r = s * CH_SUB + i;
-    float2 sum = make_float2(0.0f, 0.0f);
+    float2 sum = make_float2(0.0f, 0.0f), sum2 = sum;
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
       const int at = ch_at<DK, true>(r, c * 64 + l * 4);
@@ -279,28 +281,39 @@ __device__ __forceinline__ float ch_pairs(const float* sq, const float* sk, cons
       }
       sum = fma2(w[2 * c], make_float2(q.x, q.y), sum);
       sum = fma2(w[2 * c + 1], make_float2(q.z, q.w), sum);
+      if constexpr (TWO) {
+        const float4 k = *reinterpret_cast<const float4*>(sk + at);
+        sum2 = fma2(w[2 * c], make_float2(k.x, k.y), sum2);
+        sum2 = fma2(w[2 * c + 1], make_float2(k.z, k.w), sum2);
+      }
     }
     p[i] = sum.x + sum.y;
+    if constexpr (TWO) p2[i] = sum2.x + sum2.y;
   }
-  int n = CH_SUB;
+  auto exchange = [&](float* v) {
+    int n = CH_SUB;
 #pragma unroll
-  for (int x = 8; x >= 1; x >>= 1) {
-    n >>= 1;
-    const bool hi = (l & x) != 0;
+    for (int x = 8; x >= 1; x >>= 1) {
+      n >>= 1;
+      const bool hi = (l & x) != 0;
 #pragma unroll
-    for (int u = 0; u < CH_SUB / 2; ++u) {
-      if (u >= n) break;
-      const float other = __shfl_xor_sync(0xffffffffu, hi ? p[u] : p[u + n], x);
-      p[u] = (hi ? p[u + n] : p[u]) + other;
+      for (int u = 0; u < CH_SUB / 2; ++u) {
+        if (u >= n) break;
+        const float other = __shfl_xor_sync(0xffffffffu, hi ? v[u] : v[u + n], x);
+        v[u] = (hi ? v[u + n] : v[u]) + other;
+      }
     }
-  }
+  };
+  exchange(p);
+  if constexpr (TWO) { exchange(p2); *w2 = p2[0]; }
   return p[0];                                                 // of query l
 }
 
 // Weights of the queries of sub-block I and the keys of the sub-blocks before it: x [i][d] . y [j][d], both carried to I's beginning.  A thread
 // takes 4 queries x I keys over a quarter of the channels; the quarters meet by shuffles.
-template <int DK>
-__device__ __forceinline__ void ch_block_row(const float* x, const float* y, float* w, int I) {
+// put(query of the chunk, sub-block of the key, key of the sub-block, weight).
+template <int DK, typename Put>
+__device__ __forceinline__ void ch_block_row(const float* x, const float* y, int I, Put put) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, dg = lane >> 3, jt = (warp & 1) * 8 + (lane & 7), i0 = I * CH_SUB + (warp >> 1) * 4;
   float2 acc[4][3] = {};
 #pragma unroll 2
@@ -331,7 +344,7 @@ __device__ __forceinline__ void ch_block_row(const float* x, const float* y, flo
       s += __shfl_xor_sync(0xffffffffu, s, 16);
       if (i == dg) mine = s;
     }
-    w[(i0 + dg) * CH_T + jj * CH_SUB + jt] = mine;
+    put(i0 + dg, jj, jt, mine);
   }
 }
 
@@ -430,7 +443,7 @@ __global__ void __launch_bounds__(256, 2) gla_chunk_out_kernel(ChunkArgs<AT> a) 
         }
         __syncthreads();
       }
-      ch_block_row<DK>(sq, sk, sw, I);
+      ch_block_row<DK>(sq, sk, I, [&](int i, int J, int j, float v) { sw[i * CH_T + J * CH_SUB + j] = v; });
       __syncthreads();
     }
     if (!first) {                                              // queries from the chunk's beginning
@@ -587,12 +600,355 @@ __global__ void __launch_bounds__(256, 2) gla_chunk_out_kernel(ChunkArgs<AT> a) 
   }
 }
 
+// ---- the delta rule -------------------------------------------------------------------------------------------------------------------
+// S <- a S ;  u = beta (v - S^T k) ;  S <- S + k u^T ;  o = S^T q  (hy_delta.cuh).  Within a chunk, with K' = k carried from the chunk's beginning, the
+// corrections u solve a unit lower triangular system,  (I + M) U = beta (V - K' S),  M_ij = beta_i (k_i . a_j+1 .. a_i . k_j),  so
+//   U = U0 - W S   with (I + M) [W | U0] = beta [K' | V]        and then as above        S' = diag(a_0 .. a_63) S + k''^T U,   O = Q' S + A U.
+// delta_chunk_prep_kernel makes W, U0, Q', k'', A and the decays' product of all chunks side by side; delta_chunk_chain_kernel walks the chunks of
+// a head, 16 columns per block (columns do not meet).  |u| stays within beta times the state, so the system's solution does not grow.  One
+// decay per head is taken as the same for all channels.
+// The chain: what a chunk brings travels in two halves while the other half is worked on.  5.9 us a chunk, bound by reading operands from shared memory
+// (eight 16-byte reads for 32 fma.rn.f32x2): products with the state 5000 of 11300 cycles, corrections of the state 4400, starting copies 1600.
+// 2048 tokens, 16 heads of 128 x 128 with channel decays: 430 us token by token; prep 131 and chain 190.
+template <typename AT>
+struct DeltaArgs {
+  Batch b;
+  const float* qk; const AT* v; int ldv; const float4* sc; const float* dec; int ldd;      // as delta_head_kernel's; dec NULL: one decay per head in sc
+  int H, G, dim, vdim, vec;
+  float* work; float* state; float* o; int ldo;
+};
+// Floats of a chunk and head: W | Q' | k'' (rows in pairs, [32][DK][2]) | U0 | A | decays' product.
+template <int DK, int DV>
+struct DeltaWork {
+  static constexpr int W = 0, Q = CH_T * DK, K = 2 * CH_T * DK, U = 3 * CH_T * DK, A = U + CH_T * DV, E = A + CH_T * CH_T, SIZE = E + DK;
+};
+__host__ __device__ constexpr size_t delta_work_floats(int dk, int dv) { return (size_t)3 * CH_T * dk + (size_t)CH_T * dv + CH_T * CH_T + dk; }
+
+// M of the sub-blocks (I, J <= I), [key][query] each.
+__device__ __forceinline__ int ch_tri(int I, int J) { return (I * (I + 1) / 2 + J) * CH_SUB * CH_SUB; }
+template <int DK, int DV>
+__host__ __device__ constexpr size_t delta_prep_smem() {
+  const size_t y = (size_t)CH_T * (DK + DV) * 4, qk = 2 * (size_t)CH_T * DK * 4;
+  return (y > qk ? y : qk) + ((size_t)CH_T * DK + 10 * CH_SUB * CH_SUB + CH_SUBS * DK + CH_T) * 4;
+}
+// grid (chunks, H), 256 threads.
+template <typename AT, int DK, int DV>
+__global__ void __launch_bounds__(256, 2) delta_chunk_prep_kernel(DeltaArgs<AT> a) {
+  pdl_begin();
+  typedef DeltaWork<DK, DV> Work;
+  extern __shared__ __align__(16) unsigned char hy_smem[];
+  float* sq = reinterpret_cast<float*>(hy_smem);               // [64][DK] queries | [64][DK] keys, at last the solution [64][DK + DV]
+  float* sk = sq + CH_T * DK;
+  float* sd = sq + (DK + DV > 2 * DK ? CH_T * (DK + DV) : 2 * CH_T * DK);      // [64][DK] decays, then keys from their sub-block's beginning
+  float* sm = sd + CH_T * DK;                                  // M
+  float* se = sm + 10 * CH_SUB * CH_SUB;                       // [4][DK] products of a sub-block's decays
+  float* sb = se + CH_SUBS * DK;                               // [64] step sizes
+  const ChunkPlace p(a.b, blockIdx.x);
+  const int h = blockIdx.y, g = h / (a.H / a.G), tid = threadIdx.x, warp = tid >> 5;
+  const float* rows = a.qk + ((size_t)p.t0 * a.G + g) * 2 * a.dim;
+  const size_t ld = (size_t)a.G * 2 * a.dim;
+  ch_rows<DK, true>(sq, rows, ld, p.n, a.dim, a.vec, 0.0f);
+  ch_rows<DK, true>(sk, rows + a.dim, ld, p.n, a.dim, a.vec, 0.0f);
+  if (a.dec) ch_rows<DK, true>(sd, a.dec + (size_t)p.t0 * a.ldd + h * a.dim, a.ldd, p.n, a.dim, a.vec, 1.0f);
+  if (tid < CH_T) {
+    const float4 sc = tid < p.n ? a.sc[(size_t)(p.t0 + tid) * a.H + h] : make_float4(1.0f, 0.0f, 0.0f, 0.0f);
+    sb[tid] = sc.y;
+    se[tid] = sc.x;
+  }
+  if (!a.dec) {
+    __syncthreads();
+    for (int i = tid; i < CH_T * DK; i += 256) sd[i] = se[i / DK];
+  }
+  jf::cp_async_commit();
+  jf::cp_async_wait_all();
+  __syncthreads();
+  float* work = a.work + ((size_t)blockIdx.x * a.H + h) * Work::SIZE;
+  const int l = tid & 15, hw = tid >> 4;
+#pragma unroll 1
+  for (int s = 0; s < CH_SUBS; ++s) {                          // weights inside a sub-block: (query l, key j)
+    const int j = s & 1 ? 15 - hw : hw, jw = s & 1 ? 14 - 2 * warp : 2 * warp;
+    float m;
+    const float w = ch_pairs<DK, false, true>(sq, sk, sd, s, j, jw, l, &m);
+    work[Work::A + (s * CH_SUB + l) * CH_T + s * CH_SUB + j] = w;
+    sm[ch_tri(s, s) + j * CH_SUB + l] = l > j ? m * sb[s * CH_SUB + l] : 0.0f;
+    for (int J = s + 1; J < CH_SUBS; ++J) work[Work::A + (s * CH_SUB + l) * CH_T + J * CH_SUB + j] = 0.0f;      // what a query does not see
+  }
+  __syncthreads();
+  for (int i = tid; i < CH_SUBS * DK; i += 256) {              // queries and keys from their sub-block's beginning, keys to its end
+    const int s = i / DK, d = i % DK;
+    float w = 1.0f, dec[CH_SUB], key[CH_SUB];
+#pragma unroll
+    for (int t = 0; t < CH_SUB; ++t) {
+      const int at = ch_at<DK, true>(s * CH_SUB + t, d);
+      dec[t] = sd[at]; key[t] = sk[at];
+      w *= dec[t];
+      sq[at] *= w;
+      sd[at] = key[t] * w;
+    }
+    se[i] = w;
+    w = 1.0f;
+#pragma unroll
+    for (int t = CH_SUB - 1; t >= 0; --t) {
+      sk[ch_at<DK, true>(s * CH_SUB + t, d)] = key[t] * w;
+      w *= dec[t];
+    }
+  }
+  __syncthreads();
+#pragma unroll 1
+  for (int I = 1; I < CH_SUBS; ++I) {
+    if (I > 1) {                                               // keys of the earlier sub-blocks: on over sub-block I - 1
+      for (int i = tid; i < (I - 1) * CH_SUB * DK; i += 256) sk[ch_at<DK, true>(i / DK, i % DK)] *= se[(I - 1) * DK + i % DK];
+      __syncthreads();
+    }
+    ch_block_row<DK>(sq, sk, I, [&](int i, int J, int j, float v) { work[Work::A + i * CH_T + J * CH_SUB + j] = v; });
+    ch_block_row<DK>(sd, sk, I, [&](int i, int J, int j, float v) { sm[ch_tri(I, J) + j * CH_SUB + i - I * CH_SUB] = v * sb[i]; });
+    __syncthreads();
+  }
+  {                                                            // from the chunk's beginning and to its end
+    constexpr int PER = 256 / DK;
+    const int d = tid % DK;
+    const float last = se[(CH_SUBS - 1) * DK + d];
+    float w = 1.0f;
+#pragma unroll
+    for (int I = 0; I < CH_SUBS; ++I) {
+#pragma unroll
+      for (int r = 0; r < CH_SUB / PER; ++r) {
+        const int row = I * CH_SUB + r * PER + tid / DK, at = ch_at<DK, true>(row, d);
+        work[Work::Q + row * DK + d] = sq[at] * w;
+        sd[at] *= w;
+        work[Work::K + (row >> 1) * 2 * DK + 2 * d + (row & 1)] = sk[at] * (I < CH_SUBS - 1 ? last : 1.0f);
+      }
+      w *= se[I * DK + d];
+    }
+    if (tid < DK) work[Work::E + d] = w;
+  }
+  __syncthreads();
+  // (I + M) Y = beta [K' | V], a column per thread; what is solved stays in shared memory for the sub-blocks behind it
+  for (int c = tid; c < DK + DV; c += 256) {
+    float* y = sq + c;
+    constexpr int LD = DK + DV;
+#pragma unroll 1
+    for (int I = 0; I < CH_SUBS; ++I) {
+      float2 r[CH_SUB / 2];
+#pragma unroll
+      for (int t = 0; t < CH_SUB; ++t) {
+        const int row = I * CH_SUB + t;
+        float x;
+        if (c < DK) x = sd[ch_at<DK, true>(row, c)];
+        else x = row < p.n && c - DK < a.vdim ? to_f(a.v[(size_t)(p.t0 + row) * a.ldv + h * a.vdim + c - DK]) : 0.0f;
+        (t & 1 ? r[t / 2].y : r[t / 2].x) = x * sb[row];
+      }
+#pragma unroll 1
+      for (int J = 0; J < I; ++J) {
+        const float* m = sm + ch_tri(I, J);
+#pragma unroll 4
+        for (int j = 0; j < CH_SUB; ++j) {
+          const float u = -y[(J * CH_SUB + j) * LD];
+#pragma unroll
+          for (int t = 0; t < CH_SUB / 4; ++t) {
+            const float4 mm = *reinterpret_cast<const float4*>(m + j * CH_SUB + 4 * t);
+            r[2 * t] = fma2(make_float2(mm.x, mm.y), make_float2(u, u), r[2 * t]);
+            r[2 * t + 1] = fma2(make_float2(mm.z, mm.w), make_float2(u, u), r[2 * t + 1]);
+          }
+        }
+      }
+      const float* m = sm + ch_tri(I, I);
+#pragma unroll
+      for (int j = 0; j < CH_SUB; ++j) {
+        const float u = j & 1 ? r[j / 2].y : r[j / 2].x;
+#pragma unroll
+        for (int t = j / 4; t < CH_SUB / 4; ++t) {             // the diagonal and above: zeros
+          const float4 mm = *reinterpret_cast<const float4*>(m + j * CH_SUB + 4 * t);
+          r[2 * t] = fma2(make_float2(mm.x, mm.y), make_float2(-u, -u), r[2 * t]);
+          r[2 * t + 1] = fma2(make_float2(mm.z, mm.w), make_float2(-u, -u), r[2 * t + 1]);
+        }
+      }
+#pragma unroll
+      for (int t = 0; t < CH_SUB; ++t) {
+        const int row = I * CH_SUB + t;
+        const float x = t & 1 ? r[t / 2].y : r[t / 2].x;
+        y[row * LD] = x;
+        work[c < DK ? Work::W + row * DK + c : Work::U + row * DV + c - DK] = x;
+      }
+    }
+  }
+}
+
+// Columns of a block of the chain, and its shared memory: W and Q' (chunks of 16 bytes xor the row's low bits), k'' and A, U0, the state and the
+// corrections with rows in pairs, sums of the second half of the channels.
+constexpr int DELTA_COLS = 16;
+template <int DK>
+__host__ __device__ constexpr size_t delta_chain_smem() {
+  return ((size_t)3 * CH_T * DK + CH_T * CH_T + CH_T * DELTA_COLS + DK * DELTA_COLS + CH_T * DELTA_COLS + 128 * DELTA_COLS) * 4;
+}
+// grid (H * DV / 16, entries), 256 threads.
+template <typename AT, int DK, int DV>
+__global__ void __launch_bounds__(256) delta_chunk_chain_kernel(DeltaArgs<AT> a) {
+  pdl_begin();
+  typedef DeltaWork<DK, DV> Work;
+  constexpr int C = DELTA_COLS;
+  extern __shared__ __align__(16) unsigned char hy_smem[];
+  float* swq = reinterpret_cast<float*>(hy_smem);              // [128][DK]
+  float* skk = swq + 2 * CH_T * DK;                            // [32][DK][2]
+  float* sA = skk + CH_T * DK;                                 // [64][64]
+  float* su0 = sA + CH_T * CH_T;                               // [64][16]
+  float* sS = su0 + CH_T * C;                                  // [DK / 2][16][2]
+  float* sU = sS + DK * C;                                     // [32][16][2]
+  float* sr = sU + CH_T * C;                                   // [128][16]
+  const int e = blockIdx.y, h = blockIdx.x / (DV / C), c0 = blockIdx.x % (DV / C) * C, tid = threadIdx.x;
+  if (c0 >= a.vdim) return;
+  const int start = a.b.ent_start[e], cnt = a.b.ent_start[e + 1] - start, n = (cnt + CH_T - 1) / CH_T;
+  int chunk = 0;
+  for (int f = 0; f < e; ++f) chunk += (a.b.ent_start[f + 1] - a.b.ent_start[f] + CH_T - 1) / CH_T;
+  float* st = a.state + ((size_t)a.b.ent_slot[e] * a.H + h) * a.dim * a.vdim;
+  for (int i = tid; i < DK * C; i += 256) {
+    const int d = i / C, c = i % C;
+    sS[(d >> 1) * 2 * C + 2 * c + (d & 1)] = d < a.dim && c0 + c < a.vdim && a.b.ent_pos0[e] > 0 ? st[(size_t)d * a.vdim + c0 + c] : 0.0f;
+  }
+  const float* work = a.work + ((size_t)chunk * a.H + h) * Work::SIZE;
+  const size_t step = (size_t)a.H * Work::SIZE;
+  auto first_half = [&](const float* w) {
+    for (int i = tid; i < 2 * CH_T * (DK / 4); i += 256) {
+      const int r = i / (DK / 4), c = i % (DK / 4);
+      jf::cp_async_16(swq + r * DK + ((c ^ (r & 7)) << 2), w + Work::W + r * DK + 4 * c, 16u);
+    }
+    jf::cp_async_16(su0 + tid * 4, w + Work::U + (tid >> 2) * DV + c0 + (tid & 3) * 4, 16u);
+    jf::cp_async_commit();
+  };
+  auto second_half = [&](const float* w) {
+    for (int i = tid; i < CH_T * DK / 4; i += 256) jf::cp_async_16(skk + 4 * i, w + Work::K + 4 * i, 16u);
+    for (int i = tid; i < CH_T * CH_T / 4; i += 256) {
+      const int r = i / 16, c = i % 16;
+      jf::cp_async_16(sA + r * CH_T + ((c ^ (r & 7)) << 2), w + Work::A + 4 * i, 16u);
+    }
+    jf::cp_async_commit();
+  };
+  first_half(work);
+  second_half(work);
+  const int kh = tid >> 7, rg = (tid & 127) >> 2, cg = (tid & 3) * 4;
+#pragma unroll 1
+  for (int j = 0; j < n; ++j, work += step) {
+    jf::cp_async_wait_1();                                     // the second half of this chunk may still travel
+    __syncthreads();
+    float2 acc[4][4] = {};                                     // rows rg + 32 i of W and Q' times columns cg .. + 3 of the state, half of its channels
+#pragma unroll 4
+    for (int k = kh * (DK / 2); k < (kh + 1) * (DK / 2); k += 4) {
+      VecN<float, 4> s[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) s[i] = *reinterpret_cast<const VecN<float, 4>*>(sS + (k / 2 + (i >> 1)) * 2 * C + 2 * cg + (i & 1) * 4);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float4 w = *reinterpret_cast<const float4*>(swq + (rg + 32 * i) * DK + (((k >> 2) ^ (rg & 7)) << 2));
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          acc[i][c] = fma2(make_float2(w.x, w.y), make_float2(s[c / 2].v[2 * (c & 1)], s[c / 2].v[2 * (c & 1) + 1]), acc[i][c]);
+          acc[i][c] = fma2(make_float2(w.z, w.w), make_float2(s[2 + c / 2].v[2 * (c & 1)], s[2 + c / 2].v[2 * (c & 1) + 1]), acc[i][c]);
+        }
+      }
+    }
+    if (kh) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        *reinterpret_cast<float4*>(sr + (rg + 32 * i) * C + cg) = make_float4(acc[i][0].x + acc[i][0].y, acc[i][1].x + acc[i][1].y, acc[i][2].x + acc[i][2].y, acc[i][3].x + acc[i][3].y);
+    }
+    __syncthreads();
+    float out[2][4];                                           // Q' S of rows rg and rg + 32
+    if (!kh) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int r = rg + 32 * i;
+        const float4 more = *reinterpret_cast<const float4*>(sr + r * C + cg);
+        const float m[4] = {more.x, more.y, more.z, more.w};
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const float v = acc[i][c].x + acc[i][c].y + m[c];
+          if (i < 2) sU[(r >> 1) * 2 * C + 2 * (cg + c) + (r & 1)] = su0[r * C + cg + c] - v;
+          else out[i - 2][c] = v;
+        }
+      }
+    }
+    __syncthreads();
+    if (j + 1 < n) { first_half(work + step); jf::cp_async_wait_1(); }
+    else jf::cp_async_wait_all();
+    __syncthreads();                                           // the second half of this chunk is there
+    if (!kh) {
+      float2 o2[2][4] = {};
+      const int stop = rg + 32;
+#pragma unroll 2
+      for (int t = 0; t <= stop; t += 4) {
+        VecN<float, 4> u[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) u[i] = *reinterpret_cast<const VecN<float, 4>*>(sU + (t / 2 + (i >> 1)) * 2 * C + 2 * cg + (i & 1) * 4);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const float4 w = *reinterpret_cast<const float4*>(sA + (rg + 32 * i) * CH_T + (((t >> 2) ^ (rg & 7)) << 2));
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            o2[i][c] = fma2(make_float2(w.x, w.y), make_float2(u[c / 2].v[2 * (c & 1)], u[c / 2].v[2 * (c & 1) + 1]), o2[i][c]);
+            o2[i][c] = fma2(make_float2(w.z, w.w), make_float2(u[2 + c / 2].v[2 * (c & 1)], u[2 + c / 2].v[2 * (c & 1) + 1]), o2[i][c]);
+          }
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int t = j * CH_T + rg + 32 * i;
+        if (t >= cnt) continue;
+        float* po = a.o + (size_t)(start + t) * a.ldo + h * a.vdim + c0 + cg;
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+          if (c0 + cg + c < a.vdim) po[c] = out[i][c] + (o2[i][c].x + o2[i][c].y);
+      }
+    } else {
+#pragma unroll 1
+      for (int d = rg * 4; d < DK; d += 128) {                 // four channels x four columns of the state
+        float2 up[4][4] = {};
+#pragma unroll 4
+        for (int t = 0; t < CH_T / 2; ++t) {
+          const VecN<float, 4> k0 = *reinterpret_cast<const VecN<float, 4>*>(skk + t * 2 * DK + 2 * d), k1 = *reinterpret_cast<const VecN<float, 4>*>(skk + t * 2 * DK + 2 * d + 4);
+          const VecN<float, 4> u0 = *reinterpret_cast<const VecN<float, 4>*>(sU + t * 2 * C + 2 * cg), u1 = *reinterpret_cast<const VecN<float, 4>*>(sU + t * 2 * C + 2 * cg + 4);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const VecN<float, 4>& k = i < 2 ? k0 : k1;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              const VecN<float, 4>& u = c < 2 ? u0 : u1;
+              up[i][c] = fma2(make_float2(k.v[2 * (i & 1)], k.v[2 * (i & 1) + 1]), make_float2(u.v[2 * (c & 1)], u.v[2 * (c & 1) + 1]), up[i][c]);
+            }
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float w = __ldg(work + Work::E + d + i);
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            float& S = sS[((d + i) >> 1) * 2 * C + 2 * (cg + c) + ((d + i) & 1)];
+            S = fmaf(w, S, up[i][c].x + up[i][c].y);
+          }
+        }
+      }
+    }
+    __syncthreads();                                           // state and second half are done with
+    if (j + 1 < n) second_half(work + step);
+  }
+  for (int i = tid; i < DK * C; i += 256) {
+    const int d = i / C, c = i % C;
+    if (d < a.dim && c0 + c < a.vdim) st[(size_t)d * a.vdim + c0 + c] = sS[(d >> 1) * 2 * C + 2 * c + (d & 1)];
+  }
+}
+
 // ---- host: which recurrences run in chunks, in which steps (see step_chunks) ------------------------------------------------------------
 // From 512 tokens of the longest request on: three launches and a block's own time cost 40 us, the chain of tokens 0.1 us each.  Token by token and in
 // chunks, us: 8 heads with forget gates 512 tokens 66 and 62, 384 tokens 53 and 61; state space 512 tokens 78 and 61; gated linear, 16 heads, 512
 // tokens 97 and 75, 320 tokens 70 and 71.  Key and value sizes up to 32 have too little work per chunk for it.
 constexpr int HY_CHUNK_TOKENS = 512, HY_CHUNK_ENTRIES = 64;
 inline bool chunk_sizes(int dk, int dv) { return dk > 32 && dk <= CH_MAX_DIM && dv > 32 && dv <= CH_MAX_DIM; }
+// The delta rule's chain has a block per SM, and its blocks behind the first wave wait: 512 tokens of the longest request per wave.  Token by token and in
+// chunks, us, channel decays, 16 heads of 128 x 128: one request of 512 tokens 122 and 107, 1024 232 and 178, 2048 452 and 345; two of 2048
+// 424 and 351, four of 2048 (longest 780) 322 and 366.  One decay per head, 8 heads: 2048 tokens 365 and 263, four requests 187 and 198.
+inline bool delta_pays(int heads, int dv, int entries, int longest) {
+  const long long blocks = (long long)heads * ((dv + DELTA_COLS - 1) / DELTA_COLS) * entries;
+  return longest >= HY_CHUNK_TOKENS * ((blocks + 147) / 148);
+}
 // chunks that a step of max_step_tokens may be cut into
 inline int chunk_cap(int max_tokens) { return (5 * max_tokens + 4 * CH_T) / (4 * CH_T); }
 

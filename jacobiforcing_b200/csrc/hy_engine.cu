@@ -1504,14 +1504,15 @@ extern "C" int hy_finalize(hy_handle h) {
   }
   {
     size_t states = 0, ends = 0;                              // floats per chunk of the largest layer
-    auto layer = [&](int H, int dk, int dv) {
+    auto layer = [&](int H, int dk, int dv, bool delta = false) {
       if (!chunk_sizes(dk, dv)) return;
       const size_t k = dk <= 64 ? 64 : 128, v = dv <= 64 ? 64 : 128;
-      states = std::max(states, (size_t)H * k * v); ends = std::max(ends, (size_t)H * k);
+      states = std::max(states, (size_t)H * (delta ? delta_work_floats((int)k, (int)v) : k * v)); ends = std::max(ends, (size_t)H * k);
     };
     for (auto& c : h->lc) {
       if (c.mixer == HY_MIX_SSD) layer(c.m_heads, c.m_state, c.m_vdim);
       if (c.mixer == HY_MIX_GLR || c.mixer == HY_MIX_GLA || c.mixer == HY_MIX_RETENTION) layer(c.g_heads, c.g_dim, c.g_vdim);
+      if (c.mixer == HY_MIX_DELTA || c.mixer == HY_MIX_ATTN_DELTA) layer(c.d_heads, c.d_dim, c.d_vdim, true);
     }
     size_t scan = 0;
     for (auto& c : h->lc)
@@ -1794,16 +1795,17 @@ LinearLaunch linear_launch(int parts, int vc, int dk, int dv, const AT* v, int l
                       dv % ch == 0 && cpb % ch == 0 && ldv % ch == 0 && (reinterpret_cast<uintptr_t>(v) & 15) == 0 ? 1 : 0};
 }
 
+int longest_entry(const hy_engine* h, const Batch& b) {
+  int most = 0;
+  for (int e = 0; e < b.E; ++e) most = std::max(most, h->step_start[e + 1] - h->step_start[e]);
+  return most;
+}
 // Chunks of the running step if its matrix-state recurrences of this size run in chunks of 64 tokens (hy_chunk.cuh), else 0.
 int step_chunks(const hy_engine* h, const Batch& b, int dk, int dv) {
   if (!chunk_sizes(dk, dv) || b.E > HY_CHUNK_ENTRIES) return 0;
-  int most = 0, n = 0;
-  for (int e = 0; e < b.E; ++e) {
-    const int cnt = h->step_start[e + 1] - h->step_start[e];
-    most = std::max(most, cnt);
-    n += (cnt + CH_T - 1) / CH_T;
-  }
-  return most >= HY_CHUNK_TOKENS && n <= h->ch_cap && 4LL * n * CH_T <= 5LL * b.T + 4 * CH_T ? n : 0;
+  int n = 0;
+  for (int e = 0; e < b.E; ++e) n += (h->step_start[e + 1] - h->step_start[e] + CH_T - 1) / CH_T;
+  return longest_entry(h, b) >= HY_CHUNK_TOKENS && n <= h->ch_cap && 4LL * n * CH_T <= 5LL * b.T + 4 * CH_T ? n : 0;
 }
 
 // The recurrence of gla_kernel over a step in chunks, if the step is one for them.
@@ -1830,6 +1832,28 @@ bool gla_chunked(hy_engine* h, const Batch& b, int H, int dk, int dv, const AT* 
   else if (dv <= 64) go(c128{}, c64{});
   else go(c128{}, c128{});
   h->launches += 2;                                            // the caller counts one for the recurrence
+  return true;
+}
+
+// The recurrence of delta_head_kernel over a step in chunks, if the step is one for them (dec NULL: one decay per head, in h->lin_sc).
+template <typename AT>
+bool delta_chunked(hy_engine* h, const Batch& b, int H, int G, int dk, int dv, const AT* v, int ldv, const float* dec, int ldd, float* state, float* o, int ldo) {
+  const int chunks = step_chunks(h, b, dk, dv);
+  if (chunks == 0 || !delta_pays(H, dv, b.E, longest_entry(h, b))) return false;
+  const int vec = dk % 4 == 0 && ldd % 4 == 0 && (reinterpret_cast<uintptr_t>(dec) & 15) == 0;
+  const DeltaArgs<AT> a{b, h->lin, v, ldv, h->lin_sc, dec, ldd, H, G, dk, dv, vec, h->ch_states, state, o, ldo};
+  auto go = [&](auto k, auto c) {
+    constexpr int DK = decltype(k)::value, DV = decltype(c)::value;
+    static_assert(DeltaWork<DK, DV>::SIZE == delta_work_floats(DK, DV), "the workspace holds what the kernels lay out");
+    go_kernel(h, delta_chunk_prep_kernel<AT, DK, DV>, dim3(chunks, H), 256, delta_prep_smem<DK, DV>(), h->stream, a);
+    go_kernel(h, delta_chunk_chain_kernel<AT, DK, DV>, dim3(H * (DV / DELTA_COLS), b.E), 256, delta_chain_smem<DK>(), h->stream, a);
+  };
+  typedef std::integral_constant<int, 64> c64; typedef std::integral_constant<int, 128> c128;
+  if (dk <= 64 && dv <= 64) go(c64{}, c64{});
+  else if (dk <= 64) go(c64{}, c128{});
+  else if (dv <= 64) go(c128{}, c64{});
+  else go(c128{}, c128{});
+  h->launches += 1;                                            // the caller counts one for the recurrence
   return true;
 }
 
@@ -2711,6 +2735,7 @@ void attn_delta_mixer(hy_engine* h, const Batch& b, const LayerW& L, const hy_la
                      h->f1, h->ld_f1, c.left_scale};
   biased_attend<AT>(h, b, L, c, bc);
   ProfScope ps(h, HY_PROF_DELTA);
+  if (!delta_chunked<AT>(h, b, H, G, dk, dv, cv, h->ld_cv, nullptr, 0, L.rec_state, h->f2, h->ld_f2))
   launch_linear<AT>(dk, H, dv, E, [&](auto dr, auto parts, auto vcols) {
     constexpr int DR = decltype(dr)::value, PARTS = decltype(parts)::value, VC = decltype(vcols)::value;
     const LinearLaunch g = linear_launch<AT>(PARTS, VC, dk, dv, cv, h->ld_cv);
@@ -2967,9 +2992,7 @@ int run_step(hy_engine* h, const Batch& b, int n_want, const int* want_d, float*
                 v32 | vat << 1, c.right_scale, L.rec_state, cat + L.o_scan, h->ld_cat, seg);
             h->launches++;
           };
-          int most = 0;
-          for (int e = 0; e < E; ++e) most = std::max(most, h->step_start[e + 1] - h->step_start[e]);
-          const ScanSegments seg = scan_segments(h->scan_own, (I + PB - 1) / PB, E, most, I, N);
+          const ScanSegments seg = scan_segments(h->scan_own, (I + PB - 1) / PB, E, longest_entry(h, b), I, N);
           if (seg.count > 1) {
             pass(std::integral_constant<int, SCAN_OWN>{}, E * seg.count, seg);
             pass(std::integral_constant<int, SCAN_READ>{}, E * seg.count, seg);
@@ -3007,6 +3030,7 @@ int run_step(hy_engine* h, const Batch& b, int n_want, const int* want_d, float*
       }
       ProfScope ps(h, HY_PROF_DELTA);
       float* o = h->f2 + ((nv + 3) & ~3);                      // behind the output gates
+      if (!delta_chunked<AT>(h, b, H, G, dk, dv, cv, h->ld_cv, h->f1, h->ld_f1, L.rec_state, o, h->ld_f2))
       launch_linear<AT>(dk, H, dv, E, [&](auto dr, auto parts, auto vcols) {
         constexpr int DR = decltype(dr)::value, PARTS = decltype(parts)::value, VC = decltype(vcols)::value;
         const LinearLaunch g = linear_launch<AT>(PARTS, VC, dk, dv, cv, h->ld_cv);

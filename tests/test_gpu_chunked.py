@@ -44,10 +44,49 @@ def test_chunked_portions(mode, dim, vdim, dtype):
     assert helpers.close(got, helpers.oracle_logits(cfg, w, toks), dtype)
 
 
-@pytest.mark.parametrize("mode", MODES)
+def _delta(kind, dim, vdim, heads, kv):
+    if kind == "channel":
+        return kinetar_plain, kin, kin.model_config([kin.delta(heads=heads, kv_heads=kv, dim=dim, vdim=vdim, ff=0)])
+    return mafalorn_plain, maf, maf.model_config([maf.par(d_heads=heads, d_kv_heads=kv, d_dim=dim, d_vdim=vdim, conv=4, mlp=None)])
+
+
+def _good(kind, got, want, dtype):
+    return kin.rel_err(got, want) < kin.TOL[dtype] if kind == "channel" else maf.close(got, want, dtype)
+
+
+@pytest.mark.parametrize("dim,vdim,heads,kv,dtype", [(33, 35, 2, 1, "float32"), (64, 64, 1, 1, "bfloat16"), (64, 65, 2, 2, "float32"), (128, 48, 2, 1, "float32"),
+                                                     (100, 128, 2, 1, "bfloat16"), (127, 127, 1, 1, "float32")])
+@pytest.mark.parametrize("kind", ["channel", "head"])
+def test_chunked_delta_rule(kind, dim, vdim, heads, kv, dtype):
+    plain, helpers, cfg = _delta(kind, dim, vdim, heads, kv)
+    toks = kin.rand_tokens(sum(CUTS), cfg["vocab"], 7)
+    w = plain.random_weights(cfg, 0)
+    hz = helpers.Harness(cfg, w, dtype, num_pages=80, max_step_tokens=640)
+    try:
+        got = hz.feed("a", toks, CUTS)
+    finally:
+        hz.close()
+    assert _good(kind, got, helpers.oracle_logits(cfg, w, toks), dtype)
+
+
+@pytest.mark.parametrize("kind", ["channel", "head"])
+def test_chunked_delta_rule_of_equal_keys(kind):
+    """One token again and again: every key of the request points the same way, which is as far from independent corrections as they get."""
+    plain, helpers, cfg = _delta(kind, 64, 40, 2, 1)
+    w = plain.random_weights(cfg, 3)
+    toks = [5] * 530
+    hz = helpers.Harness(cfg, w, "float32", num_pages=80, max_step_tokens=640)
+    try:
+        got = hz.feed("a", toks, [530])
+    finally:
+        hz.close()
+    assert _good(kind, got, helpers.oracle_logits(cfg, w, toks), "float32")
+
+
+@pytest.mark.parametrize("mode", MODES + ["channel delta", "head delta"])
 def test_chunked_requests_of_a_step(mode):
     """Requests of 575, 1 and 576 tokens in one step, then again behind themselves."""
-    plain, helpers, cfg = _model(mode, 64, 36)
+    plain, helpers, cfg = _delta(mode[:-6], 64, 36, 2, 1) if mode.endswith("delta") else _model(mode, 64, 36)
     w = plain.random_weights(cfg, 1)
     lens = {"a": 575, "b": 1, "c": 576}
     toks = {k: kin.rand_tokens(2 * n if n < 100 else n + 530, cfg["vocab"], i) for i, (k, n) in enumerate(lens.items())}
@@ -62,7 +101,8 @@ def test_chunked_requests_of_a_step(mode):
         m = len(toks[k]) - n
         got = np.concatenate([first[a:a + n], second[b:b + m]], 0)
         a, b = a + n, b + m
-        assert helpers.close(got, helpers.oracle_logits(cfg, w, toks[k]), "float32"), k
+        want = helpers.oracle_logits(cfg, w, toks[k])
+        assert _good("channel", got, want, "float32") if mode == "channel delta" else helpers.close(got, want, "float32"), k
 
 
 def test_chunked_forget_gates_of_zero_and_one():
