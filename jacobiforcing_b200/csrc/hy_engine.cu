@@ -48,7 +48,7 @@ struct LayerW {
   int c_q = 0, c_k = 0, c_g = 0, c_x = 0, c_z = 0, c_v = 0, c_b = 0, c_a1 = 0, c_g1 = 0, c_up = 0;
   int o_mix = 0, o_scan = 0, o_ff = 0;
   void* conv_qk = nullptr; void* sink = nullptr;                               // attention side
-  void* conv_x = nullptr; void* conv_xb = nullptr; void* w_x = nullptr; void* w_dt = nullptr; void* dt_b = nullptr;
+  void* conv_x = nullptr; void* conv_xb = nullptr; void* w_x = nullptr; void* w_dt = nullptr; void* w_dt_t = nullptr; void* dt_b = nullptr;
   float* A_neg = nullptr; void* D = nullptr;                                    // scan side
   void* conv_qkv = nullptr; void* w_a2 = nullptr; void* w_g2 = nullptr; void* A_log = nullptr; void* dt_bias = nullptr;
   void* norm_w = nullptr;                                                        // delta
@@ -178,6 +178,7 @@ struct hy_engine {
   // its column count; rot_tables_d is what the kernel reads
   struct RotEntry { hy_layer_cfg c; RotTable t; };
   std::vector<RotEntry> rot_tables; RotTable* rot_tables_d = nullptr;
+  void* split = nullptr; int split_width = 0;    // fp32 rows in three bf16 parts (split_rows_kernel)
   float* scan_own = nullptr;                     // own states and sums of step sizes of a selective scan's segments (see scan_segments)
   float* ch_states = nullptr; float* ch_ends = nullptr; int ch_cap = 0;    // chunked recurrences (hy_chunk.cuh): chunks that the sums have room for
   float* part_o = nullptr; float* part_ml = nullptr; size_t part_rows = 0, part_dim = 0;
@@ -500,6 +501,16 @@ struct Builder {
       cudaMemcpy(d, b.data(), b.size() * 2, cudaMemcpyHostToDevice);
     }
     return d;
+  }
+  // three times side by side, for rows in three parts (split_rows_kernel)
+  void* up_split(const std::vector<float>& v, int N, int K) {
+    if (rc != HY_OK || h->m.dtype != HY_DTYPE_BF16) return nullptr;
+    const int KP = split_cols(K);
+    std::vector<float> three((size_t)N * 3 * KP, 0.0f);
+    for (int n = 0; n < N; ++n)
+      for (int p = 0; p < 3; ++p) std::copy_n(&v[(size_t)n * K], K, &three[((size_t)n * 3 + p) * KP]);
+    h->split_width = std::max(h->split_width, 3 * KP);
+    return up_tiled(three, N, 3 * KP);
   }
   void* up_tiled(const std::vector<float>& v, int N, int K) {
     if (rc != HY_OK || h->m.dtype != HY_DTYPE_BF16) return nullptr;
@@ -1326,7 +1337,7 @@ extern "C" int hy_finalize(hy_handle h) {
       if (auto t = B.get(s + "conv", I, c.s_conv)) L.conv_x = B.up(t->v);
       if (auto t = B.get(s + "conv.b", I, -1)) L.conv_xb = B.up(t->v);
       if (auto t = B.get(s + "x", R + 2 * N, I)) { L.w_x = B.up(t->v); L.w_x_t = B.up_tiled(t->v, R + 2 * N, I); }
-      if (auto t = B.get(s + "dt", I, R)) L.w_dt = B.up(t->v);
+      if (auto t = B.get(s + "dt", I, R)) { L.w_dt = B.up(t->v); L.w_dt_t = B.up_split(t->v, I, R); }
       if (auto t = B.get(s + "dt.b", I, -1)) L.dt_b = B.up(t->v);
       if (auto t = B.get(s + "A_log", I, N)) {
         std::vector<float> an(t->v.size());
@@ -1415,6 +1426,7 @@ extern "C" int hy_finalize(hy_handle h) {
   if (dev_alloc(h, (void**)&h->f2, T * h->ld_f2 * 4, &h->bytes_ws)) return HY_ERR_CUDA;
   if (mx.lin > 0 && dev_alloc(h, (void**)&h->lin, T * (size_t)mx.lin * 4, &h->bytes_ws)) return HY_ERR_CUDA;
   if (mx.lin_sc > 0 && dev_alloc(h, (void**)&h->lin_sc, T * (size_t)mx.lin_sc * sizeof(float4), &h->bytes_ws)) return HY_ERR_CUDA;
+  if (h->split_width > 0 && rt.max_step_tokens >= HY_SPLIT_ROWS && dev_alloc(h, &h->split, T * (size_t)h->split_width * 2, &h->bytes_ws)) return HY_ERR_CUDA;
   if (h->m.block_kind == HY_BLOCK_PRENORM) {
     if (dev_alloc(h, (void**)&h->hn, T * W * 4, &h->bytes_ws)) return HY_ERR_CUDA;
     if (h->m.depth_avg && dev_alloc(h, (void**)&h->kept, (h->lc.size() + 1) * T * W * 4, &h->bytes_ws)) return HY_ERR_CUDA;
@@ -1625,6 +1637,18 @@ int gemm(hy_engine* h, const TA* A, int lda, const TW* Wt, int ldw, int T, int N
       go_kernel(h, gemm_simt_kernel<TA, TW, TO, 32>, dim3((N + 31) / 32, (T + 31) / 32), 256, 0, h->stream, A, lda, Wt, ldw, T, N, K, o);
   }
   h->launches++;
+  return HY_OK;
+}
+
+// The product of fp32 rows: in three parts on the tensor cores where the rows are many (split_rows_kernel).
+template <typename TW>
+int gemm_split(hy_engine* h, const float* A, int lda, const TW* Wt, int ldw, int T, int N, int K, GemmOut o, const void* split) {
+  if (!split || T < HY_SPLIT_ROWS) return gemm<float, TW, float>(h, A, lda, Wt, ldw, T, N, K, o);
+  if (o.alpha == 0.0f) o.alpha = 1.0f;
+  const int KP = split_cols(K);
+  go_kernel(h, split_rows_kernel, std::min((T * (KP / 2) + 127) / 128, 148 * 16), 128, 0, h->stream, A, lda, T, K, KP, (bf16*)h->split);
+  h->launches++;
+  pair_product<float>(h, (const bf16*)h->split, 3 * KP, T, split, 1, 0, T, N, 3 * KP, o, 0, jf::TpGroup{});
   return HY_OK;
 }
 
@@ -2974,7 +2998,7 @@ int run_step(hy_engine* h, const Batch& b, int n_want, const int* want_d, float*
       {
       ProfScope ps(h, HY_PROF_SMALL_GEMM);
       gemm<AT, WT, float>(h, cv, h->ld_cv, (const WT*)L.w_x, I, T, R + 2 * N, I, to_buf(h->f1, h->ld_f1), L.w_x_t);
-      gemm<float, WT, float>(h, h->f1, h->ld_f1, (const WT*)L.w_dt, R, T, I, R, to_buf(h->f2, h->ld_f2));
+      gemm_split<WT>(h, h->f1, h->ld_f1, (const WT*)L.w_dt, R, T, I, R, to_buf(h->f2, h->ld_f2), L.w_dt_t);
       }
       {
         ProfScope ps(h, HY_PROF_SCAN);

@@ -113,6 +113,38 @@ struct HyEpilogue {
   }
 };
 
+// ---- products of fp32 rows with bf16 weights (step sizes) ------------------------------------------------------------------------
+// An fp32 number is the sum of three bf16 numbers, its upper, middle and lower eight bits, so the product of fp32 rows is one of bf16 rows
+// [lower | middle | upper], three times as long, with the weights side by side three times: every product of two numbers is exact as it
+// was, and the sums are the tensor cores' fp32 sums (the upper parts come last, so that what is cut off a sum is cut off few large ones).  Against 64
+// bits, K 128: 1.5e-7 of the result's norm, gemm_simt_kernel 2.0e-7; K 16: 5.1e-8 and 7.1e-8.
+// N 4096, T 2048, K 128: 85 us on the fp32 units, 21 with both kernels; from 512 rows on (N 2048, T 300, K 64: 12.4 and 11.4; T 100, K 130: 10.4 and
+// 14.5).  Not where every result goes through functions (decays, 2048 x 2048 and K 16: 36 us either way): that is what takes the time there.
+constexpr int HY_SPLIT_ROWS = 512;
+inline int split_cols(int K) { return (K + 63) / 64 * 64; }    // of each part
+// a [T, lda] (K columns) -> o [T][3][KP], zeros beyond K.  What is no number, and infinities, stay whole in the upper part.
+__global__ void __launch_bounds__(128) split_rows_kernel(const float* __restrict__ a, int lda, int T, int K, int KP, bf16* __restrict__ o) {
+  pdl_begin();
+  const int per = KP / 2;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < T * per; i += gridDim.x * blockDim.x) {
+    const int t = i / per, k = i % per * 2;
+    uint32_t part[3] = {};
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const float x = k + j < K ? a[(size_t)t * lda + k + j] : 0.0f;
+      const uint32_t u = __float_as_uint(x);
+      const bool whole = (u & 0x7f800000u) == 0x7f800000u;
+      const float hi = whole ? __bfloat162float(__float2bfloat16_rn(x)) : __uint_as_float(u & 0xffff0000u), r = whole ? 0.0f : x - hi;
+      const float mid = __uint_as_float(__float_as_uint(r) & 0xffff0000u), lo = r - mid;
+      part[0] |= (__float_as_uint(lo) >> 16) << (16 * j);      // lo has no more than eight bits left
+      part[1] |= (__float_as_uint(mid) >> 16) << (16 * j);
+      part[2] |= (__float_as_uint(hi) >> 16) << (16 * j);
+    }
+    uint32_t* row = reinterpret_cast<uint32_t*>(o + (size_t)t * 3 * KP + k);
+    row[0] = part[0]; row[KP / 2] = part[1]; row[KP] = part[2];
+  }
+}
+
 // Host-side packer: row-major [N, K] floats -> bf16 tiles [ceil(N/128)][ceil(K/64)] of 128 x 64 in the swizzled layout.
 inline void pack_tiles(const float* w, int N, int K, std::vector<uint16_t>& out) {
   const int NT = (N + 127) / 128, KT = (K + 63) / 64;
