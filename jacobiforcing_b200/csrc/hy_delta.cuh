@@ -81,7 +81,8 @@ __global__ void __launch_bounds__(128) key_value_prep_kernel(Batch b, AT* __rest
 
 // ---- operands of a matrix-state recurrence: fp32 rows [T][heads][q dim | k dim] ------------------------------------------------------
 // Rotated (rp.pairs > 0: the first 2 pairs dimensions, cs [T, ldc] from rot_tables_kernel), queries times dim^(-1/2).
-template <typename AT>
+// V > 1: without rotation.
+template <typename AT, int V>
 __global__ void __launch_bounds__(1024) linear_rows_kernel(const AT* __restrict__ in, int ld, int col_q, int col_k, int H, int dim,
                                                           const float* __restrict__ cs, int ldc, RotPair rp, float* __restrict__ qk) {
   pdl_begin();
@@ -90,6 +91,18 @@ __global__ void __launch_bounds__(1024) linear_rows_kernel(const AT* __restrict_
   const float* c = rp.pairs > 0 ? cs + (size_t)t * ldc : nullptr;
   float* out = qk + (size_t)t * H * 2 * dim;
   const float qscale = 1.0f / sqrtf((float)dim);
+  if constexpr (V > 1) {
+    for (int i = threadIdx.x * V; i < H * dim; i += blockDim.x * V) {
+      float* at = out + (size_t)(i / dim) * 2 * dim + i % dim;
+      float q[V], kk[V];
+      load_f(q, row + col_q + i); load_f(kk, row + col_k + i);
+#pragma unroll
+      for (int j = 0; j < V; ++j) q[j] *= qscale;
+      store_f(at, q);
+      store_f(at + dim, kk);
+    }
+    return;
+  }
   for (int i = threadIdx.x; i < H * dim; i += blockDim.x) {
     const int h = i / dim, k = i % dim;
     const AT* qh = row + col_q + h * dim;

@@ -1761,6 +1761,44 @@ const UnitList* biased_units(hy_engine* h, int E, int T, const BiasedCfg& c, int
   return w.commit(3, H, G, c.window, c.chunk, 0, ns);
 }
 
+// Whether a row kernel may take four elements at a time: sizes and leading dimensions in fours, rows that begin on four elements.
+template <typename... P>
+inline bool in_fours(std::initializer_list<int> sizes, const P*... rows) {
+  for (int n : sizes) if (n % 4 != 0) return false;
+  return (((reinterpret_cast<uintptr_t>(rows) % (4 * sizeof(P))) == 0) && ...);
+}
+typedef std::integral_constant<int, 4> four_t; typedef std::integral_constant<int, 1> one_t;
+template <typename AT, typename GT, int GATE>
+void launch_gla_out(hy_engine* h, int T, int H, int dv, const float* o, int ldi, const GT* g, int ldg, const float* w, float eps, float out_scale, AT* out, int ldo) {
+  auto go = [&](auto v) {
+    go_kernel(h, gla_out_kernel<AT, GT, GATE, decltype(v)::value>, (T * H + 3) / 4, 128, 0, h->stream, T, H, dv, o, ldi, g, ldg, w, eps, out_scale, out, ldo);
+  };
+  if (in_fours({dv, ldi, GATE == GATE_NONE ? 0 : ldg, ldo}, o, g, w, out)) go(four_t{});
+  else go(one_t{});
+}
+template <typename AT>
+void launch_linear_rows(hy_engine* h, int T, const AT* in, int ld, int col_q, int col_k, int H, int dim, const float* cs, int ldc, RotPair rp) {
+  auto go = [&](auto v) {
+    go_kernel(h, linear_rows_kernel<AT, decltype(v)::value>, T, T <= 8 ? 1024 : 128, 0, h->stream, in, ld, col_q, col_k, H, dim, cs, ldc, rp, h->lin);
+  };
+  if (rp.pairs == 0 && in_fours({ld, col_q, col_k, dim}, in)) go(four_t{});
+  else go(one_t{});
+}
+template <typename AT>
+void launch_tanh_norm(hy_engine* h, int rows, const int* which, const TanhNorm& n, AT* out) {
+  const int W = h->m.width;
+  auto go = [&](auto v) { go_kernel(h, tanh_norm_kernel<AT, decltype(v)::value>, rows, 256, 0, h->stream, h->x, which, n, W, out); };
+  if (in_fours({W}, n.w, n.b, out)) go(four_t{});
+  else go(one_t{});
+}
+template <typename AT>
+void launch_rmsnorm(hy_engine* h, int rows, const int* which, const AT* w, float offset, AT* out) {
+  const int W = h->m.width;
+  auto go = [&](auto v) { go_kernel(h, rmsnorm_kernel<AT, AT, decltype(v)::value>, rows, 256, 0, h->stream, h->x, which, w, h->m.norm_eps, W, offset, out); };
+  if (in_fours({W}, w, out)) go(four_t{});
+  else go(one_t{});
+}
+
 // Short convolution with its carried tail (see conv_kernel): four columns per thread where every boundary allows it.
 template <typename AT>
 void launch_conv(hy_engine* h, const Batch& b, const AT* u, int ldu, int col0, int C, int taps, const void* w, const void* bias, int silu,
@@ -2157,7 +2195,7 @@ int sandwich_layer(hy_engine* h, const Batch& b, size_t li) {
   const TanhNorm after_ff = last ? none : h->lw[li + 1].n1;
   if (li == 0) {
     ProfScope ps(h, HY_PROF_NORM);
-    go_kernel(h, tanh_norm_kernel<AT>, T, 256, 0, s, h->x, nullptr, L.n1, W, hb);
+    launch_tanh_norm<AT>(h, T, nullptr, L.n1, hb);
     h->launches++;
   }
   if (c.mixer == HY_MIX_SSD) {
@@ -2184,8 +2222,12 @@ int sandwich_layer(hy_engine* h, const Batch& b, size_t li) {
         go_kernel(h, gla_kernel<AT, DR, PARTS, VC, GLA_TOKEN>, dim3(H * g.bph, E), 128, smem, s, b, h->lin, cv, h->ld_cv, nullptr, 0, nullptr, H, N, P, g.bph,
                                                                                    g.vec, g.vvec, L.rec_state, h->f2, h->ld_f2, tk);
       });
-      go_kernel(h, gated_group_norm_kernel<AT>, dim3(T, c.m_norm_groups), 128, 0, s, h->f2, h->ld_f2, pin, h->ld_pin, L.m_norm, inner,
-                                                                          c.m_norm_groups, eps, cat, h->ld_cat);
+      const auto gate = [&](auto v) {
+        go_kernel(h, gated_group_norm_kernel<AT, decltype(v)::value>, dim3(T, c.m_norm_groups), 128, 0, s, h->f2, h->ld_f2, pin, h->ld_pin, L.m_norm, inner,
+                  c.m_norm_groups, eps, cat, h->ld_cat);
+      };
+      if (in_fours({inner / c.m_norm_groups, h->ld_f2, h->ld_pin, h->ld_cat}, h->f2, pin, cat, L.m_norm)) gate(four_t{});
+      else gate(one_t{});
       h->launches += 2;
     }
   } else if (c.mixer == HY_MIX_LATENT) {
@@ -2202,7 +2244,11 @@ int sandwich_layer(hy_engine* h, const Batch& b, size_t li) {
     }
     ProfScope ps(h, HY_PROF_DELTA);
     if (dk <= HY_LIN_MAX_DIM) {
-      go_kernel(h, forget_rows_kernel<AT>, T, T <= 8 ? 1024 : 256, 0, s, pin, h->ld_pin, L.c_q, L.c_k, L.g_fb, L.g_lower, H, dk, h->lin);
+      const auto rows = [&](auto v) {
+        go_kernel(h, forget_rows_kernel<AT, decltype(v)::value>, T, T <= 8 ? 1024 : 256, 0, s, pin, h->ld_pin, L.c_q, L.c_k, L.g_fb, L.g_lower, H, dk, h->lin);
+      };
+      if (in_fours({h->ld_pin, L.c_q, L.c_k, dk}, pin, L.g_fb, L.g_lower)) rows(four_t{});
+      else rows(one_t{});
       if (!gla_chunked<AT, GLA_FORGET>(h, b, H, dk, dv, pin + L.c_v, h->ld_pin, nullptr, 0, nullptr, L.rec_state, h->f2, h->ld_f2, GlaToken{}))
       launch_linear<AT>(dk, H, dv, E, [&](auto dr, auto parts, auto vcols) {
         constexpr int DR = decltype(dr)::value, PARTS = decltype(parts)::value, VC = decltype(vcols)::value;
@@ -2211,7 +2257,7 @@ int sandwich_layer(hy_engine* h, const Batch& b, size_t li) {
         go_kernel(h, gla_kernel<AT, DR, PARTS, VC, GLA_FORGET>, dim3(H * g.bph, E), 128, smem, s, b, h->lin, pin + L.c_v, h->ld_pin, nullptr, 0, nullptr, H, dk,
                                                                                     dv, g.bph, g.vec, g.vvec, L.rec_state, h->f2, h->ld_f2, GlaToken{});
       });
-      go_kernel(h, gla_out_kernel<AT, AT, GATE_NONE>, (T * H + 3) / 4, 128, 0, s, T, H, dv, h->f2, h->ld_f2, nullptr, 0, L.g_norm, eps, 1.0f, cat, h->ld_cat);
+      launch_gla_out<AT, AT, GATE_NONE>(h, T, H, dv, h->f2, h->ld_f2, nullptr, 0, L.g_norm, eps, 1.0f, cat, h->ld_cat);
       h->launches += 3;
     } else {
       go_kernel(h, glr_kernel<AT>, dim3(H, E), 256, ((size_t)dk * dv + 2 * dk + dv + 40) * 4, s, 
@@ -2263,7 +2309,11 @@ int sandwich_layer(hy_engine* h, const Batch& b, size_t li) {
       go_kernel(h, expert_gemm_simt_kernel<AT, WT, float, false>, dim3((W + 31) / 32, tiles), 256, 0, s, 
           pin, ldh, (const WT*)L.w_down, (size_t)W * ff, W, ff, h->x_offs, h->x_tile_e, h->x_tile_r0, h->x_meta, ys, W, -1, 0.0f);
     }
-    go_kernel(h, expert_combine_kernel<AT>, T, 256, 0, s, ys, W, few ? nullptr : h->x_pair_row, h->x_wts, top, W, L.n2b, L.ls2, h->x, after_ff, hb);
+    const auto combine = [&](auto v) {
+      go_kernel(h, expert_combine_kernel<AT, decltype(v)::value>, T, 256, 0, s, ys, W, few ? nullptr : h->x_pair_row, h->x_wts, top, W, L.n2b, L.ls2, h->x, after_ff, hb);
+    };
+    if (in_fours({W}, ys, L.n2b.w, L.n2b.b, L.ls2, after_ff.w, after_ff.b, hb)) combine(four_t{});
+    else combine(one_t{});
     h->launches += 3;
   }
   return HY_OK;
@@ -2697,7 +2747,7 @@ void gla_mixer(hy_engine* h, const Batch& b, const LayerW& L, const hy_layer_cfg
     gemm<float, WT, float>(h, h->f1, h->ld_f1, (const WT*)L.w_a2, c.g_low, T, nq, c.g_low, o);
   }
   ProfScope ps(h, HY_PROF_DELTA);
-  go_kernel(h, linear_rows_kernel<AT>, T, T <= 8 ? 1024 : 128, 0, s, pin, h->ld_pin, L.c_q, L.c_k, H, dk, nullptr, 0, RotPair{0, 1}, h->lin);
+  launch_linear_rows<AT>(h, T, pin, h->ld_pin, L.c_q, L.c_k, H, dk, nullptr, 0, RotPair{0, 1});
   if (!gla_chunked<AT, GLA_CHANNEL>(h, b, H, dk, dv, pin + L.c_v, h->ld_pin, h->f2, h->ld_f2, nullptr, L.rec_state, h->f2 + c_o, h->ld_f2, GlaToken{}))
   launch_linear<AT>(dk, H, dv, E, [&](auto dr, auto parts, auto vcols) {
     constexpr int DR = decltype(dr)::value, PARTS = decltype(parts)::value, VC = decltype(vcols)::value;
@@ -2706,7 +2756,7 @@ void gla_mixer(hy_engine* h, const Batch& b, const LayerW& L, const hy_layer_cfg
     go_kernel(h, gla_kernel<AT, DR, PARTS, VC, GLA_CHANNEL>, dim3(H * g.bph, E), 128, smem, s, b, h->lin, pin + L.c_v, h->ld_pin, h->f2, h->ld_f2, nullptr, H, dk,
                                                                            dv, g.bph, g.vec, g.vvec, L.rec_state, h->f2 + c_o, h->ld_f2, GlaToken{});
   });
-  go_kernel(h, gla_out_kernel<AT>, (T * H + 3) / 4, 128, 0, s, T, H, dv, h->f2 + c_o, h->ld_f2, pin + L.c_g, h->ld_pin, L.g_norm, h->m.norm_eps,
+  launch_gla_out<AT, AT, GATE_SILU>(h, T, H, dv, h->f2 + c_o, h->ld_f2, pin + L.c_g, h->ld_pin, L.g_norm, h->m.norm_eps,
                                                      1.0f, cat, h->ld_cat);
   h->launches += 3;
 }
@@ -2720,7 +2770,7 @@ void retention_mixer(hy_engine* h, const Batch& b, const LayerW& L, const hy_lay
   const RotTable& rot = h->rot_tables[(size_t)L.rot_table].t;
   const RotPair rp{rot.pairs, c.r_half};
   ProfScope ps(h, HY_PROF_DELTA);
-  go_kernel(h, linear_rows_kernel<AT>, T, T <= 8 ? 1024 : 128, 0, s, pin, h->ld_pin, L.c_q, L.c_k, H, dk, rot.out, rot.ld, rp, h->lin);
+  launch_linear_rows<AT>(h, T, pin, h->ld_pin, L.c_q, L.c_k, H, dk, rot.out, rot.ld, rp);
   if (!gla_chunked<AT, GLA_HEAD>(h, b, H, dk, dv, pin + L.c_v, h->ld_pin, nullptr, 0, L.decay, L.rec_state, h->f2, h->ld_f2, GlaToken{}))
   launch_linear<AT>(dk, H, dv, E, [&](auto dr, auto parts, auto vcols) {
     constexpr int DR = decltype(dr)::value, PARTS = decltype(parts)::value, VC = decltype(vcols)::value;
@@ -2729,7 +2779,7 @@ void retention_mixer(hy_engine* h, const Batch& b, const LayerW& L, const hy_lay
     go_kernel(h, gla_kernel<AT, DR, PARTS, VC, GLA_HEAD>, dim3(H * g.bph, E), 128, smem, s, b, h->lin, pin + L.c_v, h->ld_pin, nullptr, 0, L.decay, H, dk, dv,
                                                                           g.bph, g.vec, g.vvec, L.rec_state, h->f2, h->ld_f2, GlaToken{});
   });
-  go_kernel(h, gla_out_kernel<AT>, (T * H + 3) / 4, 128, 0, s, T, H, dv, h->f2, h->ld_f2, pin + L.c_g, h->ld_pin, nullptr, h->m.norm_eps, 1.0f, cat,
+  launch_gla_out<AT, AT, GATE_SILU>(h, T, H, dv, h->f2, h->ld_f2, pin + L.c_g, h->ld_pin, nullptr, h->m.norm_eps, 1.0f, cat,
                                                      h->ld_cat);
   h->launches += 3;
 }
@@ -2767,7 +2817,7 @@ void attn_delta_mixer(hy_engine* h, const Batch& b, const LayerW& L, const hy_la
     go_kernel(h, delta_head_kernel<AT, DR, PARTS, VC, false>, dim3(H * g.bph, E), 128, smem, s, b, h->lin, cv, h->ld_cv, h->lin_sc, H, G, dk, dv, g.bph, g.vec, g.vvec,
                                                                            L.rec_state, h->f2, h->ld_f2, nullptr, 0);
   });
-  go_kernel(h, gla_out_kernel<AT>, (T * H + 3) / 4, 128, 0, s, T, H, dv, h->f2, h->ld_f2, pin + L.c_g, h->ld_pin, L.g_norm, h->m.norm_eps,
+  launch_gla_out<AT, AT, GATE_SILU>(h, T, H, dv, h->f2, h->ld_f2, pin + L.c_g, h->ld_pin, L.g_norm, h->m.norm_eps,
                                                      c.right_scale, cat + L.o_scan, h->ld_cat);
   h->launches += 2;
 }
@@ -2943,7 +2993,7 @@ int run_step(hy_engine* h, const Batch& b, int n_want, const int* want_d, float*
     const int ff = c.ff_kind == HY_FF_NONE ? 0 : c.ff;
     {
       ProfScope ps(h, HY_PROF_NORM);
-      go_kernel(h, rmsnorm_kernel<WT, AT>, T, 256, 0, s, h->x, nullptr, (const WT*)L.norm1, eps, W, 1.0f, hb);
+      launch_rmsnorm<AT>(h, T, nullptr, (const AT*)L.norm1, 1.0f, hb);
       h->launches++;
     }
     // every projection that reads the normed input, in one product; the feed-forward's hidden part leaves activated,
@@ -3062,7 +3112,7 @@ int run_step(hy_engine* h, const Batch& b, int n_want, const int* want_d, float*
         go_kernel(h, delta_head_kernel<AT, DR, PARTS, VC, true>, dim3(H * g.bph, E), 128, smem, s, b, h->lin, cv, h->ld_cv, h->lin_sc, H, G, dk, dv, g.bph, g.vec,
                                                                                      g.vvec, L.rec_state, o, h->ld_f2, h->f1, h->ld_f1);
       });
-      go_kernel(h, gla_out_kernel<AT, float, GATE_SIGMOID>, (T * H + 3) / 4, 128, 0, s, T, H, dv, o, h->ld_f2, h->f2, h->ld_f2, (const float*)L.norm_w, eps,
+      launch_gla_out<AT, float, GATE_SIGMOID>(h, T, H, dv, o, h->ld_f2, h->f2, h->ld_f2, (const float*)L.norm_w, eps,
                                                                               1.0f, cat + L.o_mix, h->ld_cat);
       h->launches += 3;
     }
@@ -3079,9 +3129,8 @@ int run_step(hy_engine* h, const Batch& b, int n_want, const int* want_d, float*
   }
   if (n_want > 0) {
     ProfScope ps(h, HY_PROF_HEAD);
-    if (h->m.norm_kind == HY_NORM_TANH) go_kernel(h, tanh_norm_kernel<AT>, n_want, 256, 0, s, h->x, want_d, h->final_tanh, W, (AT*)h->hw);
-    else go_kernel(h, rmsnorm_kernel<WT, AT>, n_want, 256, 0, s, h->x, want_d, (const WT*)h->final_norm, eps, W,
-                                                       h->m.norm_kind == HY_NORM_RMS ? 0.0f : 1.0f, (AT*)h->hw);
+    if (h->m.norm_kind == HY_NORM_TANH) launch_tanh_norm<AT>(h, n_want, want_d, h->final_tanh, (AT*)h->hw);
+    else launch_rmsnorm<AT>(h, n_want, want_d, (const AT*)h->final_norm, h->m.norm_kind == HY_NORM_RMS ? 0.0f : 1.0f, (AT*)h->hw);
     h->launches++;
     GemmOut o = to_buf(h->logits, h->m.vocab);
     o.alpha = h->m.logit_scale;

@@ -336,23 +336,38 @@ __global__ void __launch_bounds__(256) expert_rows_kernel(const TA* __restrict__
 // x[t] += ls * (tanh(alpha y) w + b),  y = sum_k wts[t, k] rows[pair_row ? pair_row[t top + k] : t top + k]  (k in order).
 // post.w == NULL: x[t] += y (designs without an output norm on the feed-forward).
 // next.w != NULL: the updated stream also leaves through the next layer's input norm into next_out [T, width].
-template <typename AT>
+template <typename AT, int V>
 __global__ void expert_combine_kernel(const float* __restrict__ rows, int ldr, const int* __restrict__ pair_row,
                                       const float* __restrict__ wts, int top, int width, TanhNorm post,
                                       const float* __restrict__ ls, float* __restrict__ x, TanhNorm next,
                                       AT* __restrict__ next_out) {
   pdl_begin();
   const int t = blockIdx.x;
-  for (int c = threadIdx.x; c < width; c += blockDim.x) {
-    float y = 0.0f;
+  for (int c = threadIdx.x * V; c < width; c += blockDim.x * V) {
+    float y[V] = {}, f[V], w[V], b[V];
+#pragma unroll 4
     for (int k = 0; k < top; ++k) {
       const int i = t * top + k;
-      y = fmaf(wts[i], rows[(size_t)(pair_row ? pair_row[i] : i) * ldr + c], y);
+      load_f(f, rows + (size_t)(pair_row ? pair_row[i] : i) * ldr + c);
+      const float wt = wts[i];
+#pragma unroll
+      for (int j = 0; j < V; ++j) y[j] = fmaf(wt, f[j], y[j]);
     }
-    if (post.w) y = ls[c] * fmaf(tanhf(post.alpha * y), post.w[c], post.b[c]);
-    const float v = x[(size_t)t * width + c] + y;
-    x[(size_t)t * width + c] = v;
-    if (next.w) next_out[(size_t)t * width + c] = from_f<AT>(fmaf(tanhf(next.alpha * v), next.w[c], next.b[c]));
+    if (post.w) {
+      load_f(f, ls + c); load_f(w, post.w + c); load_f(b, post.b + c);
+#pragma unroll
+      for (int j = 0; j < V; ++j) y[j] = f[j] * fmaf(tanhf(post.alpha * y[j]), w[j], b[j]);
+    }
+    load_f(f, x + (size_t)t * width + c);
+#pragma unroll
+    for (int j = 0; j < V; ++j) f[j] += y[j];
+    store_f(x + (size_t)t * width + c, f);
+    if (next.w) {
+      load_f(w, next.w + c); load_f(b, next.b + c);
+#pragma unroll
+      for (int j = 0; j < V; ++j) y[j] = fmaf(tanhf(next.alpha * f[j]), w[j], b[j]);
+      store_f(next_out + (size_t)t * width + c, y);
+    }
   }
 }
 

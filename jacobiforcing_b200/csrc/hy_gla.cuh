@@ -210,25 +210,28 @@ __global__ void __launch_bounds__(128) gla_kernel(Batch b, const float* __restri
 }
 
 // Operand rows of the recurrence with a forget gate: [T][H][silu(q) | f], f = lower + (1 - lower) sigmoid(f_raw + f_bias).
-template <typename AT>
+template <typename AT, int V>
 __global__ void __launch_bounds__(1024) forget_rows_kernel(const AT* __restrict__ in, int ld, int col_q, int col_f,
                                                            const float* __restrict__ f_bias, const float* __restrict__ lower, int H, int dim,
                                                            float* __restrict__ qf) {
   pdl_begin();
   const AT* row = in + (size_t)blockIdx.x * ld;
   float* out = qf + (size_t)blockIdx.x * H * 2 * dim;
-  for (int i = threadIdx.x; i < H * dim; i += blockDim.x) {
+  for (int i = threadIdx.x * V; i < H * dim; i += blockDim.x * V) {
     const size_t at = (size_t)(i / dim) * 2 * dim + i % dim;
-    const float lo = lower[i];
-    out[at] = silu_f(to_f(row[col_q + i]));
-    out[at + dim] = fmaf(1.0f - lo, sigmoid_f(to_f(row[col_f + i]) + f_bias[i]), lo);
+    float q[V], f[V], lo[V], bias[V];
+    load_f(q, row + col_q + i); load_f(f, row + col_f + i); load_f(lo, lower + i); load_f(bias, f_bias + i);
+#pragma unroll
+    for (int j = 0; j < V; ++j) { q[j] = silu_f(q[j]); f[j] = fmaf(1.0f - lo[j], sigmoid_f(f[j] + bias[j]), lo[j]); }
+    store_f(out + at, q);
+    store_f(out + at + dim, f);
   }
 }
 
 // Norm per head, weight (NULL: none), output gate: out[t, h, :] = o / rms(o) * w * gate * out_scale, gate = silu(g), sigmoid(g) or one.
 // One warp per (token, head).
 enum OutGate : int { GATE_SILU = 0, GATE_SIGMOID = 1, GATE_NONE = 2 };
-template <typename AT, typename GT = AT, int GATE = GATE_SILU>
+template <typename AT, typename GT, int GATE, int V>
 __global__ void __launch_bounds__(128) gla_out_kernel(int T, int H, int vdim, const float* __restrict__ o, int ldi,
                                                       const GT* __restrict__ g, int ldg, const float* __restrict__ w, float eps,
                                                       float out_scale, AT* __restrict__ out, int ldo) {
@@ -238,13 +241,29 @@ __global__ void __launch_bounds__(128) gla_out_kernel(int T, int H, int vdim, co
   const size_t t = unit / H, c0 = (size_t)(unit % H) * vdim;
   const float* orow = o + t * ldi + c0;
   float ss = 0.0f;
-  for (int k = lane; k < vdim; k += 32) ss = fmaf(orow[k], orow[k], ss);
+  for (int k = lane * V; k < vdim; k += 32 * V) {
+    float v[V];
+    load_f(v, orow + k);
+#pragma unroll
+    for (int i = 0; i < V; ++i) ss = fmaf(v[i], v[i], ss);
+  }
   const float inv = out_scale / sqrtf(warp_sum(ss) / (float)vdim + eps);
-  for (int k = lane; k < vdim; k += 32) {
-    float v = orow[k] * inv * (w ? w[k] : 1.0f);
-    if constexpr (GATE == GATE_SILU) v *= silu_f(to_f(g[t * ldg + c0 + k]));
-    else if constexpr (GATE == GATE_SIGMOID) v *= sigmoid_f(to_f(g[t * ldg + c0 + k]));
-    out[t * ldo + c0 + k] = from_f<AT>(v);
+  for (int k = lane * V; k < vdim; k += 32 * V) {
+    float v[V], x[V];
+    load_f(v, orow + k);
+#pragma unroll
+    for (int i = 0; i < V; ++i) v[i] *= inv;
+    if (w) {
+      load_f(x, w + k);
+#pragma unroll
+      for (int i = 0; i < V; ++i) v[i] *= x[i];
+    }
+    if constexpr (GATE != GATE_NONE) {
+      load_f(x, g + t * ldg + c0 + k);
+#pragma unroll
+      for (int i = 0; i < V; ++i) v[i] *= GATE == GATE_SILU ? silu_f(x[i]) : sigmoid_f(x[i]);
+    }
+    store_f(out + t * ldo + c0 + k, v);
   }
 }
 

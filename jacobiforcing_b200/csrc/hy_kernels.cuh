@@ -102,32 +102,55 @@ __global__ void embed_kernel(Batch b, const WT* __restrict__ table, const double
   const int t = blockIdx.x;
   const int tok = b.tok[t];
   const double p = (double)b.tok_pos[t];
-  for (int c = threadIdx.x; c < width; c += blockDim.x) {
-    float pe = 0.0f;
-    if (inv_freq) {
-      const double ang = p * inv_freq[c >> 1];
-      pe = (float)((c & 1) ? cos(ang) : sin(ang));
-    }
-    x[(size_t)t * width + c] = to_f(table[(size_t)tok * width + c]) * scale + pe;
+  // a pair of channels shares its angle, and the reduction of it to a quadrant is most of what sine and cosine take
+  for (int c = 2 * threadIdx.x; c < width; c += 2 * blockDim.x) {
+    double sn = 0.0, cs = 0.0;
+    if (inv_freq) sincos(p * inv_freq[c >> 1], &sn, &cs);
+    x[(size_t)t * width + c] = to_f(table[(size_t)tok * width + c]) * scale + (float)sn;
+    if (c + 1 < width) x[(size_t)t * width + c + 1] = to_f(table[(size_t)tok * width + c + 1]) * scale + (float)cs;
   }
+}
+
+// ---- rows V elements at a time ------------------------------------------------------------------------------------------------------------
+// The kernels over rows below take V = 4 elements per thread (16 bytes of fp32) where sizes and leading dimensions are multiples of four and rows begin on
+// 16 (fp32) or 8 bytes, else one: with one element, too few bytes were in flight: 2048 rows, us, one -> four:
+// RMS norm of 2048 channels 10.5 -> 5.3, output norm and gate of 2048 columns 17.0 -> 12.1, forget-gate rows of 1024 columns 11.4 -> 6.8, gated group
+// norm of 2048 columns 24 -> 19.1, mixture of four experts' rows of 1024 channels 15.5 -> 9.2.  Positions of the embedding: 29.5 -> 12.4.
+template <typename T, int V>
+__device__ __forceinline__ void load_f(float (&f)[V], const T* p) {
+  const VecN<T, V> v = *reinterpret_cast<const VecN<T, V>*>(p);
+#pragma unroll
+  for (int i = 0; i < V; ++i) f[i] = to_f(v.v[i]);
+}
+template <typename T, int V>
+__device__ __forceinline__ void store_f(T* p, const float (&f)[V]) {
+  VecN<T, V> v;
+#pragma unroll
+  for (int i = 0; i < V; ++i) v.v[i] = from_f<T>(f[i]);
+  *reinterpret_cast<VecN<T, V>*>(p) = v;
 }
 
 // ---- element-wise tanh norm: tanh(alpha x) w + b, no statistics ------------------------------------------------------------
 // rows: NULL = row r of x, else x row rows[r].  Parameters are fp32.
 struct TanhNorm { const float* w; const float* b; float alpha; };
-template <typename OT>
+template <typename OT, int V>
 __global__ void tanh_norm_kernel(const float* __restrict__ x, const int* __restrict__ rows, TanhNorm n, int width,
                                  OT* __restrict__ out) {
   pdl_begin();
   const int r = blockIdx.x;
   const float* xr = x + (size_t)(rows ? rows[r] : r) * width;
-  for (int c = threadIdx.x; c < width; c += blockDim.x)
-    out[(size_t)r * width + c] = from_f<OT>(fmaf(tanhf(n.alpha * xr[c]), n.w[c], n.b[c]));
+  for (int c = threadIdx.x * V; c < width; c += blockDim.x * V) {
+    float v[V], w[V], b[V];
+    load_f(v, xr + c); load_f(w, n.w + c); load_f(b, n.b + c);
+#pragma unroll
+    for (int i = 0; i < V; ++i) v[i] = fmaf(tanhf(n.alpha * v[i]), w[i], b[i]);
+    store_f(out + (size_t)r * width + c, v);
+  }
 }
 
 // ---- RMS norm; the weight is w_offset + w (1: stored as an offset from one, 0: plain) -----------------------------------------
 // rows: NULL = row r of x, else x row rows[r].  out row r.
-template <typename WT, typename OT>
+template <typename WT, typename OT, int V>
 __global__ void rmsnorm_kernel(const float* __restrict__ x, const int* __restrict__ rows, const WT* __restrict__ w,
                                float eps, int width, float w_offset, OT* __restrict__ out) {
   pdl_begin();
@@ -135,11 +158,21 @@ __global__ void rmsnorm_kernel(const float* __restrict__ x, const int* __restric
   const int r = blockIdx.x;
   const float* xr = x + (size_t)(rows ? rows[r] : r) * width;
   float ss = 0.0f;
-  for (int c = threadIdx.x; c < width; c += blockDim.x) { const float v = xr[c]; ss += v * v; }
+  for (int c = threadIdx.x * V; c < width; c += blockDim.x * V) {
+    float v[V];
+    load_f(v, xr + c);
+#pragma unroll
+    for (int i = 0; i < V; ++i) ss += v[i] * v[i];
+  }
   ss = block_sum(ss, red);
   const float inv = 1.0f / sqrtf(ss / (float)width + eps);
-  for (int c = threadIdx.x; c < width; c += blockDim.x)
-    out[(size_t)r * width + c] = from_f<OT>(xr[c] * inv * (w_offset + to_f(w[c])));
+  for (int c = threadIdx.x * V; c < width; c += blockDim.x * V) {
+    float v[V], g[V];
+    load_f(v, xr + c); load_f(g, w + c);
+#pragma unroll
+    for (int i = 0; i < V; ++i) v[i] = v[i] * inv * (w_offset + g[i]);
+    store_f(out + (size_t)r * width + c, v);
+  }
 }
 
 // ---- generic matrix product C[t, n] = sum_k A[t, k] W[n, k], fp32 accumulation in k order -----------------------------------

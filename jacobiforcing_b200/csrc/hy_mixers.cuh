@@ -44,23 +44,40 @@ __device__ __forceinline__ float rotated(const Rotation& r, const float* cs, int
 // It runs as gla_kernel<GLA_TOKEN> (hy_gla.cuh); its state is [slot][heads][nstate][vdim] fp32.  y leaves in fp32 (it enters a norm).
 
 // Gate, then norm: v = y silu(z); each of `parts` equal slices of a row is divided by its own root mean square; times w.
-template <typename AT>
+template <typename AT, int V>
 __global__ void gated_group_norm_kernel(const float* __restrict__ y, int ldy, const AT* __restrict__ z, int ldz,
                                         const float* __restrict__ w, int inner, int parts, float eps, AT* __restrict__ out,
                                         int ldo) {
   pdl_begin();
   __shared__ float red[33];
   const int t = blockIdx.x, part = blockIdx.y, n = inner / parts, c0 = part * n;
-  float ss = 0.0f;
-  for (int c = threadIdx.x; c < n; c += blockDim.x) {
-    const float v = y[(size_t)t * ldy + c0 + c] * silu_f(to_f(z[(size_t)t * ldz + c0 + c]));
-    ss = fmaf(v, v, ss);
+  float ss = 0.0f, held[V];                                    // what the thread's first columns come to, for the second pass
+  auto gated = [&](float (&v)[V], int c) {
+    float g[V];
+    load_f(v, y + (size_t)t * ldy + c0 + c); load_f(g, z + (size_t)t * ldz + c0 + c);
+#pragma unroll
+    for (int i = 0; i < V; ++i) v[i] *= silu_f(g[i]);
+  };
+  for (int c = threadIdx.x * V; c < n; c += blockDim.x * V) {
+    float v[V];
+    gated(v, c);
+#pragma unroll
+    for (int i = 0; i < V; ++i) { ss = fmaf(v[i], v[i], ss); if (c == threadIdx.x * V) held[i] = v[i]; }
   }
   ss = block_sum(ss, red);
   const float inv = 1.0f / sqrtf(ss / (float)n + eps);
-  for (int c = threadIdx.x; c < n; c += blockDim.x) {
-    const float v = y[(size_t)t * ldy + c0 + c] * silu_f(to_f(z[(size_t)t * ldz + c0 + c]));
-    out[(size_t)t * ldo + c0 + c] = from_f<AT>(v * inv * w[c0 + c]);
+  for (int c = threadIdx.x * V; c < n; c += blockDim.x * V) {
+    float v[V], g[V];
+    if (c == threadIdx.x * V) {
+#pragma unroll
+      for (int i = 0; i < V; ++i) v[i] = held[i];
+    } else {
+      gated(v, c);
+    }
+    load_f(g, w + c0 + c);
+#pragma unroll
+    for (int i = 0; i < V; ++i) v[i] = v[i] * inv * g[i];
+    store_f(out + (size_t)t * ldo + c0 + c, v);
   }
 }
 
