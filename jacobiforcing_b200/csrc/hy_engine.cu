@@ -172,7 +172,8 @@ struct hy_engine {
   // row units and the requests' first rows for the kernels
   void* kv_rows = nullptr; void* kv_heads = nullptr; int kv_cap = 0;
   unsigned char* fl_h = nullptr; unsigned char* fl_d = nullptr; size_t fl_cap = 0, fl_used = 0;
-  struct FlashList { int H, window; const jf::FlashUnit* units; const int* keys_of; int n, keys; };
+  struct FlashList { int H, G, window, chunk; const jf::FlashUnit* units; const int* keys_of; int n, keys; };
+  void* page_rows = nullptr;                     // keys and values out of their pages for the length of a layer (page_gather_kernel)
   std::vector<FlashList> fl_lists;
   // cosines and sines of the step's positions, one table per distinct rotation: the layer configuration that names it, the table,
   // its column count; rot_tables_d is what the kernel reads
@@ -629,6 +630,27 @@ int load_gated_experts(hy_engine* h, Builder& B, LayerW& L, const hy_layer_cfg& 
   mx.in = std::max(mx.in, c.x_top * ((ff + 7) & ~7));
   mx.f2 = std::max(mx.f2, c.x_top * W);
   return B.rc;
+}
+
+// Attention over keys and values in pages whose prompt steps may run on jf::flash_kernel: heads of 64 or 128, scores with a positive factor, no cap, no
+// kept positions before a window, no logarithmic distances.
+struct PagedHeads { int H = 0, G = 0, dim = 0, vdim = 0, window = 0, chunk = 0, from = 256; };       // from: tokens of a step (see paged_prompt)
+static bool paged_heads(const hy_engine* h, const hy_layer_cfg& c, PagedHeads& p) {
+  if (h->m.dtype != HY_DTYPE_BF16) return false;
+  auto size = [](int d) { return d == 64 || d == 128; };
+  if (c.mixer == HY_MIX_ATTN_SCAN) {
+    p.H = c.a_heads; p.G = c.a_kv_heads; p.dim = p.vdim = c.a_dim; p.from = 512;
+    return size(c.a_dim) && c.a_scale > 0.0f && c.a_qt_coef >= 0.0f && c.a_qt_every > 0;
+  }
+  if (c.mixer == HY_MIX_BIASED || c.mixer == HY_MIX_ATTN_DELTA) {
+    p.H = c.b_heads; p.G = c.b_kv_heads; p.dim = c.b_dim; p.vdim = c.b_vdim;
+    if (c.mixer == HY_MIX_BIASED) {
+      p.window = c.b_chunk > 0 ? 0 : c.b_window; p.chunk = c.b_chunk;
+      if (c.b_keep_first > 0 || c.b_softcap > 0.0f || c.b_bias == HY_BIAS_LOG) return false;
+    }
+    return size(c.b_dim) && size(c.b_vdim) && c.b_scale > 0.0f;
+  }
+  return false;
 }
 
 // Whether prompt steps of a latent-attention layer may run over per-head keys and values: head sizes that jf::flash_kernel is built for, and a positive
@@ -1475,20 +1497,27 @@ extern "C" int hy_finalize(hy_handle h) {
     }
   }
   {
-    std::set<std::pair<int, int>> lists;                      // (heads, window): the unit lists one step may hold
-    size_t row = 0, heads = 0, maxH = 0;
-    for (auto& c : h->lc)
+    std::set<std::vector<int>> lists;                         // layouts of the unit lists that one step may hold
+    size_t row = 0, heads = 0, maxH = 0, paged = 0;
+    for (auto& c : h->lc) {
+      PagedHeads p;
       if (c.mixer == HY_MIX_LATENT && latent_prompt_sizes(h, c)) {
-        lists.insert({c.l_heads, c.l_window});
+        lists.insert({c.l_heads, c.l_heads, c.l_window, 0});
         row = std::max(row, (size_t)(c.l_kv_rank + c.l_rot_dim));
         heads = std::max(heads, (size_t)c.l_heads * (c.l_dim + c.l_rot_dim + c.l_vdim));
         maxH = std::max(maxH, (size_t)c.l_heads);
+      } else if (paged_heads(h, c, p)) {
+        lists.insert({p.H, p.G, p.window, p.chunk});
+        paged = std::max(paged, (size_t)p.G * (p.dim + p.vdim));
+        maxH = std::max(maxH, (size_t)p.H);
       }
+    }
     if (!lists.empty()) {
       h->kv_cap = 4 * rt.max_step_tokens;
       h->fl_cap = lists.size() * ((T / 128 + rt.max_step_entries) * maxH * sizeof(jf::FlashUnit) + (2 * (size_t)rt.max_step_entries + 1) * 4 + 80);
-      if (dev_alloc(h, &h->kv_rows, (size_t)h->kv_cap * row * 2, &h->bytes_ws)) return HY_ERR_CUDA;
-      if (dev_alloc(h, &h->kv_heads, (size_t)h->kv_cap * heads * 2, &h->bytes_ws)) return HY_ERR_CUDA;
+      if (row > 0 && dev_alloc(h, &h->kv_rows, (size_t)h->kv_cap * row * 2, &h->bytes_ws)) return HY_ERR_CUDA;
+      if (heads > 0 && dev_alloc(h, &h->kv_heads, (size_t)h->kv_cap * heads * 2, &h->bytes_ws)) return HY_ERR_CUDA;
+      if (paged > 0 && dev_alloc(h, &h->page_rows, (size_t)h->kv_cap * paged * 2, &h->bytes_ws)) return HY_ERR_CUDA;
       if (dev_alloc(h, (void**)&h->fl_d, h->fl_cap, &h->bytes_ws)) return HY_ERR_CUDA;
       HY_CUDA(cudaMallocHost((void**)&h->fl_h, h->fl_cap));
     }
@@ -1928,10 +1957,13 @@ bool delta_chunked(hy_engine* h, const Batch& b, int H, int G, int dk, int dv, c
 // made in vain, and steps with more than 32 of those per token keep the folded form: 127 prompt tokens beside a decoded one behind 4000: 313 us,
 // folded 328; behind 7000: 389 against 342.  So do steps whose keys exceed the gathered rows.
 constexpr int HY_FLASH_TOKENS = 64, HY_FLASH_VAIN = 32;
-const hy_engine::FlashList* flash_units(hy_engine* h, int E, int T, int H, int window) {
-  for (const auto& l : h->fl_lists) if (l.H == H && l.window == window) return &l;
+const hy_engine::FlashList* flash_units(hy_engine* h, int E, int T, int H, int G, int window, int chunk) {
+  for (const auto& l : h->fl_lists) if (l.H == H && l.G == G && l.window == window && l.chunk == chunk) return &l;
   if (T < HY_FLASH_TOKENS * E) return nullptr;
-  auto first_key = [&](int e) { return first_seen(h->step_pos0[e], window) / jf::FL_KEYS * jf::FL_KEYS; };
+  auto first_key = [&](int e) {
+    const int p = h->step_pos0[e];
+    return (chunk > 0 ? p / chunk * chunk : first_seen(p, window)) / jf::FL_KEYS * jf::FL_KEYS;
+  };
   long long keys = 0, vain = 0;
   for (int e = 0; e < E; ++e) {
     const int len = h->step_start[e + 1] - h->step_start[e], n = h->step_pos0[e] + len - first_key(e);
@@ -1950,14 +1982,14 @@ const hy_engine::FlashList* flash_units(hy_engine* h, int E, int T, int H, int w
     off[e + 1] = off[e] + h->step_pos0[e] + h->step_start[e + 1] - h->step_start[e] - first[e];
   }
   for (int e = 0; e < E; ++e) {
-    const int len = h->step_start[e + 1] - h->step_start[e];
-    for (int p = (len - 1) / 128 * 128; p >= 0; p -= 128)
-      for (int hd = 0; hd < H; ++hd) u[n++] = jf::FlashUnit{h->step_start[e], len, p, len, hd, hd, h->step_pos0[e], off[e] - first[e], -1};
+    const int len = h->step_start[e + 1] - h->step_start[e], R = H / G, pairs = R * len;
+    for (int p = (pairs - 1) / 128 * 128; p >= 0; p -= 128)
+      for (int g = 0; g < G; ++g) u[n++] = jf::FlashUnit{h->step_start[e], len, p, pairs, g * R, g, h->step_pos0[e], off[e] - first[e], -1};
   }
   const size_t bytes = (unsigned char*)(u + n) - at;
   unsigned char* d = h->fl_d + h->fl_used;
   cudaMemcpyAsync(d, at, bytes, cudaMemcpyHostToDevice, h->stream);
-  h->fl_lists.push_back({H, window, reinterpret_cast<const jf::FlashUnit*>(d + ((unsigned char*)u - at)), reinterpret_cast<const int*>(d), n, (int)keys});
+  h->fl_lists.push_back({H, G, window, chunk, reinterpret_cast<const jf::FlashUnit*>(d + ((unsigned char*)u - at)), reinterpret_cast<const int*>(d), n, (int)keys});
   h->fl_used += (bytes + 63) / 64 * 64;
   return &h->fl_lists.back();
 }
@@ -1968,11 +2000,13 @@ template <typename AT>
 void prepare_units(hy_engine* h, int E, int T) {
   if (!std::is_same<AT, bf16>::value || !h->part_o) return;
   for (const hy_layer_cfg& c : h->lc) {
+    PagedHeads p;
+    if (h->page_rows && paged_heads(h, c, p) && T >= p.from && flash_units(h, E, T, p.H, p.G, p.window, p.chunk)) continue;
     if (c.mixer == HY_MIX_ATTN_SCAN) {
       if (c.a_dim == 32 || c.a_dim == 64 || c.a_dim == 128) attn_units(h, E, T, c.a_heads, c.a_kv_heads);
     } else if (c.mixer == HY_MIX_LATENT) {
       const int Dk = c.l_kv_rank + c.l_rot_dim;
-      if (latent_prompt_sizes(h, c) && flash_units(h, E, T, c.l_heads, c.l_window)) continue;
+      if (latent_prompt_sizes(h, c) && flash_units(h, E, T, c.l_heads, c.l_heads, c.l_window, 0)) continue;
       const bool narrow = (Dk == 32 || Dk == 64 || Dk == 128) && attn_units(h, E, T, c.l_heads, 1, false, c.l_window);
       if (!narrow && Dk % 8 == 0 && c.l_kv_rank <= 512) attn_units(h, E, T, c.l_heads, 1, true, c.l_window);
     } else if (c.mixer == HY_MIX_WINDOW) {
@@ -1986,6 +2020,45 @@ void prepare_units(hy_engine* h, int E, int T) {
   }
 }
 
+// Attention of a prompt step over keys and values out of their pages: gathered once (page_gather_kernel), then as latent_prompt's.  more: the layer's own
+// factors; queries of head h at column h * dim of q, results at column h * vdim of out.  The kernels on mma.sync, which read pages themselves, take 64 keys
+// at a time for 16 rows of a warp, and those of attn_mma_kernel are split among blocks and merged.  2048 tokens of 16 heads of 128 over four key heads:
+// attn_mma_kernel and its merge 189 us, here 90; 16 heads over four, chunks of 1024 with linear distances, two requests: biased_mma_kernel 132, here 49; five
+// requests of 400 tokens, 8 heads over two: 49, here 21.  The line (a layer, us, before -> here): linear distances 250 tokens 148 -> 135, 500 tokens
+// 194 -> 166; without them 253 -> 246 and 308 -> 305; keys that are the values, whose rows go through memory once more: 243 -> 257 and 321 -> 304, so from 512 there.
+bool paged_prompt(hy_engine* h, const Batch& b, const hy_layer_cfg& c, const bf16* q, int ldq, const void* kc, const void* vc, bf16* out, int ldo, jf::FlashArgs more) {
+  PagedHeads p;
+  if (!h->page_rows || !paged_heads(h, c, p) || b.T < p.from) return false;
+  if (ldq % 8 != 0 || ldo % 8 != 0 || ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(out)) & 15) != 0) return false;
+  const hy_engine::FlashList* l = flash_units(h, b.E, b.T, p.H, p.G, p.window, p.chunk);
+  if (!l) return false;
+  if (!h->step_err.empty()) return true;
+  bf16* k = (bf16*)h->page_rows;
+  bf16* v = vc ? k + (size_t)l->keys * p.G * p.dim : k;
+  go_kernel(h, page_gather_kernel, l->keys, 128, 0, h->stream, b, l->keys_of, (const bf16*)kc, (const bf16*)vc, p.G, p.dim, p.vdim, k, v);
+  CUtensorMap km, vm;
+  if (!jf::tp_map(&km, k, (uint64_t)l->keys, (uint64_t)p.G * p.dim, (uint64_t)p.G * p.dim, 128, true) ||
+      !jf::tp_map(&vm, v, (uint64_t)l->keys, (uint64_t)p.G * p.vdim, (uint64_t)p.G * p.vdim, 128, true)) {
+    h->step_err = "a tensor map of the attention could not be made";
+    return true;
+  }
+  more.units = l->units; more.q = q; more.ldq = (size_t)ldq; more.q_head = p.dim; more.kv_heads = 1; more.window = p.window; more.chunk = p.chunk;
+  more.out = out; more.ldo = (size_t)ldo; more.err = h->err_d;
+  auto go = [&](auto dk, auto dv, auto bias) {
+    constexpr int DK = decltype(dk)::value, DV = decltype(dv)::value;
+    go_kernel(h, jf::flash_kernel<DK, DV, true, decltype(bias)::value>, l->n, jf::FL_THREADS, jf::fl_smem_bytes(DK, DV), h->stream, km, vm, more);
+  };
+  typedef std::integral_constant<int, 64> c64; typedef std::integral_constant<int, 128> c128;
+  auto sized = [&](auto bias) {
+    if (p.dim == 64) { if (p.vdim == 64) go(c64{}, c64{}, bias); else go(c64{}, c128{}, bias); }
+    else { if (p.vdim == 64) go(c128{}, c64{}, bias); else go(c128{}, c128{}, bias); }
+  };
+  if (more.slope) sized(std::true_type{});
+  else sized(std::false_type{});
+  h->launches += 2;
+  return true;
+}
+
 // Latent attention of a prompt step over per-head keys and values: one product of the cache rows that the step's requests see gives
 // them (each head's key: its part of the up-projection, then the rotated part as it is), and attention runs over heads of dim + rot
 // and vdim instead of rank + rot and rank.  1531 tokens behind 2048, 16 heads of 128 + 64 over a rank of 512: the folded form does
@@ -1996,7 +2069,7 @@ void prepare_units(hy_engine* h, int E, int T) {
 bool latent_prompt(hy_engine* h, const Batch& b, const LayerW& L, const hy_layer_cfg& c) {
   if (!L.w_kv_t) return false;
   const int H = c.l_heads, hk = c.l_dim + c.l_rot_dim, dv = c.l_vdim, K = c.l_kv_rank + c.l_rot_dim, N = H * (hk + dv);
-  const hy_engine::FlashList* l = flash_units(h, b.E, b.T, H, c.l_window);
+  const hy_engine::FlashList* l = flash_units(h, b.E, b.T, H, H, c.l_window, 0);
   if (!l) return false;
   cudaStream_t s = h->stream;
   bf16* pin = (bf16*)h->pin; bf16* kv = (bf16*)h->kv_heads;
@@ -2621,7 +2694,13 @@ void biased_attend(hy_engine* h, const Batch& b, const LayerW& L, const hy_layer
     (void)u;
     if constexpr (std::is_same<AT, bf16>::value) {
       static const bool simt_only = getenv("HY_BIASED_SIMT") != nullptr;      // developer switch
-      if (!simt_only && c.b_dim % 8 == 0 && c.b_vdim % 8 == 0 && c.b_dim <= 128 && c.b_vdim <= 128 && h->ld_pin % 8 == 0 && L.c_q % 8 == 0 && h->units_d &&
+      jf::FlashArgs fa{};
+      fa.scale = bc.scale; fa.sink_f = bc.sink; fa.slope = bc.bias == HY_BIAS_LINEAR ? bc.r1 : nullptr; fa.head_gate = bc.gate; fa.ld_head = (size_t)bc.ldg;
+      fa.scaled = 1; fa.out_scale = bc.out_scale;
+      if (!simt_only && paged_prompt(h, b, c, pin + L.c_q, h->ld_pin, L.cache, L.cache_v, cat, h->ld_cat, fa)) {
+        tc = true;
+        h->launches--;                                         // counted with the one below
+      } else if (!simt_only && c.b_dim % 8 == 0 && c.b_vdim % 8 == 0 && c.b_dim <= 128 && c.b_vdim <= 128 && h->ld_pin % 8 == 0 && L.c_q % 8 == 0 && h->units_d &&
           (u = biased_units(h, E, T, bc, dp))) {
         tc = true;
 #define HY_BIASED_ARGS b, u->d, pin + L.c_q, h->ld_pin, bc, (const bf16*)L.cache, (const bf16*)L.cache_v, cat, h->ld_cat, u->ns, h->part_o, h->part_ml
@@ -3019,7 +3098,13 @@ int run_step(hy_engine* h, const Batch& b, int n_want, const int* want_d, float*
       const UnitList* u = nullptr;
       (void)u;
       if constexpr (std::is_same<AT, bf16>::value) {
-        if ((c.a_dim == 32 || c.a_dim == 64 || c.a_dim == 128) && h->part_o && (u = attn_units(h, E, T, c.a_heads, c.a_kv_heads))) {
+        jf::FlashArgs fa{};
+        fa.scale = c.a_scale; fa.sink = (const bf16*)L.sink; fa.gate = pin + L.c_g; fa.ldg = (size_t)h->ld_pin; fa.temp_coef = c.a_qt_coef; fa.temp_every = c.a_qt_every;
+        fa.scaled = 1; fa.out_scale = c.left_scale;
+        if (paged_prompt(h, b, c, cv, h->ld_cv, L.cache, nullptr, cat + L.o_mix, h->ld_cat, fa)) {
+          tc = true;
+          h->launches--;                                       // counted with the one below
+        } else if ((c.a_dim == 32 || c.a_dim == 64 || c.a_dim == 128) && h->part_o && (u = attn_units(h, E, T, c.a_heads, c.a_kv_heads))) {
           tc = true;
 #define HY_ATTN_ARGS b, u->d, cv, h->ld_cv, (const bf16*)L.cache, c.a_heads, c.a_kv_heads, c.a_scale, c.a_qt_coef, \
           c.a_qt_every, 0, u->split, u->ns, c.a_dim, h->part_o, h->part_ml

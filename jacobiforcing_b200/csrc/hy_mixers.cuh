@@ -197,6 +197,24 @@ __global__ void __launch_bounds__(128) latent_gather_kernel(Batch b, const int* 
     reinterpret_cast<uint4*>(out + (size_t)blockIdx.x * dim)[k] = reinterpret_cast<const uint4*>(src)[k];
 }
 
+// The keys and values that a step's requests see, out of their pages and one after the other: k [keys][G dim], v [keys][G vdim] (NULL: the values are the
+// keys).  keys_of as in latent_gather_kernel; sizes in multiples of eight.
+__global__ void __launch_bounds__(128) page_gather_kernel(Batch b, const int* __restrict__ keys_of, const bf16* __restrict__ kc, const bf16* __restrict__ vc, int G,
+                                                          int dim, int vdim, bf16* __restrict__ k, bf16* __restrict__ v) {
+  pdl_begin();
+  int e = 0;
+  while ((int)blockIdx.x >= keys_of[e + 1]) ++e;
+  const int j = blockIdx.x - keys_of[e] + keys_of[b.E + 1 + e];
+  const size_t page = b.pages[(size_t)e * b.max_pages + j / b.page_size];
+  const int slot = j % b.page_size, nk = G * (dim / 8), nv = vc ? G * (vdim / 8) : 0;
+  for (int i = threadIdx.x; i < nk + nv; i += blockDim.x) {
+    const bool key = i < nk;
+    const int w = (key ? dim : vdim) / 8, at = key ? i : i - nk, g = at / w, c = at % w;
+    reinterpret_cast<uint4*>((key ? k + (size_t)blockIdx.x * G * dim : v + (size_t)blockIdx.x * G * vdim))[at] =
+        reinterpret_cast<const uint4*>((key ? kc : vc) + ((page * G + g) * b.page_size + slot) * (key ? dim : vdim))[c];
+  }
+}
+
 // The value up-projection behind the weighted sum: out[t, h, j] = sum_r w_uvT[h][r][j] o[t, h, r]  (o fp32: the weighted
 // sum of latents; w_uvT is the value up-projection transposed per head at load so that thread j reads coalesced).  gate (NULL: none):
 // the result times sigmoid(gate[t, h * vdim + j]).

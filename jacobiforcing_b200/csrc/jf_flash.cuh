@@ -45,6 +45,14 @@ struct FlashArgs {
   __nv_bfloat16* out; size_t ldo;                        // row-major [row, head * DV + d], or (packed_rows > 0) [chunk of 64][packed_rows][64] swizzled
   int packed_rows;
   int* err;
+  // beyond what every caller has (zeros: none of it)
+  int chunk;                                             // position i sees no keys before i / chunk * chunk (instead of a window)
+  float temp_coef; int temp_every;                       // scores times 1 + coef ln(floor((i + 1) / every) + 1) as well
+  const float* slope;                                    // [heads] slope (i - j) is taken off a score (kernels with BIAS)
+  const float* sink_f;                                   // the sinks as fp32
+  const float* head_gate; size_t ld_head;                // output times sigmoid(head_gate[row, head])
+  int scaled; float out_scale;                           // scaled: output times out_scale
+  __device__ __forceinline__ int first(int pos) const { return chunk > 0 ? pos / chunk * chunk : window > 0 ? max(0, pos - window + 1) : 0; }
 };
 
 constexpr int FL_MAX_STAGES = 2;
@@ -82,17 +90,17 @@ __device__ __forceinline__ void fl_load(void* dst, const CUtensorMap* map, int x
 // The key tiles of a unit, aligned to absolute positions: first one's number, how many.
 struct FlTiles {
   int lo, n;
-  __device__ FlTiles(const FlashUnit& u, int window) {
-    const int rows = min(FL_ROWS, u.pairs - u.pair0), a = u.pair0 % u.len, b = a + rows - 1;
-    const int first_tok = b < u.len ? a : 0, last_tok = b < u.len ? b : u.len - 1;
-    lo = (window > 0 ? max(0, u.pos0 + first_tok - window + 1) : 0) / FL_KEYS;
+  __device__ FlTiles(const FlashUnit& u, const FlashArgs& a) {
+    const int rows = min(FL_ROWS, u.pairs - u.pair0), i = u.pair0 % u.len, b = i + rows - 1;
+    const int first_tok = b < u.len ? i : 0, last_tok = b < u.len ? b : u.len - 1;
+    lo = a.first(u.pos0 + first_tok) / FL_KEYS;
     n = (u.pos0 + last_tok) / FL_KEYS + 1 - lo;
   }
 };
 // 2^y in units of the last place of ex2.approx; what would be subnormal is zero
 __device__ __forceinline__ float fl_exp2(float y) { float r; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(y)); return r; }
 
-template <int DK, int DV, bool SPLIT, int BLOCKS = fl_stages(DK) == 1 ? 2 : 1>
+template <int DK, int DV, bool SPLIT, bool BIAS = false, int BLOCKS = fl_stages(DK) == 1 ? 2 : 1>
 __global__ void __launch_bounds__(FL_THREADS, BLOCKS)
 flash_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap, FlashArgs a) {
   extern __shared__ __align__(1024) unsigned char fl_smem[];
@@ -117,7 +125,7 @@ flash_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ C
   pdl_trigger();                                           // this block owns its columns
   pdl_wait();
   const FlashUnit u = a.units[blockIdx.x];
-  const FlTiles t(u, a.window);
+  const FlTiles t(u, a);
   const uint32_t tm = sm->tmem_base;
 
   if (warp == 0) {
@@ -205,8 +213,10 @@ flash_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ C
         fence_proxy_async_smem();
         mbar_arrive(&sm->q_full);
       }
-      const float c2 = a.scale * 1.4426950408889634f;           // scores in units of log 2
-      const int first = a.window > 0 ? max(0, pos - a.window + 1) : 0;
+      float c2 = a.scale * 1.4426950408889634f;                 // scores in units of log 2
+      if (a.temp_every > 0) c2 *= 1.0f + a.temp_coef * logf(floorf((float)(pos + 1) / (float)a.temp_every) + 1.0f);
+      const float sl = BIAS ? a.slope[head] * 1.4426950408889634f : 0.0f;
+      const int first = a.first(pos);
       float m = -INFINITY, l = 0.0f;                            // reference point and sum of the weights so far
       bool ok = true;
       for (int i = 0; i < t.n; ++i) {
@@ -234,6 +244,11 @@ flash_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ C
             tmem_st16(ts + c * 32, *reinterpret_cast<uint32_t(*)[16]>(&v[0]));
             tmem_st16(ts + c * 32 + 16, *reinterpret_cast<uint32_t(*)[16]>(&v[16]));
           }
+          if constexpr (BIAS) {                                 // what is compared are the scores as they enter the exponential
+            const float from = sl * (float)(k0 + c * 32 - pos);
+#pragma unroll
+            for (int k = 0; k < 32; ++k) v[k] = __float_as_uint(fmaf(__uint_as_float(v[k]), c2, fmaf(sl, (float)k, from)));
+          }
 #pragma unroll
           for (int k = 0; k < 32; k += 4) {
             m0 = fmaxf(m0, __uint_as_float(v[k])); m1 = fmaxf(m1, __uint_as_float(v[k + 1]));
@@ -244,7 +259,7 @@ flash_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ C
         m0 = fmaxf(fmaxf(m0, m1), fmaxf(m2, m3));
         sm->part[half][r] = m0;
         named_bar_sync(1, 256);
-        const float top = fmaxf(m0, sm->part[half ^ 1][r]) * c2;
+        const float top = fmaxf(m0, sm->part[half ^ 1][r]) * (BIAS ? 1.0f : c2);
         const bool moves = top > m + 8.0f || (m == -INFINITY && top > -INFINITY);
         float grow = 1.0f;
         if (moves) { grow = fl_exp2(m - top); m = top; l *= grow; }
@@ -254,9 +269,11 @@ flash_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ C
         for (int c = 2 * half; c < 2 * half + 2; ++c) {         // their weights in their place: 16 columns, and 16 of the remainders
           uint32_t v[32], hi[16], rest[SPLIT ? 16 : 1];
           piece(c, v);
+          const float from = BIAS ? fmaf(sl, (float)(k0 + c * 32 - pos), -ref) : -ref;
 #pragma unroll
           for (int k = 0; k < 32; k += 2) {
-            const float e0 = fl_exp2(fmaf(__uint_as_float(v[k]), c2, -ref)), e1 = fl_exp2(fmaf(__uint_as_float(v[k + 1]), c2, -ref));
+            const float e0 = fl_exp2(fmaf(__uint_as_float(v[k]), c2, BIAS ? fmaf(sl, (float)k, from) : from));
+            const float e1 = fl_exp2(fmaf(__uint_as_float(v[k + 1]), c2, BIAS ? fmaf(sl, (float)(k + 1), from) : from));
             s0 += e0; s1 += e1;
             const uint32_t h = pack_bf16x2(e0, e1);
             hi[k >> 1] = h;
@@ -300,7 +317,10 @@ flash_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ C
       if (ok) {
         l += sm->part[half ^ 1][r];
         if (a.sink) l += exp2f(__bfloat162float(a.sink[head]) * 1.4426950408889634f - m);
-        const float inv = 1.0f / l;
+        if (a.sink_f) l += exp2f(a.sink_f[head] * 1.4426950408889634f - m);
+        float inv = 1.0f / l;
+        if (a.scaled) inv *= a.out_scale;
+        if (a.head_gate) inv *= 1.0f / (1.0f + expf(-a.head_gate[row * a.ld_head + head]));
         const __nv_bfloat16* gate = a.gate ? a.gate + row * a.ldg + (size_t)head * DV : nullptr;
 #pragma unroll 1
         for (int c = half * (DV / 32); c < (half + 1) * (DV / 32); ++c) {      // over the queries: the last scores are made
