@@ -166,7 +166,7 @@ struct hy_engine {
   AttnUnit* units_d = nullptr; AttnUnit* units_h = nullptr; size_t units_cap = 0, units_used = 0;
   std::vector<UnitList> unit_lists;
   int step_tokens = 0;
-  bool plain = false;                            // launches of the running step do not overlap (see go_kernel)
+  bool plain = false;                            // launches do not overlap (see go_kernel)
   float* part_sums = nullptr; int* part_arrived = nullptr;      // partial sums of products with few tiles (jf::PairSplit)
   // prompt steps of latent attention: keys of a step's requests one after the other (cache rows, then per-head keys and values),
   // row units and the requests' first rows for the kernels
@@ -196,16 +196,21 @@ struct hy_engine {
     }                                                                                                   \
   } while (0)
 
-// Launch of a kernel of a step.  In steps of few tokens it may start once every block of the kernel before it has started (see
-// pdl_wait), so that its own start, its barriers and its first weights overlap the end of that kernel: a Kinetar decode step is 42
-// kernels of 2 to 9 us each (request of 512 + 24 tokens: 10.66 -> 9.47 ms).  Prompt steps keep plain launches: the blocks of a
-// kernel that starts under another one's tail pile up on the SMs that are free already, and a recurrence with one block per
-// SM then runs two or three on some of them (two Kinetar layers, 2048 tokens: 2.02 ms plain, 2.35 ms overlapped).
+// Launch of a kernel of a step.  It may start once every block of the kernel before it has started (see pdl_wait), so that its own start, its barriers and
+// its first weights overlap the end of that kernel: a Kinetar decode step is 42 kernels of 2 to 9 us each (request of 512 + 24 tokens: 10.66 -> 9.47 ms),
+// and a step of prompt tokens as many.  The blocks of a kernel that starts under another one's tail pile up on the SMs that are free already, though, and
+// a recurrence with one block per SM then runs two or three on some of them (two Kinetar layers, 2048 tokens, everything overlapped: 2.02 -> 2.35 ms).  So the
+// kernels whose longest block is their time start behind the kernel before them in steps of more than HY_OVERLAP_TOKENS tokens (go_alone): recurrences and
+// attention over pages; convolutions from HY_ALONE_CONV tokens on.  A layer of one request, us, everything behind one another -> so: 77 tokens of Kinetar's
+// delta rule 146 -> 129, gated linear attention 123 -> 109, its attention beside a scan 187 -> 171; 200 tokens of latent attention 127 -> 110; 1024 tokens
+// of a state-space layer 301 -> 275, of retention 230 -> 219; 2048 tokens of latent attention 237 -> 212, of retention beside experts in four requests 294 -> 264.
+// With convolutions overlapped as well, attention beside a scan takes 445 instead of 419 (1024 tokens); with none, 208 instead of 202 (150 tokens).
+// Steps just above HY_OVERLAP_TOKENS keep plain launches, which test_which_launches_overlap holds them to.
 // Behind the first launch of a step that fails nothing else is launched; hy_step reports it.
 // More shared memory than every kernel may have (48 KiB with its static part) is asked for here, once per engine and kernel: the limit belongs to a
 // device, and a process may hold engines on several.  Always all that the device has: engines of one device share the limit, and what a
 // smaller one asked for would be too little for a larger one.
-constexpr int HY_OVERLAP_TOKENS = 64;
+constexpr int HY_OVERLAP_TOKENS = 64, HY_OVERLAP_AGAIN = 72, HY_ALONE_CONV = 256;
 constexpr size_t HY_PLAIN_SMEM = 16 * 1024;
 inline cudaError_t opt_in(hy_engine* h, const void* kernel, size_t smem) {
   if (smem <= HY_PLAIN_SMEM || h->opted_in.count(kernel)) return cudaSuccess;
@@ -222,11 +227,20 @@ inline void go_kernel(hy_engine* h, void (*kernel)(P...), dim3 grid, dim3 block,
   at.val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t c = {};
   c.gridDim = grid; c.blockDim = block; c.dynamicSmemBytes = smem; c.stream = stream; c.attrs = &at;
-  c.numAttrs = h->step_tokens <= HY_OVERLAP_TOKENS && !h->plain ? 1 : 0;
+  c.numAttrs = h->plain || (h->step_tokens > HY_OVERLAP_TOKENS && h->step_tokens < HY_OVERLAP_AGAIN) ? 0 : 1;
   if (!h->step_err.empty()) return;
   cudaError_t e = opt_in(h, (const void*)kernel, smem);
   if (e == cudaSuccess) e = cudaLaunchKernelEx(&c, kernel, std::forward<A>(args)...);
   if (e != cudaSuccess) h->step_err = cudaGetErrorString(e);
+}
+
+// A kernel that starts behind the one before it in steps of more than `tokens` tokens (see go_kernel).
+template <typename... A>
+inline void go_alone(hy_engine* h, int tokens, A&&... args) {
+  const bool was = h->plain;
+  h->plain = was || h->step_tokens > tokens;
+  go_kernel(h, std::forward<A>(args)...);
+  h->plain = was;
 }
 
 struct ProfScope {
@@ -1841,7 +1855,7 @@ void launch_conv(hy_engine* h, const Batch& b, const AT* u, int ldu, int col0, i
   auto go = [&](auto v, auto tp) {
     constexpr int V = decltype(v)::value, TP = decltype(tp)::value;
     const int per = 128 * V;
-    go_kernel(h, conv_kernel<AT, WT, V, TP>, dim3((C + per - 1) / per, chunks), 128, 0, h->stream, b, u, ldu, col0, C, taps, (const WT*)w, (const WT*)bias, silu,
+    go_alone(h, HY_ALONE_CONV - 1, conv_kernel<AT, WT, V, TP>, dim3((C + per - 1) / per, chunks), 128, 0, h->stream, b, u, ldu, col0, C, taps, (const WT*)w, (const WT*)bias, silu,
                                                                                         state, o);
   };
   if (vec && taps == 4) go(std::integral_constant<int, 4>{}, std::integral_constant<int, 4>{});
@@ -1913,9 +1927,9 @@ bool gla_chunked(hy_engine* h, const Batch& b, int H, int dk, int dv, const AT* 
   a.states = h->ch_states; a.ends = h->ch_ends; a.state = state; a.o = o; a.ldo = ldo; a.tk = tk;
   auto go = [&](auto k, auto c) {
     constexpr int DK = decltype(k)::value, DV = decltype(c)::value;
-    go_kernel(h, gla_chunk_state_kernel<AT, DK, DV, MODE>, dim3(chunks, H), 256, ch_state_smem<DK, DV, MODE>(), h->stream, a);
-    go_kernel(h, gla_chunk_scan_kernel<AT, DK, DV>, dim3(DK * DV / 1024, H, b.E), 256, 0, h->stream, a);
-    go_kernel(h, gla_chunk_out_kernel<AT, DK, DV, MODE>, dim3(chunks, H), 256, ch_out_smem<AT, DK, DV>(), h->stream, a);
+    go_alone(h, HY_OVERLAP_TOKENS, gla_chunk_state_kernel<AT, DK, DV, MODE>, dim3(chunks, H), 256, ch_state_smem<DK, DV, MODE>(), h->stream, a);
+    go_alone(h, HY_OVERLAP_TOKENS, gla_chunk_scan_kernel<AT, DK, DV>, dim3(DK * DV / 1024, H, b.E), 256, 0, h->stream, a);
+    go_alone(h, HY_OVERLAP_TOKENS, gla_chunk_out_kernel<AT, DK, DV, MODE>, dim3(chunks, H), 256, ch_out_smem<AT, DK, DV>(), h->stream, a);
   };
   typedef std::integral_constant<int, 64> c64; typedef std::integral_constant<int, 128> c128;
   if (dk <= 64 && dv <= 64) go(c64{}, c64{});
@@ -1936,8 +1950,8 @@ bool delta_chunked(hy_engine* h, const Batch& b, int H, int G, int dk, int dv, c
   auto go = [&](auto k, auto c) {
     constexpr int DK = decltype(k)::value, DV = decltype(c)::value;
     static_assert(DeltaWork<DK, DV>::SIZE == delta_work_floats(DK, DV), "the workspace holds what the kernels lay out");
-    go_kernel(h, delta_chunk_prep_kernel<AT, DK, DV>, dim3(chunks, H), 256, delta_prep_smem<DK, DV>(), h->stream, a);
-    go_kernel(h, delta_chunk_chain_kernel<AT, DK, DV>, dim3(H * (DV / DELTA_COLS), b.E), 256, delta_chain_smem<DK>(), h->stream, a);
+    go_alone(h, HY_OVERLAP_TOKENS, delta_chunk_prep_kernel<AT, DK, DV>, dim3(chunks, H), 256, delta_prep_smem<DK, DV>(), h->stream, a);
+    go_alone(h, HY_OVERLAP_TOKENS, delta_chunk_chain_kernel<AT, DK, DV>, dim3(H * (DV / DELTA_COLS), b.E), 256, delta_chain_smem<DK>(), h->stream, a);
   };
   typedef std::integral_constant<int, 64> c64; typedef std::integral_constant<int, 128> c128;
   if (dk <= 64 && dv <= 64) go(c64{}, c64{});
@@ -2152,9 +2166,9 @@ void latent_mixer(hy_engine* h, const Batch& b, const LayerW& L, const hy_layer_
         tc = true;
 #define HY_ATTN_ARGS b, u->d, cv, h->ld_cv, (const bf16*)L.cache, H, 1, c.l_scale, 0.0f, 1, c.l_window, u->split, u->ns, R, \
         h->part_o, h->part_ml
-        if (Dk == 32) go_kernel(h, attn_mma_kernel<32>, u->n, 128, 0, s, HY_ATTN_ARGS);
-        else if (Dk == 64) go_kernel(h, attn_mma_kernel<64>, u->n, 128, 0, s, HY_ATTN_ARGS);
-        else go_kernel(h, attn_mma_kernel<128>, u->n, 128, 0, s, HY_ATTN_ARGS);
+        if (Dk == 32) go_alone(h, HY_OVERLAP_TOKENS, attn_mma_kernel<32>, u->n, 128, 0, s, HY_ATTN_ARGS);
+        else if (Dk == 64) go_alone(h, HY_OVERLAP_TOKENS, attn_mma_kernel<64>, u->n, 128, 0, s, HY_ATTN_ARGS);
+        else go_alone(h, HY_OVERLAP_TOKENS, attn_mma_kernel<128>, u->n, 128, 0, s, HY_ATTN_ARGS);
 #undef HY_ATTN_ARGS
         go_kernel(h, attn_combine_kernel<WT, float>, T * H, 64, 0, s, b, h->part_o, h->part_ml, (const WT*)L.sink, nullptr, 0, H, 1, Dk, R,
                                                             c.l_window, u->split, u->ns, 1.0f, h->f2, h->ld_f2);
@@ -2179,7 +2193,7 @@ void latent_mixer(hy_engine* h, const Batch& b, const LayerW& L, const hy_layer_
       }
     }
     if (!tc) {
-      go_kernel(h, attn_sink_kernel<AT, WT, float>, (T * H + 3) / 4, 128, 4 * Dk * sizeof(float), s, 
+      go_alone(h, HY_OVERLAP_TOKENS, attn_sink_kernel<AT, WT, float>, (T * H + 3) / 4, 128, 4 * Dk * sizeof(float), s, 
           b, cv, h->ld_cv, (const AT*)L.cache, (const WT*)L.sink, (const AT*)nullptr, 0, H, 1, Dk, R, c.l_scale, 0.0f, 1, c.l_window, 1.0f,
           h->f2, h->ld_f2);
       h->launches++;
@@ -2292,7 +2306,7 @@ int sandwich_layer(hy_engine* h, const Batch& b, size_t li) {
         constexpr int DR = decltype(dr)::value, PARTS = decltype(parts)::value, VC = decltype(vcols)::value;
         const LinearLaunch g = linear_launch<AT>(PARTS, VC, N, P, cv, h->ld_cv);
         const size_t smem = lin_smem<AT>(DR, PARTS, VC, 0);
-        go_kernel(h, gla_kernel<AT, DR, PARTS, VC, GLA_TOKEN>, dim3(H * g.bph, E), 128, smem, s, b, h->lin, cv, h->ld_cv, nullptr, 0, nullptr, H, N, P, g.bph,
+        go_alone(h, HY_OVERLAP_TOKENS, gla_kernel<AT, DR, PARTS, VC, GLA_TOKEN>, dim3(H * g.bph, E), 128, smem, s, b, h->lin, cv, h->ld_cv, nullptr, 0, nullptr, H, N, P, g.bph,
                                                                                    g.vec, g.vvec, L.rec_state, h->f2, h->ld_f2, tk);
       });
       const auto gate = [&](auto v) {
@@ -2327,13 +2341,13 @@ int sandwich_layer(hy_engine* h, const Batch& b, size_t li) {
         constexpr int DR = decltype(dr)::value, PARTS = decltype(parts)::value, VC = decltype(vcols)::value;
         const LinearLaunch g = linear_launch<AT>(PARTS, VC, dk, dv, pin + L.c_v, h->ld_pin);
         const size_t smem = lin_smem<AT>(DR, PARTS, VC, 0);
-        go_kernel(h, gla_kernel<AT, DR, PARTS, VC, GLA_FORGET>, dim3(H * g.bph, E), 128, smem, s, b, h->lin, pin + L.c_v, h->ld_pin, nullptr, 0, nullptr, H, dk,
+        go_alone(h, HY_OVERLAP_TOKENS, gla_kernel<AT, DR, PARTS, VC, GLA_FORGET>, dim3(H * g.bph, E), 128, smem, s, b, h->lin, pin + L.c_v, h->ld_pin, nullptr, 0, nullptr, H, dk,
                                                                                     dv, g.bph, g.vec, g.vvec, L.rec_state, h->f2, h->ld_f2, GlaToken{});
       });
       launch_gla_out<AT, AT, GATE_NONE>(h, T, H, dv, h->f2, h->ld_f2, nullptr, 0, L.g_norm, eps, 1.0f, cat, h->ld_cat);
       h->launches += 3;
     } else {
-      go_kernel(h, glr_kernel<AT>, dim3(H, E), 256, ((size_t)dk * dv + 2 * dk + dv + 40) * 4, s, 
+      go_alone(h, HY_OVERLAP_TOKENS, glr_kernel<AT>, dim3(H, E), 256, ((size_t)dk * dv + 2 * dk + dv + 40) * 4, s, 
           b, pin, h->ld_pin, L.c_q, L.c_k, L.c_v, L.g_fb, L.g_lower, L.g_norm, H, dk, dv, eps, L.rec_state, cat, h->ld_cat);
       h->launches++;
     }
@@ -2706,11 +2720,11 @@ void biased_attend(hy_engine* h, const Batch& b, const LayerW& L, const hy_layer
 #define HY_BIASED_ARGS b, u->d, pin + L.c_q, h->ld_pin, bc, (const bf16*)L.cache, (const bf16*)L.cache_v, cat, h->ld_cat, u->ns, h->part_o, h->part_ml
         const bool pl = bc.bias == HY_BIAS_NONE && bc.cap <= 0.0f && !bc.window && !bc.keep && !bc.chunk;
         if (dp == 64) {
-          if (pl) go_kernel(h, biased_mma_kernel<64, true>, u->n, 128, window_mma_smem(64), s, HY_BIASED_ARGS);
-          else go_kernel(h, biased_mma_kernel<64, false>, u->n, 128, window_mma_smem(64), s, HY_BIASED_ARGS);
+          if (pl) go_alone(h, HY_OVERLAP_TOKENS, biased_mma_kernel<64, true>, u->n, 128, window_mma_smem(64), s, HY_BIASED_ARGS);
+          else go_alone(h, HY_OVERLAP_TOKENS, biased_mma_kernel<64, false>, u->n, 128, window_mma_smem(64), s, HY_BIASED_ARGS);
         } else {
-          if (pl) go_kernel(h, biased_mma_kernel<128, true>, u->n, 128, window_mma_smem(128), s, HY_BIASED_ARGS);
-          else go_kernel(h, biased_mma_kernel<128, false>, u->n, 128, window_mma_smem(128), s, HY_BIASED_ARGS);
+          if (pl) go_alone(h, HY_OVERLAP_TOKENS, biased_mma_kernel<128, true>, u->n, 128, window_mma_smem(128), s, HY_BIASED_ARGS);
+          else go_alone(h, HY_OVERLAP_TOKENS, biased_mma_kernel<128, false>, u->n, 128, window_mma_smem(128), s, HY_BIASED_ARGS);
         }
 #undef HY_BIASED_ARGS
         if (u->ns > 1) {
@@ -2720,7 +2734,7 @@ void biased_attend(hy_engine* h, const Batch& b, const LayerW& L, const hy_layer
       }
     }
     if (!tc)
-      go_kernel(h, biased_attn_kernel<AT, AT>, (T * c.b_heads + 3) / 4, 128, 4 * c.b_dim * sizeof(float), s, 
+      go_alone(h, HY_OVERLAP_TOKENS, biased_attn_kernel<AT, AT>, (T * c.b_heads + 3) / 4, 128, 4 * c.b_dim * sizeof(float), s, 
           b, pin + L.c_q, h->ld_pin, bc, (const AT*)L.cache, (const AT*)L.cache_v, cat, h->ld_cat);
     h->launches++;
   }
@@ -2832,7 +2846,7 @@ void gla_mixer(hy_engine* h, const Batch& b, const LayerW& L, const hy_layer_cfg
     constexpr int DR = decltype(dr)::value, PARTS = decltype(parts)::value, VC = decltype(vcols)::value;
     const LinearLaunch g = linear_launch<AT>(PARTS, VC, dk, dv, pin + L.c_v, h->ld_pin);
     const size_t smem = lin_smem<AT>(DR, PARTS, VC, DR);
-    go_kernel(h, gla_kernel<AT, DR, PARTS, VC, GLA_CHANNEL>, dim3(H * g.bph, E), 128, smem, s, b, h->lin, pin + L.c_v, h->ld_pin, h->f2, h->ld_f2, nullptr, H, dk,
+    go_alone(h, HY_OVERLAP_TOKENS, gla_kernel<AT, DR, PARTS, VC, GLA_CHANNEL>, dim3(H * g.bph, E), 128, smem, s, b, h->lin, pin + L.c_v, h->ld_pin, h->f2, h->ld_f2, nullptr, H, dk,
                                                                            dv, g.bph, g.vec, g.vvec, L.rec_state, h->f2 + c_o, h->ld_f2, GlaToken{});
   });
   launch_gla_out<AT, AT, GATE_SILU>(h, T, H, dv, h->f2 + c_o, h->ld_f2, pin + L.c_g, h->ld_pin, L.g_norm, h->m.norm_eps,
@@ -2855,7 +2869,7 @@ void retention_mixer(hy_engine* h, const Batch& b, const LayerW& L, const hy_lay
     constexpr int DR = decltype(dr)::value, PARTS = decltype(parts)::value, VC = decltype(vcols)::value;
     const LinearLaunch g = linear_launch<AT>(PARTS, VC, dk, dv, pin + L.c_v, h->ld_pin);
     const size_t smem = lin_smem<AT>(DR, PARTS, VC, 0);
-    go_kernel(h, gla_kernel<AT, DR, PARTS, VC, GLA_HEAD>, dim3(H * g.bph, E), 128, smem, s, b, h->lin, pin + L.c_v, h->ld_pin, nullptr, 0, L.decay, H, dk, dv,
+    go_alone(h, HY_OVERLAP_TOKENS, gla_kernel<AT, DR, PARTS, VC, GLA_HEAD>, dim3(H * g.bph, E), 128, smem, s, b, h->lin, pin + L.c_v, h->ld_pin, nullptr, 0, L.decay, H, dk, dv,
                                                                           g.bph, g.vec, g.vvec, L.rec_state, h->f2, h->ld_f2, GlaToken{});
   });
   launch_gla_out<AT, AT, GATE_SILU>(h, T, H, dv, h->f2, h->ld_f2, pin + L.c_g, h->ld_pin, nullptr, h->m.norm_eps, 1.0f, cat,
@@ -2893,7 +2907,7 @@ void attn_delta_mixer(hy_engine* h, const Batch& b, const LayerW& L, const hy_la
     constexpr int DR = decltype(dr)::value, PARTS = decltype(parts)::value, VC = decltype(vcols)::value;
     const LinearLaunch g = linear_launch<AT>(PARTS, VC, dk, dv, cv, h->ld_cv);
     const size_t smem = lin_smem<AT>(DR, PARTS, VC, 4);
-    go_kernel(h, delta_head_kernel<AT, DR, PARTS, VC, false>, dim3(H * g.bph, E), 128, smem, s, b, h->lin, cv, h->ld_cv, h->lin_sc, H, G, dk, dv, g.bph, g.vec, g.vvec,
+    go_alone(h, HY_OVERLAP_TOKENS, delta_head_kernel<AT, DR, PARTS, VC, false>, dim3(H * g.bph, E), 128, smem, s, b, h->lin, cv, h->ld_cv, h->lin_sc, H, G, dk, dv, g.bph, g.vec, g.vvec,
                                                                            L.rec_state, h->f2, h->ld_f2, nullptr, 0);
   });
   launch_gla_out<AT, AT, GATE_SILU>(h, T, H, dv, h->f2, h->ld_f2, pin + L.c_g, h->ld_pin, L.g_norm, h->m.norm_eps,
@@ -3108,9 +3122,9 @@ int run_step(hy_engine* h, const Batch& b, int n_want, const int* want_d, float*
           tc = true;
 #define HY_ATTN_ARGS b, u->d, cv, h->ld_cv, (const bf16*)L.cache, c.a_heads, c.a_kv_heads, c.a_scale, c.a_qt_coef, \
           c.a_qt_every, 0, u->split, u->ns, c.a_dim, h->part_o, h->part_ml
-          if (c.a_dim == 32) go_kernel(h, attn_mma_kernel<32>, u->n, 128, 0, s, HY_ATTN_ARGS);
-          else if (c.a_dim == 64) go_kernel(h, attn_mma_kernel<64>, u->n, 128, 0, s, HY_ATTN_ARGS);
-          else go_kernel(h, attn_mma_kernel<128>, u->n, 128, 0, s, HY_ATTN_ARGS);
+          if (c.a_dim == 32) go_alone(h, HY_OVERLAP_TOKENS, attn_mma_kernel<32>, u->n, 128, 0, s, HY_ATTN_ARGS);
+          else if (c.a_dim == 64) go_alone(h, HY_OVERLAP_TOKENS, attn_mma_kernel<64>, u->n, 128, 0, s, HY_ATTN_ARGS);
+          else go_alone(h, HY_OVERLAP_TOKENS, attn_mma_kernel<128>, u->n, 128, 0, s, HY_ATTN_ARGS);
 #undef HY_ATTN_ARGS
           go_kernel(h, attn_combine_kernel<WT, bf16>, T * c.a_heads, 64, 0, s, b, h->part_o, h->part_ml, (const WT*)L.sink, pin + L.c_g, h->ld_pin,
               c.a_heads, c.a_kv_heads, c.a_dim, c.a_dim, 0, u->split, u->ns, c.left_scale, cat + L.o_mix, h->ld_cat);
@@ -3118,7 +3132,7 @@ int run_step(hy_engine* h, const Batch& b, int n_want, const int* want_d, float*
         }
       }
       if (!tc)
-      go_kernel(h, attn_sink_kernel<AT, WT, AT>, (T * c.a_heads + 3) / 4, 128, 4 * c.a_dim * sizeof(float), s, 
+      go_alone(h, HY_OVERLAP_TOKENS, attn_sink_kernel<AT, WT, AT>, (T * c.a_heads + 3) / 4, 128, 4 * c.a_dim * sizeof(float), s, 
           b, cv, h->ld_cv, (const AT*)L.cache, (const WT*)L.sink, pin + L.c_g, h->ld_pin, c.a_heads, c.a_kv_heads, c.a_dim, c.a_dim,
           c.a_scale, c.a_qt_coef, c.a_qt_every, 0, c.left_scale, cat + L.o_mix, h->ld_cat);
       }
@@ -3146,7 +3160,7 @@ int run_step(hy_engine* h, const Batch& b, int n_want, const int* want_d, float*
           const int v32 = (R | N | h->ld_f1 | h->ld_f2 | I) % 4 == 0 && PB % 4 == 0;
           const int vat = (h->ld_cv | h->ld_pin | L.c_z | I) % ch == 0 && PB % ch == 0;
           auto pass = [&](auto which, int rows, ScanSegments seg) {
-            go_kernel(h, scan_kernel<AT, WT, NPER, LN, decltype(which)::value>, dim3((I + PB - 1) / PB, rows), 128, smem, s,
+            go_alone(h, HY_OVERLAP_TOKENS, scan_kernel<AT, WT, NPER, LN, decltype(which)::value>, dim3((I + PB - 1) / PB, rows), 128, smem, s,
                 b, cv, h->ld_cv, pin + L.c_z, h->ld_pin, h->f2, h->ld_f2, (const WT*)L.dt_b, h->f1, h->ld_f1, R, R + N, L.A_neg, (const WT*)L.D, I, N,
                 v32 | vat << 1, c.right_scale, L.rec_state, cat + L.o_scan, h->ld_cat, seg);
             h->launches++;
@@ -3194,7 +3208,7 @@ int run_step(hy_engine* h, const Batch& b, int n_want, const int* want_d, float*
         constexpr int DR = decltype(dr)::value, PARTS = decltype(parts)::value, VC = decltype(vcols)::value;
         const LinearLaunch g = linear_launch<AT>(PARTS, VC, dk, dv, cv, h->ld_cv);
         const size_t smem = lin_smem<AT>(DR, PARTS, VC, DR + 4);
-        go_kernel(h, delta_head_kernel<AT, DR, PARTS, VC, true>, dim3(H * g.bph, E), 128, smem, s, b, h->lin, cv, h->ld_cv, h->lin_sc, H, G, dk, dv, g.bph, g.vec,
+        go_alone(h, HY_OVERLAP_TOKENS, delta_head_kernel<AT, DR, PARTS, VC, true>, dim3(H * g.bph, E), 128, smem, s, b, h->lin, cv, h->ld_cv, h->lin_sc, H, G, dk, dv, g.bph, g.vec,
                                                                                      g.vvec, L.rec_state, o, h->ld_f2, h->f1, h->ld_f1);
       });
       launch_gla_out<AT, float, GATE_SIGMOID>(h, T, H, dv, o, h->ld_f2, h->f2, h->ld_f2, (const float*)L.norm_w, eps,

@@ -136,6 +136,29 @@ def test_which_launches_overlap(fake, tokens, dtype):
     assert sum(any(f in n for f in folded) for n, _ in fake.launches()) >= 3
 
 
+ALONE = ("scan_kernel", "gla_kernel", "gla_chunk_", "delta_head_kernel", "delta_chunk_", "attn_mma_kernel", "biased_mma_kernel", "glr_kernel", "attn_sink_kernel", "biased_attn_kernel")
+
+
+@pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
+@pytest.mark.parametrize("tokens", [71, 72, 150, 255, 256])
+@pytest.mark.parametrize("which", ["kinetar", "famepel", "kisadra", "mafalorn"])
+def test_which_launches_of_prompt_steps_overlap(fake, which, tokens, dtype):
+    """All but those whose time is their longest block, convolutions among them from 256 tokens on, and the folded form of latent attention."""
+    rt = engine(CONFIGS[which], dtype)
+    fake.reset()
+    step(rt, tokens)
+    folded = ("latent_query", "attn_", "head_rows", "latent_value")
+    seen = 0
+    for (name, _), overlaps in zip(fake.launches(), fake.overlaps()):
+        if any(f in name for f in folded) and not any(a in name for a in ALONE):
+            continue
+        alone = any(a in name for a in ALONE) or ("conv_kernel" in name and tokens >= 256)
+        assert overlaps == (tokens >= 72 and not alone), name
+        seen += alone
+    assert seen
+    rt.close()
+
+
 def latent_engine(window):
     from jacobiforcing_b200.hybrid_config import HybridConfig
     from jacobiforcing_b200.hybrid_runtime import HybridRuntime
