@@ -1,9 +1,11 @@
 """bf16 products of one to eight rows on the tensor cores: features beside the tiles of 16, k beside the blocks of 32 and beside what a batch or a split
 holds, sizes that keep the other kernel, and the routed form (experts without a row, experts that every token chose, gated and plain), against the
-fp64 restatements within the bounds of the other bf16 tests."""
+fp64 restatements within the bounds of the other bf16 tests.  Tokens without numbers, whose choices are all the same expert, beside healthy ones."""
+import numpy as np
 import pytest
 
-from oracle import kinetar_plain, mafalorn_plain, vosolorn_plain
+from oracle import famepel_plain, kinetar_plain, mafalorn_plain, vosolorn_plain
+from tests import famepel_helpers as fam
 from tests import hybrid_helpers as kin
 from tests import mafalorn_helpers as maf
 from tests import vosolorn_helpers as vos
@@ -64,3 +66,51 @@ def test_plain_experts(experts, top, ff, shared):
     finally:
         hz.close()
     assert vos.close(got, vos.oracle_logits(cfg, w, toks), "bfloat16")
+
+
+BROKEN = 7                                                     # the token whose embedding is no number
+ROUTED = {"gated, groups": (famepel_plain, fam, fam.model_config([fam.glr(mlp=fam.moe(experts=6, top=4, count=2, keep=2, ff=24))] * 2)),
+          "plain, largest": (vosolorn_plain, vos, vos.model_config([vos.mlstm(mlp=vos.moe(experts=6, top=4, ff=24))] * 2)),
+          "gated, corrected": (mafalorn_plain, maf, maf.model_config([maf.ret(mlp=maf.moe(experts=6, top=4, ff=24, identity=None, groups=None))] * 2))}
+
+
+@pytest.mark.parametrize("tokens", [[7, 7, 3], [7, 3, 7, 5, 9, 11, 2, 1], [3, 7, 7, 7, 7, 7, 7, 4], [7, 7, 7, 7, 7, 7, 7, 7]])
+@pytest.mark.parametrize("kind", sorted(ROUTED))
+def test_a_request_without_numbers_leaves_the_others_alone(kind, tokens):
+    """Their logits are those of the same step with another token in the broken one's place, bit by bit."""
+    plain, helpers, cfg = ROUTED[kind]
+    w = dict(plain.random_weights(cfg, 0))
+    w["embed"] = w["embed"].clone()
+    w["embed"][BROKEN] = float("nan")
+    columns = [c for c in range(cfg["vocab"]) if c != BROKEN]  # an output head that shares the table has one column without numbers
+    out = []
+    for row in (tokens, [6 if t == BROKEN else t for t in tokens]):
+        hz = helpers.Harness(cfg, w, "bfloat16", slots=8)
+        try:
+            for _ in range(2):                                 # what a step finds in its buffers is what one like it left there
+                out.append(hz.step([((len(out), i), [t], [0]) for i, t in enumerate(row)])[:, columns])
+                for i in range(len(row)):
+                    hz.end((len(out) - 1, i))
+        finally:
+            hz.close()
+    for i, t in enumerate(tokens):
+        assert np.isnan(out[0][i]).any() == np.isnan(out[1][i]).any() == (t == BROKEN)
+        if t != BROKEN:
+            assert np.array_equal(out[0][i], out[2][i]) and np.array_equal(out[1][i], out[2][i]), i
+
+
+@pytest.mark.parametrize("rows", [4, 5, 8])
+def test_fewer_finite_scores_than_choices(rows):
+    """A router that leaves one expert: it takes every choice, four times as many as there are tokens, and all but the first of a token weigh nothing."""
+    cfg = vos.model_config([vos.mlstm(mlp=vos.moe(experts=6, top=4, ff=24))] * 2)
+    w = dict(vosolorn_plain.random_weights(cfg, 0))
+    for name in ("l0.mlp.router.b", "l1.mlp.router.b"):
+        w[name] = w[name].clone()
+        w[name][1:] = -float("inf")
+    toks = kin.rand_tokens(3 * rows, cfg["vocab"], 6)
+    hz = vos.Harness(cfg, w, "bfloat16")
+    try:
+        got = hz.feed("a", toks, [rows])
+    finally:
+        hz.close()
+    assert vos.row_errs(got, vos.oracle_logits(cfg, w, toks)).max() < vos.TOL["bfloat16"]
