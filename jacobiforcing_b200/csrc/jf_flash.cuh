@@ -16,9 +16,10 @@
 // Keys and values travel by TMA, from pages of 256 tokens or from rows made for the step.
 //
 // Warp 0: producer (one lane).  Warp 1: owns tensor memory, one lane issues the products.  Warps 2-9: softmax, two threads per row.
-// Tensor memory: scores 128 columns (then, in the place of every 32 scores, 16 columns of weights and 16 of remainders), output 128.  The products
-// of a block execute in the order of their issue, and an mbarrier that one of them is committed to also stands for those before it: scores
-// are made behind the product that read the weights in their place, and once they are there the output holds everything before.
+// Tensor memory: scores 128 columns (then, in the place of every 32 scores, 16 columns of weights and 16 of remainders), output 128.  Products with
+// unlike accumulators are not promised to run one behind the other, so the next scores are issued once the product that reads the weights in their
+// place is over (its commit, which also gives the values' stage back).  An mbarrier that a product is committed to stands for all products
+// issued before it: once scores are there, the output holds everything before.
 // Every wait on an mbarrier is bounded (see tp_wait): on a timeout the kernel raises the error flag, stops waiting, lets its copies land
 // and frees its tensor memory.  The allocation of tensor memory waits without a limit; jf_pair.cuh says why it ends.
 #pragma once
@@ -173,7 +174,7 @@ flash_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ C
         }
         if (i + 1 < t.n) {
           const int s = (i + 1) % ST;
-          ok = fl_wait(&sm->k_full[s], ((i + 1) / ST) & 1, sm, a.err);
+          ok = fl_wait(&sm->k_full[s], ((i + 1) / ST) & 1, sm, a.err) && (i < 0 || fl_wait(&sm->v_empty[i % ST], (i / ST) & 1, sm, a.err));
           if (!ok) break;
           tc_fence_after();
           const uint64_t k = dk + (uint64_t)(s * KC * CHUNK >> 4);

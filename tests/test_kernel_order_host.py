@@ -45,3 +45,12 @@ def test_dependents_start_behind_the_allocation_of_tensor_memory(name, body):
     if "cta_group::2" in body[:last_alloc]:                   # both CTAs of a pair
         pair = body.index("tp_cluster_sync()", last_alloc)
         assert min(triggers) > pair, name
+
+
+def test_scores_wait_for_the_product_that_reads_the_weights_in_their_place():
+    """Both lie in the same columns, and products with unlike accumulators are not promised to run in the order of their issue."""
+    body = next(b for _, n, b in kernels() if n == "flash_kernel")
+    output, scores = body.index("umma_bf16_ts("), body.index("umma_bf16(tm,")
+    over = re.search(r"umma_commit\(&sm->(\w+)\[", body[output:scores])
+    assert output < scores and over, "the product of the output is committed before the scores are issued"
+    assert re.search(r"fl_wait\(&sm->%s\[" % over.group(1), body[output + over.end():scores])
