@@ -10,6 +10,8 @@
 // products of the given decays (no logarithms, no quotients: every factor is at most one and a decay of zero is just a zero).  Per
 // channel they are applied in sub-blocks of 16: inside one, pair by pair; between two, as (q from the later one's beginning) . (whole
 // sub-blocks between) . (k to the earlier one's end).
+// A token's read-out and correction meet what came up to it and nothing behind it, not even times zero: an infinity or what is no number stays with
+// the tokens from its own on, as it does token by token.
 // Operands come from shared memory, 8 x 8 and 8 x 4 sums per thread; in turn the fma pipe (a third of the time) and the reads of shared memory (half of
 // it) bound them, with two blocks of eight warps per SM.  2048 tokens, us, token by token -> chunks (three kernels): forget gates, 8
 // heads of 128 x 128, 187 -> 72; state space, 32 heads of 64 x 128, 236 -> 140; two requests of gated linear attention, 16 heads of
@@ -498,7 +500,8 @@ __global__ void __launch_bounds__(256, 2) gla_chunk_out_kernel(ChunkArgs<AT> a) 
       for (int jj = 0; jj < 4; ++jj) {
         if (jj > I) break;
         const int j = jj * 16 + tx;
-        float w = j <= r ? sa[CH_T + j] : 0.0f;                // the value's factor
+        if (j > r) continue;
+        float w = sa[CH_T + j];                                // the value's factor
         if (jj == I) { for (int m = j + 1; m <= r; ++m) w *= sa[m]; }
         else {
           w *= sl[r] * sr[j];
@@ -559,22 +562,30 @@ __global__ void __launch_bounds__(256, 2) gla_chunk_out_kernel(ChunkArgs<AT> a) 
 #pragma unroll
     for (int c = 0; c < TV; ++c) x[c] = to_f(v.v[c]);
   };
-  const int jend = min(r0 + 8, (p.n + 3) & ~3);
-#pragma unroll 1
-  for (int j = 0; j < jend; j += 4) {
+  // Values j .. j + 3; own: where they begin among the warp's eight tokens, of which a query meets those up to itself (negative: all come before).
+  auto weigh = [&](int j, auto own) {
+    constexpr int OWN = decltype(own)::value;
     float x[4][TV];
 #pragma unroll
     for (int k = 0; k < 4; ++k) value(j + k, x[k]);
 #pragma unroll
     for (int r = 0; r < 8; ++r) {
+      if (r < OWN) continue;
       const float4 w = *reinterpret_cast<const float4*>(sw + (r0 + r) * CH_T + j);
 #pragma unroll
       for (int c = 0; c < TV; ++c) {
-        acc[r][c] = fma2(make_float2(w.x, w.y), make_float2(x[0][c], x[1][c]), acc[r][c]);
-        acc[r][c] = fma2(make_float2(w.z, w.w), make_float2(x[2][c], x[3][c]), acc[r][c]);
+        if (OWN < 0 || r > OWN) acc[r][c] = fma2(make_float2(w.x, w.y), make_float2(x[0][c], x[1][c]), acc[r][c]);
+        else acc[r][c].x = fmaf(w.x, x[0][c], acc[r][c].x);
+        if (OWN < 0 || r > OWN + 2) acc[r][c] = fma2(make_float2(w.z, w.w), make_float2(x[2][c], x[3][c]), acc[r][c]);
+        else if (r == OWN + 2) acc[r][c].x = fmaf(w.z, x[2][c], acc[r][c].x);
       }
     }
-  }
+  };
+  const int before = min(r0, p.n);
+#pragma unroll 1
+  for (int j = 0; j < before; j += 4) weigh(j, std::integral_constant<int, -1>{});
+  if (r0 < p.n) weigh(r0, std::integral_constant<int, 0>{});
+  if (r0 + 4 < p.n) weigh(r0 + 4, std::integral_constant<int, 4>{});
 #pragma unroll
   for (int r = 0; r < 8; ++r) {
     const int t = r0 + r;
@@ -607,9 +618,10 @@ __global__ void __launch_bounds__(256, 2) gla_chunk_out_kernel(ChunkArgs<AT> a) 
 // delta_chunk_prep_kernel makes W, U0, Q', k'', A and the decays' product of all chunks side by side; delta_chunk_chain_kernel walks the chunks of
 // a head, 16 columns per block (columns do not meet).  |u| stays within beta times the state, so the system's solution does not grow.  One
 // decay per head is taken as the same for all channels.
-// The chain: what a chunk brings travels in two halves while the other half is worked on.  5.9 us a chunk, bound by reading operands from shared memory
-// (eight 16-byte reads for 32 fma.rn.f32x2): products with the state 5000 of 11300 cycles, corrections of the state 4400, starting copies 1600.
-// 2048 tokens, 16 heads of 128 x 128 with channel decays: 430 us token by token; prep 131 and chain 190.
+// The chain: what a chunk brings travels in two halves while the other half is worked on.  5.2 us a chunk (5.9 when a row's corrections met the
+// zeros behind its token as well), bound by reading operands from shared memory (eight 16-byte reads for 32 fma.rn.f32x2): half of it products
+// with the state, then corrections of the state and starting copies.
+// 2048 tokens, 16 heads of 128 x 128 with channel decays: 430 us token by token; prep 128 and chain 165.
 template <typename AT>
 struct DeltaArgs {
   Batch b;
@@ -670,8 +682,7 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_prep_kernel(DeltaArgs<AT> 
     float m;
     const float w = ch_pairs<DK, false, true>(sq, sk, sd, s, j, jw, l, &m);
     work[Work::A + (s * CH_SUB + l) * CH_T + s * CH_SUB + j] = w;
-    sm[ch_tri(s, s) + j * CH_SUB + l] = l > j ? m * sb[s * CH_SUB + l] : 0.0f;
-    for (int J = s + 1; J < CH_SUBS; ++J) work[Work::A + (s * CH_SUB + l) * CH_T + J * CH_SUB + j] = 0.0f;      // what a query does not see
+    sm[ch_tri(s, s) + j * CH_SUB + l] = m * sb[s * CH_SUB + l];
   }
   __syncthreads();
   for (int i = tid; i < CH_SUBS * DK; i += 256) {              // queries and keys from their sub-block's beginning, keys to its end
@@ -757,10 +768,13 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_prep_kernel(DeltaArgs<AT> 
       for (int j = 0; j < CH_SUB; ++j) {
         const float u = j & 1 ? r[j / 2].y : r[j / 2].x;
 #pragma unroll
-        for (int t = j / 4; t < CH_SUB / 4; ++t) {             // the diagonal and above: zeros
+        for (int t = j / 4; t < CH_SUB / 4; ++t) {             // of row j's own four those behind it
+          if (4 * t + 3 == j) continue;
           const float4 mm = *reinterpret_cast<const float4*>(m + j * CH_SUB + 4 * t);
-          r[2 * t] = fma2(make_float2(mm.x, mm.y), make_float2(-u, -u), r[2 * t]);
-          r[2 * t + 1] = fma2(make_float2(mm.z, mm.w), make_float2(-u, -u), r[2 * t + 1]);
+          if (4 * t > j) r[2 * t] = fma2(make_float2(mm.x, mm.y), make_float2(-u, -u), r[2 * t]);
+          else if (4 * t == j) r[2 * t].y = fmaf(mm.y, -u, r[2 * t].y);
+          if (4 * t + 1 >= j) r[2 * t + 1] = fma2(make_float2(mm.z, mm.w), make_float2(-u, -u), r[2 * t + 1]);
+          else r[2 * t + 1].y = fmaf(mm.w, -u, r[2 * t + 1].y);
         }
       }
 #pragma unroll
@@ -873,22 +887,33 @@ __global__ void __launch_bounds__(256) delta_chunk_chain_kernel(DeltaArgs<AT> a)
     __syncthreads();                                           // the second half of this chunk is there
     if (!kh) {
       float2 o2[2][4] = {};
-      const int stop = rg + 32;
-#pragma unroll 2
-      for (int t = 0; t <= stop; t += 4) {
+      // Corrections t .. t + 3 times A, for the rows rg + 32 i from i = `from` on; `own`: the row that is one of these four and meets those up to itself.
+      auto weigh = [&](int t, auto from, auto own) {
         VecN<float, 4> u[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) u[i] = *reinterpret_cast<const VecN<float, 4>*>(sU + (t / 2 + (i >> 1)) * 2 * C + 2 * cg + (i & 1) * 4);
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
+        for (int i = decltype(from)::value; i < 2; ++i) {
           const float4 w = *reinterpret_cast<const float4*>(sA + (rg + 32 * i) * CH_T + (((t >> 2) ^ (rg & 7)) << 2));
+          const int last = i == decltype(own)::value ? rg & 3 : 3;
+          auto upto = [&](int k, float v) { return k <= last ? v : 0.0f; };
+          const float2 w0 = make_float2(w.x, upto(1, w.y)), w1 = make_float2(upto(2, w.z), upto(3, w.w));
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
-            o2[i][c] = fma2(make_float2(w.x, w.y), make_float2(u[c / 2].v[2 * (c & 1)], u[c / 2].v[2 * (c & 1) + 1]), o2[i][c]);
-            o2[i][c] = fma2(make_float2(w.z, w.w), make_float2(u[2 + c / 2].v[2 * (c & 1)], u[2 + c / 2].v[2 * (c & 1) + 1]), o2[i][c]);
+            const float *x = u[c / 2].v + 2 * (c & 1), *y = u[2 + c / 2].v + 2 * (c & 1);
+            o2[i][c] = fma2(w0, make_float2(x[0], upto(1, x[1])), o2[i][c]);
+            o2[i][c] = fma2(w1, make_float2(upto(2, y[0]), upto(3, y[1])), o2[i][c]);
           }
         }
-      }
+      };
+      typedef std::integral_constant<int, 0> first; typedef std::integral_constant<int, 1> second; typedef std::integral_constant<int, 2> none;
+      const int four = rg & ~3;
+#pragma unroll 2
+      for (int t = 0; t < four; t += 4) weigh(t, first{}, none{});
+      weigh(four, first{}, first{});
+#pragma unroll 2
+      for (int t = four + 4; t < four + 32; t += 4) weigh(t, second{}, none{});
+      weigh(four + 32, second{}, second{});
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
         const int t = j * CH_T + rg + 32 * i;

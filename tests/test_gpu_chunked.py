@@ -144,3 +144,30 @@ def test_selective_scan_in_segments(state, inner, rank):
     got["c"] = np.concatenate([first[70:], second[430:]], 0)
     for k in toks:
         assert kin.rel_err(got[k], kin.oracle_logits(cfg, w, toks[k])) < kin.TOL["float32"], k
+
+
+@pytest.mark.parametrize("dim,vdim", [(64, 40), (128, 128)])
+@pytest.mark.parametrize("mode", MODES + ["channel delta", "head delta"])
+def test_what_is_no_number_stays_with_the_tokens_from_its_own_on(mode, dim, vdim):
+    """A token without numbers, at places of a chunk beside its groups of 4, 8, 16 and 32: the tokens before it come out as they do without it, bit by
+    bit, and none behind it comes out at all."""
+    plain, helpers, cfg = _delta(mode[:-6], dim, vdim, 2, 1) if mode.endswith("delta") else _model(mode, dim, vdim)
+    broken, other = 7, 6
+    w = dict(plain.random_weights(cfg, 0))
+    w["embed"] = w["embed"].clone()
+    w["embed"][broken] = float("nan")
+    columns = [c for c in range(cfg["vocab"]) if c != broken]  # an output head that shares the table has one column without numbers
+    toks = [other if t == broken else t for t in kin.rand_tokens(520, cfg["vocab"], 5)]
+    hz = helpers.Harness(cfg, w, "float32", num_pages=80, max_step_tokens=640)
+    try:
+        def run(at):
+            out = hz.feed("a", toks[:at] + [broken] + toks[at + 1:] if at else toks)[:, columns]
+            hz.end("a")
+            return out
+        clean = run(0)
+        for at in (129, 134, 139, 191, 400):
+            got = run(at)
+            assert np.array_equal(got[:at], clean[:at]) and np.isnan(got[at:]).any(1).all(), at
+    finally:
+        hz.close()
+    assert np.isfinite(clean).all()
