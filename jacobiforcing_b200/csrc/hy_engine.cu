@@ -3295,23 +3295,25 @@ extern "C" int hy_step(hy_handle h, int32_t n_entries, const int32_t* tokens, co
   HY_CUDA(cudaEventRecord(h->ev0, h->stream));
   if (h->m.dtype == HY_DTYPE_F32) run_step<float>(h, b, n_want, want_d, layers_out);
   else run_step<__nv_bfloat16>(h, b, n_want, want_d, layers_out);
+  // Copies into the caller's arrays may go on behind the calls that make them (page-locked arrays): what fails among them is kept until the stream
+  // has been waited for.
+  auto keep = [&](cudaError_t e) { if (e != cudaSuccess && h->step_err.empty()) h->step_err = cudaGetErrorString(e); };
   if (n_want > 0 && sampled_out) {
     const float* td = nullptr;
     if (temperature) {
-      HY_CUDA(cudaMemcpyAsync(h->temp_d, temperature, (size_t)n_want * 4, cudaMemcpyHostToDevice, h->stream));
+      keep(cudaMemcpyAsync(h->temp_d, temperature, (size_t)n_want * 4, cudaMemcpyHostToDevice, h->stream));
       td = h->temp_d;
     }
     go_kernel(h, sample_kernel, n_want, 1024, 0, h->stream, h->logits, h->m.vocab, td, seed, h->sampled);
     h->launches++;
-    HY_CUDA(cudaMemcpyAsync(sampled_out, h->sampled, (size_t)n_want * 4, cudaMemcpyDeviceToHost, h->stream));
+    keep(cudaMemcpyAsync(sampled_out, h->sampled, (size_t)n_want * 4, cudaMemcpyDeviceToHost, h->stream));
   }
-  HY_CUDA(cudaEventRecord(h->ev1, h->stream));
+  keep(cudaEventRecord(h->ev1, h->stream));
   if (n_want > 0 && logits_out)
-    HY_CUDA(cudaMemcpyAsync(logits_out, h->logits, (size_t)n_want * h->m.vocab * 4, cudaMemcpyDeviceToHost, h->stream));
-  HY_CUDA(cudaMemcpyAsync(h->err_h, h->err_d, 4, cudaMemcpyDeviceToHost, h->stream));
-  HY_CUDA(cudaStreamSynchronize(h->stream));
-  const cudaError_t last = cudaGetLastError();
-  if (h->step_err.empty()) HY_CUDA(last);
+    keep(cudaMemcpyAsync(logits_out, h->logits, (size_t)n_want * h->m.vocab * 4, cudaMemcpyDeviceToHost, h->stream));
+  keep(cudaMemcpyAsync(h->err_h, h->err_d, 4, cudaMemcpyDeviceToHost, h->stream));
+  keep(cudaStreamSynchronize(h->stream));
+  keep(cudaGetLastError());
   if (*h->err_h && h->step_err.empty()) h->step_err = "a wait inside a tensor-core kernel ran out (pipeline stalled)";
   if (!h->step_err.empty()) {                                // counters that kernels leave at zero, as the next step expects them
     *h->err_h = 0;

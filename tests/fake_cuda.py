@@ -12,7 +12,7 @@ import pytest
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 CSRC = os.path.join(ROOT, "jacobiforcing_b200", "csrc")
 FAKE = os.path.join(ROOT, "tests", "host", "fake_cuda.cpp")
-LAUNCH, ATTRIBUTE, TENSOR_MAP = 0, 1, 2
+LAUNCH, ATTRIBUTE, TENSOR_MAP, TO_HOST = 0, 1, 2, 3
 
 
 def build(engine: str) -> str:
@@ -50,6 +50,10 @@ class Fake:
 
     def count(self, what):
         return self.lib.fake_count(what)
+
+    def on_their_way(self):
+        """Copies to the host since the last wait for the stream."""
+        return self.lib.fake_on_their_way()
 
     def launches(self):
         """(kernel, device) of every launch that went through since the last reset."""

@@ -18,7 +18,9 @@ std::map<const void*, std::string>& names() { static std::map<const void*, std::
 struct Launch { const void* f; int device, overlaps; unsigned blocks; };
 std::vector<Launch> g_launches;
 std::map<std::pair<int, const void*>, int> g_smem;              // (device, kernel) -> opted in dynamic shared memory
-long g_count[3] = {0, 0, 0}, g_fail[3] = {-1, -1, -1};          // launches, attributes, tensor maps: how many so far, which one fails
+constexpr int kKinds = 4;                                        // launches, attributes, tensor maps, copies to the host
+long g_count[kKinds] = {}, g_fail[kKinds] = {-1, -1, -1, -1};    // how many so far, which one fails
+int g_on_their_way = 0;                                         // copies to the host that nothing has waited for
 constexpr size_t kDefaultSmem = 48 * 1024, kMostSmem = 227 * 1024;
 
 bool fails(int what) { return g_count[what]++ == g_fail[what]; }
@@ -44,9 +46,10 @@ CUresult encode(CUtensorMap* m, CUtensorMapDataType, cuuint32_t, void* p, const 
 
 extern "C" {
 // ---- what a test asks ---------------------------------------------------------------------------------------------------------------
-void fake_reset() { g_launches.clear(); for (int i = 0; i < 3; ++i) { g_count[i] = 0; g_fail[i] = -1; } g_last = cudaSuccess; }
+void fake_reset() { g_launches.clear(); for (int i = 0; i < kKinds; ++i) { g_count[i] = 0; g_fail[i] = -1; } g_last = cudaSuccess; }
 void fake_fail(int what, long at) { g_count[what] = 0; g_fail[what] = at; }
 long fake_count(int what) { return g_count[what]; }
+int fake_on_their_way() { return g_on_their_way; }
 int fake_launches() { return (int)g_launches.size(); }
 const char* fake_launch_name(int i) { return names()[g_launches[i].f].c_str(); }
 int fake_launch_device(int i) { return g_launches[i].device; }
@@ -84,13 +87,20 @@ cudaError_t cudaHostGetDevicePointer(void** d, void* p, unsigned) { *d = p; retu
 cudaError_t cudaFree(void* p) { free(p); return cudaSuccess; }
 cudaError_t cudaFreeHost(void* p) { free(p); return cudaSuccess; }
 cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind) { memcpy(d, s, n); return cudaSuccess; }
-cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t) { memcpy(d, s, n); return cudaSuccess; }
+cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind k, cudaStream_t) {
+  if (k == cudaMemcpyDeviceToHost) {
+    if (fails(3)) return last(cudaErrorInvalidValue);
+    ++g_on_their_way;
+  }
+  memcpy(d, s, n);
+  return cudaSuccess;
+}
 cudaError_t cudaMemset(void* d, int v, size_t n) { memset(d, v, n); return cudaSuccess; }
 cudaError_t cudaMemsetAsync(void* d, int v, size_t n, cudaStream_t) { memset(d, v, n); return cudaSuccess; }
 cudaError_t cudaStreamCreate(cudaStream_t* s) { *s = nullptr; return cudaSuccess; }
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) { *s = nullptr; return cudaSuccess; }
 cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
-cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t) { g_on_their_way = 0; return cudaSuccess; }
 cudaError_t cudaDeviceSynchronize() { return cudaSuccess; }
 cudaError_t cudaEventCreate(cudaEvent_t* e) { *e = nullptr; return cudaSuccess; }
 cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }

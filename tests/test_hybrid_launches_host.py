@@ -80,6 +80,24 @@ def test_nothing_is_launched_behind_a_failure(fake, what, which, tokens):
     rt.close()
 
 
+def test_nothing_writes_to_the_caller_behind_a_failure(fake):
+    """The caller's arrays may be page-locked, so that copies into them go on after the call that made them: a step that fails waits for those."""
+    rt = engine(CONFIGS["famepel"])
+    fake.reset()
+    step(rt, 5)
+    copies = fake.count(fake_cuda.TO_HOST)
+    assert copies == 3                                       # sampled tokens, logits, the kernels' error word
+    for at in range(copies):
+        fake.reset()
+        fake.fail(fake_cuda.TO_HOST, at)
+        with pytest.raises(RuntimeError, match="invalid argument"):
+            step(rt, 5)
+        assert fake.on_their_way() == 0
+        fake.reset()
+        step(rt, 5)
+    rt.close()
+
+
 @pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
 @pytest.mark.parametrize("which", sorted(CONFIGS))
 def test_steps_on_two_devices(fake, which, dtype):
