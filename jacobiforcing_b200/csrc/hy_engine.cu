@@ -266,6 +266,22 @@ static int dev_alloc(hy_engine* h, void** p, size_t bytes, int64_t* counter) {
   return HY_OK;
 }
 
+// A workspace (or weights laid out once more) of a form that is faster where there is room for it; without (NULL) a step takes the form that needs none.
+// Made behind everything that an engine cannot do without, and only if HY_ROOM is left: kernels that are loaded at their first launch take
+// memory as well.
+constexpr size_t HY_ROOM = (size_t)256 << 20;
+static void dev_try(hy_engine* h, void** p, size_t bytes, int64_t* counter) {
+  size_t left = 0, all = 0;
+  *p = nullptr;
+  if (bytes == 0 || cudaMemGetInfo(&left, &all) != cudaSuccess || left < bytes + HY_ROOM || cudaMalloc(p, bytes) != cudaSuccess) {
+    *p = nullptr;
+    cudaGetLastError();
+    return;
+  }
+  h->allocs.push_back(*p);
+  *counter += (int64_t)bytes;
+}
+
 static thread_local std::string g_create_err;
 
 extern "C" int hy_create(const hy_model_cfg* model, const hy_layer_cfg* layers, const hy_runtime_cfg* rt, hy_handle* out) {
@@ -517,15 +533,18 @@ struct Builder {
     }
     return d;
   }
-  // three times side by side, for rows in three parts (split_rows_kernel)
-  void* up_split(const std::vector<float>& v, int N, int K) {
-    if (rc != HY_OK || h->m.dtype != HY_DTYPE_BF16) return nullptr;
+  // three times side by side, for rows in three parts (split_rows_kernel): tiles that hy_finalize takes to the device at its end
+  struct Later { void** to; std::vector<uint16_t> tiles; };
+  std::vector<Later> later;
+  void up_split(void** to, const std::vector<float>& v, int N, int K) {
+    if (rc != HY_OK || h->m.dtype != HY_DTYPE_BF16 || h->rt.max_step_tokens < HY_SPLIT_ROWS) return;
     const int KP = split_cols(K);
     std::vector<float> three((size_t)N * 3 * KP, 0.0f);
     for (int n = 0; n < N; ++n)
       for (int p = 0; p < 3; ++p) std::copy_n(&v[(size_t)n * K], K, &three[((size_t)n * 3 + p) * KP]);
     h->split_width = std::max(h->split_width, 3 * KP);
-    return up_tiled(three, N, 3 * KP);
+    later.push_back({to, {}});
+    pack_tiles(three.data(), N, 3 * KP, later.back().tiles);
   }
   void* up_tiled(const std::vector<float>& v, int N, int K) {
     if (rc != HY_OK || h->m.dtype != HY_DTYPE_BF16) return nullptr;
@@ -1373,7 +1392,7 @@ extern "C" int hy_finalize(hy_handle h) {
       if (auto t = B.get(s + "conv", I, c.s_conv)) L.conv_x = B.up(t->v);
       if (auto t = B.get(s + "conv.b", I, -1)) L.conv_xb = B.up(t->v);
       if (auto t = B.get(s + "x", R + 2 * N, I)) { L.w_x = B.up(t->v); L.w_x_t = B.up_tiled(t->v, R + 2 * N, I); }
-      if (auto t = B.get(s + "dt", I, R)) { L.w_dt = B.up(t->v); L.w_dt_t = B.up_split(t->v, I, R); }
+      if (auto t = B.get(s + "dt", I, R)) { L.w_dt = B.up(t->v); B.up_split(&L.w_dt_t, t->v, I, R); }
       if (auto t = B.get(s + "dt.b", I, -1)) L.dt_b = B.up(t->v);
       if (auto t = B.get(s + "A_log", I, N)) {
         std::vector<float> an(t->v.size());
@@ -1462,7 +1481,6 @@ extern "C" int hy_finalize(hy_handle h) {
   if (dev_alloc(h, (void**)&h->f2, T * h->ld_f2 * 4, &h->bytes_ws)) return HY_ERR_CUDA;
   if (mx.lin > 0 && dev_alloc(h, (void**)&h->lin, T * (size_t)mx.lin * 4, &h->bytes_ws)) return HY_ERR_CUDA;
   if (mx.lin_sc > 0 && dev_alloc(h, (void**)&h->lin_sc, T * (size_t)mx.lin_sc * sizeof(float4), &h->bytes_ws)) return HY_ERR_CUDA;
-  if (h->split_width > 0 && rt.max_step_tokens >= HY_SPLIT_ROWS && dev_alloc(h, &h->split, T * (size_t)h->split_width * 2, &h->bytes_ws)) return HY_ERR_CUDA;
   if (h->m.block_kind == HY_BLOCK_PRENORM) {
     if (dev_alloc(h, (void**)&h->hn, T * W * 4, &h->bytes_ws)) return HY_ERR_CUDA;
     if (h->m.depth_avg && dev_alloc(h, (void**)&h->kept, (h->lc.size() + 1) * T * W * 4, &h->bytes_ws)) return HY_ERR_CUDA;
@@ -1510,9 +1528,10 @@ extern "C" int hy_finalize(hy_handle h) {
       HY_CUDA(cudaMallocHost((void**)&h->units_h, h->units_cap * sizeof(AttnUnit)));
     }
   }
+  size_t paged = 0;                                           // columns of the widest layer's keys and values out of their pages
   {
     std::set<std::vector<int>> lists;                         // layouts of the unit lists that one step may hold
-    size_t row = 0, heads = 0, maxH = 0, paged = 0;
+    size_t row = 0, heads = 0, maxH = 0;
     for (auto& c : h->lc) {
       PagedHeads p;
       if (c.mixer == HY_MIX_LATENT && latent_prompt_sizes(h, c)) {
@@ -1531,7 +1550,6 @@ extern "C" int hy_finalize(hy_handle h) {
       h->fl_cap = lists.size() * ((T / 128 + rt.max_step_entries) * maxH * sizeof(jf::FlashUnit) + (2 * (size_t)rt.max_step_entries + 1) * 4 + 80);
       if (row > 0 && dev_alloc(h, &h->kv_rows, (size_t)h->kv_cap * row * 2, &h->bytes_ws)) return HY_ERR_CUDA;
       if (heads > 0 && dev_alloc(h, &h->kv_heads, (size_t)h->kv_cap * heads * 2, &h->bytes_ws)) return HY_ERR_CUDA;
-      if (paged > 0 && dev_alloc(h, &h->page_rows, (size_t)h->kv_cap * paged * 2, &h->bytes_ws)) return HY_ERR_CUDA;
       if (dev_alloc(h, (void**)&h->fl_d, h->fl_cap, &h->bytes_ws)) return HY_ERR_CUDA;
       HY_CUDA(cudaMallocHost((void**)&h->fl_h, h->fl_cap));
     }
@@ -1557,6 +1575,16 @@ extern "C" int hy_finalize(hy_handle h) {
       HY_CUDA(cudaMemset(h->x_meta, 0, 16));
     }
   }
+  if (!h->rot_tables.empty()) {
+    std::vector<RotTable> t;
+    for (auto& r : h->rot_tables) t.push_back(r.t);
+    if (dev_alloc(h, (void**)&h->rot_tables_d, t.size() * sizeof(RotTable), &h->bytes_ws)) return HY_ERR_CUDA;
+    HY_CUDA(cudaMemcpy(h->rot_tables_d, t.data(), t.size() * sizeof(RotTable), cudaMemcpyHostToDevice));
+  }
+  if (dev_alloc(h, (void**)&h->err_d, 4, &h->bytes_ws)) return HY_ERR_CUDA;
+  HY_CUDA(cudaMemset(h->err_d, 0, 4));
+  HY_CUDA(cudaMallocHost((void**)&h->err_h, 4));
+  *h->err_h = 0;
   {
     size_t states = 0, ends = 0;                              // floats per chunk of the largest layer
     auto layer = [&](int H, int dk, int dv, bool delta = false) {
@@ -1575,23 +1603,19 @@ extern "C" int hy_finalize(hy_handle h) {
         const int lanes = c.s_state <= 4 ? 1 : c.s_state <= 8 ? 2 : c.s_state <= 16 ? 4 : c.s_state <= 32 ? 8 : c.s_state <= 64 ? 16 : 32, per = 128 / lanes;
         scan = std::max(scan, (size_t)scan_segment_rows((c.s_inner + per - 1) / per) * c.s_inner * (c.s_state + 1));
       }
-    if (scan > 0 && rt.max_step_tokens >= 3 * SCAN_SEG_TOKENS && dev_alloc(h, (void**)&h->scan_own, scan * 4, &h->bytes_ws)) return HY_ERR_CUDA;
+    if (rt.max_step_tokens >= 3 * SCAN_SEG_TOKENS) dev_try(h, (void**)&h->scan_own, scan * 4, &h->bytes_ws);
     if (states > 0 && rt.max_step_tokens >= HY_CHUNK_TOKENS) {
-      h->ch_cap = chunk_cap(rt.max_step_tokens);
-      if (dev_alloc(h, (void**)&h->ch_states, (size_t)h->ch_cap * states * 4, &h->bytes_ws)) return HY_ERR_CUDA;
-      if (dev_alloc(h, (void**)&h->ch_ends, (size_t)h->ch_cap * ends * 4, &h->bytes_ws)) return HY_ERR_CUDA;
+      const int cap = chunk_cap(rt.max_step_tokens);
+      dev_try(h, (void**)&h->ch_states, (size_t)cap * (states + ends) * 4, &h->bytes_ws);
+      if (h->ch_states) { h->ch_cap = cap; h->ch_ends = h->ch_states + (size_t)cap * states; }
+    }
+    dev_try(h, &h->page_rows, (size_t)h->kv_cap * paged * 2, &h->bytes_ws);
+    if (rt.max_step_tokens >= HY_SPLIT_ROWS) dev_try(h, &h->split, T * (size_t)h->split_width * 2, &h->bytes_ws);
+    for (auto& l : B.later) {
+      if (h->split) dev_try(h, l.to, l.tiles.size() * 2, &h->bytes_w);
+      if (*l.to) HY_CUDA(cudaMemcpy(*l.to, l.tiles.data(), l.tiles.size() * 2, cudaMemcpyHostToDevice));
     }
   }
-  if (!h->rot_tables.empty()) {
-    std::vector<RotTable> t;
-    for (auto& r : h->rot_tables) t.push_back(r.t);
-    if (dev_alloc(h, (void**)&h->rot_tables_d, t.size() * sizeof(RotTable), &h->bytes_ws)) return HY_ERR_CUDA;
-    HY_CUDA(cudaMemcpy(h->rot_tables_d, t.data(), t.size() * sizeof(RotTable), cudaMemcpyHostToDevice));
-  }
-  if (dev_alloc(h, (void**)&h->err_d, 4, &h->bytes_ws)) return HY_ERR_CUDA;
-  HY_CUDA(cudaMemset(h->err_d, 0, 4));
-  HY_CUDA(cudaMallocHost((void**)&h->err_h, 4));
-  *h->err_h = 0;
   HY_CUDA(cudaDeviceSynchronize());
   h->finalized = true;
   return HY_OK;

@@ -937,7 +937,7 @@ constexpr int SCAN_BLOCKS = 6, SCAN_SEG_TOKENS = 96;
 inline int scan_segment_rows(int blocks) { return 148 * SCAN_BLOCKS / (blocks < 1 ? 1 : blocks); }      // entries x segments at most
 inline ScanSegments scan_segments(float* own, int blocks, int entries, int longest, int inner, int nstate) {
   const int fit = scan_segment_rows(blocks) / entries, n = fit < longest / SCAN_SEG_TOKENS ? fit : longest / SCAN_SEG_TOKENS;
-  if (n < 3) return ScanSegments{0, 1, nullptr, nullptr};
+  if (!own || n < 3) return ScanSegments{0, 1, nullptr, nullptr};
   const int tokens = ((longest + n - 1) / n + 31) / 32 * 32, count = (longest + tokens - 1) / tokens;
   return ScanSegments{tokens, count, own, own + (size_t)entries * count * inner * nstate};
 }

@@ -39,6 +39,8 @@ class Fake:
         self.lib.fake_launch_name.restype = C.c_char_p
         self.lib.fake_count.restype = C.c_long
         self.lib.fake_fail.argtypes = [C.c_int, C.c_long]
+        self.lib.fake_room.argtypes = [C.c_longlong]
+        self.lib.fake_used.restype = C.c_longlong
         self.reset()
 
     def reset(self):
@@ -50,6 +52,13 @@ class Fake:
 
     def count(self, what):
         return self.lib.fake_count(what)
+
+    def room(self, size=1 << 40):
+        """The device has this many bytes."""
+        self.lib.fake_room(size)
+
+    def used(self):
+        return self.lib.fake_used()
 
     def on_their_way(self):
         """Copies to the host since the last wait for the stream."""

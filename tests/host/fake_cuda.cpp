@@ -20,6 +20,8 @@ std::vector<Launch> g_launches;
 std::map<std::pair<int, const void*>, int> g_smem;              // (device, kernel) -> opted in dynamic shared memory
 constexpr int kKinds = 4;                                        // launches, attributes, tensor maps, copies to the host
 long g_count[kKinds] = {}, g_fail[kKinds] = {-1, -1, -1, -1};    // how many so far, which one fails
+std::map<void*, size_t> g_device_blocks;                         // what is taken of the device's memory
+size_t g_used = 0, g_room = (size_t)1 << 40;
 int g_on_their_way = 0;                                         // copies to the host that nothing has waited for
 constexpr size_t kDefaultSmem = 48 * 1024, kMostSmem = 227 * 1024;
 
@@ -49,6 +51,8 @@ extern "C" {
 void fake_reset() { g_launches.clear(); for (int i = 0; i < kKinds; ++i) { g_count[i] = 0; g_fail[i] = -1; } g_last = cudaSuccess; }
 void fake_fail(int what, long at) { g_count[what] = 0; g_fail[what] = at; }
 long fake_count(int what) { return g_count[what]; }
+void fake_room(long long bytes) { g_room = (size_t)bytes; }
+long long fake_used() { return (long long)g_used; }
 int fake_on_their_way() { return g_on_their_way; }
 int fake_launches() { return (int)g_launches.size(); }
 const char* fake_launch_name(int i) { return names()[g_launches[i].f].c_str(); }
@@ -80,11 +84,22 @@ cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr a, int) {
   return cudaSuccess;
 }
 cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int* n, const void*, int, size_t, unsigned) { *n = 1; return cudaSuccess; }
-cudaError_t cudaMalloc(void** p, size_t n) { *p = calloc(n ? n : 1, 1); return *p ? cudaSuccess : cudaErrorMemoryAllocation; }
-cudaError_t cudaMallocHost(void** p, size_t n) { return cudaMalloc(p, n); }
-cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { return cudaMalloc(p, n); }
+cudaError_t cudaMallocHost(void** p, size_t n) { *p = calloc(n ? n : 1, 1); return *p ? cudaSuccess : last(cudaErrorMemoryAllocation); }
+cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { return cudaMallocHost(p, n); }
+cudaError_t cudaMalloc(void** p, size_t n) {
+  if (n > g_room - g_used) return last(cudaErrorMemoryAllocation);
+  const cudaError_t e = cudaMallocHost(p, n);
+  if (e == cudaSuccess) { g_device_blocks[*p] = n; g_used += n; }
+  return e;
+}
+cudaError_t cudaMemGetInfo(size_t* left, size_t* all) { *left = g_room - g_used; *all = g_room; return cudaSuccess; }
 cudaError_t cudaHostGetDevicePointer(void** d, void* p, unsigned) { *d = p; return cudaSuccess; }
-cudaError_t cudaFree(void* p) { free(p); return cudaSuccess; }
+cudaError_t cudaFree(void* p) {
+  const auto it = g_device_blocks.find(p);
+  if (it != g_device_blocks.end()) { g_used -= it->second; g_device_blocks.erase(it); }
+  free(p);
+  return cudaSuccess;
+}
 cudaError_t cudaFreeHost(void* p) { free(p); return cudaSuccess; }
 cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind) { memcpy(d, s, n); return cudaSuccess; }
 cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind k, cudaStream_t) {

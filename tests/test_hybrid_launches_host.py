@@ -129,6 +129,49 @@ def test_engines_of_unlike_sizes_take_turns(fake, tokens, dtype):
         rt.close()
 
 
+def roomy_engine(dtype):
+    """An engine whose prompt steps have forms with workspaces of their own: chunks, segments, keys and values out of their pages, rows in three parts."""
+    from jacobiforcing_b200.hybrid_config import HybridConfig
+    from jacobiforcing_b200.hybrid_runtime import HybridRuntime
+    cfg = kin.model_config([kin.attn_scan(heads=2, kv_heads=1, dim=64, inner=64), kin.delta(heads=2, kv_heads=1, dim=64, vdim=64)])
+    w = weights(cfg)
+    rt = HybridRuntime(HybridConfig.from_dict(cfg, {k: tuple(t.shape) for k, t in w.items()}), dtype=dtype, max_step_tokens=640, max_step_entries=2, page_size=16,
+                       num_pages=48, max_pages_per_seq=48, num_slots=2, max_want=8)
+    rt.load_state_dict(w)
+    return rt
+
+
+@pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
+def test_workspaces_that_steps_can_do_without(fake, dtype):
+    """Without room for them an engine is made all the same, down to the last byte of what it needs, and its steps take the forms that need none."""
+    def names(room):
+        fake.room(room)
+        before = fake.used()
+        try:
+            rt = roomy_engine(dtype)
+            used = fake.used() - before
+            fake.reset()
+            rt.step([([1] * 600, 0, 0, list(range(48)))], [599], want_logits=True)
+            out = [n for n, _ in fake.launches()]
+            rt.close()
+        finally:
+            fake.room()
+        return used, out
+
+    def has(out, *kernels):
+        return [any(k in n for n in out) for k in kernels]
+    held = fake.used()                                       # by engines that other tests left
+    with_own = ["delta_chunk_chain_kernel", "page_gather_kernel", "split_rows_kernel"] if dtype == "bfloat16" else ["delta_chunk_chain_kernel"]
+    plain = ["delta_head_kernel", "attn_mma_kernel", "gemm_simt_kernel"] if dtype == "bfloat16" else ["delta_head_kernel"]
+    most, fast = names(1 << 40)
+    assert all(has(fast, *with_own)) and not has(fast, "delta_head_kernel")[0] and sum("scan_kernel" in n for n in fast) == 2
+    least, slow = names(held + most)                         # they would leave nothing for kernels that are yet to be loaded
+    assert least < most and all(has(slow, *plain)) and not any(has(slow, *with_own)) and sum("scan_kernel" in n for n in slow) == 1
+    assert names(held + least) == (least, slow)
+    with pytest.raises((RuntimeError, MemoryError)):
+        names(held + least - 1)
+
+
 def test_refused_shared_memory_is_reported(fake):
     rt = engine(FLASH)
     fake.reset()
