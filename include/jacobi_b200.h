@@ -151,7 +151,7 @@ int jf_tp_import(jf_handle h, const void* handles /* tp_size x 64 bytes, rank or
 int jf_tp_attach_local(jf_handle h, const jf_handle* peers);
 
 /* Page-locked host memory for results (the device copies into it without a staging buffer).  0 or JF_ERR_CUDA. */
-int jf_host_alloc(int64_t bytes, void** out);
+int jf_host_alloc(int32_t device, int64_t bytes, void** out);
 int jf_host_free(void* p);
 
 /* Number of kernel launches issued by this handle since creation (bench.py's gpu_launches claim). */

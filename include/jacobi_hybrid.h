@@ -191,7 +191,7 @@ int hy_step(hy_handle h, int32_t n_entries, const int32_t* tokens, const int32_t
             int32_t* sampled_out, const float* temperature, uint64_t seed, float* layers_out);
 
 /* Page-locked host memory for results (the device copies into it without a staging buffer).  HY_OK or HY_ERR_CUDA. */
-int hy_host_alloc(int64_t bytes, void** out);
+int hy_host_alloc(int32_t device, int64_t bytes, void** out);
 int hy_host_free(void* p);
 
 int64_t hy_launch_count(hy_handle h);

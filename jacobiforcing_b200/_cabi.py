@@ -72,7 +72,7 @@ def load() -> C.CDLL:
     if hasattr(lib, "jf_tp_attach_local"):
         lib.jf_tp_attach_local.argtypes = [vp, C.POINTER(vp)]
     if hasattr(lib, "jf_host_alloc"):
-        lib.jf_host_alloc.argtypes = [C.c_int64, C.POINTER(vp)]
+        lib.jf_host_alloc.argtypes = [C.c_int32, C.c_int64, C.POINTER(vp)]
         lib.jf_host_free.argtypes = [vp]
     lib.jf_launch_count.argtypes = [vp]
     lib.jf_launch_count.restype = C.c_int64

@@ -110,7 +110,7 @@ def load() -> C.CDLL:
     lib.hy_last_step_ms.restype = C.c_float
     lib.hy_memory_info.argtypes = [vp, i64p, i64p, i64p, i64p]
     lib.hy_profile_enable.argtypes = [vp, i32]
-    lib.hy_host_alloc.argtypes = [C.c_int64, C.POINTER(vp)]
+    lib.hy_host_alloc.argtypes = [i32, C.c_int64, C.POINTER(vp)]
     lib.hy_host_free.argtypes = [vp]
     lib.hy_profile_read.argtypes = [vp, fp]
     for n in ("hy_host_alloc", "hy_host_free", "hy_profile_enable", "hy_profile_read", "hy_create", "hy_load_tensor", "hy_finalize", "hy_step", "hy_memory_info"):

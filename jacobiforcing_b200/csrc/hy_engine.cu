@@ -469,9 +469,10 @@ extern "C" int hy_memory_info(hy_handle h, int64_t* w, int64_t* c, int64_t* s, i
   return HY_OK;
 }
 
-extern "C" int hy_host_alloc(int64_t bytes, void** out) {
+extern "C" int hy_host_alloc(int32_t device, int64_t bytes, void** out) {
   if (!out || bytes <= 0) return HY_ERR_INVALID;
-  if (cudaHostAlloc(out, (size_t)bytes, cudaHostAllocPortable) == cudaSuccess) return HY_OK;
+  // the calling thread may be on another device, where this would be the first call of the process
+  if (cudaSetDevice(device) == cudaSuccess && cudaHostAlloc(out, (size_t)bytes, cudaHostAllocPortable) == cudaSuccess) return HY_OK;
   cudaGetLastError();                                          // the caller goes on with pageable memory
   return HY_ERR_CUDA;
 }

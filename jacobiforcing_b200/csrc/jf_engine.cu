@@ -608,9 +608,10 @@ static int pack_staged(jf_engine* h, __nv_bfloat16* dst, int R, int K, int dest_
   return JF_OK;
 }
 
-extern "C" int jf_host_alloc(int64_t bytes, void** out) {
+extern "C" int jf_host_alloc(int32_t device, int64_t bytes, void** out) {
   if (!out || bytes <= 0) return JF_ERR_INVALID;
-  if (cudaHostAlloc(out, (size_t)bytes, cudaHostAllocPortable) == cudaSuccess) return JF_OK;
+  // the calling thread may be on another device, where this would be the first call of the process
+  if (cudaSetDevice(device) == cudaSuccess && cudaHostAlloc(out, (size_t)bytes, cudaHostAllocPortable) == cudaSuccess) return JF_OK;
   cudaGetLastError();                                          // the caller goes on with pageable memory
   return JF_ERR_CUDA;
 }

@@ -67,7 +67,7 @@ class HybridRuntime:
         h = C.c_void_p()
         cabi.check(self.lib.hy_create(C.byref(m), layers, C.byref(rt), C.byref(h)), None)
         self.h = h
-        self._results = hostmem.of_library(self.lib.hy_host_alloc, self.lib.hy_host_free, 8 * self.max_want * self.vocab * 4)
+        self._results = hostmem.of_library(self.lib.hy_host_alloc, self.lib.hy_host_free, device, 8 * self.max_want * self.vocab * 4)
         self.stats = {"steps": 0, "tokens": 0, "device_ms": 0.0}
 
     # ---- lifecycle -------------------------------------------------------------------------------------------------

@@ -92,7 +92,7 @@ class JacobiRuntime:
         h = C.c_void_p()
         _cabi.check(self.lib.jf_create(C.byref(self.model_cfg), C.byref(self.runtime_cfg), C.byref(h)), None)
         self.h = h
-        self._results = hostmem.of_library(self.lib.jf_host_alloc, self.lib.jf_host_free)
+        self._results = hostmem.of_library(self.lib.jf_host_alloc, self.lib.jf_host_free, device)
         self.free_pages = list(range(num_kv_pages - 1, -1, -1))
         self._next_seq = 0
         self.stats = {"forwards": 0, "device_ms": 0.0, "rows": 0}

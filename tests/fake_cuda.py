@@ -60,6 +60,10 @@ class Fake:
     def used(self):
         return self.lib.fake_used()
 
+    def pinned(self):
+        """The device of every page-locked region that was made for results since the last reset."""
+        return [self.lib.fake_pinned_device(i) for i in range(self.lib.fake_pinned())]
+
     def on_their_way(self):
         """Copies to the host since the last wait for the stream."""
         return self.lib.fake_on_their_way()

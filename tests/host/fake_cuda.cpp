@@ -22,6 +22,7 @@ constexpr int kKinds = 4;                                        // launches, at
 long g_count[kKinds] = {}, g_fail[kKinds] = {-1, -1, -1, -1};    // how many so far, which one fails
 std::map<void*, size_t> g_device_blocks;                         // what is taken of the device's memory
 size_t g_used = 0, g_room = (size_t)1 << 40;
+std::vector<int> g_pinned;                                       // devices on which results' memory was page-locked
 int g_on_their_way = 0;                                         // copies to the host that nothing has waited for
 constexpr size_t kDefaultSmem = 48 * 1024, kMostSmem = 227 * 1024;
 
@@ -48,11 +49,13 @@ CUresult encode(CUtensorMap* m, CUtensorMapDataType, cuuint32_t, void* p, const 
 
 extern "C" {
 // ---- what a test asks ---------------------------------------------------------------------------------------------------------------
-void fake_reset() { g_launches.clear(); for (int i = 0; i < kKinds; ++i) { g_count[i] = 0; g_fail[i] = -1; } g_last = cudaSuccess; }
+void fake_reset() { g_launches.clear(); g_pinned.clear(); for (int i = 0; i < kKinds; ++i) { g_count[i] = 0; g_fail[i] = -1; } g_last = cudaSuccess; }
 void fake_fail(int what, long at) { g_count[what] = 0; g_fail[what] = at; }
 long fake_count(int what) { return g_count[what]; }
 void fake_room(long long bytes) { g_room = (size_t)bytes; }
 long long fake_used() { return (long long)g_used; }
+int fake_pinned() { return (int)g_pinned.size(); }
+int fake_pinned_device(int i) { return g_pinned[i]; }
 int fake_on_their_way() { return g_on_their_way; }
 int fake_launches() { return (int)g_launches.size(); }
 const char* fake_launch_name(int i) { return names()[g_launches[i].f].c_str(); }
@@ -85,7 +88,10 @@ cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr a, int) {
 }
 cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int* n, const void*, int, size_t, unsigned) { *n = 1; return cudaSuccess; }
 cudaError_t cudaMallocHost(void** p, size_t n) { *p = calloc(n ? n : 1, 1); return *p ? cudaSuccess : last(cudaErrorMemoryAllocation); }
-cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { return cudaMallocHost(p, n); }
+cudaError_t cudaHostAlloc(void** p, size_t n, unsigned f) {
+  if (f & cudaHostAllocPortable) g_pinned.push_back(g_device);
+  return cudaMallocHost(p, n);
+}
 cudaError_t cudaMalloc(void** p, size_t n) {
   if (n > g_room - g_used) return last(cudaErrorMemoryAllocation);
   const cudaError_t e = cudaMallocHost(p, n);

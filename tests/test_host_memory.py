@@ -1,7 +1,10 @@
 """Page-locked memory of results: parts are given back when the last view is gone and used again, what does not fit is pageable, the region outlives its
-pool for as long as an array lives, and threads may take and drop at once."""
+pool for as long as an array lives, and threads may take and drop at once.  Nothing is page-locked before a large result is there, and a forked process
+keeps what it saw."""
 import ctypes as C
 import gc
+import mmap
+import os
 import threading
 
 import numpy as np
@@ -90,3 +93,64 @@ def test_threads():
     [t.start() for t in ts]
     [t.join() for t in ts]
     assert not wrong and len(c.blocks) == 1
+
+
+def test_regions_are_made_for_the_results_that_need_them():
+    mb = 1 << 20
+    c, m = make(64 * mb)
+    held = [m.empty((SMALLEST - 1,), np.uint8)]
+    assert not c.blocks                                                    # small ones need none
+
+    def sizes():
+        return [len(b) // mb for b in c.blocks.values()]
+    held += [m.empty((SMALLEST,), np.uint8) for _ in range(64)]
+    assert sizes() == [4]
+    held += [m.empty((5 * mb,), np.uint8) for _ in range(8)]               # no room: a second region, for eight of these
+    assert sizes() == [4, 40]
+    held += [m.empty((5 * mb,), np.uint8) for _ in range(5)]               # and one with what is left of the limit
+    assert sizes() == [4, 40, 20] and sum(inside(c, a) for a in held) == 64 + 8 + 4
+    held += [m.empty((SMALLEST,), np.uint8)]
+    assert sizes() == [4, 40, 20]
+    m.close()
+    del held
+    gc.collect()
+    assert not c.blocks
+
+
+def test_a_forked_process_keeps_what_it_saw():
+    """Memory as page-locked memory is: shared between the processes."""
+    class Shared(Counted):
+        def alloc(self, size):
+            b = mmap.mmap(-1, size)
+            at = C.addressof(C.c_char.from_buffer(b))
+            self.blocks[at] = b
+            return at
+
+        def free(self, at):
+            self.blocks.pop(at)
+    c = Shared()
+    m = ResultMemory(c.alloc, c.free, 8 * SMALLEST)
+    a = m.empty((SMALLEST,), np.uint8)
+    assert inside(c, a)
+    a.fill(3)
+    there = os.pipe()
+    pid = os.fork()
+    if pid == 0:
+        ok = False
+        try:
+            os.read(there[0], 1)                                           # the parent has dropped its array and made others
+            mine = m.empty((SMALLEST,), np.uint8)
+            ok = bool((a == 3).all()) and not inside(c, mine)
+            mine.fill(9)
+        finally:
+            os._exit(0 if ok else 1)
+    del a
+    gc.collect()
+    others = [m.empty((SMALLEST,), np.uint8) for _ in range(8)]
+    for o in others:
+        o.fill(5)
+    os.write(there[1], b"x")
+    assert os.waitstatus_to_exitcode(os.waitpid(pid, 0)[1]) == 0
+    assert all(inside(c, o) and (o == 5).all() for o in others) and len(c.blocks) == 1      # a new region, the old one is gone
+    for fd in there:
+        os.close(fd)

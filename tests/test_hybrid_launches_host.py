@@ -129,6 +129,20 @@ def test_engines_of_unlike_sizes_take_turns(fake, tokens, dtype):
         rt.close()
 
 
+def test_results_take_page_locked_memory_when_they_are_large(fake):
+    """And on the engine's device, whatever the calling thread was on."""
+    fake.reset()
+    cfg = kin.model_config([kin.delta()], vocab=1100)
+    one, other = engine(cfg, device=1), engine(cfg)
+    step(one, 5)
+    step(other, 5)
+    assert fake.pinned() == []
+    one._results.empty((16, 1100))
+    assert fake.pinned() == [1]
+    one.close()
+    other.close()
+
+
 def roomy_engine(dtype):
     """An engine whose prompt steps have forms with workspaces of their own: chunks, segments, keys and values out of their pages, rows in three parts."""
     from jacobiforcing_b200.hybrid_config import HybridConfig

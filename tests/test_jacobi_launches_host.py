@@ -132,3 +132,15 @@ def test_the_last_layer_of_rows_that_nobody_reads(fake, logits, hidden):
     assert "wide_rope_kernel" in fake.launches()[10][0]
     rt.release(s)
     rt.close()
+
+
+def test_results_take_page_locked_memory_when_they_are_large(fake):
+    """And on the engine's device, whatever the calling thread was on."""
+    fake.reset()
+    one, other = engine(device=1), engine()
+    chunk(other)
+    assert fake.pinned() == []
+    one._results.empty((64 << 10,))
+    assert fake.pinned() == [1]
+    one.close()
+    other.close()
