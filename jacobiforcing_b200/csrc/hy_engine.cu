@@ -201,16 +201,16 @@ struct hy_engine {
 // and a step of prompt tokens as many.  The blocks of a kernel that starts under another one's tail pile up on the SMs that are free already, though, and
 // a recurrence with one block per SM then runs two or three on some of them (two Kinetar layers, 2048 tokens, everything overlapped: 2.02 -> 2.35 ms).  So the
 // kernels whose longest block is their time start behind the kernel before them in steps of more than HY_OVERLAP_TOKENS tokens (go_alone): recurrences and
-// attention over pages; convolutions from HY_ALONE_CONV tokens on.  A layer of one request, us, everything behind one another -> so: 77 tokens of Kinetar's
+// attention over pages; convolutions from HY_ALONE_CONV tokens on.  A layer of one request, us, everything behind one another -> so: 66 tokens of state space
+// 258 -> 231, of retention 241 -> 207, of its attention beside a scan 268 -> 252; 77 tokens of Kinetar's
 // delta rule 146 -> 129, gated linear attention 123 -> 109, its attention beside a scan 187 -> 171; 200 tokens of latent attention 127 -> 110; 1024 tokens
 // of a state-space layer 301 -> 275, of retention 230 -> 219; 2048 tokens of latent attention 237 -> 212, of retention beside experts in four requests 294 -> 264.
 // With convolutions overlapped as well, attention beside a scan takes 445 instead of 419 (1024 tokens); with none, 208 instead of 202 (150 tokens).
-// Steps just above HY_OVERLAP_TOKENS keep plain launches, which test_which_launches_overlap holds them to.
 // Behind the first launch of a step that fails nothing else is launched; hy_step reports it.
 // More shared memory than every kernel may have (48 KiB with its static part) is asked for here, once per engine and kernel: the limit belongs to a
 // device, and a process may hold engines on several.  Always all that the device has: engines of one device share the limit, and what a
 // smaller one asked for would be too little for a larger one.
-constexpr int HY_OVERLAP_TOKENS = 64, HY_OVERLAP_AGAIN = 72, HY_ALONE_CONV = 256;
+constexpr int HY_OVERLAP_TOKENS = 64, HY_ALONE_CONV = 256;
 constexpr size_t HY_PLAIN_SMEM = 16 * 1024;
 inline cudaError_t opt_in(hy_engine* h, const void* kernel, size_t smem) {
   if (smem <= HY_PLAIN_SMEM || h->opted_in.count(kernel)) return cudaSuccess;
@@ -227,7 +227,7 @@ inline void go_kernel(hy_engine* h, void (*kernel)(P...), dim3 grid, dim3 block,
   at.val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t c = {};
   c.gridDim = grid; c.blockDim = block; c.dynamicSmemBytes = smem; c.stream = stream; c.attrs = &at;
-  c.numAttrs = h->plain || (h->step_tokens > HY_OVERLAP_TOKENS && h->step_tokens < HY_OVERLAP_AGAIN) ? 0 : 1;
+  c.numAttrs = h->plain ? 0 : 1;
   if (!h->step_err.empty()) return;
   cudaError_t e = opt_in(h, (const void*)kernel, smem);
   if (e == cudaSuccess) e = cudaLaunchKernelEx(&c, kernel, std::forward<A>(args)...);
