@@ -538,7 +538,7 @@ struct Builder {
   struct Later { void** to; std::vector<uint16_t> tiles; };
   std::vector<Later> later;
   void up_split(void** to, const std::vector<float>& v, int N, int K) {
-    if (rc != HY_OK || h->m.dtype != HY_DTYPE_BF16 || h->rt.max_step_tokens < HY_SPLIT_ROWS) return;
+    if (rc != HY_OK || h->m.dtype != HY_DTYPE_BF16 || h->rt.max_step_tokens < HY_SPLIT_ROWS || K > HY_SPLIT_K) return;
     const int KP = split_cols(K);
     std::vector<float> three((size_t)N * 3 * KP, 0.0f);
     for (int n = 0; n < N; ++n)
@@ -1708,7 +1708,7 @@ int gemm(hy_engine* h, const TA* A, int lda, const TW* Wt, int ldw, int T, int N
   return HY_OK;
 }
 
-// The product of fp32 rows: in three parts on the tensor cores where the rows are many (split_rows_kernel).
+// The product of fp32 rows: in three parts on the tensor cores where the rows are many and short (split_rows_kernel; split NULL: not this layer's).
 template <typename TW>
 int gemm_split(hy_engine* h, const float* A, int lda, const TW* Wt, int ldw, int T, int N, int K, GemmOut o, const void* split) {
   if (!split || T < HY_SPLIT_ROWS) return gemm<float, TW, float>(h, A, lda, Wt, ldw, T, N, K, o);

@@ -116,11 +116,13 @@ struct HyEpilogue {
 // ---- products of fp32 rows with bf16 weights (step sizes) ------------------------------------------------------------------------
 // An fp32 number is the sum of three bf16 numbers, its upper, middle and lower eight bits, so the product of fp32 rows is one of bf16 rows
 // [lower | middle | upper], three times as long, with the weights side by side three times: every product of two numbers is exact as it
-// was, and the sums are the tensor cores' fp32 sums (the upper parts come last, so that what is cut off a sum is cut off few large ones).  Against 64
-// bits, K 128: 1.5e-7 of the result's norm, gemm_simt_kernel 2.0e-7; K 16: 5.1e-8 and 7.1e-8.
+// was, and the sums are the tensor cores' fp32 sums (the upper parts come last, so that what is cut off a sum is cut off few large ones).  Those lose
+// more with every block of k than sums of fp32 additions do, so up to K 128 only.  Against 64 bits, of the result's norm, gemm_simt_kernel -> this:
+// operands of both signs K 16 7.5e-8 -> 5.0e-8, K 64 1.4e-7 -> 7.7e-8, K 128 2.1e-7 -> 1.3e-7, K 256 2.8e-7 -> 2.3e-7, K 512 4.0e-7 -> 4.8e-7; of one
+// sign, where the cut goes the same way every time, K 64 1.2e-7 -> 9.0e-8, K 128 1.7e-7 -> 1.8e-7, K 256 2.4e-7 -> 3.7e-7, K 512 3.3e-7 -> 8.7e-7.
 // N 4096, T 2048, K 128: 85 us on the fp32 units, 21 with both kernels; from 512 rows on (N 2048, T 300, K 64: 12.4 and 11.4; T 100, K 130: 10.4 and
 // 14.5).  Not where every result goes through functions (decays, 2048 x 2048 and K 16: 36 us either way): that is what takes the time there.
-constexpr int HY_SPLIT_ROWS = 512;
+constexpr int HY_SPLIT_ROWS = 512, HY_SPLIT_K = 128;
 inline int split_cols(int K) { return (K + 63) / 64 * 64; }    // of each part
 // a [T, lda] (K columns) -> o [T][3][KP], zeros beyond K.  What is no number, and infinities, stay whole in the upper part.
 __global__ void __launch_bounds__(128) split_rows_kernel(const float* __restrict__ a, int lda, int T, int K, int KP, bf16* __restrict__ o) {

@@ -272,3 +272,19 @@ def test_flash_takes_positive_scales_only(fake, scale, flash):
     step(rt, 150)
     assert any("flash_kernel" in n for n, _ in fake.launches()) == flash
     rt.close()
+
+
+@pytest.mark.parametrize("rank,split", [(128, True), (129, False)])
+def test_rows_in_three_parts_are_short(fake, rank, split):
+    """The tensor cores' sums lose more with every block of k than fp32 additions do."""
+    from jacobiforcing_b200.hybrid_config import HybridConfig
+    from jacobiforcing_b200.hybrid_runtime import HybridRuntime
+    cfg = kin.model_config([kin.attn_scan(inner=64, dt_rank=rank)])
+    w = weights(cfg)
+    rt = HybridRuntime(HybridConfig.from_dict(cfg, {k: tuple(t.shape) for k, t in w.items()}), max_step_tokens=512, max_step_entries=1, page_size=16, num_pages=32,
+                       max_pages_per_seq=32, num_slots=1, max_want=8)
+    rt.load_state_dict(w)
+    fake.reset()
+    rt.step([([1] * 512, 0, 0, list(range(32)))], [511])
+    assert bool(fake.blocks("split_rows_kernel")) == split
+    rt.close()
