@@ -217,8 +217,19 @@ inline bool few_takes(const void* A, int lda, const void* W, size_t ldw, int T, 
   return T <= FEW_ROWS && K % 8 == 0 && lda % 8 == 0 && ldw % 8 == 0 && few_smem(K) <= 200 * 1024 &&
          ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W)) & 15) == 0;
 }
-// One row over few weights stays with a column per warp (gemm_rows_kernel): nothing is shared between rows there, and a block starts sooner.
-inline bool few_pays(int T, int N, int K) { return T > 1 || (N >= 2048 && (long long)N * K >= 6000000); }
+// One or two rows over few weights stay with a column per warp (gemm_rows_kernel): a block starts sooner there.  Behind a small kernel, weights from HBM,
+// us, that kernel and this one, at N x K:
+//   one row     2048 x 2048 5.7 5.6   1024 x 4096 6.1 7.2   3072 x 2048 8.5 7.1   1024 x 7168 9.6 10.1   4096 x 2048 9.2 7.4   32000 x 256 12.2 5.8
+//   two rows    256 x 4096 3.8 7.5    2048 x 1024 3.7 5.3   512 x 7168 6.7 10.4   1024 x 4096 7.4 7.6   2048 x 2048 7.3 6.1   1024 x 7168 12.2 10.7
+//   four rows   512 x 512 3.4 4.5     1024 x 1024 5.2 5.4   256 x 4096 6.7 7.7    2048 x 1024 5.6 5.4   1024 x 2048 5.6 5.8   2048 x 2048 9.8 6.2
+//   five rows   512 x 512 4.8 4.6     256 x 4096 10.1 7.9   2048 x 2048 15.4 6.4
+// Two requests of 24 tokens, every product here -> by this rule: 9.07 -> 8.77 ms and, with experts, 10.63 -> 10.25.  With four, behind longer kernels than that
+// small one, weights that travel ahead make up for the start: the other kernel below two million weights 9.64 ms, every product here 9.53 (11.57 and 11.47); with
+// three 9.11 and 9.14 (11.38 and 11.32).
+inline bool few_pays(int T, int N, int K) {
+  const long long weights = (long long)N * K;
+  return T == 1 ? N >= 2048 && weights >= 6000000 : T > 2 || (N >= 1024 && weights >= 4000000);
+}
 // Warps per tile: as many as bring the SMs a block and a half each, four blocks of 32 k at least for each.  Where a tile for every SM is too many already,
 // blocks are 16 warps on one tile (eight rows, N 1024, K 4096: 11.6 -> 9.2 us; K 7168: 16.8 -> 12.7).
 inline int few_ksplit(long long tiles, int K, int most = 8) {

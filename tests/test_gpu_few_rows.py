@@ -1,14 +1,17 @@
 """bf16 products of one to eight rows on the tensor cores: features beside the tiles of 16, k beside the blocks of 32 and beside what a batch or a split
 holds, sizes that keep the other kernel, and the routed form (experts without a row, experts that every token chose, gated and plain), against the
-fp64 restatements within the bounds of the other bf16 tests.  Tokens without numbers, whose choices are all the same expert, beside healthy ones."""
+fp64 restatements within the bounds of the other bf16 tests.  Tokens without numbers, whose choices are all the same expert, beside healthy ones.
+The kernel by itself where a model takes the other one."""
 import numpy as np
 import pytest
+import torch
 
 from oracle import famepel_plain, kinetar_plain, mafalorn_plain, vosolorn_plain
 from tests import famepel_helpers as fam
 from tests import hybrid_helpers as kin
 from tests import mafalorn_helpers as maf
 from tests import vosolorn_helpers as vos
+from tests.row_ops import RowOps
 
 pytestmark = pytest.mark.gpu
 
@@ -114,3 +117,21 @@ def test_fewer_finite_scores_than_choices(rows):
     finally:
         hz.close()
     assert vos.row_errs(got, vos.oracle_logits(cfg, w, toks)).max() < vos.TOL["bfloat16"]
+
+
+@pytest.fixture(scope="module")
+def ops():
+    return RowOps()
+
+
+@pytest.mark.parametrize("features,cols", [(32000, 1024), (2112, 2048), (1024, 7168), (17, 512), (300, 12280), (40, 8), (33, 264)])
+@pytest.mark.parametrize("rows", [1, 2, 3, 5, 8])
+def test_sums_of_few_rows(ops, rows, features, cols):
+    """fp32 sums outside the tensor core: a sum that stayed in it over 1024 columns would be 3.8e-7 of its norm away.  The bound: a lane adds up to
+    cols / 32 / 4 products of blocks of 16 one behind the other, each with a rounding of 2^-24 of a sum that grows to the result, root mean square of both; a
+    factor of two for what a block's product loses by itself."""
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    a, w = (torch.randn(n, cols, generator=g, device="cuda").bfloat16() for n in (rows, features))
+    want = a.to(torch.float64) @ w.to(torch.float64).T
+    err = ((ops.few(a, w).to(torch.float64) - want).norm() / want.norm()).item()
+    assert err < min(2.0 * max(cols / 128, 8) ** 0.5 * 2.0 ** -24, 3e-7), err

@@ -288,3 +288,14 @@ def test_rows_in_three_parts_are_short(fake, rank, split):
     rt.step([([1] * 512, 0, 0, list(range(32)))], [511])
     assert bool(fake.blocks("split_rows_kernel")) == split
     rt.close()
+
+
+@pytest.mark.parametrize("rows,vocab,few", [(1, 5859, False), (1, 5860, True), (2, 3906, False), (2, 3907, True), (3, 100, True), (8, 100, True)])
+def test_which_products_of_few_rows_run_on_the_tensor_cores(fake, rows, vocab, few):
+    """The output head over 1024 channels, at both sides of each line."""
+    rt = engine(kin.model_config([kin.delta(ff=0)], width=1024, vocab=vocab))
+    fake.reset()
+    rt.step([([1] * 8, 0, 0, list(range(16)))], list(range(rows)))
+    name = fake.launches()[-1][0]
+    assert ("gemm_few_kernel" in name) == few and ("gemm_rows_kernel" in name) != few
+    rt.close()
