@@ -17,6 +17,16 @@ namespace hy {
 
 struct RouteCfg { int experts, top, groups, keep; float scale; };
 
+// What a token chooses when no score compares (scores that are no numbers, or fewer finite ones than choices): the lowest expert that is not among
+// its k choices so far.  A token's choices are distinct in every case: the products of few rows rely on it.
+__device__ __forceinline__ int lowest_free(const int* chosen, int k) {
+  for (int e = 0;; ++e) {
+    bool taken = false;
+    for (int i = 0; i < k; ++i) taken |= chosen[i] == e;
+    if (!taken) return e;
+  }
+}
+
 // One warp per token.  Scores live in shared memory; lane 0 makes the (tiny, serial) choice.  Ties go to the lower index.
 // A group is worth the sum of its two best scores (its single score when groups hold one expert).
 __global__ void __launch_bounds__(32) route_kernel(const float* __restrict__ logits, int ldl, RouteCfg c, int* __restrict__ ids,
@@ -47,11 +57,12 @@ __global__ void __launch_bounds__(32) route_kernel(const float* __restrict__ log
   }
   float sum = 0.0f;
   for (int k = 0; k < c.top; ++k) {
-    int best = 0; float bv = -1.0f;
+    int best = -1; float bv = -1.0f;
     for (int g = 0; g < c.groups; ++g) {
       if (gs[g] != -2.0f) continue;
       for (int i = 0; i < per; ++i) { const float v = s[g * per + i]; if (v > bv) { bv = v; best = g * per + i; } }
     }
+    if (best < 0) best = lowest_free(ids + (size_t)t * c.top, k);
     ids[(size_t)t * c.top + k] = best;
     wts[(size_t)t * c.top + k] = bv;
     sum += bv;
@@ -76,8 +87,9 @@ __global__ void __launch_bounds__(32) route_top_kernel(const float* __restrict__
   if (lane != 0) return;
   float mx = 0.0f, sum = 0.0f;
   for (int k = 0; k < top; ++k) {
-    int best = 0; float bv = -INFINITY;
+    int best = -1; float bv = -INFINITY;
     for (int e = 0; e < experts; ++e) if (s[e] > bv) { bv = s[e]; best = e; }
+    if (best < 0) best = lowest_free(ids + (size_t)t * top, k);
     if (k == 0) mx = bv;                                       // the first choice is the largest: the softmax's maximum
     const float w = expf(bv - mx);
     ids[(size_t)t * top + k] = best;
@@ -137,7 +149,7 @@ __global__ void __launch_bounds__(32) route_corrected_kernel(const float* __rest
       const int oi = __shfl_xor_sync(0xffffffffu, best, o);
       if (ov > bv || (ov == bv && oi < best)) { bv = ov; best = oi; }
     }
-    if (best >= outputs) best = k;                             // only when a logit is not a number: stay inside the tables
+    if (best >= outputs) best = lowest_free(ids + (size_t)t * top, k);      // the warp has seen lane 0's choices (__syncwarp below)
     if (lane == 0) {
       ids[(size_t)t * top + k] = best;
       wts[(size_t)t * top + k] = s[best];

@@ -137,9 +137,8 @@ __global__ void __launch_bounds__(WARPS * 32, 16 / WARPS) gemm_few_kernel(const 
 }
 
 // The routed form: block row e takes the choices of expert e, found among the step's, A row = token (per_token) or pair, output row = pair, as
-// expert_rows_kernel.  Eight at a time: tokens choose an expert once, and a step here has up to eight of them, but a row whose scores are no numbers
-// (or with too few finite ones) has the same expert in several of its choices, and every pair's row is read by the sum behind it.
-// GLU: a tile is 8 gate rows and the 8 up rows N further on.
+// expert_rows_kernel.  They are at most eight, because a step here has at most eight tokens and a token's choices are distinct, whatever its scores (see
+// lowest_free); walking an expert's pairs eight at a time instead cost decode steps up to 1 %.  GLU: a tile is 8 gate rows and the 8 up rows N further on.
 template <typename TO, bool GLU>
 __global__ void __launch_bounds__(256, 2) expert_few_kernel(const bf16* __restrict__ A, int lda, const int* __restrict__ ids, int pairs, int top, int per_token,
                                                             const bf16* __restrict__ W, size_t w_stride, int N, int K, int ksplit, TO* __restrict__ out,
@@ -150,6 +149,20 @@ __global__ void __launch_bounds__(256, 2) expert_few_kernel(const bf16* __restri
   bf16* xs = reinterpret_cast<bf16*>(hy_smem);
   pdl_begin();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, k0 = (lane & 3) * 8;
+  if (warp == 0) {
+    int n = 0;
+    for (int i0 = 0; i0 < pairs; i0 += 32) {
+      const bool hit = i0 + lane < pairs && ids[i0 + lane] == (int)blockIdx.y;
+      const unsigned m = __ballot_sync(0xffffffffu, hit);
+      const int at = n + __popc(m & ((1u << lane) - 1));
+      if (hit && at < FEW_ROWS) mine[at] = i0 + lane;
+      n += __popc(m);
+    }
+    if (lane == 0) count = min(n, FEW_ROWS);
+  }
+  __syncthreads();
+  const int rows = count;
+  if (rows == 0) return;
   constexpr int TN = GLU ? 8 : 16;
   const int per = 8 / ksplit, steps = (K + 31) / 32, each = (steps + ksplit - 1) / ksplit;
   const int s0 = warp % ksplit * each, s1 = min(steps, s0 + each), tiles = (N + TN - 1) / TN;
@@ -160,54 +173,36 @@ __global__ void __launch_bounds__(256, 2) expert_few_kernel(const bf16* __restri
     const bf16* hi = GLU ? (lo ? lo + (size_t)N * K : nullptr) : n + 8 < N ? We + (size_t)(n + 8) * K + k0 : nullptr;
     few_fetch(w, lo, hi, s, s1, k0, K);
   };
-  for (int first = 0;; first += FEW_ROWS) {
-    if (warp == 0) {
-      int n = 0;
-      for (int i0 = 0; i0 < pairs; i0 += 32) {
-        const bool hit = i0 + lane < pairs && ids[i0 + lane] == (int)blockIdx.y;
-        const unsigned m = __ballot_sync(0xffffffffu, hit);
-        const int at = n + __popc(m & ((1u << lane) - 1)) - first;
-        if (hit && at >= 0 && at < FEW_ROWS) mine[at] = i0 + lane;
-        n += __popc(m);
-      }
-      if (lane == 0) count = n;
+  FewBatch w;
+  int tile = blockIdx.x * per + warp / ksplit;
+  fetch(w, tile, s0);
+  few_stage(xs, K, [&](int r) { return r < rows ? A + (size_t)(per_token ? mine[r] / top : mine[r]) * lda : nullptr; });
+  __syncthreads();
+  const bf16* x = xs + g * few_stride(K) + k0;
+  for (int base = blockIdx.x * per; base < tiles; base += gridDim.x * per) {
+    FewSums sums;
+    const int next = tile + gridDim.x * per;
+    for (int s = s0; s < s1; s += FEW_BATCH) {
+      FewBatch n;
+      if (s + FEW_BATCH < s1) fetch(n, tile, s + FEW_BATCH);
+      else fetch(n, next, s0);
+      few_products(sums, w, x, s, s1);
+      w = n;
     }
-    __syncthreads();
-    const int all = count, rows = min(all - first, FEW_ROWS);
-    if (rows <= 0) return;
-    FewBatch w;
-    int tile = blockIdx.x * per + warp / ksplit;
-    fetch(w, tile, s0);
-    few_stage(xs, K, [&](int r) { return r < rows ? A + (size_t)(per_token ? mine[r] / top : mine[r]) * lda : nullptr; });
-    __syncthreads();
-    const bf16* x = xs + g * few_stride(K) + k0;
-    for (int base = blockIdx.x * per; base < tiles; base += gridDim.x * per) {
-      FewSums sums;
-      const int next = tile + gridDim.x * per;
-      for (int s = s0; s < s1; s += FEW_BATCH) {
-        FewBatch n;
-        if (s + FEW_BATCH < s1) fetch(n, tile, s + FEW_BATCH);
-        else fetch(n, next, s0);
-        few_products(sums, w, x, s, s1);
-        w = n;
-      }
-      float c[4];
+    float c[4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) c[i] = sums.total(i);
-      if (ksplit > 1) few_add_parts(c, parts, ksplit, warp, lane);
-      if (warp % ksplit == 0) {
+    for (int i = 0; i < 4; ++i) c[i] = sums.total(i);
+    if (ksplit > 1) few_add_parts(c, parts, ksplit, warp, lane);
+    if (warp % ksplit == 0) {
 #pragma unroll
-        for (int i = 0; i < (GLU ? 2 : 4); ++i) {
-          const int n = tile * TN + g + (i >> 1) * 8, t = (lane & 3) * 2 + (i & 1);
-          if (t >= rows || n >= N) continue;
-          const float v = GLU ? gated_pair_f(act, c[i], c[i + 2], limit) : act >= 0 ? act_f(act, c[i]) : c[i];
-          out[(size_t)mine[t] * ldo + n] = from_f<TO>(v);
-        }
+      for (int i = 0; i < (GLU ? 2 : 4); ++i) {
+        const int n = tile * TN + g + (i >> 1) * 8, t = (lane & 3) * 2 + (i & 1);
+        if (t >= rows || n >= N) continue;
+        const float v = GLU ? gated_pair_f(act, c[i], c[i + 2], limit) : act >= 0 ? act_f(act, c[i]) : c[i];
+        out[(size_t)mine[t] * ldo + n] = from_f<TO>(v);
       }
-      tile = next;
     }
-    if (all <= first + FEW_ROWS) return;
-    __syncthreads();                                           // the rows and their places may be written over
+    tile = next;
   }
 }
 

@@ -1,6 +1,6 @@
 """bf16 products of one to eight rows on the tensor cores: features beside the tiles of 16, k beside the blocks of 32 and beside what a batch or a split
 holds, sizes that keep the other kernel, and the routed form (experts without a row, experts that every token chose, gated and plain), against the
-fp64 restatements within the bounds of the other bf16 tests.  Tokens without numbers, whose choices are all the same expert, beside healthy ones.
+fp64 restatements within the bounds of the other bf16 tests.  Tokens whose router scores do not compare, beside healthy ones.
 The kernel by itself where a model takes the other one."""
 import numpy as np
 import pytest
@@ -104,7 +104,7 @@ def test_a_request_without_numbers_leaves_the_others_alone(kind, tokens):
 
 @pytest.mark.parametrize("rows", [4, 5, 8])
 def test_fewer_finite_scores_than_choices(rows):
-    """A router that leaves one expert: it takes every choice, four times as many as there are tokens, and all but the first of a token weigh nothing."""
+    """A router with one finite score: a token's other choices weigh nothing, and are distinct all the same (an expert takes a token once)."""
     cfg = vos.model_config([vos.mlstm(mlp=vos.moe(experts=6, top=4, ff=24))] * 2)
     w = dict(vosolorn_plain.random_weights(cfg, 0))
     for name in ("l0.mlp.router.b", "l1.mlp.router.b"):
