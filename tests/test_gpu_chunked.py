@@ -28,6 +28,11 @@ def _model(mode, dim, vdim, heads=2):
 MODES = ["state space", "forget", "gated linear", "retention"]
 
 
+def _every_row(helpers, got, want, dtype):
+    """These models choose no experts, so that rounding to bf16 has nothing to flip: it makes up to 2e-2 of a row."""
+    return helpers.close(got, want, dtype) if dtype == "float32" else helpers.row_errs(got, want).max() < 4e-2
+
+
 @pytest.mark.parametrize("dim,vdim,dtype", [(33, 35, "float32"), (64, 64, "float32"), (66, 40, "bfloat16"), (128, 64, "bfloat16"), (100, 128, "float32"), (128, 127, "bfloat16")])
 @pytest.mark.parametrize("mode", MODES)
 def test_chunked_portions(mode, dim, vdim, dtype):
@@ -41,7 +46,7 @@ def test_chunked_portions(mode, dim, vdim, dtype):
         got = hz.feed("a", toks, CUTS)
     finally:
         hz.close()
-    assert helpers.close(got, helpers.oracle_logits(cfg, w, toks), dtype)
+    assert _every_row(helpers, got, helpers.oracle_logits(cfg, w, toks), dtype)
 
 
 def _delta(kind, dim, vdim, heads, kv):
@@ -51,7 +56,7 @@ def _delta(kind, dim, vdim, heads, kv):
 
 
 def _good(kind, got, want, dtype):
-    return kin.rel_err(got, want) < kin.TOL[dtype] if kind == "channel" else maf.close(got, want, dtype)
+    return kin.rel_err(got, want) < kin.TOL[dtype] if kind == "channel" else _every_row(maf, got, want, dtype)
 
 
 @pytest.mark.parametrize("dim,vdim,heads,kv,dtype", [(33, 35, 2, 1, "float32"), (64, 64, 1, 1, "bfloat16"), (64, 65, 2, 2, "float32"), (128, 48, 2, 1, "float32"),

@@ -3,13 +3,17 @@ value columns that fill a block's eight, miss one or need another block, portion
 batch, and the size behind which another kernel takes over; the selective scan's lane layouts and the short convolution's
 chunks; fp32 build against the plain fp64 restatements, within the
 bound of the other fp32 tests (3e-4)."""
+import math
+
 import pytest
+import torch
 
 from oracle import famepel_plain, kinetar_plain, kisadra_plain, mafalorn_plain
 from tests import famepel_helpers as fam
 from tests import hybrid_helpers as kin
 from tests import kisadra_helpers as kis
 from tests import mafalorn_helpers as maf
+from tests.row_ops import RowOps
 
 pytestmark = pytest.mark.gpu
 
@@ -138,3 +142,28 @@ def test_fp32_product_tiles(width, ff, tokens):
 def test_few_rows_many_columns(dtype):
     """Products of five to eight rows with more columns than four blocks per SM hold at eight a block: warps walk several columns."""
     assert _kinetar(kin.delta(ff=4999), cuts=[5, 8, 7, 6], dtype=dtype) < kin.TOL[dtype]
+
+
+@pytest.mark.parametrize("low,high", [(1e-30, 1e-3), (1e-3, 1.0), (1.0, 40.0), (40.0, 87.0)])
+def test_decays_of_the_selective_scan(low, high):
+    """exp(dt a) against 64 bits: the exponential of the hardware is 2^-22 of itself away at most, and three roundings of 2^-24 of a factor near one follow."""
+    g = torch.Generator(device="cuda").manual_seed(1)
+    n = 1 << 20
+    u = torch.rand(n, generator=g, device="cuda", dtype=torch.float64)
+    size = torch.exp(math.log(low) + u * math.log(high / low))
+    dt = torch.exp(math.log(1e-5) + torch.rand(n, generator=g, device="cuda", dtype=torch.float64) * math.log(1e7)).float()
+    a = -(size / dt).float()
+    dt, a = dt.repeat_interleave(2), torch.stack([a, a * 0.9], 1).flatten()
+    want = torch.exp(dt.to(torch.float64) * a.to(torch.float64))
+    got = RowOps().exp_rates(dt, a).to(torch.float64)
+    assert ((got - want).abs() / want).max() < 2.0 ** -22 + 3 * 2.0 ** -24
+
+
+def test_decays_of_the_selective_scan_at_their_ends():
+    """Steps of nothing and of more than can be, rates of nothing and beyond counting, results below the smallest normal number, and what is no number."""
+    inf, nan, big = float("inf"), float("nan"), torch.finfo(torch.float32).max
+    dt = torch.tensor([0.0, 0.0, 1e18, 1e18, big, big, inf, inf, 1.0, 1.0, 1.0, 1.0, nan, nan], device="cuda")
+    a = torch.tensor([-1.0, 0.0, -1e-3, -0.0, -1.0, 0.0, -1.0, 0.0, -inf, -1e30, -88.0, -104.0, -1.0, 0.0], device="cuda")
+    got = RowOps().exp_rates(dt, a).tolist()
+    assert got[:10] == [1.0, 1.0, 0.0, 1.0, 0.0, 1.0, 0.0, 1.0, 0.0, 0.0]
+    assert all(0.0 <= g < 1.2e-38 for g in got[10:12]) and all(math.isnan(g) for g in got[12:])
