@@ -969,7 +969,8 @@ constexpr int HY_CHUNK_TOKENS = 512, HY_CHUNK_ENTRIES = 64;
 inline bool chunk_sizes(int dk, int dv) { return dk > 32 && dk <= CH_MAX_DIM && dv > 32 && dv <= CH_MAX_DIM; }
 // The delta rule's chain has a block per SM, and its blocks behind the first wave wait: 512 tokens of the longest request per wave.  Token by token and in
 // chunks, us, channel decays, 16 heads of 128 x 128: one request of 512 tokens 122 and 107, 1024 232 and 178, 2048 452 and 345; two of 2048
-// 424 and 351, four of 2048 (longest 780) 322 and 366.  One decay per head, 8 heads: 2048 tokens 365 and 263, four requests 187 and 198.
+// 424 and 351, four of 2048 (longest 780) 322 and 366.  One decay per head, 8 heads: 2048 tokens 365 and 263, four requests 187 and 198.  (With a
+// chain of 5.9 us a chunk; at 5.2, one request of 2048 tokens 320, four about 330.)
 inline bool delta_pays(int heads, int dv, int entries, int longest) {
   const long long blocks = (long long)heads * ((dv + DELTA_COLS - 1) / DELTA_COLS) * entries;
   return longest >= HY_CHUNK_TOKENS * ((blocks + 147) / 148);

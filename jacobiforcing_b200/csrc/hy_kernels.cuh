@@ -691,10 +691,9 @@ __global__ void __launch_bounds__(128) attn_sink_kernel(Batch b, const AT* __res
 }
 
 // ---- decays exp(dt a) of two states at a time ---------------------------------------------------------------------------------------
-// dt a log2(e) as a rounded product and its remainder: 2^(y + e) = 2^y + 2^y e ln 2 for the |e| <= 2^-24 |y| that is left.  expf spends eight
-// instructions per state on its argument and its result's exponent, this five and a half; its error
-// against 64 bits is 2.0e-7 at most and 6.5e-8 root mean square from |dt a| = 1 to 80, where expf of the rounded product comes to 3.9e-6 and 9.0e-7, and
-// below one the same as expf's (1.9e-7 and 4.4e-8 against 1.6e-7 and 4.0e-8).
+// dt a log2(e) as a rounded product and its remainder: 2^(y + e) = 2^y + 2^y e ln 2 for the |e| <= 2^-24 |y| that is left; for two states the products
+// run as pairs.  The error against 64 bits is 2.0e-7 at most and 6.5e-8 root mean square from |dt a| = 1 to 87, where expf of the rounded product
+// comes to 3.9e-6 and 7.1e-7, and below one the same as expf's (1.9e-7 and 4.2e-8 against 1.6e-7 and 3.6e-8).
 struct RatePair {
   float2 hi, neg, lo;                                          // a log2(e), its negative, what rounding took off it
   RatePair() = default;
@@ -723,7 +722,7 @@ __device__ __forceinline__ float finite_step(float dt) { return dt > 1e18f ? 1e1
 // L lanes share a channel, each holding NPER CONSECUTIVE states (NPER * L >= nstate; the staged B and C are zero beyond nstate).
 // Inputs of TB tokens are copied asynchronously while the batch before them runs; the read-outs of eight tokens are reduced
 // in one exchange in which every step halves the tokens a lane keeps, so eight tokens run without a shuffle between them.
-// The arithmetic bounds it: about 6 instructions and one exponential per state and token (exp_rates), so the fewer lanes
+// The arithmetic bounds it: half a dozen operations and one exponential per state and token (exp_rates), so the fewer lanes
 // share a channel the less is spent on the exchange and on indices: four states per lane.
 // 2048 tokens, 4096 channels of 16 states: one state per lane, a five-step exchange per token and loads waited for took 949 us
 // (0.46 us per token), this form 369 us.
