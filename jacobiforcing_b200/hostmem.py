@@ -31,8 +31,8 @@ class _Region:
         self.gaps = [(0, size)]                                            # free parts: (offset, size), by offset
         self.returned = deque()                                            # appended by whoever drops an array, drained by take()
 
-    def __del__(self):
-        if self.owner == os.getpid():
+    def __del__(self, getpid=os.getpid):                                   # also when the interpreter ends and modules are empty
+        if self.owner == getpid():
             self.free(self.at)
 
     def take(self, need):

@@ -5,6 +5,8 @@ import ctypes as C
 import gc
 import mmap
 import os
+import subprocess
+import sys
 import threading
 
 import numpy as np
@@ -154,3 +156,12 @@ def test_a_forked_process_keeps_what_it_saw():
     assert all(inside(c, o) and (o == 5).all() for o in others) and len(c.blocks) == 1      # a new region, the old one is gone
     for fd in there:
         os.close(fd)
+
+
+def test_a_region_at_the_interpreters_end():
+    """A pool and an array that a program never lets go of."""
+    src = ("import ctypes as C, sys\nfrom jacobiforcing_b200 import hostmem\nkept = {}\n"
+           "def alloc(n):\n    b = (C.c_char * n)()\n    kept[C.addressof(b)] = b\n    return C.addressof(b)\n"
+           "m = hostmem.ResultMemory(alloc, lambda at: None)\na = m.empty((100000,))\nhostmem.forever = sys.forever = (m, a)\n")
+    r = subprocess.run([sys.executable, "-c", src], capture_output=True, text=True, cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    assert r.returncode == 0 and r.stderr == ""
