@@ -730,7 +730,7 @@ __device__ __forceinline__ float finite_step(float dt) { return dt > 1e18f ? 1e1
 // pass (SCAN_OWN) leaves each segment's own state (the first one's behind the request's, the others' from zero; in the last one's place
 // the request's, which the second pass writes over) and the sum of its step sizes, of which exp(A sum) is the decay over the segment; the
 // second (SCAN_READ) begins with what the segments before it add up to and makes the read-outs.  Most of the arithmetic is
-// done twice, so with the blocks of four requests and more a scan stays whole.  2048 tokens, 4096 channels of 16 states, us, whole -> segments: one
+// done twice, so with many requests, whose blocks fill the SMs, a scan stays whole (see scan_segments).  2048 tokens, 4096 channels of 16 states, us, whole -> segments: one
 // request 371 -> 221 (195 with exp_rates), two 286 -> 250 (224); 288 tokens of one request 60 -> 49 (44), of two 49 -> 46 (43).
 enum ScanPass : int { SCAN_WHOLE = 0, SCAN_OWN = 1, SCAN_READ = 2 };
 // tokens per segment, segments per entry (grid y: entry by entry); own states [entry, segment][inner][nstate], sums of step sizes
@@ -931,12 +931,16 @@ __global__ void __launch_bounds__(128) scan_kernel(Batch b, const AT* __restrict
   if (live && ends) to_rows(st);
 }
 
-// Segments of a scan: as many as give every SM SCAN_BLOCKS blocks, at least three of at least SCAN_SEG_TOKENS tokens.
+// Segments of a scan: as many as give every SM SCAN_BLOCKS blocks, at least three (four with four requests and more) of at least SCAN_SEG_TOKENS tokens.
+// 16 states, us, whole -> segments.  4096 channels: 288 tokens 45 -> 39, 512 78 -> 57, 1024 152 -> 106, 2048 298 -> 190; 2048 tokens of two requests 251 -> 218
+// in three segments, of three 171 -> 180 in four (for which SCAN_BLOCKS has no room).  2048 channels: 288 tokens 45 -> 33, 512 77 -> 45, 2048 297 -> 103; of two
+// requests 218 -> 119, of three 157 -> 105, of four 125 -> 136 in three segments and 104 in six, of eight 80 -> 114 in three.  Segments of no less than 192
+// tokens: 288 tokens 45 (none), 512 78 (none).
 constexpr int SCAN_BLOCKS = 6, SCAN_SEG_TOKENS = 96;
 inline int scan_segment_rows(int blocks) { return 148 * SCAN_BLOCKS / (blocks < 1 ? 1 : blocks); }      // entries x segments at most
 inline ScanSegments scan_segments(float* own, int blocks, int entries, int longest, int inner, int nstate) {
   const int fit = scan_segment_rows(blocks) / entries, n = fit < longest / SCAN_SEG_TOKENS ? fit : longest / SCAN_SEG_TOKENS;
-  if (!own || n < 3) return ScanSegments{0, 1, nullptr, nullptr};
+  if (!own || n < (entries < 4 ? 3 : 4)) return ScanSegments{0, 1, nullptr, nullptr};
   const int tokens = ((longest + n - 1) / n + 31) / 32 * 32, count = (longest + tokens - 1) / tokens;
   return ScanSegments{tokens, count, own, own + (size_t)entries * count * inner * nstate};
 }

@@ -299,3 +299,20 @@ def test_which_products_of_few_rows_run_on_the_tensor_cores(fake, rows, vocab, f
     name = fake.launches()[-1][0]
     assert ("gemm_few_kernel" in name) == few and ("gemm_rows_kernel" in name) != few
     rt.close()
+
+
+@pytest.mark.parametrize("entries,inner,tokens,passes", [(1, 2048, 287, 1), (1, 2048, 288, 2), (3, 2048, 400, 2), (4, 2048, 400, 1), (4, 1024, 383, 1), (4, 1024, 384, 2),
+                                                         (3, 4096, 600, 1), (2, 4096, 288, 2)])
+def test_which_scans_run_in_segments(fake, entries, inner, tokens, passes):
+    """The longest request has so many tokens, the others ten."""
+    from jacobiforcing_b200.hybrid_config import HybridConfig
+    from jacobiforcing_b200.hybrid_runtime import HybridRuntime
+    cfg = kin.model_config([kin.attn_scan(inner=inner, state=16)])
+    w = weights(cfg)
+    rt = HybridRuntime(HybridConfig.from_dict(cfg, {k: tuple(t.shape) for k, t in w.items()}), max_step_tokens=640, max_step_entries=4, page_size=16,
+                       num_pages=160, max_pages_per_seq=40, num_slots=4, max_want=8)
+    rt.load_state_dict(w)
+    fake.reset()
+    rt.step([([1] * (10 if e else tokens), 0, e, list(range(40 * e, 40 * e + 40))) for e in range(entries)], [0])
+    assert sum("scan_kernel" in n for n, _ in fake.launches()) == passes
+    rt.close()
