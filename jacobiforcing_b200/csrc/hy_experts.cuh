@@ -18,8 +18,9 @@ namespace hy {
 struct RouteCfg { int experts, top, groups, keep; float scale; };
 
 // What a token chooses when no score compares (scores that are no numbers, or fewer finite ones than choices): the lowest expert that is not among
-// its k choices so far.  A token's choices are distinct in every case: the products of few rows rely on it.
-__device__ __forceinline__ int lowest_free(const int* chosen, int k) {
+// its k choices so far.  A token's choices are distinct in every case: the products of few rows rely on it.  Out of line, where it costs choices that
+// compare nothing (in line, steps of eight tokens took 0.5 to 0.9 % longer).
+__device__ __noinline__ int lowest_free(const int* chosen, int k) {
   for (int e = 0;; ++e) {
     bool taken = false;
     for (int i = 0; i < k; ++i) taken |= chosen[i] == e;
