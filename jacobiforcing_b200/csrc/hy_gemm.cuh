@@ -120,8 +120,9 @@ struct HyEpilogue {
 // more with every block of k than sums of fp32 additions do, so up to K 128 only.  Against 64 bits, of the result's norm, gemm_simt_kernel -> this:
 // operands of both signs K 16 7.5e-8 -> 5.0e-8, K 64 1.4e-7 -> 7.7e-8, K 128 2.1e-7 -> 1.3e-7, K 256 2.8e-7 -> 2.3e-7, K 512 4.0e-7 -> 4.8e-7; of one
 // sign, where the cut goes the same way every time, K 64 1.2e-7 -> 9.0e-8, K 128 1.7e-7 -> 1.8e-7, K 256 2.4e-7 -> 3.7e-7, K 512 3.3e-7 -> 8.7e-7.
-// N 4096, T 2048, K 128: 85 us on the fp32 units, 21 with both kernels; from 512 rows on (N 2048, T 300, K 64: 12.4 and 11.4; T 100, K 130: 10.4 and
-// 14.5).  Not where every result goes through functions (decays, 2048 x 2048 and K 16: 36 us either way): that is what takes the time there.
+// us, gemm_simt_kernel and both kernels here: N 4096, K 128, T 100 10.7 11.7, T 300 18.5 11.8, T 512 36.2 12.2, T 2048 88.3 18.4; N 2048, K 128, T 200 10.6
+// 11.5, T 512 16.4 12.0; N 2048, K 64, T 200 6.4 10.3, T 300 10.5 10.5, T 512 11.8 10.6, T 2048 35.6 12.6.  From 512 rows on nothing is slower.  Not
+// where every result goes through functions (decays, 2048 x 2048 and K 16: 36 us either way): that is what takes the time there.
 constexpr int HY_SPLIT_ROWS = 512, HY_SPLIT_K = 128;
 inline int split_cols(int K) { return (K + 63) / 64 * 64; }    // of each part
 // a [T, lda] (K columns) -> o [T][3][KP], zeros beyond K.  What is no number, and infinities, stay whole in the upper part.
