@@ -91,9 +91,11 @@ class ResultMemory:
         return np.asarray(_Part(*part, need, tuple(shape), dtype))
 
     def _take(self, need):
-        for region in self._regions:
+        for i, region in enumerate(self._regions):
             offset = region.take(need)
             if offset is not None:
+                if i:                                                      # the next one is tried there first
+                    self._regions[0], self._regions[i] = region, self._regions[0]
                 return region, offset
         size = min(self._size - sum(r.size for r in self._alive), max(RESULTS * need, LEAST))
         if size < need:
@@ -103,7 +105,7 @@ class ResultMemory:
             self._size = 0                                                 # nothing more to be had
             return None
         region = _Region(at, size, self._free)
-        self._regions.append(region)
+        self._regions.insert(0, region)
         self._alive.add(region)
         return region, region.take(need)
 
