@@ -13,6 +13,7 @@
 
 #include "jf_kernel.cuh"
 #include "jf_wide.cuh"
+#include "jf_step.cuh"
 #include "../../include/jacobi_b200.h"
 
 using namespace jf;
@@ -21,6 +22,7 @@ static_assert(sizeof(jf_policy_knobs) == sizeof(PolicyKnobs), "jf_policy_knobs m
 static_assert(sizeof(DevCtx) % 16 == 0 && sizeof(DevCtx) <= 5120, "DevCtx is staged in shared memory");
 
 static thread_local std::string g_create_error;
+constexpr size_t kStepWeights = 7000000;       // bytes of a layer's weights (step_pays)
 
 struct jf_engine {
   int device = 0;
@@ -58,6 +60,8 @@ struct jf_engine {
   FlashUnit* wide_units_d = nullptr;
   size_t wide_units_cap = 0;
   int* wide_err = nullptr;
+  bool by_stages = false;            // forwards run as one kernel per stage (jf_step.cuh)
+  PlanHdr* run_hdr = nullptr;        // page-locked: the header of the forward that a Jacobi run is about to make
   // per-call draft sources of jf_jacobi_run (first-call tokens, MT19937 states, pad streams): grown on demand, kept
   int* run_scratch[3] = {nullptr, nullptr, nullptr};
   size_t run_scratch_words[3] = {0, 0, 0};
@@ -410,7 +414,9 @@ extern "C" int jf_create(const jf_model_cfg* m, const jf_runtime_cfg* r, jf_hand
 #undef ALLOC
   if (cudaFuncSetAttribute(jf_persistent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, h->smem_optin) != cudaSuccess)
     return fail(JF_ERR_CUDA, "cannot opt in to the full shared memory carve-out");
-  if (tp == 1 && wide_opt_in(md.d) != cudaSuccess) return fail(JF_ERR_CUDA, "cannot opt in to the prompt kernels' shared memory");
+  h->by_stages = tp == 1 && 2 * ((size_t)md.h * (md.qkv_dim + md.q_dim) + (size_t)3 * md.h * md.inter) >= kStepWeights;
+  if (const char* es = getenv("JF_BY_STAGES")) h->by_stages = tp == 1 && atoi(es) != 0;
+  if (tp == 1 && (wide_opt_in(md.d) != cudaSuccess || step_opt_in(h->smem_optin) != cudaSuccess)) return fail(JF_ERR_CUDA, "cannot opt in to the prompt kernels' shared memory");
   int occ = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, jf_persistent_kernel, kNumThreads, h->smem_optin);
   if (occ < 1) return fail(JF_ERR_CUDA, "persistent kernel does not fit on an SM");
@@ -426,6 +432,7 @@ extern "C" int jf_destroy(jf_handle h) {
   for (void* p : h->ipc_maps) cudaIpcCloseMemHandle(p);
   for (void* p : h->allocs) cudaFree(p);
   for (int* p : h->run_scratch) if (p) cudaFree(p);
+  if (h->run_hdr) cudaFreeHost(h->run_hdr);
   cudaEventDestroy(h->ev0);
   cudaEventDestroy(h->ev1);
   cudaStreamDestroy(h->stream);
@@ -873,6 +880,96 @@ static int run_wide(jf_engine* h, int T, const std::vector<Group>& groups, int l
   return JF_OK;
 }
 
+// Whether forwards run as one kernel per stage: an engine on one GPU whose layers hold kStepWeights bytes or more (jf_step.cuh says why
+// the results are the same).  Small models keep the persistent kernel, for which a forward, and a run of any number of forwards, is one
+// launch and none of the host's time; stages would be faster there too, by tens of microseconds a forward.  us a forward, persistent ->
+// stages, in a run of one sequence in blocks of 16 / of four with lookahead blocks / a planned one of 8 rows, by a layer's bytes:
+// 1.2 MB 112 -> 99 / 335 -> 148 / 197 -> 150;  5.6 MB 221 -> 193 / 543 -> 277 / 295 -> 230;  7.6 MB 587 -> 462 / 1436 -> 700 /
+// 666 -> 503;  30 MB 1287 -> 1128 / 2736 -> 1780 / 1337 -> 1175;  466 MB (7B), blocks of 32, one / eight sequences 3260 -> 3040 / 7300 -> 4340.
+// Sampling verification, tensor parallelism and profiles of the stages keep the persistent kernel as well.
+static bool step_pays(const jf_engine* h) {
+  const DevCtx& c = h->hctx;
+  return h->by_stages && c.ng_mode == 0 && c.debug_skip == 0 && !(c.prof && c.prof_forward >= 0);
+}
+
+// What went through ends, and the argmax keys are clean for the next forward.
+static int step_failed(jf_engine* h, const char* what) {
+  cudaMemsetAsync(h->hctx.argmax_keys, 0, (size_t)2 * h->hctx.T_cap * 8, h->stream);
+  cudaStreamSynchronize(h->stream);
+  cudaGetLastError();
+  h->err = std::string("forward by stages: ") + what;
+  return JF_ERR_CUDA;
+}
+
+// One forward of a plan that is on the device, enqueued as one kernel per stage.
+static int run_step(jf_engine* h, const PlanHdr& p, int n_commit) {
+  DevCtx& c = h->hctx;
+  if (h->wide_err == nullptr) {
+    int rc = dev_alloc(h, &h->wide_err, 4, &h->bytes_act);
+    if (rc != JF_OK) return rc;
+  }
+  const StepPlan sp{p.T, p.G, std::max(1, p.attn_hsplit), p.attn_units, p.max_len, n_commit, p.n_lm_tasks, p.iter & 1, p.want_logits, p.lm_row0, p.lm_rows, c.tag_base + 1u};
+  c.tag_base += 2u;
+  WideStream w{h->stream};
+  step_forward(w, c, sp, h->num_ctas, h->smem_optin, h->wide_err);
+  h->launches += w.launches;
+  return w.failed ? step_failed(h, w.failed) : JF_OK;
+}
+static int step_check(jf_engine* h) {
+  int e = 0;
+  JF_CUDA(h, cudaMemcpy(&e, h->wide_err, 4, cudaMemcpyDeviceToHost));
+  if (e) {
+    cudaMemset(h->wide_err, 0, 4);
+    return step_failed(h, "a wait inside a tensor-core kernel ran out (pipeline stalled)");
+  }
+  return JF_OK;
+}
+static int run_step_planned(jf_engine* h, const PlanHdr& p, float* elapsed_ms) {
+  DevCtx& c = h->hctx;
+  JF_CUDA(h, cudaEventRecord(h->ev0, h->stream));
+  int rc = run_step(h, p, 0);
+  if (rc != JF_OK) return rc;
+  WideStream w{h->stream};
+  for (int i = 0; i < p.n_lm_tasks; ++i)
+    w.launch(step_greedy_kernel, (p.lm_rows[i] + 255) / 256, 256, 0, c.argmax_keys + (size_t)(p.iter & 1) * c.T_cap, p.lm_row0[i], p.lm_rows[i], c.greedy);
+  step_commit(w, c, p.n_commit_after);
+  h->launches += w.launches;
+  if (w.failed) return step_failed(h, w.failed);
+  JF_CUDA(h, cudaEventRecord(h->ev1, h->stream));
+  JF_CUDA(h, cudaStreamSynchronize(h->stream));
+  JF_CUDA(h, cudaGetLastError());
+  if (elapsed_ms) cudaEventElapsedTime(elapsed_ms, h->ev0, h->ev1);
+  return step_check(h);
+}
+
+// A Jacobi run: the policy on the device, the forward that it asks for by stages, until every sequence is done.
+static int run_steps(jf_engine* h, int max_forwards, float* elapsed_ms) {
+  DevCtx& c = h->hctx;
+  if (h->run_hdr == nullptr) JF_CUDA(h, cudaMallocHost(&h->run_hdr, sizeof(PlanHdr)));
+  JF_CUDA(h, cudaEventRecord(h->ev0, h->stream));
+  bool any = false;
+  for (;;) {
+    step_policy_kernel<<<1, kNumThreads, kPolicySmem, h->stream>>>(h->dctx, !any, max_forwards);
+    JF_CUDA(h, cudaGetLastError());
+    ++h->launches;
+    JF_CUDA(h, cudaMemcpyAsync(h->run_hdr, c.hdr, sizeof(PlanHdr), cudaMemcpyDeviceToHost, h->stream));
+    JF_CUDA(h, cudaStreamSynchronize(h->stream));
+    if (h->run_hdr->done || h->run_hdr->T < 1) break;
+    const int rc = run_step(h, *h->run_hdr, h->run_hdr->n_commit);
+    if (rc != JF_OK) return rc;
+    any = true;
+  }
+  WideStream w{h->stream};
+  step_commit(w, c, h->run_hdr->n_commit);
+  h->launches += w.launches;
+  if (w.failed) return step_failed(h, w.failed);
+  JF_CUDA(h, cudaMemsetAsync(c.argmax_keys, 0, (size_t)2 * c.T_cap * 8, h->stream));      // clean for the next run
+  JF_CUDA(h, cudaEventRecord(h->ev1, h->stream));
+  JF_CUDA(h, cudaStreamSynchronize(h->stream));
+  cudaEventElapsedTime(elapsed_ms, h->ev0, h->ev1);
+  return any ? step_check(h) : JF_OK;
+}
+
 extern "C" int jf_forward(jf_handle h, int32_t T, const int32_t* tokens, int32_t G, const int32_t* groups,
                           int32_t n_seqs, const int32_t* block_tables, int32_t lm_row0, int32_t lm_rows,
                           int32_t n_commit, const int32_t* commits, int32_t* greedy, float* logits, void* hidden,
@@ -924,6 +1021,7 @@ extern "C" int jf_forward(jf_handle h, int32_t T, const int32_t* tokens, int32_t
   hdr.T = T; hdr.G = G; hdr.done = 0; hdr.n_commit = 0; hdr.n_commit_after = n_commit; hdr.attn_units = units;
   hdr.attn_slots = slots;
   hdr.attn_hsplit = hsplit;
+  hdr.max_len = max_len;
   hdr.n_lm_tasks = 0;
   for (int r = 0; r < lm_rows; r += kArgmaxRows) {
     if (hdr.n_lm_tasks >= kMaxLmTasks) { h->err = "too many LM rows"; return JF_ERR_CAPACITY; }
@@ -953,9 +1051,11 @@ extern "C" int jf_forward(jf_handle h, int32_t T, const int32_t* tokens, int32_t
   JF_CUDA(h, cudaMemcpyAsync(c.block_tables, block_tables, (size_t)n_seqs * c.max_pages_per_seq * 4, cudaMemcpyHostToDevice, h->stream));
   JF_CUDA(h, cudaStreamSynchronize(h->stream));     // the host vectors above go out of scope
   const bool wide = takes_wide(h, T, hg, row_group, lm_rows, hc, n_commit);
-  int rc = wide ? run_wide(h, T, hg, lm_row0, lm_rows, hidden != nullptr, elapsed_ms) : launch_persistent(h, RUN_PLAN, 1, elapsed_ms);
+  const bool step = !wide && step_pays(h);
+  int rc = wide ? run_wide(h, T, hg, lm_row0, lm_rows, hidden != nullptr, elapsed_ms)
+                : step ? run_step_planned(h, hdr, elapsed_ms) : launch_persistent(h, RUN_PLAN, 1, elapsed_ms);
   if (rc != JF_OK) return rc;
-  if (!wide) {
+  if (!wide && !step) {
     int dev_err = 0;
     JF_CUDA(h, cudaMemcpy(&dev_err, reinterpret_cast<const uint8_t*>(c.hdr) + offsetof(PlanHdr, error), 4, cudaMemcpyDeviceToHost));
     if (dev_err != 0) { h->err = "device-side error " + std::to_string(dev_err) + " during the forward"; return JF_ERR_CUDA; }
@@ -1100,10 +1200,16 @@ extern "C" int jf_jacobi_run(jf_handle h, int32_t n_seqs, const jf_policy_knobs*
   }
   TRYC(cudaStreamSynchronize(h->stream));
   float ms = 0.f;
-  TRY(launch_persistent(h, RUN_JACOBI, max_forwards > 0 ? max_forwards : (1 << 30), &ms));
-  // results
+  const int forwards = max_forwards > 0 ? max_forwards : (1 << 30);
   PlanHdr hdr;
-  TRYC(cudaMemcpy(&hdr, c.hdr, sizeof(hdr), cudaMemcpyDeviceToHost));
+  if (step_pays(h)) {
+    TRY(run_steps(h, forwards, &ms));
+    hdr = *h->run_hdr;
+  } else {
+    TRY(launch_persistent(h, RUN_JACOBI, forwards, &ms));
+    TRYC(cudaMemcpy(&hdr, c.hdr, sizeof(hdr), cudaMemcpyDeviceToHost));
+  }
+  // results
   TRYC(cudaMemcpy(hgen.data(), c.gen, hgen.size() * 4, cudaMemcpyDeviceToHost));
   int policy_err = 0;
   for (int s = 0; s < n_seqs; ++s) {

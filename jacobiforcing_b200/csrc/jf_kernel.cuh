@@ -258,7 +258,7 @@ __device__ __noinline__ void policy_stage_jacobi(const DevCtx& c, const WorkerSh
       T += B * L;
     }
     hdr->rows_total = (first ? 0 : ld_weak(&hdr->rows_total)) + T;
-    hdr->T = T; hdr->G = G; hdr->n_commit = nc; hdr->attn_units = units; hdr->attn_slots = slots; hdr->attn_hsplit = hsplit;
+    hdr->T = T; hdr->G = G; hdr->n_commit = nc; hdr->attn_units = units; hdr->attn_slots = slots; hdr->attn_hsplit = hsplit; hdr->max_len = max_len;
     hdr->iter = iter_done;
     hdr->want_logits = 0;
     if (err) hdr->error = err;

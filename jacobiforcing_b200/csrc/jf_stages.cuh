@@ -767,8 +767,9 @@ __device__ __noinline__ void qkv_rope_tail(const DevCtx& c, const WorkerShared* 
 // Chunks are aligned to ABSOLUTE key positions, so a query's result does not depend on how its keys are split between
 // committed pages and in-flight scratch rows (AR decoding and Jacobi decoding of the same prefix agree bit for bit).
 // ---------------------------------------------------------------------------------------------------------------
-template <int D>
-__device__ __forceinline__ void attention_unit(const DevCtx& c, const WorkerCtx& w, int layer, const Group& grp, int g_kvh, int chunk,
+// ONE_ROUND: no more 16-row tiles than warps
+template <int D, bool ONE_ROUND = false, class C, class W>
+__device__ __forceinline__ void attention_unit(const C& c, const W& w, int layer, const Group& grp, int g_kvh, int chunk,
                                int qs, int hs, bool prefetched, int hsplit) {
   constexpr int LDS = D + 8;                  // padded smem row (bf16 elements) -> conflict-free fragment loads
   constexpr int VPR = D / 8;                  // 16-byte chunks per row
@@ -845,7 +846,7 @@ __device__ __forceinline__ void attention_unit(const DevCtx& c, const WorkerCtx&
     }
   };
   uint32_t qnx[D / 16][4];
-  for (int tb = 0; tb * 4 < tiles; ++tb) {
+  for (int tb = 0; tb * 4 < (ONE_ROUND ? 1 : tiles); ++tb) {
     const int tile = tb * 4 + w.wwarp();
     const bool tvalid = tile < tiles;
     const int j = j_lo + (tvalid ? tile / ntt : 0);
@@ -862,7 +863,7 @@ __device__ __forceinline__ void attention_unit(const DevCtx& c, const WorkerCtx&
 #pragma unroll
       for (int ks = 0; ks < D / 16; ++ks) { qf[ks][0] = qnx[ks][0]; qf[ks][1] = qnx[ks][1]; qf[ks][2] = qnx[ks][2]; qf[ks][3] = qnx[ks][3]; }
     }
-    if ((tb + 1) * 4 < tiles) load_q(tile + 4, qnx);       // next round's queries are in flight while this round computes
+    if (!ONE_ROUND && (tb + 1) * 4 < tiles) load_q(tile + 4, qnx);       // next round's queries are in flight while this round computes
     if (nsub == 1 && tb == 0) {
       cp_async_wait_all();
       workers_sync();
@@ -1288,7 +1289,8 @@ __device__ __noinline__ void stage_attention(const DevCtx& c, WorkerShared* ws, 
 // merge the per-chunk partials of every (token, head) in chunk order; write bf16 into the O-projection operand.
 // One warp per (token, head), two items in flight per warp; lane ch holds the statistics of chunk ch, the chunk
 // vectors are fetched 8 at a time per item.  (Rows with more than 32 visible chunks take the generic two-pass path.)
-__device__ __forceinline__ void combine_store(const DevCtx& c, int t, int head, int lane, int vpl, int D,
+template <class C>
+__device__ __forceinline__ void combine_store(const C& c, int t, int head, int lane, int vpl, int D,
                                               const float (&acc)[4], float l) {
   const float inv = 1.0f / l;
   const int f = head * D + lane * vpl;                      // feature index = k index of the O projection
@@ -1301,6 +1303,43 @@ __device__ __forceinline__ void combine_store(const DevCtx& c, int t, int head, 
   } else {
     *reinterpret_cast<uint32_t*>(dst) = pack_bf16x2(acc[0] * inv, acc[1] * inv);
   }
+}
+
+// long contexts: generic two-pass merge over all chunks of one (token, head), by a warp
+template <class C>
+__device__ __forceinline__ void attn_merge_long(const C& c, int t, int head, size_t base, int cmax, int lane, int vpl, int D) {
+  const size_t cstride = c.md.n_q;
+  float mg = -INFINITY;
+  for (int c0 = 0; c0 <= cmax; c0 += 32) {
+    const int ch = c0 + lane;
+    const float mc = (ch <= cmax) ? ld_weak(c.attn_ml + (base + ch * cstride) * 2) : -INFINITY;
+    mg = fmaxf(mg, mc);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) mg = fmaxf(mg, __shfl_xor_sync(0xffffffffu, mg, o));
+  float lg = 0.f;
+  float ag[4] = {0.f, 0.f, 0.f, 0.f};
+  for (int c0 = 0; c0 <= cmax; c0 += 32) {
+    const int chl = c0 + lane;
+    float2 ml = make_float2(-INFINITY, 0.f);
+    if (chl <= cmax) ml = ld_weak(reinterpret_cast<const float2*>(c.attn_ml + (base + chl * cstride) * 2));
+    const float wq = (ml.x == -INFINITY) ? 0.f : __expf(ml.x - mg);
+    const float lq = wq * ml.y;
+    const int nch = min(32, cmax + 1 - c0);
+    for (int u = 0; u < nch; ++u) {
+      const float wgt = __shfl_sync(0xffffffffu, wq, u);
+      lg += __shfl_sync(0xffffffffu, lq, u);
+      const float* op = c.attn_o + (base + (size_t)(c0 + u) * cstride) * D + lane * vpl;
+      if (vpl == 4) {
+        const float4 v = ld_weak(reinterpret_cast<const float4*>(op));
+        ag[0] += wgt * v.x; ag[1] += wgt * v.y; ag[2] += wgt * v.z; ag[3] += wgt * v.w;
+      } else {
+        const float2 v = ld_weak(reinterpret_cast<const float2*>(op));
+        ag[0] += wgt * v.x; ag[1] += wgt * v.y;
+      }
+    }
+  }
+  combine_store(c, t, head, lane, vpl, D, ag, lg);
 }
 
 __device__ __noinline__ void stage_attn_combine(const DevCtx& c, const WorkerShared* ws, int T) {
@@ -1377,38 +1416,8 @@ __device__ __noinline__ void stage_attn_combine(const DevCtx& c, const WorkerSha
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
       if (tt[q] < 0) continue;
-      if (cmax[q] >= 32) {                                   // long contexts: generic two-pass merge over all chunks
-        float mg = -INFINITY;
-        for (int c0 = 0; c0 <= cmax[q]; c0 += 32) {
-          const int ch = c0 + w.lane();
-          const float mc = (ch <= cmax[q]) ? ld_weak(c.attn_ml + (base[q] + ch * cstride) * 2) : -INFINITY;
-          mg = fmaxf(mg, mc);
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) mg = fmaxf(mg, __shfl_xor_sync(0xffffffffu, mg, o));
-        float lg = 0.f;
-        float ag[4] = {0.f, 0.f, 0.f, 0.f};
-        for (int c0 = 0; c0 <= cmax[q]; c0 += 32) {
-          const int chl = c0 + w.lane();
-          float2 ml = make_float2(-INFINITY, 0.f);
-          if (chl <= cmax[q]) ml = ld_weak(reinterpret_cast<const float2*>(c.attn_ml + (base[q] + chl * cstride) * 2));
-          const float wq = (ml.x == -INFINITY) ? 0.f : __expf(ml.x - mg);
-          const float lq = wq * ml.y;
-          const int nch = min(32, cmax[q] + 1 - c0);
-          for (int u = 0; u < nch; ++u) {
-            const float wgt = __shfl_sync(0xffffffffu, wq, u);
-            lg += __shfl_sync(0xffffffffu, lq, u);
-            const float* op = c.attn_o + (base[q] + (size_t)(c0 + u) * cstride) * D + w.lane() * vpl;
-            if (vpl == 4) {
-              const float4 v = ld_weak(reinterpret_cast<const float4*>(op));
-              ag[0] += wgt * v.x; ag[1] += wgt * v.y; ag[2] += wgt * v.z; ag[3] += wgt * v.w;
-            } else {
-              const float2 v = ld_weak(reinterpret_cast<const float2*>(op));
-              ag[0] += wgt * v.x; ag[1] += wgt * v.y;
-            }
-          }
-        }
-        combine_store(c, tt[q], hh[q], w.lane(), vpl, D, ag, lg);
+      if (cmax[q] >= 32) {
+        attn_merge_long(c, tt[q], hh[q], base[q], cmax[q], w.lane(), vpl, D);
       } else {
         combine_store(c, tt[q], hh[q], w.lane(), vpl, D, acc[q], l[q]);
       }

@@ -69,6 +69,7 @@ struct PlanHdr {
   int n_commit_after;        // plan mode: commit entries to apply once the forward is done
   int rows_total;            // sum of T over the forwards of this launch
   int attn_hsplit;           // attention units per kv head along its q heads, chosen per forward (pick_attn_hsplit)
+  int max_len;               // rows of the longest group
 };
 
 struct SeqSlot {             // per-sequence bookkeeping owned by the policy stage

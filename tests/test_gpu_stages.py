@@ -1,0 +1,124 @@
+"""Forwards as one kernel per stage (jf_step.cuh) against the persistent kernel: the same bits, so nothing depends on which of the two runs
+a forward.  Row counts around the tiles of 16, 128 and 256 rows and where the rings and accumulators change, groups beyond a warp,
+odd contexts, contexts of more than 32 chunks, rows behind the last one that a head takes, commits, hidden rows, whole Jacobi runs;
+heads of 64 and 128, gate/up with and without k-splits."""
+import random
+
+import numpy as np
+import pytest
+import torch
+
+from jacobiforcing_b200.runtime import hf_generate
+from tests.gpu_helpers import make_pair
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = {"tiny": ("tiny", "4"), "tiny128": ("tiny128", "4"), "tiny-whole-gate": ("tiny", "1"), "tiny128-whole-gate": ("tiny128", "1")}
+
+
+@pytest.fixture(scope="module", params=list(SHAPES))
+def both(request):
+    name, gate = SHAPES[request.param]
+    mp, made = pytest.MonkeyPatch(), []
+    mp.setenv("JF_GU_SPLITS", gate)
+    for stages in "01":
+        mp.setenv("JF_BY_STAGES", stages)
+        made.append(make_pair(name, max_rows=640, max_seqs=8, num_kv_pages=40, max_pages_per_seq=12))
+    mp.undo()
+    yield made[0][0].config, [rt for _, rt in made]
+    for _, rt in made:
+        rt.close()
+
+
+def tokens(n, seed, vocab):
+    return torch.randint(0, vocab, (n,), generator=torch.Generator().manual_seed(seed)).tolist()
+
+
+def cached(rt, n, vocab, seed=3):
+    """A sequence with n tokens in its pages."""
+    s = rt.new_sequence()
+    rt.ensure_capacity(s, n + 300)
+    toks = tokens(n, seed, vocab)
+    for a in range(0, n, 200):
+        part = toks[a:a + 200]
+        rt.forward(part, [(0, len(part), 0, a)], [s], 0, 0, [(i, 0, a + i) for i in range(len(part))])
+    s.ctx = n
+    return s
+
+
+def same(got):
+    a, b = got
+    assert a.keys() == b.keys()
+    for k in a:
+        if isinstance(a[k], np.ndarray):
+            assert a[k].tobytes() == b[k].tobytes(), k
+    return a
+
+
+@pytest.mark.parametrize("rows", [1, 7, 16, 17, 33, 64, 65, 120, 128, 129, 200, 255, 256, 257, 400, 513])
+@pytest.mark.parametrize("ctx", [0, 77])
+def test_rows(both, rows, ctx):
+    cfg, rts = both
+    got = []
+    for rt in rts:
+        s = cached(rt, ctx, cfg.vocab_size)
+        rt.ensure_capacity(s, ctx + rows)
+        row0 = (max(0, rows - 256) + 7) // 8 * 8
+        launches = rt.launches
+        out = rt.forward(tokens(rows, rows, cfg.vocab_size), [(0, rows, 0, ctx)], [s], row0, rows - row0, want_logits=True, want_hidden=True)
+        got.append({k: out[k] for k in ("logits", "hidden")})
+        got[-1]["greedy"] = np.asarray(out["greedy"])[row0:].copy()
+        assert (rt.launches - launches > 1) == (rt is rts[1])
+        rt.release(s)
+    out = same(got)
+    assert (out["logits"][np.arange(rows - row0), out["greedy"]] >= out["logits"].max(1) - 2.0 ** -7 * np.abs(out["logits"]).max(1)).all()      # the first of the largest bf16 values
+
+
+def test_groups(both):
+    """Forty groups of up to eleven rows over three contexts, then their rows in the pages and what follows them."""
+    cfg, rts = both
+    got = []
+    for rt in rts:
+        seqs = [cached(rt, n, cfg.vocab_size, 5 + n) for n in (70, 131, 255)]
+        groups, row = [], 0
+        for g in range(40):
+            n = 1 + g * 7 % 11
+            groups.append((row, n, g % 3, seqs[g % 3].ctx))
+            row += n
+        last = {g[2]: g for g in groups}
+        commits = [(g[0] + i, g[2], g[3] + i) for g in last.values() for i in range(g[1])]
+        for s in seqs:
+            rt.ensure_capacity(s, s.ctx + 40)
+        out = rt.forward(tokens(row, 8, cfg.vocab_size), groups, seqs, 0, row, commits, want_logits=True)
+        after = rt.forward(tokens(9, 9, cfg.vocab_size), [(0, 9, 1, seqs[1].ctx + last[1][1])], seqs, 0, 9, want_logits=True)
+        got.append({"logits": out["logits"], "greedy": np.asarray(out["greedy"])[:row].copy(), "after": after["logits"]})
+        for s in seqs:
+            rt.release(s)
+    same(got)
+
+
+@pytest.mark.parametrize("ctx", [1985, 2048, 2100])
+def test_more_chunks_than_lanes(both, ctx):
+    cfg, rts = both
+    got = []
+    for rt in rts:
+        s = cached(rt, ctx, cfg.vocab_size)
+        rt.ensure_capacity(s, ctx + 70)
+        got.append({"logits": rt.forward(tokens(66, 4, cfg.vocab_size), [(0, 66, 0, ctx)], [s], 0, 66, want_logits=True)["logits"]})
+        rt.release(s)
+    same(got)
+
+
+@pytest.mark.parametrize("batch,n,mode", [(1, 8, "single"), (1, 32, "multiblock"), (5, 16, "multiblock"), (8, 24, "single")])
+def test_jacobi_runs(both, batch, n, mode):
+    cfg, rts = both
+    got = []
+    for rt in rts:
+        prompts = [tokens(20 + 13 * i, 30 + i, cfg.vocab_size) for i in range(batch)]
+        seqs, results, run = hf_generate(rt, prompts, n=n, max_new_tokens=70, mode=mode, pad=0, K=2, r=0.85, n_gram_pool_size=4,
+                                         rngs=[random.Random(2 + i) for i in range(batch)])
+        after = rt.forward(tokens(9, 9, cfg.vocab_size), [(0, 9, 0, 20)], seqs[:1], 0, 9, want_logits=True)["logits"]
+        got.append({"after": after, "tokens": np.array([t for r in results for t in r.tokens]), "forwards": np.array([run["forwards"]])})
+        for s in seqs:
+            rt.release(s)
+    same(got)

@@ -144,3 +144,42 @@ def test_results_take_page_locked_memory_when_they_are_large(fake):
     assert fake.pinned() == [1]
     one.close()
     other.close()
+
+
+@pytest.mark.parametrize("what", ["launch", "commit"])
+def test_a_forward_by_stages_stops_at_the_first_launch_that_fails(fake, what, monkeypatch):
+    """An error, nothing launched behind it, and the engine works on: the next forward finds the argmax keys clean."""
+    monkeypatch.setenv("JF_BY_STAGES", "1")
+    rt = engine()
+    s = rt.new_sequence()
+    rt.ensure_capacity(s, 40)
+    commits = [(i, 0, i) for i in range(40)] if what == "commit" else []
+
+    def forward():
+        fake.reset()
+        return rt.forward([1] * 40, [(0, 40, 0, 0)], [s], 0, 40, commits)
+    forward()
+    names = [n for n, _ in fake.launches()]
+    assert len(names) == 1 + 2 * 9 + 2 + (what == "commit") and not any("persistent" in n for n in names) and all(fake.overlaps())
+    for at in range(len(names)):
+        fake.reset()
+        fake.fail(fake_cuda.LAUNCH, at)
+        with pytest.raises(RuntimeError, match="forward by stages: launch refused"):
+            rt.forward([1] * 40, [(0, 40, 0, 0)], [s], 0, 40, commits)
+        assert [n for n, _ in fake.launches()] == names[:at]
+    forward()
+    assert [n for n, _ in fake.launches()] == names
+    rt.release(s)
+    rt.close()
+
+
+def test_small_models_keep_the_persistent_kernel(fake):
+    """A forward of theirs is one launch; the line is a layer's weights."""
+    rt = engine()
+    s = rt.new_sequence()
+    rt.ensure_capacity(s, 40)
+    fake.reset()
+    rt.forward([1] * 40, [(0, 40, 0, 0)], [s], 0, 40)
+    assert ["persistent" in n for n, _ in fake.launches()] == [True]
+    rt.release(s)
+    rt.close()
