@@ -98,31 +98,6 @@ __device__ __forceinline__ unsigned long long step_max16(unsigned long long (&k)
   return got > k[0] ? got : k[0];
 }
 
-// up <- bf16(g / (1 + exp(-g))) * up of 16 rows, all of bf16 values, with the quotients that IEEE division gives.  The fast division is within
-// 2 ulp of it, so both round to the same bf16 unless its lower half lies within 4 of the middle between two; those, and divisors beyond its
-// range, are divided behind all others: a division's rare path is a branch, and sixteen of them in a row leave one row in
-// flight (gate/up of the 7B shape at 128 rows: 54.7 us, 45.6 so).
-__device__ __forceinline__ void step_swiglu16(const uint32_t (&gate)[16], const uint32_t (&up)[16], float (&o)[16]) {
-  uint32_t bad = 0u;
-#pragma unroll
-  for (int j = 0; j < 16; ++j) {
-    const float g = bf16_round(__uint_as_float(gate[j])), d = 1.f + __expf(-g);
-    o[j] = __fdividef(g, d);
-    const uint32_t off = (__float_as_uint(o[j]) & 0xffffu) - 0x7ffcu;
-    bad |= (off <= 8u || d > 1e36f) ? 1u << j : 0u;
-  }
-  if (bad) {
-#pragma unroll
-    for (int j = 0; j < 16; ++j)
-      if ((bad >> j) & 1u) {
-        const float g = bf16_round(__uint_as_float(gate[j]));
-        o[j] = g / (1.f + __expf(-g));
-      }
-  }
-#pragma unroll
-  for (int j = 0; j < 16; ++j) o[j] = bf16_round(o[j]) * bf16_round(__uint_as_float(up[j]));
-}
-
 template <int EPI>
 __global__ void __launch_bounds__(STEP_MAX_THREADS, 1) step_gemm_kernel(const __grid_constant__ StepGemm g, int* err) {
   extern __shared__ __align__(16) unsigned char step_smem[];
@@ -302,8 +277,10 @@ __global__ void __launch_bounds__(STEP_MAX_THREADS, 1) step_gemm_kernel(const __
         } else if (EPI == STEP_SWIGLU) {                       // rounding points: gemm_epilogue
           uint8_t* dst = reinterpret_cast<uint8_t*>(g.out) + ((size_t)(n >> 6) * g.out_rows_cap + r0) * 128 + (n & 7) * 2;      // r0: a multiple of 16
           const uint32_t chunk = (n & 63) >> 3;
-          float res[16];
-          step_swiglu16(v, up, res);
+          float gate[16], res[16];
+#pragma unroll
+          for (int j = 0; j < 16; ++j) { gate[j] = bf16_round(__uint_as_float(v[j])); res[j] = bf16_round(__uint_as_float(up[j])); }
+          swiglu_rows(gate, res);
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
             const __nv_bfloat16 o = __float2bfloat16_rn(res[j]);

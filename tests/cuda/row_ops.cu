@@ -4,6 +4,7 @@
 #include <type_traits>
 #include <vector>
 
+#include "jf_wide.cuh"
 #include "hy_gemm.cuh"
 #include "hy_few.cuh"
 
@@ -22,9 +23,30 @@ __global__ void exp_rates_kernel(const float* dt, const float* a, float* out, in
     out[i] = e.x; out[i + 1] = e.y;
   }
 }
+__global__ void sigmoid_kernel(const float* z, float* out, int n) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) out[i] = sigmoid_f(z[i]);
+}
+// bf16(g / (1 + exp(-g))) * u of eight rows at a time, by swiglu_rows or with IEEE division; n is a multiple of 8
+__global__ void swiglu_kernel(const float* gate, const float* up, float* out, int n, bool divide) {
+  for (int i = 8 * (blockIdx.x * blockDim.x + threadIdx.x); i < n; i += 8 * gridDim.x * blockDim.x) {
+    float g[8], u[8];
+    for (int j = 0; j < 8; ++j) { g[j] = gate[i + j]; u[j] = up[i + j]; }
+    if (divide) for (int j = 0; j < 8; ++j) u[j] *= jf::bf16_round(g[j] / (1.f + __expf(-g[j])));
+    else jf::swiglu_rows(g, u);
+    for (int j = 0; j < 8; ++j) out[i + j] = u[j];
+  }
+}
 }  // namespace
 
 extern "C" {
+int ops_sigmoid(const float* z, float* out, int n) {
+  sigmoid_kernel<<<148, 256>>>(z, out, n);
+  return done();
+}
+int ops_swiglu(const float* gate, const float* up, float* out, int n, int divide) {
+  swiglu_kernel<<<148, 128>>>(gate, up, out, n, divide != 0);
+  return done();
+}
 int ops_exp_rates(const float* dt, const float* a, float* out, int n) {
   exp_rates_kernel<<<148, 128>>>(dt, a, out, n);
   return done();

@@ -47,6 +47,19 @@ class RowOps:
         self._ok(self.lib.ops_exp_rates(_at(dt), _at(a), _at(out), dt.numel()))
         return out
 
+    def sigmoid(self, z):
+        out = torch.empty_like(z)
+        torch.cuda.synchronize()
+        self._ok(self.lib.ops_sigmoid(_at(z), _at(out), z.numel()))
+        return out
+
+    def swiglu(self, gate, up, divide):
+        """bf16(g / (1 + exp(-g))) * u of fp32 vectors of bf16 values, a multiple of eight long; divide: with IEEE division."""
+        out = torch.empty_like(up)
+        torch.cuda.synchronize()
+        self._ok(self.lib.ops_swiglu(_at(gate), _at(up), _at(out), gate.numel(), int(divide)))
+        return out
+
     def few(self, a, w, kernel="few", out=None, wait=True):
         """a [T, K] w [N, K]^T in bf16 -> fp32, by the kernel of few rows ("few") or the one beside it ("rows")."""
         t, k = a.shape
