@@ -112,6 +112,7 @@ struct UnitList { int kind, H, G, a, b; AttnUnit* d; int n, split, ns; };
 
 using namespace hy;
 
+constexpr size_t HY_SMALL_RESULT = 64 << 10;                 // bytes of logits up to which the caller's array is pageable (hostmem.py)
 struct hy_engine {
   hy_model_cfg m{};
   hy_runtime_cfg rt{};
@@ -134,6 +135,7 @@ struct hy_engine {
   void* x_rows = nullptr;                        // activation rows in the expert-sorted order
   int x_max_tiles = 0, x_max_experts = 0, x_set = 0;
   int* err_d = nullptr; int* err_h = nullptr;
+  unsigned char* out_h = nullptr;    // page-locked: a step's sampled tokens and small results on their way to the caller's arrays
   // per-category device times (hy_profile_enable): event pairs recorded around groups of launches
   bool prof_on = false;
   float prof_ms[HY_PROFILE_CATEGORIES] = {};
@@ -440,6 +442,7 @@ extern "C" void hy_destroy(hy_handle h) {
   if (h->units_h) cudaFreeHost(h->units_h);
   if (h->fl_h) cudaFreeHost(h->fl_h);
   if (h->err_h) cudaFreeHost(h->err_h);
+  if (h->out_h) cudaFreeHost(h->out_h);
   cudaEventDestroy(h->ev0);
   cudaEventDestroy(h->ev1);
   cudaStreamDestroy(h->stream);
@@ -1585,6 +1588,7 @@ extern "C" int hy_finalize(hy_handle h) {
   if (dev_alloc(h, (void**)&h->err_d, 4, &h->bytes_ws)) return HY_ERR_CUDA;
   HY_CUDA(cudaMemset(h->err_d, 0, 4));
   HY_CUDA(cudaMallocHost((void**)&h->err_h, 4));
+  HY_CUDA(cudaMallocHost((void**)&h->out_h, (size_t)h->rt.max_want * 4 + HY_SMALL_RESULT));
   *h->err_h = 0;
   {
     size_t states = 0, ends = 0;                              // floats per chunk of the largest layer
@@ -3333,11 +3337,14 @@ extern "C" int hy_step(hy_handle h, int32_t n_entries, const int32_t* tokens, co
     }
     go_kernel(h, sample_kernel, n_want, 1024, 0, h->stream, h->logits, h->m.vocab, td, seed, h->sampled);
     h->launches++;
-    keep(cudaMemcpyAsync(sampled_out, h->sampled, (size_t)n_want * 4, cudaMemcpyDeviceToHost, h->stream));
+    keep(cudaMemcpyAsync(h->out_h + HY_SMALL_RESULT, h->sampled, (size_t)n_want * 4, cudaMemcpyDeviceToHost, h->stream));
   }
   keep(cudaEventRecord(h->ev1, h->stream));
-  if (n_want > 0 && logits_out)
-    keep(cudaMemcpyAsync(logits_out, h->logits, (size_t)n_want * h->m.vocab * 4, cudaMemcpyDeviceToHost, h->stream));
+  // Tokens and small logits come by way of page-locked memory: the caller's arrays for them are pageable, and a copy into those waits for the
+  // step before the next copy is made (10 us each).
+  const size_t logit_bytes = (size_t)n_want * h->m.vocab * 4;
+  const bool small = logit_bytes <= HY_SMALL_RESULT;
+  if (n_want > 0 && logits_out) keep(cudaMemcpyAsync(small ? (void*)h->out_h : (void*)logits_out, h->logits, logit_bytes, cudaMemcpyDeviceToHost, h->stream));
   keep(cudaMemcpyAsync(h->err_h, h->err_d, 4, cudaMemcpyDeviceToHost, h->stream));
   keep(cudaStreamSynchronize(h->stream));
   keep(cudaGetLastError());
@@ -3351,6 +3358,8 @@ extern "C" int hy_step(hy_handle h, int32_t n_entries, const int32_t* tokens, co
     h->prof_list.clear();
     return fail(h, HY_ERR_CUDA, h->step_err);
   }
+  if (n_want > 0 && sampled_out) memcpy(sampled_out, h->out_h + HY_SMALL_RESULT, (size_t)n_want * 4);
+  if (n_want > 0 && logits_out && small) memcpy(logits_out, h->out_h, logit_bytes);
   cudaEventElapsedTime(&h->last_ms, h->ev0, h->ev1);
   for (auto& r : h->prof_list) {
     float ms = 0.0f;

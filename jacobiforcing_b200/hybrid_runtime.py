@@ -21,22 +21,27 @@ def _i32(x) -> np.ndarray:
     return np.ascontiguousarray(np.asarray(x, dtype=np.int32))
 
 
-def _packed(parts) -> Tuple[np.ndarray, List[int]]:
-    """Token lists end to end as int32, and where each begins (the last: their length).  array.array converts and range-checks Python integers in native code (2048 of them: 34 us, a
+def _add(out: array.array, values) -> None:
+    """Integers to the end of an int32 array.  array.array converts and range-checks Python integers in native code (2048 of them: 34 us, a
     generator and numpy 161 us, a tenth of a prompt step); whatever has no integer form of its own goes through int()."""
+    t = values.tolist() if isinstance(values, np.ndarray) and values.ndim == 1 else values if isinstance(values, (list, tuple)) else list(values)
+    try:
+        out.extend(array.array("i", t))
+    except TypeError:
+        out.extend(int(x) for x in t)
+
+
+def _packed(parts) -> Tuple[np.ndarray, List[int]]:
+    """Token lists end to end as int32, and where each begins (the last: their length)."""
     out, start = array.array("i"), [0]
     for t in parts:
-        t = t.tolist() if isinstance(t, np.ndarray) and t.ndim == 1 else t if isinstance(t, (list, tuple)) else list(t)
-        try:
-            out.extend(array.array("i", t))
-        except TypeError:
-            out.extend(int(x) for x in t)
+        _add(out, t)
         start.append(len(out))
     return np.array(out, dtype=np.int32), start
 
 
 def _ptr(a: Optional[np.ndarray]):
-    return None if a is None else a.ctypes.data_as(C.c_void_p)
+    return None if a is None else a.ctypes.data
 
 
 class HybridRuntime:
@@ -53,6 +58,7 @@ class HybridRuntime:
         self.max_step_tokens, self.max_step_entries = max_step_tokens, max_step_entries
         self.max_pages_per_seq = max_pages_per_seq
         self.max_want = max_want or max_step_tokens
+        self._no_pages = array.array("i", [0] * max_pages_per_seq)
         m = cabi.ModelCfg(config.width, config.vocab, len(config.layers), DTYPES[dtype], config.emb_scale,
                           config.logit_scale, config.norm_eps, config.norm_kind, config.block_kind, config.pos_kind,
                           int(config.embed_norm), int(config.tied_head), config.resid_mult, config.canon_taps,
@@ -131,25 +137,29 @@ class HybridRuntime:
              seed: int = 0, want_layers: bool = False):
         """entries: (tokens, pos0, slot, pages) per request; want: indices into the packed token list.
         Returns {"logits": [n_want, vocab] float32 or None, "sampled": int32 [n_want] or None, "layers": ...}."""
-        E = len(entries)
+        E, width = len(entries), self.max_pages_per_seq
         a_tok, start = _packed([e[0] for e in entries])
-        pages = np.zeros((E, self.max_pages_per_seq), dtype=np.int32)
-        for e, (_, _, _, pg) in enumerate(entries):
-            if len(pg) > self.max_pages_per_seq:
+        T, n_want = len(a_tok), len(want)
+        # where each entry's tokens begin, positions, slots, pages, wanted rows: one array, whose address is asked for once
+        a = array.array("i", start)
+        _add(a, [e[1] for e in entries])
+        _add(a, [e[2] for e in entries])
+        for _, _, _, pg in entries:
+            if len(pg) > width:
                 raise RuntimeError("request holds more pages than max_pages_per_seq")
-            pages[e, :len(pg)] = pg
-        T = len(a_tok)
-        n_want = len(want)
+            _add(a, pg)
+            a.extend(self._no_pages[len(pg):])
+        if n_want:
+            _add(a, want)
         logits = self._results.empty((n_want, self.vocab)) if (n_want and want_logits) else None
         sampled = np.empty((n_want,), dtype=np.int32) if (n_want and sample) else None
         temp = np.ascontiguousarray(np.asarray(temperature, dtype=np.float32)) if (temperature is not None and n_want) else None
         layers = np.empty((len(self.config.layer_runs()), T, self.width), dtype=np.float32) if want_layers else None
-        a_start = _i32(start)
-        a_pos0, a_slot = _i32([e[1] for e in entries]), _i32([e[2] for e in entries])
-        a_want = _i32(list(want)) if n_want else None
-        cabi.check(self.lib.hy_step(self.h, E, _ptr(a_tok), _ptr(a_start), _ptr(a_pos0), _ptr(a_slot), _ptr(pages), n_want,
-                                    _ptr(a_want), _ptr(logits), _ptr(sampled), _ptr(temp), C.c_uint64(seed & (2 ** 64 - 1)),
-                                    _ptr(layers)), self.h)
+        at = a.buffer_info()[0]
+        pos0 = at + 4 * (E + 1)
+        pages = pos0 + 8 * E
+        cabi.check(self.lib.hy_step(self.h, E, _ptr(a_tok), at, pos0, pos0 + 4 * E, pages, n_want, pages + 4 * E * width if n_want else None,
+                                    _ptr(logits), _ptr(sampled), _ptr(temp), seed & (2 ** 64 - 1), _ptr(layers)), self.h)
         self.stats["steps"] += 1
         self.stats["tokens"] += T
         self.stats["device_ms"] += float(self.lib.hy_last_step_ms(self.h))
