@@ -767,8 +767,8 @@ __device__ __noinline__ void qkv_rope_tail(const DevCtx& c, const WorkerShared* 
 // Chunks are aligned to ABSOLUTE key positions, so a query's result does not depend on how its keys are split between
 // committed pages and in-flight scratch rows (AR decoding and Jacobi decoding of the same prefix agree bit for bit).
 // ---------------------------------------------------------------------------------------------------------------
-// ONE_ROUND: no more 16-row tiles than warps
-template <int D, bool ONE_ROUND = false, class C, class W>
+// ONE_ROUND: no more 16-row tiles than warps; ONE_SUB: chunks of one sub-tile
+template <int D, bool ONE_ROUND = false, bool ONE_SUB = false, class C, class W>
 __device__ __forceinline__ void attention_unit(const C& c, const W& w, int layer, const Group& grp, int g_kvh, int chunk,
                                int qs, int hs, bool prefetched, int hsplit) {
   constexpr int LDS = D + 8;                  // padded smem row (bf16 elements) -> conflict-free fragment loads
@@ -787,7 +787,7 @@ __device__ __forceinline__ void attention_unit(const C& c, const W& w, int layer
   const int hp = (md.n_rep + hsplit - 1) / hsplit;      // q heads of this kv head handled by one unit
   const int j_lo = hs * hp, j_hi = min(md.n_rep, j_lo + hp);
   const int tiles = max(0, j_hi - j_lo) * ntt;
-  const int nsub = (key_hi - key_lo + kAttnSub - 1) / kAttnSub;
+  const int nsub = ONE_SUB ? 1 : (key_hi - key_lo + kAttnSub - 1) / kAttnSub;
   const int* bt = c.block_tables + (size_t)grp.seq * c.max_pages_per_seq;
   const float scale = rsqrtf((float)D);
   const int r0 = w.lane() >> 2, c2 = (w.lane() & 3) * 2;

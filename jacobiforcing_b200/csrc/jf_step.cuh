@@ -471,7 +471,9 @@ __global__ void __launch_bounds__(256) step_rope_kernel(const StepRope a) {
 }
 
 // ---- attention -----------------------------------------------------------------------------------------------------------------------
-// The persistent kernel's unit (attention_unit) and merge (attn_combine_impl), one unit per block of four warps.
+// The persistent kernel's unit (attention_unit) and merge (attn_combine_impl), one unit per block of four warps.  ONE_SUB: chunks of 64 keys, whose
+// output starts at zero instead of being scaled: three blocks per SM without spills.  Eight sequences of the 7B shape (200 rows, 768 units) 15.9 -> 13.2 us
+// against the general form; four blocks per SM (128 registers) 13.7, five (96) 14.0: bound by mma.sync and the fragments' loads, not by latency.
 struct StepCtx {
   ModelDims md;
   int attn_chunk, max_pages_per_seq, num_pages, T_cap, xrows_cap;
@@ -492,8 +494,8 @@ struct StepWorker {
 };
 __device__ __forceinline__ void prof_mark(const StepCtx&, const StepWorker&, int) {}
 
-template <int D>
-__global__ void __launch_bounds__(128, D == 128 ? 3 : 4) step_attention_kernel(const __grid_constant__ StepCtx c, const Group* __restrict__ groups, int G, int layer, int plan_hs, int hs) {
+template <int D, bool ONE_SUB>
+__global__ void __launch_bounds__(128, 3) step_attention_kernel(const __grid_constant__ StepCtx c, const Group* __restrict__ groups, int G, int layer, int plan_hs, int hs) {
   extern __shared__ __align__(16) uint8_t step_attn_smem[];
   pdl_trigger();
   const StepWorker w{step_attn_smem};
@@ -528,7 +530,7 @@ __global__ void __launch_bounds__(128, D == 128 ? 3 : 4) step_attention_kernel(c
     cp_async_commit();
   }
   pdl_wait();
-  attention_unit<D, true>(c, w, layer, grp, kvh, chunk, local / grp.nchunks, h, true, hs);
+  attention_unit<D, true, ONE_SUB>(c, w, layer, grp, kvh, chunk, local / grp.nchunks, h, true, hs);
 }
 
 // attn_combine's merge of up to 32 chunks with a row's statistics and first eight chunks in flight at once, one (row, head) per warp.
@@ -719,8 +721,9 @@ inline void step_forward(WideStream& w, const DevCtx& c, const StepPlan& p, int 
                      c.kv_scratch + kv_scratch_offset(md, c.T_cap, l, 0, 0, 0), c.kv_scratch + kv_scratch_offset(md, c.T_cap, l, 1, 0, 0),
                      T, md.n_q, md.n_kv, md.d, md.max_pos};
     if (md.d == 128) step_rope<2>(w, r, c.splits_qkv); else step_rope<1>(w, r, c.splits_qkv);
-    if (md.d == 128) w.launch(step_attention_kernel<128>, units, 128, attn_smem, sc, c.groups, p.G, l, p.hsplit, hs);
-    else w.launch(step_attention_kernel<64>, units, 128, attn_smem, sc, c.groups, p.G, l, p.hsplit, hs);
+    auto attention = [&](auto kernel) { w.launch(kernel, units, 128, attn_smem, sc, c.groups, p.G, l, p.hsplit, hs); };
+    if (md.d == 128) { if (c.attn_chunk == kAttnSub) attention(step_attention_kernel<128, true>); else attention(step_attention_kernel<128, false>); }
+    else { if (c.attn_chunk == kAttnSub) attention(step_attention_kernel<64, true>); else attention(step_attention_kernel<64, false>); }
     if (md.d == 128) w.launch(step_combine_kernel<4>, combine, 256, 0, sc, T); else w.launch(step_combine_kernel<2>, combine, 256, 0, sc, T);
     partial(L.wo, c.xa, c.part_rs[0], nt_h, kc_q, c.splits_o, md.h);
     step_norm(w, c, T, c.splits_o, c.part_rs[0], L.ln2);
