@@ -1564,7 +1564,8 @@ extern "C" int hy_finalize(hy_handle h) {
       if (c.ff_kind == HY_FF_ROUTED) { maxE = std::max(maxE, c.x_experts); maxTop = std::max(maxTop, c.x_top); }
     if (maxE > 0) {
       const size_t P = T * (size_t)maxTop;
-      h->x_max_tiles = (int)(P / HY_XT) + maxE + 1;          // enough for tiles of HY_XT rows and of 128 rows
+      // enough for tiles of HY_XT rows and of 128 rows, and of 32 where few pairs take those (simt_tile_rows)
+      h->x_max_tiles = (int)std::max((size_t)P / HY_XT, std::min((size_t)P, (size_t)24 * maxE) / 32) + maxE + 1;
       if (dev_alloc(h, (void**)&h->x_ids, P * 4, &h->bytes_ws)) return HY_ERR_CUDA;
       if (dev_alloc(h, (void**)&h->x_wts, P * 4, &h->bytes_ws)) return HY_ERR_CUDA;
       if (dev_alloc(h, &h->x_rows, P * W * es, &h->bytes_ws)) return HY_ERR_CUDA;
@@ -2249,13 +2250,23 @@ int* next_counts(hy_engine* h) { h->x_set ^= 1; return h->x_counts + (size_t)h->
 // step, 32 experts, us with 128 -> 256: 128 rows per expert, width 1024 53.9 -> 61.0 and (larger experts) 72.8 -> 71.3; 160 rows 73.1 -> 61.5 and 85.5 ->
 // 77.2, width 2048 186 -> 146; 256 rows 74.7 -> 65.6, 99.6 -> 95.3, 231 -> 190.
 int expert_tile_rows(int P, int NE) { return P >= 144 * NE ? 256 : 128; }
+// A product of the sorted rows on the fp32 units, in the tiles that route_place_kernel listed.
+template <typename TA, typename TO, bool GLU>
+void simt_experts(hy_engine* h, int P, int NE, const TA* A, int lda, const void* W, size_t stride, int N, int K, TO* out, int ldo, int act, float limit) {
+  auto go = [&](auto rows) {
+    constexpr int BM = decltype(rows)::value;
+    go_kernel(h, expert_gemm_simt_kernel<TA, TA, TO, GLU, BM>, dim3((N + 31) / 32, std::min(h->x_max_tiles, P / BM + NE + 1)), 256, 0, h->stream, A, lda, (const TA*)W, stride, N, K,
+              h->x_offs, h->x_tile_e, h->x_tile_r0, h->x_meta, out, ldo, act, limit);
+  };
+  if (simt_tile_rows(P, NE) == 32) go(std::integral_constant<int, 32>{}); else go(std::integral_constant<int, HY_XT>{});
+}
 template <typename AT>
 void place_rows(hy_engine* h, int T, const AT* hb, const LayerW& L, const hy_layer_cfg& c, AT* rows) {
   const int P = T * c.x_top, W = h->m.width, E = h->x_max_experts;
   const bool tc = std::is_same<AT, bf16>::value && L.w_gu_t != nullptr;
   int* now = h->x_counts + (size_t)h->x_set * 2 * E;
   int* old = h->x_counts + (size_t)(h->x_set ^ 1) * 2 * E;
-  go_kernel(h, route_place_kernel<AT>, P + 1, 128, 0, h->stream, P, c.x_top, c.x_experts, E, tc ? expert_tile_rows(P, c.x_experts) : HY_XT, h->x_ids, now, now + E,
+  go_kernel(h, route_place_kernel<AT>, P + 1, 128, 0, h->stream, P, c.x_top, c.x_experts, E, tc ? expert_tile_rows(P, c.x_experts) : simt_tile_rows(P, c.x_experts), h->x_ids, now, now + E,
                                                        old, old + E, hb, W, W % (16 / (int)sizeof(AT)) == 0, h->x_offs, h->x_tile_e, h->x_tile_r0,
                                                        h->x_meta, h->x_pair_row, rows);
   h->launches++;
@@ -2421,11 +2432,8 @@ int sandwich_layer(hy_engine* h, const Batch& b, size_t li) {
         pair_product<float>(h, pin, ldh, P, L.w_down_t, NE, L.down_t_stride, P, W, ff, o2, expert_tile_rows(P, NE), grp);
       }
     } else {
-      const int tiles = std::min(h->x_max_tiles, P / HY_XT + NE + 1);
-      go_kernel(h, expert_gemm_simt_kernel<AT, WT, AT, true>, dim3((ff + 31) / 32, tiles), 256, 0, s, 
-          x_rows, W, (const WT*)L.w_gu, (size_t)2 * ff * W, ff, W, h->x_offs, h->x_tile_e, h->x_tile_r0, h->x_meta, pin, ldh, 0, 0.0f);
-      go_kernel(h, expert_gemm_simt_kernel<AT, WT, float, false>, dim3((W + 31) / 32, tiles), 256, 0, s, 
-          pin, ldh, (const WT*)L.w_down, (size_t)W * ff, W, ff, h->x_offs, h->x_tile_e, h->x_tile_r0, h->x_meta, ys, W, -1, 0.0f);
+      simt_experts<AT, AT, true>(h, P, NE, x_rows, W, L.w_gu, (size_t)2 * ff * W, ff, W, pin, ldh, 0, 0.0f);
+      simt_experts<AT, float, false>(h, P, NE, pin, ldh, L.w_down, (size_t)W * ff, W, ff, ys, W, -1, 0.0f);
     }
     const auto combine = [&](auto v) {
       go_kernel(h, expert_combine_kernel<AT, decltype(v)::value>, T, 256, 0, s, ys, W, few ? nullptr : h->x_pair_row, h->x_wts, top, W, L.n2b, L.ls2, h->x, after_ff, hb);
@@ -2609,11 +2617,8 @@ int postnorm_layer(hy_engine* h, const Batch& b, size_t li) {
         pair_product<float>(h, pin, ldh, P, L.w_down_t, NE, L.down_t_stride, P, W, ff, o2, expert_tile_rows(P, NE), grp);
       }
     } else {
-      const int tiles = std::min(h->x_max_tiles, P / HY_XT + NE + 1);
-      go_kernel(h, expert_gemm_simt_kernel<AT, WT, AT, false>, dim3((ff + 31) / 32, tiles), 256, 0, s, 
-          x_rows, W, (const WT*)L.w_gu, (size_t)ff * W, ff, W, h->x_offs, h->x_tile_e, h->x_tile_r0, h->x_meta, pin, ldh, c.x_act, c.ff_limit);
-      go_kernel(h, expert_gemm_simt_kernel<AT, WT, float, false>, dim3((W + 31) / 32, tiles), 256, 0, s, 
-          pin, ldh, (const WT*)L.w_down, (size_t)W * ff, W, ff, h->x_offs, h->x_tile_e, h->x_tile_r0, h->x_meta, ys, W, -1, 0.0f);
+      simt_experts<AT, AT, false>(h, P, NE, x_rows, W, L.w_gu, (size_t)ff * W, ff, W, pin, ldh, c.x_act, c.ff_limit);
+      simt_experts<AT, float, false>(h, P, NE, pin, ldh, L.w_down, (size_t)W * ff, W, ff, ys, W, -1, 0.0f);
     }
     h->launches += 2;
     if (c.x_shared_ff > 0) {
@@ -2673,11 +2678,8 @@ bool routed_gated_experts(hy_engine* h, int T, const AT* hb, const LayerW& L, co
       pair_product<float>(h, pin, ldh, P, L.w_down_t, NE, L.down_t_stride, P, W, ff, o2, expert_tile_rows(P, NE), grp);
     }
   } else {
-    const int tiles = std::min(h->x_max_tiles, P / HY_XT + NE + 1);
-    go_kernel(h, expert_gemm_simt_kernel<AT, WT, AT, true>, dim3((ff + 31) / 32, tiles), 256, 0, s, 
-        x_rows, W, (const WT*)L.w_gu, (size_t)2 * ff * W, ff, W, h->x_offs, h->x_tile_e, h->x_tile_r0, h->x_meta, pin, ldh, c.x_act, c.ff_limit);
-    go_kernel(h, expert_gemm_simt_kernel<AT, WT, float, false>, dim3((W + 31) / 32, tiles), 256, 0, s, 
-        pin, ldh, (const WT*)L.w_down, (size_t)W * ff, W, ff, h->x_offs, h->x_tile_e, h->x_tile_r0, h->x_meta, ys, W, -1, 0.0f);
+    simt_experts<AT, AT, true>(h, P, NE, x_rows, W, L.w_gu, (size_t)2 * ff * W, ff, W, pin, ldh, c.x_act, c.ff_limit);
+    simt_experts<AT, float, false>(h, P, NE, pin, ldh, L.w_down, (size_t)W * ff, W, ff, ys, W, -1, 0.0f);
   }
   h->launches += 2;
   return few;

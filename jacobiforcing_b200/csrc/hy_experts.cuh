@@ -178,6 +178,10 @@ __global__ void gated_act_kernel(const AT* __restrict__ in, int ldi, int n, int 
 // at a time.  Offsets by one thread, the order, and rows fetched through it inside the products took 7 + 4 us and held the products
 // back; this takes 11 us for 2048 tokens x 4 choices of 1024 channels.
 constexpr int HY_XT = 64;
+// Rows of a tile of expert_gemm_simt_kernel: most of a tile of 64 is padding where an expert has a handful of rows.  32 experts with ten rows each, width
+// 256, of 128 (gate and up) and back: 33.6 and 9.8 us with 64 rows, 12.6 and 6.1 with 32.  A step of two layers, rows an expert, us with 64 -> 32: 10 218 -> 205,
+// 16 233 -> 222, 24 264 -> 247, 31 282 -> 296, 50 314 -> 329.
+inline int simt_tile_rows(int pairs, int experts) { return pairs <= 24 * experts ? 32 : HY_XT; }
 template <typename AT>
 __global__ void __launch_bounds__(128) route_place_kernel(int pairs, int top, int experts, int most_experts, int tile_rows,
                                                           const int* __restrict__ ids, const int* __restrict__ counts, int* __restrict__ fill,
@@ -235,14 +239,14 @@ __global__ void __launch_bounds__(128) route_place_kernel(int pairs, int top, in
 // the activation when act >= 0 (act: 0 silu, 1 tanh-gelu, 2 erf-gelu; see act_f).  Tiled SIMT, fp32 FMAs in k order: both builds can use it.
 // Bound by the chain of its k blocks (few rows per expert): the next block travels while this one is summed up, and 32 columns per block give
 // twice the blocks of 64; two layers of 77 tokens x 2 experts, width 256: 134 -> 44 us.
-template <typename TA, typename TW, typename TO, bool GLU>
+template <typename TA, typename TW, typename TO, bool GLU, int BM>
 __global__ void __launch_bounds__(256) expert_gemm_simt_kernel(const TA* __restrict__ A, int lda,
                                                                const TW* __restrict__ W, size_t w_stride, int N, int K,
                                                                const int* __restrict__ offs, const int* __restrict__ tile_expert,
                                                                const int* __restrict__ tile_row0, const int* __restrict__ meta,
                                                                TO* __restrict__ out, int ldo, int act, float limit) {
   pdl_begin();
-  constexpr int BM = HY_XT, BN = 32, R = BM / 16, C = BN / 16, NA = BM * SIMT_BK / 1024;
+  constexpr int BN = 32, R = BM / 16, C = BN / 16, NA = BM * SIMT_BK / 1024;
   static_assert(BM % 32 == 0 && (R == 2 || R == 4), "a thread's rows are one read of two or four");
   __shared__ __align__(16) float As[2][SIMT_BK][BM];
   __shared__ __align__(16) float Ws[2][GLU ? 2 : 1][SIMT_BK][BN];

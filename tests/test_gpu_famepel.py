@@ -41,6 +41,17 @@ def test_router_shapes(kw, dtype):
     assert close(got, want, dtype)
 
 
+@pytest.mark.parametrize("tokens", [47, 48, 49, 96, 97])
+@pytest.mark.parametrize("experts", [4, 8])
+def test_expert_tiles_of_32_and_64_rows(tokens, experts):
+    """Two choices of a token, so 24 pairs an expert, where tiles of the fp32 products change, are 48 tokens of four experts and 96 of eight; experts with
+    more and fewer rows than a tile on both sides."""
+    kw = dict(experts=experts, top=2, count=2, keep=2)
+    cfg = model_config([glr(heads=1, dim=4, vdim=4, mlp=moe(**kw)), ssd(heads=2, vdim=4, state=3, groups=1, norm_groups=1, mlp=moe(ff=70, **kw))])
+    got, want = run(cfg, rand_tokens(tokens, cfg["vocab"], 4), "float32", max_step_tokens=128)
+    assert close(got, want, "float32")
+
+
 # ---- prefill == decode, portions -------------------------------------------------------------------------------------------
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_prefill_equals_token_by_token(dtype):
