@@ -209,7 +209,7 @@ __global__ void __launch_bounds__(128) delta_head_kernel(Batch b, const float* _
                                                          const float4* __restrict__ scal, int H, int G, int dim, int vdim,
                                                          int blocks_per_head, int vec, int vvec, float* __restrict__ state,
                                                          float* __restrict__ o, int ldo, const float* __restrict__ dec, int ldd) {
-  pdl_begin();
+  pdl_trigger();
   constexpr int TB = lin_tb(DR), RP = DR / PARTS, CW = 32 / PARTS, CPB = lin_cpb(PARTS, VC), VW = CPB < 8 ? 8 : CPB;
   constexpr int RW = CHAN ? 3 * DR : 2 * DR;                   // floats of a staged row: q | k (| decays)
   extern __shared__ __align__(16) unsigned char hy_smem[];
@@ -232,6 +232,7 @@ __global__ void __launch_bounds__(128) delta_head_kernel(Batch b, const float* _
       S[c][i / 2] = make_float2((col + c < vdim && r < dim && pos0 > 0) ? st[(size_t)r * vdim + col + c] : 0.0f,
                                 (col + c < vdim && r + 1 < dim && pos0 > 0) ? st[(size_t)(r + 1) * vdim + col + c] : 0.0f);
   }
+  pdl_wait();
   if (dim < DR)                                                // rows beyond the head's key size stay zero
     for (int i = tid; i < 2 * TB * RW; i += 128) if (i % DR >= dim) sqk[i] = 0.0f;
   auto fetch = [&](int j0, int buf) {

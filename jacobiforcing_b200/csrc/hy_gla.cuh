@@ -37,7 +37,7 @@ __global__ void __launch_bounds__(128) gla_kernel(Batch b, const float* __restri
                                                   const float* __restrict__ decay, int ldd, const float* __restrict__ head_decay, int H,
                                                   int dim, int vdim, int blocks_per_head, int vec, int vvec, float* __restrict__ state,
                                                   float* __restrict__ o, int ldo, GlaToken tk) {
-  pdl_begin();
+  pdl_trigger();
   constexpr int TB = lin_tb(DR), RP = DR / PARTS, CW = 32 / PARTS, CPB = lin_cpb(PARTS, VC), VW = CPB < 8 ? 8 : CPB;
   constexpr bool HEAD = MODE == GLA_HEAD;
   constexpr int RW = MODE == GLA_CHANNEL ? 3 * DR : 2 * DR;    // floats of a staged row: q | k (| decays)
@@ -64,6 +64,7 @@ __global__ void __launch_bounds__(128) gla_kernel(Batch b, const float* __restri
   const int rows_per_token = MODE == GLA_TOKEN ? tk.G : H, row_of = MODE == GLA_TOKEN ? h / (H / tk.G) : h;
   const float rate = MODE == GLA_TOKEN ? expf(tk.A_log[h]) : 0.0f, dt_bias = MODE == GLA_TOKEN ? tk.dt_bias[h] : 0.0f;
   const float skip = MODE == GLA_TOKEN ? tk.D[h] : 0.0f;
+  pdl_wait();
   float raw = 0.0f;                                            // raw step size of token tid of the batch in flight
   if (dim < DR)                                                // rows beyond the head's key size stay zero
     for (int i = tid; i < 2 * TB * RW; i += 128) if (i % DR >= dim) sqk[i] = 0.0f;

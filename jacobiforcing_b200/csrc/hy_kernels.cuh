@@ -23,6 +23,8 @@ typedef __nv_bfloat16 bf16;
 using jf::pdl_trigger;
 using jf::pdl_wait;
 __device__ __forceinline__ void pdl_begin() { pdl_trigger(); pdl_wait(); }
+// Ahead of pdl_wait a kernel of a step may read weights, the step's batch (its copy is over before the step's first kernel begins) and what a recurrence or
+// convolution keeps of a request between steps: of a layer's run that is read and written by one kernel of a step, where launches overlap.
 
 template <typename T> __device__ __forceinline__ float to_f(T v);
 template <> __device__ __forceinline__ float to_f<float>(float v) { return v; }
@@ -524,7 +526,7 @@ constexpr int HY_CONV_TT = 16;                                 // tokens per thr
 template <typename AT, typename WT, int V, int TAPS>
 __global__ void __launch_bounds__(128) conv_kernel(Batch b, const AT* __restrict__ u, int ldu, int col0, int C, int taps_, const WT* __restrict__ w,
                                                    const WT* __restrict__ bias, int act_silu, float* __restrict__ state, ConvOut<AT> o) {
-  pdl_begin();
+  pdl_trigger();
   const int taps = TAPS ? TAPS : taps_;
   int e = 0, chunk = blockIdx.y, start, cnt;
   for (;; ++e) {                                               // entry and chunk of this block
@@ -544,14 +546,23 @@ __global__ void __launch_bounds__(128) conv_kernel(Batch b, const AT* __restrict
   };
   constexpr int NW = TAPS > 1 ? TAPS - 1 : 1;
   float win[NW][V], wv[V][TAPS ? TAPS : 1], bv[V];
+  auto window = [&] {
+#pragma unroll
+    for (int k = 0; k < V; ++k)
+#pragma unroll
+      for (int i = 0; i < TAPS - 1; ++i) win[i][k] = input(j0 - (TAPS - 1) + i, k);
+  };
+  // The entry, weights and an entry's first window come while the kernel before this one ends, as the states of recurrences do: a request of 24 tokens, one
+  // each step, 7847 -> 7665 us, eight requests 8800 -> 8716.
 #pragma unroll
   for (int k = 0; k < V; ++k) {
     bv[k] = bias ? to_f(bias[c + k]) : 0.0f;
 #pragma unroll
     for (int i = 0; i < TAPS; ++i) wv[k][i] = to_f(w[(size_t)(c + k) * TAPS + i]);
-#pragma unroll
-    for (int i = 0; i < TAPS - 1; ++i) win[i][k] = input(j0 - (TAPS - 1) + i, k);
   }
+  if (j0 == 0) window();
+  pdl_wait();
+  if (j0 > 0) window();
 #pragma unroll 4
   for (int j = j0; j < j1; ++j) {
     const int t = start + j;
@@ -756,7 +767,8 @@ __global__ void __launch_bounds__(128) scan_kernel(Batch b, const AT* __restrict
                                                    const float* __restrict__ low, int ldl, int col_b, int col_c,
                                                    const float* __restrict__ A, const WT* __restrict__ D, int inner, int nstate,
                                                    int vec, float out_scale, float* __restrict__ state, AT* __restrict__ out, int ldo, ScanSegments seg) {
-  pdl_begin();
+  pdl_trigger();
+  if (PASS != SCAN_WHOLE) pdl_wait();
   constexpr int NP = NPER * L, PB = 128 / L, TB = scan_tb(NP), TG = 8, CH = 16 / (int)sizeof(AT);
   extern __shared__ __align__(16) unsigned char hy_smem[];
   float* sB = reinterpret_cast<float*>(hy_smem);               // [2][TB][NP]
@@ -794,6 +806,7 @@ __global__ void __launch_bounds__(128) scan_kernel(Batch b, const AT* __restrict
     const float* row = A + (size_t)cc * nstate;
     a[i / 2] = RatePair(n0 + i < nstate ? row[n0 + i] : 0.0f, n0 + i + 1 < nstate ? row[n0 + i + 1] : 0.0f);
   }
+  if (PASS == SCAN_WHOLE) pdl_wait();
   if (PASS == SCAN_OWN && ends) {                              // what the request came with, for the first segment of the second pass
     if (live) to_rows(seg.own + ((size_t)blockIdx.y * inner + c) * nstate);
     return;
