@@ -8,7 +8,7 @@ block size n=32, synthetic 512-token prompt / 512 new tokens, random-init weight
 A "step" = one generation: the device-resident Jacobi loop produces `--gen` new tokens for every sequence of the batch
 from an already prefilled prompt (the reference's metric excludes prefill: toks_per_sec = new_tokens / gen_only_time,
 JacobiForcing/jacobi_forcing_inference_MR_humaneval.py:217-230, 250).
-  value  = new tokens / device time of the persistent kernel (inputs resident in HBM), max over ranks
+  value  = new tokens / device time of the generation's kernels, first to last (inputs resident in HBM), max over ranks
   e2e    = new tokens / wall time of the C-ABI call jf_jacobi_run with HOST buffers (H2D of prompts, drafts, block
            tables and D2H of the generated ids inside the timed region)
 One JSON line on stdout (rank 0).
@@ -379,7 +379,8 @@ def run_ours(args, rank: int, local_rank: int, world: int):
     value = toks_all / dev_s_max
     e2e = toks_all / wall_s_max
     peak, peak_src = measured_peaks()
-    # roofline of the dominant kernel (the persistent Jacobi kernel; one launch per step) on rank 0
+    # roofline of a generation's kernels on rank 0: the persistent Jacobi kernel (one launch per step), or one kernel per stage
+    one_launch = launches <= len(steps)
     mean_rows = rows / max(1, fwd)
     mean_ctx = P + G / 2.0
     groups_per_fwd = mean_rows / max(1.0, float(n)) if args.mode == "single" else max(1.0, mean_rows / (2.0 * n))
@@ -389,11 +390,12 @@ def run_ours(args, rank: int, local_rank: int, world: int):
     launch_s = dev_s / max(1, len(steps))
     achieved = bytes_launch / launch_s / 1e9
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                "traffic": None, "kernel": "jf_persistent_kernel", "peak_source": peak_src,
+                "traffic": None, "kernel": "jf_persistent_kernel" if one_launch else "one kernel per stage (jf_step.cuh), a generation's together",
+                "peak_source": peak_src,
                 "algorithmic_bytes_per_forward": bytes_fwd, "forwards_per_launch": fwd / max(1, len(steps)),
                 "ms_per_forward": 1e3 * dev_s / max(1, fwd)}
     prof = os.path.join(ROOT, "profiles", "traffic.json")
-    if os.path.exists(prof) and tp == 1 and args.model == "qwen2.5-coder-7b" and B == 1:
+    if os.path.exists(prof) and one_launch and tp == 1 and args.model == "qwen2.5-coder-7b" and B == 1:
         try:
             per_fwd = json.load(open(prof)).get("dram_bytes_per_forward")
             # ncu capture was one 32-forward launch; a bench launch runs `forwards_per_launch` forwards of the same shape

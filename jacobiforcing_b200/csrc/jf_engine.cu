@@ -834,10 +834,11 @@ static int launch_persistent(jf_engine* h, int run_mode, int max_forwards, float
   return JF_OK;
 }
 
-// Whether a planned forward runs as one kernel per stage (jf_wide.cuh): prompt rows, that is every row is committed at its own
-// position, kWideRows of them or more, on one GPU, without a stage profile.  Verification rows keep the persistent kernel however many they are, so
-// that planned forwards and the device-resident loop agree bit for bit.  7B shape, 28 layers, ms: 256 rows 9.28 persistent, 7.8 wide;
-// 512 rows 18.7, 9.0; 1000 rows 38.4, 12.6; below 200 rows the persistent kernel's weight stream is the faster one.
+// Whether a planned forward runs on the prompt kernels (jf_wide.cuh): prompt rows, that is every row is committed at its own
+// position, kWideRows of them or more, on one GPU, without a stage profile.  Verification rows keep the arithmetic of decoding however many they are
+// (the persistent kernel, or its stages: jf_step.cuh), so that planned forwards and Jacobi runs agree bit for bit.  7B shape, 28 layers, ms:
+// 256 rows 9.28 persistent, 7.8 wide; 512 rows 18.7, 9.0; 1000 rows 38.4, 12.6.  By stages 240 rows take 4.9; the line stays at a page,
+// the unit in which prompts are cut for these kernels.
 static bool takes_wide(const jf_engine* h, int T, const std::vector<Group>& groups, const std::vector<int>& row_group, int lm_rows,
                        const std::vector<CommitEntry>& commits, int n_commit) {
   const DevCtx& c = h->hctx;

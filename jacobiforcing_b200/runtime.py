@@ -1,7 +1,7 @@
 """JacobiRuntime — Python host of the C-ABI library: the per-rank pieces the reference's ModelRunner owns
 (inference_engine/engine/model_runner.py): weights (HF tensor names, loader.py:27-47), the paged KV cache with its
 block manager (engine/block_manager.py, pages of 256 tokens), prefill-with-drafting (:777-963; HF: unified.py:175-225)
-and the Jacobi decode operator, here ONE device-resident loop per call instead of a Python loop of forwards.
+and the Jacobi decode operator, here ONE call of the library per generation instead of a Python loop of forwards.
 
 numpy carries host buffers across the ABI; torch tensors are accepted for weights (host or device pointers).
 """
@@ -322,18 +322,18 @@ class JacobiRuntime:
             end = min(total, start + self.max_rows)
             if end < total and total - end < n + 1:   # keep the n+1 logit rows inside one chunk
                 end = max(start + 1, total - (n + 1))
-            # Chunks of whole pages, all of whose rows are committed, are what the library runs as one kernel per stage; the rest of
-            # the row follows on the persistent kernel.  A prefix hit on pages that such chunks filled changes nothing, bit for bit: a row's
-            # result does not depend on the cut, and the rest is forwarded by the same kernel.  Pages that the rest of a prompt or decoding
-            # filled come from the persistent kernel; a longer prompt that hits them differs from one that does not by bf16 rounding.
+            # Chunks of whole pages, all of whose rows are committed, are what the library runs on its prompt kernels; the rest of the row follows
+            # as decoding does (the persistent kernel, or its arithmetic by stages).  A prefix hit on pages that such chunks filled changes
+            # nothing, bit for bit: a row's result does not depend on the cut, and the rest is forwarded alike.  Pages that the rest of a prompt or
+            # decoding filled come from the latter; a longer prompt that hits them differs from one that does not by bf16 rounding.
             if start % PAGE == 0 and pages_end - start >= PAGE and self.max_rows >= PAGE and self.tp_size == 1:
                 end = start + min(pages_end - start, self.max_rows // PAGE * PAGE)
             toks = row[start:end]
             T = end - start
             own = np.arange(max(0, min(T, P - start)), dtype=np.int32)
             commits, late = np.stack([own, np.zeros_like(own), own + start], axis=1), ()
-            # Without a draft the rest may be a whole page of committed rows.  A full hit forwards the last prompt token on the persistent
-            # kernel; the call of its own that commits the last row keeps a miss there too
+            # Without a draft the rest may be a whole page of committed rows.  A full hit forwards the last prompt token as decoding does; the
+            # call of its own that commits the last row keeps a miss there too
             if end == total and len(commits) == T >= PAGE and self.tp_size == 1:
                 commits, late = commits[:-1], commits[-1:]
             lm0 = max(0, want_from - start)
