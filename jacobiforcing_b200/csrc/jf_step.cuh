@@ -624,7 +624,7 @@ struct StepPlan {
   unsigned int tag;
 };
 
-constexpr int kStepAhead = 4, kStepAheadFrom = 12, kStepAheadRows = 64;      // see step_forward
+constexpr int kStepAhead = 4, kStepAheadFrom = 12, kStepAheadRows = 96;      // see step_forward
 constexpr size_t kStepAheadBytes = 24 << 20;
 inline size_t step_smem_bytes(const StepGemm& g, bool head) {
   return (size_t)g.stages * g.slot + sizeof(StepSmem) + (head ? 4 * 256 * 8 : 0) + 1024;
@@ -648,7 +648,11 @@ inline void step_product(WideStream& w, StepGemm g, int ctas, int smem_max, int*
   for (g.cols = 32; g.cols < g.mt_rows;) g.cols <<= 1;
   const int items = g.n_tiles * g.splits * g.m_tiles, grid = std::min(items, ctas);
   g.bufs = items > grid && g.cols * (DUAL ? 4 : 2) <= 512 ? 2 : 1;
-  g.groups = g.mt_rows > 128 ? 4 : g.mt_rows > 16 ? 2 : 1;
+  // Epilogue groups: one per 16 rows up to two, four where that measured faster.  A 7B forward (11 chunks of k and more a block), us, with two -> four: 24 rows
+  // the same, 40 rows 2955 -> 2905, 64 rows 3063 -> 3025, 72 rows 3095 -> 3046, 100 rows the same, 128 rows 3423 -> 3450.  With few chunks a block of 600
+  // threads starts later than it is done: 0.5B shape (5 to 10 chunks), 64 rows 1205 -> 1360.
+  const int each = (g.k_chunks + g.splits - 1) / g.splits;
+  g.groups = g.mt_rows > 128 || (g.mt_rows > 32 && g.mt_rows <= 96 && each >= 11) ? 4 : g.mt_rows > 16 ? 2 : 1;
   g.xslot = (g.mt_rows * 128 + 1023) & ~1023;
   g.stages = 0;
   const int room = smem_max - (int)step_smem_bytes(g, HEAD);
@@ -708,8 +712,8 @@ inline void step_forward(WideStream& w, const DevCtx& c, const StepPlan& p, int 
   // HBM has nothing to do while the rotary stage, attention and its merge run, and again while the output projection ends: the weights of
   // gate and up that come behind the stages which their own kernel fills early are asked for from L2 then, by the products of queries and
   // outputs (`nth` 0 and 1), kStepAhead chunks of every tile each.  Few rows only, where weights are what a layer waits for: one 7B
-  // sequence in blocks of 32 100.2 -> 97.8 ms; with eight sequences 142.9 and 143.0.  Four chunks from the twelfth on, twice; two 98.0, six 98.0,
-  // from the sixth 98.2; by the attention kernel instead, whose own keys come from HBM, 98.6 with four and 102.5 with twelve.
+  // sequence in blocks of 32 100.2 -> 97.8 ms.  Four chunks from the twelfth on, twice; two 98.0, six 98.0,
+  // from the sixth 98.2; a forward of 72 rows 3140 -> 3110 us, of 128 rows 3421 -> 3460.  By the attention kernel instead, whose own keys come from HBM, 98.6 with four and 102.5 with twelve.
   auto ahead = [&](StepGemm& g, const LayerW& L, int nth) {
     const int from = kStepAheadFrom + nth * kStepAhead;
     if (T > kStepAheadRows || c.splits_gu > 1 || from + kStepAhead > kc_h || (size_t)2 * nt_i * kStepAhead * kWTileBytes > kStepAheadBytes) return;
