@@ -27,14 +27,14 @@ def _i32(x) -> np.ndarray:
 
 
 def _triples(x) -> np.ndarray:
-    """[n, 3] int32 of a sequence of triples (1000 tuples: 100 us, numpy by itself 210)."""
-    if isinstance(x, np.ndarray) or not len(x) or not isinstance(x[0], tuple):
-        return _i32(x).reshape(-1, 3)
-    try:
-        flat = np.array(array("i", list(chain.from_iterable(x))), dtype=np.int32)
-    except TypeError:                                        # not integers
-        return _i32(x).reshape(-1, 3)
-    return flat.reshape(-1, 3) if len(flat) == 3 * len(x) else _i32(x).reshape(-1, 3)
+    """[n, 3] int32 of a sequence of triples.  Tuples of three each go end to end through array.array (1000 of them: 130 us, numpy by itself 210);
+    whatever else numpy takes, or refuses, is left to it."""
+    if isinstance(x, (list, tuple)) and set(map(type, x)) == {tuple} and set(map(len, x)) == {3}:
+        try:
+            return np.array(array("i", list(chain.from_iterable(x))), dtype=np.int32).reshape(-1, 3)
+        except TypeError:                                    # not integers
+            pass
+    return _i32(x).reshape(-1, 3)
 
 
 def _ptr(a: Optional[np.ndarray]):
