@@ -56,10 +56,9 @@ struct jf_engine {
   bool finalized = false;
   // host mirrors
   std::vector<SeqState> h_states;
-  // forwards of many rows (jf_wide.cuh): attention row units, error flag
+  // forwards of many rows (jf_wide.cuh): attention row units
   FlashUnit* wide_units_d = nullptr;
   size_t wide_units_cap = 0;
-  int* wide_err = nullptr;
   bool by_stages = false;            // forwards run as one kernel per stage (jf_step.cuh)
   // page-locked: a plan on its way to the device; the header of a Jacobi run's next forward; a forward's error word and tokens
   uint8_t* plan_h = nullptr;
@@ -860,7 +859,6 @@ static int run_wide(jf_engine* h, int T, const std::vector<Group>& groups, int l
   if (h->wide_units_d == nullptr) {
     h->wide_units_cap = (size_t)h->md.n_kv * ((size_t)h->md.n_rep * c.T_cap / 128 + c.G_cap + 1);
     int rc = dev_alloc(h, &h->wide_units_d, h->wide_units_cap, &h->bytes_act);
-    if (rc == JF_OK) rc = dev_alloc(h, &h->wide_err, 4, &h->bytes_act);
     if (rc != JF_OK) return rc;
   }
   if (units.size() > h->wide_units_cap) { h->err = "attention units exceed capacity"; return JF_ERR_CAPACITY; }
@@ -872,7 +870,7 @@ static int run_wide(jf_engine* h, int T, const std::vector<Group>& groups, int l
   JF_CUDA(h, cudaMemcpyAsync(h->wide_units_d, units.data(), units.size() * sizeof(FlashUnit), cudaMemcpyHostToDevice, h->stream));
   JF_CUDA(h, cudaEventRecord(h->ev0, h->stream));
   WideStream w{h->stream};
-  wide_forward(w, c, T, h->wide_units_d, (int)units.size(), lm_row0, lm_rows, want_hidden, h->wide_err);
+  wide_forward(w, c, T, h->wide_units_d, (int)units.size(), lm_row0, lm_rows, want_hidden, &c.hdr->stalled);
   JF_CUDA(h, cudaEventRecord(h->ev1, h->stream));
   h->launches += w.launches;
   if (w.failed) { h->err = std::string("prompt forward: ") + w.failed; return JF_ERR_CUDA; }
@@ -903,21 +901,14 @@ static int step_failed(jf_engine* h, const char* what) {
 // One forward of a plan that is on the device, enqueued as one kernel per stage.
 static int run_step(jf_engine* h, const PlanHdr& p, int n_commit) {
   DevCtx& c = h->hctx;
-  if (h->wide_err == nullptr) {
-    int rc = dev_alloc(h, &h->wide_err, 4, &h->bytes_act);
-    if (rc != JF_OK) return rc;
-  }
   const StepPlan sp{p.T, p.G, std::max(1, p.attn_hsplit), p.attn_units, p.max_len, n_commit, p.n_lm_tasks, p.iter & 1, p.want_logits, p.lm_row0, p.lm_rows, c.tag_base + 1u};
   c.tag_base += 2u;
   WideStream w{h->stream};
-  step_forward(w, c, sp, h->num_ctas, h->smem_optin, h->wide_err);
+  step_forward(w, c, sp, h->num_ctas, h->smem_optin, &c.hdr->stalled);
   h->launches += w.launches;
   return w.failed ? step_failed(h, w.failed) : JF_OK;
 }
-static int step_stalled(jf_engine* h) {
-  cudaMemset(h->wide_err, 0, 4);
-  return step_failed(h, "a wait inside a tensor-core kernel ran out (pipeline stalled)");
-}
+static int step_stalled(jf_engine* h) { return step_failed(h, "a wait inside a tensor-core kernel ran out (pipeline stalled)"); }
 static int run_step_planned(jf_engine* h, const PlanHdr& p) {
   DevCtx& c = h->hctx;
   JF_CUDA(h, cudaEventRecord(h->ev0, h->stream));
@@ -933,7 +924,8 @@ static int run_step_planned(jf_engine* h, const PlanHdr& p) {
   return JF_OK;
 }
 
-// A Jacobi run: the policy on the device, the forward that it asks for by stages, until every sequence is done.
+// A Jacobi run: the policy on the device, the forward that it asks for by stages, until every sequence is done.  Whether a wait of the forward before
+// ran out comes with the header: nothing is committed of such a forward, and none follows it.
 static int run_steps(jf_engine* h, int max_forwards, float* elapsed_ms) {
   DevCtx& c = h->hctx;
   JF_CUDA(h, cudaEventRecord(h->ev0, h->stream));
@@ -944,6 +936,7 @@ static int run_steps(jf_engine* h, int max_forwards, float* elapsed_ms) {
     ++h->launches;
     JF_CUDA(h, cudaMemcpyAsync(h->run_hdr, c.hdr, sizeof(PlanHdr), cudaMemcpyDeviceToHost, h->stream));
     JF_CUDA(h, cudaStreamSynchronize(h->stream));
+    if (h->run_hdr->stalled) return step_stalled(h);
     if (h->run_hdr->done || h->run_hdr->T < 1) break;
     const int rc = run_step(h, *h->run_hdr, h->run_hdr->n_commit);
     if (rc != JF_OK) return rc;
@@ -957,9 +950,7 @@ static int run_steps(jf_engine* h, int max_forwards, float* elapsed_ms) {
   JF_CUDA(h, cudaEventRecord(h->ev1, h->stream));
   JF_CUDA(h, cudaStreamSynchronize(h->stream));
   cudaEventElapsedTime(elapsed_ms, h->ev0, h->ev1);
-  if (!any) return JF_OK;
-  JF_CUDA(h, cudaMemcpy(h->out_h, h->wide_err, 4, cudaMemcpyDeviceToHost));
-  return *h->out_h ? step_stalled(h) : JF_OK;
+  return JF_OK;
 }
 
 extern "C" int jf_forward(jf_handle h, int32_t T, const int32_t* tokens, int32_t G, const int32_t* groups,
@@ -1062,7 +1053,7 @@ extern "C" int jf_forward(jf_handle h, int32_t T, const int32_t* tokens, int32_t
   cudaError_t e = cudaSuccess;
   auto keep = [&](cudaError_t x) { if (e == cudaSuccess) e = x; };
   if (rc == JF_OK) {
-    keep(cudaMemcpyAsync(h->out_h, h->wide_err, 4, cudaMemcpyDeviceToHost, h->stream));
+    keep(cudaMemcpyAsync(h->out_h, &c.hdr->stalled, 4, cudaMemcpyDeviceToHost, h->stream));
     if (greedy) keep(cudaMemcpyAsync(h->out_h + 1, c.greedy, (size_t)T * 4, cudaMemcpyDeviceToHost, h->stream));
     if (logits && lm_rows > 0) keep(cudaMemcpyAsync(logits, c.logits, (size_t)lm_rows * md.vocab * 4, cudaMemcpyDeviceToHost, h->stream));
     if (hidden) keep(cudaMemcpyAsync(hidden, c.hidden, (size_t)T * md.h * 2, cudaMemcpyDeviceToHost, h->stream));

@@ -70,6 +70,7 @@ struct PlanHdr {
   int rows_total;            // sum of T over the forwards of this launch
   int attn_hsplit;           // attention units per kv head along its q heads, chosen per forward (pick_attn_hsplit)
   int max_len;               // rows of the longest group
+  int stalled;               // set by a kernel of a forward by stages, or of a prompt, one of whose waits ran out
 };
 
 struct SeqSlot {             // per-sequence bookkeeping owned by the policy stage

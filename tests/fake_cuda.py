@@ -41,6 +41,7 @@ class Fake:
         self.lib.fake_fail.argtypes = [C.c_int, C.c_long]
         self.lib.fake_room.argtypes = [C.c_longlong]
         self.lib.fake_used.restype = C.c_longlong
+        self.lib.fake_plant.argtypes = [C.c_long, C.c_long, C.c_int, C.c_long]
         self.reset()
 
     def reset(self):
@@ -67,6 +68,11 @@ class Fake:
     def on_their_way(self):
         """Copies to the host since the last wait for the stream."""
         return self.lib.fake_on_their_way()
+
+    def plant(self, size, at, value, first=0):
+        """Copies to the host of `size` bytes bring this int at byte `at`, from copy number `first` of that size on, until the next reset: what kernels that ran would
+        have left there."""
+        self.lib.fake_plant(size, at, value, first)
 
     def launches(self):
         """(kernel, device) of every launch that went through since the last reset."""

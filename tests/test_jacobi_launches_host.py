@@ -1,5 +1,8 @@
 """Host side of the Jacobi engine's prompt forwards: kernels are set up on every device that an engine is made on, a forward stops at
 the first call that fails, and which rows of a prompt run on which kernel."""
+import os
+import re
+
 import pytest
 
 from tests import fake_cuda
@@ -182,4 +185,48 @@ def test_small_models_keep_the_persistent_kernel(fake):
     rt.forward([1] * 40, [(0, 40, 0, 0)], [s], 0, 40)
     assert ["persistent" in n for n, _ in fake.launches()] == [True]
     rt.release(s)
+    rt.close()
+
+
+def header(fake, first=0, **fields):
+    """What the policy kernel leaves in the header of a run's forward, as the host reads it."""
+    source = open(os.path.join(fake_cuda.CSRC, "jf_types.h")).read()
+    size, at = 0, {}
+    for name, many in re.findall(r"^  int (\w+)(\[kMaxLmTasks\])?;", source[source.index("struct PlanHdr"):source.index("struct SeqSlot")], re.M):
+        at[name], size = size, size + 4 * (int(re.search(r"kMaxLmTasks *= (\d+)", source).group(1)) if many else 1)
+    for name, value in fields.items():
+        fake.plant(size, at[name], value, first)
+
+
+def run(rt):
+    from jacobiforcing_b200.policy import MODES, PolicyKnobs
+    s = rt.new_sequence()
+    s.tokens, s.ctx = [1] * 20, 20
+    try:
+        return rt.jacobi_run([s], PolicyKnobs(mode=MODES["single"], n=8, max_new_tokens=16, max_calls=4, vocab=rt.vocab), [1], [[1] * 8])[1]
+    finally:
+        rt.release(s)
+
+
+def test_a_run_by_stages_ends_at_the_first_wait_that_ran_out(fake, monkeypatch):
+    """The error comes before another forward, and before anything of the stalled one is committed.  The engine works on."""
+    monkeypatch.setenv("JF_BY_STAGES", "1")
+    rt = engine()
+
+    def names(stalled):
+        fake.reset()
+        header(fake, T=8, G=1, max_len=8, n_lm_tasks=1, lm_rows=8, n_commit=3)
+        header(fake, first=2, stalled=stalled)
+        header(fake, first=3, done=1)
+        try:
+            return run(rt), [n for n, _ in fake.launches()]
+        except RuntimeError as e:
+            return str(e), [n for n, _ in fake.launches()]
+    done, whole = names(0)
+    assert isinstance(done, dict) and sum("policy" in n for n in whole) == 4 and sum("commit" in n for n in whole) == 4
+    error, short = names(1)
+    assert "a wait inside a tensor-core kernel ran out" in error
+    ends = [i for i, n in enumerate(whole) if "policy" in n]
+    assert short == whole[:ends[2] + 1]
+    assert names(0)[1] == whole
     rt.close()
