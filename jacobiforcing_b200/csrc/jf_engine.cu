@@ -57,7 +57,7 @@ struct jf_engine {
   // host mirrors
   std::vector<SeqState> h_states;
   // forwards of many rows (jf_wide.cuh): attention row units
-  FlashUnit* wide_units_d = nullptr;
+  FlashUnit *wide_units_d = nullptr, *wide_units_h = nullptr;      // the latter page-locked, on their way to the former
   size_t wide_units_cap = 0;
   bool by_stages = false;            // forwards run as one kernel per stage (jf_step.cuh)
   // page-locked: a plan on its way to the device; the header of a Jacobi run's next forward; a forward's error word and tokens
@@ -438,6 +438,7 @@ extern "C" int jf_destroy(jf_handle h) {
   for (void* p : h->ipc_maps) cudaIpcCloseMemHandle(p);
   for (void* p : h->allocs) cudaFree(p);
   for (int* p : h->run_scratch) if (p) cudaFree(p);
+  if (h->wide_units_h) cudaFreeHost(h->wide_units_h);
   if (h->plan_h) cudaFreeHost(h->plan_h);
   if (h->run_hdr) cudaFreeHost(h->run_hdr);
   if (h->out_h) cudaFreeHost(h->out_h);
@@ -858,6 +859,7 @@ static int run_wide(jf_engine* h, int T, const std::vector<Group>& groups, int l
   const std::vector<FlashUnit> units = wide_units(h->md, groups, c.max_pages_per_seq);
   if (h->wide_units_d == nullptr) {
     h->wide_units_cap = (size_t)h->md.n_kv * ((size_t)h->md.n_rep * c.T_cap / 128 + c.G_cap + 1);
+    if (h->wide_units_h == nullptr) JF_CUDA(h, cudaMallocHost((void**)&h->wide_units_h, h->wide_units_cap * sizeof(FlashUnit)));
     int rc = dev_alloc(h, &h->wide_units_d, h->wide_units_cap, &h->bytes_act);
     if (rc != JF_OK) return rc;
   }
@@ -867,7 +869,9 @@ static int run_wide(jf_engine* h, int T, const std::vector<Group>& groups, int l
     if (rc != JF_OK) return rc;
     JF_CUDA(h, cudaMemcpyAsync(h->dctx, &h->hctx, sizeof(DevCtx), cudaMemcpyHostToDevice, h->stream));
   }
-  JF_CUDA(h, cudaMemcpyAsync(h->wide_units_d, units.data(), units.size() * sizeof(FlashUnit), cudaMemcpyHostToDevice, h->stream));
+  // The caller waits for the copy, behind the kernels: its source outlives this call.
+  memcpy(h->wide_units_h, units.data(), units.size() * sizeof(FlashUnit));
+  JF_CUDA(h, cudaMemcpyAsync(h->wide_units_d, h->wide_units_h, units.size() * sizeof(FlashUnit), cudaMemcpyHostToDevice, h->stream));
   JF_CUDA(h, cudaEventRecord(h->ev0, h->stream));
   WideStream w{h->stream};
   wide_forward(w, c, T, h->wide_units_d, (int)units.size(), lm_row0, lm_rows, want_hidden, &c.hdr->stalled);

@@ -74,6 +74,14 @@ class Fake:
         have left there."""
         self.lib.fake_plant(size, at, value, first)
 
+    def watch(self, on):
+        """From here on, look whether the sources of copies to the device stay as they are until the wait behind them."""
+        self.lib.fake_watch(int(on))
+
+    def changed(self):
+        """How many did not."""
+        return self.lib.fake_changed()
+
     def launches(self):
         """(kernel, device) of every launch that went through since the last reset."""
         return [(self.lib.fake_launch_name(i).decode(), self.lib.fake_launch_device(i)) for i in range(self.lib.fake_launches())]

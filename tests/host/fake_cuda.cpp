@@ -28,6 +28,11 @@ int g_on_their_way = 0;                                         // copies to the
 struct Planted { size_t bytes, at; int value; long from; };
 std::vector<Planted> g_planted;
 std::map<size_t, long> g_of_size;                                // copies to the host by their size
+// copies to the device since the last wait, whose sources have to stay as they were until it (a test asks for this)
+struct Source { const void* at; std::string was; };
+std::vector<Source> g_sources;
+bool g_watching = false;
+int g_changed = 0;
 constexpr size_t kDefaultSmem = 48 * 1024, kMostSmem = 227 * 1024;
 
 bool fails(int what) { return g_count[what]++ == g_fail[what]; }
@@ -62,6 +67,8 @@ int fake_pinned() { return (int)g_pinned.size(); }
 int fake_pinned_device(int i) { return g_pinned[i]; }
 int fake_on_their_way() { return g_on_their_way; }
 void fake_plant(long bytes, long at, int value, long from) { g_planted.push_back({(size_t)bytes, (size_t)at, value, from}); }
+void fake_watch(int on) { g_watching = on != 0; g_sources.clear(); g_changed = 0; }
+int fake_changed() { return g_changed; }
 int fake_launches() { return (int)g_launches.size(); }
 const char* fake_launch_name(int i) { return names()[g_launches[i].f].c_str(); }
 int fake_launch_device(int i) { return g_launches[i].device; }
@@ -119,6 +126,7 @@ cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind k, 
     ++g_on_their_way;
   }
   memcpy(d, s, n);
+  if (g_watching && k == cudaMemcpyHostToDevice) g_sources.push_back({s, std::string((const char*)s, n)});
   if (k == cudaMemcpyDeviceToHost) {
     const long number = g_of_size[n]++;
     for (const Planted& p : g_planted)
@@ -131,7 +139,12 @@ cudaError_t cudaMemsetAsync(void* d, int v, size_t n, cudaStream_t) { memset(d, 
 cudaError_t cudaStreamCreate(cudaStream_t* s) { *s = nullptr; return cudaSuccess; }
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) { *s = nullptr; return cudaSuccess; }
 cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
-cudaError_t cudaStreamSynchronize(cudaStream_t) { g_on_their_way = 0; return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t) {
+  g_on_their_way = 0;
+  for (const Source& x : g_sources) g_changed += memcmp(x.at, x.was.data(), x.was.size()) != 0;
+  g_sources.clear();
+  return cudaSuccess;
+}
 cudaError_t cudaDeviceSynchronize() { return cudaSuccess; }
 cudaError_t cudaEventCreate(cudaEvent_t* e) { *e = nullptr; return cudaSuccess; }
 cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }

@@ -176,6 +176,21 @@ def test_a_forward_by_stages_stops_at_the_first_launch_that_fails(fake, what, mo
     rt.close()
 
 
+@pytest.mark.parametrize("rows,stages", [(256, "0"), (512, "0"), (40, "1"), (40, "0")])
+def test_what_is_on_its_way_to_the_device_outlives_the_copy(fake, rows, stages, monkeypatch):
+    """A forward waits once, behind its kernels: whatever it copies to the device is still there then, as it was."""
+    monkeypatch.setenv("JF_BY_STAGES", stages)
+    rt = engine()
+    fake.watch(True)
+    try:
+        for _ in range(2):
+            chunk(rt, rows)
+        assert fake.changed() == 0
+    finally:
+        fake.watch(False)
+    rt.close()
+
+
 def test_small_models_keep_the_persistent_kernel(fake):
     """A forward of theirs is one launch; the line is a layer's weights."""
     rt = engine()
