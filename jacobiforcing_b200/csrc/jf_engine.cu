@@ -936,10 +936,13 @@ static int run_steps(jf_engine* h, int max_forwards, float* elapsed_ms) {
   bool any = false;
   for (;;) {
     step_policy_kernel<<<1, kNumThreads, kPolicySmem, h->stream>>>(h->dctx, !any, max_forwards);
-    JF_CUDA(h, cudaGetLastError());
-    ++h->launches;
-    JF_CUDA(h, cudaMemcpyAsync(h->run_hdr, c.hdr, sizeof(PlanHdr), cudaMemcpyDeviceToHost, h->stream));
-    JF_CUDA(h, cudaStreamSynchronize(h->stream));
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) {
+      ++h->launches;
+      e = cudaMemcpyAsync(h->run_hdr, c.hdr, sizeof(PlanHdr), cudaMemcpyDeviceToHost, h->stream);
+    }
+    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+    if (e != cudaSuccess) return step_failed(h, cudaGetErrorString(e));      // the forward before left its argmax keys
     if (h->run_hdr->stalled) return step_stalled(h);
     if (h->run_hdr->done || h->run_hdr->T < 1) break;
     const int rc = run_step(h, *h->run_hdr, h->run_hdr->n_commit);

@@ -41,6 +41,7 @@ class Fake:
         self.lib.fake_fail.argtypes = [C.c_int, C.c_long]
         self.lib.fake_room.argtypes = [C.c_longlong]
         self.lib.fake_used.restype = C.c_longlong
+        self.lib.fake_cleared.restype, self.lib.fake_cleared.argtypes = C.c_long, [C.c_long]
         self.lib.fake_plant.argtypes = [C.c_long, C.c_long, C.c_int, C.c_long]
         self.reset()
 
@@ -81,6 +82,10 @@ class Fake:
     def changed(self):
         """How many did not."""
         return self.lib.fake_changed()
+
+    def cleared(self, size):
+        """How often this many bytes were set on the stream since the last reset."""
+        return self.lib.fake_cleared(size)
 
     def launches(self):
         """(kernel, device) of every launch that went through since the last reset."""

@@ -27,7 +27,7 @@ int g_on_their_way = 0;                                         // copies to the
 // what a test has kernels leave on the device: copies to the host of exactly `bytes`, from the number `from` on, bring `value` at `at`
 struct Planted { size_t bytes, at; int value; long from; };
 std::vector<Planted> g_planted;
-std::map<size_t, long> g_of_size;                                // copies to the host by their size
+std::map<size_t, long> g_of_size, g_cleared;                     // copies to the host, memory set, by their size
 // copies to the device since the last wait, whose sources have to stay as they were until it (a test asks for this)
 struct Source { const void* at; std::string was; };
 std::vector<Source> g_sources;
@@ -58,7 +58,7 @@ CUresult encode(CUtensorMap* m, CUtensorMapDataType, cuuint32_t, void* p, const 
 
 extern "C" {
 // ---- what a test asks ---------------------------------------------------------------------------------------------------------------
-void fake_reset() { g_launches.clear(); g_pinned.clear(); g_planted.clear(); g_of_size.clear(); for (int i = 0; i < kKinds; ++i) { g_count[i] = 0; g_fail[i] = -1; } g_last = cudaSuccess; }
+void fake_reset() { g_launches.clear(); g_pinned.clear(); g_planted.clear(); g_of_size.clear(); g_cleared.clear(); for (int i = 0; i < kKinds; ++i) { g_count[i] = 0; g_fail[i] = -1; } g_last = cudaSuccess; }
 void fake_fail(int what, long at) { g_count[what] = 0; g_fail[what] = at; }
 long fake_count(int what) { return g_count[what]; }
 void fake_room(long long bytes) { g_room = (size_t)bytes; }
@@ -69,6 +69,7 @@ int fake_on_their_way() { return g_on_their_way; }
 void fake_plant(long bytes, long at, int value, long from) { g_planted.push_back({(size_t)bytes, (size_t)at, value, from}); }
 void fake_watch(int on) { g_watching = on != 0; g_sources.clear(); g_changed = 0; }
 int fake_changed() { return g_changed; }
+long fake_cleared(long bytes) { return g_cleared[(size_t)bytes]; }
 int fake_launches() { return (int)g_launches.size(); }
 const char* fake_launch_name(int i) { return names()[g_launches[i].f].c_str(); }
 int fake_launch_device(int i) { return g_launches[i].device; }
@@ -135,7 +136,7 @@ cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind k, 
   return cudaSuccess;
 }
 cudaError_t cudaMemset(void* d, int v, size_t n) { memset(d, v, n); return cudaSuccess; }
-cudaError_t cudaMemsetAsync(void* d, int v, size_t n, cudaStream_t) { memset(d, v, n); return cudaSuccess; }
+cudaError_t cudaMemsetAsync(void* d, int v, size_t n, cudaStream_t) { ++g_cleared[n]; memset(d, v, n); return cudaSuccess; }
 cudaError_t cudaStreamCreate(cudaStream_t* s) { *s = nullptr; return cudaSuccess; }
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) { *s = nullptr; return cudaSuccess; }
 cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }

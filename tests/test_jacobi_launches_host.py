@@ -245,3 +245,31 @@ def test_a_run_by_stages_ends_at_the_first_wait_that_ran_out(fake, monkeypatch):
     assert short == whole[:ends[2] + 1]
     assert names(0)[1] == whole
     rt.close()
+
+
+@pytest.mark.parametrize("what", ["launch", "header"])
+def test_a_run_by_stages_that_fails_leaves_the_argmax_keys_clean(fake, what, monkeypatch):
+    """Whichever launch, or copy of a header, is refused: an error, nothing behind it, and a forward before it has left nothing for the next run."""
+    monkeypatch.setenv("JF_BY_STAGES", "1")
+    rt = engine()
+    keys, kind = 2 * 512 * 8, fake_cuda.LAUNCH if what == "launch" else fake_cuda.TO_HOST
+
+    def plan():
+        fake.reset()
+        header(fake, T=8, G=1, max_len=8, n_lm_tasks=1, lm_rows=8, n_commit=3)
+        header(fake, first=2, done=1)
+    plan()
+    run(rt)
+    whole, calls = [n for n, _ in fake.launches()], fake.count(fake_cuda.LAUNCH) if what == "launch" else 3
+    assert fake.cleared(keys) == 1 and sum("policy" in n for n in whole) == 3
+    for at in range(calls):
+        plan()
+        fake.fail(kind, at)
+        with pytest.raises(RuntimeError, match="forward by stages: " + ("launch refused" if what == "launch" else "invalid argument")):
+            run(rt)
+        went = [n for n, _ in fake.launches()]
+        assert went == whole[:len(went)] and (what == "header" or len(went) == at) and fake.cleared(keys) == 1
+    plan()
+    run(rt)
+    assert [n for n, _ in fake.launches()] == whole
+    rt.close()
