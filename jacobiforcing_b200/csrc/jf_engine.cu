@@ -888,9 +888,9 @@ static int run_wide(jf_engine* h, int T, const std::vector<Group>& groups, int l
 // 1.2 MB 112 -> 99 / 335 -> 148 / 197 -> 150;  5.6 MB 221 -> 193 / 543 -> 277 / 295 -> 230;  7.6 MB 587 -> 462 / 1436 -> 700 /
 // 666 -> 503;  30 MB 1287 -> 1128 / 2736 -> 1780 / 1337 -> 1175;  466 MB (7B), blocks of 32, one / eight sequences 3260 -> 3040 / 7300 -> 4340.
 // Sampling verification, tensor parallelism and profiles of the stages keep the persistent kernel as well.
-static bool step_pays(const jf_engine* h) {
+static bool step_pays(const jf_engine* h, bool sampling) {
   const DevCtx& c = h->hctx;
-  return h->by_stages && c.ng_mode == 0 && c.debug_skip == 0 && !(c.prof && c.prof_forward >= 0);
+  return h->by_stages && !sampling && c.debug_skip == 0 && !(c.prof && c.prof_forward >= 0);
 }
 
 // What went through ends, and the argmax keys are clean for the next forward.
@@ -1045,7 +1045,7 @@ extern "C" int jf_forward(jf_handle h, int32_t T, const int32_t* tokens, int32_t
   put(c.commits, hc.data(), (size_t)n_commit * sizeof(CommitEntry));
   JF_CUDA(h, cudaMemcpyAsync(first, h->plan_h, (size_t)(reinterpret_cast<uint8_t*>(c.commits + n_commit) - first), cudaMemcpyHostToDevice, h->stream));
   const bool wide = takes_wide(h, T, hg, row_group, lm_rows, hc, n_commit);
-  if (!wide && !step_pays(h)) {
+  if (!wide && !step_pays(h, false)) {
     int rc = launch_persistent(h, RUN_PLAN, 1, elapsed_ms);
     if (rc != JF_OK) { cudaStreamSynchronize(h->stream); return rc; }
     int dev_err = 0;
@@ -1211,7 +1211,7 @@ extern "C" int jf_jacobi_run(jf_handle h, int32_t n_seqs, const jf_policy_knobs*
   float ms = 0.f;
   const int forwards = max_forwards > 0 ? max_forwards : (1 << 30);
   PlanHdr hdr;
-  if (step_pays(h)) {
+  if (step_pays(h, kn.mode == MODE_ENGINE_NG)) {
     TRY(run_steps(h, forwards, &ms));
     hdr = *h->run_hdr;
   } else {

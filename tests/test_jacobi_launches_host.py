@@ -213,12 +213,12 @@ def header(fake, first=0, **fields):
         fake.plant(size, at[name], value, first)
 
 
-def run(rt):
+def run(rt, mode="single", **knobs):
     from jacobiforcing_b200.policy import MODES, PolicyKnobs
     s = rt.new_sequence()
     s.tokens, s.ctx = [1] * 20, 20
     try:
-        return rt.jacobi_run([s], PolicyKnobs(mode=MODES["single"], n=8, max_new_tokens=16, max_calls=4, vocab=rt.vocab), [1], [[1] * 8])[1]
+        return rt.jacobi_run([s], PolicyKnobs(mode=MODES[mode], n=8, max_new_tokens=16, max_calls=4, vocab=rt.vocab, **knobs), [1], [[1] * 8])[1]
     finally:
         rt.release(s)
 
@@ -272,4 +272,24 @@ def test_a_run_by_stages_that_fails_leaves_the_argmax_keys_clean(fake, what, mon
     plan()
     run(rt)
     assert [n for n, _ in fake.launches()] == whole
+    rt.close()
+
+
+def test_a_sampling_run_says_nothing_about_the_calls_behind_it(fake, monkeypatch):
+    """It takes the persistent kernel; forwards and greedy runs behind it go by stages as those before it do."""
+    monkeypatch.setenv("JF_BY_STAGES", "1")
+    rt = engine()
+
+    def kernels(call):
+        fake.reset()
+        header(fake, T=8, G=1, max_len=8, n_lm_tasks=1, lm_rows=8)
+        header(fake, first=1, done=1)
+        call()
+        return [n for n, _ in fake.launches()]
+    forward, greedy = kernels(lambda: chunk(rt, 40)), kernels(lambda: run(rt))
+    assert len(forward) > 1 and len(greedy) > 1 and not any("persistent" in n for n in forward + greedy)
+    for _ in range(2):
+        assert ["persistent" in n for n in kernels(lambda: run(rt, "engine_nongreedy", temperature=0.7))] == [True]
+        assert kernels(lambda: chunk(rt, 40)) == forward
+    assert kernels(lambda: run(rt)) == greedy and kernels(lambda: chunk(rt, 40)) == forward
     rt.close()
