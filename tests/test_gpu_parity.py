@@ -284,6 +284,7 @@ def _run_mid(monkeypatch, fused: bool, rows_list, gen_kw):
     from jacobiforcing_b200.runtime import hf_generate
     for k in ("JF_FUSE_NORM", "JF_FUSE_ROPE"):
         monkeypatch.setenv(k, "1" if fused else "0")          # read once, when the engine is created
+    monkeypatch.setenv("JF_BY_STAGES", "0")                   # the tails are the persistent kernel's
     # (mid128 also runs the split-K gate/up projection - 4 k-splits, SwiGLU in the tail - in BOTH engines: that is a
     # property of the engine, not of the fusion switches)
     model, rt = make_pair("mid128")
@@ -292,7 +293,9 @@ def _run_mid(monkeypatch, fused: bool, rows_list, gen_kw):
         ids = _prompt(model, rows, seed=3)
         seq = rt.new_sequence()
         rt.ensure_capacity(seq, len(ids))
+        launches = rt.launches
         res = rt.forward(ids, [(0, len(ids), 0, 0)], [seq], 0, len(ids), want_logits=True)
+        assert rt.launches == launches + 1
         out["logits"].append(res["logits"].copy())
         out["greedy"].append(np.asarray(res["greedy"]).copy())
         rt.release(seq)
@@ -335,7 +338,7 @@ def _run_switches(monkeypatch, shape, env, rows_list, gen_kw):
     import random
     from tests.gpu_helpers import make_pair
     from jacobiforcing_b200.runtime import hf_generate
-    for k, v in env.items():
+    for k, v in dict(env, JF_BY_STAGES="0").items():          # the switches are the persistent kernel's
         monkeypatch.setenv(k, v)                              # read once, when the engine is created
     model, rt = make_pair(shape)
     out = {"logits": []}
@@ -343,7 +346,9 @@ def _run_switches(monkeypatch, shape, env, rows_list, gen_kw):
         ids = _prompt(model, rows, seed=11)
         seq = rt.new_sequence()
         rt.ensure_capacity(seq, len(ids))
+        launches = rt.launches
         res = rt.forward(ids, [(0, len(ids), 0, 0)], [seq], 0, len(ids), want_logits=True)
+        assert rt.launches == launches + 1
         out["logits"].append(res["logits"].copy())
         rt.release(seq)
     prompt = _prompt(model, 40, seed=5)
