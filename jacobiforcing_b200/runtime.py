@@ -453,8 +453,8 @@ class ThreadedTensorParallel:
     """tensor_parallel_size ranks inside ONE process: one JacobiRuntime per rank, each driven by its own host thread (the
     launches must overlap: the ranks meet inside the kernels), wired with tp.LocalTPGroup / jf_tp_attach_local.  What the
     reference gets by spawning worker processes behind `LLM(..., tensor_parallel_size=N)` (engine/llm_engine.py:31-44,
-    model_runner.py:423-458) - a plain script, no torchrun.  `devices[r]` is rank r's CUDA device; ranks may share a device
-    (its SMs are then divided between them), which is how the single-GPU tests cover this class.
+    model_runner.py:423-458) - a plain script, no torchrun.  `devices[r]` is rank r's CUDA device.  Ranks that share one divide its SMs
+    between them; nothing promises that their kernels, which wait for one another, then run at the same time.
 
     The object has the JacobiRuntime surface the engine uses; every call is collective (fanned out to all ranks) and
     returns rank 0's result.  Host bookkeeping objects (SeqHandle) passed in are mutated by rank 0 only: the other ranks

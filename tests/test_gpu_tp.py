@@ -1,5 +1,5 @@
-"""Tensor parallelism on real GPUs (needs >= 2 B200 with NVLink peer access; skipped otherwise - the same kernels are
-covered on one GPU by tests/test_gpu_tp_virtual.py): one process per GPU, the persistent kernel on every rank pushing
+"""Tensor parallelism on real GPUs (needs >= 2 B200 with NVLink peer access; skipped otherwise; tests/test_gpu_tp_virtual.py
+has the same with a thread per rank): one process per GPU, the persistent kernel on every rank pushing
 its row-split partial sums / finished rows into the peers' memory and reading their argmax keys over NVLink.
 Checks: both ranks return identical ids / iteration counts; the gathered logits match the single-GPU engine and the HF
 fp32 oracle within the bf16 tolerance; Jacobi == AR on the sharded engine; ids equal the single-GPU ids up to near-ties
