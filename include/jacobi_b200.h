@@ -132,7 +132,8 @@ int jf_jacobi_run(jf_handle h, int32_t n_seqs, const jf_policy_knobs* knobs, con
 
 /* Stage profile (the reference's PROFILE=1 ProfileTimer, engine/model_runner.py:26-152, without its synchronising
  * side effects): record SM-clock stamps (arrival of CTA 0, barrier release) at every grid barrier of forward number
- * `forward_index` of the following launches (-1 = off); read them back after a run.  sm_clock_khz converts to time. */
+ * `forward_index` of the following calls (-1 = off); read them back after a run.  sm_clock_khz converts to time.  A forward that runs
+ * as one kernel per stage is profiled by events behind its stages (both stamps the same), which then follow one another without overlap. */
 int jf_profile_enable(jf_handle h, int32_t forward_index);
 int jf_profile_read(jf_handle h, int64_t* stamps, int32_t capacity, int32_t* n_stamps, int32_t* sm_clock_khz);
 

@@ -59,6 +59,7 @@ struct jf_engine {
   // forwards of many rows (jf_wide.cuh): attention row units
   FlashUnit *wide_units_d = nullptr, *wide_units_h = nullptr;      // the latter page-locked, on their way to the former
   size_t wide_units_cap = 0;
+  std::vector<int64_t> stage_stamps; // of the last forward by stages that was profiled (jf_profile_read)
   bool by_stages = false;            // forwards run as one kernel per stage (jf_step.cuh)
   // page-locked: a plan on its way to the device; the header of a Jacobi run's next forward; a forward's error word and tokens
   uint8_t* plan_h = nullptr;
@@ -556,6 +557,12 @@ extern "C" int jf_profile_read(jf_handle h, int64_t* stamps, int32_t capacity, i
   DevCtx& c = h->hctx;
   *n_stamps = 0;
   if (c.prof == nullptr) return JF_OK;
+  if (!h->stage_stamps.empty()) {
+    *n_stamps = (int32_t)std::min(h->stage_stamps.size(), (size_t)std::max(0, capacity));
+    memcpy(stamps, h->stage_stamps.data(), (size_t)*n_stamps * 8);
+    if (sm_clock_khz) cudaDeviceGetAttribute(sm_clock_khz, cudaDevAttrClockRate, h->device);
+    return JF_OK;
+  }
   int n = 0;
   JF_CUDA(h, cudaMemcpy(&n, c.prof_count, 4, cudaMemcpyDeviceToHost));
   if (n > capacity) n = capacity;
@@ -780,6 +787,7 @@ extern "C" int jf_set_rope_tables(jf_handle h, const float* cosv, const float* s
 // launch
 // ---------------------------------------------------------------------------------------------------------------
 static int launch_persistent(jf_engine* h, int run_mode, int max_forwards, float* elapsed_ms) {
+  if (h->hctx.prof && h->hctx.prof_forward >= 0) h->stage_stamps.clear();
   JF_CUDA(h, cudaMemsetAsync(h->hctx.bar_counter, 0, (4 + 3 * kMaxTilesPerKind) * sizeof(unsigned int), h->stream));
   if (h->hctx.tag_base > 0xE0000000u) {          // 32-bit stage tags about to wrap: forget every stored tag (0 is never used)
     DevCtx& c = h->hctx;
@@ -887,10 +895,10 @@ static int run_wide(jf_engine* h, int T, const std::vector<Group>& groups, int l
 // stages, in a run of one sequence in blocks of 16 / of four with lookahead blocks / a planned one of 8 rows, by a layer's bytes:
 // 1.2 MB 112 -> 99 / 335 -> 148 / 197 -> 150;  5.6 MB 221 -> 193 / 543 -> 277 / 295 -> 230;  7.6 MB 587 -> 462 / 1436 -> 700 /
 // 666 -> 503;  30 MB 1287 -> 1128 / 2736 -> 1780 / 1337 -> 1175;  466 MB (7B), blocks of 32, one / eight sequences 3260 -> 3040 / 7300 -> 4340.
-// Sampling verification, tensor parallelism and profiles of the stages keep the persistent kernel as well.
+// Sampling verification, tensor parallelism and marks inside the persistent kernel (JF_PROF_MARKS) keep that kernel as well.
 static bool step_pays(const jf_engine* h, bool sampling) {
   const DevCtx& c = h->hctx;
-  return h->by_stages && !sampling && c.debug_skip == 0 && !(c.prof && c.prof_forward >= 0);
+  return h->by_stages && !sampling && c.debug_skip == 0 && !(c.prof_marks && c.prof_forward >= 0);
 }
 
 // What went through ends, and the argmax keys are clean for the next forward.
@@ -902,15 +910,35 @@ static int step_failed(jf_engine* h, const char* what) {
   return JF_ERR_CUDA;
 }
 
-// One forward of a plan that is on the device, enqueued as one kernel per stage.
+// A profiled forward's stages, in the records of the persistent kernel's profile: (stage, its end, its end), first and last the start and the end with
+// minus the nanoseconds in the stage's place; in clocks of the device's rate.  The forward is over.
+static void keep_stages(jf_engine* h, const StageClock& clock) {
+  int khz = 0;
+  cudaDeviceGetAttribute(&khz, cudaDevAttrClockRate, h->device);
+  h->stage_stamps.clear();
+  float ms = 0.f;
+  for (size_t i = 0; i < clock.events.size(); ++i) {
+    if (i && cudaEventElapsedTime(&ms, clock.events[0], clock.events[i]) != cudaSuccess) return;
+    const int64_t at = (int64_t)((double)ms * khz);
+    h->stage_stamps.insert(h->stage_stamps.end(), {i ? (int64_t)clock.ids[i] : -1, at, at});
+  }
+  const int64_t end = (int64_t)((double)ms * khz);
+  h->stage_stamps.insert(h->stage_stamps.end(), {-1 - (int64_t)((double)ms * 1e6), end, end});
+}
+
+// One forward of a plan that is on the device, enqueued as one kernel per stage; profiled, it is waited for.
 static int run_step(jf_engine* h, const PlanHdr& p, int n_commit) {
   DevCtx& c = h->hctx;
+  StageClock clock;
   const StepPlan sp{p.T, p.G, std::max(1, p.attn_hsplit), p.attn_units, p.max_len, n_commit, p.n_lm_tasks, p.iter & 1, p.want_logits, p.lm_row0, p.lm_rows, c.tag_base + 1u};
   c.tag_base += 2u;
   WideStream w{h->stream};
+  if (c.prof && c.prof_forward == p.iter) w.clock = &clock;
   step_forward(w, c, sp, h->num_ctas, h->smem_optin, &c.hdr->stalled);
   h->launches += w.launches;
-  return w.failed ? step_failed(h, w.failed) : JF_OK;
+  if (w.failed) return step_failed(h, w.failed);
+  if (w.clock && cudaStreamSynchronize(h->stream) == cudaSuccess) keep_stages(h, clock);
+  return JF_OK;
 }
 static int step_stalled(jf_engine* h) { return step_failed(h, "a wait inside a tensor-core kernel ran out (pipeline stalled)"); }
 static int run_step_planned(jf_engine* h, const PlanHdr& p) {

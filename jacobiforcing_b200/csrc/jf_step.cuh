@@ -732,21 +732,29 @@ inline void step_forward(WideStream& w, const DevCtx& c, const StepPlan& p, int 
   const int row_tiles = (std::min(p.max_len, kQTokPerUnit) + 15) / 16, hs = (md.n_rep + 4 / row_tiles - 1) / (4 / row_tiles), units = p.units / p.hsplit * hs;
   const size_t attn_smem = (size_t)2 * kAttnSub * (md.d + 8) * 2;
   const int combine = (T * md.n_q + 7) / 8;
+  w.mark(SID_NONE);
   step_commit(w, c, p.n_commit);
   step_norm(w, c, T, 0, nullptr, c.layer[0].ln1);
+  w.mark(SID_EMBED);
   for (int l = 0; l < md.layers && !w.failed; ++l) {
     const LayerW& L = c.layer[l];
     partial(L.wqkv, c.xn, c.part, nt_qkv, kc_h, c.splits_qkv, md.qkv_dim, &L, 0);
+    w.mark(SID_QKV);
     const StepRope r{c.part, c.part_splits * c.part_n, c.part_n, L.bqkv, c.row_pos, c.rope_cos, c.rope_sin, c.qbuf,
                      c.kv_scratch + kv_scratch_offset(md, c.T_cap, l, 0, 0, 0), c.kv_scratch + kv_scratch_offset(md, c.T_cap, l, 1, 0, 0),
                      T, md.n_q, md.n_kv, md.d, md.max_pos};
     if (md.d == 128) step_rope<2>(w, r, c.splits_qkv); else step_rope<1>(w, r, c.splits_qkv);
+    w.mark(SID_ROPE);
     auto attention = [&](auto kernel) { w.launch(kernel, units, 128, attn_smem, sc, c.groups, p.G, l, p.hsplit, hs); };
     if (md.d == 128) { if (c.attn_chunk == kAttnSub) attention(step_attention_kernel<128, true>); else attention(step_attention_kernel<128, false>); }
     else { if (c.attn_chunk == kAttnSub) attention(step_attention_kernel<64, true>); else attention(step_attention_kernel<64, false>); }
+    w.mark(SID_ATTN);
     if (md.d == 128) w.launch(step_combine_kernel<4>, combine, 256, 0, sc, T); else w.launch(step_combine_kernel<2>, combine, 256, 0, sc, T);
+    w.mark(SID_COMBINE);
     partial(L.wo, c.xa, c.part_rs[0], nt_h, kc_q, c.splits_o, md.h, &L, 1);
+    w.mark(SID_O);
     step_norm(w, c, T, c.splits_o, c.part_rs[0], L.ln2);
+    w.mark(SID_O_NORM);
     if (c.splits_gu > 1) {
       StepGemm g = product(L.wgu, c.xn, c.tgu, nt_i, kc_h, c.splits_gu, md.inter);
       g.tag = p.tag; g.row_stride = c.splits_gu * 2 * md.inter; g.split_stride = 2 * md.inter;
@@ -760,8 +768,11 @@ inline void step_forward(WideStream& w, const DevCtx& c, const StepPlan& p, int 
     } else {
       step_product<STEP_SWIGLU>(w, product(L.wgu, c.xn, c.xact, nt_i, kc_h, 1, md.inter), ctas, smem_max, err);
     }
+    w.mark(SID_GU);
     partial(L.wd, c.xact, c.part_rs[1], nt_h, kc_i, c.splits_down, md.h);
+    w.mark(SID_DOWN);
     step_norm(w, c, T, c.splits_down, c.part_rs[1], l + 1 < md.layers ? c.layer[l + 1].ln1 : c.final_norm);
+    w.mark(SID_DOWN_NORM);
   }
   for (int i = 0; i < p.n_lm; ++i) {
     StepGemm g = product(c.lm_head, c.xn, i == 0 && p.want_logits ? c.logits : nullptr, nt_v, kc_h, 1, md.vocab);
@@ -769,6 +780,7 @@ inline void step_forward(WideStream& w, const DevCtx& c, const StepPlan& p, int 
     g.keys = c.argmax_keys + (size_t)p.parity * c.T_cap;
     step_product<STEP_HEAD>(w, g, ctas, smem_max, err);
   }
+  w.mark(SID_LM);
 }
 
 }  // namespace jf

@@ -230,12 +230,27 @@ __global__ void __launch_bounds__(1024) wide_argmax_kernel(const float* __restri
 }
 
 // ---- host ----------------------------------------------------------------------------------------------------------------------------
+// Ends of a forward's stages on the device, for a stage profile: an event behind each (jf_profile_enable).
+struct StageClock {
+  std::vector<cudaEvent_t> events;                              // the first: the forward's start
+  std::vector<int> ids;
+  void mark(cudaStream_t s, int id) {
+    cudaEvent_t e;
+    if (cudaEventCreate(&e) != cudaSuccess) return;
+    events.push_back(e); ids.push_back(id);
+    cudaEventRecord(e, s);
+  }
+  ~StageClock() { for (cudaEvent_t e : events) cudaEventDestroy(e); }
+};
+
 // The launches of a forward: behind the first that fails nothing else is launched (a stage over what another one did not make would
 // leave keys and values of stale rows in the pages).
 struct WideStream {
   cudaStream_t s;
   int launches = 0;
   const char* failed = nullptr;                                 // what failed first
+  StageClock* clock = nullptr;                                  // of a profiled forward
+  void mark(int id) { if (clock && !failed) clock->mark(s, id); }
   template <typename... P, typename... A>
   void launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, A&&... args) {
     if (failed) return;

@@ -173,7 +173,8 @@ class JacobiRuntime:
 
     def profile_read(self) -> dict:
         """Per grid barrier of the profiled forward: microseconds CTA 0 spent working in the stage that ends at the
-        barrier and waiting at it; stage names follow the kernel's static schedule."""
+        barrier and waiting at it; stage names follow the kernel's static schedule.  Per kernel, or group of kernels, of a forward by stages: its microseconds, one behind
+        the other, and no waiting."""
         stamps = np.zeros(4096, np.int64)
         n, khz = C.c_int32(0), C.c_int32(0)
         _cabi.check(self.lib.jf_profile_read(self.h, stamps.ctypes.data_as(C.POINTER(C.c_int64)), 4096, C.byref(n),

@@ -169,6 +169,29 @@ def test_sampling_between_greedy_calls(both):
     same(got)
 
 
+def test_profiles(both):
+    """Of a run's second forward, on either path: nothing comes out otherwise, and the stages' times add up to less than the run's."""
+    cfg, rts = both
+    got = []
+    for rt in rts:
+        mine = {}
+        for forward in (-1, 1, -1):
+            rt.profile_enable(forward)
+            seqs, results, run = hf_generate(rt, [tokens(25, 11, cfg.vocab_size)], n=16, max_new_tokens=30, mode="single", pad=0, rngs=[random.Random(4)])
+            mine["tokens%d" % len(mine)] = np.array(results[0].tokens)
+            rt.release(seqs[0])
+            if forward == 1:
+                stages = rt.profile_read()["stages"]
+                names = [s["stage"] for s in stages]
+                for name in ("embed+norm", "L0.attention", "lm_head_argmax"):
+                    assert name in names, names
+                assert all(s["work_us"] > 0.0 for s in stages if "attention" in s["stage"])
+                assert sum(s["work_us"] + s["wait_us"] for s in stages) < 1e3 * run["device_ms"]
+        assert mine["tokens0"].tolist() == mine["tokens1"].tolist() == mine["tokens2"].tolist()
+        got.append(mine)
+    same(got)
+
+
 @pytest.fixture(scope="module", params=["qwen2-0.5b", "qwen2.5-coder-7b"])
 def real(request):
     """Two layers of the real widths: k-splits 3/3/8/3 and 4/5/5/1, a head of 1187 and 1188 tiles for 148 blocks."""

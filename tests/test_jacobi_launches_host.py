@@ -293,3 +293,31 @@ def test_a_sampling_run_says_nothing_about_the_calls_behind_it(fake, monkeypatch
         assert kernels(lambda: chunk(rt, 40)) == forward
     assert kernels(lambda: run(rt)) == greedy and kernels(lambda: chunk(rt, 40)) == forward
     rt.close()
+
+
+def test_a_profile_shows_the_kernels_that_run(fake, monkeypatch):
+    """Profiling a forward by stages changes nothing about which kernels run it; only marks inside the persistent kernel need that one."""
+    monkeypatch.setenv("JF_BY_STAGES", "1")
+    rt = engine()
+
+    def kernels():
+        fake.reset()
+        header(fake, T=8, G=1, max_len=8, n_lm_tasks=1, lm_rows=8)
+        header(fake, first=1, iter=1)
+        header(fake, first=2, done=1)
+        run(rt)
+        return [n for n, _ in fake.launches()]
+    plain = kernels()
+    assert rt.profile_read()["stages"] == []
+    rt.profile_enable(1)
+    assert kernels() == plain
+    layer = ["qkv_gemm", "qkv_rope", "attention", "attn_combine", "o_gemm", "o_reduce_norm", "gate_up_gemm", "down_gemm", "down_reduce_norm"]
+    assert [s["stage"] for s in rt.profile_read()["stages"]] == ["embed+norm"] + ["L%d.%s" % (i, n) for i in range(2) for n in layer] + ["lm_head_argmax"]
+    rt.profile_enable(-1)
+    assert kernels() == plain
+    rt.close()
+    monkeypatch.setenv("JF_PROF_MARKS", "marks.txt")
+    rt = engine()
+    rt.profile_enable(1)
+    assert ["persistent" in n for n in kernels()] == [True]
+    rt.close()

@@ -1,6 +1,7 @@
-"""Per-stage timing of one Jacobi forward inside the persistent kernel (run on a GPU box):
+"""Per-stage timing of one Jacobi forward, as it runs: inside the persistent kernel, or as one kernel per stage (run on a GPU box):
     python tools/stage_profile.py [--model qwen2.5-coder-7b] [--forward 3] [--gen 128]
-Prints the mean microseconds per stage kind (work of CTA 0 + wait at the grid barrier) and writes the raw rows."""
+Prints the mean microseconds per stage kind (work of CTA 0 + wait at the grid barrier; by stages the kernels' own, which overlap when nothing
+profiles them) and writes the raw rows."""
 import argparse
 import json
 import os
