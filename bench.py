@@ -293,13 +293,17 @@ def run_ours(args, rank: int, local_rank: int, world: int):
             seqs.append(s); fcs.append(fc); fcts.append(drafted)
             chs.append(mt_state_words(rng))
         torch.cuda.synchronize()
+        launched = rt.launches
         t0 = time.perf_counter()
         results, run = rt.jacobi_run(seqs, knobs, fcs, fcts, rng_states=chs)     # host buffers in, host ids out
         wall = time.perf_counter() - t0
+        by_stages = rt.launches - launched > 1
         toks = sum(len(r.tokens) for r in results)
         iters = run["forwards"]
         h2d = 4 * (B * P + B * n + B * 625 + B * pages + 3 * B) + 64 * B
         d2h = 4 * (B * (G + 3 * n + 1) + 8 * B + B * rt.max_calls) + 16
+        if by_stages:
+            d2h += 188 * (iters + 1)                 # the plan's header, which the host reads before every forward (struct PlanHdr)
         for s in seqs:
             rt.release(s)
         return {"tokens": toks, "forwards": iters, "device_ms": run["device_ms"], "wall_s": wall, "rows": run["rows"],
@@ -395,13 +399,13 @@ def run_ours(args, rank: int, local_rank: int, world: int):
                 "algorithmic_bytes_per_forward": bytes_fwd, "forwards_per_launch": fwd / max(1, len(steps)),
                 "ms_per_forward": 1e3 * dev_s / max(1, fwd)}
     prof = os.path.join(ROOT, "profiles", "traffic.json")
-    if os.path.exists(prof) and one_launch and tp == 1 and args.model == "qwen2.5-coder-7b" and B == 1:
+    if os.path.exists(prof) and tp == 1 and args.model == "qwen2.5-coder-7b" and B == 1:
         try:
-            per_fwd = json.load(open(prof)).get("dram_bytes_per_forward")
-            # ncu capture was one 32-forward launch; a bench launch runs `forwards_per_launch` forwards of the same shape
+            per_fwd = json.load(open(prof)).get("dram_bytes_per_forward" if one_launch else "dram_bytes_per_forward_by_stages")
+            # bytes of one forward of this shape; a generation runs `forwards_per_launch` of them
             roofline["traffic"] = per_fwd * roofline["forwards_per_launch"] if per_fwd else None
             roofline["traffic_source"] = ("not measured in this run: dram__bytes_read+write per forward from the ncu "
-                                          "--set full capture recorded in profiles/traffic.json, times this launch's "
+                                          "capture recorded in profiles/traffic.json, times this launch's "
                                           "forward count")
             roofline["achieved_bytes_per_launch"] = bytes_launch
         except Exception:

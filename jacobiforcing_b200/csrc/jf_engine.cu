@@ -890,11 +890,13 @@ static int run_wide(jf_engine* h, int T, const std::vector<Group>& groups, int l
 }
 
 // Whether forwards run as one kernel per stage: an engine on one GPU whose layers hold kStepWeights bytes or more (jf_step.cuh says why
-// the results are the same).  Small models keep the persistent kernel, for which a forward, and a run of any number of forwards, is one
-// launch and none of the host's time; stages would be faster there too, by tens of microseconds a forward.  us a forward, persistent ->
+// the results are the same).  The line is not where one overtakes the other: stages are the faster ones on both sides.  us a forward, persistent ->
 // stages, in a run of one sequence in blocks of 16 / of four with lookahead blocks / a planned one of 8 rows, by a layer's bytes:
 // 1.2 MB 112 -> 99 / 335 -> 148 / 197 -> 150;  5.6 MB 221 -> 193 / 543 -> 277 / 295 -> 230;  7.6 MB 587 -> 462 / 1436 -> 700 /
 // 666 -> 503;  30 MB 1287 -> 1128 / 2736 -> 1780 / 1337 -> 1175;  466 MB (7B), blocks of 32, one / eight sequences 3260 -> 3040 / 7300 -> 4340.
+// It stands where the gain of a forward stops being worth what only the persistent kernel has: a run of any number of forwards that is one launch and needs
+// nothing of the host.  By stages the host launches for 2.4 us a kernel, half the time of a forward of one sequence at 1.2 MB (50 of 99 us), 7.6 MB (288 of 462)
+// and 30 MB (560 of 1128) alike, and a host that is held up holds up the run; below the line that would buy 28 us of a forward of one sequence at most, above it 125 and more.
 // Sampling verification, tensor parallelism and marks inside the persistent kernel (JF_PROF_MARKS) keep that kernel as well.
 static bool step_pays(const jf_engine* h, bool sampling) {
   const DevCtx& c = h->hctx;

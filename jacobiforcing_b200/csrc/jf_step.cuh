@@ -4,8 +4,8 @@
 // The persistent kernel has four worker warps per SM for everything that is no product, because its roles share one block's
 // registers.  At 230 rows of the 7B shape that is what a forward waits for (us a layer, of 270: SwiGLU epilogue 24, output and down
 // epilogues 16, reduce + norm tails 42, attention 40, merge of its chunks 21, rotary stage 21).  Here every stage has the blocks that its
-// rows need, launches overlap (pdl_trigger), and a product's weight tiles travel while the stage before it still runs.  A layer at 230
-// rows so: 150 us.
+// rows need, launches overlap (pdl_trigger), and a product's weight tiles travel while the stage before it still runs.  A layer at 32 / 72 / 128 / 230
+// rows of one sequence so: 100 / 107 / 121 / 146 us (72 of them the weights' at HBM's rate).
 //
 // Same sums in the same order: k-splits and their order, 64-key chunks of the attention and their merge, the row statistic by tiles
 // of 128 columns, every rounding to bf16.  A forward so leaves the same bits whichever of the two runs it, and the choice between
@@ -648,9 +648,11 @@ inline void step_product(WideStream& w, StepGemm g, int ctas, int smem_max, int*
   for (g.cols = 32; g.cols < g.mt_rows;) g.cols <<= 1;
   const int items = g.n_tiles * g.splits * g.m_tiles, grid = std::min(items, ctas);
   g.bufs = items > grid && g.cols * (DUAL ? 4 : 2) <= 512 ? 2 : 1;
-  // Epilogue groups: one per 16 rows up to two, four where that measured faster.  A 7B forward (11 chunks of k and more a block), us, with two -> four: 24 rows
-  // the same, 40 rows 2955 -> 2905, 64 rows 3063 -> 3025, 72 rows 3095 -> 3046, 100 rows the same, 128 rows 3423 -> 3450.  With few chunks a block of 600
-  // threads starts later than it is done: 0.5B shape (5 to 10 chunks), 64 rows 1205 -> 1360.
+  // Epilogue groups: one per 16 rows up to two, four where that measured faster.  A 7B forward (12 to 60 chunks of k a block), us, with two -> four: 24 rows
+  // 2998 -> 2999, 33 rows 3023 -> 2995, 64 rows of ten layers 1235 -> 1219, 96 rows 3323 -> 3318, 100 rows 3452 -> 3435, 112 rows the same, 128 rows 3600 -> 3591
+  // (3423 -> 3450 in another run): from 96 to 128 rows it makes no difference.  With few chunks a block of 600 threads starts later than it is done: the 0.5B shape's layers (5 to 10
+  // chunks), 33 rows 1111 -> 1119, 64 rows 1197 -> 1352, 128 rows 1545 -> 1644.  Eleven stands between the two shapes; nothing in between was measured.  The head's tiles (14 and 56 chunks)
+  // take as long with either, at 24 to 128 rows of both shapes.
   const int each = (g.k_chunks + g.splits - 1) / g.splits;
   g.groups = g.mt_rows > 128 || (g.mt_rows > 32 && g.mt_rows <= 96 && each >= 11) ? 4 : g.mt_rows > 16 ? 2 : 1;
   g.xslot = (g.mt_rows * 128 + 1023) & ~1023;
@@ -711,9 +713,11 @@ inline void step_forward(WideStream& w, const DevCtx& c, const StepPlan& p, int 
   };
   // HBM has nothing to do while the rotary stage, attention and its merge run, and again while the output projection ends: the weights of
   // gate and up that come behind the stages which their own kernel fills early are asked for from L2 then, by the products of queries and
-  // outputs (`nth` 0 and 1), kStepAhead chunks of every tile each.  Few rows only, where weights are what a layer waits for: one 7B
-  // sequence in blocks of 32 100.2 -> 97.8 ms.  Four chunks from the twelfth on, twice; two 98.0, six 98.0,
-  // from the sixth 98.2; a forward of 72 rows 3140 -> 3110 us, of 128 rows 3421 -> 3460.  By the attention kernel instead, whose own keys come from HBM, 98.6 with four and 102.5 with twelve.
+  // outputs (`nth` 0 and 1), kStepAhead chunks of every tile each.  One 7B sequence in blocks of 32 100.2 -> 97.8 ms.  Four chunks from the twelfth on, twice; two
+  // 98.0, six 98.0, from the sixth 98.2.  By the attention kernel instead, whose own keys come from HBM, 98.6 with four and 102.5 with twelve.
+  // Where weights are what a layer waits for; with more rows it hides less of a layer.  A 7B forward, us, without -> with: 24 rows 3100 -> 3028, 64 rows 3188 -> 3163,
+  // 96 rows 3366 -> 3356, where the line is; beyond it no more than at it is won or lost: 100 rows 3508 -> 3482, 128 rows 3645 -> 3635 (3421 -> 3460 in another run),
+  // 160 rows 3870 -> 3843.
   auto ahead = [&](StepGemm& g, const LayerW& L, int nth) {
     const int from = kStepAheadFrom + nth * kStepAhead;
     if (T > kStepAheadRows || c.splits_gu > 1 || from + kStepAhead > kc_h || (size_t)2 * nt_i * kStepAhead * kWTileBytes > kStepAheadBytes) return;

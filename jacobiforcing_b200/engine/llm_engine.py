@@ -1,5 +1,5 @@
 """LLMEngine — request queue + step loop (inference_engine/engine/llm_engine.py:17-202).  Rank 0 lives in the caller's
-process; there is no worker RPC because a launch of the persistent kernel already covers a whole decode call."""
+process; there is no worker RPC because one call of the library already covers a whole decode call."""
 from __future__ import annotations
 
 import atexit

@@ -1,6 +1,7 @@
 """Host-side preparation of the device policy inputs (csrc/jf_policy.h).
 
-The accept / shift / re-draft state machine itself runs inside the persistent kernel; the host only turns the
+The accept / shift / re-draft state machine itself runs on the device, inside the persistent kernel or as a kernel between
+forwards; the host only turns the
 reference's floating-point knobs into the integers the device compares against, and pre-draws the random draft
 choices the reference's driver makes between calls (JacobiForcing/jacobi_forcing_inference_MR_humaneval.py:176-180,
 210-215 use the unseeded global `random`; here the RNG is an explicit argument - SURVEY.md finding 10).
