@@ -1,6 +1,6 @@
 #!/usr/bin/env python
 """bench.py — greedy Jacobi decoding throughput (tokens/sec + Jacobi iterations to fixed point), Qwen2.5-7B shape,
-block size n=32, synthetic 512-token prompt / 512 new tokens, random-init weights (BASELINE.json).
+block size n=32, synthetic 512-token prompt / 512 new tokens, random-init weights.
 
   python bench.py --gpus N --steps K --warmup W            this repo's B200 path (one process per GPU under torchrun)
   python bench.py --impl reference --gpus N --steps K ...  the reference's CPU path (oracle port) on the host cores
@@ -49,7 +49,7 @@ SHAPES = {
 
 def algorithmic_bytes_per_forward(cfg: dict, rows: float, ctx: float, batch_groups: float, tp: int = 1,
                                   shard_attention: bool = False) -> float:
-    """SURVEY.md section 8(d), per GPU: every layer weight + LM head once, committed KV once per group, in-flight KV
+    """Per GPU: every layer weight + LM head once, committed KV once per group, in-flight KV
     written and read, embedding rows gathered.  Logits are never materialised.  Tensor parallelism: the MLP and the LM
     head are sharded tp ways; the attention block (weights, KV) is sharded only with shard_attention, else replicated."""
     h, L, I, V = cfg["hidden_size"], cfg["num_hidden_layers"], cfg["intermediate_size"], cfg["vocab_size"]
@@ -64,7 +64,7 @@ def algorithmic_bytes_per_forward(cfg: dict, rows: float, ctx: float, batch_grou
 
 
 class ClockSampler:
-    """nvidia-smi clocks / throttle reasons sampled DURING the timed region (B200_PROFILING.md)."""
+    """nvidia-smi clocks / throttle reasons sampled DURING the timed region."""
     Q = ("index,clocks.sm,clocks.max.sm,power.draw,clocks_event_reasons.active,clocks_event_reasons.hw_slowdown,"
          "clocks_event_reasons.hw_thermal_slowdown,clocks_event_reasons.sw_thermal_slowdown,"
          "clocks_event_reasons.sw_power_cap")
@@ -173,7 +173,7 @@ def measured_peaks():
             p = json.load(f)
         return float(p["hbm_gbs"]), "measured (MEASURED_PEAKS.json)"
     except Exception:
-        return 6650.0, "fallback (B200_PROFILING.md)"
+        return 6650.0, "fallback (an earlier copy measurement)"
 
 
 # --------------------------------------------------------------------------------------------------------------------
@@ -248,7 +248,7 @@ def run_ours(args, rank: int, local_rank: int, world: int):
     torch.cuda.set_device(local_rank)
     device = f"cuda:{local_rank}"
     cfg = SHAPES[args.model]
-    # Layout at N GPUs (BASELINE.json north_star): ONE tensor-parallel group of N ranks - the path shards along the
+    # Layout at N GPUs: ONE tensor-parallel group of N ranks - the path shards along the
     # intermediate / vocabulary dimensions (and the heads with --tp-shard-attention), strong scaling of the batch-1
     # headline.  --tp T < N: N / T groups with independent sequence batches; --replicas: N independent engines (how the
     # reference's own sweep uses several GPUs, scripts/inference/scanning_hyperparameter_jacobi_decoding_mr.sh:31-45).

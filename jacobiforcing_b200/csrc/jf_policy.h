@@ -10,8 +10,7 @@
 //   engine policy  inference_engine/engine/jacobi_decoding.py:303-445 (fixed length L, draft[0] = cached seed)
 //   non-greedy     inference_engine/engine/jacobi_decoding_nongreedy.py:300-355 (accept draft token x with probability
 //                  p(x); on the first rejection commit a token drawn from p conditioned on != x), :385-470 (loop, next draft)
-// `num_blocks`, `active_blocks` and the block-list length are three separate things, exactly as in the reference
-// (SURVEY.md finding 5 / Appendix A).
+// `num_blocks`, `active_blocks` and the block-list length are three separate things, exactly as in the reference.
 #pragma once
 #include <stdint.h>
 

@@ -1,6 +1,6 @@
 // jf_ptx.cuh — thin inline-PTX wrappers for the sm_100a features the Jacobi hot path uses:
 // mbarrier, the bulk async-copy engine (TMA, 1-D cp.async.bulk), tcgen05 (MMA / TMEM alloc / ld / commit)
-// and the bounded-spin helpers that turn a would-be hang into a trap (a hung GPU box is a strike).
+// and the bounded-spin helpers that turn a would-be hang into a trap.
 //
 // Layout conventions shared by every kernel in this directory:
 //   * operand tiles are "K-major, 128-byte swizzle" (UMMA LayoutType::SWIZZLE_128B): a tile is R rows of

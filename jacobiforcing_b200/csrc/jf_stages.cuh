@@ -7,7 +7,7 @@
 //   stage_attention   causal GQA attention over [committed pages | in-flight rows]   layers/attention.py:133-136
 //   stage_attn_combine  split-KV merge, output in the O-projection's operand layout
 //   stage_commit      accepted in-flight K/V -> paged cache (replaces DynamicCache trim / trim_kv_only_fast)
-// Rounding points follow the HF bf16 modules (SURVEY.md Appendix D): linear outputs, RMSNorm (fp32 statistics, bf16
+// Rounding points follow the HF bf16 modules: linear outputs, RMSNorm (fp32 statistics, bf16
 // normalised value times bf16 weight), rotary products and sums, residual adds are each rounded to bf16.
 #pragma once
 #include <type_traits>
@@ -366,7 +366,7 @@ __device__ __noinline__ void gemm_norm_tail_impl(const DevCtx& c, const WorkerSh
   // they are there) and added per row in the canonical order (lane l: tiles l, l+16, ...; 16-lane xor tree); the row
   // itself is read back from `hidden` (this thread's own store) in the same round trip.  NB = 4 for forwards whose CTAs
   // own several row steps; Jacobi-sized forwards (at most one row step per CTA) run the NB = 1 body - a quarter of the code,
-  // and this code runs cold every time (DESIGN.md section 4)
+  // and this code runs cold every time
   float wt[8];
   unpack8(wraw, wt);
   auto phase2 = [&](auto nbtag) {

@@ -105,7 +105,7 @@ struct alignas(16) DevCtx {
   __nv_bfloat16* xa;                 // packed [q_dim/64][...]          attention output
   __nv_bfloat16* xact;               // packed [inter/64][...]          silu(gate)*up
   float* part;                       // [T_cap][part_splits][part_n] split-K partial sums, row-major by ROW so the live
-                                     // rows of a forward share a few 2 MB pages (TLB reach matters: see DESIGN.md)
+                                     // rows of a forward share a few 2 MB pages (TLB reach matters)
   int part_splits, part_n;
   unsigned long long* tpart;         // [kFuseRopeRows][part_splits][part_n] tagged {stage tag, fp32} partial sums of the fused QKV stage
   unsigned long long* tpart_rs[2];   // [fuse_rows][part_splits][h] the same for the fused O / down stages

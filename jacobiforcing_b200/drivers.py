@@ -1,4 +1,4 @@
-"""Drivers around the device-resident loop that mirror the reference's user-level scripts (SURVEY.md section 8 f.3):
+"""Drivers around the device-resident loop that mirror the reference's user-level scripts:
 
   profile_rows(...)      the per-prompt benchmark loop of JacobiForcing/jacobi_forcing_inference_MR_humaneval.py:152-273
                          with its CSV schema (index, task_id, prompt_tokens, new_tokens, calls, total_iterations,

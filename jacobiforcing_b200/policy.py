@@ -1,10 +1,9 @@
 """Host-side preparation of the device policy inputs (csrc/jf_policy.h).
 
 The accept / shift / re-draft state machine itself runs on the device, inside the persistent kernel or as a kernel between
-forwards; the host only turns the
-reference's floating-point knobs into the integers the device compares against, and pre-draws the random draft
-choices the reference's driver makes between calls (JacobiForcing/jacobi_forcing_inference_MR_humaneval.py:176-180,
-210-215 use the unseeded global `random`; here the RNG is an explicit argument - SURVEY.md finding 10).
+forwards; the host only turns the reference's floating-point knobs into the integers the device compares against, and
+pre-draws the random draft choices the reference's driver makes between calls (JacobiForcing/jacobi_forcing_inference_MR_humaneval.py:176-180,
+210-215 use the unseeded global `random`; here the RNG is an explicit argument).
 """
 from __future__ import annotations
 
@@ -52,7 +51,7 @@ class PolicyKnobs:
             raise ValueError("non-greedy Jacobi decoding needs temperature > 0")
         if self.mode == MODE_HF_MULTI:
             if not (1 <= self.K <= 2):
-                raise NotImplementedError("K >= 3 relies on the reference's block-list drift (SURVEY.md finding 5); "
+                raise NotImplementedError("K >= 3 relies on the reference's block-list drift; "
                                           "the device policy supports K in {1, 2}")
             if not (0 <= self.n_gram_pool_size <= POOL_MAX):
                 raise ValueError(f"n_gram_pool_size outside [0, {POOL_MAX}]")

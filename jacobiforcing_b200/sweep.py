@@ -11,7 +11,7 @@ same per-run CSV (`<run_id>_<csv basename>`, schema of drivers.CSV_COLUMNS = MR_
 `sweep_summary.csv` with the aggregate row of every grid point.  DF_FILE is a parquet / jsonl file with a `prompt` column
 (wrapped in the reference's HumanEval instruction + chat template when the tokenizer has one) or `synthetic:N:P` for N
 random prompts of P tokens (there are no datasets offline).  K >= 3 relies on a block-list drift of the reference
-(SURVEY finding 5) and is reported as unsupported, not run.
+and is reported as unsupported, not run.
 """
 from __future__ import annotations
 

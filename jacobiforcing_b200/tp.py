@@ -13,8 +13,7 @@ SUPPORTED_TP = (1, 2, 4, 8)
 
 def shard_dim(name: str, shard_attention: bool = True) -> Tuple[int, bool]:
     """(dimension to narrow or -1, applies_to_bias).  shard_attention=False: MLP-only tensor parallelism - the attention
-    block (q/k/v/o) is replicated on every rank, only gate/up/down and the LM head are sharded (SURVEY 8(e) option A:
-    one exchange per transformer block, no head-divisibility constraint)."""
+    block (q/k/v/o) is replicated on every rank, only gate/up/down and the LM head are sharded (one exchange per transformer block, no head-divisibility constraint)."""
     if name == "lm_head.weight":
         return 0, False
     if not shard_attention and "self_attn." in name:

@@ -1,6 +1,6 @@
 """CPU ORACLE (test / measurement infrastructure): the reference's HF Jacobi path timed on the host cores.
 
-`/root/reference` is Python and does not travel to the GPU box, so the timed code is the pinned restatement
+The reference is Python and its tree is not part of this repository, so the timed code is the pinned restatement
 (oracle/jacobi_policy.py, bit-exact against the reference's golden forwards) driving the SAME library forward the
 reference calls (transformers Qwen2 on CPU) - cpu_baseline.kind = "port".  Used only by bench.py (cpu_baseline leg and
 `--impl reference`).

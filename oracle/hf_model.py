@@ -1,12 +1,12 @@
 """CPU ORACLE (test infrastructure, not product code): the Qwen2 forward the reference's Jacobi functions call.
 
-The arithmetic of the hot path is NOT in /root/reference: modeling/cllm2_..._multiblock_lookahead_unified.py:429-463 calls
+The arithmetic of the hot path is NOT in the reference: modeling/cllm2_..._multiblock_lookahead_unified.py:429-463 calls
 `self.model.embed_tokens`, `self.model.rotary_emb`, every `Qwen2DecoderLayer`, `self.model.norm` and `self.lm_head`
 of the third-party `transformers` package (pinned transformers==4.53.0 in requirements.txt:97; this image has 5.5.0,
 whose Qwen2 math is unchanged: fp32 RMSNorm statistics with a bf16 weight multiply, bf16 rotary tables, GQA, SwiGLU).
 This module therefore does not restate the math - it *executes* the same library the reference executes, on CPU,
-behind the small `fwd` interface oracle/jacobi_policy.py drives.  No golden logits exist in the reference
-(SURVEY.md section 4), so floating-point parity is "unpinned" beyond: same library, same weights, same inputs.
+behind the small `fwd` interface oracle/jacobi_policy.py drives.  No golden logits exist in the reference,
+so floating-point parity is "unpinned" beyond: same library, same weights, same inputs.
 
 Also here: the seeded random-init checkpoints every test / bench uses (there are no model files offline).
 """
@@ -17,7 +17,7 @@ from typing import Dict, List, Optional, Sequence
 
 import torch
 
-# Published shapes (HF model cards); the reference ships no config.json (SURVEY.md section 8).
+# Published shapes (HF model cards); the reference ships no config.json.
 QWEN_SHAPES: Dict[str, dict] = {
     # small shapes the CUDA path supports (head_dim in {64,128}, hidden % 64 == 0) for fast CPU parity runs
     "tiny": dict(hidden_size=256, num_hidden_layers=2, num_attention_heads=4, num_key_value_heads=2, head_dim=64,

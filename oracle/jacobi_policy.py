@@ -2,7 +2,7 @@
 decoding state machines.  Only tests/, __graft_entry__.smoke() and bench.py's cpu_baseline/reference arm may import
 this module; the product path (jacobiforcing_b200/) never does.
 
-Every function restates one reference function and cites it (paths relative to /root/reference):
+Every function restates one reference function and cites it (paths within the reference):
 
   hf_prefill            modeling/cllm2_qwen2_modeling_kv_terminate_on_eos_improved_multiblock_lookahead_unified.py:175-225
   hf_single_block       modeling/cllm2_qwen2_modeling_kv_terminate_on_eos_improved.py:140-276
@@ -20,7 +20,7 @@ The model is reached only through a small "forward" object mirroring what the re
   fwd.trim(n)             -> None                     delete_false_key_value(n) (:36-59); n <= 0 is a no-op
 
 greedy[b][j] = argmax of the logits at position j of row b (first index wins ties, torch.argmax on CPU).
-Pinned against the unmodified reference run in this container: tests/golden/*.json (generated by oracle/make_golden.py).
+Pinned against the unmodified reference: tests/golden/*.json (generated by oracle/make_golden.py).
 """
 from __future__ import annotations
 
@@ -151,7 +151,7 @@ def hf_multiblock(fwd, input_ids: Sequence[int], n: int, K: int = 2, r: float = 
                   lookahead_start_ratio: float = 0.0, n_gram_pool_size: int = 4, eos: Optional[int] = None,
                   pad: Optional[int] = None, max_iteration_count: int = 128, trace: Optional[Trace] = None):
     """Returns (next_token or None, accepted tokens, iters).  `num_blocks`, `active_blocks` and the list index
-    space are three separate things, exactly as in the reference (SURVEY.md finding 5 / Appendix A)."""
+    space are three separate things, exactly as in the reference."""
     pool: deque = deque(maxlen=n_gram_pool_size)           # :238
     out_acc: List[List[int]] = [[]]                        # :249  accepted prefix per block (always one row)
     q_draft: List[List[List[int]]] = [[[int(t) for t in input_ids]]]   # :252 rows x L per block
@@ -322,7 +322,7 @@ def hf_multiblock(fwd, input_ids: Sequence[int], n: int, K: int = 2, r: float = 
 
 
 # --------------------------------------------------------------------------------------------------------------
-# driver protocol (MR_humaneval.py:152-250): explicit RNG so iteration counts are reproducible (SURVEY finding 10)
+# driver protocol (MR_humaneval.py:152-250): explicit RNG so iteration counts are reproducible
 # --------------------------------------------------------------------------------------------------------------
 @dataclass
 class DriverResult:

@@ -1,7 +1,7 @@
 """CPU ORACLE tooling: generate tests/golden/*.json by running the UNMODIFIED reference functions (under
 oracle/ref_shim.py) on seeded random-init Qwen2 models, through a driver loop that follows
 JacobiForcing/jacobi_forcing_inference_MR_humaneval.py:152-240 call for call but draws its random draft tokens from
-an explicit random.Random(seed) (the reference uses the unseeded global RNG - SURVEY.md finding 10).
+an explicit random.Random(seed) (the reference uses the unseeded global RNG).
 
 Run here (needs /root/reference):   python -m oracle.make_golden
 Each golden file records, for one (model, prompt, knobs) case:
@@ -199,9 +199,8 @@ def main():
     run_case("multi_n8_k3_quirk", "tiny", 0, 24, 8, 40, "multiblock", K=3, r=0.5, pool=4, max_iteration_count=40)
 
 
-def main_r2():
-    """Round-2 additions: the headline block size n=32 and the README-recommended n=64
-    (config 5), single block and multiblock + rejection recycling."""
+def main_headline():
+    """The headline block size n=32 and the README-recommended n=64, single block and multiblock + rejection recycling."""
     torch.set_num_threads(max(1, os.cpu_count() or 1))
     run_case("single_n32", "tiny", 11, 40, 32, 64, "single")
     run_case("multi_n32_k2_pool4", "tiny", 12, 40, 32, 96, "multiblock", K=2, r=0.85, pool=4)
@@ -211,7 +210,7 @@ def main_r2():
 if __name__ == "__main__" and "--engine" not in sys.argv and "--r2" not in sys.argv:
     main()
 if __name__ == "__main__" and "--r2" in sys.argv:
-    main_r2()
+    main_headline()
 
 
 # --------------------------------------------------------------------------------------------------------------------

@@ -1,9 +1,9 @@
-"""CPU ORACLE tooling (not product code): run the UNMODIFIED reference Jacobi functions in this container.
+"""CPU ORACLE tooling (not product code): run the UNMODIFIED reference Jacobi functions.
 
 The reference pins transformers 4.53.0 (requirements.txt:97); this image has 5.5.0.  Five monkey-patches, applied to
 `transformers` (never to the reference files, which are imported as they lie under /root/reference), make
 modeling/cllm2_qwen2_modeling_kv_terminate_on_eos_improved_multiblock_lookahead_unified.py and
-modeling/cllm2_qwen2_modeling_kv_terminate_on_eos_improved.py run on CPU (SURVEY.md Appendix E):
+modeling/cllm2_qwen2_modeling_kv_terminate_on_eos_improved.py run on CPU:
 
   1. Qwen2DecoderLayer.attention_type        attribute read at unified.py:207,455; removed in transformers 5
   2. Qwen2DecoderLayer.forward               accept legacy `past_key_value=` / `cache_position=`, return a 1-tuple
@@ -13,7 +13,7 @@ modeling/cllm2_qwen2_modeling_kv_terminate_on_eos_improved.py run on CPU (SURVEY
                                              `input_embeds` -> `inputs_embeds`
   5. DynamicCache.delete_false_key_value     re-bound to the multiblock module's guarded version (import-order hazard)
 
-/root/reference does not exist on the GPU box: only oracle/make_golden.py (run here, output committed under
+Machines without /root/reference have what it made: only oracle/make_golden.py (run here, output committed under
 tests/golden/) and the `-m "not gpu"` pinning test that skips when the reference is absent use this module.
 """
 from __future__ import annotations

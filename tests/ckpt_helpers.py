@@ -1,6 +1,6 @@
 """Synthetic checkpoint directory (there are no model files offline): what `LLM("<dir>")` needs from disk - config.json,
 *.safetensors with the HF tensor names the reference's loader walks (inference_engine/utils/loader.py:12-47) and the
-files AutoTokenizer reads - written the way SURVEY.md section 8(c) probed: Qwen2ForCausalLM.save_pretrained(safe
+files AutoTokenizer reads - written as Qwen2ForCausalLM.save_pretrained(safe
 serialization) + a PreTrainedTokenizerFast over a WordLevel vocabulary."""
 from __future__ import annotations
 

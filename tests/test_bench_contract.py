@@ -1,5 +1,5 @@
 """bench.py contract on a CPU-only box: the reference arm (`--impl reference`, the reference's CPU path = the oracle
-port) runs on a tiny shape and prints ONE JSON line with the keys the driver reads; non-zero ranks print nothing."""
+port) runs on a tiny shape and prints ONE JSON line with the contract's keys; non-zero ranks print nothing."""
 import json
 import os
 import subprocess

@@ -1,4 +1,4 @@
-"""Size-independent properties at BASELINE.json's full size (Qwen2.5-7B shape, random-init, n=32) - the sizes the CPU
+"""Size-independent properties at full size (Qwen2.5-7B shape, random-init, n=32) - the sizes the CPU
 oracle cannot reach in test time:
   * Jacobi(n=32) ids == autoregressive (n=1) ids, bit for bit (the fixed-point property the reference's tests pin,
     inference_engine/tests/test_jacobi_decoding_greedy.py:180-206, exact here by construction of the attention chunks)

@@ -3,11 +3,11 @@
 Floating point: the device computes in bf16 with fp32 accumulation at the HF modules' rounding points.  Tolerance on
 logits: max |d| <= 2.5e-2 and mean |d| <= 4e-3 against the fp32 HF forward with the same bf16-rounded weights (logits of
 magnitude ~1-4, where one bf16 ulp is 0.0078-0.0156: the reference's own bf16 logits are quantised coarser than the
-1e-3 the north star quotes, so 1e-3 is only meaningful for fp16/fp32 activations).  The test also requires the device
+an absolute 1e-3, which is only meaningful for fp16/fp32 activations).  The test also requires the device
 to be no further from the fp32 oracle than 1.5x the reference-dtype (HF bf16 on CPU) forward is.
 Integer work (accepted ids, iteration counts, forwards issued) is bit-exact against the oracle policy driven by the
 device forward; against the HF-forward oracle, a token mismatch is accepted only where the oracle's top-2 margin is a
-near-tie (hard part 1).
+near-tie.
 """
 import random
 
@@ -89,7 +89,7 @@ def test_prefill_chunked_equals_unchunked(pair):
 CASES = [("single", 8, 40, dict()), ("multiblock", 8, 40, dict(K=2, r=0.85, pool=4)),
          ("multiblock", 16, 64, dict(K=2, r=0.5, pool=8)), ("multiblock", 8, 32, dict(K=1, r=0.85, pool=1)),
          ("multiblock", 8, 40, dict(K=2, r=0.85, pool=4, lsr=0.5)),
-         # the headline block size and the README-recommended n=64 (config 5)
+         # the headline block size and the README-recommended n=64
          ("single", 32, 96, dict()), ("multiblock", 32, 96, dict(K=2, r=0.85, pool=4)),
          ("multiblock", 64, 160, dict(K=2, r=0.85, pool=4)), ("multiblock", 32, 64, dict(K=2, r=0.5, pool=8))]
 
@@ -144,7 +144,7 @@ def test_device_loop_equals_oracle_policy_bit_exact(pair, mode, n, max_new, kw):
 
 
 def test_batch8_multiblock_equals_oracle_policy_bit_exact():
-    """BASELINE config 3 shape of work (B=8 multiblock + rejection recycling, n=32): every sequence of the batched
+    """The shape of work of a served batch (B=8 multiblock + rejection recycling, n=32): every sequence of the batched
     device-resident loop equals the oracle policy run on that sequence alone (ids, per-call iterations, stop reason)."""
     from jacobiforcing_b200.runtime import hf_generate
     from tests.gpu_helpers import make_pair

@@ -1,4 +1,4 @@
-"""GPU parity at the BASELINE widths (-m gpu): a 2-layer model with Qwen2.5-7B's hidden 3584 / intermediate 18944 /
+"""GPU parity at the 7B widths (-m gpu): a 2-layer model with Qwen2.5-7B's hidden 3584 / intermediate 18944 /
 vocabulary 152064 / 28:4 GQA heads of 128 - the shapes whose tiling the toy models do not reach (5-way split-K, 1188
 vocabulary tiles, 7 query heads per KV head) - against the HF fp32 oracle (transformers Qwen2 on CPU, the library the
 reference's modeling/..._multiblock_lookahead_unified.py:429-463 calls).  Two layers keep the oracle at seconds per

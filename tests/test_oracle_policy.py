@@ -5,7 +5,7 @@
               restatement, driven by a table-lookup forward, must issue the SAME forwards and return the SAME ids and
               iteration counts - no model, no floating point, machine independent.
   * hf:       the same cases re-run with the HF-transformers forward (oracle/hf_model.py) on the seeded model.
-  * live:     when /root/reference is present (this container, not the GPU box) the reference is re-run and compared.
+  * live:     when the reference's tree is present the reference is re-run and compared.
 """
 import glob
 import json
@@ -108,7 +108,7 @@ def test_hf_forward_matches_reference(case):
 def test_live_reference_matches_golden(case):
     from oracle import ref_shim
     if not ref_shim.reference_available():
-        pytest.skip("reference tree not present (GPU box)")
+        pytest.skip("reference tree not present")
     import torch
     from oracle import make_golden
     g = load(case)

@@ -1,4 +1,4 @@
-"""Per-stage timing of one Jacobi forward, as it runs: inside the persistent kernel, or as one kernel per stage (run on a GPU box):
+"""Per-stage timing of one Jacobi forward, as it runs: inside the persistent kernel, or as one kernel per stage:
     python tools/stage_profile.py [--model qwen2.5-coder-7b] [--forward 3] [--gen 128]
 Prints the mean microseconds per stage kind (work of CTA 0 + wait at the grid barrier; by stages the kernels' own, which overlap when nothing
 profiles them) and writes the raw rows."""
